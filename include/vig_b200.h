@@ -127,6 +127,22 @@ VIG_API int vig_bigla_bwd(const void* q, const void* k, const void* v, const voi
                   void* workspace, size_t workspace_bytes, void* stream);
 
 /*
+ * The whole backward in one call: like vig_bigla_bwd, but with the forward's gate form (gate_logit_normalizer > 0: raw
+ * logits; clamp_min: NaN = none) and with finished gate gradients dg_* = d loss / d g_* ([B,H,L,dk] contiguous, input dtype,
+ * or fp32 with dg_fp32 != 0).  (dk, dv) of (16,32), (32,32), (32,64), (64,64) with 16-byte-aligned rows run on the tensor
+ * cores with operands split into bf16 terms (16 mantissa bits for 16-bit inputs, 24 for fp32), chunks whose gates leave the
+ * factorisation's range and all other calls token by token in fp32.
+ */
+VIG_API size_t vig_bigla_bwd_full_workspace_bytes(int B, int H, int L, int dk, int dv);
+VIG_API int vig_bigla_bwd_full(const void* q, const void* k, const void* v, const void* g_fwd, const void* g_bwd, const void* d_out,
+                  void* dq, void* dk_out, void* dv_out, void* dg_fwd, void* dg_bwd, int dg_fp32,
+                  int B, int H, int L, int dk, int dv, int dtype,
+                  const int64_t* strides_q, const int64_t* strides_k, const int64_t* strides_v,
+                  const int64_t* strides_gf, const int64_t* strides_gb, const int64_t* strides_do,
+                  float scale, float out_scale, float gate_logit_normalizer, float clamp_min, int dir_mask,
+                  void* workspace, size_t workspace_bytes, void* stream);
+
+/*
  * Bi-GLA forward for callers that cannot allocate device memory (no counterpart in the reference: its
  * operators allocate their temporaries through PyTorch on every call).
  *

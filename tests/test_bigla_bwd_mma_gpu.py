@@ -1,0 +1,44 @@
+"""Tensor-core backward of bi-GLA (vig_bigla_bwd_full) where it can go wrong: chunk edges (64 tokens), a lone chunk, every
+head size, chunks whose gates leave the factorisation's range (exact per-chunk form), unaligned strides (exact form)."""
+import pytest
+import torch
+
+import oracle
+from conftest import rel_err
+from test_bigla_bwd_gpu import _reference_grads
+
+pytestmark = pytest.mark.gpu
+NAMES = ["dq", "dk", "dv", "dg_fwd", "dg_bwd"]
+
+
+# fp32: operands carry 24 bits, what remains is the rounding of 64-token cumulative gates of up to 24 (2^-24 * 24 = 1.4e-6
+# per factor) summed over a few factors; 16-bit types: the rounding of the results (2^-9, 2^-12) against the max norm.
+TOL = {torch.float32: 2e-5, torch.bfloat16: 5e-3, torch.float16: 1e-3}
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("L,dk,dv,dir_mask,strength", [(63, 64, 64, 3, 1.0), (64, 32, 64, 3, 1.0), (65, 64, 64, 3, 1.0), (128, 16, 32, 3, 1.0),
+                                                        (193, 32, 32, 1, 1.0), (129, 64, 64, 2, 1.0), (150, 64, 64, 3, 60.0), (40, 32, 64, 3, 60.0)])
+def test_gradients_at_chunk_edges(dtype, L, dk, dv, dir_mask, strength):
+    import vig_b200
+    q, k, v, gf, gb = oracle.make_bigla_inputs(2, 2, L, dk, dv, seed=L + dk)
+    gf = gf * strength                                       # 60: every chunk of the forward direction leaves the range
+    q, k, v, gf, gb = (t.to(dtype) for t in (q, k, v, gf, gb))
+    d_out = torch.randn(2, 2, L, dv, generator=torch.Generator().manual_seed(1)).to(dtype)
+    _, ref = _reference_grads(q.float(), k.float(), v.float(), gf.float(), gb.float(), d_out.float(), 0.5, dir_mask)
+    got = vig_b200.bi_gla_backward(*[t.cuda() for t in (q, k, v, gf, gb, d_out)], out_scale=0.5, dir_mask=dir_mask)
+    errs = {n: rel_err(g.float(), r) for n, g, r in zip(NAMES, got, ref) if g is not None}
+    assert all(e < TOL[dtype] for e in errs.values()), errs
+
+
+def test_unaligned_rows_take_the_exact_form():
+    import vig_b200
+    B, H, L, d = 1, 2, 70, 32
+    q, k, v, gf, gb = oracle.make_bigla_inputs(B, H, L, d, d, seed=4)
+    d_out = torch.randn(B, H, L, d, generator=torch.Generator().manual_seed(2))
+    _, ref = _reference_grads(q, k, v, gf, gb, d_out, 1.0, 3)
+    odd = torch.zeros(B, H, L, d + 1, device="cuda")
+    odd[..., 1:] = q.cuda()
+    got = vig_b200.bi_gla_backward(odd[..., 1:], *[t.cuda() for t in (k, v, gf, gb, d_out)])
+    errs = {n: rel_err(g.float(), r) for n, g, r in zip(NAMES, got, ref)}
+    assert all(e < 2e-5 for e in errs.values()), errs

@@ -1,0 +1,546 @@
+// Backward of the bi-directional gated linear attention on the tensor cores: gradients of q, k, v and of both gate tensors
+// (finished: cumulative sums and the derivative of the gate transform included).  Replaces, for the merged operator, the
+// reference's FusedChunkGLAFunction.backward (flash-linear-attention/fla/ops/gla/chunk_fuse.py:413-518).
+//
+// Per scan direction, chunks of 64 tokens, in scan order: G_i inclusive cumulative log-gate, r its value at the chunk's
+// middle, l its total, S the state entering the chunk, Z the adjoint state entering it from the far side, c = scale:
+//   Qt = c q 2^(G-r),  Kt = k 2^(r-G),  P = mask(dO V^T),  A^T = mask(Kt Qt^T)
+//   dQ = c 2^(G-r) (P Kt + dO (2^r S)^T)           dK = 2^(r-G) (P^T Qt + V (2^(l-r) Z)^T)
+//   dV = A^T dO + Kt (2^(l-r) Z)                   e  = dQ q - dK k
+//   dg_t = <S_next, Z> over value columns + sum of e over the chunk's tokens scanned at or after t
+// The first term of dg is the gate gradient just past the chunk: d loss / d g_T = <a_T S_{T-1}, D_T> = <S_{T-1}, Z_T>, so no
+// sum ever runs over the whole sequence.  Three launches: chunk states (U = (k 2^(l-G))^T V and its adjoint), a scan over
+// chunks, chunk gradients.  A chunk whose |G - r| exceeds the range set below raises its flag and is left to the exact
+// token-by-token kernel, which runs afterwards and returns at once for every other chunk.
+#include "bigla_bwd.cuh"
+#include "mma_common.cuh"
+
+namespace vig {
+namespace {
+
+using namespace mm;
+static_assert(C == BWD_CHUNK, "both forms share the workspace");
+
+// Largest |G - r| (log2 units) of the factorised form.  The exponent's own rounding grows with it (2^-24 |G|): 24 keeps it
+// below 2e-6 for fp32 callers, 96 below 1e-5 for 16-bit ones and every scaled operand inside bf16's exponent range.
+template <typename T> __device__ __forceinline__ float range_limit() { return sizeof(T) == 4 ? 24.f : 96.f; }
+
+template <typename T> __device__ __forceinline__ const T* head_ptr(const void* base, const int64_t* s, int b, int h, int64_t t0) {
+    return reinterpret_cast<const T*>(base) + b * s[0] + h * s[1] + t0 * s[2];
+}
+
+// ---- chunk states: local S (scan order, from zero) and local Z (against it) of one chunk -----------------------------
+template <int DK, int DV, typename T> struct StatesSmem {
+    static constexpr uint32_t V = 0, O = V + Terms<T>::RAW * C * Pitch<DV>::B, K = O + Terms<T>::RAW * C * Pitch<DV>::B,
+                              Q = K + Terms<T>::SC * C * Pitch<DK>::B, SUM = Q + Terms<T>::SC * C * Pitch<DK>::B, BYTES = SUM + 2 * NT * 4;
+};
+
+// acc[NTILES][4] += X^T Y: X [C tokens][DK] scaled tiles (my 16 rows of X^T at column byte offset), Y [C][DV] raw tiles
+template <int DK, int DV, int NA, int NB, int NTILES> __device__ __forceinline__ void state_mma(float (*acc)[4], uint32_t x, uint32_t y, int lane) {
+    constexpr uint32_t PX = Pitch<DK>::B, PY = Pitch<DV>::B;
+    x += frag_cols<PX>(lane);
+    y += frag_rows<PY>(lane);
+#pragma unroll
+    for (int ks = 0; ks < C / 16; ++ks) {
+        uint32_t a[NA][4];
+#pragma unroll
+        for (int t = 0; t < NA; ++t) ldsm4t(x + t * C * PX + ks * 16 * PX, a[t]);
+        if constexpr (NTILES == 1) {
+            uint32_t b[NB][2];
+#pragma unroll
+            for (int t = 0; t < NB; ++t) ldsm2t(y + t * C * PY + ks * 16 * PY, b[t]);
+            mma_terms<NA, NB>(acc[0], a, b);
+        } else {
+#pragma unroll
+            for (int n = 0; n < NTILES; n += 2) {
+                uint32_t b0[NB][2], b1[NB][2];
+#pragma unroll
+                for (int t = 0; t < NB; ++t) {
+                    uint32_t r[4];
+                    ldsm4t(y + t * C * PY + ks * 16 * PY + n * 16, r);
+                    b0[t][0] = r[0]; b0[t][1] = r[1]; b1[t][0] = r[2]; b1[t][1] = r[3];
+                }
+                mma_terms<NA, NB>(acc[n], a, b0);
+                mma_terms<NA, NB>(acc[n + 1], a, b1);
+            }
+        }
+    }
+}
+
+template <int DK, int DV, typename T>
+__global__ void __launch_bounds__(NT) bwd_states_mma_kernel(const __grid_constant__ BwdParams p) {
+    using CL = ColLay<DK>;
+    using SM = StatesSmem<DK, DV, T>;
+    constexpr int RAW = Terms<T>::RAW, SC = Terms<T>::SC;
+    constexpr int MT = DK / 16, WN = 4 / MT, NC = DV / WN, NTL = NC / 8;      // warps: MT row tiles x WN column groups
+    extern __shared__ __align__(16) uint8_t smem[];
+    const uint32_t sb = tc::smem_u32(smem);
+    float* gsum = reinterpret_cast<float*>(smem + SM::SUM);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int c = blockIdx.x, bh = blockIdx.y, b = bh / p.H, h = bh % p.H;
+    const int64_t t0 = (int64_t)c * C;
+    const int n = min(C, p.L - (int)t0);
+    const int pr = threadIdx.x % CL::PAIRS, r0 = (threadIdx.x / CL::PAIRS) * CL::RPG;
+    load_raw<T, DV, RAW>(smem + SM::V, head_ptr<T>(p.v, p.sv, b, h, t0), p.sv[2], n);
+    load_raw<T, DV, RAW>(smem + SM::O, head_ptr<T>(p.dout, p.sdo, b, h, t0), p.sdo[2], n);
+    const T* qp = head_ptr<T>(p.q, p.sq, b, h, t0);
+    const T* kp = head_ptr<T>(p.k, p.sk, b, h, t0);
+    for (int dir = gridDim.z == 1 ? 0 : blockIdx.z; dir < 2; dir += gridDim.z == 1 ? 1 : 2) {
+        if (!(p.dir_mask & (1 << dir))) continue;
+        const size_t slot = ((size_t)bh * p.nchunk + c) * 2 + dir;
+        float2 G[CL::RPG], ref, tot;
+        const T* gp = dir ? head_ptr<T>(p.gb, p.sgb, b, h, t0) : head_ptr<T>(p.gf, p.sgf, b, h, t0);
+        cum_gates<DK, T>(G, ref, tot, gsum, gp, dir ? p.sgb[2] : p.sgf[2], n, dir, p.gate_norm, p.clamp_min);
+        if (r0 == 0) *reinterpret_cast<float2*>(p.ws_decay + slot * DK + 2 * pr) = tot;
+#pragma unroll
+        for (int r = 0; r < CL::RPG; ++r) {
+            float2 q = make_float2(0.f, 0.f), k = q;
+            if (r0 + r < n) { q = load2<T>(qp + (r0 + r) * p.sq[2] + 2 * pr); k = load2<T>(kp + (r0 + r) * p.sk[2] + 2 * pr); }
+            uint32_t t[SC];
+            split2<SC>(k.x * ex2_t<T>(tot.x - G[r].x), k.y * ex2_t<T>(tot.y - G[r].y), t);
+#pragma unroll
+            for (int i = 0; i < SC; ++i) *reinterpret_cast<uint32_t*>(smem + SM::K + i * C * Pitch<DK>::B + (r0 + r) * Pitch<DK>::B + pr * 4) = t[i];
+            split2<SC>(p.c * q.x * ex2_t<T>(G[r].x), p.c * q.y * ex2_t<T>(G[r].y), t);
+#pragma unroll
+            for (int i = 0; i < SC; ++i) *reinterpret_cast<uint32_t*>(smem + SM::Q + i * C * Pitch<DK>::B + (r0 + r) * Pitch<DK>::B + pr * 4) = t[i];
+        }
+        __syncthreads();
+        const int mt = warp % MT, wn = warp / MT;
+#pragma unroll
+        for (int which = 0; which < 2; ++which) {
+            float acc[NTL][4];
+#pragma unroll
+            for (int i = 0; i < NTL; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+            state_mma<DK, DV, SC, RAW, NTL>(acc, sb + (which ? SM::Q : SM::K) + mt * 32, sb + (which ? SM::O : SM::V) + wn * NC * 2, lane);
+            float* out = (which ? p.ws_Z : p.ws_S) + slot * DK * DV + (mt * 16 + (lane >> 2)) * DV + wn * NC + 2 * (lane & 3);
+#pragma unroll
+            for (int i = 0; i < NTL; ++i) {
+                *reinterpret_cast<float2*>(out + i * 8) = make_float2(acc[i][0], acc[i][1]);
+                *reinterpret_cast<float2*>(out + 8 * DV + i * 8) = make_float2(acc[i][2], acc[i][3]);
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// ---- scan over chunks: local states -> entering states, in place.  S in scan order, Z against it. ---------------------
+// A thread owns four neighbouring state values; the loads of PF chunks are in flight ahead of the dependent chain.
+__global__ void __launch_bounds__(256) bwd_scan_kernel(const __grid_constant__ BwdParams p) {
+    const int per = p.dk * p.dv / 4;
+    const int64_t it = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    const int e = (int)(it % per);
+    int64_t r = it / per;
+    const int which = (int)(r & 1); r >>= 1;
+    const int ndir = p.dir_mask == 3 ? 2 : 1;
+    const int dir = p.dir_mask == 3 ? (int)(r % 2) : p.dir_mask - 1;
+    const int64_t bh = r / ndir;
+    if (bh >= (int64_t)p.B * p.H) return;
+    const int d = e * 4 / p.dv;
+    float4* ws = reinterpret_cast<float4*>(which ? p.ws_Z : p.ws_S);
+    const bool descending = (dir != 0) != (which != 0);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    constexpr int PF = 8;
+    for (int cc0 = 0; cc0 < p.nchunk; cc0 += PF) {
+        float4 u[PF];
+        float g[PF];
+        size_t at[PF];
+#pragma unroll
+        for (int i = 0; i < PF; ++i) {
+            const int cc = min(cc0 + i, p.nchunk - 1);
+            const size_t slot = ((size_t)bh * p.nchunk + (descending ? p.nchunk - 1 - cc : cc)) * 2 + dir;
+            at[i] = slot * per + e;
+            u[i] = __ldcg(ws + at[i]);
+            g[i] = __ldcg(p.ws_decay + slot * p.dk + d);
+        }
+#pragma unroll
+        for (int i = 0; i < PF; ++i) {
+            if (cc0 + i >= p.nchunk) break;
+            ws[at[i]] = acc;
+            const float a = exp2f(g[i]);
+            acc.x = fmaf(acc.x, a, u[i].x); acc.y = fmaf(acc.y, a, u[i].y); acc.z = fmaf(acc.z, a, u[i].z); acc.w = fmaf(acc.w, a, u[i].w);
+        }
+    }
+}
+
+// ---- chunk gradients -----------------------------------------------------------------------------------------------
+template <int DK, int DV, typename T> struct GradSmem {
+    static constexpr uint32_t EP = DK + 8;                             // row pitch of the fp32 tile (floats)
+    static constexpr uint32_t V = 0, O = V + Terms<T>::RAW * C * Pitch<DV>::B, K = O + Terms<T>::RAW * C * Pitch<DV>::B,
+                              Q = K + Terms<T>::SC * C * Pitch<DK>::B, S = Q + Terms<T>::SC * C * Pitch<DK>::B,
+                              E = S + Terms<T>::SC * DK * Pitch<DV>::B, SUM = E + C * EP * 4, CARRY = SUM + 2 * NT * 4,
+                              SCL = CARRY + DK * 4, BYTES = SCL + 2 * DK * 4;
+};
+
+// fp32 state [DK][DV] times a per-row scale -> bf16 terms; with ``carry`` also carry[d] = <state[d], other[d]>
+template <int DK, int DV, int SC> __device__ __forceinline__ void load_state(uint8_t* dst, const float* st, const float* scale, const float* other, float* carry) {
+    constexpr uint32_t P = Pitch<DV>::B;
+    constexpr int TPR = DV / 4;                                          // threads per row (8 .. 16)
+#pragma unroll 4
+    for (int i0 = 0; i0 < DK * TPR; i0 += NT) {
+        const int i = i0 + threadIdx.x, d = i / TPR, v = i % TPR;
+        const float4 x = st ? __ldcg(reinterpret_cast<const float4*>(st) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float s = scale[d];
+        uint32_t ta[SC], tb[SC];
+        split2<SC>(x.x * s, x.y * s, ta); split2<SC>(x.z * s, x.w * s, tb);
+#pragma unroll
+        for (int t = 0; t < SC; ++t) *reinterpret_cast<uint2*>(dst + t * DK * P + d * P + v * 8) = make_uint2(ta[t], tb[t]);
+        if (carry) {
+            const float4 y = other ? __ldcg(reinterpret_cast<const float4*>(other) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            float a = x.x * y.x + x.y * y.y + x.z * y.z + x.w * y.w;
+#pragma unroll
+            for (int m = 1; m < TPR; m <<= 1) a += __shfl_xor_sync(0xffffffffu, a, m);
+            if (v == 0) carry[d] = a;
+        }
+    }
+}
+
+// acc[2][4] += A_rows B_rows^T over KD: A fragments of my 16 rows (tile a, [row][k]), B rows jb*16.. (tile b, [n][k])
+template <int KD, int NA, int NB> __device__ __forceinline__ void block_nt(float (*acc)[4], uint32_t a, uint32_t a_term, uint32_t b, uint32_t b_term) {
+#pragma unroll
+    for (int ks = 0; ks < KD / 16; ++ks) {
+        uint32_t fa[NA][4], b0[NB][2], b1[NB][2];
+#pragma unroll
+        for (int t = 0; t < NA; ++t) ldsm4(a + t * a_term + ks * 32, fa[t]);
+#pragma unroll
+        for (int t = 0; t < NB; ++t) {
+            uint32_t r[4];
+            ldsm4(b + t * b_term + ks * 32, r);
+            b0[t][0] = r[0]; b0[t][1] = r[1]; b1[t][0] = r[2]; b1[t][1] = r[3];
+        }
+        mma_terms<NA, NB>(acc[0], fa, b0);
+        mma_terms<NA, NB>(acc[1], fa, b1);
+    }
+}
+
+// zero the entries of a diagonal 16 x 16 block that ``keep(row, col)`` rejects, then split it into an A operand
+template <int SC, typename F> __device__ __forceinline__ void mask_split(float (*p)[4], bool diag, int lane, F keep, uint32_t (*out)[4]) {
+    if (diag) {
+        const int r = lane >> 2, q = 2 * (lane & 3);
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) if (!keep(r + 8 * (j >> 1), nt * 8 + q + (j & 1))) p[nt][j] = 0.f;
+    }
+    uint32_t t[SC];
+    split2<SC>(p[0][0], p[0][1], t);
+#pragma unroll
+    for (int i = 0; i < SC; ++i) out[i][0] = t[i];
+    split2<SC>(p[0][2], p[0][3], t);
+#pragma unroll
+    for (int i = 0; i < SC; ++i) out[i][1] = t[i];
+    split2<SC>(p[1][0], p[1][1], t);
+#pragma unroll
+    for (int i = 0; i < SC; ++i) out[i][2] = t[i];
+    split2<SC>(p[1][2], p[1][3], t);
+#pragma unroll
+    for (int i = 0; i < SC; ++i) out[i][3] = t[i];
+}
+
+// acc[ND/8][4] += A (16 x 16, registers) B: B rows of one k step in a [k][n] tile
+template <int ND, int NA, int NB> __device__ __forceinline__ void block_nn(float (*acc)[4], const uint32_t (*a)[4], uint32_t b, uint32_t b_term) {
+#pragma unroll
+    for (int n = 0; n < ND / 8; n += 2) {
+        uint32_t b0[NB][2], b1[NB][2];
+#pragma unroll
+        for (int t = 0; t < NB; ++t) {
+            uint32_t r[4];
+            ldsm4t(b + t * b_term + n * 16, r);
+            b0[t][0] = r[0]; b0[t][1] = r[1]; b1[t][0] = r[2]; b1[t][1] = r[3];
+        }
+        mma_terms<NA, NB>(acc[n], a, b0);
+        mma_terms<NA, NB>(acc[n + 1], a, b1);
+    }
+}
+
+// acc[ND/8][4] += A B^T over KD: A = my 16 rows of an [m][k] tile, B an [n][k] tile of ND rows with pitch PB
+template <int ND, int KD, uint32_t PB, int NA, int NB> __device__ __forceinline__ void rows_nt(float (*acc)[4], uint32_t a, uint32_t a_term, uint32_t b, uint32_t b_term) {
+#pragma unroll
+    for (int ks = 0; ks < KD / 16; ++ks) {
+        uint32_t fa[NA][4];
+#pragma unroll
+        for (int t = 0; t < NA; ++t) ldsm4(a + t * a_term + ks * 32, fa[t]);
+#pragma unroll
+        for (int n = 0; n < ND / 8; n += 2) {
+            uint32_t b0[NB][2], b1[NB][2];
+#pragma unroll
+            for (int t = 0; t < NB; ++t) {
+                uint32_t r[4];
+                ldsm4(b + t * b_term + n * 8 * PB + ks * 32, r);
+                b0[t][0] = r[0]; b0[t][1] = r[1]; b1[t][0] = r[2]; b1[t][1] = r[3];
+            }
+            mma_terms<NA, NB>(acc[n], fa, b0);
+            mma_terms<NA, NB>(acc[n + 1], fa, b1);
+        }
+    }
+}
+
+template <int DK, int DV, typename T>
+__global__ void __launch_bounds__(NT, 2) bwd_grads_mma_kernel(const __grid_constant__ BwdParams p) {
+    using CL = ColLay<DK>;
+    using SM = GradSmem<DK, DV, T>;
+    constexpr int RAW = Terms<T>::RAW, SC = Terms<T>::SC;
+    constexpr uint32_t PK = Pitch<DK>::B, PV = Pitch<DV>::B, EP = SM::EP;
+    constexpr uint32_t TK = C * PK, TV = C * PV, TS = DK * PV;          // bytes from one term's tile to the next
+    extern __shared__ __align__(16) uint8_t smem[];
+    const uint32_t sb = tc::smem_u32(smem);
+    float* E = reinterpret_cast<float*>(smem + SM::E);
+    float* gsum = reinterpret_cast<float*>(smem + SM::SUM);
+    float* carry = reinterpret_cast<float*>(smem + SM::CARRY);
+    float* scl = reinterpret_cast<float*>(smem + SM::SCL);              // [0]: 2^r, [1]: 2^(l-r)
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int c = blockIdx.x, bh = blockIdx.y, b = bh / p.H, h = bh % p.H;
+    const int64_t t0 = (int64_t)c * C;
+    const int n = min(C, p.L - (int)t0);
+    const int pr = threadIdx.x % CL::PAIRS, gr = threadIdx.x / CL::PAIRS, r0 = gr * CL::RPG;
+    const int fr = 16 * w + (lane >> 2), fc = 2 * (lane & 3);           // my fragment rows fr, fr + 8; columns 8 nt + fc, + 1
+    const T* qp = head_ptr<T>(p.q, p.sq, b, h, t0);
+    const T* kp = head_ptr<T>(p.k, p.sk, b, h, t0);
+    load_raw<T, DV, RAW>(smem + SM::V, head_ptr<T>(p.v, p.sv, b, h, t0), p.sv[2], n);
+    load_raw<T, DV, RAW>(smem + SM::O, head_ptr<T>(p.dout, p.sdo, b, h, t0), p.sdo[2], n);
+    const uint32_t aV = sb + SM::V + 16 * w * PV + frag_rows<PV>(lane), aO = sb + SM::O + 16 * w * PV + frag_rows<PV>(lane);
+    const uint32_t aK = sb + SM::K + 16 * w * PK + frag_rows<PK>(lane);
+    const uint32_t bV = sb + SM::V + frag_cols<PV>(lane), bO = sb + SM::O + frag_cols<PV>(lane), bQ = sb + SM::Q + frag_cols<PK>(lane);
+    const uint32_t tK = sb + SM::K + frag_rows<PK>(lane), tQ = sb + SM::Q + frag_rows<PK>(lane), tO = sb + SM::O + frag_rows<PV>(lane);
+    const uint32_t bS = sb + SM::S + frag_cols<PV>(lane), tS = sb + SM::S + frag_rows<PV>(lane);
+    float dqt[DK / 8][4], dkt[DK / 8][4], dv[DV / 8][4];
+#pragma unroll
+    for (int i = 0; i < DK / 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { dqt[i][j] = 0.f; dkt[i][j] = 0.f; }
+#pragma unroll
+    for (int i = 0; i < DV / 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dv[i][j] = 0.f;
+    const bool have_states = p.nchunk > 1;
+#pragma unroll 1
+    for (int dir = 0; dir < 2; ++dir) {
+        if (!(p.dir_mask & (1 << dir))) continue;
+        const T* gp = dir ? head_ptr<T>(p.gb, p.sgb, b, h, t0) : head_ptr<T>(p.gf, p.sgf, b, h, t0);
+        const int64_t sgl = dir ? p.sgb[2] : p.sgf[2];
+        const size_t slot = ((size_t)bh * p.nchunk + c) * 2 + dir;
+        // ---- gates, scaled operand tiles
+        {
+            float2 G[CL::RPG], ref, tot;
+            cum_gates<DK, T>(G, ref, tot, gsum, gp, sgl, n, dir, p.gate_norm, p.clamp_min);
+            const float lim = range_limit<T>();
+            bool fine = fabsf(ref.x) <= lim && fabsf(ref.y) <= lim && fabsf(tot.x - ref.x) <= lim && fabsf(tot.y - ref.y) <= lim;
+            if (gr == 0) {
+                *reinterpret_cast<float2*>(scl + 2 * pr) = make_float2(ex2_t<T>(ref.x), ex2_t<T>(ref.y));
+                *reinterpret_cast<float2*>(scl + DK + 2 * pr) = make_float2(ex2_t<T>(tot.x - ref.x), ex2_t<T>(tot.y - ref.y));
+            }
+#pragma unroll
+            for (int r = 0; r < CL::RPG; ++r) {
+                float2 q = make_float2(0.f, 0.f), k = q;
+                if (r0 + r < n) { q = load2<T>(qp + (r0 + r) * p.sq[2] + 2 * pr); k = load2<T>(kp + (r0 + r) * p.sk[2] + 2 * pr); }
+                const float x = G[r].x - ref.x, y = G[r].y - ref.y;
+                fine = fine && fabsf(x) <= lim && fabsf(y) <= lim;
+                const float ex = ex2_t<T>(x), ey = ex2_t<T>(y);
+                *reinterpret_cast<float2*>(E + (r0 + r) * EP + 2 * pr) = make_float2(ex, ey);
+                uint32_t t[SC];
+                split2<SC>(p.c * q.x * ex, p.c * q.y * ey, t);
+#pragma unroll
+                for (int i = 0; i < SC; ++i) *reinterpret_cast<uint32_t*>(smem + SM::Q + i * TK + (r0 + r) * PK + pr * 4) = t[i];
+                split2<SC>(k.x * ex2_t<T>(-x), k.y * ex2_t<T>(-y), t);
+#pragma unroll
+                for (int i = 0; i < SC; ++i) *reinterpret_cast<uint32_t*>(smem + SM::K + i * TK + (r0 + r) * PK + pr * 4) = t[i];
+            }
+            if (__syncthreads_or(!fine)) {                               // left to the exact kernel, outputs included
+                if (threadIdx.x == 0) p.flags[(size_t)bh * p.nchunk + c] = 1;
+                return;
+            }
+        }
+        const int klo = dir ? w : 0, khi = dir ? C / 16 : w + 1;         // 16-token blocks scanned at or before mine
+        const int qlo = dir ? 0 : w, qhi = dir ? w + 1 : C / 16;         // ... at or after mine
+        const int next = dir ? c - 1 : c + 1;                           // the chunk scanned after this one
+        const bool last = next < 0 || next >= p.nchunk;
+        if (have_states) {
+            load_state<DK, DV, SC>(smem + SM::S, p.ws_S + slot * DK * DV, scl, nullptr, nullptr);
+            __syncthreads();
+        }
+        float ev[DK / 8][4];
+        {   // ---- dQ of my rows
+            float dq[DK / 8][4];
+#pragma unroll
+            for (int i = 0; i < DK / 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) dq[i][j] = 0.f;
+#pragma unroll 1
+            for (int jb = klo; jb < khi; ++jb) {
+                float pb[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+                uint32_t ap[SC][4];
+                block_nt<DV, RAW, RAW>(pb, aO, TV, bV + jb * 16 * PV, TV);
+                mask_split<SC>(pb, jb == w, lane, [&](int r, int j) { return dir ? j >= r : j <= r; }, ap);
+                block_nn<DK, SC, SC>(dq, ap, tK + jb * 16 * PK, TK);
+            }
+            if (have_states) rows_nt<DK, DV, PV, RAW, SC>(dq, aO, TV, bS, TS);
+#pragma unroll
+            for (int i = 0; i < DK / 8; ++i)
+#pragma unroll
+                for (int hf = 0; hf < 2; ++hf) {
+                    const int row = fr + 8 * hf, col = 8 * i + fc;
+                    const float2 ex = *reinterpret_cast<const float2*>(E + row * EP + col);
+                    const float2 q = row < n ? load2<T>(qp + row * p.sq[2] + col) : make_float2(0.f, 0.f);
+                    const float a = p.c * ex.x * dq[i][2 * hf], d = p.c * ex.y * dq[i][2 * hf + 1];
+                    dqt[i][2 * hf] += a; dqt[i][2 * hf + 1] += d;
+                    ev[i][2 * hf] = a * q.x; ev[i][2 * hf + 1] = d * q.y;
+                }
+        }
+        if (have_states) {
+            __syncthreads();                                             // S is read
+            load_state<DK, DV, SC>(smem + SM::S, p.ws_Z + slot * DK * DV, scl + DK,
+                                   last ? nullptr : p.ws_S + (((size_t)bh * p.nchunk + next) * 2 + dir) * DK * DV, carry);
+            __syncthreads();
+        }
+        {   // ---- dK and dV of my rows
+            float dk[DK / 8][4];
+#pragma unroll
+            for (int i = 0; i < DK / 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) dk[i][j] = 0.f;
+#pragma unroll 1
+            for (int ib = qlo; ib < qhi; ++ib) {
+                auto keep = [&](int j, int i) { return dir ? i <= j : i >= j; };
+                float pb[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+                uint32_t ap[SC][4];
+                block_nt<DV, RAW, RAW>(pb, aV, TV, bO + ib * 16 * PV, TV);
+                mask_split<SC>(pb, ib == w, lane, keep, ap);
+                block_nn<DK, SC, SC>(dk, ap, tQ + ib * 16 * PK, TK);
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) pb[i][j] = 0.f;
+                block_nt<DK, SC, SC>(pb, aK, TK, bQ + ib * 16 * PK, TK);
+                mask_split<SC>(pb, ib == w, lane, keep, ap);
+                block_nn<DV, SC, RAW>(dv, ap, tO + ib * 16 * PV, TV);
+            }
+            if (have_states) {
+                rows_nt<DK, DV, PV, RAW, SC>(dk, aV, TV, bS, TS);
+#pragma unroll
+                for (int ks = 0; ks < DK / 16; ++ks) {
+                    uint32_t fa[SC][4];
+#pragma unroll
+                    for (int t = 0; t < SC; ++t) ldsm4(aK + t * TK + ks * 32, fa[t]);
+                    block_nn<DV, SC, SC>(dv, fa, tS + ks * 16 * PV, TS);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < DK / 8; ++i)
+#pragma unroll
+                for (int hf = 0; hf < 2; ++hf) {
+                    const int row = fr + 8 * hf, col = 8 * i + fc;
+                    float2* e = reinterpret_cast<float2*>(E + row * EP + col);
+                    const float2 ex = *e;
+                    const float2 k = row < n ? load2<T>(kp + row * p.sk[2] + col) : make_float2(0.f, 0.f);
+                    const float a = __fdividef(dk[i][2 * hf], ex.x), d = __fdividef(dk[i][2 * hf + 1], ex.y);
+                    dkt[i][2 * hf] += a; dkt[i][2 * hf + 1] += d;
+                    *e = make_float2(ev[i][2 * hf] - a * k.x, ev[i][2 * hf + 1] - d * k.y);
+                }
+        }
+        __syncthreads();
+        {   // ---- gate gradient: sum of e over the tokens scanned at or after t, plus the value just past the chunk
+            float2 x[CL::RPG], sum = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int r = 0; r < CL::RPG; ++r) { x[r] = *reinterpret_cast<const float2*>(E + (r0 + r) * EP + 2 * pr); sum.x += x[r].x; sum.y += x[r].y; }
+            *reinterpret_cast<float2*>(gsum + gr * DK + 2 * pr) = sum;
+            __syncthreads();
+            float2 run = have_states ? *reinterpret_cast<const float2*>(carry + 2 * pr) : make_float2(0.f, 0.f);
+#pragma unroll
+            for (int o = 0; o < CL::GROUPS; ++o)
+                if (dir ? o < gr : o > gr) { const float2 s = *reinterpret_cast<const float2*>(gsum + o * DK + 2 * pr); run.x += s.x; run.y += s.y; }
+            const int64_t base = ((int64_t)bh * p.L + t0) * DK + 2 * pr;
+#pragma unroll
+            for (int rr = 0; rr < CL::RPG; ++rr) {
+                // static register indices for both orders: the backward direction sums upwards, the forward one downwards
+                const float2 xv = dir ? x[rr] : x[CL::RPG - 1 - rr];
+                const int row = r0 + (dir ? rr : CL::RPG - 1 - rr);
+                run.x += xv.x; run.y += xv.y;
+                if (row < n) {
+                    float2 dg = run;
+                    if (p.gate_norm > 0.f || p.clamp_min == p.clamp_min) {
+                        const float2 gx = load2<T>(gp + row * sgl + 2 * pr);
+                        dg.x = through_gate(dg.x, gx.x, p.gate_norm, p.clamp_min); dg.y = through_gate(dg.y, gx.y, p.gate_norm, p.clamp_min);
+                    }
+                    void* out = dir ? p.dgb : p.dgf;
+                    if (p.dg_f32) store2<float>(reinterpret_cast<float*>(out) + base + (int64_t)row * DK, dg.x, dg.y);
+                    else store2<T>(reinterpret_cast<T*>(out) + base + (int64_t)row * DK, dg.x, dg.y);
+                }
+            }
+        }
+        __syncthreads();                                                // E, gsum, carry and the tiles may be rewritten
+    }
+    if (threadIdx.x == 0) p.flags[(size_t)bh * p.nchunk + c] = 0;
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) {
+        const int row = fr + 8 * hf;
+        if (row >= n) continue;
+        const int64_t at = (int64_t)bh * p.L + t0 + row;
+#pragma unroll
+        for (int i = 0; i < DK / 8; ++i) {
+            store2<T>(reinterpret_cast<T*>(p.out_dq) + at * DK + 8 * i + fc, dqt[i][2 * hf], dqt[i][2 * hf + 1]);
+            store2<T>(reinterpret_cast<T*>(p.out_dk) + at * DK + 8 * i + fc, dkt[i][2 * hf], dkt[i][2 * hf + 1]);
+        }
+#pragma unroll
+        for (int i = 0; i < DV / 8; ++i) store2<T>(reinterpret_cast<T*>(p.out_dv) + at * DV + 8 * i + fc, dv[i][2 * hf], dv[i][2 * hf + 1]);
+    }
+}
+
+template <int DK, int DV, typename T>
+int launch_typed(const BwdParams& p, cudaStream_t stream) {
+    const int BH = p.B * p.H;
+    constexpr uint32_t smA = StatesSmem<DK, DV, T>::BYTES, smC = GradSmem<DK, DV, T>::BYTES;
+    auto kA = bwd_states_mma_kernel<DK, DV, T>;
+    auto kC = bwd_grads_mma_kernel<DK, DV, T>;
+    cudaError_t e;
+    if (p.nchunk > 1) {                                                  // one chunk: both entering states are zero
+        if ((e = tc::ensure_smem_attr(reinterpret_cast<const void*>(kA), (int)smA)) != cudaSuccess) return (int)e;
+        // few chunks: one CTA per direction, so that more of the GPU works; many: one CTA reads v and d_out once for both
+        const int gz = p.dir_mask == 3 && (int64_t)p.nchunk * BH < 148 * 4 ? 2 : 1;
+        kA<<<dim3(p.nchunk, BH, gz), NT, smA, stream>>>(p);
+        if (int s = bigla_bwd_scan_launch(p, stream)) return s;
+    }
+    if ((e = tc::ensure_smem_attr(reinterpret_cast<const void*>(kC), (int)smC)) != cudaSuccess) return (int)e;
+    kC<<<dim3(p.nchunk, BH), NT, smC, stream>>>(p);
+    return (int)cudaGetLastError();
+}
+
+template <typename T>
+int launch_dims(const BwdParams& p, cudaStream_t stream) {
+#define VIG_CASE(DKV, DVV) if (p.dk == DKV && p.dv == DVV) return launch_typed<DKV, DVV, T>(p, stream);
+    VIG_CASE(16, 32) VIG_CASE(32, 32) VIG_CASE(32, 64) VIG_CASE(64, 64)
+#undef VIG_CASE
+    return VIG_ERR_SHAPE;
+}
+
+}  // namespace
+
+int bigla_bwd_scan_launch(const BwdParams& p, cudaStream_t stream) {
+    const int64_t threads = (int64_t)p.B * p.H * (p.dir_mask == 3 ? 2 : 1) * 2 * (p.dk * p.dv / 4);
+    bwd_scan_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, stream>>>(p);
+    return (int)cudaGetLastError();
+}
+
+// Rows are read as 16-byte vectors (16-bit v, d_out) or as pairs of values: base pointers on 16 bytes, strides that are
+// multiples of 16 bytes.  Everything else, and heads whose tiles exceed the registers of one warp row (dv = 128), takes
+// the token-by-token form.  grid.y holds B*H, hence its limit.
+bool bigla_bwd_mma_supported(const BwdParams& p) {
+    if (!((p.dk == 16 && p.dv == 32) || (p.dk == 32 && p.dv == 32) || (p.dk == 32 && p.dv == 64) || (p.dk == 64 && p.dv == 64))) return false;
+    if ((int64_t)p.B * p.H > 65535) return false;
+    const int unit = p.dtype == VIG_DTYPE_F32 ? 4 : 8;
+    auto ok = [&](const void* base, const int64_t* s) {
+        return !base || (!(reinterpret_cast<uintptr_t>(base) & 15) && s[0] % unit == 0 && s[1] % unit == 0 && s[2] % unit == 0);
+    };
+    return ok(p.q, p.sq) && ok(p.k, p.sk) && ok(p.v, p.sv) && ok(p.dout, p.sdo) && ok(p.gf, p.sgf) && ok(p.gb, p.sgb);
+}
+
+int bigla_bwd_mma_launch(const BwdParams& p, cudaStream_t stream) {
+    switch (p.dtype) {
+        case VIG_DTYPE_F32: return launch_dims<float>(p, stream);
+        case VIG_DTYPE_BF16: return launch_dims<__nv_bfloat16>(p, stream);
+        case VIG_DTYPE_F16: return launch_dims<__half>(p, stream);
+    }
+    return VIG_ERR_DTYPE;
+}
+
+}  // namespace vig

@@ -12,26 +12,17 @@
 //     e_t  = dq_t * q_t - dk_t * k_t ;  dg_t = sum of e over the tokens scanned at or after t
 // The kernels are chunk-parallel like the forward SIMT path: local S and Z per 64-token chunk, a scan over
 // chunks in each direction, then one CTA per chunk that replays both recurrences from its entering states.
-// This file writes e per direction; the host wrapper takes the cumulative sums.
-#include "common.cuh"
+// Exact for any gates.  It is the whole backward where the tensor-core form (bigla_bwd_mma.cu) does not take the call, the
+// per-chunk fallback of that form, and it writes either e per direction or the finished gate gradients.
+#include <cmath>
+#include "bigla_bwd.cuh"
+#include "mma_common.cuh"
 
 namespace vig {
 namespace {
 
-constexpr int CH = 64;
+constexpr int CH = BWD_CHUNK;
 constexpr int NT = 256;
-
-struct BwdParams {
-    const void *q, *k, *v, *gf, *gb, *dout;
-    void *out_dq, *out_dk, *out_dv;  // [B,H,L,d] contiguous, input dtype
-    float *ef, *eb;                  // [B,H,L,dk] contiguous fp32
-    int64_t sq[3], sk[3], sv[3], sgf[3], sgb[3], sdo[3];
-    int B, H, L, dk, dv, dtype;
-    float c;
-    int dir_mask;
-    float *ws_S, *ws_Z, *ws_decay;   // [BH][nchunk][2][dk*dv] x2, [BH][nchunk][2][dk]
-    int nchunk;
-};
 
 template <typename T>
 __device__ __forceinline__ const T* rowp(const void* base, const int64_t* s, int b, int h, int l) {
@@ -46,15 +37,18 @@ __device__ __forceinline__ void load_tile(float* dst, const void* x, const int64
     }
 }
 
-// gates of the chunk -> per-channel sum to `sum_out` (may be null) -> decay factors exp(g) in place
+// gates of the chunk (raw logits transformed) -> per-channel sum in log2 units to `sum_out` (may be null) -> decay factors
+// exp(g) in place
 template <int DK, typename T>
-__device__ __forceinline__ void load_gates_exp(float* g, const void* src, const int64_t* sg, int b, int h, int t0, int n, float* sum_out) {
-    load_tile<DK, T>(g, src, sg, b, h, t0, n);           // rows past the end: log-gate 0, decay 1
+__device__ __forceinline__ void load_gates_exp(float* g, const BwdParams& p, int dir, int b, int h, int t0, int n, float* sum_out) {
+    load_tile<DK, T>(g, dir ? p.gb : p.gf, dir ? p.sgb : p.sgf, b, h, t0, n);           // rows past the end: log-gate 0, decay 1
+    if (p.gate_norm > 0.f || p.clamp_min == p.clamp_min)
+        for (int idx = threadIdx.x; idx < n * DK; idx += NT) g[idx] = gate_transform(g[idx], p.gate_norm, p.clamp_min);
     __syncthreads();
     if (threadIdx.x < DK && sum_out) {
         float s = 0.f;
         for (int i = 0; i < CH; ++i) s += g[i * DK + threadIdx.x];
-        sum_out[threadIdx.x] = s;
+        sum_out[threadIdx.x] = s * tc::LOG2E;
     }
     __syncthreads();
     for (int idx = threadIdx.x; idx < CH * DK; idx += NT) g[idx] = __expf(g[idx]);
@@ -88,7 +82,7 @@ __global__ void __launch_bounds__(NT) bwd_chunk_states(BwdParams p) {
         if (!(p.dir_mask & (1 << dir))) continue;
         const size_t slot = ((size_t)bh * p.nchunk + c) * 2 + dir;
         __syncthreads();
-        load_gates_exp<DK, T>(sg, dir ? p.gb : p.gf, dir ? p.sgb : p.sgf, b, h, t0, n, p.ws_decay + slot * DK);
+        load_gates_exp<DK, T>(sg, p, dir, b, h, t0, n, p.ws_decay + slot * DK);
         float st[A::DPT];
 #pragma unroll
         for (int dd = 0; dd < A::DPT; ++dd) st[dd] = 0.f;
@@ -119,35 +113,9 @@ __global__ void __launch_bounds__(NT) bwd_chunk_states(BwdParams p) {
     }
 }
 
-// ---- phase B: local states -> entering states, in place.  S is scanned in scan order, Z against it. -------------
-__global__ void __launch_bounds__(NT) bwd_state_scan(BwdParams p) {
-    const int DKDV = p.dk * p.dv;
-    const int per = (DKDV + NT - 1) / NT;
-    int blk = blockIdx.x;
-    const int part = blk % per; blk /= per;
-    const int dir = blk % 2; blk /= 2;
-    const int which = blk % 2;                                        // 0: S, 1: Z
-    const int bh = blk / 2;
-    if (!(p.dir_mask & (1 << dir))) return;
-    const int e = part * NT + threadIdx.x;
-    if (e >= DKDV) return;
-    const int d = e / p.dv;
-    float* ws = which ? p.ws_Z : p.ws_S;
-    const bool descending = (dir != 0) != (which != 0);               // chunk order of this scan
-    float acc = 0.f;
-    for (int cc = 0; cc < p.nchunk; ++cc) {
-        const int c = descending ? p.nchunk - 1 - cc : cc;
-        const size_t slot = ((size_t)bh * p.nchunk + c) * 2 + dir;
-        float* u = ws + slot * DKDV + e;
-        const float local = *u;
-        *u = acc;                                                     // state entering chunk c
-        acc = fmaf(acc, __expf(p.ws_decay[slot * p.dk + d]), local);
-    }
-}
-
 // ---- phase C: gradients of one chunk -----------------------------------------------------------------------------
 template <int DK, int DV, typename T>
-__global__ void __launch_bounds__(NT) bwd_chunk_grads(BwdParams p) {
+__global__ void __launch_bounds__(NT) bwd_chunk_grads(BwdParams p, int flagged_only) {
     using A = LayA<DK, DV>;
     using Bl = LayB<DK, DV>;
     extern __shared__ float smem[];
@@ -160,7 +128,11 @@ __global__ void __launch_bounds__(NT) bwd_chunk_grads(BwdParams p) {
     float* sv = sdk + CH * DK;
     float* sdo = sv + CH * DV;
     float* sdv = sdo + CH * DV;
-    const int c = blockIdx.x, bh = blockIdx.y, b = bh / p.H, h = bh % p.H;
+    const bool have_states = !flagged_only || p.nchunk > 1;          // the tensor-core form leaves the states of a lone chunk unwritten (zero)
+    const int items = p.nchunk * p.B * p.H;
+    for (int item = blockIdx.x; item < items; item += gridDim.x) {
+    if (flagged_only && !p.flags[item]) continue;
+    const int c = item % p.nchunk, bh = item / p.nchunk, b = bh / p.H, h = bh % p.H;
     const int t0 = c * CH, n = min(CH, p.L - t0);
     load_tile<DK, T>(sq, p.q, p.sq, b, h, t0, n);
     load_tile<DK, T>(sk, p.k, p.sk, b, h, t0, n);
@@ -172,13 +144,13 @@ __global__ void __launch_bounds__(NT) bwd_chunk_grads(BwdParams p) {
         if (!(p.dir_mask & (1 << dir))) continue;
         const size_t slot = ((size_t)bh * p.nchunk + c) * 2 + dir;
         __syncthreads();
-        load_gates_exp<DK, T>(sg, dir ? p.gb : p.gf, dir ? p.sgb : p.sgf, b, h, t0, n, nullptr);
+        load_gates_exp<DK, T>(sg, p, dir, b, h, t0, n, nullptr);
         {   // layout B: dq from the rebuilt state (scan order), then dk from Z (reverse scan order)
             const int d = threadIdx.x / Bl::TPB, s = threadIdx.x % Bl::TPB;
             float st[Bl::JPT];
             const float* Sin = p.ws_S + slot * DK * DV + d * DV + s * Bl::JPT;
 #pragma unroll
-            for (int jj = 0; jj < Bl::JPT; ++jj) st[jj] = Sin[jj];
+            for (int jj = 0; jj < Bl::JPT; ++jj) st[jj] = have_states ? Sin[jj] : 0.f;
             for (int ii = 0; ii < n; ++ii) {
                 const int i = dir ? n - 1 - ii : ii;
                 const float a = sg[i * DK + d], kd = sk[i * DK + d];
@@ -199,7 +171,7 @@ __global__ void __launch_bounds__(NT) bwd_chunk_grads(BwdParams p) {
             }
             const float* Zin = p.ws_Z + slot * DK * DV + d * DV + s * Bl::JPT;
 #pragma unroll
-            for (int jj = 0; jj < Bl::JPT; ++jj) st[jj] = Zin[jj];
+            for (int jj = 0; jj < Bl::JPT; ++jj) st[jj] = have_states ? Zin[jj] : 0.f;
             for (int ii = n - 1; ii >= 0; --ii) {
                 const int i = dir ? n - 1 - ii : ii;
                 const float a = sg[i * DK + d], cq = p.c * sq[i * DK + d];
@@ -224,7 +196,7 @@ __global__ void __launch_bounds__(NT) bwd_chunk_grads(BwdParams p) {
             float st[A::DPT];
             const float* Zin = p.ws_Z + slot * DK * DV;
 #pragma unroll
-            for (int dd = 0; dd < A::DPT; ++dd) st[dd] = Zin[(s * A::DPT + dd) * DV + j];
+            for (int dd = 0; dd < A::DPT; ++dd) st[dd] = have_states ? Zin[(s * A::DPT + dd) * DV + j] : 0.f;
             for (int ii = n - 1; ii >= 0; --ii) {
                 const int i = dir ? n - 1 - ii : ii;
                 const float dj = p.c * sdo[i * DV + j];
@@ -242,8 +214,36 @@ __global__ void __launch_bounds__(NT) bwd_chunk_grads(BwdParams p) {
             }
         }
         __syncthreads();
-        float* e_out = (dir ? p.eb : p.ef) + ((size_t)bh * p.L + t0) * DK;
-        for (int idx = threadIdx.x; idx < n * DK; idx += NT) e_out[idx] = se[idx];
+        if (float* e_dir = dir ? p.eb : p.ef) {
+            float* e_out = e_dir + ((size_t)bh * p.L + t0) * DK;
+            for (int idx = threadIdx.x; idx < n * DK; idx += NT) e_out[idx] = se[idx];
+        }
+        if (void* dg = dir ? p.dgb : p.dgf) {
+            // finished gate gradient: the value just past the chunk, <state leaving the chunk, adjoint state entering from
+            // there>, plus the sum of e over the tokens scanned at or after t; then the derivative of the gate transform
+            const int next = dir ? c - 1 : c + 1;
+            if (threadIdx.x < DK) {
+                const int d = threadIdx.x;
+                float run = 0.f;
+                if (have_states && next >= 0 && next < p.nchunk) {
+                    const float* Zin = p.ws_Z + slot * DK * DV + d * DV;
+                    const float* Sn = p.ws_S + (((size_t)bh * p.nchunk + next) * 2 + dir) * DK * DV + d * DV;
+                    for (int j = 0; j < DV; ++j) run = fmaf(Sn[j], Zin[j], run);
+                }
+                for (int ii = n - 1; ii >= 0; --ii) {
+                    const int i = dir ? n - 1 - ii : ii;
+                    run += se[i * DK + d];
+                    float g = run;
+                    if (p.gate_norm > 0.f || p.clamp_min == p.clamp_min) {
+                        const float x = DType<T>::to_f(rowp<T>(dir ? p.gb : p.gf, dir ? p.sgb : p.sgf, b, h, t0 + i)[d]);
+                        g = mm::through_gate(g, x, p.gate_norm, p.clamp_min);
+                    }
+                    const size_t at = ((size_t)bh * p.L + t0 + i) * DK + d;
+                    if (p.dg_f32) reinterpret_cast<float*>(dg)[at] = g;
+                    else reinterpret_cast<T*>(dg)[at] = DType<T>::from_f(g);
+                }
+            }
+        }
     }
     __syncthreads();
     T* dq = reinterpret_cast<T*>(p.out_dq) + ((size_t)bh * p.L + t0) * DK;
@@ -251,28 +251,34 @@ __global__ void __launch_bounds__(NT) bwd_chunk_grads(BwdParams p) {
     T* dv = reinterpret_cast<T*>(p.out_dv) + ((size_t)bh * p.L + t0) * DV;
     for (int idx = threadIdx.x; idx < n * DK; idx += NT) { dq[idx] = DType<T>::from_f(sdq[idx]); dk[idx] = DType<T>::from_f(sdk[idx]); }
     for (int idx = threadIdx.x; idx < n * DV; idx += NT) dv[idx] = DType<T>::from_f(sdv[idx]);
+    __syncthreads();
+    }
 }
 
 template <int DK, int DV, typename T>
-int launch_typed(const BwdParams& p, cudaStream_t stream) {
+int launch_typed(const BwdParams& p, int flagged_only, cudaStream_t stream) {
     dim3 grid(p.nchunk, p.B * p.H);
     const size_t smA = (size_t)CH * (3 * DK + 2 * DV) * sizeof(float);
     const size_t smC = (size_t)CH * (6 * DK + 3 * DV) * sizeof(float);
     auto kA = bwd_chunk_states<DK, DV, T>;
     auto kC = bwd_chunk_grads<DK, DV, T>;
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(kA, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smA)) != cudaSuccess) return (int)e;
-    if ((e = cudaFuncSetAttribute(kC, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smC)) != cudaSuccess) return (int)e;
-    kA<<<grid, NT, smA, stream>>>(p);
-    const int per = (DK * DV + NT - 1) / NT;
-    bwd_state_scan<<<p.B * p.H * 2 * 2 * per, NT, 0, stream>>>(p);
-    kC<<<grid, NT, smC, stream>>>(p);
+    if ((e = tc::ensure_smem_attr(reinterpret_cast<const void*>(kC), (int)smC)) != cudaSuccess) return (int)e;
+    if (!flagged_only) {
+        if ((e = tc::ensure_smem_attr(reinterpret_cast<const void*>(kA), (int)smA)) != cudaSuccess) return (int)e;
+        kA<<<grid, NT, smA, stream>>>(p);
+        if (int st = bigla_bwd_scan_launch(p, stream)) return st;
+    }
+    const int items = p.nchunk * p.B * p.H;
+    // flagged chunks are rare: a CTA per SM (the tiles fill its shared memory) walks the flags; as one CTA per chunk the
+    // launch alone took 15 us for 3072 unflagged chunks
+    kC<<<flagged_only ? (items < 148 ? items : 148) : items, NT, smC, stream>>>(p, flagged_only);
     return (int)cudaGetLastError();
 }
 
 template <typename T>
-int launch_dims(const BwdParams& p, cudaStream_t stream) {
-#define VIG_CASE(DKV, DVV) if (p.dk == DKV && p.dv == DVV) return launch_typed<DKV, DVV, T>(p, stream);
+int launch_dims(const BwdParams& p, int flagged_only, cudaStream_t stream) {
+#define VIG_CASE(DKV, DVV) if (p.dk == DKV && p.dv == DVV) return launch_typed<DKV, DVV, T>(p, flagged_only, stream);
     VIG_CASE(16, 32) VIG_CASE(32, 32) VIG_CASE(32, 64) VIG_CASE(64, 64) VIG_CASE(64, 128)   // larger heads exceed shared memory
 #undef VIG_CASE
     return VIG_ERR_SHAPE;
@@ -288,10 +294,52 @@ void fill(int64_t* dst, const int64_t* src, int H, int L, int d) {
 
 using namespace vig;
 
+static size_t bwd_ws_bytes(int B, int H, int L, int dk, int dv) {
+    const size_t nchunk = (L + BWD_CHUNK - 1) / BWD_CHUNK;
+    return (size_t)B * H * nchunk * 2 * (2 * (size_t)dk * dv + dk) * sizeof(float);
+}
+
+static int bwd_fill(BwdParams& p, const void* q, const void* k, const void* v, const void* g_fwd, const void* g_bwd, const void* d_out,
+                    void* dq, void* dk_out, void* dv_out, int B, int H, int L, int dk, int dv, int dtype,
+                    const int64_t* strides_q, const int64_t* strides_k, const int64_t* strides_v,
+                    const int64_t* strides_gf, const int64_t* strides_gb, const int64_t* strides_do,
+                    float scale, float out_scale, int dir_mask, void* workspace) {
+    if (dtype < 0 || dtype > 2) return VIG_ERR_DTYPE;
+    if (B < 0 || H <= 0 || L < 0) return VIG_ERR_SHAPE;
+    if (dir_mask < 1 || dir_mask > 3) return VIG_ERR_ARG;
+    if (B == 0 || L == 0) return VIG_OK;
+    if (!q || !k || !v || !d_out || !dq || !dk_out || !dv_out) return VIG_ERR_NULL;
+    if (((dir_mask & 1) && !g_fwd) || ((dir_mask & 2) && !g_bwd)) return VIG_ERR_NULL;
+    p.q = q; p.k = k; p.v = v; p.gf = g_fwd; p.gb = g_bwd; p.dout = d_out;
+    p.out_dq = dq; p.out_dk = dk_out; p.out_dv = dv_out;
+    fill(p.sq, strides_q, H, L, dk); fill(p.sk, strides_k, H, L, dk); fill(p.sv, strides_v, H, L, dv);
+    fill(p.sgf, strides_gf, H, L, dk); fill(p.sgb, strides_gb, H, L, dk); fill(p.sdo, strides_do, H, L, dv);
+    p.B = B; p.H = H; p.L = L; p.dk = dk; p.dv = dv; p.dtype = dtype;
+    if (scale < 0.f) scale = 1.0f / sqrtf((float)dk);
+    p.c = scale * out_scale;
+    p.gate_norm = 0.f; p.clamp_min = nanf("");
+    p.dir_mask = dir_mask;
+    p.nchunk = (L + BWD_CHUNK - 1) / BWD_CHUNK;
+    const size_t states = bwd_state_floats(B, H, p.nchunk, dk, dv);
+    p.ws_S = reinterpret_cast<float*>(workspace);
+    p.ws_Z = p.ws_S + states;
+    p.ws_decay = p.ws_Z + states;
+    p.flags = reinterpret_cast<int32_t*>(p.ws_decay + (size_t)B * H * p.nchunk * 2 * dk);   // past vig_bigla_bwd's workspace, which has none
+    return VIG_OK;
+}
+
+static int bwd_simt(const BwdParams& p, int flagged_only, cudaStream_t stream) {
+    switch (p.dtype) {
+        case VIG_DTYPE_F32: return launch_dims<float>(p, flagged_only, stream);
+        case VIG_DTYPE_BF16: return launch_dims<__nv_bfloat16>(p, flagged_only, stream);
+        case VIG_DTYPE_F16: return launch_dims<__half>(p, flagged_only, stream);
+    }
+    return VIG_ERR_DTYPE;
+}
+
 extern "C" size_t vig_bigla_bwd_workspace_bytes(int B, int H, int L, int dk, int dv) {
     if (B <= 0 || H <= 0 || L <= 0 || dk <= 0 || dv <= 0) return 0;
-    const size_t nchunk = (L + CH - 1) / CH;
-    return (size_t)B * H * nchunk * 2 * (2 * (size_t)dk * dv + dk) * sizeof(float);
+    return bwd_ws_bytes(B, H, L, dk, dv);
 }
 
 extern "C" int vig_bigla_bwd(const void* q, const void* k, const void* v, const void* g_fwd, const void* g_bwd, const void* d_out,
@@ -301,33 +349,40 @@ extern "C" int vig_bigla_bwd(const void* q, const void* k, const void* v, const 
                              const int64_t* strides_gf, const int64_t* strides_gb, const int64_t* strides_do,
                              float scale, float out_scale, int dir_mask,
                              void* workspace, size_t workspace_bytes, void* stream) {
-    if (dtype < 0 || dtype > 2) return VIG_ERR_DTYPE;
-    if (B < 0 || H <= 0 || L < 0) return VIG_ERR_SHAPE;
-    if (dir_mask < 1 || dir_mask > 3) return VIG_ERR_ARG;
-    if (B == 0 || L == 0) return VIG_OK;
-    if (!q || !k || !v || !d_out || !dq || !dk_out || !dv_out) return VIG_ERR_NULL;
-    if ((dir_mask & 1) && (!g_fwd || !e_fwd)) return VIG_ERR_NULL;
-    if ((dir_mask & 2) && (!g_bwd || !e_bwd)) return VIG_ERR_NULL;
-    const size_t need = vig_bigla_bwd_workspace_bytes(B, H, L, dk, dv);
-    if (!workspace || workspace_bytes < need) return VIG_ERR_WORKSPACE;
     BwdParams p{};
-    p.q = q; p.k = k; p.v = v; p.gf = g_fwd; p.gb = g_bwd; p.dout = d_out;
-    p.out_dq = dq; p.out_dk = dk_out; p.out_dv = dv_out; p.ef = e_fwd; p.eb = e_bwd;
-    fill(p.sq, strides_q, H, L, dk); fill(p.sk, strides_k, H, L, dk); fill(p.sv, strides_v, H, L, dv);
-    fill(p.sgf, strides_gf, H, L, dk); fill(p.sgb, strides_gb, H, L, dk); fill(p.sdo, strides_do, H, L, dv);
-    p.B = B; p.H = H; p.L = L; p.dk = dk; p.dv = dv; p.dtype = dtype;
-    if (scale < 0.f) scale = 1.0f / sqrtf((float)dk);
-    p.c = scale * out_scale;
-    p.dir_mask = dir_mask;
-    p.nchunk = (L + CH - 1) / CH;
-    const size_t states = (size_t)B * H * p.nchunk * 2 * dk * dv;
-    p.ws_S = reinterpret_cast<float*>(workspace);
-    p.ws_Z = p.ws_S + states;
-    p.ws_decay = p.ws_Z + states;
-    switch (dtype) {
-        case VIG_DTYPE_F32: return launch_dims<float>(p, (cudaStream_t)stream);
-        case VIG_DTYPE_BF16: return launch_dims<__nv_bfloat16>(p, (cudaStream_t)stream);
-        case VIG_DTYPE_F16: return launch_dims<__half>(p, (cudaStream_t)stream);
-    }
-    return VIG_ERR_DTYPE;
+    const int s = bwd_fill(p, q, k, v, g_fwd, g_bwd, d_out, dq, dk_out, dv_out, B, H, L, dk, dv, dtype, strides_q, strides_k, strides_v,
+                           strides_gf, strides_gb, strides_do, scale, out_scale, dir_mask, workspace);
+    if (s || B == 0 || L == 0) return s;
+    if (((dir_mask & 1) && !e_fwd) || ((dir_mask & 2) && !e_bwd)) return VIG_ERR_NULL;
+    if (!workspace || workspace_bytes < bwd_ws_bytes(B, H, L, dk, dv)) return VIG_ERR_WORKSPACE;
+    p.ef = e_fwd; p.eb = e_bwd;
+    return bwd_simt(p, 0, (cudaStream_t)stream);
+}
+
+extern "C" size_t vig_bigla_bwd_full_workspace_bytes(int B, int H, int L, int dk, int dv) {
+    if (B <= 0 || H <= 0 || L <= 0 || dk <= 0 || dv <= 0) return 0;
+    const size_t nchunk = (L + BWD_CHUNK - 1) / BWD_CHUNK;
+    return bwd_ws_bytes(B, H, L, dk, dv) + (size_t)B * H * nchunk * sizeof(int32_t);
+}
+
+extern "C" int vig_bigla_bwd_full(const void* q, const void* k, const void* v, const void* g_fwd, const void* g_bwd, const void* d_out,
+                                  void* dq, void* dk_out, void* dv_out, void* dg_fwd, void* dg_bwd, int dg_fp32,
+                                  int B, int H, int L, int dk, int dv, int dtype,
+                                  const int64_t* strides_q, const int64_t* strides_k, const int64_t* strides_v,
+                                  const int64_t* strides_gf, const int64_t* strides_gb, const int64_t* strides_do,
+                                  float scale, float out_scale, float gate_logit_normalizer, float clamp_min, int dir_mask,
+                                  void* workspace, size_t workspace_bytes, void* stream) {
+    BwdParams p{};
+    const int s = bwd_fill(p, q, k, v, g_fwd, g_bwd, d_out, dq, dk_out, dv_out, B, H, L, dk, dv, dtype, strides_q, strides_k, strides_v,
+                           strides_gf, strides_gb, strides_do, scale, out_scale, dir_mask, workspace);
+    if (s || B == 0 || L == 0) return s;
+    if (((dir_mask & 1) && !dg_fwd) || ((dir_mask & 2) && !dg_bwd)) return VIG_ERR_NULL;
+    if (!(gate_logit_normalizer >= 0.f)) return VIG_ERR_ARG;
+    if (!workspace || workspace_bytes < vig_bigla_bwd_full_workspace_bytes(B, H, L, dk, dv)) return VIG_ERR_WORKSPACE;
+    if (reinterpret_cast<uintptr_t>(workspace) & 15) return VIG_ERR_ALIGN;
+    p.dgf = dg_fwd; p.dgb = dg_bwd; p.dg_f32 = dg_fp32 != 0;
+    p.gate_norm = gate_logit_normalizer; p.clamp_min = clamp_min;
+    if (!bigla_bwd_mma_supported(p)) return bwd_simt(p, 0, (cudaStream_t)stream);
+    const int st = bigla_bwd_mma_launch(p, (cudaStream_t)stream);
+    return st ? st : bwd_simt(p, 1, (cudaStream_t)stream);             // the chunks whose gates left the factorisation range
 }

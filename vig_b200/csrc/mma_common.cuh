@@ -1,0 +1,181 @@
+// Register-level tensor-core building blocks (mma.sync m16n8k16, ldmatrix) for the chunked bi-GLA kernels whose operands
+// change with every chunk and head size: the backward pass and the forward at full precision.
+//
+// Precision: an operand that is not exactly a bf16 number is carried as a sum of bf16 terms, x = t0 + t1 (+ t2) with
+// t_i = bf16(x - t_0 - .. - t_{i-1}): two terms hold 16 mantissa bits, three hold fp32's 24.  A product of two such
+// operands is the sum of the term products of order < max(terms); accumulation is fp32 in the tensor core.  So bf16 inputs
+// enter with one (exact) term, fp16 inputs with two (exact), fp32 inputs with three, and every scaled or intermediate
+// operand with two (16-bit callers: 2^-17 relative, far below the rounding of the results) or three (fp32 callers).
+#pragma once
+#include "tc_common.cuh"
+
+namespace vig {
+namespace mm {
+
+constexpr int C = 64;                  // tokens per chunk: 4 warps x 16 rows
+constexpr int NT = 128;                // threads per CTA
+
+template <typename T> struct Terms;    // RAW: terms of an input value, SC: terms of a scaled / intermediate value
+template <> struct Terms<__nv_bfloat16> { static constexpr int RAW = 1, SC = 2; };
+template <> struct Terms<__half> { static constexpr int RAW = 2, SC = 2; };
+template <> struct Terms<float> { static constexpr int RAW = 3, SC = 3; };
+
+// pitch of a bf16 tile row in bytes: 16 bytes of padding make the 8 rows of an ldmatrix hit 8 different 16-byte bank groups
+template <int COLS> struct Pitch { static constexpr uint32_t B = COLS * 2 + 16; };
+
+__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t* r) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ldsm4t(uint32_t addr, uint32_t* r) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ldsm2(uint32_t addr, uint32_t* r) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
+}
+__device__ __forceinline__ void ldsm2t(uint32_t addr, uint32_t* r) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
+}
+__device__ __forceinline__ void mma16816(float* c, const uint32_t* a, const uint32_t* b) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
+// Lane's address offset inside a tile for the four 8x8 matrices of an ldmatrix.x4 (PITCH in bytes):
+//   frag_rows: matrices (rows 0-7, cols 0-7), (rows 8-15, cols 0-7), (rows 0-7, cols 8-15), (rows 8-15, cols 8-15)
+//              A operand of a [m][k] tile; with .trans the B operand pair (n tiles 0, 1) of a [k][n] tile
+//   frag_cols: matrices (0-7, 0-7), (0-7, 8-15), (8-15, 0-7), (8-15, 8-15)
+//              B operand pair of an [n][k] tile; with .trans the A operand of a [k][m] tile
+template <uint32_t PITCH> __device__ __forceinline__ uint32_t frag_rows(int lane) { return (lane & 15) * PITCH + (lane >> 4) * 16; }
+template <uint32_t PITCH> __device__ __forceinline__ uint32_t frag_cols(int lane) { return ((lane & 7) + (lane >> 4) * 8) * PITCH + ((lane >> 3) & 1) * 16; }
+
+// two fp32 values -> NTERM packed bf16 pairs
+template <int NTERM> __device__ __forceinline__ void split2(float a, float b, uint32_t* t) {
+#pragma unroll
+    for (int i = 0; i < NTERM; ++i) {
+        t[i] = tc::Pack2<__nv_bfloat16>::pack(a, b);
+        if (i + 1 < NTERM) {
+            const float2 f = tc::Pack2<__nv_bfloat16>::unpack(t[i]);
+            a -= f.x; b -= f.y;
+        }
+    }
+}
+
+// c += a b over one k step, all term pairs of order < max(NA, NB); a[term][4], b[term][2]
+template <int NA, int NB> __device__ __forceinline__ void mma_terms(float* c, const uint32_t (*a)[4], const uint32_t (*b)[2]) {
+    constexpr int ORD = NA > NB ? NA : NB;
+#pragma unroll
+    for (int o = ORD - 1; o >= 0; --o)               // small terms first
+#pragma unroll
+        for (int i = 0; i < NA; ++i) {
+            const int j = o - i;
+            if (j >= 0 && j < NB) mma16816(c, a[i], b[j]);
+        }
+}
+
+template <typename T> __device__ __forceinline__ float2 load2(const T* p);
+template <> __device__ __forceinline__ float2 load2<float>(const float* p) { return __ldg(reinterpret_cast<const float2*>(p)); }
+template <> __device__ __forceinline__ float2 load2<__nv_bfloat16>(const __nv_bfloat16* p) { return tc::Pack2<__nv_bfloat16>::unpack(__ldg(reinterpret_cast<const uint32_t*>(p))); }
+template <> __device__ __forceinline__ float2 load2<__half>(const __half* p) { return tc::Pack2<__half>::unpack(__ldg(reinterpret_cast<const uint32_t*>(p))); }
+template <typename T> __device__ __forceinline__ void store2(T* p, float a, float b);
+template <> __device__ __forceinline__ void store2<float>(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
+template <> __device__ __forceinline__ void store2<__nv_bfloat16>(__nv_bfloat16* p, float a, float b) { *reinterpret_cast<uint32_t*>(p) = tc::Pack2<__nv_bfloat16>::pack(a, b); }
+template <> __device__ __forceinline__ void store2<__half>(__half* p, float a, float b) { *reinterpret_cast<uint32_t*>(p) = tc::Pack2<__half>::pack(a, b); }
+
+// log-gate in log2 units: the short hardware form for 16-bit callers, the exact form for fp32
+template <typename T> __device__ __forceinline__ float gate_log2(float x, float gate_norm, float inv_norm, float clamp_min) {
+    float g;
+    if (sizeof(T) == 4) g = (gate_norm > 0.f ? log_sigmoid(x) / gate_norm : x) * tc::LOG2E;
+    else g = tc::fast_gate2(x, gate_norm > 0.f, inv_norm);
+    return clamp_min == clamp_min ? fmaxf(g, clamp_min * tc::LOG2E) : g;
+}
+
+// derivative of the gate transform: d loss / d (gate input x) from d loss / d (log-gate)
+__device__ __forceinline__ float through_gate(float dg, float x, float gate_norm, float clamp_min) {
+    if (clamp_min == clamp_min) {                                       // the gradient passes where the unclamped gate is at or above the bound
+        const float g = gate_norm > 0.f ? log_sigmoid(x) / gate_norm : x;
+        if (!(g >= clamp_min)) return 0.f;
+    }
+    return gate_norm > 0.f ? dg * __fdividef(1.f, 1.f + __expf(x)) / gate_norm : dg;
+}
+
+// 2^x: the hardware form for 16-bit callers, the 2-ulp one for fp32
+template <typename T> __device__ __forceinline__ float ex2_t(float x) { return sizeof(T) == 4 ? exp2f(x) : tc::ex2(x); }
+
+// [C x COLS] rows of a strided tensor -> TERMS bf16 tiles (rows past n are zero); tile t at dst + t * C * pitch
+template <typename T, int COLS, int TERMS> __device__ __forceinline__ void load_raw(uint8_t* dst, const T* src, int64_t stride_l, int n) {
+    constexpr uint32_t P = Pitch<COLS>::B;
+    if constexpr (sizeof(T) == 2 && TERMS == 1) {
+        constexpr int VPR = COLS / 8;                                  // 16-byte vectors per row
+#pragma unroll
+        for (int i0 = 0; i0 < C * VPR; i0 += NT) {
+            const int i = i0 + threadIdx.x, r = i / VPR, v = i % VPR;
+            uint4 x = make_uint4(0u, 0u, 0u, 0u);
+            if (r < n) x = __ldg(reinterpret_cast<const uint4*>(src + r * stride_l) + v);
+            *reinterpret_cast<uint4*>(dst + r * P + v * 16) = x;
+        }
+    } else {
+        constexpr int PPR = COLS / 4;                                  // groups of four values per row
+#pragma unroll 4
+        for (int i0 = 0; i0 < C * PPR; i0 += NT) {
+            const int i = i0 + threadIdx.x, r = i / PPR, v = i % PPR;
+            float2 a = make_float2(0.f, 0.f), b = a;
+            if (r < n) { a = load2<T>(src + r * stride_l + 4 * v); b = load2<T>(src + r * stride_l + 4 * v + 2); }
+            uint32_t ta[TERMS], tb[TERMS];
+            split2<TERMS>(a.x, a.y, ta); split2<TERMS>(b.x, b.y, tb);
+#pragma unroll
+            for (int t = 0; t < TERMS; ++t) *reinterpret_cast<uint2*>(dst + t * C * P + r * P + v * 8) = make_uint2(ta[t], tb[t]);
+        }
+    }
+}
+
+// Thread layout of the per-channel passes over a chunk: thread = (pair of channels, group of RPG consecutive tokens).
+template <int DK> struct ColLay {
+    static constexpr int PAIRS = DK / 2, GROUPS = NT / PAIRS, RPG = C / GROUPS;
+    static_assert(PAIRS <= NT && RPG >= 1, "head size");
+};
+
+// Inclusive cumulative log-gates of the chunk in scan order (log2 units): G[r] of my rows; also the sum at the chunk's
+// middle (reference of the factorisation) and the total.  gsum: GROUPS x DK floats of shared memory; contains two barriers.
+template <int DK, typename T> __device__ __forceinline__ void cum_gates(float2 (&G)[ColLay<DK>::RPG], float2& ref, float2& tot, float* gsum, const T* g, int64_t stride_l,
+                                                                        int n, int dir, float gate_norm, float clamp_min) {
+    using CL = ColLay<DK>;
+    const int pr = threadIdx.x % CL::PAIRS, gr = threadIdx.x / CL::PAIRS, r0 = gr * CL::RPG;
+    const float inv = gate_norm > 0.f ? 1.f / gate_norm : 0.f;
+    float2 x[CL::RPG];
+#pragma unroll
+    for (int r = 0; r < CL::RPG; ++r) x[r] = r0 + r < n ? load2<T>(g + (r0 + r) * stride_l + 2 * pr) : make_float2(0.f, 0.f);
+    float2 run = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int rr = 0; rr < CL::RPG; ++rr) {
+        const int r = rr;
+        if (r0 + r < n) {
+            x[r].x = gate_log2<T>(x[r].x, gate_norm, inv, clamp_min);
+            x[r].y = gate_log2<T>(x[r].y, gate_norm, inv, clamp_min);
+        }
+        run.x += x[r].x; run.y += x[r].y;
+        G[r] = run;                                                      // inclusive prefix inside the group
+    }
+    *reinterpret_cast<float2*>(gsum + gr * DK + 2 * pr) = run;
+    __syncthreads();
+    float2 off = make_float2(0.f, 0.f), lo = off, hi = off;
+#pragma unroll
+    for (int o = 0; o < CL::GROUPS; ++o) {
+        const float2 s = *reinterpret_cast<const float2*>(gsum + o * DK + 2 * pr);
+        if (dir ? o > gr : o < gr) { off.x += s.x; off.y += s.y; }
+        if (o < CL::GROUPS / 2) { lo.x += s.x; lo.y += s.y; } else { hi.x += s.x; hi.y += s.y; }
+    }
+    __syncthreads();
+    ref = dir ? hi : lo;
+    tot = make_float2(lo.x + hi.x, lo.y + hi.y);
+#pragma unroll
+    for (int r = 0; r < CL::RPG; ++r) {
+        if (dir) {                                                       // suffix of the group = its sum - exclusive prefix
+            G[r].x = run.x - G[r].x + x[r].x + off.x; G[r].y = run.y - G[r].y + x[r].y + off.y;
+        } else {
+            G[r].x += off.x; G[r].y += off.y;
+        }
+    }
+}
+
+}  // namespace mm
+}  // namespace vig

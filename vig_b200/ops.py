@@ -197,10 +197,8 @@ def bi_gla(q, k, v, g_fwd, g_bwd, scale=-1, out_scale=1.0, *, out=None, gate_log
     return out
 
 
-def bi_gla_backward(q, k, v, g_fwd, g_bwd, d_out, scale=-1, out_scale=1.0, dir_mask=3):
-    """Gradients of ``bi_gla`` with log-space gates: ``(dq, dk, dv, dg_fwd, dg_bwd)`` (``None`` for a direction that
-    is masked out).  The kernels deliver ``e = dq*q - dk*k`` per direction; the gate gradients are its cumulative
-    sums over the tokens (``fla/ops/gla/chunk_fuse.py:506-516`` does the same in PyTorch)."""
+def _backward(q, k, v, g_fwd, g_bwd, d_out, scale, out_scale, gate_norm, clamp_min, dir_mask, dg_fp32):
+    """All gradients of ``bi_gla`` in one library call; gate gradients in fp32 or in the gates' dtype."""
     dev = _same_device(q, k, v, g_fwd, g_bwd, d_out)
     _check_scan_shapes(q, k, v, g_fwd, g_bwd, d_out)
     B, H, L, dk = k.shape
@@ -208,63 +206,49 @@ def bi_gla_backward(q, k, v, g_fwd, g_bwd, d_out, scale=-1, out_scale=1.0, dir_m
     if (dk, dv) not in BWD_HEAD_DIMS:
         raise NotImplementedError(f"the backward kernels cover (dk, dv) in {sorted(BWD_HEAD_DIMS)}; got ({dk}, {dv})")
     dq, dk_, dv_ = (torch.empty(B, H, L, d, dtype=k.dtype, device=dev) for d in (dk, dk, dv))
-    e_f = torch.empty(B, H, L, dk, dtype=torch.float32, device=dev) if dir_mask & 1 else None
-    e_b = torch.empty(B, H, L, dk, dtype=torch.float32, device=dev) if dir_mask & 2 else None
+    dg_f, dg_b = (torch.empty(B, H, L, dk, dtype=torch.float32 if dg_fp32 else k.dtype, device=dev) if dir_mask & m else None for m in (1, 2))
     L_ = _lib.lib()
     s3 = lambda t: None if t is None else _lib.strides3(t)
     with torch.cuda.device(dev):
-        nbytes = L_.vig_bigla_bwd_workspace_bytes(B, H, L, dk, dv)
-        ws = _workspace(nbytes, dev)
-        st = L_.vig_bigla_bwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(g_fwd), _lib.ptr(g_bwd), _lib.ptr(d_out),
-                              _lib.ptr(dq), _lib.ptr(dk_), _lib.ptr(dv_), _lib.ptr(e_f), _lib.ptr(e_b),
-                              B, H, L, dk, dv, _lib.dtype_code(k), s3(q), s3(k), s3(v), s3(g_fwd), s3(g_bwd), s3(d_out),
-                              float(scale if scale is not None else -1), float(out_scale), dir_mask,
-                              _lib.ptr(ws), ws.numel() if ws is not None else 0, _lib.stream_ptr())
-    _lib.check(st, "vig_bigla_bwd")
-    dg_f = e_f.flip(2).cumsum(2).flip(2) if e_f is not None else None
-    dg_b = e_b.cumsum(2) if e_b is not None else None
+        ws = _workspace(L_.vig_bigla_bwd_full_workspace_bytes(B, H, L, dk, dv), dev)
+        st = L_.vig_bigla_bwd_full(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(g_fwd), _lib.ptr(g_bwd), _lib.ptr(d_out),
+                                   _lib.ptr(dq), _lib.ptr(dk_), _lib.ptr(dv_), _lib.ptr(dg_f), _lib.ptr(dg_b), int(dg_fp32),
+                                   B, H, L, dk, dv, _lib.dtype_code(k), s3(q), s3(k), s3(v), s3(g_fwd), s3(g_bwd), s3(d_out),
+                                   float(scale if scale is not None else -1), float(out_scale), float(gate_norm),
+                                   _NAN if clamp_min is None else float(clamp_min), dir_mask,
+                                   _lib.ptr(ws), ws.numel() if ws is not None else 0, _lib.stream_ptr())
+    _lib.check(st, "vig_bigla_bwd_full")
     return dq, dk_, dv_, dg_f, dg_b
 
 
+def bi_gla_backward(q, k, v, g_fwd, g_bwd, d_out, scale=-1, out_scale=1.0, dir_mask=3):
+    """Gradients of ``bi_gla`` with log-space gates: ``(dq, dk, dv, dg_fwd, dg_bwd)``, the gate gradients in fp32 (``None``
+    for a direction that is masked out)."""
+    return _backward(q, k, v, g_fwd if dir_mask & 1 else None, g_bwd if dir_mask & 2 else None, d_out, scale, out_scale, 0.0, None, dir_mask, True)
+
+
 class _BiGLAFunction(torch.autograd.Function):
-    """Differentiable ``bi_gla``: forward through ``vig_bigla_fwd``, backward through ``vig_bigla_bwd``.  Raw gate
-    logits are turned into log-gates here so that one backward kernel serves both forms."""
+    """Differentiable ``bi_gla``: forward through ``vig_bigla_fwd``, backward through ``vig_bigla_bwd_full``; both apply the
+    gate transform (and its derivative) inside their kernels."""
 
     @staticmethod
     def forward(ctx, q, k, v, g_fwd, g_bwd, scale, out_scale, gate_norm, clamp_min, dir_mask, impl):
-        def to_log(x):
-            if x is None:
-                return None, None
-            g = torch.nn.functional.logsigmoid(x.float()) / gate_norm if gate_norm > 0 else x.float()
-            # gradient passes where the unclamped fp32 gate is at or above the bound (torch.clamp_min's rule)
-            keep = None
-            if clamp_min is not None:
-                keep = g >= clamp_min
-                g = torch.clamp_min(g, clamp_min)
-            return g.to(x.dtype), keep
-        gf, keep_f = to_log(g_fwd)
-        gb, keep_b = to_log(g_bwd)
         with torch.no_grad():
-            o = bi_gla(q, k, v, gf, gb, scale=scale, out_scale=out_scale, dir_mask=dir_mask, impl=impl)
-        ctx.save_for_backward(q, k, v, g_fwd, g_bwd, gf, gb, keep_f, keep_b)
+            o = bi_gla(q, k, v, g_fwd, g_bwd, scale=scale, out_scale=out_scale, gate_logit_normalizer=gate_norm, clamp_min=clamp_min,
+                       dir_mask=dir_mask, impl=impl)
+        ctx.save_for_backward(q, k, v, g_fwd, g_bwd)
         ctx.cfg = (scale, out_scale, gate_norm, clamp_min, dir_mask)
         return o
 
     @staticmethod
     def backward(ctx, d_out):
-        q, k, v, x_f, x_b, gf, gb, keep_f, keep_b = ctx.saved_tensors
+        q, k, v, g_f, g_b = ctx.saved_tensors
         scale, out_scale, gate_norm, clamp_min, dir_mask = ctx.cfg
-        dq, dk, dv, dg_f, dg_b = bi_gla_backward(q, k, v, gf, gb, d_out.contiguous(), scale, out_scale, dir_mask)
-
-        def through_gate(dg, x, keep):
-            if dg is None or x is None:
-                return None
-            if keep is not None:
-                dg = dg * keep
-            if gate_norm > 0:                                       # d logsigmoid(x) / dx = sigmoid(-x)
-                dg = dg * torch.sigmoid(-x.float()) / gate_norm
-            return dg.to(x.dtype)
-        return dq, dk, dv, through_gate(dg_f, x_f, keep_f), through_gate(dg_b, x_b, keep_b), None, None, None, None, None, None
+        if d_out.stride(-1) != 1:
+            d_out = d_out.contiguous()
+        grads = _backward(q, k, v, g_f if dir_mask & 1 else None, g_b if dir_mask & 2 else None, d_out, scale, out_scale, gate_norm,
+                          clamp_min, dir_mask, False)
+        return (*grads, None, None, None, None, None, None)
 
 
 def bi_gla_noalloc(q, k, v, g_fwd, g_bwd, out, scale=-1, out_scale=1.0, gate_logit_normalizer=0.0, clamp_min=None,
