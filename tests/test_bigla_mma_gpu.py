@@ -1,0 +1,47 @@
+"""Full-precision tensor-core forward (fp32, and 16-bit heads with dv = 32) at chunk edges (64 tokens), with entering and
+final states, one direction, gates that leave the factorisation's range, and rows only the token-by-token form can read."""
+import pytest
+import torch
+
+import oracle
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+# fp32: operands carry 24 bits; 64-token cumulative gates of up to 24 round to 2^-24 * 24 = 1.4e-6 per factor.  16-bit: the
+# output's rounding (2^-9, 2^-12) in the max norm plus 2^-17 operand splits.
+TOL = {torch.float32: 2e-5, torch.bfloat16: 5e-3, torch.float16: 1e-3}
+DIMS = {torch.float32: [(16, 32), (32, 32), (32, 64), (64, 64)], torch.bfloat16: [(16, 32), (32, 32)], torch.float16: [(16, 32), (32, 32)]}
+
+
+@pytest.mark.parametrize("dtype,dk,dv", [(t, *d) for t in DIMS for d in DIMS[t]])
+@pytest.mark.parametrize("L,strength", [(1, 1.0), (63, 1.0), (64, 1.0), (65, 1.0), (200, 1.0), (150, 60.0)])
+def test_forward_at_chunk_edges(dtype, dk, dv, L, strength):
+    import vig_b200
+    q, k, v, gf, gb = oracle.make_bigla_inputs(2, 2, L, dk, dv, seed=L + dk)
+    ins = [t.to(dtype) for t in (q, k, v, gf * strength, gb)]
+    ref = oracle.naive_bi_gla(*[t.float() for t in ins])
+    assert rel_err(vig_b200.bi_gla(*[t.cuda() for t in ins]).float(), ref) < TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype,dk,dv", [(torch.float32, 64, 64), (torch.float16, 16, 32)])
+@pytest.mark.parametrize("L", [64, 130])
+def test_one_direction_continues_from_a_state(dtype, dk, dv, L):
+    import vig_b200
+    q, k, v, g, _ = [t.to(dtype) for t in oracle.make_bigla_inputs(1, 2, L, dk, dv, seed=3)]
+    cut = L // 2
+    full, h_full = vig_b200.fused_chunk_gla(*[t.cuda() for t in (q, k, v, g)], output_final_state=True)
+    first = [t[:, :, :cut].cuda() for t in (q, k, v, g)]
+    rest = [t[:, :, cut:].cuda() for t in (q, k, v, g)]
+    _, h = vig_b200.fused_chunk_gla(*first, output_final_state=True)
+    o, h_end = vig_b200.fused_chunk_gla(*rest, initial_state=h, output_final_state=True)
+    ref, ref_h = oracle.naive_gla(*[t.float() for t in (q, k, v, g)])
+    assert rel_err(full.float(), ref) < TOL[dtype] and rel_err(h_full, ref_h) < 1e-4
+    assert rel_err(o.float(), ref[:, :, cut:]) < TOL[dtype] and rel_err(h_end, ref_h) < 1e-4
+
+
+def test_unaligned_rows_take_the_exact_form():
+    import vig_b200
+    ins = oracle.make_bigla_inputs(1, 2, 70, 32, 32, seed=4)
+    odd = torch.zeros(1, 2, 70, 33, device="cuda")
+    odd[..., 1:] = ins[0].cuda()
+    assert rel_err(vig_b200.bi_gla(odd[..., 1:], *[t.cuda() for t in ins[1:]]), oracle.naive_bi_gla(*ins)) < 2e-5

@@ -139,5 +139,6 @@ int vig::bigla_fwd_internal(const void* q, const void* k, const void* v, const v
     const size_t nchunk = (L + 63) / 64;
     p.ws_state = reinterpret_cast<float*>(workspace);
     p.ws_decay = p.ws_state ? p.ws_state + (size_t)B * H * nchunk * 2 * dk * dv : nullptr;
+    if (impl == VIG_IMPL_AUTO && bigla_mma_supported(p)) return bigla_mma_launch(p, (cudaStream_t)stream);   // same workspace layout
     return bigla_simt_launch(p, (cudaStream_t)stream);
 }

@@ -177,5 +177,148 @@ template <int DK, typename T> __device__ __forceinline__ void cum_gates(float2 (
     }
 }
 
+// Largest |G - r| (log2 units) of the factorised form.  The exponent's own rounding grows with it (2^-24 |G|): 24 keeps it
+// below 2e-6 for fp32 callers, 96 below 1e-5 for 16-bit ones and every scaled operand inside bf16's exponent range.
+template <typename T> __device__ __forceinline__ float range_limit() { return sizeof(T) == 4 ? 24.f : 96.f; }
+
+template <typename T> __device__ __forceinline__ const T* head_ptr(const void* base, const int64_t* s, int b, int h, int64_t t0) {
+    return reinterpret_cast<const T*>(base) + b * s[0] + h * s[1] + t0 * s[2];
+}
+
+// acc[NTILES][4] += X^T Y: X [C tokens][DK] scaled tiles (my 16 rows of X^T at column byte offset), Y [C][DV] raw tiles
+template <int DK, int DV, int NA, int NB, int NTILES> __device__ __forceinline__ void state_mma(float (*acc)[4], uint32_t x, uint32_t y, int lane) {
+    constexpr uint32_t PX = Pitch<DK>::B, PY = Pitch<DV>::B;
+    x += frag_cols<PX>(lane);
+    y += frag_rows<PY>(lane);
+#pragma unroll
+    for (int ks = 0; ks < C / 16; ++ks) {
+        uint32_t a[NA][4];
+#pragma unroll
+        for (int t = 0; t < NA; ++t) ldsm4t(x + t * C * PX + ks * 16 * PX, a[t]);
+        if constexpr (NTILES == 1) {
+            uint32_t b[NB][2];
+#pragma unroll
+            for (int t = 0; t < NB; ++t) ldsm2t(y + t * C * PY + ks * 16 * PY, b[t]);
+            mma_terms<NA, NB>(acc[0], a, b);
+        } else {
+#pragma unroll
+            for (int n = 0; n < NTILES; n += 2) {
+                uint32_t b0[NB][2], b1[NB][2];
+#pragma unroll
+                for (int t = 0; t < NB; ++t) {
+                    uint32_t r[4];
+                    ldsm4t(y + t * C * PY + ks * 16 * PY + n * 16, r);
+                    b0[t][0] = r[0]; b0[t][1] = r[1]; b1[t][0] = r[2]; b1[t][1] = r[3];
+                }
+                mma_terms<NA, NB>(acc[n], a, b0);
+                mma_terms<NA, NB>(acc[n + 1], a, b1);
+            }
+        }
+    }
+}
+
+// fp32 state [DK][DV] times a per-row scale -> bf16 terms; with ``carry`` also carry[d] = <state[d], other[d]>
+template <int DK, int DV, int SC> __device__ __forceinline__ void load_state(uint8_t* dst, const float* st, const float* scale, const float* other, float* carry) {
+    constexpr uint32_t P = Pitch<DV>::B;
+    constexpr int TPR = DV / 4;                                          // threads per row (8 .. 16)
+#pragma unroll 4
+    for (int i0 = 0; i0 < DK * TPR; i0 += NT) {
+        const int i = i0 + threadIdx.x, d = i / TPR, v = i % TPR;
+        const float4 x = st ? __ldcg(reinterpret_cast<const float4*>(st) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float s = scale[d];
+        uint32_t ta[SC], tb[SC];
+        split2<SC>(x.x * s, x.y * s, ta); split2<SC>(x.z * s, x.w * s, tb);
+#pragma unroll
+        for (int t = 0; t < SC; ++t) *reinterpret_cast<uint2*>(dst + t * DK * P + d * P + v * 8) = make_uint2(ta[t], tb[t]);
+        if (carry) {
+            const float4 y = other ? __ldcg(reinterpret_cast<const float4*>(other) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            float a = x.x * y.x + x.y * y.y + x.z * y.z + x.w * y.w;
+#pragma unroll
+            for (int m = 1; m < TPR; m <<= 1) a += __shfl_xor_sync(0xffffffffu, a, m);
+            if (v == 0) carry[d] = a;
+        }
+    }
+}
+
+// acc[2][4] += A_rows B_rows^T over KD: A fragments of my 16 rows (tile a, [row][k]), B rows jb*16.. (tile b, [n][k])
+template <int KD, int NA, int NB> __device__ __forceinline__ void block_nt(float (*acc)[4], uint32_t a, uint32_t a_term, uint32_t b, uint32_t b_term) {
+#pragma unroll
+    for (int ks = 0; ks < KD / 16; ++ks) {
+        uint32_t fa[NA][4], b0[NB][2], b1[NB][2];
+#pragma unroll
+        for (int t = 0; t < NA; ++t) ldsm4(a + t * a_term + ks * 32, fa[t]);
+#pragma unroll
+        for (int t = 0; t < NB; ++t) {
+            uint32_t r[4];
+            ldsm4(b + t * b_term + ks * 32, r);
+            b0[t][0] = r[0]; b0[t][1] = r[1]; b1[t][0] = r[2]; b1[t][1] = r[3];
+        }
+        mma_terms<NA, NB>(acc[0], fa, b0);
+        mma_terms<NA, NB>(acc[1], fa, b1);
+    }
+}
+
+// zero the entries of a diagonal 16 x 16 block that ``keep(row, col)`` rejects, then split it into an A operand
+template <int SC, typename F> __device__ __forceinline__ void mask_split(float (*p)[4], bool diag, int lane, F keep, uint32_t (*out)[4]) {
+    if (diag) {
+        const int r = lane >> 2, q = 2 * (lane & 3);
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) if (!keep(r + 8 * (j >> 1), nt * 8 + q + (j & 1))) p[nt][j] = 0.f;
+    }
+    uint32_t t[SC];
+    split2<SC>(p[0][0], p[0][1], t);
+#pragma unroll
+    for (int i = 0; i < SC; ++i) out[i][0] = t[i];
+    split2<SC>(p[0][2], p[0][3], t);
+#pragma unroll
+    for (int i = 0; i < SC; ++i) out[i][1] = t[i];
+    split2<SC>(p[1][0], p[1][1], t);
+#pragma unroll
+    for (int i = 0; i < SC; ++i) out[i][2] = t[i];
+    split2<SC>(p[1][2], p[1][3], t);
+#pragma unroll
+    for (int i = 0; i < SC; ++i) out[i][3] = t[i];
+}
+
+// acc[ND/8][4] += A (16 x 16, registers) B: B rows of one k step in a [k][n] tile
+template <int ND, int NA, int NB> __device__ __forceinline__ void block_nn(float (*acc)[4], const uint32_t (*a)[4], uint32_t b, uint32_t b_term) {
+#pragma unroll
+    for (int n = 0; n < ND / 8; n += 2) {
+        uint32_t b0[NB][2], b1[NB][2];
+#pragma unroll
+        for (int t = 0; t < NB; ++t) {
+            uint32_t r[4];
+            ldsm4t(b + t * b_term + n * 16, r);
+            b0[t][0] = r[0]; b0[t][1] = r[1]; b1[t][0] = r[2]; b1[t][1] = r[3];
+        }
+        mma_terms<NA, NB>(acc[n], a, b0);
+        mma_terms<NA, NB>(acc[n + 1], a, b1);
+    }
+}
+
+// acc[ND/8][4] += A B^T over KD: A = my 16 rows of an [m][k] tile, B an [n][k] tile of ND rows with pitch PB
+template <int ND, int KD, uint32_t PB, int NA, int NB> __device__ __forceinline__ void rows_nt(float (*acc)[4], uint32_t a, uint32_t a_term, uint32_t b, uint32_t b_term) {
+#pragma unroll
+    for (int ks = 0; ks < KD / 16; ++ks) {
+        uint32_t fa[NA][4];
+#pragma unroll
+        for (int t = 0; t < NA; ++t) ldsm4(a + t * a_term + ks * 32, fa[t]);
+#pragma unroll
+        for (int n = 0; n < ND / 8; n += 2) {
+            uint32_t b0[NB][2], b1[NB][2];
+#pragma unroll
+            for (int t = 0; t < NB; ++t) {
+                uint32_t r[4];
+                ldsm4(b + t * b_term + n * 8 * PB + ks * 32, r);
+                b0[t][0] = r[0]; b0[t][1] = r[1]; b1[t][0] = r[2]; b1[t][1] = r[3];
+            }
+            mma_terms<NA, NB>(acc[n], fa, b0);
+            mma_terms<NA, NB>(acc[n + 1], fa, b1);
+        }
+    }
+}
+
 }  // namespace mm
 }  // namespace vig
