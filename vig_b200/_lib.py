@@ -69,6 +69,23 @@ def lib():
     return _lib
 
 
+_host_module = None
+
+
+def host():
+    """The package's C++ host module (``vig_b200/csrc/host_ops.cpp``), bound to the same copy of the kernel library."""
+    global _host_module
+    if _host_module is None:
+        lib()
+        try:
+            from . import _host
+        except ImportError as exc:
+            raise RuntimeError("vig_b200._host is missing: build it with `python -m vig_b200.build`") from exc
+        _host.init(LIB_PATH)
+        _host_module = _host
+    return _host_module
+
+
 def register(name, restype, argtypes):
     """Declare the signature of an additional entry point."""
     _SIGNATURES[name] = (restype, argtypes)

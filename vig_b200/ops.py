@@ -4,7 +4,7 @@
 ``fused_chunk_gla`` mirrors ``fla/ops/gla/chunk_fuse.py:554-572`` and ``chunk_gla``
 ``fla/ops/gla/chunk.py:561-580``; ``bi_gla`` is the explicit form of the merged operator.
 Tensors are ``[B, H, L, d]`` views with a contiguous last dimension; no copies are made.
-``bi_gla`` and the one-direction entry points are differentiable (``vig_bigla_bwd``); the block's other kernels
+``bi_gla`` and the one-direction entry points are differentiable (``vig_bigla_bwd_full``); the block's other kernels
 are inference-only.
 """
 import math
@@ -16,7 +16,6 @@ from . import _lib
 _NAN = float("nan")
 # (dk, dv) pairs the backward kernels are compiled for (vig_bigla_bwd)
 BWD_HEAD_DIMS = {(16, 32), (32, 32), (32, 64), (64, 64), (64, 128)}
-_ws_cache = {}
 _status_words = {}
 
 
@@ -75,6 +74,7 @@ def status_word(device=None):
     sw = _status_words.get(device)
     if sw is None:
         sw = _status_words[device] = StatusWord(device)
+        _lib.host().set_status(device.index, sw.tensor)
     return sw
 
 
@@ -117,16 +117,8 @@ def _check_scan_shapes(q, k, v, g_fwd, g_bwd, out=None):
 
 
 def _workspace(nbytes, device):
-    """Per-device scratch buffer that only grows (allocated through torch's caching allocator)."""
-    if nbytes == 0:
-        return None
-    if torch.cuda.is_current_stream_capturing():
-        return torch.empty(nbytes, dtype=torch.uint8, device=device)
-    buf = _ws_cache.get(device)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.empty(int(nbytes * 1.25) + 256, dtype=torch.uint8, device=device)
-        _ws_cache[device] = buf
-    return buf
+    """Scratch of one call, from torch's caching allocator: ordered with the stream's other work, given back right after."""
+    return torch.empty(nbytes, dtype=torch.uint8, device=device) if nbytes else None
 
 
 def bi_gla(q, k, v, g_fwd, g_bwd, scale=-1, out_scale=1.0, *, out=None, gate_logit_normalizer=0.0, clamp_min=None,
@@ -140,6 +132,12 @@ def bi_gla(q, k, v, g_fwd, g_bwd, scale=-1, out_scale=1.0, *, out=None, gate_log
     Returns ``o`` or ``(o, extras)`` where ``extras`` holds ``final_fwd/final_bwd`` ([B,H,dk,dv] fp32) and
     ``logdecay_fwd/logdecay_bwd`` ([B,H,dk] fp32) when requested.
     """
+    plain = out is None and init_state_fwd is None and init_state_bwd is None and not output_final_state and not output_logdecay and want_output
+    if plain and status is None:
+        o = _lib.host().bi_gla(q, k, v, g_fwd, g_bwd, -1 if scale is None else scale, out_scale, gate_logit_normalizer,
+                               _NAN if clamp_min is None else clamp_min, dir_mask, impl)
+        if o is not None:
+            return o
     dev = _same_device(q, k, v, g_fwd, g_bwd, out, init_state_fwd, init_state_bwd, status)
     _check_scan_shapes(q if want_output else None, k, v, g_fwd, g_bwd, out)
     if want_output and q is None:
@@ -147,13 +145,16 @@ def bi_gla(q, k, v, g_fwd, g_bwd, scale=-1, out_scale=1.0, *, out=None, gate_log
     B, H, L, dk = k.shape
     dv = v.shape[-1]
     if torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (q, k, v, g_fwd, g_bwd)):
-        if (init_state_fwd is not None or init_state_bwd is not None or output_final_state or output_logdecay
-                or out is not None or not want_output):
+        if not plain:
             raise NotImplementedError("the differentiable form takes no states and allocates its own output")
         if (dk, dv) not in BWD_HEAD_DIMS:
             raise NotImplementedError(f"the backward kernels cover (dk, dv) in {sorted(BWD_HEAD_DIMS)}; got ({dk}, {dv})")
-        return _BiGLAFunction.apply(q, k, v, g_fwd, g_bwd, float(scale if scale is not None else -1), float(out_scale),
-                                    float(gate_logit_normalizer), clamp_min, dir_mask, impl)
+        status_word(dev)
+        o = _lib.host().bi_gla(q, k, v, g_fwd if dir_mask & 1 else None, g_bwd if dir_mask & 2 else None, -1 if scale is None else scale,
+                               out_scale, gate_logit_normalizer, _NAN if clamp_min is None else clamp_min, dir_mask, impl)
+        if o is None:
+            raise ValueError("q, k, v and the gates of the active directions need one supported dtype and a contiguous last dimension")
+        return o
     code = _lib.dtype_code(k)
     if want_output:
         if out is None:
@@ -227,30 +228,6 @@ def bi_gla_backward(q, k, v, g_fwd, g_bwd, d_out, scale=-1, out_scale=1.0, dir_m
     return _backward(q, k, v, g_fwd if dir_mask & 1 else None, g_bwd if dir_mask & 2 else None, d_out, scale, out_scale, 0.0, None, dir_mask, True)
 
 
-class _BiGLAFunction(torch.autograd.Function):
-    """Differentiable ``bi_gla``: forward through ``vig_bigla_fwd``, backward through ``vig_bigla_bwd_full``; both apply the
-    gate transform (and its derivative) inside their kernels."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, g_fwd, g_bwd, scale, out_scale, gate_norm, clamp_min, dir_mask, impl):
-        with torch.no_grad():
-            o = bi_gla(q, k, v, g_fwd, g_bwd, scale=scale, out_scale=out_scale, gate_logit_normalizer=gate_norm, clamp_min=clamp_min,
-                       dir_mask=dir_mask, impl=impl)
-        ctx.save_for_backward(q, k, v, g_fwd, g_bwd)
-        ctx.cfg = (scale, out_scale, gate_norm, clamp_min, dir_mask)
-        return o
-
-    @staticmethod
-    def backward(ctx, d_out):
-        q, k, v, g_f, g_b = ctx.saved_tensors
-        scale, out_scale, gate_norm, clamp_min, dir_mask = ctx.cfg
-        if d_out.stride(-1) != 1:
-            d_out = d_out.contiguous()
-        grads = _backward(q, k, v, g_f if dir_mask & 1 else None, g_b if dir_mask & 2 else None, d_out, scale, out_scale, gate_norm,
-                          clamp_min, dir_mask, False)
-        return (*grads, None, None, None, None, None, None)
-
-
 def bi_gla_noalloc(q, k, v, g_fwd, g_bwd, out, scale=-1, out_scale=1.0, gate_logit_normalizer=0.0, clamp_min=None,
                    impl=_lib.IMPL_AUTO, status=None):
     """``bi_gla`` through the entry point that allocates nothing: the caller supplies ``out`` and the scan's
@@ -282,10 +259,14 @@ def bid_fused_recurrent_gla(q, k, v, gk=None, gv=None, scale=-1, initial_state=N
     B = q.shape[0]
     if gk.shape[0] != 2 * B:
         raise ValueError("gk must stack forward and backward gates along the batch: [2B,H,L,dk]")
-    return bi_gla(q, k, v, gk[:B], gk[B:], scale=scale, out_scale=0.5), None
+    o = _lib.host().bi_gla_stacked(q, k, v, gk, -1 if scale is None else scale, 0.5)
+    return (bi_gla(q, k, v, gk[:B], gk[B:], scale=scale, out_scale=0.5) if o is None else o), None
 
 
 def _one_direction(q, k, v, g, scale, initial_state, output_final_state, reverse):
+    res = _lib.host().scan(q, k, v, g, -1 if scale is None else scale, initial_state, bool(output_final_state), reverse)
+    if res is not None:
+        return res
     mask = 2 if reverse else 1
     kw = dict(init_state_bwd=initial_state) if reverse else dict(init_state_fwd=initial_state)
     if initial_state is not None:
