@@ -251,6 +251,13 @@ VIG_API int vig_layernorm_act_add_rmsnorm_fwd(const void* x, const void* pre_bia
                                               int64_t post_period, void* y, const void* rms_w, float rms_eps, void* h, int64_t rows, int N,
                                               float eps, int act_swish, int dtype, void* stream);
 
+/* r = x + residual (residual optional; the sum is rounded to the tensor dtype and written to sum_out when given), then
+ * y = LayerNorm(r) * w + bias, then act: 0 none, 1 swish, 2 GELU (erf form) -- the pre-norms of the hierarchical model's
+ * blocks with the residual add in front of them (classification/models/vig_h.py:672-683) and its patch embedding's
+ * LayerNorm + GELU.  Contiguous [rows, N], N * element size a multiple of 16. */
+VIG_API int vig_add_layernorm_fwd(const void* x, const void* residual, const void* w, const void* bias, void* y, void* sum_out, int64_t rows,
+                                  int N, float eps, int act, int dtype, void* stream);
+
 /*
  * Space-to-depth of the input image for the stem's first convolution (`V2PatchEmbed`, classification/models/vig.py:
  * 650-651: kernel s+1, stride s, padding 1), which is then a 2x2 convolution over s x s pixel blocks:

@@ -1,0 +1,56 @@
+"""The C++ forward of the models against the Python modules it stands for (same kernels, so the same bits), and its plan's
+staleness: changed parameters and attributes are seen, hooks and overridden forwards send the call to the modules."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _model(kind, dtype):
+    import vig_b200
+    torch.manual_seed(1)
+    if kind == "hier":
+        m = vig_b200.HierViG(depths=[1, 1, 1, 1], dims=64, num_heads=[2, 4, 8, 16], norm_layer="ln2d", patchembed_version="v2", downsample_version="v3",
+                             gmlp=True, num_classes=12)
+    elif kind == "hier_mlp":
+        m = vig_b200.HierViG(depths=[1, 1, 1, 1], dims=64, num_heads=[2, 4, 8, 16], num_classes=12, expand_k=1.0)
+    else:
+        m = vig_b200.ViG(depth=2, num_classes=12, **vig_b200.vig._PRESETS[kind])
+    return m.to("cuda", dtype).eval().requires_grad_(False)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("kind,size", [("vig_t", (224, 224)), ("vig_t", (80, 112)), ("vig_s", (64, 96)), ("hier", (64, 96)), ("hier_mlp", (96, 64))])
+def test_native_forward_equals_the_modules(kind, size, dtype):
+    from vig_b200 import native
+    m = _model(kind, dtype)
+    x = torch.randn(2, 3, *size, device="cuda").to(dtype)
+    with torch.no_grad():
+        run = native.hier_forward if kind.startswith("hier") else native.vig_forward
+        got = run(m, x)
+        assert got is not None
+        handle = m.register_forward_hook(lambda *a: None)               # a hook anywhere: the modules run
+        assert run(m, x) is None
+        ref = m(x)
+        handle.remove()
+    rel = float((got.float() - ref.float()).norm() / ref.float().norm())
+    assert rel < (1e-2 if kind.startswith("hier") else 1e-6), rel       # hier: the branch's add is fused into the next norm
+
+
+def test_plan_follows_the_model():
+    from vig_b200 import native
+    m = _model("vig_t", torch.bfloat16)
+    x = torch.randn(1, 3, 64, 64, device="cuda").bfloat16()
+    with torch.no_grad():
+        a = m(x)
+        assert native._plans.get(m)
+        m.blocks[1].mlp.down_proj.weight.mul_(2.0)                      # in place
+        b = m(x)
+        m.blocks[0].attn.out_scale = 0.5                                # attribute
+        c = m(x)
+        m.blocks[0].attn_norm.weight = torch.nn.Parameter(m.blocks[0].attn_norm.weight * 1.5, requires_grad=False)   # replaced
+        d = m(x)
+        m.blocks[0].forward = lambda *a, **k: None
+        assert native.vig_forward(m, x) is None
+    outs = [a, b, c, d]
+    assert all(not torch.equal(outs[i], outs[i + 1]) for i in range(3))

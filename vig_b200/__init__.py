@@ -5,3 +5,4 @@ from .ops import (bi_gla, bi_gla_backward, bid_fused_recurrent_gla, fused_chunk_
 from .modules import RMSNorm, GatedLinearAttention, GLAMLP, GLABlock  # noqa: F401
 from .vig import ViG, build_vig  # noqa: F401
 from .hier import HierViG, GLA2D, VSSBlock  # noqa: F401
+from . import native  # noqa: F401  (imported here so that it knows the operators as they are before anyone wraps them)

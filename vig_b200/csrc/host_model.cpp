@@ -1,0 +1,402 @@
+// Inference forward of the ViG and HierViG models in C++: the same sequence of library calls, GEMMs and kernels as the Python
+// modules, without their per-step cost.  A ViG forward is about 100 launches; in Python they took 3.2 ms, five times the
+// kernels' time for one 224 x 224 image.
+//
+// A Plan is built by the Python layer (vig_b200/native.py) from a model's modules and stays valid while nothing it was built
+// from changes: it watches every parameter (identity, version, storage, type), every module's children, hooks, plain
+// attributes and overridden forwards, and answers None as soon as one differs, so that the caller rebuilds it or runs the
+// modules themselves.  The check is some hundred pointer comparisons.
+#include "host.h"
+#include <cuda_runtime_api.h>
+#include <ATen/autocast_mode.h>
+#include <ATen/ops/empty.h>
+
+namespace vig_host {
+namespace {
+
+using OptT = std::optional<Tensor>;
+
+// ---- library calls on tensors --------------------------------------------------------------------------------------
+struct Ctx { void* stream; int32_t* status; int code; };
+
+Tensor dwconv(const Ctx& c, const Tensor& x, const Tensor& taps, const Tensor& bias, int64_t h, int64_t w, bool act) {
+    Tensor y = at::empty_like(x);
+    ok(api.vig_dwconv3x3_fwd(ptr(x), ptr(taps), ptr(bias), ptr(y), x.size(0), h, w, x.size(2), act, c.code, c.status, c.stream), "vig_dwconv3x3_fwd");
+    return y;
+}
+std::pair<Tensor, Tensor> add_rmsnorm(const Ctx& c, const Tensor& x, const Tensor& w, const Tensor& res, double eps, bool prenorm) {
+    const int64_t N = x.size(-1);
+    Tensor y = at::empty_like(x), r = prenorm && res.defined() ? at::empty_like(x) : Tensor();
+    ok(api.vig_add_rmsnorm_fwd(ptr(x), ptr(res), ptr(w), ptr(y), ptr(r), x.numel() / N, N, (float)eps, c.code, c.stream), "vig_add_rmsnorm_fwd");
+    return {y, r};
+}
+Tensor layernorm(const Ctx& c, const Tensor& x, const Tensor& w, const Tensor& b, double eps, bool swish, const Tensor& pre_bias) {
+    const int64_t N = x.size(-1);
+    Tensor y = at::empty_like(x);
+    ok(api.vig_layernorm_act_fwd(ptr(x), ptr(pre_bias), ptr(w), ptr(b), ptr(y), x.numel() / N, N, (float)eps, swish, c.code, c.stream), "vig_layernorm_act_fwd");
+    return y;
+}
+// swiglu(x W^T): one kernel where it is the faster one, GEMM + activation kernel otherwise
+Tensor mlp_in(const Ctx& c, const Tensor& x, const Tensor& w) {
+    const int64_t K = x.size(-1), I = w.size(0) / 2, M = x.numel() / K;
+    Tensor out = at::empty({x.size(0), x.size(1), I}, x.options());
+    if (api.vig_linear_swiglu_preferred(M, K, I, c.code)) {
+        ok(api.vig_linear_swiglu_fwd(ptr(x), K, ptr(w), ptr(out), I, M, K, I, c.code, c.status, c.stream), "vig_linear_swiglu_fwd");
+        return out;
+    }
+    const Tensor z = at::linear(x, w);
+    ok(api.vig_swiglu_fwd(ptr(z), (uint8_t*)ptr(z) + I * z.element_size(), ptr(out), M, I, 2 * I, I, c.code, c.stream), "vig_swiglu_fwd");
+    return out;
+}
+std::pair<Tensor, Tensor> linear_add_rmsnorm(const Ctx& c, const Tensor& x, const Tensor& w, const Tensor& res, const Tensor& nw, double eps) {
+    const int64_t K = x.size(-1), N = w.size(0), M = x.numel() / K;
+    Tensor h = at::empty({x.size(0), x.size(1), N}, x.options()), r = at::empty({x.size(0), x.size(1), N}, x.options());
+    ok(api.vig_linear_add_rmsnorm_fwd(ptr(x), K, ptr(w), ptr(res), ptr(nw), ptr(r), ptr(h), M, K, N, (float)eps, c.code, c.status, c.stream), "vig_linear_add_rmsnorm_fwd");
+    return {h, r};
+}
+
+// ---- the attention module ------------------------------------------------------------------------------------------
+struct Attn {
+    Tensor taps, conv_b, w_z, b_z, gn_w, ln_w, o_w;
+    int64_t H, dk, dv;
+    bool act_conv, out_act;
+    double eps, out_scale, norm, clamp;
+
+    // everything up to (not including) the output projection; h [B,L,C] contiguous
+    Tensor forward(const Ctx& c, const Tensor& x, int64_t h, int64_t w) const {
+        const int64_t B = x.size(0), L = x.size(1), kd = H * dk, vd = H * dv;
+        const Tensor xs = dwconv(c, x, taps, conv_b, h, w, act_conv);
+        const Tensor z = at::linear(xs, w_z, b_z);
+        const int64_t W = z.size(2);
+        auto view = [&](int64_t col, int64_t d) { return z.as_strided({B, H, L, d}, {L * W, d, W, 1}, z.storage_offset() + col); };
+        Tensor o = at::empty({B, L, H, dv}, x.options());
+        bi_gla_into(view(0, dk), view(kd, dk), view(2 * kd, dv), view(2 * kd + 2 * vd, dk), view(3 * kd + 2 * vd, dk),
+                    o.as_strided({B, H, L, dv}, {L * vd, dv, vd, 1}), -1.0, out_scale, norm, clamp, {}, {}, {}, {}, 3, VIG_IMPL_AUTO);
+        const int64_t so[3] = {L * vd, dv, vd};
+        Tensor y = at::empty({B, L, vd}, x.options());
+        ok(api.vig_gate_inject_fwd(ptr(o), so, ptr(xs), (uint8_t*)ptr(z) + (2 * kd + vd) * z.element_size(), ptr(gn_w), ptr(ln_w), ptr(y), vd, W, vd, B, H, L, dv,
+                                   (float)eps, out_act, c.code, c.stream), "vig_gate_inject_fwd");
+        return y;
+    }
+};
+
+// ---- what a plan was built from --------------------------------------------------------------------------------------
+struct Watch {
+    struct Item { py::object dict, key, value; };
+    struct Param { Tensor t; int64_t version; void* data; at::ScalarType type; };
+    std::vector<Item> items;
+    std::vector<std::pair<py::object, Py_ssize_t>> sizes;
+    std::vector<std::pair<py::object, py::object>> absent;
+    std::vector<Param> params;
+
+    void item(py::object d, py::object k, py::object v) { items.push_back({d, k, v}); }
+    void size(py::object d) { sizes.emplace_back(d, PyDict_Size(d.ptr())); }
+    void missing(py::object d, py::object k) { absent.emplace_back(d, k); }
+    void param(const Tensor& t) { params.push_back({t, (int64_t)t._version(), t.data_ptr(), t.scalar_type()}); }
+    // a module's plain attributes, parameters, children, hooks and the absence of an overridden forward
+    void module(py::handle m) {
+        const py::dict d = m.attr("__dict__");
+        const py::str fwd("forward");
+        for (auto kv : d) {
+            const std::string name = py::cast<std::string>(kv.first);
+            PyObject* v = kv.second.ptr();
+            if (name[0] != '_' && (v == Py_None || PyBool_Check(v) || PyLong_Check(v) || PyFloat_Check(v) || PyUnicode_Check(v) || PyTuple_Check(v)))
+                item(d, py::reinterpret_borrow<py::object>(kv.first), py::reinterpret_borrow<py::object>(kv.second));
+        }
+        for (const char* table : {"_parameters", "_modules"}) {
+            const py::dict t = d[table];
+            for (auto kv : t) {
+                item(t, py::reinterpret_borrow<py::object>(kv.first), py::reinterpret_borrow<py::object>(kv.second));
+                if (table[1] == 'p' && !kv.second.is_none()) param(kv.second.cast<Tensor>());
+            }
+            size(t);
+        }
+        for (const char* h : {"_forward_hooks", "_forward_pre_hooks"}) size(d[h]);
+        missing(d, fwd);
+    }
+    bool same() const {
+        for (const auto& i : items) if (PyDict_GetItem(i.dict.ptr(), i.key.ptr()) != i.value.ptr()) return false;
+        for (const auto& s : sizes) if (PyDict_Size(s.first.ptr()) != s.second) return false;
+        for (const auto& a : absent) if (PyDict_GetItem(a.first.ptr(), a.second.ptr())) return false;
+        for (const auto& p : params) if ((int64_t)p.t._version() != p.version || p.t.data_ptr() != p.data || p.t.scalar_type() != p.type) return false;
+        return true;
+    }
+};
+
+// The device's error word looked at without stalling the stream: the value copied by an earlier forward, if it has landed.
+struct StatusPeek {
+    int32_t* host = nullptr;
+    cudaEvent_t event = nullptr;
+    bool pending = false;
+    static StatusPeek& of(int device) { static StatusPeek s[64]; return s[device]; }
+    int poll(bool capturing) {
+        if (capturing || !pending || cudaEventQuery(event) != cudaSuccess) return 0;
+        pending = false;
+        return *host;
+    }
+    void snapshot(int device, cudaStream_t st, bool capturing) {
+        if (capturing || pending) return;
+        if (!host) {
+            if (cudaHostAlloc(reinterpret_cast<void**>(&host), sizeof(int32_t), cudaHostAllocDefault) != cudaSuccess) { host = nullptr; return; }
+            if (cudaEventCreateWithFlags(&event, cudaEventDisableTiming) != cudaSuccess) return;
+        }
+        if (!event || cudaMemcpyAsync(host, status_ptr(device), sizeof(int32_t), cudaMemcpyDeviceToHost, st) != cudaSuccess) return;
+        pending = cudaEventRecord(event, st) == cudaSuccess;
+    }
+};
+
+struct Conv {
+    Tensor w, b;                                         // channels-last weight; bias may be undefined
+    int64_t stride = 1, pad = 0;
+    // NHWC in, NHWC out
+    Tensor forward(const Tensor& x, bool with_bias) const {
+        const Tensor y = at::conv2d(x.permute({0, 3, 1, 2}), w, with_bias && b.defined() ? OptT(b) : std::nullopt, {stride, stride}, {pad, pad});
+        return y.permute({0, 2, 3, 1}).contiguous();
+    }
+};
+
+struct PlanBase {
+    Watch watch;
+    at::ScalarType type = at::kBFloat16;
+    at::Device device = at::Device(at::kCPU);
+    Tensor head_w, head_b;
+    py::object on_status;                                // called with the error word's value when an earlier forward left one
+
+    bool takes(const Tensor& x) const {
+        return x.is_cuda() && x.device() == device && x.scalar_type() == type && x.dim() == 4 && x.size(1) == 3 && x.numel() > 0 &&
+               !(at::GradMode::is_enabled()) && !at::autocast::is_autocast_enabled(at::kCUDA) && status_known(device.index()) && watch.same();
+    }
+    Tensor finish(const Tensor& pooled) const { return at::linear(pooled, head_w, head_b.defined() ? OptT(head_b) : std::nullopt); }
+    template <typename F> OptT run(const Tensor& x, F body) const {
+        if (!takes(x)) return std::nullopt;
+        c10::cuda::CUDAGuard guard(device);
+        at::NoGradGuard ng;
+        auto st = at::cuda::getCurrentCUDAStream();
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        cudaStreamIsCapturing(st.stream(), &cap);
+        const bool capturing = cap != cudaStreamCaptureStatusNone;
+        StatusPeek& peek = StatusPeek::of(device.index());
+        if (const int v = peek.poll(capturing)) { on_status(v); }
+        const Ctx c{st.stream(), status_ptr(device.index()), type == at::kBFloat16 ? VIG_DTYPE_BF16 : VIG_DTYPE_F16};
+        Tensor y = body(c, x.contiguous());
+        peek.snapshot(device.index(), st.stream(), capturing);
+        return y;
+    }
+};
+
+// ---- ViG -----------------------------------------------------------------------------------------------------------
+struct VigBlock {
+    Tensor n1, n2, gate_w, down_w;
+    double e1, e2;
+    Attn attn;
+};
+
+struct VigPlan : PlanBase {
+    // stem: first convolution as one kernel with its LayerNorm (w_gemm) where the library has it, or as a 2x2 convolution over
+    // unfolded cells (w_cells) followed by the LayerNorm kernel; second convolution and LayerNorm
+    Tensor w_gemm, b1, ln1_w, ln1_b, ln2_w, ln2_b;
+    Conv cells, conv2;
+    double ln1_e, ln2_e;
+    int64_t C = 0;
+    bool fused_norms = false;
+    std::vector<VigBlock> blocks;
+    Tensor norm_w;
+    double norm_e;
+    py::object pos_fn;                                   // (h, w) -> [1, h*w, C], the module's own cache
+    mutable Tensor pos;
+    mutable int64_t pos_h = 0, pos_w = 0;
+
+    OptT forward(const Tensor& x) const {
+        const int64_t H = x.dim() == 4 ? x.size(2) : 0, W = x.dim() == 4 ? x.size(3) : 0;
+        if (H % 8 || W % 8 || H == 0) return std::nullopt;
+        return run(x, [&](const Ctx& c, const Tensor& img) { return body(c, img); });
+    }
+    Tensor body(const Ctx& c, const Tensor& img) const {
+        const int64_t B = img.size(0), H = img.size(2), W = img.size(3);
+        Tensor y;
+        if (w_gemm.defined() && api.vig_stem_conv_ln_supported(B, H / 8, W / 8, 192, C / 2, c.code)) {
+            Tensor f = at::empty({B, H / 8, W / 8, 192}, img.options());
+            ok(api.vig_stem_fold_fwd(ptr(img), ptr(f), B, 3, H, W, c.code, c.stream), "vig_stem_fold_fwd");
+            y = at::empty({B, H / 8, W / 8, C / 2}, img.options());
+            ok(api.vig_stem_conv_ln_fwd(ptr(f), ptr(w_gemm), ptr(b1), ptr(ln1_w), ptr(ln1_b), ptr(y), B, H / 8, W / 8, 192, C / 2, (float)ln1_e, 1, c.code, c.status,
+                                        c.stream), "vig_stem_conv_ln_fwd");
+        } else {
+            Tensor u = at::empty({B, H / 8 + 1, W / 8 + 1, 192}, img.options());
+            ok(api.vig_stem_unfold_fwd(ptr(img), ptr(u), B, 3, H, W, 8, c.code, c.stream), "vig_stem_unfold_fwd");
+            y = layernorm(c, cells.forward(u, false), ln1_w, ln1_b, ln1_e, true, b1);
+        }
+        y = conv2.forward(y, false);
+        const int64_t h = y.size(1), w = y.size(2), L = h * w, rows = B * L;
+        if (!pos.defined() || pos_h != h || pos_w != w) {
+            pos = pos_fn(py::make_tuple(h, w)).cast<Tensor>().to(type).contiguous();
+            pos_h = h; pos_w = w;
+        }
+        Tensor tok = at::empty({B, L, C}, img.options());
+        if (fused_norms) {
+            Tensor n = at::empty({B, L, C}, img.options());
+            ok(api.vig_layernorm_act_add_rmsnorm_fwd(ptr(y), ptr(conv2.b), ptr(ln2_w), ptr(ln2_b), ptr(pos), L, ptr(tok), ptr(blocks[0].n1), (float)blocks[0].e1,
+                                                     ptr(n), rows, C, (float)ln2_e, 0, c.code, c.stream), "vig_layernorm_act_add_rmsnorm_fwd");
+            for (size_t i = 0; i < blocks.size(); ++i) {
+                const VigBlock& b = blocks[i];
+                const bool last = i + 1 == blocks.size();
+                std::tie(n, tok) = linear_add_rmsnorm(c, b.attn.forward(c, n, h, w), b.attn.o_w, tok, b.n2, b.e2);
+                std::tie(n, tok) = linear_add_rmsnorm(c, mlp_in(c, n, b.gate_w), b.down_w, tok, last ? norm_w : blocks[i + 1].n1, last ? norm_e : blocks[i + 1].e1);
+            }
+            return finish(n.mean(1));
+        }
+        ok(api.vig_layernorm_act_add_fwd(ptr(y), ptr(conv2.b), ptr(ln2_w), ptr(ln2_b), ptr(pos), L, ptr(tok), rows, C, (float)ln2_e, 0, c.code, c.stream),
+           "vig_layernorm_act_add_fwd");
+        Tensor branch;                                   // the residual add of a branch rides in the next norm
+        for (const VigBlock& b : blocks) {
+            Tensor n, r;
+            std::tie(n, r) = branch.defined() ? add_rmsnorm(c, branch, b.n1, tok, b.e1, true) : add_rmsnorm(c, tok, b.n1, {}, b.e1, false);
+            if (r.defined()) tok = r;
+            std::tie(n, tok) = add_rmsnorm(c, at::linear(b.attn.forward(c, n, h, w), b.attn.o_w), b.n2, tok, b.e2, true);
+            branch = at::linear(mlp_in(c, n, b.gate_w), b.down_w);
+        }
+        return finish(add_rmsnorm(c, branch, norm_w, tok, norm_e, false).first.mean(1));
+    }
+};
+
+// ---- HierViG -------------------------------------------------------------------------------------------------------
+struct Norm { Tensor w, b; double eps = 0; };
+// r = x + residual (optional), LayerNorm(r) with an activation: {LayerNorm, r}
+std::pair<Tensor, Tensor> add_layernorm(const Ctx& c, const Tensor& x, const Tensor& res, const Norm& n, int act) {
+    const int64_t N = x.size(-1);
+    Tensor y = at::empty_like(x), r = res.defined() ? at::empty_like(x) : Tensor();
+    ok(api.vig_add_layernorm_fwd(ptr(x), ptr(res), ptr(n.w), ptr(n.b), ptr(y), ptr(r), x.numel() / N, N, (float)n.eps, act, c.code, c.stream), "vig_add_layernorm_fwd");
+    return {y, r};
+}
+
+struct HierBlock {
+    Norm n1, n2;
+    Attn attn;
+    bool gated = false;
+    Tensor fc1_w, fc1_b, fc2_w, fc2_b;
+};
+struct HierStage {
+    std::vector<HierBlock> blocks;
+    bool down = false;
+    Conv conv;
+    Norm norm;
+};
+
+struct HierPlan : PlanBase {
+    std::vector<std::tuple<Conv, bool, Norm, int>> embed;   // convolution, whether a LayerNorm follows, the norm, activation (0 / 2 = GELU)
+    std::vector<HierStage> stages;
+    Norm last;
+
+    OptT forward(const Tensor& x) const {
+        return run(x, [&](const Ctx& c, const Tensor& img) { return body(c, img); });
+    }
+    Tensor body(const Ctx& c, const Tensor& img) const {
+        Tensor y = img.permute({0, 2, 3, 1}).contiguous();
+        for (const auto& [conv, has_norm, norm, act] : embed) {
+            y = conv.forward(y, true);
+            if (has_norm) y = add_layernorm(c, y, {}, norm, act).first;
+            else if (act == 2) y = at::gelu(y);
+        }
+        int64_t h = y.size(1), w = y.size(2);
+        Tensor x = y.view({y.size(0), h * w, y.size(3)}), branch;
+        for (const HierStage& st : stages) {
+            for (const HierBlock& b : st.blocks) {
+                Tensor n, r;
+                std::tie(n, r) = add_layernorm(c, branch.defined() ? branch : x, branch.defined() ? x : Tensor(), b.n1, 0);   // the branch's add rides in the norm
+                if (r.defined()) x = r;
+                std::tie(n, x) = add_layernorm(c, at::linear(b.attn.forward(c, n, h, w), b.attn.o_w), x, b.n2, 0);
+                branch = b.gated ? at::linear(mlp_in(c, n, b.fc1_w), b.fc2_w)
+                                 : at::linear(at::gelu(at::linear(n, b.fc1_w, b.fc1_b)), b.fc2_w, b.fc2_b);
+            }
+            if (st.down) {
+                if (branch.defined()) { x = x + branch; branch = Tensor(); }
+                y = st.conv.forward(x.view({x.size(0), h, w, x.size(2)}), true);
+                h = y.size(1); w = y.size(2);
+                x = add_layernorm(c, y.view({y.size(0), h * w, y.size(3)}), {}, st.norm, 0).first;
+            }
+        }
+        const Tensor n = branch.defined() ? add_layernorm(c, branch, x, last, 0).first : add_layernorm(c, x, {}, last, 0).first;
+        return finish(n.mean(1));
+    }
+};
+
+// ---- plans from Python dictionaries ----------------------------------------------------------------------------------
+Tensor tensor_of(const py::dict& d, const char* key) { return d.contains(key) && !d[key].is_none() ? d[key].cast<Tensor>() : Tensor(); }
+Attn attn_of(const py::dict& d) {
+    Attn a;
+    a.taps = tensor_of(d, "taps"); a.conv_b = tensor_of(d, "conv_b"); a.w_z = tensor_of(d, "w_z"); a.b_z = tensor_of(d, "b_z");
+    a.gn_w = tensor_of(d, "gn_w"); a.ln_w = tensor_of(d, "ln_w"); a.o_w = tensor_of(d, "o_w");
+    a.H = d["H"].cast<int64_t>(); a.dk = d["dk"].cast<int64_t>(); a.dv = d["dv"].cast<int64_t>();
+    a.act_conv = d["act_conv"].cast<bool>(); a.out_act = d["out_act"].cast<bool>();
+    a.eps = d["eps"].cast<double>(); a.out_scale = d["out_scale"].cast<double>(); a.norm = d["norm"].cast<double>(); a.clamp = d["clamp"].cast<double>();
+    return a;
+}
+Norm norm_of(const py::dict& d) { return {tensor_of(d, "w"), tensor_of(d, "b"), d["eps"].cast<double>()}; }
+Conv conv_of(const py::dict& d) { return {tensor_of(d, "w"), tensor_of(d, "b"), d["stride"].cast<int64_t>(), d["pad"].cast<int64_t>()}; }
+void base_of(PlanBase& p, const py::dict& d) {
+    p.head_w = tensor_of(d, "head_w"); p.head_b = tensor_of(d, "head_b");
+    p.type = p.head_w.scalar_type(); p.device = p.head_w.device();
+    p.on_status = d["on_status"];
+}
+
+VigPlan* make_vig(const py::dict& d) {
+    auto p = std::make_unique<VigPlan>();
+    base_of(*p, d);
+    p->w_gemm = tensor_of(d, "w_gemm"); p->b1 = tensor_of(d, "b1");
+    const Norm n1 = norm_of(d["ln1"]), n2 = norm_of(d["ln2"]);
+    p->ln1_w = n1.w; p->ln1_b = n1.b; p->ln1_e = n1.eps; p->ln2_w = n2.w; p->ln2_b = n2.b; p->ln2_e = n2.eps;
+    p->cells = conv_of(d["cells"]); p->conv2 = conv_of(d["conv2"]);
+    p->C = p->conv2.w.size(0);
+    p->fused_norms = d["fused_norms"].cast<bool>();
+    p->norm_w = tensor_of(d, "norm_w"); p->norm_e = d["norm_e"].cast<double>();
+    p->pos_fn = d["pos_fn"];
+    for (auto item : d["blocks"].cast<py::list>()) {
+        const py::dict b = item.cast<py::dict>();
+        p->blocks.push_back({tensor_of(b, "n1"), tensor_of(b, "n2"), tensor_of(b, "gate_w"), tensor_of(b, "down_w"), b["e1"].cast<double>(), b["e2"].cast<double>(),
+                             attn_of(b["attn"])});
+    }
+    return p.release();
+}
+
+HierPlan* make_hier(const py::dict& d) {
+    auto p = std::make_unique<HierPlan>();
+    base_of(*p, d);
+    for (auto item : d["embed"].cast<py::list>()) {
+        const py::dict e = item.cast<py::dict>();
+        const bool has = !e["norm"].is_none();
+        p->embed.emplace_back(conv_of(e["conv"]), has, has ? norm_of(e["norm"]) : Norm(), e["act"].cast<int>());
+    }
+    for (auto item : d["stages"].cast<py::list>()) {
+        const py::dict s = item.cast<py::dict>();
+        HierStage st;
+        for (auto bi : s["blocks"].cast<py::list>()) {
+            const py::dict b = bi.cast<py::dict>();
+            st.blocks.push_back({norm_of(b["n1"]), norm_of(b["n2"]), attn_of(b["attn"]), b["gated"].cast<bool>(), tensor_of(b, "fc1_w"), tensor_of(b, "fc1_b"),
+                                 tensor_of(b, "fc2_w"), tensor_of(b, "fc2_b")});
+        }
+        if (!s["conv"].is_none()) { st.down = true; st.conv = conv_of(s["conv"]); st.norm = norm_of(s["norm"]); }
+        p->stages.push_back(std::move(st));
+    }
+    p->last = norm_of(d["last"]);
+    return p.release();
+}
+
+}  // namespace
+
+void bind_model(py::module_& m) {
+    auto watch = [](auto& cls) {
+        using P = typename std::decay_t<decltype(cls)>::type;
+        cls.def("watch_item", [](P& p, py::object d, py::object k, py::object v) { p.watch.item(d, k, v); })
+            .def("watch_size", [](P& p, py::object d) { p.watch.size(d); })
+            .def("watch_modules", [](P& p, const py::list& ms) { for (auto m : ms) p.watch.module(m); })
+            .def("valid", [](const P& p) { return p.watch.same(); })
+            .def("forward", &P::forward);
+    };
+    py::class_<VigPlan> vig(m, "VigPlan");
+    vig.def(py::init(&make_vig));
+    watch(vig);
+    py::class_<HierPlan> hier(m, "HierPlan");
+    hier.def(py::init(&make_hier));
+    watch(hier);
+}
+
+}  // namespace vig_host

@@ -9,7 +9,7 @@
 namespace vig_host {
 
 Api api;
-static Tensor g_status[64];
+static Tensor* const g_status = new Tensor[64];         // never destroyed: outlives the interpreter and the CUDA context's teardown
 
 int32_t* status_ptr(int device) { return device >= 0 && device < 64 && g_status[device].defined() ? g_status[device].data_ptr<int32_t>() : nullptr; }
 bool status_known(int device) { return status_ptr(device) != nullptr; }
@@ -162,4 +162,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("bi_gla", &bi_gla);
     m.def("bi_gla_stacked", &bi_gla_stacked);
     m.def("scan", &scan);
+    bind_model(m);
 }

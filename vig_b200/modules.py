@@ -62,26 +62,25 @@ class GatedLinearAttention(nn.Module):
         self.fold_gate_bottleneck = True
         self.own_in_proj_gemm = False
 
-    def _pack(self):
-        """Derived weight layouts, built once per dtype/device: the conv taps as [9, C] and one stacked
-        matrix for the three projections that read the conv output (qkv, gate low-rank, output gate)."""
+    def _pack(self, fold):
+        """Derived weight layouts ``(taps, w_in, b_in)``, built once per dtype/device and form: the conv taps as [9, C] and one
+        stacked matrix for the projections that read the conv output -- qkv, output gate and the gate's low-rank features, or
+        with ``fold`` the raw gate logits themselves (the rank-16 bottleneck folded into one [2*key_dim, d_model] matrix,
+        product in fp32, rounded once: a K = d_model GEMM of a friendly width instead of 16 odd columns plus a K = 16 GEMM)."""
         w = self.in_proj[0].weight
-        key = (w.dtype, w.device, w._version, self.qkv_proj.weight._version)
+        src = (w, *self.qkv_proj.parameters(), *self.g_proj.parameters(), *self.gk_proj.parameters())
+        key = (fold, w.dtype, w.device, *((t.data_ptr(), t._version) for t in src))
         if self._packed is None or self._packed[0] != key:
-            C = self.d_model
-            taps = w.detach().reshape(C, 9).t().contiguous()
-            stacked = torch.cat([self.qkv_proj.weight, self.g_proj.weight, self.gk_proj[0].weight], dim=0).detach().contiguous()
-            bias = torch.cat([torch.zeros(self.qkv_proj.out_features, dtype=w.dtype, device=w.device), self.g_proj.bias.detach(),
-                              torch.zeros(self.gk_proj[0].out_features, dtype=w.dtype, device=w.device)])
-            # the rank-16 gate bottleneck folded into one [2*key_dim, d_model] matrix (product in fp32, rounded once):
-            # a K = d_model GEMM of a friendly width replaces the 16 odd columns of the stacked projection plus a K = 16 GEMM
-            folded = (self.gk_proj[1].weight.detach().float() @ self.gk_proj[0].weight.detach().float()).to(w.dtype).contiguous()
-            # with the bottleneck folded, its rows join the stacked projection: one GEMM reads the conv output once
-            n_main = self.qkv_proj.out_features + self.g_proj.out_features
-            gk_bias = self.gk_proj[1].bias
-            gk_bias = torch.zeros(folded.shape[0], dtype=w.dtype, device=w.device) if gk_bias is None else gk_bias.detach()
-            merged = (torch.cat([stacked[:n_main], folded], dim=0).contiguous(), torch.cat([bias[:n_main], gk_bias]))
-            self._packed = (key, taps, stacked, bias, merged)
+            taps = w.detach().reshape(self.d_model, 9).t().contiguous()
+            qkv, g, (low, high) = self.qkv_proj, self.g_proj, self.gk_proj
+            if fold:
+                last = (high.weight.detach().float() @ low.weight.detach().float()).to(w.dtype)
+                tail_bias = high.bias if high.bias is not None else w.new_zeros(high.out_features)
+            else:
+                last, tail_bias = low.weight, w.new_zeros(low.out_features)
+            stacked = torch.cat([qkv.weight, g.weight, last], dim=0).detach()
+            bias = torch.cat([w.new_zeros(qkv.out_features), g.bias, tail_bias]).detach()
+            self._packed = (key, taps, stacked, bias)
         return self._packed[1:]
 
     def forward(self, x, lower_bound=0, **kwargs):
@@ -90,7 +89,9 @@ class GatedLinearAttention(nn.Module):
         B, L, C = x.shape
         hw = kwargs["patch_resolution"]
         H, dk, dv, kd, vd = self.num_heads, self.head_qk_dim, self.head_v_dim, self.key_dim, self.value_dim
-        taps, w_in, b_in, merged = self._pack()
+        fold = self.fold_gate_bottleneck and x.dtype != torch.float32
+        # one GEMM for [q | k | v | output-gate logits | low-rank gate features] (folded: | raw gate logits)
+        taps, w_z, b_z = self._pack(fold)
         # ``local_fn`` / ``scan_fn`` let a caller substitute the two steps that look beyond the tokens at hand (the
         # 3x3 neighbourhood and the scan) -- the sequence-parallel driver supplies halo and boundary-state versions
         local_fn, scan_fn = kwargs.get("local_fn"), kwargs.get("scan_fn")
@@ -98,10 +99,7 @@ class GatedLinearAttention(nn.Module):
             xs = ops.dwconv3x3(x, taps, self.in_proj[0].bias, hw, self.use_act_in_conv)
         else:
             xs = local_fn(x, taps, self.in_proj[0].bias, hw, self.use_act_in_conv)
-        fold = self.fold_gate_bottleneck and x.dtype != torch.float32
         n_main = 2 * kd + 2 * vd
-        # one GEMM for [q | k | v | output-gate logits | low-rank gate features] (folded: | raw gate logits)
-        w_z, b_z = (merged[0], merged[1]) if fold else (w_in, b_in)
         # the vendor GEMM by default: the library's own kernel for this product (``ops.linear_bias``) measures 171 us against
         # 160-165 us at the benchmark's shape; ``own_in_proj_gemm`` switches it in where it is supported
         use_own = self.own_in_proj_gemm and ops.linear_bias_supported(xs, w_z)

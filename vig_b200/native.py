@@ -1,0 +1,144 @@
+"""Plans for the C++ forward of the models (``vig_b200/csrc/host_model.cpp``): what the Python modules hold, collected once.
+
+``forward(model, images)`` runs the model's plan, building or rebuilding it when something it was built from has changed, and
+answers ``None`` whenever the modules themselves have to run: a precision or configuration without a plan, subclassed or
+hooked modules, an overridden ``forward``, replaced operators of ``vig_b200.ops``, gradients enabled, autocast."""
+import math
+import weakref
+
+import torch
+import torch.nn as nn
+
+from . import _lib, hier, modules, ops, vig
+
+_plans = weakref.WeakKeyDictionary()          # model -> plan, or False where the model has none
+_OPS = {n: getattr(ops, n) for n in ("bi_gla", "dwconv3x3", "gate_inject", "add_rmsnorm", "layernorm_act", "add_layernorm", "linear_swiglu",
+                                     "linear_add_rmsnorm", "linear_bias", "swiglu", "stem_fold", "stem_unfold", "stem_conv_ln")}
+_CLASSES = (vig.ViG, vig.V2PatchEmbed, vig.LayerNorm2d, modules.GLABlock, modules.GatedLinearAttention, modules.GLAMLP, modules.RMSNorm,
+            hier.HierViG, hier.VSSBlock, hier.GLA2D, hier.Mlp, hier.gMlp, nn.Linear, nn.Conv2d, nn.LayerNorm, nn.SiLU, nn.GELU, nn.Identity,
+            nn.Sequential, nn.ModuleList)
+
+
+def _status_seen(device):
+    return lambda value: ops.status_word(device)._raise(value)
+
+
+def _watch(plan, mods):
+    """Everything whose change makes the plan stale (the C++ side compares identities, versions and sizes)."""
+    plan.watch_modules(mods)
+    for name in ("_global_forward_hooks", "_global_forward_pre_hooks"):
+        plan.watch_size(getattr(nn.modules.module, name))
+    for name, fn in _OPS.items():
+        plan.watch_item(ops.__dict__, name, fn)
+
+
+def _norm(m):
+    return dict(w=m.weight, b=getattr(m, "bias", None), eps=m.eps)
+
+
+def _conv(m, weight=None, stride=None, pad=None):
+    w = (m.weight.detach() if weight is None else weight).contiguous(memory_format=torch.channels_last)
+    return dict(w=w, b=m.bias, stride=m.stride[0] if stride is None else stride, pad=m.padding[0] if pad is None else pad)
+
+
+def _attn(a):
+    if not a.fold_gate_bottleneck or a.own_in_proj_gemm or a.o_proj.bias is not None:
+        return None
+    taps, w_z, b_z = a._pack(True)
+    return dict(taps=taps, conv_b=a.in_proj[0].bias, w_z=w_z, b_z=b_z, gn_w=a.g_norm.weight, ln_w=a.l_norm.weight, o_w=a.o_proj.weight,
+                H=a.num_heads, dk=a.head_qk_dim, dv=a.head_v_dim, act_conv=bool(a.use_act_in_conv), out_act=bool(a.use_out_act), eps=a.g_norm.eps,
+                out_scale=a.out_scale, norm=float(a.gate_logit_normalizer), clamp=math.nan if a.clamp_min is None else float(a.clamp_min))
+
+
+def _vig(model):
+    pe, conv1 = model.patch_embed, model.patch_embed.proj[0]
+    if pe.stride != 8 or conv1.weight.shape[1] != 3 or not isinstance(model.head, nn.Linear) or not len(model.blocks):
+        return None
+    blocks = []
+    for b in model.blocks:
+        attn = _attn(b.attn)
+        if attn is None or b.mlp.down_proj.bias is not None or b.mlp.gate_proj.bias is not None:
+            return None
+        blocks.append(dict(n1=b.attn_norm.weight, e1=b.attn_norm.eps, n2=b.mlp_norm.weight, e2=b.mlp_norm.eps, gate_w=b.mlp.gate_proj.weight,
+                           down_w=b.mlp.down_proj.weight, attn=attn))
+    probe = model.head.weight.new_empty(1, 1, model.embed_dim)
+    fused = model.fuse_norm_epilogues and all(b.fused_epilogues_supported(probe) for b in model.blocks)
+    one_kernel = pe.fuse_conv1 and conv1.weight.shape[0] == 96
+    ref = weakref.ref(model)
+    return _lib.host().VigPlan(dict(
+        head_w=model.head.weight, head_b=model.head.bias, on_status=_status_seen(model.head.weight.device), blocks=blocks, fused_norms=fused,
+        w_gemm=pe._gemm_weight() if one_kernel else None, b1=conv1.bias, ln1=_norm(pe.proj[1]), ln2=_norm(pe.proj[4]),
+        cells=_conv(conv1, weight=pe._block_weight(), stride=1, pad=0), conv2=_conv(pe.proj[3]), norm_w=model.norm.weight, norm_e=model.norm.eps,
+        pos_fn=lambda hw: ref()._pos(hw)))
+
+
+def _hier(model):
+    embed, pe = [], list(model.patch_embed)
+    for i, m in enumerate(pe):
+        if isinstance(m, nn.Conv2d):
+            rest = pe[i + 1:]
+            rest = rest[:next((j for j, r in enumerate(rest) if isinstance(r, nn.Conv2d)), len(rest))]
+            norm = next((r for r in rest if isinstance(r, nn.LayerNorm)), None)
+            gelu = next((r for r in rest if isinstance(r, nn.GELU)), None)
+            if gelu is not None and gelu.approximate != "none":
+                return None
+            embed.append(dict(conv=_conv(m), norm=None if norm is None else _norm(norm), act=0 if gelu is None else 2))
+    stages = []
+    for layer in model.layers:
+        blocks = []
+        for b in layer.blocks:
+            attn, gated = _attn(b.op), isinstance(b.mlp, hier.gMlp)
+            if attn is None or not (gated or isinstance(b.mlp.act, nn.GELU) and b.mlp.act.approximate == "none"):
+                return None
+            blocks.append(dict(n1=_norm(b.norm), n2=_norm(b.norm2), attn=attn, gated=gated, fc1_w=b.mlp.fc1.weight, fc1_b=b.mlp.fc1.bias,
+                               fc2_w=b.mlp.fc2.weight, fc2_b=b.mlp.fc2.bias))
+        down = layer.downsample
+        has = not isinstance(down, nn.Identity)
+        stages.append(dict(blocks=blocks, conv=_conv(down[1]) if has else None, norm=_norm(down[3]) if has else None))
+    head = model.classifier.head
+    return _lib.host().HierPlan(dict(head_w=head.weight, head_b=head.bias, on_status=_status_seen(head.weight.device), embed=embed, stages=stages,
+                                     last=_norm(model.classifier.norm)))
+
+
+def _build(model, make):
+    mods = list(model.modules())
+    if model.training or any(type(m) not in _CLASSES or "forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks for m in mods):
+        return False
+    params = [p for m in mods for p in m._parameters.values() if p is not None]
+    if any(p.dtype != params[0].dtype or p.device != params[0].device for p in params):
+        return False
+    with torch.no_grad():
+        plan = make(model)
+    if plan is None:
+        return False
+    _watch(plan, mods)
+    return plan
+
+
+def _forward(model, images, head, make):
+    if torch.is_grad_enabled() or head.dtype not in (torch.bfloat16, torch.float16) or type(images) is not torch.Tensor or not images.is_cuda:
+        return None
+    plan = _plans.get(model)
+    if plan:
+        y = plan.forward(images)
+        if y is not None or plan.valid():
+            return y
+    elif plan is False and model.__dict__.get("_plan_refused") is head.dtype:
+        return None
+    if any(ops.__dict__[n] is not fn for n, fn in _OPS.items()) or head.device != images.device:
+        return None
+    ops.status_word(images.device)
+    plan = _plans[model] = _build(model, make)
+    if not plan:
+        model._plan_refused = head.dtype              # not asked again for this precision: the modules run instead
+        return None
+    return plan.forward(images)
+
+
+def vig_forward(model, images):
+    head = model.head
+    return _forward(model, images, head.weight, _vig) if isinstance(head, nn.Linear) else None
+
+
+def hier_forward(model, images):
+    return _forward(model, images, model.classifier.head.weight, _hier)

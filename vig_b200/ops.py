@@ -395,6 +395,21 @@ def layernorm_act(x, weight, bias, eps=1e-5, act_swish=False, pre_bias=None, pos
     return y
 
 
+def add_layernorm(x, weight, bias, eps=1e-5, residual=None, act=0):
+    """``r = x + residual`` (optional), ``y = LayerNorm(r) * weight + bias`` over the last dimension, then ``act``: 0 none,
+    1 swish, 2 GELU (erf form).  Returns ``y``, or ``(y, r)`` with a residual."""
+    _lib.require_cuda(x, weight, bias, residual)
+    N = x.shape[-1]
+    if not x.is_contiguous() or (residual is not None and (not residual.is_contiguous() or residual.shape != x.shape or residual.dtype != x.dtype)):
+        raise ValueError("x and residual must be contiguous tensors of one shape and dtype")
+    y = torch.empty_like(x)
+    r = torch.empty_like(x) if residual is not None else None
+    st = _lib.lib().vig_add_layernorm_fwd(_lib.ptr(x), _lib.ptr(residual), _lib.ptr(weight), _lib.ptr(bias), _lib.ptr(y), _lib.ptr(r), x.numel() // N, N,
+                                          float(eps), int(act), _lib.dtype_code(x), _lib.stream_ptr())
+    _lib.check(st, "vig_add_layernorm_fwd")
+    return y if residual is None else (y, r)
+
+
 def linear_add_rmsnorm_supported(x, w):
     """True when ``linear_add_rmsnorm`` can run on these operands (16-bit CUDA tensors, K % 64 == 0, N in {64, 128, 192, 256, 384})."""
     if not (x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and w.dtype == x.dtype and x.stride(-1) == 1):

@@ -201,7 +201,11 @@ class ViG(nn.Module):
         """Logits.  The kernels' error word is looked at without stalling the stream: this call raises if a kernel of an
         EARLIER forward reported an error (its status copy has landed by now), and queues the copy for its own;
         ``vig_b200.check_status()`` is the blocking form."""
-        from . import ops
+        from . import native, ops
+        if not kwargs:
+            logits = native.vig_forward(self, x)        # the same kernels launched from C++; None where the modules have to run
+            if logits is not None:
+                return logits
         status = ops.status_word(x.device)
         status.poll()
         logits = self.head(self.forward_features(x))
