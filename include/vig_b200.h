@@ -59,6 +59,9 @@ extern "C" {
                               CTA per SM, states handed from segment to segment; built for batches with at least as
                               many (sequence, direction) chains as the GPU has SMs */
 
+#define VIG_IMPL_SEG 6       /* mma.sync form, both directions of a 64- or 128-token segment in one sweep ((dk, dv) of (16,32), (32,32),
+                              (32,64), (64,64), every type) */
+
 VIG_API int vig_version(void);
 VIG_API const char* vig_strerror(int status);
 

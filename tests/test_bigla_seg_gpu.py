@@ -1,5 +1,6 @@
-"""Full-precision tensor-core forward (fp32, and 16-bit heads with dv = 32) at chunk edges (64 tokens), with entering and
-final states, one direction, gates that leave the factorisation's range, and rows only the token-by-token form can read."""
+"""The segment form of the forward (mma.sync; fp32, dv = 32, short and medium 16-bit sequences): segment edges, one-launch
+clusters of 1 to 8 segments and the three-launch form above, entering and final states, one direction, gates that leave the
+factorisation's range, and rows only the token-by-token form can read."""
 import pytest
 import torch
 
@@ -23,8 +24,22 @@ def test_forward_at_chunk_edges(dtype, dk, dv, L, strength):
     assert rel_err(vig_b200.bi_gla(*[t.cuda() for t in ins]).float(), ref) < TOL[dtype]
 
 
+@pytest.mark.parametrize("dtype,dk,dv", [(torch.bfloat16, 64, 64), (torch.bfloat16, 32, 64), (torch.float16, 64, 64)])
+@pytest.mark.parametrize("B,L,strength", [(1, 64, 1.0), (1, 100, 1.0), (1, 513, 1.0), (40, 130, 1.0), (1, 1024, 1.0), (1, 1030, 1.0), (1, 300, 60.0)])
+def test_forward_of_16_bit_heads(dtype, dk, dv, B, L, strength):
+    """64- and 128-token segments, 1 to 8 of them in a cluster, nine and more in three launches.  bf16 runs on bf16 operands (one
+    term): three roundings of 2^-9 per product on random signs, in the max norm."""
+    import vig_b200
+    from vig_b200 import _lib
+    q, k, v, gf, gb = oracle.make_bigla_inputs(B, 2, L, dk, dv, seed=L + dk)
+    ins = [t.to(dtype) for t in (q, k, v, gf * strength, gb)]
+    ref = oracle.naive_bi_gla(*[t.float() for t in ins])
+    tol = 1.5e-2 if dtype == torch.bfloat16 else 2e-3
+    assert rel_err(vig_b200.bi_gla(*[t.cuda() for t in ins], impl=_lib.IMPL_SEG).float(), ref) < tol
+
+
 @pytest.mark.parametrize("dtype,dk,dv", [(torch.float32, 64, 64), (torch.float16, 16, 32)])
-@pytest.mark.parametrize("L", [64, 130])
+@pytest.mark.parametrize("L", [64, 130, 1200])
 def test_one_direction_continues_from_a_state(dtype, dk, dv, L):
     import vig_b200
     q, k, v, g, _ = [t.to(dtype) for t in oracle.make_bigla_inputs(1, 2, L, dk, dv, seed=3)]

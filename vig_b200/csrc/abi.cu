@@ -85,7 +85,7 @@ int vig::bigla_fwd_internal(const void* q, const void* k, const void* v, const v
     if (dtype < 0 || dtype > 2) return VIG_ERR_DTYPE;
     if (B < 0 || H <= 0 || L < 0 || !dims_ok(dk, dv)) return VIG_ERR_SHAPE;
     if (dir_mask < 1 || dir_mask > 3) return VIG_ERR_ARG;
-    if (impl < VIG_IMPL_AUTO || impl > VIG_IMPL_TC_WAVE) return VIG_ERR_ARG;
+    if (impl < VIG_IMPL_AUTO || impl > VIG_IMPL_SEG) return VIG_ERR_ARG;
     if (B == 0 || L == 0) return VIG_OK;
     if (!k || !v) return VIG_ERR_NULL;
     if (o && !q) return VIG_ERR_NULL;
@@ -114,6 +114,14 @@ int vig::bigla_fwd_internal(const void* q, const void* k, const void* v, const v
         if (workspace && (reinterpret_cast<uintptr_t>(workspace) & 255)) return VIG_ERR_ALIGN;
         return bigla_wave_launch(p, workspace, workspace_bytes, (cudaStream_t)stream);
     }
+    if (impl == VIG_IMPL_SEG || (impl == VIG_IMPL_AUTO && !no_single && bigla_seg_supported(p) && bigla_seg_preferred(p))) {
+        if (!bigla_seg_supported(p)) return VIG_ERR_SHAPE;
+        const bool needs_ws = need_states || L > 64;
+        if (needs_ws && (!workspace || workspace_bytes < bigla_simt_workspace(B, H, L, dk, dv))) return VIG_ERR_WORKSPACE;
+        if (needs_ws && (reinterpret_cast<uintptr_t>(workspace) & 15)) return VIG_ERR_ALIGN;
+        p.ws_state = reinterpret_cast<float*>(workspace);
+        return bigla_seg_launch(p, (cudaStream_t)stream);
+    }
     if (impl == VIG_IMPL_AUTO && !no_single && bigla_wave_supported(p) && bigla_wave_preferred(p) && workspace &&
         !(reinterpret_cast<uintptr_t>(workspace) & 255) && workspace_bytes >= bigla_wave_workspace(B, H, L, dk, dv))
         return bigla_wave_launch(p, workspace, workspace_bytes, (cudaStream_t)stream);
@@ -139,6 +147,5 @@ int vig::bigla_fwd_internal(const void* q, const void* k, const void* v, const v
     const size_t nchunk = (L + 63) / 64;
     p.ws_state = reinterpret_cast<float*>(workspace);
     p.ws_decay = p.ws_state ? p.ws_state + (size_t)B * H * nchunk * 2 * dk * dv : nullptr;
-    if (impl == VIG_IMPL_AUTO && bigla_mma_supported(p)) return bigla_mma_launch(p, (cudaStream_t)stream);   // same workspace layout
     return bigla_simt_launch(p, (cudaStream_t)stream);
 }

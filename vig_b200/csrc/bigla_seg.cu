@@ -1,0 +1,623 @@
+// Bi-directional gated linear attention, segments of up to 64 or 128 tokens on mma.sync tensor cores, both directions of a
+// segment in one sweep: the forward of short and medium sequences, of head sizes the tcgen05 kernels do not take (dv = 32),
+// and of fp32 calls.
+//
+// Inside a segment the two directions are one product.  With G the cumulative log-gate of a direction in its scan order, r
+// its value near the segment's middle, Q = q 2^(G-r), K = k 2^(r-G):
+//     P_ij = Qf_i Kf_j (j < i),  Qb_i Kb_j (j > i),  both for j = i           o_i = c (P_i V + Qf_i (2^rf Sf) + Qb_i (2^rb Sb))
+// so a 16 x 16 block off the diagonal is computed once, with the tiles of the direction that owns it, and P V once for both.
+// Sf, Sb are the states entering the segment from its two sides.  A segment's own contribution, U = 2^(l-r) K^T V (l = total),
+// goes to the workspace; the segments of a sequence form one thread-block cluster, meet at its barrier after their products
+// (which need no state) and each sums the contributions that reach it: one launch, every input read once, for sequences of up
+// to 8 segments.  Longer ones run as states, scan over segments (bigla_simt_state_scan), outputs.
+//
+// Against the two-CTAs-per-SM tcgen05 form, which walks 128-token chunks one after the other in each direction with a tensor
+// memory round trip for the scores: P stays in registers, a segment's rows spread over all warps at once.  One segment takes
+// about 22 k cycles alone (loads and gates 6, tiles 3, contribution 4, products 3, states 3, read-out 2): a call of few
+// segments is that latency, one of many is bound by instruction issue at 16 warps an SM.
+// Operands are split into bf16 terms (mma_common.cuh): one term for bf16 with dv = 64 (as in the tcgen05 kernels), two for
+// fp16 and for dv = 32, three for fp32.  A segment whose |G - r| leaves the factorisation's range is evaluated token by token.
+#include "mma_common.cuh"
+
+namespace vig {
+namespace {
+
+using namespace mm;
+using tc::F2; using tc::f2_make; using tc::f2_lo; using tc::f2_hi; using tc::f2_add; using tc::f2_mul; using tc::f2_fma;
+
+enum { SEG_ONE = 0, SEG_STATES = 1, SEG_OUT = 2 };       // one launch (cluster = sequence) / contributions only / outputs from entering states
+
+template <int DK, int DV, typename T> struct SegTerms {
+    static constexpr int RAW = Terms<T>::RAW, SC = (sizeof(T) == 2 && RAW == 1 && DV == 64) ? 1 : Terms<T>::SC;
+};
+
+template <int DK, int DV, typename T, int TOK> struct SegSmem {
+    using TT = SegTerms<DK, DV, T>;
+    static constexpr uint32_t QT = TT::SC * TOK * Pitch<DK>::B;        // one direction's Q or K terms
+    static constexpr uint32_t V = 0, K = TT::RAW * TOK * Pitch<DV>::B, Q = K + 2 * QT, SUM = Q + 2 * QT,
+                              SCL = SUM + 2 * (TOK / 16) * DK * 4,      // per direction and warp: summed log-gates of the warp's rows
+                              BYTES = SCL + 4 * DK * 4;                 // [dir][0: 2^r, 1: 2^(l-r)]
+    static_assert(TT::SC * DK * Pitch<DV>::B <= QT, "the entering states reuse the K tiles");
+    static_assert(SUM >= TOK * DV * 4, "the exact form keeps its outputs in the tiles");
+};
+
+// Two neighbouring values as they lie in memory.  ``open_gate``: a pair that stands for log-gate 0 (rows past the end) --
+// the logit +inf, or the log-gate 0 itself.
+template <typename T> struct Raw2 {
+    uint32_t w;
+    __device__ __forceinline__ void load(const T* p) { w = __ldg(reinterpret_cast<const uint32_t*>(p)); }
+    __device__ __forceinline__ void zero() { w = 0u; }
+    __device__ __forceinline__ void open_gate(bool logits) { w = logits ? (std::is_same<T, __half>::value ? 0x7C007C00u : 0x7F807F80u) : 0u; }
+    __device__ __forceinline__ F2 f2() const {
+        if constexpr (std::is_same<T, __half>::value) { const float2 f = tc::Pack2<__half>::unpack(w); return f2_make(f.x, f.y); }
+        else return f2_make(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
+    }
+};
+template <> struct Raw2<float> {
+    float2 w;
+    __device__ __forceinline__ void load(const float* p) { w = __ldg(reinterpret_cast<const float2*>(p)); }
+    __device__ __forceinline__ void zero() { w = make_float2(0.f, 0.f); }
+    __device__ __forceinline__ void open_gate(bool logits) { w.x = w.y = logits ? INFINITY : 0.f; }
+    __device__ __forceinline__ F2 f2() const { return f2_make(w.x, w.y); }
+};
+// x * e of a raw pair and a pair of fp32 factors, in SC bf16 terms (one term: factors rounded to bf16, packed multiply)
+template <typename T, int SC> __device__ __forceinline__ void scaled(const Raw2<T>& x, float ex, float ey, uint32_t* t) {
+    if constexpr (SC == 1) {
+        const __nv_bfloat162 e = __floats2bfloat162_rn(ex, ey), r = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&x.w), e);
+        t[0] = *reinterpret_cast<const uint32_t*>(&r);
+    } else {
+        const F2 v = f2_mul(x.f2(), f2_make(ex, ey));
+        split2<SC>(f2_lo(v), f2_hi(v), t);
+    }
+}
+
+template <typename T, int COLS, int TERMS, int TOK> __device__ __forceinline__ void seg_load_v(uint8_t* dst, const T* src, int64_t stride_l, int n) {
+    constexpr uint32_t P = Pitch<COLS>::B;
+    constexpr int NTH = 2 * TOK;
+    if constexpr (TERMS == 1) {
+        constexpr int VPR = COLS / 8;
+#pragma unroll
+        for (int i0 = 0; i0 < TOK * VPR; i0 += NTH) {
+            const int i = i0 + threadIdx.x, r = i / VPR, v = i % VPR;
+            const uint32_t d = tc::smem_u32(dst + r * P + v * 16);
+            const T* s = src + (r < n ? r : 0) * stride_l + v * 8;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(s), "r"(r < n ? 16 : 0) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    } else {
+        constexpr int PPR = COLS / 4;
+#pragma unroll 4
+        for (int i0 = 0; i0 < TOK * PPR; i0 += NTH) {
+            const int i = i0 + threadIdx.x, r = i / PPR, v = i % PPR;
+            float2 a = make_float2(0.f, 0.f), b = a;
+            if (r < n) { a = load2<T>(src + r * stride_l + 4 * v); b = load2<T>(src + r * stride_l + 4 * v + 2); }
+            uint32_t ta[TERMS], tb[TERMS];
+            split2<TERMS>(a.x, a.y, ta); split2<TERMS>(b.x, b.y, tb);
+#pragma unroll
+            for (int t = 0; t < TERMS; ++t) *reinterpret_cast<uint2*>(dst + t * TOK * P + r * P + v * 8) = make_uint2(ta[t], tb[t]);
+        }
+    }
+}
+
+struct SegParams {
+    BiglaParams p;
+    int nseg, seglen;            // segments per sequence, tokens per segment (a multiple of 16; the last one may be shorter)
+    int need_states;             // contributions are wanted (more than one segment, or final states)
+};
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// State entering segment c from the side a direction comes from, four values starting at e4 (SEG_ONE: summed here from the
+// segments' contributions; SEG_OUT: what the scan left in the segment's slot).
+template <int DK, int DV, int MODE> __device__ __forceinline__ float4 entering(const SegParams& s, int bh, int c, int dir, int e4) {
+    const BiglaParams& p = s.p;
+    const float4* U = reinterpret_cast<const float4*>(p.ws_state);
+    constexpr int per = DK * DV / 4;
+    if (MODE == SEG_OUT) return __ldcg(U + (((size_t)bh * s.nseg + c) * 2 + dir) * per + e4);
+    const float* init = dir ? p.init_b : p.init_f;
+    float4 S = init ? __ldg(reinterpret_cast<const float4*>(init) + (size_t)bh * per + e4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int d = e4 * 4 / DV, m = dir ? s.nseg - 1 - c : c;
+#pragma unroll 4
+    for (int i = 0; i < m; ++i) {
+        const size_t slot = ((size_t)bh * s.nseg + (dir ? s.nseg - 1 - i : i)) * 2 + dir;
+        const float4 u = __ldcg(U + slot * per + e4);
+        const float a = __expf(__ldcg(p.ws_decay + slot * DK + d));
+        S.x = fmaf(S.x, a, u.x); S.y = fmaf(S.y, a, u.y); S.z = fmaf(S.z, a, u.z); S.w = fmaf(S.w, a, u.w);
+    }
+    return S;
+}
+
+// A segment token by token (any gates); so: [seglen][DV] floats of shared memory.  Thread j < DV owns value column j.
+template <int DK, int DV, typename T, int MODE> __device__ __noinline__ void exact_segment(const SegParams& s, float* so, int bh, int c, int n) {
+    const BiglaParams& p = s.p;
+    const int b = bh / p.H, h = bh % p.H, j = threadIdx.x;
+    const int64_t t0 = (int64_t)c * s.seglen;
+    if (j >= DV) return;
+    for (int i = 0; i < n; ++i) so[i * DV + j] = 0.f;
+    for (int dir = 0; dir < 2; ++dir) {
+        if (!(p.dir_mask & (1 << dir))) continue;
+        float st[DK];
+        for (int d = 0; d < DK; ++d) {
+            const float4 x = entering<DK, DV, MODE>(s, bh, c, dir, (d * DV + j) / 4);
+            st[d] = (j & 3) == 0 ? x.x : (j & 3) == 1 ? x.y : (j & 3) == 2 ? x.z : x.w;
+        }
+        for (int ii = 0; ii < n; ++ii) {
+            const int i = dir ? n - 1 - ii : ii;
+            const T* g = (dir ? head_ptr<T>(p.gb, p.sgb, b, h, t0 + i) : head_ptr<T>(p.gf, p.sgf, b, h, t0 + i));
+            const T *q = head_ptr<T>(p.q, p.sq, b, h, t0 + i), *k = head_ptr<T>(p.k, p.sk, b, h, t0 + i);
+            const float v = DType<T>::to_f(head_ptr<T>(p.v, p.sv, b, h, t0 + i)[j]);
+            float acc = 0.f;
+            for (int d = 0; d < DK; ++d) {
+                st[d] = fmaf(st[d], __expf(gate_transform(DType<T>::to_f(g[d]), p.gate_norm, p.clamp_min)), DType<T>::to_f(k[d]) * v);
+                acc = fmaf(p.qscale * DType<T>::to_f(q[d]), st[d], acc);
+            }
+            so[i * DV + j] += acc;
+        }
+    }
+    for (int i = 0; i < n; ++i)
+        (reinterpret_cast<T*>(p.o) + b * p.so[0] + h * p.so[1] + (t0 + i) * p.so[2])[j] = DType<T>::from_f(so[i * DV + j]);
+}
+
+template <int DK, int DV, typename T, int TOK> constexpr int seg_min_blocks() {
+    constexpr int fit = 225 * 1024 / (int)(SegSmem<DK, DV, T, TOK>::BYTES + 1024), regs = 512 / (2 * TOK);      // 128 registers a thread
+    return fit < 1 ? 1 : fit < regs ? fit : regs;
+}
+
+template <int DK, int DV, typename T, int TOK, int MODE>
+__global__ void __launch_bounds__(2 * TOK, seg_min_blocks<DK, DV, T, TOK>()) bigla_seg_kernel(const __grid_constant__ SegParams s) {
+    using SM = SegSmem<DK, DV, T, TOK>;
+    constexpr int RAW = SM::TT::RAW, SC = SM::TT::SC, NTH = 2 * TOK, W = NTH / 32;
+    constexpr int PAIRS = DK / 2, SUB = 32 / PAIRS, RPG = 16 / SUB, MT = DK / 16;   // a warp's gates: 16 rows, SUB groups of RPG
+    constexpr uint32_t PK = Pitch<DK>::B, PV = Pitch<DV>::B, TK = TOK * PK, TV = TOK * PV, TS = DK * PV;   // TK, TV, TS: from term to term
+    const BiglaParams& p = s.p;
+    extern __shared__ __align__(16) uint8_t smem[];
+    const uint32_t sb = tc::smem_u32(smem);
+    float* gsum = reinterpret_cast<float*>(smem + SM::SUM);              // [dir][warp][DK]
+    float* scl = reinterpret_cast<float*>(smem + SM::SCL);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int c = blockIdx.x, bh = blockIdx.y, b = bh / p.H, h = bh % p.H;
+    const int64_t t0 = (int64_t)c * s.seglen;
+    const int n = min(s.seglen, p.L - (int)t0), nb = (n + 15) / 16;
+    const int pr = threadIdx.x % PAIRS, gr = threadIdx.x / PAIRS, r0 = gr * RPG;   // my channel pair, my rows
+    const bool want_out = MODE != SEG_STATES && p.o;
+    const bool fwd = p.dir_mask & 1, bwd = p.dir_mask & 2;
+    F2 G[2][RPG], ref[2], tot[2];
+    Raw2<T> kr[RPG];
+    bool fine = true;
+    {   // ---- every input of the segment requested at once, gates cumulated, operand tiles written
+        seg_load_v<T, DV, RAW, TOK>(smem + SM::V, head_ptr<T>(p.v, p.sv, b, h, t0), p.sv[2], n);
+        const bool logits = p.gate_norm > 0.f, clamp = p.clamp_min == p.clamp_min;
+        Raw2<T> qr[RPG];
+        {
+            Raw2<T> xr[2][RPG];
+            // rows past the end read the last row (no branch between the loads) and are neutralised afterwards; an absent
+            // tensor reads k in its place
+            const T* kp = head_ptr<T>(p.k, p.sk, b, h, t0) + 2 * pr;
+            const T* qp = want_out ? head_ptr<T>(p.q, p.sq, b, h, t0) + 2 * pr : kp;
+            const T* fp = fwd ? head_ptr<T>(p.gf, p.sgf, b, h, t0) + 2 * pr : kp;
+            const T* bp = bwd ? head_ptr<T>(p.gb, p.sgb, b, h, t0) + 2 * pr : kp;
+            const int64_t lk = p.sk[2], lq = want_out ? p.sq[2] : lk, lf = fwd ? p.sgf[2] : lk, lb = bwd ? p.sgb[2] : lk;
+#pragma unroll
+            for (int r = 0; r < RPG; ++r) {
+                const int64_t row = min(r0 + r, n - 1);
+                xr[0][r].load(fp + row * lf);
+                xr[1][r].load(bp + row * lb);
+                kr[r].load(kp + row * lk);
+                if (MODE != SEG_STATES) qr[r].load(qp + row * lq); else qr[r].zero();
+            }
+            if (r0 + RPG > n) {
+#pragma unroll
+                for (int r = 0; r < RPG; ++r)
+                    if (r0 + r >= n) { kr[r].zero(); qr[r].zero(); xr[0][r].open_gate(logits); xr[1][r].open_gate(logits); }
+            }
+            const F2 zero = f2_make(0.f, 0.f), one = f2_make(1.f, 1.f);
+            const F2 nlog2e = f2_make(-tc::LOG2E, -tc::LOG2E);
+#pragma unroll
+            for (int dir = 0; dir < 2; ++dir) {
+                F2 run = zero;
+                if (sizeof(T) == 2 && logits && !clamp) {                // the models' form: -log2(1 + 2^(-x log2 e)) / norm
+                    const float ni = -1.f / p.gate_norm;
+                    const F2 ninv = f2_make(ni, ni);
+#pragma unroll
+                    for (int rr = 0; rr < RPG; ++rr) {
+                        const int r = dir ? RPG - 1 - rr : rr;
+                        const F2 y = f2_mul(xr[dir][r].f2(), nlog2e);
+                        const F2 z = f2_add(f2_make(tc::ex2(f2_lo(y)), tc::ex2(f2_hi(y))), one);
+                        run = f2_fma(f2_make(tc::lg2(f2_lo(z)), tc::lg2(f2_hi(z))), ninv, run);
+                        G[dir][r] = run;
+                    }
+                } else {
+                    const float inv = logits ? 1.f / p.gate_norm : 0.f;
+                    float top = 0.f;
+#pragma unroll
+                    for (int rr = 0; rr < RPG; ++rr) {
+                        const int r = dir ? RPG - 1 - rr : rr;
+                        const F2 x = xr[dir][r].f2();
+                        const float gx = gate_log2<T>(f2_lo(x), p.gate_norm, inv, p.clamp_min), gy = gate_log2<T>(f2_hi(x), p.gate_norm, inv, p.clamp_min);
+                        if (r0 + r < n && (dir ? bwd : fwd)) { top = fmaxf(top, fmaxf(gx, gy)); run = f2_add(run, f2_make(gx, gy)); }
+                        G[dir][r] = run;
+                    }
+                    fine = fine && top <= 0.f;                            // growing gates: G is not monotone, its ends do not bound it
+                }
+                // across the warp's groups: what those scanned before mine contribute, and the warp's sum
+                const F2 mine = run;
+                F2 ahead = zero;
+#pragma unroll
+                for (int k = 1; k < SUB; ++k) {
+                    const int from = dir ? lane + k * PAIRS : lane - k * PAIRS;
+                    const F2 x = __shfl_sync(0xffffffffu, mine, from & 31);
+                    if (dir ? from < 32 : from >= 0) ahead = f2_add(ahead, x);
+                }
+                if constexpr (SUB > 1) {
+#pragma unroll
+                    for (int r = 0; r < RPG; ++r) G[dir][r] = f2_add(G[dir][r], ahead);
+                }
+                if (lane / PAIRS == (dir ? 0 : SUB - 1)) *reinterpret_cast<F2*>(gsum + (dir * W + w) * DK + 2 * pr) = f2_add(ahead, mine);
+            }
+        }
+        __syncthreads();
+        const int wm = nb / 2;                                           // the reference lies between the rows of warps wm - 1 and wm
+        const float lim = range_limit<T>();
+#pragma unroll
+        for (int dir = 0; dir < 2; ++dir) {
+            F2 run = f2_make(0.f, 0.f), before = run, lo = run, mine = run;
+#pragma unroll
+            for (int o = 0; o < W; ++o) {
+                const F2 x = *reinterpret_cast<const F2*>(gsum + (dir * W + o) * DK + 2 * pr);
+                if (o == w) { before = run; mine = x; }
+                if (o == wm) lo = run;
+                run = f2_add(run, x);
+            }
+            tot[dir] = run;
+            const F2 minus = f2_make(-1.f, -1.f);
+            const F2 off = dir ? f2_fma(f2_add(before, mine), minus, run) : before;        // what the warps scanned earlier contribute
+            ref[dir] = dir ? f2_fma(lo, minus, run) : lo;
+            const F2 rest = f2_fma(ref[dir], minus, run);
+            // gates are <= 0, so |G - ref| is largest at the segment's two ends
+            if (dir ? bwd : fwd) fine = fine && fabsf(f2_lo(ref[dir])) <= lim && fabsf(f2_hi(ref[dir])) <= lim && fabsf(f2_lo(rest)) <= lim && fabsf(f2_hi(rest)) <= lim;
+            if (gr == 0) {
+                float* sc = scl + dir * 2 * DK + 2 * pr;
+                *reinterpret_cast<float2*>(sc) = make_float2(ex2_t<T>(f2_lo(ref[dir])), ex2_t<T>(f2_hi(ref[dir])));
+                *reinterpret_cast<float2*>(sc + DK) = MODE == SEG_STATES ? make_float2(1.f, 1.f) : make_float2(ex2_t<T>(f2_lo(rest)), ex2_t<T>(f2_hi(rest)));
+                if (MODE != SEG_OUT && s.need_states && (dir ? bwd : fwd))
+                    *reinterpret_cast<float2*>(p.ws_decay + (((size_t)bh * s.nseg + c) * 2 + dir) * DK + 2 * pr) = make_float2(f2_lo(run) * tc::LN2, f2_hi(run) * tc::LN2);
+            }
+            if (!(dir ? bwd : fwd) || w >= nb) continue;
+            uint8_t* kt = smem + SM::K + dir * SM::QT + r0 * PK + pr * 4;
+            uint8_t* qt = smem + SM::Q + dir * SM::QT + r0 * PK + pr * 4;
+            const F2 shift = MODE == SEG_STATES ? f2_fma(run, minus, off) : f2_fma(ref[dir], minus, off);    // G - (total or reference)
+#pragma unroll
+            for (int r = 0; r < RPG; ++r) {
+                const F2 x = f2_add(G[dir][r], shift);
+                if (MODE == SEG_ONE) G[dir][r] = x;
+                uint32_t t[SC];
+                if (MODE != SEG_STATES) {
+                    scaled<T, SC>(qr[r], ex2_t<T>(f2_lo(x)), ex2_t<T>(f2_hi(x)), t);
+#pragma unroll
+                    for (int i = 0; i < SC; ++i) *reinterpret_cast<uint32_t*>(qt + i * TK + r * PK) = t[i];
+                }
+                scaled<T, SC>(kr[r], ex2_t<T>(-f2_lo(x)), ex2_t<T>(-f2_hi(x)), t);
+#pragma unroll
+                for (int i = 0; i < SC; ++i) *reinterpret_cast<uint32_t*>(kt + i * TK + r * PK) = t[i];
+            }
+        }
+    }
+    if (RAW == 1) asm volatile("cp.async.wait_all;" ::: "memory");
+    const bool bad = __syncthreads_or(!fine && MODE != SEG_STATES);
+    if (bad && MODE == SEG_ONE && s.need_states) {                       // the contribution from tiles whose exponents are all <= 0
+        const F2 minus = f2_make(-1.f, -1.f);
+#pragma unroll
+        for (int dir = 0; dir < 2; ++dir) {
+            if (gr == 0) *reinterpret_cast<float2*>(scl + dir * 2 * DK + DK + 2 * pr) = make_float2(1.f, 1.f);
+            if (w >= nb) continue;
+            const F2 rest = f2_fma(ref[dir], minus, tot[dir]);           // G holds G - ref
+#pragma unroll
+            for (int r = 0; r < RPG; ++r) {
+                const F2 x = f2_fma(G[dir][r], minus, rest);
+                uint32_t t[SC];
+                scaled<T, SC>(kr[r], ex2_t<T>(f2_lo(x)), ex2_t<T>(f2_hi(x)), t);
+#pragma unroll
+                for (int i = 0; i < SC; ++i) *reinterpret_cast<uint32_t*>(smem + SM::K + dir * SM::QT + i * TK + (r0 + r) * PK + pr * 4) = t[i];
+            }
+        }
+        __syncthreads();
+    }
+    if (MODE != SEG_OUT && s.need_states) {                              // ---- contributions: units of 16 key channels x NC value columns of one direction
+        constexpr int UNITS = 2 * MT, NSPLIT = W <= UNITS ? 1 : W / UNITS < DV / 8 ? W / UNITS : DV / 8, NC = DV / NSPLIT, NTL = NC / 8;
+        for (int u = w; u < UNITS * NSPLIT; u += W) {
+            const int dir = u / (MT * NSPLIT), mt = (u / NSPLIT) % MT, ns = u % NSPLIT;
+            if (!(dir ? bwd : fwd)) continue;
+            float acc[NTL][4];
+#pragma unroll
+            for (int i = 0; i < NTL; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+            const uint32_t x = sb + SM::K + dir * SM::QT + mt * 32 + frag_cols<PK>(lane), y = sb + SM::V + ns * NC * 2 + frag_rows<PV>(lane);
+#pragma unroll 2
+            for (int ks = 0; ks < nb; ++ks) {
+                uint32_t a[SC][4];
+#pragma unroll
+                for (int t = 0; t < SC; ++t) ldsm4t(x + t * TK + ks * 16 * PK, a[t]);
+                block_nn<NC, SC, RAW>(acc, a, y + ks * 16 * PV, TV);
+            }
+            const float* sc = scl + dir * 2 * DK + DK + mt * 16 + (lane >> 2);
+            const float s0 = sc[0], s1 = sc[8];
+            float* out = p.ws_state + (((size_t)bh * s.nseg + c) * 2 + dir) * DK * DV + (mt * 16 + (lane >> 2)) * DV + ns * NC + 2 * (lane & 3);
+#pragma unroll
+            for (int i = 0; i < NTL; ++i) {
+                *reinterpret_cast<float2*>(out + i * 8) = make_float2(acc[i][0] * s0, acc[i][1] * s0);
+                *reinterpret_cast<float2*>(out + 8 * DV + i * 8) = make_float2(acc[i][2] * s1, acc[i][3] * s1);
+            }
+        }
+        if (MODE == SEG_STATES) return;
+        if (s.nseg > 1) cluster_arrive();
+    }
+    float o[DV / 8][4];
+#pragma unroll
+    for (int i = 0; i < DV / 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[i][j] = 0.f;
+    const uint32_t aQ = sb + SM::Q + 16 * w * PK + frag_rows<PK>(lane);
+    if (want_out && !bad && w < nb) {                                    // ---- products inside the segment, my 16 rows
+        const uint32_t bK = sb + SM::K + frag_cols<PK>(lane), tV = sb + SM::V + frag_rows<PV>(lane);
+        uint32_t ap[SC][4];
+#pragma unroll 1
+        for (int dir = 0; dir < 2; ++dir) {                              // off-diagonal blocks: before mine with the forward tiles, after it with the backward ones
+            if (!(dir ? bwd : fwd)) continue;
+            const uint32_t q = aQ + dir * SM::QT, k = bK + dir * SM::QT;
+            uint32_t fq[DK / 16][SC][4];
+#pragma unroll
+            for (int ks = 0; ks < DK / 16; ++ks)
+#pragma unroll
+                for (int t = 0; t < SC; ++t) ldsm4(q + t * TK + ks * 32, fq[ks][t]);
+            const int j1 = dir ? nb : w;
+#pragma unroll 1
+            for (int jb = dir ? w + 1 : 0; jb < j1; jb += 2) {           // two blocks at a time: four independent chains of products
+                const bool two = jb + 1 < j1;
+                float pb[4][4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) pb[i][j] = 0.f;
+#pragma unroll
+                for (int ks = 0; ks < DK / 16; ++ks) {
+                    uint32_t bf[4][SC][2];
+                    if (two) {
+                        load_b_nt<SC, 4, PK>(bf, k + jb * 16 * PK + ks * 32, TK);
+                        mma_group<SC, SC, 4>(pb, fq[ks], bf);
+                    } else {
+                        load_b_nt<SC, 2, PK>(bf, k + jb * 16 * PK + ks * 32, TK);
+                        mma_group<SC, SC, 2>(pb, fq[ks], bf);
+                    }
+                }
+                mask_split<SC>(pb, false, lane, [](int, int) { return true; }, ap);
+                block_nn<DV, SC, RAW>(o, ap, tV + jb * 16 * PV, TV);
+                if (two) {
+                    mask_split<SC>(pb + 2, false, lane, [](int, int) { return true; }, ap);
+                    block_nn<DV, SC, RAW>(o, ap, tV + (jb + 1) * 16 * PV, TV);
+                }
+            }
+        }
+        float pd[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+        for (int dir = 0; dir < 2; ++dir) {                              // the diagonal block: both directions' halves, a token sees itself in each
+            if (!(dir ? bwd : fwd)) continue;
+            float pb[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+            block_nt<DK, SC, SC>(pb, aQ + dir * SM::QT, TK, bK + dir * SM::QT + w * 16 * PK, TK);
+            const int r = lane >> 2, q = 2 * (lane & 3);
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int row = r + 8 * (j >> 1), col = nt * 8 + q + (j & 1);
+                    if (dir ? col >= row : col <= row) pd[nt][j] += pb[nt][j];
+                }
+        }
+        mask_split<SC>(pd, false, lane, [](int, int) { return true; }, ap);
+        block_nn<DV, SC, RAW>(o, ap, tV + w * 16 * PV, TV);
+    }
+    const bool has_init = MODE == SEG_ONE && (p.init_f || p.init_b);
+    if (MODE == SEG_ONE && s.nseg > 1) cluster_wait();                   // the other segments' contributions have landed
+    else __syncthreads();
+    if (MODE == SEG_ONE && s.need_states) {
+#pragma unroll 1
+        for (int dir = 0; dir < 2; ++dir) {                              // final states, summed log-gates: by the segment scanned last
+            float* fin = dir ? p.final_b : p.final_f;
+            float* ld = dir ? p.logdecay_b : p.logdecay_f;
+            if (!(dir ? bwd : fwd) || (!fin && !ld) || c != (dir ? 0 : s.nseg - 1)) continue;
+            const size_t slot = ((size_t)bh * s.nseg + c) * 2 + dir;
+            for (int i = threadIdx.x; i < DK * DV / 4; i += NTH) {
+                const int d = i * 4 / DV;
+                if (fin) {
+                    float4 S = entering<DK, DV, MODE>(s, bh, c, dir, i);
+                    const float4 u = __ldcg(reinterpret_cast<const float4*>(p.ws_state) + slot * (DK * DV / 4) + i);
+                    const float a = __expf(__ldcg(p.ws_decay + slot * DK + d));
+                    S.x = fmaf(S.x, a, u.x); S.y = fmaf(S.y, a, u.y); S.z = fmaf(S.z, a, u.z); S.w = fmaf(S.w, a, u.w);
+                    reinterpret_cast<float4*>(fin)[(size_t)bh * (DK * DV / 4) + i] = S;
+                }
+                if (ld && i * 4 % DV == 0) {
+                    float g = 0.f;
+                    for (int k = 0; k < s.nseg; ++k) g += __ldcg(p.ws_decay + (((size_t)bh * s.nseg + k) * 2 + dir) * DK + d);
+                    ld[(size_t)bh * DK + d] = g;
+                }
+            }
+        }
+    }
+    if (!want_out) return;
+    if (bad) {
+        exact_segment<DK, DV, T, MODE>(s, reinterpret_cast<float*>(smem), bh, c, n);
+        return;
+    }
+    if (MODE == SEG_OUT || s.nseg > 1 || has_init) {                     // ---- entering states, scaled, over the K tiles
+        if (MODE == SEG_ONE && s.nseg > 1) __syncthreads();              // all warps are past their products (they arrived at the cluster barrier before them)
+#pragma unroll 1
+        for (int dir = 0; dir < 2; ++dir) {
+            if (!(dir ? bwd : fwd)) continue;
+            // KB states of four values per thread and pass, the contributions of two segments in flight for all of them: a
+            // chain of dependent loads per state took as long as everything else in the kernel
+            constexpr int KN = (DK * DV / 4 + NTH - 1) / NTH, KB = KN < 4 ? KN : 4;
+            const int m = MODE == SEG_OUT ? 0 : dir ? s.nseg - 1 - c : c;
+            const float* init = dir ? p.init_b : p.init_f;
+#pragma unroll 1
+            for (int k0 = 0; k0 < KN; k0 += KB) {
+                float4 S[KB];
+                const int i0 = threadIdx.x + k0 * NTH;
+                if (DK * DV / 4 < NTH && i0 >= DK * DV / 4) break;
+#pragma unroll
+                for (int k = 0; k < KB; ++k) {
+                    const int i = i0 + k * NTH;
+                    S[k] = MODE == SEG_OUT ? __ldcg(reinterpret_cast<const float4*>(p.ws_state) + (((size_t)bh * s.nseg + c) * 2 + dir) * (DK * DV / 4) + i)
+                           : init ? __ldg(reinterpret_cast<const float4*>(init) + (size_t)bh * (DK * DV / 4) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll 2
+                for (int g = 0; g < m; ++g) {
+                    const size_t from = ((size_t)bh * s.nseg + (dir ? s.nseg - 1 - g : g)) * 2 + dir;
+                    float4 u[KB];
+                    float a[KB];
+#pragma unroll
+                    for (int k = 0; k < KB; ++k) {
+                        u[k] = __ldcg(reinterpret_cast<const float4*>(p.ws_state) + from * (DK * DV / 4) + i0 + k * NTH);
+                        a[k] = __ldcg(p.ws_decay + from * DK + (i0 + k * NTH) * 4 / DV);
+                    }
+#pragma unroll
+                    for (int k = 0; k < KB; ++k) {
+                        const float e = __expf(a[k]);
+                        S[k].x = fmaf(S[k].x, e, u[k].x); S[k].y = fmaf(S[k].y, e, u[k].y); S[k].z = fmaf(S[k].z, e, u[k].z); S[k].w = fmaf(S[k].w, e, u[k].w);
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < KB; ++k) {
+                    const int i = i0 + k * NTH, d = i * 4 / DV, v = i % (DV / 4);
+                    const float a = scl[dir * 2 * DK + d];
+                    uint32_t ta[SC], tb[SC];
+                    split2<SC>(S[k].x * a, S[k].y * a, ta); split2<SC>(S[k].z * a, S[k].w * a, tb);
+#pragma unroll
+                    for (int t = 0; t < SC; ++t) *reinterpret_cast<uint2*>(smem + SM::K + dir * SM::QT + t * TS + d * PV + v * 8) = make_uint2(ta[t], tb[t]);
+                }
+            }
+        }
+        __syncthreads();
+        if (w < nb) {
+#pragma unroll 1
+            for (int dir = 0; dir < 2; ++dir) {
+                if (!(dir ? bwd : fwd)) continue;
+                const uint32_t tS = sb + SM::K + dir * SM::QT + frag_rows<PV>(lane);
+#pragma unroll
+                for (int ks = 0; ks < DK / 16; ++ks) {
+                    uint32_t fa[SC][4];
+#pragma unroll
+                    for (int t = 0; t < SC; ++t) ldsm4(aQ + dir * SM::QT + t * TK + ks * 32, fa[t]);
+                    block_nn<DV, SC, SC>(o, fa, tS + ks * 16 * PV, TS);
+                }
+            }
+        }
+    }
+    if (w >= nb) return;
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) {
+        const int row = 16 * w + (lane >> 2) + 8 * hf;
+        if (row >= n) continue;
+        T* out = reinterpret_cast<T*>(p.o) + b * p.so[0] + h * p.so[1] + (t0 + row) * p.so[2] + 2 * (lane & 3);
+#pragma unroll
+        for (int i = 0; i < DV / 8; ++i) store2<T>(out + 8 * i, p.qscale * o[i][2 * hf], p.qscale * o[i][2 * hf + 1]);
+    }
+}
+
+template <int DK, int DV, typename T, int TOK, int MODE>
+int seg_launch_mode(const SegParams& s, cudaStream_t stream) {
+    auto kern = bigla_seg_kernel<DK, DV, T, TOK, MODE>;
+    constexpr uint32_t smem = SegSmem<DK, DV, T, TOK>::BYTES;
+    cudaError_t e = tc::ensure_smem_attr(reinterpret_cast<const void*>(kern), (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(s.nseg, s.p.B * s.p.H);
+    cfg.blockDim = dim3(2 * TOK);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = s.nseg; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = MODE == SEG_ONE && s.nseg > 1 ? 1 : 0;
+    e = cudaLaunchKernelEx(&cfg, kern, s);
+    return (int)(e != cudaSuccess ? e : cudaGetLastError());
+}
+
+template <int DK, int DV, typename T, int TOK>
+int seg_launch(SegParams& s, cudaStream_t stream) {
+    constexpr int CLUSTER = 8;                           // largest portable cluster
+    BiglaParams& p = s.p;
+    s.nseg = (p.L + TOK - 1) / TOK;
+    s.seglen = ((p.L + s.nseg - 1) / s.nseg + 15) / 16 * 16;   // even segments: no nearly empty last one
+    s.nseg = (p.L + s.seglen - 1) / s.seglen;
+    const bool finals = p.final_f || p.final_b || p.logdecay_f || p.logdecay_b;
+    s.need_states = s.nseg > 1 || finals;
+    p.nchunk = s.nseg;
+    p.ws_decay = p.ws_state ? p.ws_state + (size_t)p.B * p.H * s.nseg * 2 * DK * DV : nullptr;
+    if (s.nseg <= CLUSTER) return seg_launch_mode<DK, DV, T, TOK, SEG_ONE>(s, stream);
+    if (int e = seg_launch_mode<DK, DV, T, TOK, SEG_STATES>(s, stream)) return e;
+    if (int e = bigla_scan_launch(p, stream)) return e;
+    return p.o ? seg_launch_mode<DK, DV, T, TOK, SEG_OUT>(s, stream) : 0;
+}
+
+template <int DK, int DV, typename T>
+int seg_launch_tok(SegParams& s, int tok, cudaStream_t stream) {
+    if constexpr (sizeof(T) == 4) return seg_launch<DK, DV, T, 64>(s, stream);
+    else if constexpr (DV == 32) return seg_launch<DK, DV, T, 64>(s, stream);
+    else return tok == 64 ? seg_launch<DK, DV, T, 64>(s, stream) : seg_launch<DK, DV, T, 128>(s, stream);
+}
+
+template <typename T>
+int seg_launch_dims(SegParams& s, int tok, cudaStream_t stream) {
+#define VIG_CASE(DKV, DVV) if (s.p.dk == DKV && s.p.dv == DVV) return seg_launch_tok<DKV, DVV, T>(s, tok, stream);
+    VIG_CASE(16, 32) VIG_CASE(32, 32) VIG_CASE(32, 64) VIG_CASE(64, 64)
+#undef VIG_CASE
+    return VIG_ERR_SHAPE;
+}
+
+}  // namespace
+
+// Rows are read as pairs of values and (16-bit v) 16-byte vectors: base pointers on 16 bytes, strides multiples of 16 bytes.
+// grid.y holds B*H, hence its limit.  Everything else stays with the other forms.
+bool bigla_seg_supported(const BiglaParams& p) {
+    if (!((p.dk == 16 && p.dv == 32) || (p.dk == 32 && p.dv == 32) || (p.dk == 32 && p.dv == 64) || (p.dk == 64 && p.dv == 64))) return false;
+    if ((int64_t)p.B * p.H > 65535) return false;
+    const int unit = p.dtype == VIG_DTYPE_F32 ? 4 : 8;
+    auto ok = [&](const void* base, const int64_t* s) {
+        return !base || (!(reinterpret_cast<uintptr_t>(base) & 15) && s[0] % unit == 0 && s[1] % unit == 0 && s[2] % unit == 0);
+    };
+    auto ok16 = [](const void* x) { return !(reinterpret_cast<uintptr_t>(x) & 15); };
+    return ok(p.q, p.sq) && ok(p.k, p.sk) && ok(p.v, p.sv) && ok(p.gf, p.sgf) && ok(p.gb, p.sgb) && ok(p.o, p.so) && ok16(p.init_f) && ok16(p.init_b) &&
+           ok16(p.final_f) && ok16(p.final_b);
+}
+
+// Against the tcgen05 forms (16-bit, dv = 64), by the number of 128-token segments in the call; microseconds here / the
+// better of theirs at B x H x L:
+//   bf16 dk = 64: 1x3x196 11 / 16, 5x6x450 14 / 22, 8x3x1024 21 / 35, 8x3x4096 85 / 79, 128x6x196 90 / 76
+//   bf16 dk = 32: 1x3x196 8 / 16, 8x3x1024 15 / 31, 6x12x999 39 / 45, 128x6x196 64 / 68, 32x3x3136 150 / 125, 1x3x16384 49 / 54
+//   fp16 (two operand terms): dk = 32 3x3x836 15 / 30, dk = 64 4x12x1000 80 / 41
+// Small calls are bound by the latency of one segment, where this form is two to three times shorter; large ones by
+// instruction issue, where the persistent forms overlap their phases better.
+bool bigla_seg_preferred(const BiglaParams& p) {
+    if (p.dtype == VIG_DTYPE_F32 || p.dv != 64) return true;
+    const int64_t segs = (int64_t)p.B * p.H * ((p.L + 127) / 128);
+    if (p.dtype == VIG_DTYPE_F16) return segs <= (p.dk == 32 ? 200 : 120);
+    return segs <= (p.dk == 32 ? (p.L <= 256 ? 1600 : p.L <= 1024 ? 600 : 400) : p.L <= 1024 ? 400 : 200);
+}
+
+int bigla_seg_launch(const BiglaParams& p, cudaStream_t stream) {
+    SegParams s{};
+    s.p = p;
+    // 64-token segments where more SMs can share the work of few sequences (1x3x196 dk = 64: 11 us against 13) and for dv = 32,
+    // whose segments are too little work for eight warps (64x12x196 dk = 16: 47 us against 57); otherwise 128, half as many states
+    const int tok = p.dv == 32 || p.L <= 64 || (p.L <= 512 && (int64_t)p.B * p.H * ((p.L + 63) / 64) <= 148) ? 64 : 128;
+    switch (p.dtype) {
+        case VIG_DTYPE_F32: return seg_launch_dims<float>(s, 64, stream);
+        case VIG_DTYPE_BF16: return seg_launch_dims<__nv_bfloat16>(s, tok, stream);
+        case VIG_DTYPE_F16: return seg_launch_dims<__half>(s, tok, stream);
+    }
+    return VIG_ERR_DTYPE;
+}
+
+}  // namespace vig

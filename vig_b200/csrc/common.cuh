@@ -88,9 +88,10 @@ __device__ __forceinline__ float gate_transform(float x, float gate_norm, float 
 
 int bigla_simt_launch(const BiglaParams& p, cudaStream_t stream);
 size_t bigla_simt_workspace(int B, int H, int L, int dk, int dv);
-// chunked tensor-core form at full operand precision (fp32, and 16-bit heads with dv = 32)
-bool bigla_mma_supported(const BiglaParams& p);
-int bigla_mma_launch(const BiglaParams& p, cudaStream_t stream);
+// mma.sync form, both directions of a segment in one sweep (short and medium sequences, dv = 32, fp32)
+bool bigla_seg_supported(const BiglaParams& p);
+bool bigla_seg_preferred(const BiglaParams& p);
+int bigla_seg_launch(const BiglaParams& p, cudaStream_t stream);
 // scan over p.nchunk per-chunk (or per-segment) local states in the workspace, in place (phase B)
 int bigla_scan_launch(const BiglaParams& p, cudaStream_t stream);
 int bigla_tc_launch(const BiglaParams& p, void* ws, size_t ws_bytes, bool allow_fused, cudaStream_t stream);

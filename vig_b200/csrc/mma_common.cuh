@@ -36,7 +36,7 @@ __device__ __forceinline__ void ldsm2t(uint32_t addr, uint32_t* r) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
 }
 __device__ __forceinline__ void mma16816(float* c, const uint32_t* a, const uint32_t* b) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
@@ -60,15 +60,19 @@ template <int NTERM> __device__ __forceinline__ void split2(float a, float b, ui
     }
 }
 
-// c += a b over one k step, all term pairs of order < max(NA, NB); a[term][4], b[term][2]
-template <int NA, int NB> __device__ __forceinline__ void mma_terms(float* c, const uint32_t (*a)[4], const uint32_t (*b)[2]) {
+// c[g] += a b[g] over one k step for G accumulators, all term pairs of order < max(NA, NB); a[term][4], b[g][term][2].  The
+// accumulators alternate, so that a chain of dependent products never waits for its own latency.
+template <int NA, int NB, int G> __device__ __forceinline__ void mma_group(float (*c)[4], const uint32_t (*a)[4], const uint32_t (*b)[NB][2]) {
     constexpr int ORD = NA > NB ? NA : NB;
 #pragma unroll
     for (int o = ORD - 1; o >= 0; --o)               // small terms first
 #pragma unroll
         for (int i = 0; i < NA; ++i) {
             const int j = o - i;
-            if (j >= 0 && j < NB) mma16816(c, a[i], b[j]);
+            if (j >= 0 && j < NB) {
+#pragma unroll
+                for (int g = 0; g < G; ++g) mma16816(c[g], a[i], b[g][j]);
+            }
         }
 }
 
@@ -185,9 +189,39 @@ template <typename T> __device__ __forceinline__ const T* head_ptr(const void* b
     return reinterpret_cast<const T*>(base) + b * s[0] + h * s[1] + t0 * s[2];
 }
 
+// B operands of G neighbouring n tiles (8 columns each) of one k step: [k][n] tile (trans) or [n][k] tile of pitch PB
+template <int NB, int G> __device__ __forceinline__ void load_b_nn(uint32_t (*b)[NB][2], uint32_t at, uint32_t b_term) {
+    if constexpr (G == 1) {
+#pragma unroll
+        for (int t = 0; t < NB; ++t) ldsm2t(at + t * b_term, b[0][t]);
+    } else {
+#pragma unroll
+        for (int n = 0; n < G; n += 2)
+#pragma unroll
+            for (int t = 0; t < NB; ++t) {
+                uint32_t r[4];
+                ldsm4t(at + t * b_term + n * 16, r);
+                b[n][t][0] = r[0]; b[n][t][1] = r[1]; b[n + 1][t][0] = r[2]; b[n + 1][t][1] = r[3];
+            }
+    }
+}
+template <int NB, int G, uint32_t PB> __device__ __forceinline__ void load_b_nt(uint32_t (*b)[NB][2], uint32_t at, uint32_t b_term) {
+#pragma unroll
+    for (int n = 0; n < G; n += 2)
+#pragma unroll
+        for (int t = 0; t < NB; ++t) {
+            uint32_t r[4];
+            ldsm4(at + t * b_term + n * 8 * PB, r);
+            b[n][t][0] = r[0]; b[n][t][1] = r[1]; b[n + 1][t][0] = r[2]; b[n + 1][t][1] = r[3];
+        }
+}
+// n tiles handled together: four, where there are four
+template <int TILES> struct Group { static constexpr int G = TILES < 4 ? TILES : 4; static_assert(TILES % G == 0, "tiles"); };
+
 // acc[NTILES][4] += X^T Y: X [C tokens][DK] scaled tiles (my 16 rows of X^T at column byte offset), Y [C][DV] raw tiles
 template <int DK, int DV, int NA, int NB, int NTILES> __device__ __forceinline__ void state_mma(float (*acc)[4], uint32_t x, uint32_t y, int lane) {
     constexpr uint32_t PX = Pitch<DK>::B, PY = Pitch<DV>::B;
+    constexpr int G = Group<NTILES>::G;
     x += frag_cols<PX>(lane);
     y += frag_rows<PY>(lane);
 #pragma unroll
@@ -195,24 +229,11 @@ template <int DK, int DV, int NA, int NB, int NTILES> __device__ __forceinline__
         uint32_t a[NA][4];
 #pragma unroll
         for (int t = 0; t < NA; ++t) ldsm4t(x + t * C * PX + ks * 16 * PX, a[t]);
-        if constexpr (NTILES == 1) {
-            uint32_t b[NB][2];
 #pragma unroll
-            for (int t = 0; t < NB; ++t) ldsm2t(y + t * C * PY + ks * 16 * PY, b[t]);
-            mma_terms<NA, NB>(acc[0], a, b);
-        } else {
-#pragma unroll
-            for (int n = 0; n < NTILES; n += 2) {
-                uint32_t b0[NB][2], b1[NB][2];
-#pragma unroll
-                for (int t = 0; t < NB; ++t) {
-                    uint32_t r[4];
-                    ldsm4t(y + t * C * PY + ks * 16 * PY + n * 16, r);
-                    b0[t][0] = r[0]; b0[t][1] = r[1]; b1[t][0] = r[2]; b1[t][1] = r[3];
-                }
-                mma_terms<NA, NB>(acc[n], a, b0);
-                mma_terms<NA, NB>(acc[n + 1], a, b1);
-            }
+        for (int n = 0; n < NTILES; n += G) {
+            uint32_t b[G][NB][2];
+            load_b_nn<NB, G>(b, y + ks * 16 * PY + n * 16, C * PY);
+            mma_group<NA, NB, G>(acc + n, a, b);
         }
     }
 }
@@ -240,21 +261,15 @@ template <int DK, int DV, int SC> __device__ __forceinline__ void load_state(uin
     }
 }
 
-// acc[2][4] += A_rows B_rows^T over KD: A fragments of my 16 rows (tile a, [row][k]), B rows jb*16.. (tile b, [n][k])
+// acc[2][4] += A_rows B_rows^T over KD: A fragments of my 16 rows (tile a, [row][k]), 16 B rows (tile b, [n][k], pitch PB)
 template <int KD, int NA, int NB> __device__ __forceinline__ void block_nt(float (*acc)[4], uint32_t a, uint32_t a_term, uint32_t b, uint32_t b_term) {
 #pragma unroll
     for (int ks = 0; ks < KD / 16; ++ks) {
-        uint32_t fa[NA][4], b0[NB][2], b1[NB][2];
+        uint32_t fa[NA][4], fb[2][NB][2];
 #pragma unroll
         for (int t = 0; t < NA; ++t) ldsm4(a + t * a_term + ks * 32, fa[t]);
-#pragma unroll
-        for (int t = 0; t < NB; ++t) {
-            uint32_t r[4];
-            ldsm4(b + t * b_term + ks * 32, r);
-            b0[t][0] = r[0]; b0[t][1] = r[1]; b1[t][0] = r[2]; b1[t][1] = r[3];
-        }
-        mma_terms<NA, NB>(acc[0], fa, b0);
-        mma_terms<NA, NB>(acc[1], fa, b1);
+        load_b_nt<NB, 2, 0>(fb, b + ks * 32, b_term);
+        mma_group<NA, NB, 2>(acc, fa, fb);
     }
 }
 
@@ -284,38 +299,28 @@ template <int SC, typename F> __device__ __forceinline__ void mask_split(float (
 
 // acc[ND/8][4] += A (16 x 16, registers) B: B rows of one k step in a [k][n] tile
 template <int ND, int NA, int NB> __device__ __forceinline__ void block_nn(float (*acc)[4], const uint32_t (*a)[4], uint32_t b, uint32_t b_term) {
+    constexpr int G = Group<ND / 8>::G;
 #pragma unroll
-    for (int n = 0; n < ND / 8; n += 2) {
-        uint32_t b0[NB][2], b1[NB][2];
-#pragma unroll
-        for (int t = 0; t < NB; ++t) {
-            uint32_t r[4];
-            ldsm4t(b + t * b_term + n * 16, r);
-            b0[t][0] = r[0]; b0[t][1] = r[1]; b1[t][0] = r[2]; b1[t][1] = r[3];
-        }
-        mma_terms<NA, NB>(acc[n], a, b0);
-        mma_terms<NA, NB>(acc[n + 1], a, b1);
+    for (int n = 0; n < ND / 8; n += G) {
+        uint32_t fb[G][NB][2];
+        load_b_nn<NB, G>(fb, b + n * 16, b_term);
+        mma_group<NA, NB, G>(acc + n, a, fb);
     }
 }
 
 // acc[ND/8][4] += A B^T over KD: A = my 16 rows of an [m][k] tile, B an [n][k] tile of ND rows with pitch PB
 template <int ND, int KD, uint32_t PB, int NA, int NB> __device__ __forceinline__ void rows_nt(float (*acc)[4], uint32_t a, uint32_t a_term, uint32_t b, uint32_t b_term) {
+    constexpr int G = Group<ND / 8>::G;
 #pragma unroll
     for (int ks = 0; ks < KD / 16; ++ks) {
         uint32_t fa[NA][4];
 #pragma unroll
         for (int t = 0; t < NA; ++t) ldsm4(a + t * a_term + ks * 32, fa[t]);
 #pragma unroll
-        for (int n = 0; n < ND / 8; n += 2) {
-            uint32_t b0[NB][2], b1[NB][2];
-#pragma unroll
-            for (int t = 0; t < NB; ++t) {
-                uint32_t r[4];
-                ldsm4(b + t * b_term + n * 8 * PB + ks * 32, r);
-                b0[t][0] = r[0]; b0[t][1] = r[1]; b1[t][0] = r[2]; b1[t][1] = r[3];
-            }
-            mma_terms<NA, NB>(acc[n], fa, b0);
-            mma_terms<NA, NB>(acc[n + 1], fa, b1);
+        for (int n = 0; n < ND / 8; n += G) {
+            uint32_t fb[G][NB][2];
+            load_b_nt<NB, G, PB>(fb, b + n * 8 * PB + ks * 32, b_term);
+            mma_group<NA, NB, G>(acc + n, fa, fb);
         }
     }
 }
