@@ -54,3 +54,29 @@ def test_plan_follows_the_model():
         assert native.vig_forward(m, x) is None
     outs = [a, b, c, d]
     assert all(not torch.equal(outs[i], outs[i + 1]) for i in range(3))
+
+
+def test_small_forwards_are_replayed_and_stay_independent():
+    """From the second call of a shape a small forward is a replayed graph: results of earlier calls stay what they were, other
+    shapes, strides and streams get their own, and a changed weight reaches the next call."""
+    from vig_b200 import native
+    m = _model("vig_t", torch.bfloat16)
+    xs = [torch.randn(1, 3, 64, 64, device="cuda").bfloat16() for _ in range(3)]
+    wide = torch.randn(2, 3, 64, 96, device="cuda").bfloat16()
+    with torch.no_grad():
+        ref = []
+        for x in (*xs, wide):
+            native._plans.clear()
+            ref.append(m(x))                                            # first call of a plan: launched one by one
+        for _ in range(3):
+            got = [m(x) for x in (*xs, wide)]
+            assert all(torch.equal(a, b) for a, b in zip(got, ref))
+        assert torch.equal(m(xs[0].contiguous(memory_format=torch.channels_last)), ref[0])
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            outs = [m(xs[i % 3]) for i in range(6)]
+        torch.cuda.current_stream().wait_stream(side)
+        assert all(torch.equal(o, ref[i % 3]) for i, o in enumerate(outs))
+        m.head.bias.add_(1.0)
+        assert torch.equal(m(xs[0]), m(xs[0])) and not torch.equal(m(xs[0]), ref[0])

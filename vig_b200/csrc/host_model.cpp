@@ -8,7 +8,10 @@
 // modules themselves.  The check is some hundred pointer comparisons.
 #include "host.h"
 #include <cuda_runtime_api.h>
+#include <unordered_map>
 #include <ATen/autocast_mode.h>
+#include <ATen/cuda/CUDAEvent.h>
+#include <ATen/cuda/CUDAGraph.h>
 #include <ATen/ops/empty.h>
 
 namespace vig_host {
@@ -167,7 +170,75 @@ struct PlanBase {
                !(at::GradMode::is_enabled()) && !at::autocast::is_autocast_enabled(at::kCUDA) && status_known(device.index()) && watch.same();
     }
     Tensor finish(const Tensor& pooled) const { return at::linear(pooled, head_w, head_b.defined() ? OptT(head_b) : std::nullopt); }
-    template <typename F> OptT run(const Tensor& x, F body) const {
+    // One forward.  ``work``: a measure of the activations (tokens x channels).  Small forwards are bound by their launches, on
+    // the host (5 - 10 us each through the GEMM library) and on the device (1.4 us between kernels): from the second call of a
+    // shape on a stream they are captured into a CUDA graph and replayed, with the images copied into the graph's input.  The
+    // graph and its memory (about 24 bytes per activation element, GRAPH_WORK elements in all per plan) belong to this plan, one
+    // per shape and stream, the least recently used given back first, and go with it.
+    static constexpr int64_t GRAPH_WORK = 8 << 20;
+    struct Captured {
+        int64_t B, H, W, work;
+        cudaStream_t stream;
+        int seen;
+        bool failed;
+        uint64_t used;
+        std::unique_ptr<at::cuda::CUDAGraph> graph;
+        std::unique_ptr<at::cuda::CUDAEvent> done;       // behind the last replay: the graph's memory is not given back before
+        Tensor in, out;
+        Captured(const Tensor& x, int64_t work, cudaStream_t st, uint64_t now)
+            : B(x.size(0)), H(x.size(2)), W(x.size(3)), work(work), stream(st), seen(0), failed(false), used(now) {}
+        Captured(Captured&&) = default;
+        Captured& operator=(Captured&& o) { std::swap(B, o.B); std::swap(H, o.H); std::swap(W, o.W); std::swap(work, o.work); std::swap(stream, o.stream);
+            std::swap(seen, o.seen); std::swap(failed, o.failed); std::swap(used, o.used); std::swap(graph, o.graph); std::swap(done, o.done);
+            std::swap(in, o.in); std::swap(out, o.out); return *this; }
+        ~Captured() {
+            if (done) { try { done->synchronize(); } catch (...) {} }
+        }
+    };
+    std::vector<Captured> captured;
+    uint64_t clock = 0;
+
+    Captured& entry(const Tensor& x, cudaStream_t st, int64_t work) {
+        for (Captured& e : captured)
+            if (e.B == x.size(0) && e.H == x.size(2) && e.W == x.size(3) && e.stream == st) { e.used = ++clock; return e; }
+        int64_t held = work;
+        for (const Captured& e : captured) held += e.work;
+        while (!captured.empty() && (held > GRAPH_WORK || captured.size() >= 8)) {
+            size_t oldest = 0;
+            for (size_t i = 1; i < captured.size(); ++i) if (captured[i].used < captured[oldest].used) oldest = i;
+            held -= captured[oldest].work;
+            captured.erase(captured.begin() + oldest);
+        }
+        captured.emplace_back(x, work, st, ++clock);
+        return captured.back();
+    }
+    template <typename F> void capture(Captured& e, const Tensor& x, F body, const Ctx& c) {
+        // one capture stream per device; a GEMM on it beforehand, so that the library's workspace for it is an ordinary allocation
+        static std::unordered_map<int, at::cuda::CUDAStream>* streams = new std::unordered_map<int, at::cuda::CUDAStream>();
+        auto it = streams->find(device.index());
+        const bool fresh = it == streams->end();
+        if (fresh) it = streams->emplace(device.index(), at::cuda::getStreamFromPool(false, device.index())).first;
+        e.in = at::empty(x.sizes(), x.options());
+        c10::cuda::CUDAStreamGuard guard(it->second);
+        if (fresh) {
+            const Tensor a = at::zeros({16, 64}, x.options()), b = at::zeros({64}, x.options());
+            at::linear(a, at::zeros({64, 64}, x.options()), b);
+            at::linear(a, at::zeros({64, 64}, x.options()));
+        }
+        auto g = std::make_unique<at::cuda::CUDAGraph>();
+        g->capture_begin({0, 0}, cudaStreamCaptureModeThreadLocal);
+        try {
+            e.out = body(Ctx{it->second.stream(), c.status, c.code}, e.in);
+        } catch (...) {
+            e.failed = true;
+        }
+        try { g->capture_end(); } catch (...) { e.failed = true; }
+        if (e.failed) { e.in = e.out = Tensor(); return; }
+        e.graph = std::move(g);
+        e.done = std::make_unique<at::cuda::CUDAEvent>();
+    }
+
+    template <typename F> OptT run(const Tensor& x, int64_t work, F body) {
         if (!takes(x)) return std::nullopt;
         c10::cuda::CUDAGuard guard(device);
         at::NoGradGuard ng;
@@ -178,7 +249,18 @@ struct PlanBase {
         StatusPeek& peek = StatusPeek::of(device.index());
         if (const int v = peek.poll(capturing)) { on_status(v); }
         const Ctx c{st.stream(), status_ptr(device.index()), type == at::kBFloat16 ? VIG_DTYPE_BF16 : VIG_DTYPE_F16};
-        Tensor y = body(c, x.contiguous());
+        Tensor y;
+        if (!capturing && work <= GRAPH_WORK) {
+            Captured& e = entry(x, st.stream(), work);
+            if (!e.graph && !e.failed && e.seen++ > 0) capture(e, x, body, c);
+            if (e.graph) {
+                e.in.copy_(x, true);
+                e.graph->replay();
+                y = e.out.clone();
+                e.done->record(st);
+            }
+        }
+        if (!y.defined()) y = body(c, x.contiguous());
         peek.snapshot(device.index(), st.stream(), capturing);
         return y;
     }
@@ -206,10 +288,10 @@ struct VigPlan : PlanBase {
     mutable Tensor pos;
     mutable int64_t pos_h = 0, pos_w = 0;
 
-    OptT forward(const Tensor& x) const {
+    OptT forward(const Tensor& x) {
         const int64_t H = x.dim() == 4 ? x.size(2) : 0, W = x.dim() == 4 ? x.size(3) : 0;
         if (H % 8 || W % 8 || H == 0) return std::nullopt;
-        return run(x, [&](const Ctx& c, const Tensor& img) { return body(c, img); });
+        return run(x, x.size(0) * ((H + 15) / 16) * ((W + 15) / 16) * C, [&](const Ctx& c, const Tensor& img) { return body(c, img); });
     }
     Tensor body(const Ctx& c, const Tensor& img) const {
         const int64_t B = img.size(0), H = img.size(2), W = img.size(3);
@@ -286,8 +368,8 @@ struct HierPlan : PlanBase {
     std::vector<HierStage> stages;
     Norm last;
 
-    OptT forward(const Tensor& x) const {
-        return run(x, [&](const Ctx& c, const Tensor& img) { return body(c, img); });
+    OptT forward(const Tensor& x) {
+        return run(x, x.dim() == 4 ? x.size(0) * ((x.size(2) + 3) / 4) * ((x.size(3) + 3) / 4) * std::get<0>(embed.back()).w.size(0) : 0, [&](const Ctx& c, const Tensor& img) { return body(c, img); });
     }
     Tensor body(const Ctx& c, const Tensor& img) const {
         Tensor y = img.permute({0, 2, 3, 1}).contiguous();
