@@ -63,6 +63,9 @@ extern "C" {
                               (32,64), (64,64), every type) */
 
 VIG_API int vig_version(void);
+/* Lets this thread's launches overlap the end of the kernel before them (programmatic dependent launch); returns the previous
+ * setting.  Set it only around calls whose weights are not written by the work queued just before them. */
+VIG_API int vig_chain_launches(int on);
 VIG_API const char* vig_strerror(int status);
 
 /*
@@ -144,6 +147,21 @@ VIG_API int vig_bigla_bwd_full(const void* q, const void* k, const void* v, cons
                   const int64_t* strides_gf, const int64_t* strides_gb, const int64_t* strides_do,
                   float scale, float out_scale, float gate_logit_normalizer, float clamp_min, int dir_mask,
                   void* workspace, size_t workspace_bytes, void* stream);
+
+/*
+ * The row-local half of a block of width 192 (3 heads of 64) in one kernel, bf16 / fp16, any M: y = gating injection of
+ * (o, local, gate_logits) as vig_gate_inject_fwd, r = y W_o^T + residual, h = RMSNorm(r) * norm_w,
+ * z = swiglu(h W_gate^T) as vig_linear_swiglu_fwd, out_r = z W_down^T + r, out_h = RMSNorm(out_r) * next_w
+ * (classification/models/vig.py:444-463, 494-497, 596-618), with the roundings of the separate calls.  o, local, residual,
+ * out_*: contiguous [M, 192]; gate_logits: [M, 192] with row stride ld_gate; w_o [192,192], w_gate [2I,192], w_down [192,I],
+ * I a multiple of 64 up to 512.  ``preferred``: whether it beats the separate kernels at this M.
+ */
+VIG_API int vig_block_tail_supported(int64_t M, int H, int dv, int I, int dtype);
+VIG_API int vig_block_tail_preferred(int64_t M, int H, int dv, int I, int dtype);
+VIG_API int vig_block_tail_fwd(const void* o, const void* local, const void* gate_logits, int64_t ld_gate, const void* w_gnorm, const void* w_lnorm,
+                       float inject_eps, int out_act_swish, const void* w_o, const void* residual, const void* norm_w, float norm_eps,
+                       const void* w_gate, const void* w_down, const void* next_w, float next_eps, void* out_r, void* out_h,
+                       int64_t M, int H, int dv, int I, int dtype, int32_t* status_dev, void* stream);
 
 /*
  * Bi-GLA forward for callers that cannot allocate device memory (no counterpart in the reference: its

@@ -34,7 +34,9 @@ def test_native_forward_equals_the_modules(kind, size, dtype):
         ref = m(x)
         handle.remove()
     rel = float((got.float() - ref.float()).norm() / ref.float().norm())
-    assert rel < (1e-2 if kind.startswith("hier") else 1e-6), rel       # hier: the branch's add is fused into the next norm
+    # hier: the branch's add is fused into the next norm; vig_t: the row-local half of a block is one kernel whose sums run in
+    # another order, which flips roundings (2^-9) of stored activations
+    assert rel < (1e-6 if kind == "vig_s" else 1e-2), rel
 
 
 def test_plan_follows_the_model():

@@ -6,6 +6,9 @@ using namespace vig;
 
 extern "C" int vig_version(void) { return 100; }
 
+thread_local int vig::chain_launches = 0;
+extern "C" int vig_chain_launches(int on) { const int was = chain_launches; chain_launches = on; return was; }
+
 extern "C" const char* vig_strerror(int status) {
     switch (status) {
         case VIG_OK: return "ok";

@@ -57,6 +57,30 @@ template <typename T> __device__ __forceinline__ float sigmoid_t(float x) {
     return fmaf(0.5f, t, 0.5f);
 }
 
+// Programmatic dependent launch.  A kernel that calls pdl_wait() before it touches what an earlier kernel wrote may be launched
+// while that kernel still runs (launch_chained); pdl_launch() lets the next kernel of the stream do the same.  Both do nothing
+// in an ordinary launch.  A kernel allocates tensor memory only after pdl_wait(): earlier it could hold what a kernel it
+// waits for still has to allocate.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Whether this thread's launches may be chained: set around a model's forward, whose kernels read weights -- which none of them
+// writes -- before pdl_wait().
+extern thread_local int chain_launches;
+
+template <typename... K, typename... A>
+inline cudaError_t launch_chained(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = chain_launches ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, K(args)...);
+    return e != cudaSuccess ? e : cudaGetLastError();
+}
+
 // Parameter block of the bi-GLA launchers (host fills it from the C ABI arguments).
 struct BiglaParams {
     const void *q, *k, *v, *gf, *gb;

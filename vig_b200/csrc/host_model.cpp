@@ -21,6 +21,10 @@ using OptT = std::optional<Tensor>;
 
 // ---- library calls on tensors --------------------------------------------------------------------------------------
 struct Ctx { void* stream; int32_t* status; int code; };
+struct Chained {                                             // launches of this scope may overlap the end of the kernel before them
+    const int was = api.vig_chain_launches(1);
+    ~Chained() { api.vig_chain_launches(was); }
+};
 
 Tensor dwconv(const Ctx& c, const Tensor& x, const Tensor& taps, const Tensor& bias, int64_t h, int64_t w, bool act) {
     Tensor y = at::empty_like(x);
@@ -65,8 +69,8 @@ struct Attn {
     bool act_conv, out_act;
     double eps, out_scale, norm, clamp;
 
-    // everything up to (not including) the output projection; h [B,L,C] contiguous
-    Tensor forward(const Ctx& c, const Tensor& x, int64_t h, int64_t w) const {
+    struct Scanned { Tensor o, xs, z; };                     // scan output [B,L,H,dv], conv output, stacked projection
+    Scanned scan(const Ctx& c, const Tensor& x, int64_t h, int64_t w) const {
         const int64_t B = x.size(0), L = x.size(1), kd = H * dk, vd = H * dv;
         const Tensor xs = dwconv(c, x, taps, conv_b, h, w, act_conv);
         const Tensor z = at::linear(xs, w_z, b_z);
@@ -75,9 +79,17 @@ struct Attn {
         Tensor o = at::empty({B, L, H, dv}, x.options());
         bi_gla_into(view(0, dk), view(kd, dk), view(2 * kd, dv), view(2 * kd + 2 * vd, dk), view(3 * kd + 2 * vd, dk),
                     o.as_strided({B, H, L, dv}, {L * vd, dv, vd, 1}), -1.0, out_scale, norm, clamp, {}, {}, {}, {}, 3, VIG_IMPL_AUTO);
+        return {o, xs, z};
+    }
+    const void* gate_logits(const Tensor& z) const { return (const uint8_t*)ptr(z) + (2 * H * dk + H * dv) * z.element_size(); }
+
+    // everything up to (not including) the output projection; h [B,L,C] contiguous
+    Tensor forward(const Ctx& c, const Tensor& x, int64_t h, int64_t w) const {
+        const auto [o, xs, z] = scan(c, x, h, w);
+        const int64_t B = x.size(0), L = x.size(1), vd = H * dv, W = z.size(2);
         const int64_t so[3] = {L * vd, dv, vd};
         Tensor y = at::empty({B, L, vd}, x.options());
-        ok(api.vig_gate_inject_fwd(ptr(o), so, ptr(xs), (uint8_t*)ptr(z) + (2 * kd + vd) * z.element_size(), ptr(gn_w), ptr(ln_w), ptr(y), vd, W, vd, B, H, L, dv,
+        ok(api.vig_gate_inject_fwd(ptr(o), so, ptr(xs), gate_logits(z), ptr(gn_w), ptr(ln_w), ptr(y), vd, W, vd, B, H, L, dv,
                                    (float)eps, out_act, c.code, c.stream), "vig_gate_inject_fwd");
         return y;
     }
@@ -249,6 +261,7 @@ struct PlanBase {
         StatusPeek& peek = StatusPeek::of(device.index());
         if (const int v = peek.poll(capturing)) { on_status(v); }
         const Ctx c{st.stream(), status_ptr(device.index()), type == at::kBFloat16 ? VIG_DTYPE_BF16 : VIG_DTYPE_F16};
+        const Chained chained;
         Tensor y;
         if (!capturing && work <= GRAPH_WORK) {
             Captured& e = entry(x, st.stream(), work);
@@ -321,8 +334,20 @@ struct VigPlan : PlanBase {
             for (size_t i = 0; i < blocks.size(); ++i) {
                 const VigBlock& b = blocks[i];
                 const bool last = i + 1 == blocks.size();
+                const int64_t I = b.down_w.size(1);
+                const Tensor& next_w = last ? norm_w : blocks[i + 1].n1;
+                const double next_e = last ? norm_e : blocks[i + 1].e1;
+                if (api.vig_block_tail_preferred(rows, b.attn.H, b.attn.dv, I, c.code)) {
+                    const auto [o, xs, z] = b.attn.scan(c, n, h, w);
+                    Tensor r = at::empty_like(tok), hn = at::empty_like(tok);
+                    ok(api.vig_block_tail_fwd(ptr(o), ptr(xs), b.attn.gate_logits(z), z.size(2), ptr(b.attn.gn_w), ptr(b.attn.ln_w), (float)b.attn.eps, b.attn.out_act,
+                                              ptr(b.attn.o_w), ptr(tok), ptr(b.n2), (float)b.e2, ptr(b.gate_w), ptr(b.down_w), ptr(next_w), (float)next_e, ptr(r),
+                                              ptr(hn), rows, b.attn.H, b.attn.dv, I, c.code, c.status, c.stream), "vig_block_tail_fwd");
+                    tok = r; n = hn;
+                    continue;
+                }
                 std::tie(n, tok) = linear_add_rmsnorm(c, b.attn.forward(c, n, h, w), b.attn.o_w, tok, b.n2, b.e2);
-                std::tie(n, tok) = linear_add_rmsnorm(c, mlp_in(c, n, b.gate_w), b.down_w, tok, last ? norm_w : blocks[i + 1].n1, last ? norm_e : blocks[i + 1].e1);
+                std::tie(n, tok) = linear_add_rmsnorm(c, mlp_in(c, n, b.gate_w), b.down_w, tok, next_w, next_e);
             }
             return finish(n.mean(1));
         }

@@ -518,6 +518,22 @@ def swiglu(gate, y):
     return out
 
 
+def block_tail(o, local, gate_logits, w_gnorm, w_lnorm, w_o, residual, norm_w, w_gate, w_down, next_w, *, inject_eps=1e-6, norm_eps=1e-6,
+               next_eps=1e-6, out_act=False):
+    """The row-local half of a block of width 192 in one kernel (see ``vig_block_tail_fwd``): ``o``, ``local`` and ``residual``
+    contiguous ``[M, 192]``, ``gate_logits`` ``[M, 192]`` rows of a wider tensor.  Returns ``(h, r)``."""
+    dev = _same_device(o, local, gate_logits, w_o, residual, w_gate, w_down)
+    M = o.shape[0]
+    r, h = torch.empty_like(o), torch.empty_like(o)
+    with torch.cuda.device(dev):
+        st = _lib.lib().vig_block_tail_fwd(_lib.ptr(o), _lib.ptr(local), _lib.ptr(gate_logits), gate_logits.stride(0), _lib.ptr(w_gnorm), _lib.ptr(w_lnorm),
+                                           float(inject_eps), int(bool(out_act)), _lib.ptr(w_o), _lib.ptr(residual), _lib.ptr(norm_w), float(norm_eps),
+                                           _lib.ptr(w_gate), _lib.ptr(w_down), _lib.ptr(next_w), float(next_eps), _lib.ptr(r), _lib.ptr(h), M,
+                                           o.shape[1] // 64, 64, w_down.shape[1], _lib.dtype_code(o), _status_ptr(None, dev), _lib.stream_ptr())
+    _lib.check(st, "vig_block_tail_fwd")
+    return h, r
+
+
 def linear_swiglu_supported(x, weight, preferred=False):
     """True when ``linear_swiglu`` has a fused kernel for this input (bf16 / fp16, K % 64 == 0, K <= 384, I % 64 == 0);
     with ``preferred`` also that it beats the library GEMM followed by the SwiGLU kernel (K <= 192)."""
