@@ -41,45 +41,52 @@ __global__ void __launch_bounds__(NT) bwd_states_mma_kernel(const __grid_constan
     const int64_t t0 = (int64_t)c * C;
     const int n = min(C, p.L - (int)t0);
     const int pr = threadIdx.x % CL::PAIRS, r0 = (threadIdx.x / CL::PAIRS) * CL::RPG;
+    const bool one_dir = gridDim.z != 1;
+    Raw2<T> x[CL::RPG], q[CL::RPG], k[CL::RPG];
+    auto load_gate = [&](int dir) {
+        load_rows(x, (dir ? head_ptr<T>(p.gb, p.sgb, b, h, t0) : head_ptr<T>(p.gf, p.sgf, b, h, t0)) + 2 * pr, dir ? p.sgb[2] : p.sgf[2], r0, n);
+    };
+    const int first = one_dir ? blockIdx.z : p.dir_mask & 1 ? 0 : 1;
+    load_gate(first);
+    load_rows(k, head_ptr<T>(p.k, p.sk, b, h, t0) + 2 * pr, p.sk[2], r0, n);
+    load_rows(q, head_ptr<T>(p.q, p.sq, b, h, t0) + 2 * pr, p.sq[2], r0, n);
     load_raw<T, DV, RAW>(smem + SM::V, head_ptr<T>(p.v, p.sv, b, h, t0), p.sv[2], n);
     load_raw<T, DV, RAW>(smem + SM::O, head_ptr<T>(p.dout, p.sdo, b, h, t0), p.sdo[2], n);
-    const T* qp = head_ptr<T>(p.q, p.sq, b, h, t0);
-    const T* kp = head_ptr<T>(p.k, p.sk, b, h, t0);
-    for (int dir = gridDim.z == 1 ? 0 : blockIdx.z; dir < 2; dir += gridDim.z == 1 ? 1 : 2) {
-        if (!(p.dir_mask & (1 << dir))) continue;
+    zero_rows(k, r0, n); zero_rows(q, r0, n);
+    const int last = one_dir ? first : p.dir_mask & 2 ? 1 : 0;
+    for (int dir = first; dir <= last; ++dir) {
         const size_t slot = ((size_t)bh * p.nchunk + c) * 2 + dir;
-        float2 G[CL::RPG], ref, tot;
-        const T* gp = dir ? head_ptr<T>(p.gb, p.sgb, b, h, t0) : head_ptr<T>(p.gf, p.sgf, b, h, t0);
-        cum_gates<DK, T>(G, ref, tot, gsum, gp, dir ? p.sgb[2] : p.sgf[2], n, dir, p.gate_norm, p.clamp_min);
-        if (r0 == 0) *reinterpret_cast<float2*>(p.ws_decay + slot * DK + 2 * pr) = tot;
+        F2 G[CL::RPG], ref, tot;
+        cum_gates<DK, T>(G, ref, tot, gsum, x, n, dir, p.gate_norm, p.clamp_min);
+        if (dir < last) load_gate(dir + 1);
+        if (r0 == 0) *reinterpret_cast<F2*>(p.ws_decay + slot * DK + 2 * pr) = tot;
+        const F2 minus = f2_make(-1.f, -1.f), cc = f2_make(p.c, p.c);
 #pragma unroll
         for (int r = 0; r < CL::RPG; ++r) {
-            float2 q = make_float2(0.f, 0.f), k = q;
-            if (r0 + r < n) { q = load2<T>(qp + (r0 + r) * p.sq[2] + 2 * pr); k = load2<T>(kp + (r0 + r) * p.sk[2] + 2 * pr); }
+            const F2 y = f2_fma(G[r], minus, tot);
             uint32_t t[SC];
-            split2<SC>(k.x * ex2_t<T>(tot.x - G[r].x), k.y * ex2_t<T>(tot.y - G[r].y), t);
+            const F2 ks = f2_mul(k[r].f2(), f2_make(ex2_t<T>(f2_lo(y)), ex2_t<T>(f2_hi(y))));
+            split2<SC>(f2_lo(ks), f2_hi(ks), t);
 #pragma unroll
             for (int i = 0; i < SC; ++i) *reinterpret_cast<uint32_t*>(smem + SM::K + i * C * Pitch<DK>::B + (r0 + r) * Pitch<DK>::B + pr * 4) = t[i];
-            split2<SC>(p.c * q.x * ex2_t<T>(G[r].x), p.c * q.y * ex2_t<T>(G[r].y), t);
+            const F2 qs = f2_mul(f2_mul(q[r].f2(), cc), f2_make(ex2_t<T>(f2_lo(G[r])), ex2_t<T>(f2_hi(G[r]))));
+            split2<SC>(f2_lo(qs), f2_hi(qs), t);
 #pragma unroll
             for (int i = 0; i < SC; ++i) *reinterpret_cast<uint32_t*>(smem + SM::Q + i * C * Pitch<DK>::B + (r0 + r) * Pitch<DK>::B + pr * 4) = t[i];
         }
         __syncthreads();
-        const int mt = warp % MT, wn = warp / MT;
+        const int which = warp >> 2, mt = (warp & 3) % MT, wn = (warp & 3) / MT;          // warps 0 - 3: S, 4 - 7: Z
+        float acc[NTL][4];
 #pragma unroll
-        for (int which = 0; which < 2; ++which) {
-            float acc[NTL][4];
+        for (int i = 0; i < NTL; ++i)
 #pragma unroll
-            for (int i = 0; i < NTL; ++i)
+            for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+        state_mma<DK, DV, SC, RAW, NTL>(acc, sb + (which ? SM::Q : SM::K) + mt * 32, sb + (which ? SM::O : SM::V) + wn * NC * 2, lane);
+        float* out = (which ? p.ws_Z : p.ws_S) + slot * DK * DV + (mt * 16 + (lane >> 2)) * DV + wn * NC + 2 * (lane & 3);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-            state_mma<DK, DV, SC, RAW, NTL>(acc, sb + (which ? SM::Q : SM::K) + mt * 32, sb + (which ? SM::O : SM::V) + wn * NC * 2, lane);
-            float* out = (which ? p.ws_Z : p.ws_S) + slot * DK * DV + (mt * 16 + (lane >> 2)) * DV + wn * NC + 2 * (lane & 3);
-#pragma unroll
-            for (int i = 0; i < NTL; ++i) {
-                *reinterpret_cast<float2*>(out + i * 8) = make_float2(acc[i][0], acc[i][1]);
-                *reinterpret_cast<float2*>(out + 8 * DV + i * 8) = make_float2(acc[i][2], acc[i][3]);
-            }
+        for (int i = 0; i < NTL; ++i) {
+            *reinterpret_cast<float2*>(out + i * 8) = make_float2(acc[i][0], acc[i][1]);
+            *reinterpret_cast<float2*>(out + 8 * DV + i * 8) = make_float2(acc[i][2], acc[i][3]);
         }
         __syncthreads();
     }
@@ -126,80 +133,90 @@ __global__ void __launch_bounds__(256) bwd_scan_kernel(const __grid_constant__ B
 
 // ---- chunk gradients -----------------------------------------------------------------------------------------------
 template <int DK, int DV, typename T> struct GradSmem {
-    static constexpr uint32_t EP = DK + 8;                             // row pitch of the fp32 tile (floats)
+    static constexpr uint32_t EP = DK + 8, VP = DV + 8;                // row pitches of the fp32 tiles (floats)
+    static constexpr uint32_t TQ = Terms<T>::SC * C * Pitch<DK>::B, TS = Terms<T>::SC * DK * Pitch<DV>::B;
     static constexpr uint32_t V = 0, O = V + Terms<T>::RAW * C * Pitch<DV>::B, K = O + Terms<T>::RAW * C * Pitch<DV>::B,
-                              Q = K + Terms<T>::SC * C * Pitch<DK>::B, S = Q + Terms<T>::SC * C * Pitch<DK>::B,
-                              E = S + Terms<T>::SC * DK * Pitch<DV>::B, SUM = E + C * EP * 4, CARRY = SUM + 2 * NT * 4,
+                              Q = K + TQ, S = Q + TQ, Z = S + TS, X = Z + TS, SUM = X + C * DK * 4, CARRY = SUM + 2 * NT * 4,
                               SCL = CARRY + DK * 4, BYTES = SCL + 2 * DK * 4;
+    static_assert(C * EP * 4 <= TQ && C * VP * 4 <= 2 * TQ, "the fp32 tiles reuse the operand tiles");
 };
 
+// Eight warps on a chunk: warps 0 - 3 form dQ and the state term of dV, warps 4 - 7 dK and the term of dV inside the chunk, 16
+// rows each.  (Four warps with all of it in 255 registers: two CTAs, eight warps an SM, 12 % of the tensor rate.)  What follows
+// the products -- the factors 2^(G-r), e and its sums, both directions' totals -- is done by channel pairs, in which q, k and
+// the gates are read coalesced.
 template <int DK, int DV, typename T>
-__global__ void __launch_bounds__(NT, 2) bwd_grads_mma_kernel(const __grid_constant__ BwdParams p) {
+__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 1 : 2) bwd_grads_mma_kernel(const __grid_constant__ BwdParams p) {
     using CL = ColLay<DK>;
     using SM = GradSmem<DK, DV, T>;
-    constexpr int RAW = Terms<T>::RAW, SC = Terms<T>::SC;
-    constexpr uint32_t PK = Pitch<DK>::B, PV = Pitch<DV>::B, EP = SM::EP;
+    constexpr int RAW = Terms<T>::RAW, SC = Terms<T>::SC, RPG = CL::RPG;
+    constexpr uint32_t PK = Pitch<DK>::B, PV = Pitch<DV>::B;
     constexpr uint32_t TK = C * PK, TV = C * PV, TS = DK * PV;          // bytes from one term's tile to the next
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t sb = tc::smem_u32(smem);
-    float* E = reinterpret_cast<float*>(smem + SM::E);
+    F2* X = reinterpret_cast<F2*>(smem + SM::X);                        // [RPG][NT]: 2^(G-r) of each thread's rows, private
     float* gsum = reinterpret_cast<float*>(smem + SM::SUM);
     float* carry = reinterpret_cast<float*>(smem + SM::CARRY);
     float* scl = reinterpret_cast<float*>(smem + SM::SCL);              // [0]: 2^r, [1]: 2^(l-r)
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    float* EQ = reinterpret_cast<float*>(smem + SM::Q);                 // dQ, dK of a direction once the products are done
+    float* EK = reinterpret_cast<float*>(smem + SM::K);
+    const int lane = threadIdx.x & 31, role = threadIdx.x >> 7, w = (threadIdx.x >> 5) & 3;
     const int c = blockIdx.x, bh = blockIdx.y, b = bh / p.H, h = bh % p.H;
     const int64_t t0 = (int64_t)c * C;
     const int n = min(C, p.L - (int)t0);
-    const int pr = threadIdx.x % CL::PAIRS, gr = threadIdx.x / CL::PAIRS, r0 = gr * CL::RPG;
+    const int pr = threadIdx.x % CL::PAIRS, gr = threadIdx.x / CL::PAIRS, r0 = gr * RPG;
     const int fr = 16 * w + (lane >> 2), fc = 2 * (lane & 3);           // my fragment rows fr, fr + 8; columns 8 nt + fc, + 1
-    const T* qp = head_ptr<T>(p.q, p.sq, b, h, t0);
-    const T* kp = head_ptr<T>(p.k, p.sk, b, h, t0);
+    const T* qp = head_ptr<T>(p.q, p.sq, b, h, t0) + 2 * pr;
+    const T* kp = head_ptr<T>(p.k, p.sk, b, h, t0) + 2 * pr;
+    const F2 cc = f2_make(p.c, p.c), minus = f2_make(-1.f, -1.f);
     load_raw<T, DV, RAW>(smem + SM::V, head_ptr<T>(p.v, p.sv, b, h, t0), p.sv[2], n);
     load_raw<T, DV, RAW>(smem + SM::O, head_ptr<T>(p.dout, p.sdo, b, h, t0), p.sdo[2], n);
     const uint32_t aV = sb + SM::V + 16 * w * PV + frag_rows<PV>(lane), aO = sb + SM::O + 16 * w * PV + frag_rows<PV>(lane);
     const uint32_t aK = sb + SM::K + 16 * w * PK + frag_rows<PK>(lane);
     const uint32_t bV = sb + SM::V + frag_cols<PV>(lane), bO = sb + SM::O + frag_cols<PV>(lane), bQ = sb + SM::Q + frag_cols<PK>(lane);
     const uint32_t tK = sb + SM::K + frag_rows<PK>(lane), tQ = sb + SM::Q + frag_rows<PK>(lane), tO = sb + SM::O + frag_rows<PV>(lane);
-    const uint32_t bS = sb + SM::S + frag_cols<PV>(lane), tS = sb + SM::S + frag_rows<PV>(lane);
-    float dqt[DK / 8][4], dkt[DK / 8][4], dv[DV / 8][4];
-#pragma unroll
-    for (int i = 0; i < DK / 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) { dqt[i][j] = 0.f; dkt[i][j] = 0.f; }
+    float dv[DV / 8][4];
 #pragma unroll
     for (int i = 0; i < DV / 8; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) dv[i][j] = 0.f;
+    F2 dqt[RPG], dkt[RPG];
+#pragma unroll
+    for (int r = 0; r < RPG; ++r) dqt[r] = dkt[r] = f2_make(0.f, 0.f);
     const bool have_states = p.nchunk > 1;
 #pragma unroll 1
     for (int dir = 0; dir < 2; ++dir) {
         if (!(p.dir_mask & (1 << dir))) continue;
-        const T* gp = dir ? head_ptr<T>(p.gb, p.sgb, b, h, t0) : head_ptr<T>(p.gf, p.sgf, b, h, t0);
+        const T* gp = (dir ? head_ptr<T>(p.gb, p.sgb, b, h, t0) : head_ptr<T>(p.gf, p.sgf, b, h, t0)) + 2 * pr;
         const int64_t sgl = dir ? p.sgb[2] : p.sgf[2];
         const size_t slot = ((size_t)bh * p.nchunk + c) * 2 + dir;
-        // ---- gates, scaled operand tiles
-        {
-            float2 G[CL::RPG], ref, tot;
-            cum_gates<DK, T>(G, ref, tot, gsum, gp, sgl, n, dir, p.gate_norm, p.clamp_min);
+        {   // ---- gates, scaled operand tiles
+            Raw2<T> x[RPG], q[RPG], k[RPG];
+            load_rows(x, gp, sgl, r0, n);
+            load_rows(q, qp, p.sq[2], r0, n);
+            load_rows(k, kp, p.sk[2], r0, n);
+            F2 G[RPG], ref, tot;
+            cum_gates<DK, T>(G, ref, tot, gsum, x, n, dir, p.gate_norm, p.clamp_min);
+            zero_rows(q, r0, n); zero_rows(k, r0, n);
             const float lim = range_limit<T>();
-            bool fine = fabsf(ref.x) <= lim && fabsf(ref.y) <= lim && fabsf(tot.x - ref.x) <= lim && fabsf(tot.y - ref.y) <= lim;
+            const F2 rest = f2_fma(ref, minus, tot);
+            bool fine = fabsf(f2_lo(ref)) <= lim && fabsf(f2_hi(ref)) <= lim && fabsf(f2_lo(rest)) <= lim && fabsf(f2_hi(rest)) <= lim;
             if (gr == 0) {
-                *reinterpret_cast<float2*>(scl + 2 * pr) = make_float2(ex2_t<T>(ref.x), ex2_t<T>(ref.y));
-                *reinterpret_cast<float2*>(scl + DK + 2 * pr) = make_float2(ex2_t<T>(tot.x - ref.x), ex2_t<T>(tot.y - ref.y));
+                *reinterpret_cast<float2*>(scl + 2 * pr) = make_float2(ex2_t<T>(f2_lo(ref)), ex2_t<T>(f2_hi(ref)));
+                *reinterpret_cast<float2*>(scl + DK + 2 * pr) = make_float2(ex2_t<T>(f2_lo(rest)), ex2_t<T>(f2_hi(rest)));
             }
 #pragma unroll
-            for (int r = 0; r < CL::RPG; ++r) {
-                float2 q = make_float2(0.f, 0.f), k = q;
-                if (r0 + r < n) { q = load2<T>(qp + (r0 + r) * p.sq[2] + 2 * pr); k = load2<T>(kp + (r0 + r) * p.sk[2] + 2 * pr); }
-                const float x = G[r].x - ref.x, y = G[r].y - ref.y;
-                fine = fine && fabsf(x) <= lim && fabsf(y) <= lim;
-                const float ex = ex2_t<T>(x), ey = ex2_t<T>(y);
-                *reinterpret_cast<float2*>(E + (r0 + r) * EP + 2 * pr) = make_float2(ex, ey);
+            for (int r = 0; r < RPG; ++r) {
+                const F2 y = f2_fma(ref, minus, G[r]);
+                fine = fine && fabsf(f2_lo(y)) <= lim && fabsf(f2_hi(y)) <= lim;
+                const F2 ex = f2_make(ex2_t<T>(f2_lo(y)), ex2_t<T>(f2_hi(y)));
+                X[r * NT + threadIdx.x] = ex;
                 uint32_t t[SC];
-                split2<SC>(p.c * q.x * ex, p.c * q.y * ey, t);
+                const F2 qs = f2_mul(f2_mul(q[r].f2(), cc), ex), ks = f2_mul(k[r].f2(), f2_make(ex2_t<T>(-f2_lo(y)), ex2_t<T>(-f2_hi(y))));
+                split2<SC>(f2_lo(qs), f2_hi(qs), t);
 #pragma unroll
                 for (int i = 0; i < SC; ++i) *reinterpret_cast<uint32_t*>(smem + SM::Q + i * TK + (r0 + r) * PK + pr * 4) = t[i];
-                split2<SC>(k.x * ex2_t<T>(-x), k.y * ex2_t<T>(-y), t);
+                split2<SC>(f2_lo(ks), f2_hi(ks), t);
 #pragma unroll
                 for (int i = 0; i < SC; ++i) *reinterpret_cast<uint32_t*>(smem + SM::K + i * TK + (r0 + r) * PK + pr * 4) = t[i];
             }
@@ -208,62 +225,47 @@ __global__ void __launch_bounds__(NT, 2) bwd_grads_mma_kernel(const __grid_const
                 return;
             }
         }
-        const int klo = dir ? w : 0, khi = dir ? C / 16 : w + 1;         // 16-token blocks scanned at or before mine
-        const int qlo = dir ? 0 : w, qhi = dir ? w + 1 : C / 16;         // ... at or after mine
-        const int next = dir ? c - 1 : c + 1;                           // the chunk scanned after this one
-        const bool last = next < 0 || next >= p.nchunk;
         if (have_states) {
+            const int next = dir ? c - 1 : c + 1;                       // the chunk scanned after this one
             load_state<DK, DV, SC>(smem + SM::S, p.ws_S + slot * DK * DV, scl, nullptr, nullptr);
+            load_state<DK, DV, SC>(smem + SM::Z, p.ws_Z + slot * DK * DV, scl + DK,
+                                   next < 0 || next >= p.nchunk ? nullptr : p.ws_S + (((size_t)bh * p.nchunk + next) * 2 + dir) * DK * DV, carry);
             __syncthreads();
         }
-        float ev[DK / 8][4];
-        {   // ---- dQ of my rows
-            float dq[DK / 8][4];
+        float acc[DK / 8][4];
 #pragma unroll
-            for (int i = 0; i < DK / 8; ++i)
+        for (int i = 0; i < DK / 8; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) dq[i][j] = 0.f;
+            for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+        if (role == 0) {                                                 // ---- dQ of my rows: 16-token blocks scanned at or before mine
 #pragma unroll 1
-            for (int jb = klo; jb < khi; ++jb) {
+            for (int jb = dir ? w : 0; jb < (dir ? C / 16 : w + 1); ++jb) {
                 float pb[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
                 uint32_t ap[SC][4];
                 block_nt<DV, RAW, RAW>(pb, aO, TV, bV + jb * 16 * PV, TV);
                 mask_split<SC>(pb, jb == w, lane, [&](int r, int j) { return dir ? j >= r : j <= r; }, ap);
-                block_nn<DK, SC, SC>(dq, ap, tK + jb * 16 * PK, TK);
+                block_nn<DK, SC, SC>(acc, ap, tK + jb * 16 * PK, TK);
             }
-            if (have_states) rows_nt<DK, DV, PV, RAW, SC>(dq, aO, TV, bS, TS);
+            if (have_states) {
+                rows_nt<DK, DV, PV, RAW, SC>(acc, aO, TV, sb + SM::S + frag_cols<PV>(lane), TS);
+                const uint32_t tZ = sb + SM::Z + frag_rows<PV>(lane);
 #pragma unroll
-            for (int i = 0; i < DK / 8; ++i)
+                for (int ks = 0; ks < DK / 16; ++ks) {
+                    uint32_t fa[SC][4];
 #pragma unroll
-                for (int hf = 0; hf < 2; ++hf) {
-                    const int row = fr + 8 * hf, col = 8 * i + fc;
-                    const float2 ex = *reinterpret_cast<const float2*>(E + row * EP + col);
-                    const float2 q = row < n ? load2<T>(qp + row * p.sq[2] + col) : make_float2(0.f, 0.f);
-                    const float a = p.c * ex.x * dq[i][2 * hf], d = p.c * ex.y * dq[i][2 * hf + 1];
-                    dqt[i][2 * hf] += a; dqt[i][2 * hf + 1] += d;
-                    ev[i][2 * hf] = a * q.x; ev[i][2 * hf + 1] = d * q.y;
+                    for (int t = 0; t < SC; ++t) ldsm4(aK + t * TK + ks * 32, fa[t]);
+                    block_nn<DV, SC, SC>(dv, fa, tZ + ks * 16 * PV, TS);
                 }
-        }
-        if (have_states) {
-            __syncthreads();                                             // S is read
-            load_state<DK, DV, SC>(smem + SM::S, p.ws_Z + slot * DK * DV, scl + DK,
-                                   last ? nullptr : p.ws_S + (((size_t)bh * p.nchunk + next) * 2 + dir) * DK * DV, carry);
-            __syncthreads();
-        }
-        {   // ---- dK and dV of my rows
-            float dk[DK / 8][4];
-#pragma unroll
-            for (int i = 0; i < DK / 8; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) dk[i][j] = 0.f;
+            }
+        } else {                                                         // ---- dK and dV of my rows: blocks scanned at or after mine
+            auto keep = [&](int j, int i) { return dir ? i <= j : i >= j; };
 #pragma unroll 1
-            for (int ib = qlo; ib < qhi; ++ib) {
-                auto keep = [&](int j, int i) { return dir ? i <= j : i >= j; };
+            for (int ib = dir ? 0 : w; ib < (dir ? w + 1 : C / 16); ++ib) {
                 float pb[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
                 uint32_t ap[SC][4];
                 block_nt<DV, RAW, RAW>(pb, aV, TV, bO + ib * 16 * PV, TV);
                 mask_split<SC>(pb, ib == w, lane, keep, ap);
-                block_nn<DK, SC, SC>(dk, ap, tQ + ib * 16 * PK, TK);
+                block_nn<DK, SC, SC>(acc, ap, tQ + ib * 16 * PK, TK);
 #pragma unroll
                 for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -272,52 +274,52 @@ __global__ void __launch_bounds__(NT, 2) bwd_grads_mma_kernel(const __grid_const
                 mask_split<SC>(pb, ib == w, lane, keep, ap);
                 block_nn<DV, SC, RAW>(dv, ap, tO + ib * 16 * PV, TV);
             }
-            if (have_states) {
-                rows_nt<DK, DV, PV, RAW, SC>(dk, aV, TV, bS, TS);
-#pragma unroll
-                for (int ks = 0; ks < DK / 16; ++ks) {
-                    uint32_t fa[SC][4];
-#pragma unroll
-                    for (int t = 0; t < SC; ++t) ldsm4(aK + t * TK + ks * 32, fa[t]);
-                    block_nn<DV, SC, SC>(dv, fa, tS + ks * 16 * PV, TS);
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < DK / 8; ++i)
-#pragma unroll
-                for (int hf = 0; hf < 2; ++hf) {
-                    const int row = fr + 8 * hf, col = 8 * i + fc;
-                    float2* e = reinterpret_cast<float2*>(E + row * EP + col);
-                    const float2 ex = *e;
-                    const float2 k = row < n ? load2<T>(kp + row * p.sk[2] + col) : make_float2(0.f, 0.f);
-                    const float a = __fdividef(dk[i][2 * hf], ex.x), d = __fdividef(dk[i][2 * hf + 1], ex.y);
-                    dkt[i][2 * hf] += a; dkt[i][2 * hf + 1] += d;
-                    *e = make_float2(ev[i][2 * hf] - a * k.x, ev[i][2 * hf + 1] - d * k.y);
-                }
+            if (have_states) rows_nt<DK, DV, PV, RAW, SC>(acc, aV, TV, sb + SM::Z + frag_cols<PV>(lane), TS);
         }
-        __syncthreads();
-        {   // ---- gate gradient: sum of e over the tokens scanned at or after t, plus the value just past the chunk
-            float2 x[CL::RPG], sum = make_float2(0.f, 0.f);
+        __syncthreads();                                                 // the operand tiles are read
+        {
+            float* E = (role ? EK : EQ) + fr * SM::EP + fc;
 #pragma unroll
-            for (int r = 0; r < CL::RPG; ++r) { x[r] = *reinterpret_cast<const float2*>(E + (r0 + r) * EP + 2 * pr); sum.x += x[r].x; sum.y += x[r].y; }
-            *reinterpret_cast<float2*>(gsum + gr * DK + 2 * pr) = sum;
+            for (int i = 0; i < DK / 8; ++i) {
+                *reinterpret_cast<float2*>(E + 8 * i) = make_float2(acc[i][0], acc[i][1]);
+                *reinterpret_cast<float2*>(E + 8 * SM::EP + 8 * i) = make_float2(acc[i][2], acc[i][3]);
+            }
+        }
+        Raw2<T> x[RPG], q[RPG], k[RPG];
+        load_rows(q, qp, p.sq[2], r0, n);
+        load_rows(k, kp, p.sk[2], r0, n);
+        if (p.gate_norm > 0.f || p.clamp_min == p.clamp_min) load_rows(x, gp, sgl, r0, n);
+        __syncthreads();
+        {   // ---- by channel pairs: totals, e, and the gate gradient = sum of e over the tokens scanned at or after t plus the value just past the chunk
+            F2 e[RPG], sum = f2_make(0.f, 0.f);
+            zero_rows(q, r0, n); zero_rows(k, r0, n);
+#pragma unroll
+            for (int r = 0; r < RPG; ++r) {
+                const F2 ex = X[r * NT + threadIdx.x];
+                const F2 dq = f2_mul(f2_mul(*reinterpret_cast<const F2*>(EQ + (r0 + r) * SM::EP + 2 * pr), ex), cc);
+                const F2 dk = f2_mul(*reinterpret_cast<const F2*>(EK + (r0 + r) * SM::EP + 2 * pr), f2_make(__fdividef(1.f, f2_lo(ex)), __fdividef(1.f, f2_hi(ex))));
+                dqt[r] = f2_add(dqt[r], dq); dkt[r] = f2_add(dkt[r], dk);
+                e[r] = f2_fma(f2_mul(dk, minus), k[r].f2(), f2_mul(dq, q[r].f2()));
+                sum = f2_add(sum, e[r]);
+            }
+            *reinterpret_cast<F2*>(gsum + gr * DK + 2 * pr) = sum;
             __syncthreads();
-            float2 run = have_states ? *reinterpret_cast<const float2*>(carry + 2 * pr) : make_float2(0.f, 0.f);
+            F2 run = have_states ? *reinterpret_cast<const F2*>(carry + 2 * pr) : f2_make(0.f, 0.f);
 #pragma unroll
             for (int o = 0; o < CL::GROUPS; ++o)
-                if (dir ? o < gr : o > gr) { const float2 s = *reinterpret_cast<const float2*>(gsum + o * DK + 2 * pr); run.x += s.x; run.y += s.y; }
+                if (dir ? o < gr : o > gr) run = f2_add(run, *reinterpret_cast<const F2*>(gsum + o * DK + 2 * pr));
             const int64_t base = ((int64_t)bh * p.L + t0) * DK + 2 * pr;
 #pragma unroll
-            for (int rr = 0; rr < CL::RPG; ++rr) {
+            for (int rr = 0; rr < RPG; ++rr) {
                 // static register indices for both orders: the backward direction sums upwards, the forward one downwards
-                const float2 xv = dir ? x[rr] : x[CL::RPG - 1 - rr];
-                const int row = r0 + (dir ? rr : CL::RPG - 1 - rr);
-                run.x += xv.x; run.y += xv.y;
+                const F2 ev = dir ? e[rr] : e[RPG - 1 - rr];
+                const int row = r0 + (dir ? rr : RPG - 1 - rr);
+                run = f2_add(run, ev);
                 if (row < n) {
-                    float2 dg = run;
+                    float2 dg = make_float2(f2_lo(run), f2_hi(run));
                     if (p.gate_norm > 0.f || p.clamp_min == p.clamp_min) {
-                        const float2 gx = load2<T>(gp + row * sgl + 2 * pr);
-                        dg.x = through_gate(dg.x, gx.x, p.gate_norm, p.clamp_min); dg.y = through_gate(dg.y, gx.y, p.gate_norm, p.clamp_min);
+                        const F2 gx = dir ? x[rr].f2() : x[RPG - 1 - rr].f2();
+                        dg.x = through_gate(dg.x, f2_lo(gx), p.gate_norm, p.clamp_min); dg.y = through_gate(dg.y, f2_hi(gx), p.gate_norm, p.clamp_min);
                     }
                     void* out = dir ? p.dgb : p.dgf;
                     if (p.dg_f32) store2<float>(reinterpret_cast<float*>(out) + base + (int64_t)row * DK, dg.x, dg.y);
@@ -325,21 +327,36 @@ __global__ void __launch_bounds__(NT, 2) bwd_grads_mma_kernel(const __grid_const
                 }
             }
         }
-        __syncthreads();                                                // E, gsum, carry and the tiles may be rewritten
+        __syncthreads();                                                // the tiles, gsum and carry may be rewritten
     }
     if (threadIdx.x == 0) p.flags[(size_t)bh * p.nchunk + c] = 0;
+#pragma unroll
+    for (int r = 0; r < RPG; ++r) {
+        if (r0 + r >= n) break;
+        const int64_t at = ((int64_t)bh * p.L + t0 + r0 + r) * DK + 2 * pr;
+        store2<T>(reinterpret_cast<T*>(p.out_dq) + at, f2_lo(dqt[r]), f2_hi(dqt[r]));
+        store2<T>(reinterpret_cast<T*>(p.out_dk) + at, f2_lo(dkt[r]), f2_hi(dkt[r]));
+    }
+    float* D = reinterpret_cast<float*>(smem + SM::K) + fr * SM::VP + fc;    // the two parts of dV meet in shared memory
+    if (role == 0) {
+#pragma unroll
+        for (int i = 0; i < DV / 8; ++i) {
+            *reinterpret_cast<float2*>(D + 8 * i) = make_float2(dv[i][0], dv[i][1]);
+            *reinterpret_cast<float2*>(D + 8 * SM::VP + 8 * i) = make_float2(dv[i][2], dv[i][3]);
+        }
+    }
+    __syncthreads();
+    if (role == 0) return;
 #pragma unroll
     for (int hf = 0; hf < 2; ++hf) {
         const int row = fr + 8 * hf;
         if (row >= n) continue;
-        const int64_t at = (int64_t)bh * p.L + t0 + row;
+        T* out = reinterpret_cast<T*>(p.out_dv) + ((int64_t)bh * p.L + t0 + row) * DV + fc;
 #pragma unroll
-        for (int i = 0; i < DK / 8; ++i) {
-            store2<T>(reinterpret_cast<T*>(p.out_dq) + at * DK + 8 * i + fc, dqt[i][2 * hf], dqt[i][2 * hf + 1]);
-            store2<T>(reinterpret_cast<T*>(p.out_dk) + at * DK + 8 * i + fc, dkt[i][2 * hf], dkt[i][2 * hf + 1]);
+        for (int i = 0; i < DV / 8; ++i) {
+            const float2 o = *reinterpret_cast<const float2*>(D + 8 * hf * SM::VP + 8 * i);
+            store2<T>(out + 8 * i, dv[i][2 * hf] + o.x, dv[i][2 * hf + 1] + o.y);
         }
-#pragma unroll
-        for (int i = 0; i < DV / 8; ++i) store2<T>(reinterpret_cast<T*>(p.out_dv) + at * DV + 8 * i + fc, dv[i][2 * hf], dv[i][2 * hf + 1]);
     }
 }
 

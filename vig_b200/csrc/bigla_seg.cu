@@ -23,7 +23,6 @@ namespace vig {
 namespace {
 
 using namespace mm;
-using tc::F2; using tc::f2_make; using tc::f2_lo; using tc::f2_hi; using tc::f2_add; using tc::f2_mul; using tc::f2_fma;
 
 enum { SEG_ONE = 0, SEG_STATES = 1, SEG_OUT = 2 };       // one launch (cluster = sequence) / contributions only / outputs from entering states
 
@@ -41,25 +40,6 @@ template <int DK, int DV, typename T, int TOK> struct SegSmem {
     static_assert(SUM >= TOK * DV * 4, "the exact form keeps its outputs in the tiles");
 };
 
-// Two neighbouring values as they lie in memory.  ``open_gate``: a pair that stands for log-gate 0 (rows past the end) --
-// the logit +inf, or the log-gate 0 itself.
-template <typename T> struct Raw2 {
-    uint32_t w;
-    __device__ __forceinline__ void load(const T* p) { w = __ldg(reinterpret_cast<const uint32_t*>(p)); }
-    __device__ __forceinline__ void zero() { w = 0u; }
-    __device__ __forceinline__ void open_gate(bool logits) { w = logits ? (std::is_same<T, __half>::value ? 0x7C007C00u : 0x7F807F80u) : 0u; }
-    __device__ __forceinline__ F2 f2() const {
-        if constexpr (std::is_same<T, __half>::value) { const float2 f = tc::Pack2<__half>::unpack(w); return f2_make(f.x, f.y); }
-        else return f2_make(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
-    }
-};
-template <> struct Raw2<float> {
-    float2 w;
-    __device__ __forceinline__ void load(const float* p) { w = __ldg(reinterpret_cast<const float2*>(p)); }
-    __device__ __forceinline__ void zero() { w = make_float2(0.f, 0.f); }
-    __device__ __forceinline__ void open_gate(bool logits) { w.x = w.y = logits ? INFINITY : 0.f; }
-    __device__ __forceinline__ F2 f2() const { return f2_make(w.x, w.y); }
-};
 // x * e of a raw pair and a pair of fp32 factors, in SC bf16 terms (one term: factors rounded to bf16, packed multiply)
 template <typename T, int SC> __device__ __forceinline__ void scaled(const Raw2<T>& x, float ex, float ey, uint32_t* t) {
     if constexpr (SC == 1) {

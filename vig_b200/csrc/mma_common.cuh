@@ -12,8 +12,10 @@
 namespace vig {
 namespace mm {
 
-constexpr int C = 64;                  // tokens per chunk: 4 warps x 16 rows
-constexpr int NT = 128;                // threads per CTA
+using tc::F2; using tc::f2_make; using tc::f2_lo; using tc::f2_hi; using tc::f2_add; using tc::f2_mul; using tc::f2_fma;
+
+constexpr int C = 64;                  // tokens per chunk
+constexpr int NT = 256;                // threads per CTA: two warps per 16 rows
 
 template <typename T> struct Terms;    // RAW: terms of an input value, SC: terms of a scaled / intermediate value
 template <> struct Terms<__nv_bfloat16> { static constexpr int RAW = 1, SC = 2; };
@@ -138,47 +140,85 @@ template <int DK> struct ColLay {
     static_assert(PAIRS <= NT && RPG >= 1, "head size");
 };
 
+// Two neighbouring values as they lie in memory.  ``open_gate``: a pair that stands for log-gate 0 (rows past the end) --
+// the logit +inf, or the log-gate 0 itself.
+template <typename T> struct Raw2 {
+    uint32_t w;
+    __device__ __forceinline__ void load(const T* p) { w = __ldg(reinterpret_cast<const uint32_t*>(p)); }
+    __device__ __forceinline__ void zero() { w = 0u; }
+    __device__ __forceinline__ void open_gate(bool logits) { w = logits ? (std::is_same<T, __half>::value ? 0x7C007C00u : 0x7F807F80u) : 0u; }
+    __device__ __forceinline__ F2 f2() const {
+        if constexpr (std::is_same<T, __half>::value) { const float2 f = tc::Pack2<__half>::unpack(w); return f2_make(f.x, f.y); }
+        else return f2_make(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
+    }
+};
+template <> struct Raw2<float> {
+    float2 w;
+    __device__ __forceinline__ void load(const float* p) { w = __ldg(reinterpret_cast<const float2*>(p)); }
+    __device__ __forceinline__ void zero() { w = make_float2(0.f, 0.f); }
+    __device__ __forceinline__ void open_gate(bool logits) { w.x = w.y = logits ? INFINITY : 0.f; }
+    __device__ __forceinline__ F2 f2() const { return f2_make(w.x, w.y); }
+};
+// The RPG rows of a thread's channel pair, from row r0 of the chunk; rows past the end read the last row (no branch between
+// the loads) and are neutralised afterwards.
+template <int RPG, typename T> __device__ __forceinline__ void load_rows(Raw2<T> (&x)[RPG], const T* p, int64_t stride_l, int r0, int n) {
+#pragma unroll
+    for (int r = 0; r < RPG; ++r) x[r].load(p + min(r0 + r, n - 1) * stride_l);
+}
+template <int RPG, typename T> __device__ __forceinline__ void zero_rows(Raw2<T> (&x)[RPG], int r0, int n) {
+    if (r0 + RPG > n) {
+#pragma unroll
+        for (int r = 0; r < RPG; ++r) if (r0 + r >= n) x[r].zero();
+    }
+}
+
 // Inclusive cumulative log-gates of the chunk in scan order (log2 units): G[r] of my rows; also the sum at the chunk's
 // middle (reference of the factorisation) and the total.  gsum: GROUPS x DK floats of shared memory; contains two barriers.
-template <int DK, typename T> __device__ __forceinline__ void cum_gates(float2 (&G)[ColLay<DK>::RPG], float2& ref, float2& tot, float* gsum, const T* g, int64_t stride_l,
+template <int DK, typename T> __device__ __forceinline__ void cum_gates(F2 (&G)[ColLay<DK>::RPG], F2& ref, F2& tot, float* gsum, Raw2<T> (&x)[ColLay<DK>::RPG],
                                                                         int n, int dir, float gate_norm, float clamp_min) {
     using CL = ColLay<DK>;
     const int pr = threadIdx.x % CL::PAIRS, gr = threadIdx.x / CL::PAIRS, r0 = gr * CL::RPG;
-    const float inv = gate_norm > 0.f ? 1.f / gate_norm : 0.f;
-    float2 x[CL::RPG];
+    const bool logits = gate_norm > 0.f, clamp = clamp_min == clamp_min;
+    if (r0 + CL::RPG > n) {
 #pragma unroll
-    for (int r = 0; r < CL::RPG; ++r) x[r] = r0 + r < n ? load2<T>(g + (r0 + r) * stride_l + 2 * pr) : make_float2(0.f, 0.f);
-    float2 run = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int rr = 0; rr < CL::RPG; ++rr) {
-        const int r = rr;
-        if (r0 + r < n) {
-            x[r].x = gate_log2<T>(x[r].x, gate_norm, inv, clamp_min);
-            x[r].y = gate_log2<T>(x[r].y, gate_norm, inv, clamp_min);
-        }
-        run.x += x[r].x; run.y += x[r].y;
-        G[r] = run;                                                      // inclusive prefix inside the group
+        for (int r = 0; r < CL::RPG; ++r) if (r0 + r >= n) x[r].open_gate(logits);
     }
-    *reinterpret_cast<float2*>(gsum + gr * DK + 2 * pr) = run;
-    __syncthreads();
-    float2 off = make_float2(0.f, 0.f), lo = off, hi = off;
-#pragma unroll
-    for (int o = 0; o < CL::GROUPS; ++o) {
-        const float2 s = *reinterpret_cast<const float2*>(gsum + o * DK + 2 * pr);
-        if (dir ? o > gr : o < gr) { off.x += s.x; off.y += s.y; }
-        if (o < CL::GROUPS / 2) { lo.x += s.x; lo.y += s.y; } else { hi.x += s.x; hi.y += s.y; }
-    }
-    __syncthreads();
-    ref = dir ? hi : lo;
-    tot = make_float2(lo.x + hi.x, lo.y + hi.y);
+    const F2 zero = f2_make(0.f, 0.f), one = f2_make(1.f, 1.f), nlog2e = f2_make(-tc::LOG2E, -tc::LOG2E);
+    const float ni = logits ? -1.f / gate_norm : 0.f;
+    const F2 ninv = f2_make(ni, ni);
+    F2 run = zero;
 #pragma unroll
     for (int r = 0; r < CL::RPG; ++r) {
-        if (dir) {                                                       // suffix of the group = its sum - exclusive prefix
-            G[r].x = run.x - G[r].x + x[r].x + off.x; G[r].y = run.y - G[r].y + x[r].y + off.y;
+        const F2 v = x[r].f2();
+        F2 g;
+        if (sizeof(T) == 2 && logits && !clamp) {                        // the models' form: -log2(1 + 2^(-x log2 e)) / norm
+            const F2 y = f2_mul(v, nlog2e), z = f2_add(f2_make(tc::ex2(f2_lo(y)), tc::ex2(f2_hi(y))), one);
+            g = f2_mul(f2_make(tc::lg2(f2_lo(z)), tc::lg2(f2_hi(z))), ninv);
         } else {
-            G[r].x += off.x; G[r].y += off.y;
+            g = r0 + r < n ? f2_make(gate_log2<T>(f2_lo(v), gate_norm, -ni, clamp_min), gate_log2<T>(f2_hi(v), gate_norm, -ni, clamp_min)) : zero;
         }
+        // inclusive prefix inside the group; the backward direction keeps the exclusive one (suffix = sum - exclusive prefix)
+        const F2 next = f2_add(run, g);
+        G[r] = dir ? run : next;
+        run = next;
     }
+    *reinterpret_cast<F2*>(gsum + gr * DK + 2 * pr) = run;
+    __syncthreads();
+    F2 sum = zero, before = zero, lo = zero;
+#pragma unroll
+    for (int o = 0; o < CL::GROUPS; ++o) {
+        if (o == gr) before = sum;
+        if (o == CL::GROUPS / 2) lo = sum;
+        sum = f2_add(sum, *reinterpret_cast<const F2*>(gsum + o * DK + 2 * pr));
+    }
+    __syncthreads();
+    const F2 minus = f2_make(-1.f, -1.f);
+    ref = dir ? f2_fma(lo, minus, sum) : lo;
+    tot = sum;
+    // forward: what the groups before mine add; backward: total minus everything before the row
+    const F2 rest = f2_fma(before, minus, sum);
+#pragma unroll
+    for (int r = 0; r < CL::RPG; ++r) G[r] = dir ? f2_fma(G[r], minus, rest) : f2_add(G[r], before);
 }
 
 // Largest |G - r| (log2 units) of the factorised form.  The exponent's own rounding grows with it (2^-24 |G|): 24 keeps it
@@ -245,6 +285,7 @@ template <int DK, int DV, int SC> __device__ __forceinline__ void load_state(uin
 #pragma unroll 4
     for (int i0 = 0; i0 < DK * TPR; i0 += NT) {
         const int i = i0 + threadIdx.x, d = i / TPR, v = i % TPR;
+        if (DK * TPR < NT && i >= DK * TPR) break;                       // whole warps
         const float4 x = st ? __ldcg(reinterpret_cast<const float4*>(st) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
         const float s = scale[d];
         uint32_t ta[SC], tb[SC];
