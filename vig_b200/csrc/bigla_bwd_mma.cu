@@ -74,6 +74,7 @@ __global__ void __launch_bounds__(NT) bwd_states_mma_kernel(const __grid_constan
 #pragma unroll
             for (int i = 0; i < SC; ++i) *reinterpret_cast<uint32_t*>(smem + SM::Q + i * C * Pitch<DK>::B + (r0 + r) * Pitch<DK>::B + pr * 4) = t[i];
         }
+        wait_raw();
         __syncthreads();
         const int which = warp >> 2, mt = (warp & 3) % MT, wn = (warp & 3) / MT;          // warps 0 - 3: S, 4 - 7: Z
         float acc[NTL][4];
@@ -175,6 +176,17 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 1 : 2) bwd_grads_mma_kern
     const uint32_t aK = sb + SM::K + 16 * w * PK + frag_rows<PK>(lane);
     const uint32_t bV = sb + SM::V + frag_cols<PV>(lane), bO = sb + SM::O + frag_cols<PV>(lane), bQ = sb + SM::Q + frag_cols<PK>(lane);
     const uint32_t tK = sb + SM::K + frag_rows<PK>(lane), tQ = sb + SM::Q + frag_rows<PK>(lane), tO = sb + SM::O + frag_rows<PV>(lane);
+    const bool have_states = p.nchunk > 1;
+    if (have_states) {                                                   // both directions' states on their way to L2 while the tiles are made
+        constexpr int LINES = DK * DV * 4 / 128;
+        for (int i = threadIdx.x; i < 4 * LINES; i += NT) {
+            const int dir = i / (2 * LINES), which = i / LINES % 2;
+            if (p.dir_mask & (1 << dir)) {
+                const float* at = (which ? p.ws_Z : p.ws_S) + (((size_t)bh * p.nchunk + c) * 2 + dir) * DK * DV + i % LINES * 32;
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(at));
+            }
+        }
+    }
     float dv[DV / 8][4];
 #pragma unroll
     for (int i = 0; i < DV / 8; ++i)
@@ -183,7 +195,6 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 1 : 2) bwd_grads_mma_kern
     F2 dqt[RPG], dkt[RPG];
 #pragma unroll
     for (int r = 0; r < RPG; ++r) dqt[r] = dkt[r] = f2_make(0.f, 0.f);
-    const bool have_states = p.nchunk > 1;
 #pragma unroll 1
     for (int dir = 0; dir < 2; ++dir) {
         if (!(p.dir_mask & (1 << dir))) continue;
@@ -220,6 +231,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 1 : 2) bwd_grads_mma_kern
 #pragma unroll
                 for (int i = 0; i < SC; ++i) *reinterpret_cast<uint32_t*>(smem + SM::K + i * TK + (r0 + r) * PK + pr * 4) = t[i];
             }
+            wait_raw();
             if (__syncthreads_or(!fine)) {                               // left to the exact kernel, outputs included
                 if (threadIdx.x == 0) p.flags[(size_t)bh * p.nchunk + c] = 1;
                 return;

@@ -107,7 +107,8 @@ __device__ __forceinline__ float through_gate(float dg, float x, float gate_norm
 // 2^x: the hardware form for 16-bit callers, the 2-ulp one for fp32
 template <typename T> __device__ __forceinline__ float ex2_t(float x) { return sizeof(T) == 4 ? exp2f(x) : tc::ex2(x); }
 
-// [C x COLS] rows of a strided tensor -> TERMS bf16 tiles (rows past n are zero); tile t at dst + t * C * pitch
+// [C x COLS] rows of a strided tensor -> TERMS bf16 tiles (rows past n are zero); tile t at dst + t * C * pitch.  One term is
+// copied asynchronously: wait_raw() before the barrier that publishes the tiles.
 template <typename T, int COLS, int TERMS> __device__ __forceinline__ void load_raw(uint8_t* dst, const T* src, int64_t stride_l, int n) {
     constexpr uint32_t P = Pitch<COLS>::B;
     if constexpr (sizeof(T) == 2 && TERMS == 1) {
@@ -115,9 +116,8 @@ template <typename T, int COLS, int TERMS> __device__ __forceinline__ void load_
 #pragma unroll
         for (int i0 = 0; i0 < C * VPR; i0 += NT) {
             const int i = i0 + threadIdx.x, r = i / VPR, v = i % VPR;
-            uint4 x = make_uint4(0u, 0u, 0u, 0u);
-            if (r < n) x = __ldg(reinterpret_cast<const uint4*>(src + r * stride_l) + v);
-            *reinterpret_cast<uint4*>(dst + r * P + v * 16) = x;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(tc::smem_u32(dst + r * P + v * 16)), "l"(src + (r < n ? r : 0) * stride_l + v * 8),
+                         "r"(r < n ? 16 : 0) : "memory");
         }
     } else {
         constexpr int PPR = COLS / 4;                                  // groups of four values per row
@@ -139,6 +139,8 @@ template <int DK> struct ColLay {
     static constexpr int PAIRS = DK / 2, GROUPS = NT / PAIRS, RPG = C / GROUPS;
     static_assert(PAIRS <= NT && RPG >= 1, "head size");
 };
+
+__device__ __forceinline__ void wait_raw() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Two neighbouring values as they lie in memory.  ``open_gate``: a pair that stands for log-gate 0 (rows past the end) --
 // the logit +inf, or the log-gate 0 itself.
