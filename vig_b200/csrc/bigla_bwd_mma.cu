@@ -94,8 +94,7 @@ __global__ void __launch_bounds__(NT) bwd_states_mma_kernel(const __grid_constan
 }
 
 // ---- scan over chunks: local states -> entering states, in place.  S in scan order, Z against it. ---------------------
-// A thread owns four neighbouring state values; the loads of PF chunks are in flight ahead of the dependent chain.
-__global__ void __launch_bounds__(256) bwd_scan_kernel(const __grid_constant__ BwdParams p) {
+__global__ void __launch_bounds__(256, 2) bwd_scan_kernel(const __grid_constant__ BwdParams p) {
     const int per = p.dk * p.dv / 4;
     const int64_t it = (int64_t)blockIdx.x * 256 + threadIdx.x;
     const int e = (int)(it % per);
@@ -105,31 +104,10 @@ __global__ void __launch_bounds__(256) bwd_scan_kernel(const __grid_constant__ B
     const int dir = p.dir_mask == 3 ? (int)(r % 2) : p.dir_mask - 1;
     const int64_t bh = r / ndir;
     if (bh >= (int64_t)p.B * p.H) return;
-    const int d = e * 4 / p.dv;
-    float4* ws = reinterpret_cast<float4*>(which ? p.ws_Z : p.ws_S);
     const bool descending = (dir != 0) != (which != 0);
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    constexpr int PF = 8;
-    for (int cc0 = 0; cc0 < p.nchunk; cc0 += PF) {
-        float4 u[PF];
-        float g[PF];
-        size_t at[PF];
-#pragma unroll
-        for (int i = 0; i < PF; ++i) {
-            const int cc = min(cc0 + i, p.nchunk - 1);
-            const size_t slot = ((size_t)bh * p.nchunk + (descending ? p.nchunk - 1 - cc : cc)) * 2 + dir;
-            at[i] = slot * per + e;
-            u[i] = __ldcg(ws + at[i]);
-            g[i] = __ldcg(p.ws_decay + slot * p.dk + d);
-        }
-#pragma unroll
-        for (int i = 0; i < PF; ++i) {
-            if (cc0 + i >= p.nchunk) break;
-            ws[at[i]] = acc;
-            const float a = exp2f(g[i]);
-            acc.x = fmaf(acc.x, a, u[i].x); acc.y = fmaf(acc.y, a, u[i].y); acc.z = fmaf(acc.z, a, u[i].z); acc.w = fmaf(acc.w, a, u[i].w);
-        }
-    }
+    float gsum = 0.f;
+    scan_states(reinterpret_cast<float4*>(which ? p.ws_Z : p.ws_S), p.ws_decay, per, e, p.dk, e * 4 / p.dv, p.nchunk, make_float4(0.f, 0.f, 0.f, 0.f), gsum,
+                [&](int cc) { return ((size_t)bh * p.nchunk + (descending ? p.nchunk - 1 - cc : cc)) * 2 + dir; }, [](float g) { return exp2f(g); });
 }
 
 // ---- chunk gradients -----------------------------------------------------------------------------------------------

@@ -130,8 +130,20 @@ __global__ void __launch_bounds__(NT) bwd_chunk_grads(BwdParams p, int flagged_o
     float* sdv = sdo + CH * DV;
     const bool have_states = !flagged_only || p.nchunk > 1;          // the tensor-core form leaves the states of a lone chunk unwritten (zero)
     const int items = p.nchunk * p.B * p.H;
-    for (int item = blockIdx.x; item < items; item += gridDim.x) {
-    if (flagged_only && !p.flags[item]) continue;
+    for (int item = blockIdx.x, look = 0; item < items; item += gridDim.x, ++look) {
+    if (flagged_only) {
+        // the flags of my next NT items at once: a chain of dependent loads otherwise
+        if (look % NT == 0) {
+            const int64_t mine = item + (int64_t)threadIdx.x * gridDim.x;
+            if (!__syncthreads_or(mine < items && p.flags[mine])) {
+                const int64_t next = item + (int64_t)(NT - 1) * gridDim.x;
+                if (next >= items) break;
+                item = (int)next; look += NT - 1;
+                continue;
+            }
+        }
+        if (!p.flags[item]) continue;
+    }
     const int c = item % p.nchunk, bh = item / p.nchunk, b = bh / p.H, h = bh % p.H;
     const int t0 = c * CH, n = min(CH, p.L - t0);
     load_tile<DK, T>(sq, p.q, p.sq, b, h, t0, n);

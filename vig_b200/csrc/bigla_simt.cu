@@ -98,45 +98,23 @@ __global__ void __launch_bounds__(NT) bigla_simt_chunk_state(BiglaParams p) {
     }
 }
 
-// Phase B: one thread per state element, sequential over chunks in scan order.
-__global__ void __launch_bounds__(NT) bigla_simt_state_scan(BiglaParams p) {
-    const int DKDV = p.dk * p.dv;
-    const int per = (DKDV + NT - 1) / NT;              // CTAs per (bh, dir)
-    const int blk = blockIdx.x;
-    const int part = blk % per, dir = (blk / per) % 2, bh = blk / (per * 2);
-    if (!(p.dir_mask & (1 << dir))) return;
-    const int e = part * NT + threadIdx.x;
-    if (e >= DKDV) return;
-    const int d = e / p.dv;
+// Phase B: one thread per four neighbouring state elements, sequential over chunks in scan order.
+__global__ void __launch_bounds__(NT, 2) bigla_simt_state_scan(BiglaParams p) {
+    const int per = p.dk * p.dv / 4;
+    const int64_t it = (int64_t)blockIdx.x * NT + threadIdx.x;
+    const int e = (int)(it % per), dir = (int)(it / per % 2);
+    const int64_t bh = it / per / 2;
+    if (bh >= (int64_t)p.B * p.H || !(p.dir_mask & (1 << dir))) return;
+    const int d = e * 4 / p.dv;
     const float* init = dir ? p.init_b : p.init_f;
-    float S = init ? init[(size_t)bh * DKDV + e] : 0.f;
+    const size_t at = (size_t)bh * per * 4 + e * 4;
+    float4 S = init ? make_float4(init[at], init[at + 1], init[at + 2], init[at + 3]) : make_float4(0.f, 0.f, 0.f, 0.f);
     float gsum = 0.f;
-    constexpr int PF = 4;                               // loads of PF chunks are in flight before the dependent chain runs
-    for (int cc0 = 0; cc0 < p.nchunk; cc0 += PF) {
-        float u[PF], g[PF];
-        float* slotp[PF];
-#pragma unroll
-        for (int i = 0; i < PF; ++i) {
-            const int cc = cc0 + i;
-            const int c = dir ? p.nchunk - 1 - cc : cc;
-            const size_t slot = ((size_t)bh * p.nchunk + (cc < p.nchunk ? c : 0)) * 2 + dir;
-            slotp[i] = p.ws_state + slot * DKDV + e;
-            u[i] = cc < p.nchunk ? __ldcg(slotp[i]) : 0.f;
-            g[i] = cc < p.nchunk ? __ldcg(p.ws_decay + slot * p.dk + d) : 0.f;
-        }
-#pragma unroll
-        for (int i = 0; i < PF; ++i) {
-            if (cc0 + i < p.nchunk) {
-                *slotp[i] = S;                          // state entering chunk c
-                S = fmaf(S, __expf(g[i]), u[i]);
-                gsum += g[i];
-            }
-        }
-    }
-    float* fin = dir ? p.final_b : p.final_f;
-    if (fin) fin[(size_t)bh * DKDV + e] = S;
+    S = scan_states(reinterpret_cast<float4*>(p.ws_state), p.ws_decay, per, e, p.dk, d, p.nchunk, S, gsum,
+                    [&](int cc) { return ((size_t)bh * p.nchunk + (dir ? p.nchunk - 1 - cc : cc)) * 2 + dir; }, [](float g) { return __expf(g); });
+    if (float* fin = dir ? p.final_b : p.final_f) { fin[at] = S.x; fin[at + 1] = S.y; fin[at + 2] = S.z; fin[at + 3] = S.w; }
     float* ld = dir ? p.logdecay_b : p.logdecay_f;
-    if (ld && (e % p.dv) == 0) ld[(size_t)bh * p.dk + d] = gsum;
+    if (ld && e * 4 % p.dv == 0) ld[(size_t)bh * p.dk + d] = gsum;
 }
 
 template <int DK, int DV, typename T>
@@ -201,8 +179,7 @@ int launch_typed(const BiglaParams& p, cudaStream_t stream) {
         cudaError_t e = cudaFuncSetAttribute(kA, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smA);
         if (e != cudaSuccess) return (int)e;
         kA<<<grid, NT, smA, stream>>>(p);
-        const int per = (DK * DV + NT - 1) / NT;
-        bigla_simt_state_scan<<<BH * 2 * per, NT, 0, stream>>>(p);
+        if (int s = bigla_scan_launch(p, stream)) return s;
     }
     if (p.o) {
         const size_t smC = (size_t)CH * (3 * DK + 2 * DV) * sizeof(float);
@@ -231,8 +208,8 @@ size_t bigla_simt_workspace(int B, int H, int L, int dk, int dv) {
 }
 
 int bigla_scan_launch(const BiglaParams& p, cudaStream_t stream) {
-    const int per = (p.dk * p.dv + NT - 1) / NT;
-    bigla_simt_state_scan<<<p.B * p.H * 2 * per, NT, 0, stream>>>(p);
+    const int64_t threads = (int64_t)p.B * p.H * 2 * (p.dk * p.dv / 4);
+    bigla_simt_state_scan<<<(unsigned)((threads + NT - 1) / NT), NT, 0, stream>>>(p);
     return (int)cudaGetLastError();
 }
 

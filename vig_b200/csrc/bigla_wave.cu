@@ -812,7 +812,11 @@ bool bigla_wave_supported(const BiglaParams& p) {
 bool bigla_wave_preferred(const BiglaParams& p) {
     const int sms = wave_sm_count();
     const int ndir = p.dir_mask == 3 ? 2 : 1;
-    return sms > 0 && p.L > W_SEG_CHUNKS_MIN * CHUNK && (long long)p.B * p.H * ndir >= sms;
+    // Below one chain per SM this form still takes the time of one chain, the segment-parallel one time in proportion to the
+    // work: 96 chains of 4096 tokens, dk = 64, 110 us against 142; 48 chains 107 against 79.  (dk = 32: 192 chains of 3136, 125
+    // against 175.)
+    const long long chains = (long long)p.B * p.H * ndir;
+    return sms > 0 && p.L > W_SEG_CHUNKS_MIN * CHUNK && chains * 16 >= sms * (p.dk == 64 ? 9ll : 13ll);
 }
 
 // Counters (ticket, chain progress, chunk flags) followed by the state mailboxes.

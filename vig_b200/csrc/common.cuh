@@ -57,6 +57,46 @@ template <typename T> __device__ __forceinline__ float sigmoid_t(float x) {
     return fmaf(0.5f, t, 0.5f);
 }
 
+// Scan of states over chunks, four neighbouring values of one key channel: in place, local states become the states that
+// enter each chunk.  slot(i): index of the i-th chunk in scan order; the loads of 8 to 16 chunks are in flight ahead of the
+// dependent chain (with 4, long scans took 1.4 to 1.7 times as long: few threads, each waiting).  Returns the state after the last chunk; gsum: summed log-gates of the channel.
+template <typename Slot, typename Decay>
+__device__ __forceinline__ float4 scan_states(float4* ws, const float* decay, int per, int e, int dk, int d, int nchunk, float4 S, float& gsum, Slot slot, Decay factor) {
+    constexpr int PF = 8;
+    float4 u[2][PF];
+    float g[2][PF];
+    auto fetch = [&](int c0, int b) {
+#pragma unroll
+        for (int i = 0; i < PF; ++i) {
+            if (c0 + i < nchunk) {
+                const size_t s = slot(c0 + i);
+                u[b][i] = __ldcg(ws + s * per + e);
+                g[b][i] = __ldcg(decay + s * dk + d);
+            }
+        }
+    };
+    auto run = [&](int c0, int b) {
+#pragma unroll
+        for (int i = 0; i < PF; ++i) {
+            if (c0 + i < nchunk) {
+                __stcg(ws + slot(c0 + i) * per + e, S);
+                const float a = factor(g[b][i]);
+                gsum += g[b][i];
+                S.x = fmaf(S.x, a, u[b][i].x); S.y = fmaf(S.y, a, u[b][i].y); S.z = fmaf(S.z, a, u[b][i].z); S.w = fmaf(S.w, a, u[b][i].w);
+            }
+        }
+    };
+    fetch(0, 0);
+    for (int c0 = 0; c0 < nchunk; c0 += 2 * PF) {
+        if (c0 + PF < nchunk) fetch(c0 + PF, 1);
+        run(c0, 0);
+        if (c0 + PF >= nchunk) break;
+        if (c0 + 2 * PF < nchunk) fetch(c0 + 2 * PF, 0);
+        run(c0 + PF, 1);
+    }
+    return S;
+}
+
 // Programmatic dependent launch.  A kernel that calls pdl_wait() before it touches what an earlier kernel wrote may be launched
 // while that kernel still runs (launch_chained); pdl_launch() lets the next kernel of the stream do the same.  Both do nothing
 // in an ordinary launch.  A kernel allocates tensor memory only after pdl_wait(): earlier it could hold what a kernel it
