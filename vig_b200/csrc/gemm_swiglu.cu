@@ -266,46 +266,47 @@ __global__ void __launch_bounds__(GS_THREADS, 1) linear_swiglu_kernel(const __gr
 
 
 // ---------------------------------------------------------------------------------------------------
-// Weight-stationary form, for K <= 192 and I % 128 == 0 (the shipped MLP shapes at widths up to 192) and many rows.
+// Weight-stationary form, for K <= 384 and many rows.
 //
-// A 128x128x16 MMA takes ~80-130 cycles here where a 128x256x16 one takes ~130: at N = 128 the tensor pipe runs at half its
-// rate.  This form multiplies a 128-row tile of x by 128 gate rows and their 128 y rows at once (N = 256).  A persistent CTA
-// owns ONE block of 128 features for the whole launch: its [256 x K] slice of W (96 KB at K = 192) is loaded once and stays
-// in shared memory, the x tiles stream through a two-stage ring (48 KB each), the accumulator [128 x 256] takes half of
-// tensor memory and the two halves double-buffer (tile t+1 is multiplied while tile t is read out).  The CTAs that hold
-// the feature blocks of the same row tile have consecutive block indices and run in step, so a tile of x comes from DRAM
-// once and from L2 for the others.  (An earlier N = 256 form kept 256 rows of x resident and streamed the weights through
-// a ring that held exactly one block's boxes: every block began by waiting for reloads, 134 us; before that the N = 128
-// form, 155-165 us.)
-constexpr int WB_FEAT = 128;                         // features per block
-constexpr int WB_BOX_BYTES = 2 * WB_FEAT * BK * 2;   // one k box of the CTA's weight slice: 128 gate rows + 128 y rows, 32 KB
-constexpr int WB_XSTAGES = 2;
+// A 128x128x16 MMA takes ~80-130 cycles here where a 128x256x16 one takes ~130.  A persistent CTA owns ONE block of FEAT
+// features for the whole launch: its [2 FEAT x K] slice of W (gate rows and their y rows, 96 KB) is loaded once and stays in
+// shared memory, the x tiles stream through a ring of six [128 x 64] boxes (96 KB: two tiles at K = 192, one at K = 384), the
+// accumulator [128 x 2 FEAT] is double-buffered in tensor memory (tile t+1 is multiplied while tile t is read out).  FEAT =
+// 128 (N = 256) up to K = 192, 64 (N = 128) up to K = 384, where the slice of 128 features would leave no room for x.  The
+// CTAs that hold the feature blocks of the same row tile have consecutive block indices and run in step, so a tile of x comes
+// from DRAM once and from L2 for the others.  (An earlier N = 256 form kept 256 rows of x resident and streamed the weights
+// through a ring that held exactly one block's boxes: every block began by waiting for reloads, 134 us at M = 262144, K = 192,
+// I = 512; before that the N = 128 form, 155-165 us; this one 113.)
+constexpr int WB_XBOXES = 6;
 
 struct GsWideMaps { CUtensorMap x, w, o; };
 
 // grid = row_groups * nblocks CTAs; CTA i holds feature block i % nblocks and walks row tiles i / nblocks, + row_groups, ...
-template <typename T>
+template <typename T, int FEAT>
 __global__ void __launch_bounds__(GS_THREADS, 1) linear_swiglu_wide_kernel(const __grid_constant__ GsWideMaps maps, int M, int I, int KB, int nblocks,
                                                                            int row_groups, int32_t* status) {
     extern __shared__ uint8_t gs_smem_raw[];
     uint8_t* smem = gs_smem_raw + ((1024u - (smem_u32(gs_smem_raw) & 1023u)) & 1023u);
     const uint32_t sbase = smem_u32(smem);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t off_x = (uint32_t)KB * WB_BOX_BYTES;                     // after the weight slice
-    const uint32_t x_stage = (uint32_t)KB * A_BOX_BYTES;
-    const uint32_t off_out = off_x + WB_XSTAGES * x_stage;
+    constexpr uint32_t W_BOX = 2 * FEAT * BK * 2;                           // one k box of the weight slice: FEAT gate rows + FEAT y rows
+    const uint32_t off_x = (uint32_t)KB * W_BOX;                            // after the weight slice
+    // boxes handed over together: a whole tile at K <= 192 (a barrier costs 200-400 cycles to ask about), one by one above
+    const int G = FEAT == 128 ? KB : 1;
+    const uint32_t NST = FEAT == 128 ? 2u : (uint32_t)WB_XBOXES;
+    const uint32_t off_out = off_x + WB_XBOXES * A_BOX_BYTES;
     const uint32_t off_bar = off_out + OUT_STAGE_BYTES;
-    // barriers: weight slice full; x stages full / empty; accumulator halves full / empty
+    // barriers: weight slice full; x boxes full / empty; accumulator halves full / empty
     const uint32_t bar_w = sbase + off_bar;
-    const uint32_t bar_x_full = bar_w + 8, bar_x_empty = bar_x_full + 8 * WB_XSTAGES;
-    const uint32_t bar_acc_full = bar_x_empty + 8 * WB_XSTAGES, bar_acc_empty = bar_acc_full + 16;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + off_bar + 8 * (1 + 2 * WB_XSTAGES + 4));
+    const uint32_t bar_x_full = bar_w + 8, bar_x_empty = bar_x_full + 8 * WB_XBOXES;
+    const uint32_t bar_acc_full = bar_x_empty + 8 * WB_XBOXES, bar_acc_empty = bar_acc_full + 16;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + off_bar + 8 * (1 + 2 * WB_XBOXES + 4));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const Waiter waiter{abort_flag, status};
 
     if (tid == 0) {
         mbar_init(bar_w, 1);
-        for (int i = 0; i < WB_XSTAGES; ++i) { mbar_init(bar_x_full + 8 * i, 1); mbar_init(bar_x_empty + 8 * i, 1); }
+        for (int i = 0; i < WB_XBOXES; ++i) { mbar_init(bar_x_full + 8 * i, 1); mbar_init(bar_x_empty + 8 * i, 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(bar_acc_full + 8 * b, 1); mbar_init(bar_acc_empty + 8 * b, GS_EPI_WARPS / 2); }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -321,24 +322,25 @@ __global__ void __launch_bounds__(GS_THREADS, 1) linear_swiglu_wide_kernel(const
 
     const int ntiles = (M + 127) / 128;
     const int nb = (int)blockIdx.x % nblocks, rg = (int)blockIdx.x / nblocks;
-    constexpr uint32_t IDESC = make_idesc(Pk<T>::FMT, 0, 0, 128, 256);
+    constexpr uint32_t IDESC = make_idesc(Pk<T>::FMT, 0, 0, 128, 2 * FEAT);
 
     if (warp == 0) {
         if (lane == 0) {                          // ---- TMA producer -------------------------------------------
-            mbar_expect_tx(bar_w, (uint32_t)KB * WB_BOX_BYTES);
+            mbar_expect_tx(bar_w, (uint32_t)KB * W_BOX);
             for (int kb = 0; kb < KB; ++kb) {
-                tma_load_2d(sbase + kb * WB_BOX_BYTES, &maps.w, kb * BK, nb * WB_FEAT, bar_w);                          // gate rows
-                tma_load_2d(sbase + kb * WB_BOX_BYTES + WB_FEAT * BK * 2, &maps.w, kb * BK, I + nb * WB_FEAT, bar_w);   // matching y rows
+                tma_load_2d(sbase + kb * W_BOX, &maps.w, kb * BK, nb * FEAT, bar_w);                           // gate rows
+                tma_load_2d(sbase + kb * W_BOX + FEAT * BK * 2, &maps.w, kb * BK, I + nb * FEAT, bar_w);       // matching y rows
             }
             uint32_t st = 0, phase = 0;
-            for (int tile = rg; tile < ntiles; tile += row_groups) {
-                waiter.wait(bar_x_empty + 8 * st, phase ^ 1u);            // the MMAs of the tile two back have read this stage
-                if (*abort_flag) break;
-                mbar_expect_tx(bar_x_full + 8 * st, x_stage);
-                for (int kb = 0; kb < KB; ++kb)
-                    tma_load_2d(sbase + off_x + st * x_stage + kb * A_BOX_BYTES, &maps.x, kb * BK, tile * 128, bar_x_full + 8 * st);
-                if (++st == WB_XSTAGES) { st = 0; phase ^= 1u; }
-            }
+            for (int tile = rg; tile < ntiles; tile += row_groups)
+                for (int kb = 0; kb < KB; kb += G) {
+                    waiter.wait(bar_x_empty + 8 * st, phase ^ 1u);        // the MMAs of the group a ring back have read it
+                    if (*abort_flag) break;
+                    mbar_expect_tx(bar_x_full + 8 * st, G * A_BOX_BYTES);
+                    for (int g = 0; g < G; ++g)
+                        tma_load_2d(sbase + off_x + (st * G + g) * A_BOX_BYTES, &maps.x, (kb + g) * BK, tile * 128, bar_x_full + 8 * st);
+                    if (++st == NST) { st = 0; phase ^= 1u; }
+                }
         }
     } else if (warp == 1) {                       // ---- MMA issuer ---------------------------------------------
         const bool issuer = lane == 0;
@@ -349,34 +351,39 @@ __global__ void __launch_bounds__(GS_THREADS, 1) linear_swiglu_wide_kernel(const
         for (int tile = rg; tile < ntiles; tile += row_groups, ++it) {
             const uint32_t buf = it & 1u;
             if (!pre_acc) waiter.wait_lite(bar_acc_empty + 8 * buf, ((it >> 1) & 1u) ^ 1u);   // the epilogue has read this half out
-            if (!pre_x) waiter.wait_lite(bar_x_full + 8 * st, phase);
             if (*abort_flag) break;
             tc_fence_after();
-            // asked before this tile's MMAs, answered while they are issued: the next tile's stage and accumulator half
-            const uint32_t st_next = st + 1 == WB_XSTAGES ? 0u : st + 1, ph_next = st + 1 == WB_XSTAGES ? phase ^ 1u : phase;
-            pre_x = mbar_test_wait(bar_x_full + 8 * st_next, ph_next);
+            // asked before this tile's MMAs, answered while they are issued: the next tile's accumulator half; and before each
+            // box's MMAs the next box
             pre_acc = mbar_test_wait(bar_acc_empty + 8 * (buf ^ 1u), (((it + 1) >> 1) & 1u) ^ 1u);
             const uint32_t d = tmem + buf * 256u;
-            for (int kb = 0; kb < KB; ++kb) {
-                const uint32_t a_lo = x_lo0 + (st * x_stage >> 4) + (uint32_t)kb * (A_BOX_BYTES >> 4);
-                const uint32_t b_lo = w_lo0 + (uint32_t)kb * (WB_BOX_BYTES >> 4);
+            for (int kb = 0; kb < KB; kb += G) {
+                if (!pre_x) waiter.wait_lite(bar_x_full + 8 * st, phase);
+                tc_fence_after();
+                const uint32_t st_next = st + 1 == NST ? 0u : st + 1, ph_next = st + 1 == NST ? phase ^ 1u : phase;
+                pre_x = mbar_test_wait(bar_x_full + 8 * st_next, ph_next);
+                for (int g = 0; g < G; ++g) {
+                    const uint32_t a_lo = x_lo0 + (st * G + g) * (A_BOX_BYTES >> 4);
+                    const uint32_t b_lo = w_lo0 + (uint32_t)(kb + g) * (W_BOX >> 4);
 #pragma unroll
-                for (uint32_t k4 = 0; k4 < 4; ++k4) { if (issuer) tc_mma(d, a_lo + 2 * k4, b_lo + 2 * k4, IDESC, (kb | k4) > 0 ? 1u : 0u); }
+                    for (uint32_t k4 = 0; k4 < 4; ++k4) { if (issuer) tc_mma(d, a_lo + 2 * k4, b_lo + 2 * k4, IDESC, (kb | g | k4) > 0 ? 1u : 0u); }
+                }
+                if (issuer) tc_commit(bar_x_empty + 8 * st);
+                st = st_next; phase = ph_next;
             }
-            if (issuer) { tc_commit(bar_x_empty + 8 * st); tc_commit(bar_acc_full + 8 * buf); }
-            st = st_next; phase = ph_next;
+            if (issuer) tc_commit(bar_acc_full + 8 * buf);
         }
     } else {                                      // ---- epilogue: silu(gate) * y -> out ----------------------------
         // Two sets of eight warps take alternate tiles (set = accumulator half), so a warp has two tile periods for its
-        // [32 rows x 64 features]: the epilogue of a tile is a chain of latencies (accumulator ready -> TMEM load -> 32 sigmoids
+        // [32 rows x FEAT / 2 features]: the epilogue of a tile is a chain of latencies (accumulator ready -> TMEM load -> 32 sigmoids
         // -> box -> store, ~3 k cycles) longer than the tile's MMAs, and with all sixteen warps on every tile it set the pace.
         const int ew = warp - 2;                  // 0..15
         const uint32_t set = (uint32_t)ew >> 3;   // tiles of which parity / which accumulator half
-        const int fh = (ew >> 2) & 1;             // which 64 of the block's 128 features (taken as two halves of 32)
+        const int fh = (ew >> 2) & 1;             // which half of the block's features (128: taken as two pieces of 32)
         const uint32_t lane_base = (uint32_t)(32 * (warp & 3)) << 16;   // a warp reads the TMEM lanes of its quarter
         uint8_t* my_row = smem + off_out + ew * OUT_BOX_BYTES + lane * 64;
         const uint32_t box_u32 = sbase + off_out + ew * OUT_BOX_BYTES;
-        const uint32_t acc = tmem + lane_base + set * 256u + 64u * fh;
+        const uint32_t acc = tmem + lane_base + set * 256u + (FEAT / 2) * fh;
         uint32_t it = 0, uses = 0;
         for (int tile = rg; tile < ntiles; tile += row_groups, ++it) {
             if ((it & 1u) != set) continue;
@@ -385,22 +392,24 @@ __global__ void __launch_bounds__(GS_THREADS, 1) linear_swiglu_wide_kernel(const
             if (*abort_flag) break;
             tc_fence_after();
             const int row0 = tile * 128 + 32 * (warp & 3);
-            const int col0 = nb * WB_FEAT + 64 * fh;
+            const int col0 = nb * FEAT + (FEAT / 2) * fh;
             float g[32], y[32];
             uint32_t pk[16];
             tc_ld32(acc, g);
-            tc_ld32(acc + WB_FEAT, y);
+            tc_ld32(acc + FEAT, y);
             tc_wait_ld();
-            swiglu_pack<T>(g, y, pk);
-            tc_ld32(acc + 32, g);
-            tc_ld32(acc + WB_FEAT + 32, y);
-            tc_wait_ld();
+            if constexpr (FEAT == 128) {
+                swiglu_pack<T>(g, y, pk);
+                tc_ld32(acc + 32, g);
+                tc_ld32(acc + FEAT + 32, y);
+                tc_wait_ld();
+            }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_plain(bar_acc_empty + 8 * set);   // the accumulator is in registers: the MMA warp may refill it
-            send_box(my_row, box_u32, pk, &maps.o, col0, row0, row0 < M, lane);
+            if constexpr (FEAT == 128) send_box(my_row, box_u32, pk, &maps.o, col0, row0, row0 < M, lane);
             swiglu_pack<T>(g, y, pk);
-            send_box(my_row, box_u32, pk, &maps.o, col0 + 32, row0, row0 < M, lane);
+            send_box(my_row, box_u32, pk, &maps.o, col0 + FEAT / 2 - 32, row0, row0 < M, lane);
         }
         if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // every store has landed before the CTA exits
     }
@@ -435,10 +444,24 @@ extern "C" int vig_linear_swiglu_supported(int64_t M, int K, int I, int dtype) {
     return tc::encode_fn() != nullptr;
 }
 
-// Measured on B200 against cuBLAS + the SwiGLU kernel: 1.5-1.7x faster while two 128-row subtiles of x fit in shared
-// memory (K <= 192: the weights are then streamed from L2 once per 256 rows), slower at K = 384.
+static int wide_feat(int K) { return K <= 192 ? 128 : 64; }
+// Whether the weight-stationary form has rows enough: a few row tiles for each CTA of a feature block.
+static bool wide_takes(int64_t M, int K, int I, int sms) {
+    const int F = wide_feat(K);
+    if (K > 384 || I % F || I / F > sms) return false;
+    return (M + 127) / 128 >= (K <= 192 ? 2 * (int64_t)sms : 8 * (int64_t)(sms / (I / F)));
+}
+static int sm_count() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    return sms;
+}
+
+// Measured on B200 against cuBLAS + the SwiGLU kernel: 1.5-1.7x faster at K <= 192; at K = 384 where the weight-stationary
+// form has rows enough: I = 1024, M = 7000 20 us against 19, 12544 29 / 32, 25088 51 / 66, 200704 351 / 474 (a box of x feeds
+// four N = 128 MMAs there, 320 cycles: the ring's depth against the load latency is the bound).
 extern "C" int vig_linear_swiglu_preferred(int64_t M, int K, int I, int dtype) {
-    return vig_linear_swiglu_supported(M, K, I, dtype) && (int64_t)256 * K * 2 <= MAX_A_BYTES;
+    return vig_linear_swiglu_supported(M, K, I, dtype) && ((int64_t)256 * K * 2 <= MAX_A_BYTES || wide_takes(M, K, I, sm_count()));
 }
 
 extern "C" int vig_linear_swiglu_fwd(const void* x, int64_t ldx, const void* w, void* out, int64_t ldo,
@@ -449,30 +472,29 @@ extern "C" int vig_linear_swiglu_fwd(const void* x, int64_t ldx, const void* w, 
     if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out)) & 15) return VIG_ERR_ALIGN;
     if (ldx < K || ldo < I || (ldx * 2) % 16 || (ldo * 2) % 16 || M >= (1ll << 31)) return VIG_ERR_ARG;
     const int KB = K / BK;
-    int dev = 0, sms = 0;
+    const int sms = sm_count();
+    if (!sms) return VIG_ERR_DEVICE;
     cudaError_t e;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return (int)e;
-    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return (int)e;
-    if (KB <= 3 && I % WB_FEAT == 0 && M >= 256 * (int64_t)sms && I / WB_FEAT <= sms) {
-        // weight-stationary form: N = 256 MMAs, a CTA per feature block and row group, when there are enough rows to fill the machine
+    if (wide_takes(M, K, I, sms)) {
+        const int F = wide_feat(K);
         GsWideMaps maps;
-        if (!tc::make_map_2d(&maps.x, x, M, K, ldx, 128, dtype) || !tc::make_map_2d(&maps.w, w, 2 * (int64_t)I, K, K, WB_FEAT, dtype) ||
+        if (!tc::make_map_2d(&maps.x, x, M, K, ldx, 128, dtype) || !tc::make_map_2d(&maps.w, w, 2 * (int64_t)I, K, K, F, dtype) ||
             !make_out_map(&maps.o, out, M, I, ldo, dtype)) return VIG_ERR_DEVICE;
-        const int smem = KB * WB_BOX_BYTES + WB_XSTAGES * KB * A_BOX_BYTES + OUT_STAGE_BYTES + 8 * (1 + 2 * WB_XSTAGES + 4) + 16 + 1024;
-        const int nblocks = I / WB_FEAT;
+        const int smem = KB * 2 * F * BK * 2 + WB_XBOXES * A_BOX_BYTES + OUT_STAGE_BYTES + 8 * (1 + 2 * WB_XBOXES + 4) + 16 + 1024;
+        const int nblocks = I / F;
         const int ntiles = (int)((M + 127) / 128);
         int row_groups = sms / nblocks;                        // CTAs per feature block
         if (row_groups > ntiles) row_groups = ntiles;
         const int grid = row_groups * nblocks;
-        if (dtype == VIG_DTYPE_BF16) {
-            auto kfn = linear_swiglu_wide_kernel<__nv_bfloat16>;
-            if ((e = tc::ensure_smem_attr(reinterpret_cast<const void*>(kfn), smem)) != cudaSuccess) return (int)e;
-            kfn<<<grid, GS_THREADS, smem, (cudaStream_t)stream>>>(maps, (int)M, I, KB, nblocks, row_groups, status_dev);
-        } else {
-            auto kfn = linear_swiglu_wide_kernel<__half>;
-            if ((e = tc::ensure_smem_attr(reinterpret_cast<const void*>(kfn), smem)) != cudaSuccess) return (int)e;
-            kfn<<<grid, GS_THREADS, smem, (cudaStream_t)stream>>>(maps, (int)M, I, KB, nblocks, row_groups, status_dev);
-        }
+#define VIG_WIDE(TT, FF)                                                                                                        \
+    {                                                                                                                           \
+        auto kfn = linear_swiglu_wide_kernel<TT, FF>;                                                                           \
+        if ((e = tc::ensure_smem_attr(reinterpret_cast<const void*>(kfn), smem)) != cudaSuccess) return (int)e;                  \
+        kfn<<<grid, GS_THREADS, smem, (cudaStream_t)stream>>>(maps, (int)M, I, KB, nblocks, row_groups, status_dev);            \
+    }
+        if (dtype == VIG_DTYPE_BF16) { if (F == 128) VIG_WIDE(__nv_bfloat16, 128) else VIG_WIDE(__nv_bfloat16, 64) }
+        else { if (F == 128) VIG_WIDE(__half, 128) else VIG_WIDE(__half, 64) }
+#undef VIG_WIDE
         return (int)cudaGetLastError();
     }
     GsMaps maps;
