@@ -279,6 +279,10 @@ VIG_API int vig_layernorm_act_add_rmsnorm_fwd(const void* x, const void* pre_bia
 VIG_API int vig_add_layernorm_fwd(const void* x, const void* residual, const void* w, const void* bias, void* y, void* sum_out, int64_t rows,
                                   int N, float eps, int act, int dtype, void* stream);
 
+/* y[b, c] = mean over l of x[b, l, c] (fp32 sums, rounded once): the models' pooling.  x contiguous [B, L, C], C * element size a
+ * multiple of 16. */
+VIG_API int vig_token_mean_fwd(const void* x, void* y, int B, int L, int C, int dtype, void* stream);
+
 /*
  * Space-to-depth of the input image for the stem's first convolution (`V2PatchEmbed`, classification/models/vig.py:
  * 650-651: kernel s+1, stride s, padding 1), which is then a 2x2 convolution over s x s pixel blocks:

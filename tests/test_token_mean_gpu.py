@@ -1,0 +1,16 @@
+"""Mean over tokens: one, few and many tokens a CTA, one to eight CTAs of a cluster, channel counts that do not fill 64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,L,C", [(1, 1, 64), (2, 49, 768), (3, 129, 192), (2, 300, 200), (1, 836, 96), (2, 5000, 192)])
+def test_token_mean(dtype, B, L, C):
+    from vig_b200 import ops
+    x = torch.randn(B, L, C, generator=torch.Generator(device="cuda").manual_seed(L), device="cuda").to(dtype) + 1
+    got, ref = ops.token_mean(x), x.double().mean(1)
+    # fp32 sums in blocks of a few dozen, one rounding to the type
+    tol = {torch.float32: 1e-6, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]
+    assert float((got.double() - ref).abs().max()) <= tol * float(ref.abs().max())

@@ -43,6 +43,7 @@ _SIGNATURES = {
     "vig_linear_add_rmsnorm_fwd": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_float, c_int, c_void_p, c_void_p]),
     "vig_layernorm_act_add_fwd": (c_int, [c_void_p] * 5 + [c_int64, c_void_p, c_int64, c_int, c_float, c_int, c_int, c_void_p]),
     "vig_layernorm_act_add_rmsnorm_fwd": (c_int, [c_void_p] * 5 + [c_int64, c_void_p, c_void_p, c_float, c_void_p, c_int64, c_int, c_float, c_int, c_int, c_void_p]),
+    "vig_token_mean_fwd": (c_int, [c_void_p] * 2 + [c_int] * 4 + [c_void_p]),
     "vig_chain_launches": (c_int, [c_int]),
     "vig_block_tail_supported": (c_int, [c_int64] + [c_int] * 4),
     "vig_block_tail_preferred": (c_int, [c_int64] + [c_int] * 4),

@@ -160,6 +160,7 @@ __global__ void __launch_bounds__(2 * TOK, seg_min_blocks<DK, DV, T, TOK>()) big
     const int64_t t0 = (int64_t)c * s.seglen;
     const int n = min(s.seglen, p.L - (int)t0), nb = (n + 15) / 16;
     const int pr = threadIdx.x % PAIRS, gr = threadIdx.x / PAIRS, r0 = gr * RPG;   // my channel pair, my rows
+    pdl_launch();                                                        // a chained successor may fetch its weights meanwhile
     const bool want_out = MODE != SEG_STATES && p.o;
     const bool fwd = p.dir_mask & 1, bwd = p.dir_mask & 2;
     F2 G[2][RPG], ref[2], tot[2];

@@ -43,6 +43,11 @@ Tensor layernorm(const Ctx& c, const Tensor& x, const Tensor& w, const Tensor& b
     ok(api.vig_layernorm_act_fwd(ptr(x), ptr(pre_bias), ptr(w), ptr(b), ptr(y), x.numel() / N, N, (float)eps, swish, c.code, c.stream), "vig_layernorm_act_fwd");
     return y;
 }
+Tensor token_mean(const Ctx& c, const Tensor& x) {
+    Tensor y = at::empty({x.size(0), x.size(2)}, x.options());
+    ok(api.vig_token_mean_fwd(ptr(x), ptr(y), x.size(0), x.size(1), x.size(2), c.code, c.stream), "vig_token_mean_fwd");
+    return y;
+}
 // swiglu(x W^T): one kernel where it is the faster one, GEMM + activation kernel otherwise
 Tensor mlp_in(const Ctx& c, const Tensor& x, const Tensor& w) {
     const int64_t K = x.size(-1), I = w.size(0) / 2, M = x.numel() / K;
@@ -349,7 +354,7 @@ struct VigPlan : PlanBase {
                 std::tie(n, tok) = linear_add_rmsnorm(c, b.attn.forward(c, n, h, w), b.attn.o_w, tok, b.n2, b.e2);
                 std::tie(n, tok) = linear_add_rmsnorm(c, mlp_in(c, n, b.gate_w), b.down_w, tok, next_w, next_e);
             }
-            return finish(n.mean(1));
+            return finish(token_mean(c, n));
         }
         ok(api.vig_layernorm_act_add_fwd(ptr(y), ptr(conv2.b), ptr(ln2_w), ptr(ln2_b), ptr(pos), L, ptr(tok), rows, C, (float)ln2_e, 0, c.code, c.stream),
            "vig_layernorm_act_add_fwd");
@@ -361,7 +366,7 @@ struct VigPlan : PlanBase {
             std::tie(n, tok) = add_rmsnorm(c, at::linear(b.attn.forward(c, n, h, w), b.attn.o_w), b.n2, tok, b.e2, true);
             branch = at::linear(mlp_in(c, n, b.gate_w), b.down_w);
         }
-        return finish(add_rmsnorm(c, branch, norm_w, tok, norm_e, false).first.mean(1));
+        return finish(token_mean(c, add_rmsnorm(c, branch, norm_w, tok, norm_e, false).first));
     }
 };
 
@@ -422,7 +427,7 @@ struct HierPlan : PlanBase {
             }
         }
         const Tensor n = branch.defined() ? add_layernorm(c, branch, x, last, 0).first : add_layernorm(c, x, {}, last, 0).first;
-        return finish(n.mean(1));
+        return finish(token_mean(c, n));
     }
 };
 

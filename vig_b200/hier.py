@@ -180,7 +180,7 @@ class HierViG(nn.Module):
         status = ops.status_word(images.device)
         status.poll()
         x = self.forward_features(images)
-        x = _layer_norm(x, self.classifier.norm).mean(dim=1)
+        x = ops.token_mean(_layer_norm(x, self.classifier.norm))
         logits = self.classifier.head(x)
         status.snapshot()
         return logits

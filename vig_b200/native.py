@@ -13,7 +13,7 @@ from . import _lib, hier, modules, ops, vig
 
 _plans = weakref.WeakKeyDictionary()          # model -> plan, or False where the model has none
 _OPS = {n: getattr(ops, n) for n in ("bi_gla", "dwconv3x3", "gate_inject", "add_rmsnorm", "layernorm_act", "add_layernorm", "linear_swiglu",
-                                     "linear_add_rmsnorm", "linear_bias", "swiglu", "stem_fold", "stem_unfold", "stem_conv_ln")}
+                                     "linear_add_rmsnorm", "linear_bias", "swiglu", "token_mean", "stem_fold", "stem_unfold", "stem_conv_ln")}
 _CLASSES = (vig.ViG, vig.V2PatchEmbed, vig.LayerNorm2d, modules.GLABlock, modules.GatedLinearAttention, modules.GLAMLP, modules.RMSNorm,
             hier.HierViG, hier.VSSBlock, hier.GLA2D, hier.Mlp, hier.gMlp, nn.Linear, nn.Conv2d, nn.LayerNorm, nn.SiLU, nn.GELU, nn.Identity,
             nn.Sequential, nn.ModuleList)

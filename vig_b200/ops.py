@@ -410,6 +410,19 @@ def add_layernorm(x, weight, bias, eps=1e-5, residual=None, act=0):
     return y if residual is None else (y, r)
 
 
+def token_mean(x):
+    """``x.mean(dim=1)`` of contiguous ``[B, L, C]`` tokens: fp32 sums, one rounding."""
+    _lib.require_cuda(x)
+    if x.dim() != 3 or not x.is_contiguous():
+        raise ValueError("x must be contiguous [B, L, C]")
+    B, L, C = x.shape
+    y = torch.empty(B, C, dtype=x.dtype, device=x.device)
+    with torch.cuda.device(x.device):
+        st = _lib.lib().vig_token_mean_fwd(_lib.ptr(x), _lib.ptr(y), B, L, C, _lib.dtype_code(x), _lib.stream_ptr())
+    _lib.check(st, "vig_token_mean_fwd")
+    return y
+
+
 def linear_add_rmsnorm_supported(x, w):
     """True when ``linear_add_rmsnorm`` can run on these operands (16-bit CUDA tensors, K % 64 == 0, N in {64, 128, 192, 256, 384})."""
     if not (x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and w.dtype == x.dtype and x.stride(-1) == 1):

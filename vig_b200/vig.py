@@ -182,6 +182,7 @@ class ViG(nn.Module):
         # ``fuse_norm_epilogues``: every residual add + RMSNorm runs as the epilogue of the projection in front of it
         # (hidden size <= 192, 16-bit tensors; measured 74 + 104 us against 112 + 141 us for cuBLAS + the norm kernel),
         # and the first block's norm comes out of the stem's last kernel.
+        from . import ops
         probe = x.new_empty(1, 1, self.embed_dim)
         if self.fuse_norm_epilogues and len(self.blocks) and all(blk.fused_epilogues_supported(probe) for blk in self.blocks):
             x, hw, h = self.patch_embed(x, pos_fn=self._pos, next_norm=self.blocks[0].attn_norm)
@@ -189,13 +190,13 @@ class ViG(nn.Module):
             for i, blk in enumerate(self.blocks):
                 nxt = self.blocks[i + 1].attn_norm if i + 1 < len(self.blocks) else self.norm
                 h, residual = blk.forward_prenormed(h, residual, nxt, patch_resolution=hw)
-            return h.mean(dim=1)
+            return ops.token_mean(h)
         x, hw = self.patch_embed(x, pos_fn=self._pos)  # position embedding added by the stem's last kernel
         h, residual = x, None
         for blk in self.blocks:
             h, residual = blk.forward_deferred(h, residual, patch_resolution=hw)
         x = self.norm(h, residual)                      # last residual add fused into the final norm
-        return x.mean(dim=1)
+        return ops.token_mean(x)
 
     def forward(self, x, **kwargs):
         """Logits.  The kernels' error word is looked at without stalling the stream: this call raises if a kernel of an
