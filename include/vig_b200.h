@@ -272,12 +272,19 @@ VIG_API int vig_layernorm_act_add_rmsnorm_fwd(const void* x, const void* pre_bia
                                               int64_t post_period, void* y, const void* rms_w, float rms_eps, void* h, int64_t rows, int N,
                                               float eps, int act_swish, int dtype, void* stream);
 
-/* r = x + residual (residual optional; the sum is rounded to the tensor dtype and written to sum_out when given), then
+/* r = x + pre_bias + residual (each optional, each sum rounded to the tensor dtype; pre_bias: [N], the bias of the convolution
+ * that produced x; r is written to sum_out when given), then
  * y = LayerNorm(r) * w + bias, then act: 0 none, 1 swish, 2 GELU (erf form) -- the pre-norms of the hierarchical model's
  * blocks with the residual add in front of them (classification/models/vig_h.py:672-683) and its patch embedding's
  * LayerNorm + GELU.  Contiguous [rows, N], N * element size a multiple of 16. */
-VIG_API int vig_add_layernorm_fwd(const void* x, const void* residual, const void* w, const void* bias, void* y, void* sum_out, int64_t rows,
+VIG_API int vig_add_layernorm_fwd(const void* x, const void* pre_bias, const void* residual, const void* w, const void* bias, void* y, void* sum_out, int64_t rows,
                                   int N, float eps, int act, int dtype, void* stream);
+
+/* First convolution of the hierarchical model's patch embedding (3 -> O channels, 3 x 3, stride 2, padding 1) + bias + LayerNorm
+ * over channels (+ GELU, erf form), each step rounded to the dtype: x [B,3,H,W] -> y [B, (H+1)/2, (W+1)/2, O].  bf16 / fp16, O of
+ * 32, 48, 64; w [O,3,3,3] contiguous, conv_bias optional (classification/models/vig_h.py, patch embedding "v2"). */
+VIG_API int vig_embed_conv_ln_fwd(const void* x, const void* w, const void* conv_bias, const void* ln_w, const void* ln_b, void* y, int B, int H, int W, int O,
+                                  float eps, int act_gelu, int dtype, void* stream);
 
 /* y[b, c] = mean over l of x[b, l, c] (fp32 sums, rounded once): the models' pooling.  x contiguous [B, L, C], C * element size a
  * multiple of 16. */

@@ -43,13 +43,14 @@ _SIGNATURES = {
     "vig_linear_add_rmsnorm_fwd": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_float, c_int, c_void_p, c_void_p]),
     "vig_layernorm_act_add_fwd": (c_int, [c_void_p] * 5 + [c_int64, c_void_p, c_int64, c_int, c_float, c_int, c_int, c_void_p]),
     "vig_layernorm_act_add_rmsnorm_fwd": (c_int, [c_void_p] * 5 + [c_int64, c_void_p, c_void_p, c_float, c_void_p, c_int64, c_int, c_float, c_int, c_int, c_void_p]),
+    "vig_embed_conv_ln_fwd": (c_int, [c_void_p] * 6 + [c_int] * 4 + [c_float, c_int, c_int, c_void_p]),
     "vig_token_mean_fwd": (c_int, [c_void_p] * 2 + [c_int] * 4 + [c_void_p]),
     "vig_chain_launches": (c_int, [c_int]),
     "vig_block_tail_supported": (c_int, [c_int64] + [c_int] * 4),
     "vig_block_tail_preferred": (c_int, [c_int64] + [c_int] * 4),
     "vig_block_tail_fwd": (c_int, [c_void_p] * 3 + [c_int64] + [c_void_p] * 2 + [c_float, c_int] + [c_void_p] * 3 + [c_float] + [c_void_p] * 3 +
                            [c_float] + [c_void_p] * 2 + [c_int64] + [c_int] * 4 + [c_void_p] * 2),
-    "vig_add_layernorm_fwd": (c_int, [c_void_p] * 6 + [c_int64, c_int, c_float, c_int, c_int, c_void_p]),
+    "vig_add_layernorm_fwd": (c_int, [c_void_p] * 7 + [c_int64, c_int, c_float, c_int, c_int, c_void_p]),
     "vig_stem_unfold_fwd": (c_int, [c_void_p, c_void_p] + [c_int] * 6 + [c_void_p]),
     "vig_stem_fold_fwd": (c_int, [c_void_p, c_void_p] + [c_int] * 5 + [c_void_p]),
     "vig_stem_conv_ln_supported": (c_int, [c_int] * 6),

@@ -97,6 +97,17 @@ __device__ __forceinline__ float4 scan_states(float4* ws, const float* decay, in
     return S;
 }
 
+// GELU in its erf form.  16-bit results: erf by Abramowitz & Stegun 7.1.26 (|error| <= 1.5e-7), one exponential and one
+// reciprocal; fp32 keeps erff.
+template <typename T> __device__ __forceinline__ float gelu_t(float x) {
+    const float z = x * 0.70710678118654752f;
+    if (sizeof(T) == 4) return 0.5f * x * (1.f + erff(z));
+    const float az = fabsf(z), t = __fdividef(1.f, fmaf(0.3275911f, az, 1.f));
+    const float poly = t * fmaf(t, fmaf(t, fmaf(t, fmaf(t, 1.061405429f, -1.453152027f), 1.421413741f), -0.284496736f), 0.254829592f);
+    const float q = poly * __expf(-az * az);                     // 1 - erf(|z|)
+    return 0.5f * x * (z < 0.f ? q : 2.f - q);
+}
+
 // Programmatic dependent launch.  A kernel that calls pdl_wait() before it touches what an earlier kernel wrote may be launched
 // while that kernel still runs (launch_chained); pdl_launch() lets the next kernel of the stream do the same.  Both do nothing
 // in an ordinary launch.  A kernel allocates tensor memory only after pdl_wait(): earlier it could hold what a kernel it

@@ -1,6 +1,7 @@
 // Bandwidth-bound kernels of the ViG block: depthwise 3x3 conv in token-major layout, the 2-D gating
 // locality injection, residual-add + RMSNorm, SwiGLU.  Every global access is a 16-byte vector;
 // arithmetic and statistics are fp32.
+#include <initializer_list>
 #include <type_traits>
 #include "common.cuh"
 
@@ -420,85 +421,104 @@ __global__ void __launch_bounds__(EW_THREADS) layernorm_act_kernel(const T* __re
     }
 }
 
-// (x + residual) -> LayerNorm (-> swish / GELU): the pre-norm blocks of the hierarchical model, whose residual adds were passes
-// of their own, and its patch embedding.  LPR lanes share a row and hold it in registers (MAXV vectors each, the pair chosen so
-// that few lanes idle at 96, 192, 384 and 768 channels); U rows per lane group are in flight, because a row's two dependent
-// reductions leave the memory system idle otherwise.
+// (x + pre_bias + residual) -> LayerNorm (-> swish / GELU): the pre-norm blocks of the hierarchical model, whose residual adds
+// were passes of their own, and the norms behind its convolutions, whose bias adds were.  LPR lanes share a row and hold it in
+// registers (MAXV vectors each, the pair chosen so that no lane idles at 48 .. 768 channels and a row takes few shuffles); U
+// rows per lane group are in flight and share the unpacked parameters: bound by instruction issue at narrow rows (200704 x 96
+// with a residual: 52 us with 16 lanes a row, one vector each; 4 lanes, three vectors: 31; floor 24).
 template <typename T, int LPR, int MAXV, int U>
-__global__ void __launch_bounds__(EW_THREADS) add_layernorm_kernel(const T* __restrict__ x, const T* __restrict__ res, const T* __restrict__ w,
-                                                                   const T* __restrict__ bias, T* __restrict__ y, T* __restrict__ sum_out,
-                                                                   int64_t rows, int N, float eps, int act) {
+__global__ void __launch_bounds__(EW_THREADS, U * MAXV <= 4 ? 3 : 1) add_layernorm_kernel(const T* __restrict__ x, const T* __restrict__ pre_bias, const T* __restrict__ res,
+                                                                   const T* __restrict__ w, const T* __restrict__ bias, T* __restrict__ y,
+                                                                   T* __restrict__ sum_out, int64_t rows, int N, float eps, int act) {
     constexpr int V = DType<T>::VEC;
     const int sub = threadIdx.x % LPR, nv = N / V;
     const int64_t g0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / LPR, ng = ((int64_t)gridDim.x * blockDim.x) / LPR;
+    const float inv_n = 1.f / (float)N;
     for (int64_t r0 = g0; r0 < rows; r0 += U * ng) {
         Vec16<T> xv[U][MAXV], rv[U][MAXV];
 #pragma unroll
-        for (int u = 0; u < U; ++u)
+        for (int u = 0; u < U; ++u) {
+            const int64_t at = min(r0 + u * ng, rows - 1) * N;
 #pragma unroll
             for (int m = 0; m < MAXV; ++m) {
                 const int vi = sub + m * LPR;
-                const int64_t r = r0 + u * ng;
-                if (vi < nv && r < rows) {
-                    xv[u][m].load_nc(x + r * N + vi * V);
-                    if (res) rv[u][m].load_nc(res + r * N + vi * V);
+                if (vi < nv) {
+                    xv[u][m].load_nc(x + at + vi * V);
+                    if (res) rv[u][m].load_nc(res + at + vi * V);
                 }
             }
+        }
+        float val[U][MAXV][V], mean[U], rstd[U];
+#pragma unroll
+        for (int m = 0; m < MAXV; ++m) {
+            const int vi = sub + m * LPR;
+            float pf[V];
+            if (pre_bias && vi < nv) { Vec16<T> pv; pv.load_nc(pre_bias + vi * V); pv.to_float(pf); }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+#pragma unroll
+                for (int i = 0; i < V; ++i) val[u][m][i] = 0.f;
+                if (vi >= nv) continue;
+                xv[u][m].to_float(val[u][m]);
+                if (pre_bias) {                                  // each sum is rounded to T, as a separate add would
+#pragma unroll
+                    for (int i = 0; i < V; ++i) val[u][m][i] = DType<T>::to_f(DType<T>::from_f(val[u][m][i] + pf[i]));
+                }
+                if (res) {
+                    float rf[V];
+                    rv[u][m].to_float(rf);
+#pragma unroll
+                    for (int i = 0; i < V; ++i) val[u][m][i] += rf[i];
+                    xv[u][m].from_float(val[u][m]);
+                    xv[u][m].to_float(val[u][m]);
+                    if (sum_out && r0 + u * ng < rows) xv[u][m].store(sum_out + (r0 + u * ng) * N + vi * V);
+                }
+            }
+        }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int64_t r = r0 + u * ng;
-            float val[MAXV][V], sum = 0.f;
+            float sum = 0.f;
 #pragma unroll
-            for (int m = 0; m < MAXV; ++m) {
-                const int vi = sub + m * LPR;
-                if (vi < nv && r < rows) {
-                    xv[u][m].to_float(val[m]);
-                    if (res) {                                   // the sum is rounded to T before the statistics, as a separate add would
-                        float rf[V];
-                        rv[u][m].to_float(rf);
+            for (int m = 0; m < MAXV; ++m)
 #pragma unroll
-                        for (int i = 0; i < V; ++i) val[m][i] += rf[i];
-                        xv[u][m].from_float(val[m]);
-                        xv[u][m].to_float(val[m]);
-                        if (sum_out) xv[u][m].store(sum_out + r * N + vi * V);
-                    }
-#pragma unroll
-                    for (int i = 0; i < V; ++i) sum += val[m][i];
-                }
-            }
+                for (int i = 0; i < V; ++i) sum += val[u][m][i];
 #pragma unroll
             for (int k = LPR / 2; k >= 1; k >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, k);
-            const float mean = sum / (float)N;
+            mean[u] = sum * inv_n;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
             float ss = 0.f;
 #pragma unroll
-            for (int m = 0; m < MAXV; ++m) {
-                if (sub + m * LPR < nv && r < rows) {
+            for (int m = 0; m < MAXV; ++m)
+                if (sub + m * LPR < nv) {
 #pragma unroll
-                    for (int i = 0; i < V; ++i) { const float d = val[m][i] - mean; ss = fmaf(d, d, ss); }
+                    for (int i = 0; i < V; ++i) { val[u][m][i] -= mean[u]; ss = fmaf(val[u][m][i], val[u][m][i], ss); }
                 }
-            }
 #pragma unroll
             for (int k = LPR / 2; k >= 1; k >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, k);
-            const float rstd = rsqrtf(ss / (float)N + eps);
+            rstd[u] = rsqrtf(ss * inv_n + eps);
+        }
 #pragma unroll
-            for (int m = 0; m < MAXV; ++m) {
-                const int vi = sub + m * LPR;
-                if (vi < nv && r < rows) {
-                    Vec16<T> wv, bv;
-                    wv.load_nc(w + vi * V); bv.load_nc(bias + vi * V);
-                    float wf[V], bf[V];
-                    wv.to_float(wf); bv.to_float(bf);
+        for (int m = 0; m < MAXV; ++m) {
+            const int vi = sub + m * LPR;
+            if (vi >= nv) continue;
+            Vec16<T> wv, bv;
+            float wf[V], bf[V];
+            wv.load_nc(w + vi * V); bv.load_nc(bias + vi * V);
+            wv.to_float(wf); bv.to_float(bf);
 #pragma unroll
-                    for (int i = 0; i < V; ++i) {
-                        float t = (val[m][i] - mean) * rstd * wf[i] + bf[i];
-                        if (act == 1) t *= sigmoid_t<T>(t);
-                        // GELU of the rounded value, as a separate activation would see it
-                        if (act == 2) { t = DType<T>::to_f(DType<T>::from_f(t)); t = 0.5f * t * (1.f + erff(t * 0.70710678118654752f)); }
-                        val[m][i] = t;
-                    }
-                    Vec16<T> ov;
-                    ov.from_float(val[m]); ov.store(y + r * N + vi * V);
+            for (int u = 0; u < U; ++u) {
+#pragma unroll
+                for (int i = 0; i < V; ++i) {
+                    float t = val[u][m][i] * rstd[u] * wf[i] + bf[i];
+                    if (act == 1) t *= sigmoid_t<T>(t);
+                    if (act == 2) t = gelu_t<T>(DType<T>::to_f(DType<T>::from_f(t)));      // of the rounded value, as a separate activation would see it
+                    val[u][m][i] = t;
                 }
+                Vec16<T> ov;
+                ov.from_float(val[u][m]);
+                if (r0 + u * ng < rows) ov.store(y + (r0 + u * ng) * N + vi * V);
             }
         }
     }
@@ -713,15 +733,16 @@ int layernorm_act_t(const void* x, const void* pb, const void* w, const void* b,
 }
 
 template <typename T>
-int add_layernorm_t(const void* x, const void* res, const void* w, const void* b, void* y, void* sum_out, int64_t rows, int N, float eps, int act, cudaStream_t s) {
+int add_layernorm_t(const void* x, const void* pb, const void* res, const void* w, const void* b, void* y, void* sum_out, int64_t rows, int N, float eps, int act,
+                    cudaStream_t s) {
     constexpr int V = DType<T>::VEC;
     if (N % V) return VIG_ERR_SHAPE;
     const int nv = N / V;
 #define VIG_AL(LPR, MV, U) add_layernorm_kernel<T, LPR, MV, U><<<grid_for((rows + U - 1) / U * LPR, EW_THREADS), EW_THREADS, 0, s>>>( \
-        (const T*)x, (const T*)res, (const T*)w, (const T*)b, (T*)y, (T*)sum_out, rows, N, eps, act)
-    if (nv <= 8) VIG_AL(8, 1, 4); else if (nv <= 16) VIG_AL(16, 1, 4); else if (nv <= 24) VIG_AL(8, 3, 2); else if (nv <= 32) VIG_AL(32, 1, 4);
-    else if (nv <= 48) VIG_AL(16, 3, 2); else if (nv <= 64) VIG_AL(32, 2, 2); else if (nv <= 96) VIG_AL(32, 3, 2); else if (nv <= 128) VIG_AL(32, 4, 1);
-    else if (nv <= 256) VIG_AL(32, 8, 1); else return VIG_ERR_SHAPE;
+        (const T*)x, (const T*)pb, (const T*)res, (const T*)w, (const T*)b, (T*)y, (T*)sum_out, rows, N, eps, act)
+    if (nv == 6) VIG_AL(2, 3, 1); else if (nv == 12) VIG_AL(4, 3, 1); else if (nv <= 8) VIG_AL(8, 1, 4); else if (nv <= 16) VIG_AL(16, 1, 4);
+    else if (nv <= 24) VIG_AL(8, 3, 1); else if (nv <= 32) VIG_AL(32, 1, 4); else if (nv <= 48) VIG_AL(16, 3, 1); else if (nv <= 64) VIG_AL(32, 2, 1);
+    else if (nv <= 96) VIG_AL(32, 3, 1); else if (nv <= 128) VIG_AL(32, 4, 1); else if (nv <= 256) VIG_AL(32, 8, 1); else return VIG_ERR_SHAPE;
 #undef VIG_AL
     return (int)cudaGetLastError();
 }
@@ -855,15 +876,15 @@ extern "C" int vig_token_mean_fwd(const void* x, void* y, int B, int L, int C, i
     VIG_DISPATCH(dtype, token_mean_t<T>(x, y, B, L, C, (cudaStream_t)stream))
 }
 
-extern "C" int vig_add_layernorm_fwd(const void* x, const void* residual, const void* w, const void* bias, void* y, void* sum_out, int64_t rows,
-                                     int N, float eps, int act, int dtype, void* stream) {
+extern "C" int vig_add_layernorm_fwd(const void* x, const void* pre_bias, const void* residual, const void* w, const void* bias, void* y, void* sum_out,
+                                     int64_t rows, int N, float eps, int act, int dtype, void* stream) {
     if (!x || !w || !bias || !y) return VIG_ERR_NULL;
     if (rows < 0 || N <= 0) return VIG_ERR_SHAPE;
     if (act < 0 || act > 2 || (sum_out && !residual)) return VIG_ERR_ARG;
     if (rows == 0) return VIG_OK;
-    if (!aligned16(x) || !aligned16(w) || !aligned16(bias) || !aligned16(y) || (residual && !aligned16(residual)) || (sum_out && !aligned16(sum_out)))
-        return VIG_ERR_ALIGN;
-    VIG_DISPATCH(dtype, add_layernorm_t<T>(x, residual, w, bias, y, sum_out, rows, N, eps, act, (cudaStream_t)stream))
+    for (const void* p : {x, pre_bias, residual, w, bias, (const void*)y, (const void*)sum_out})
+        if (p && !aligned16(p)) return VIG_ERR_ALIGN;
+    VIG_DISPATCH(dtype, add_layernorm_t<T>(x, pre_bias, residual, w, bias, y, sum_out, rows, N, eps, act, (cudaStream_t)stream))
 }
 
 extern "C" int vig_stem_unfold_fwd(const void* x, void* cells, int B, int Cin, int H, int W, int s, int dtype, void* stream) {

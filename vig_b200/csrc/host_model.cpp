@@ -373,10 +373,10 @@ struct VigPlan : PlanBase {
 // ---- HierViG -------------------------------------------------------------------------------------------------------
 struct Norm { Tensor w, b; double eps = 0; };
 // r = x + residual (optional), LayerNorm(r) with an activation: {LayerNorm, r}
-std::pair<Tensor, Tensor> add_layernorm(const Ctx& c, const Tensor& x, const Tensor& res, const Norm& n, int act) {
+std::pair<Tensor, Tensor> add_layernorm(const Ctx& c, const Tensor& x, const Tensor& res, const Norm& n, int act, const Tensor& pre_bias = {}) {
     const int64_t N = x.size(-1);
     Tensor y = at::empty_like(x), r = res.defined() ? at::empty_like(x) : Tensor();
-    ok(api.vig_add_layernorm_fwd(ptr(x), ptr(res), ptr(n.w), ptr(n.b), ptr(y), ptr(r), x.numel() / N, N, (float)n.eps, act, c.code, c.stream), "vig_add_layernorm_fwd");
+    ok(api.vig_add_layernorm_fwd(ptr(x), ptr(pre_bias), ptr(res), ptr(n.w), ptr(n.b), ptr(y), ptr(r), x.numel() / N, N, (float)n.eps, act, c.code, c.stream), "vig_add_layernorm_fwd");
     return {y, r};
 }
 
@@ -396,16 +396,29 @@ struct HierStage {
 struct HierPlan : PlanBase {
     std::vector<std::tuple<Conv, bool, Norm, int>> embed;   // convolution, whether a LayerNorm follows, the norm, activation (0 / 2 = GELU)
     std::vector<HierStage> stages;
+    Tensor first_w;                                          // [O,3,3,3] contiguous where the embedding's first convolution has a kernel of its own
     Norm last;
 
     OptT forward(const Tensor& x) {
         return run(x, x.dim() == 4 ? x.size(0) * ((x.size(2) + 3) / 4) * ((x.size(3) + 3) / 4) * std::get<0>(embed.back()).w.size(0) : 0, [&](const Ctx& c, const Tensor& img) { return body(c, img); });
     }
     Tensor body(const Ctx& c, const Tensor& img) const {
-        Tensor y = img.permute({0, 2, 3, 1}).contiguous();
-        for (const auto& [conv, has_norm, norm, act] : embed) {
-            y = conv.forward(y, true);
-            if (has_norm) y = add_layernorm(c, y, {}, norm, act).first;
+        Tensor y;
+        size_t done = 0;
+        if (first_w.defined()) {                             // the first convolution with its norm and activation, from the image as it is
+            const auto& [conv, has_norm, norm, act] = embed[0];
+            const int64_t B = img.size(0), H = img.size(2), W = img.size(3), O = first_w.size(0);
+            y = at::empty({B, (H + 1) / 2, (W + 1) / 2, O}, img.options());
+            ok(api.vig_embed_conv_ln_fwd(ptr(img), ptr(first_w), ptr(conv.b), ptr(norm.w), ptr(norm.b), ptr(y), B, H, W, O, (float)norm.eps, act == 2, c.code, c.stream),
+               "vig_embed_conv_ln_fwd");
+            done = 1;
+        } else {
+            y = img.permute({0, 2, 3, 1}).contiguous();
+        }
+        for (size_t i = done; i < embed.size(); ++i) {
+            const auto& [conv, has_norm, norm, act] = embed[i];
+            y = conv.forward(y, !has_norm);                      // the bias rides in the norm
+            if (has_norm) y = add_layernorm(c, y, {}, norm, act, conv.b).first;
             else if (act == 2) y = at::gelu(y);
         }
         int64_t h = y.size(1), w = y.size(2);
@@ -421,9 +434,9 @@ struct HierPlan : PlanBase {
             }
             if (st.down) {
                 if (branch.defined()) { x = x + branch; branch = Tensor(); }
-                y = st.conv.forward(x.view({x.size(0), h, w, x.size(2)}), true);
+                y = st.conv.forward(x.view({x.size(0), h, w, x.size(2)}), false);
                 h = y.size(1); w = y.size(2);
-                x = add_layernorm(c, y.view({y.size(0), h * w, y.size(3)}), {}, st.norm, 0).first;
+                x = add_layernorm(c, y.view({y.size(0), h * w, y.size(3)}), {}, st.norm, 0, st.conv.b).first;
             }
         }
         const Tensor n = branch.defined() ? add_layernorm(c, branch, x, last, 0).first : add_layernorm(c, x, {}, last, 0).first;
@@ -477,6 +490,7 @@ HierPlan* make_hier(const py::dict& d) {
         const bool has = !e["norm"].is_none();
         p->embed.emplace_back(conv_of(e["conv"]), has, has ? norm_of(e["norm"]) : Norm(), e["act"].cast<int>());
     }
+    p->first_w = tensor_of(d, "first_w");
     for (auto item : d["stages"].cast<py::list>()) {
         const py::dict s = item.cast<py::dict>();
         HierStage st;

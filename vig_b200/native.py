@@ -83,6 +83,9 @@ def _hier(model):
             if gelu is not None and gelu.approximate != "none":
                 return None
             embed.append(dict(conv=_conv(m), norm=None if norm is None else _norm(norm), act=0 if gelu is None else 2))
+    c = pe[0]
+    own = (tuple(c.kernel_size) == (3, 3) and tuple(c.stride) == (2, 2) and tuple(c.padding) == (1, 1) and c.weight.shape[1] == 3 and
+           c.weight.shape[0] in (32, 48, 64) and c.groups == 1 and embed[0]["norm"] is not None)
     stages = []
     for layer in model.layers:
         blocks = []
@@ -97,6 +100,7 @@ def _hier(model):
         stages.append(dict(blocks=blocks, conv=_conv(down[1]) if has else None, norm=_norm(down[3]) if has else None))
     head = model.classifier.head
     return _lib.host().HierPlan(dict(head_w=head.weight, head_b=head.bias, on_status=_status_seen(head.weight.device), embed=embed, stages=stages,
+                                     first_w=c.weight.detach().contiguous() if own else None,
                                      last=_norm(model.classifier.norm)))
 
 

@@ -395,8 +395,8 @@ def layernorm_act(x, weight, bias, eps=1e-5, act_swish=False, pre_bias=None, pos
     return y
 
 
-def add_layernorm(x, weight, bias, eps=1e-5, residual=None, act=0):
-    """``r = x + residual`` (optional), ``y = LayerNorm(r) * weight + bias`` over the last dimension, then ``act``: 0 none,
+def add_layernorm(x, weight, bias, eps=1e-5, residual=None, act=0, pre_bias=None):
+    """``r = x + pre_bias + residual`` (each optional), ``y = LayerNorm(r) * weight + bias`` over the last dimension, then ``act``: 0 none,
     1 swish, 2 GELU (erf form).  Returns ``y``, or ``(y, r)`` with a residual."""
     _lib.require_cuda(x, weight, bias, residual)
     N = x.shape[-1]
@@ -404,7 +404,7 @@ def add_layernorm(x, weight, bias, eps=1e-5, residual=None, act=0):
         raise ValueError("x and residual must be contiguous tensors of one shape and dtype")
     y = torch.empty_like(x)
     r = torch.empty_like(x) if residual is not None else None
-    st = _lib.lib().vig_add_layernorm_fwd(_lib.ptr(x), _lib.ptr(residual), _lib.ptr(weight), _lib.ptr(bias), _lib.ptr(y), _lib.ptr(r), x.numel() // N, N,
+    st = _lib.lib().vig_add_layernorm_fwd(_lib.ptr(x), _lib.ptr(pre_bias), _lib.ptr(residual), _lib.ptr(weight), _lib.ptr(bias), _lib.ptr(y), _lib.ptr(r), x.numel() // N, N,
                                           float(eps), int(act), _lib.dtype_code(x), _lib.stream_ptr())
     _lib.check(st, "vig_add_layernorm_fwd")
     return y if residual is None else (y, r)
@@ -420,6 +420,21 @@ def token_mean(x):
     with torch.cuda.device(x.device):
         st = _lib.lib().vig_token_mean_fwd(_lib.ptr(x), _lib.ptr(y), B, L, C, _lib.dtype_code(x), _lib.stream_ptr())
     _lib.check(st, "vig_token_mean_fwd")
+    return y
+
+
+def embed_conv_ln(x, weight, conv_bias, ln_weight, ln_bias, eps=1e-5, act_gelu=True):
+    """Convolution 3 -> O channels, 3 x 3, stride 2, padding 1 + bias + LayerNorm over channels (+ GELU) of a 16-bit image (see
+    ``vig_embed_conv_ln_fwd``): ``[B,3,H,W] -> [B, (H+1)/2, (W+1)/2, O]``, O of 32, 48, 64."""
+    _lib.require_cuda(x, weight, ln_weight, ln_bias)
+    B, _, H, W = x.shape
+    O = weight.shape[0]
+    x, weight = x.contiguous(), weight.contiguous()
+    y = torch.empty(B, (H + 1) // 2, (W + 1) // 2, O, dtype=x.dtype, device=x.device)
+    with torch.cuda.device(x.device):
+        st = _lib.lib().vig_embed_conv_ln_fwd(_lib.ptr(x), _lib.ptr(weight), _lib.ptr(conv_bias), _lib.ptr(ln_weight), _lib.ptr(ln_bias), _lib.ptr(y), B, H, W, O,
+                                              float(eps), int(bool(act_gelu)), _lib.dtype_code(x), _lib.stream_ptr())
+    _lib.check(st, "vig_embed_conv_ln_fwd")
     return y
 
 
