@@ -129,7 +129,7 @@ template <> struct ScalePair<__half> {
     }
 };
 
-template <typename T, bool RAW, bool CLAMP, bool SO>
+template <typename T, bool RAW, bool CLAMP, bool SO, bool D32>
 __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_constant__ WaveMaps maps, const WaveParams wp) {
     const BiglaParams& p = wp.p;
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -163,6 +163,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_c
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (D32) for (int i = tid; i < 4 * 2 * 64; i += W_THREADS) vec[i] = 0.f;      // the padding channels' entries are read, never written
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(WT_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -280,7 +281,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_c
                 // (a) scores, and right behind them the state update: it needs only the prepared tiles, and the
                 // state chain -- the one sequential dependency of the kernel -- waits for nothing else
 #pragma unroll
-                for (uint32_t k4 = 0; k4 < WDK / 16; ++k4) { if (issuer) tc_mma(tmem + WT_P, q_lo + 2 * k4, k_lo + 2 * k4, IDESC_QK, k4 > 0); }
+                for (uint32_t k4 = 0; k4 < (D32 ? 2 : WDK / 16); ++k4) { if (issuer) tc_mma(tmem + WT_P, q_lo + 2 * k4, k_lo + 2 * k4, IDESC_QK, k4 > 0); }
                 if (issuer) tc_commit(bar(B_PFULL));
 #pragma unroll
                 for (uint32_t k8 = 0; k8 < CHUNK / 16; ++k8) { if (issuer) tc_mma(u_acc, k_lo + 128 * k8, v_lo + 128 * k8, IDESC_U, k8 > 0); }
@@ -292,7 +293,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_c
                 tc_fence_after();
                 if (!s_zero) {
 #pragma unroll
-                    for (uint32_t k4 = 0; k4 < WDK / 16; ++k4) { if (issuer) tc_mma(o_acc, q_lo + 2 * k4, st_lo + 128 * k4, IDESC_OV, k4 > 0); }
+                    for (uint32_t k4 = 0; k4 < (D32 ? 2 : WDK / 16); ++k4) { if (issuer) tc_mma(o_acc, q_lo + 2 * k4, st_lo + 128 * k4, IDESC_OV, k4 > 0); }
                 }
                 if (issuer) tc_commit(bar(B_STFREE));          // the state operand may be overwritten
                 // (c) masked scores x v
@@ -355,10 +356,15 @@ __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_c
         // (8-byte shared-memory accesses: a half-warp covers one 128-byte token row).  Scan position sp = 4*half + u is
         // token 8*warp + (sp ^ dmask): the same code serves both directions.  Gate form (raw logits or log-gates) and the
         // lower clamp are template parameters: the token loops carry no branch, so their 16 elements overlap.
+        // dk = 32: the rows are half as long, so a quarter-warp takes 2 consecutive scan positions and nobody works on the
+        // zero channels (96 sequences of 3136 tokens 124 -> 111 us); quarters lie so that the two of a half-warp read rows
+        // whose swizzled chunks fall into different halves of the banks.
+        constexpr int NTK = D32 ? 2 : 4, NPART = D32 ? 4 : 2;    // tokens of a lane; parts of a warp, in scan order
         const int grp = warp;
         const float coef = RAW ? -1.f / p.gate_norm : LOG2E;  // log2-gate = coef * (RAW ? log2(1 + 2^(-x log2 e)) : x)
         const float clamp_lo = CLAMP ? p.clamp_min * LOG2E : -INFINITY;
-        const int half = lane >> 4, c4l = lane & 15;          // my half of the group, my 4 channels: 4*c4l .. 4*c4l+3
+        const int half = D32 ? ((lane >> 3) & 1) * 2 + (lane >> 4) : lane >> 4, c4l = D32 ? lane & 7 : lane & 15;   // my part of the group, my 4 channels: 4*c4l .. 4*c4l+3
+        auto lane_of = [&](int part) { return D32 ? (part >> 1) * 8 + (part & 1) * 16 + c4l : part * 16 + c4l; };
         const uint32_t sw_in = (uint32_t)(c4l & 1) * 8, chunk = (uint32_t)c4l >> 1;
         // The same warps mask the scores of the iteration before and stage the output of the one before that (a warp owns
         // the 32 query rows of its TMEM lane quadrant and a quarter of the columns): by the time a trip reaches them the
@@ -377,7 +383,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_c
             const uint32_t s = m % 3;
             bool have = false;
             const int dir_mask_it = dir_prev;                 // direction of iteration m - 1 (the one whose scores are masked in this trip)
-            float4 gl[4];                                     // cumulative log2-gates of my 4 tokens, from the group's first token
+            float4 gl[NTK];                                   // cumulative log2-gates of my tokens, from the group's first token
             uint8_t* stg = smem + s * W_STAGE_B;
             int dmask = 0;
             // A test of an mbarrier costs a few hundred cycles even when its phase completed long ago (it queues behind the
@@ -404,13 +410,13 @@ __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_c
             dmask = cur.dir ? 7 : 0;
             // ---- gate phase: transform, running sums over my 4 tokens, group sum published ----
             {
-                uint2 raw[4];
+                uint2 raw[NTK];
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    raw[u] = *reinterpret_cast<const uint2*>(stg + WS_G + (grp * 8 + ((half * 4 + u) ^ dmask)) * 128 + c4l * 8);
+                for (int u = 0; u < NTK; ++u)
+                    raw[u] = *reinterpret_cast<const uint2*>(stg + WS_G + (grp * 8 + ((half * NTK + u) ^ dmask)) * 128 + c4l * 8);
                 float4 run = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
+                for (int u = 0; u < NTK; ++u) {
                     const float2 a = Pack2<T>::unpack(raw[u].x), b2 = Pack2<T>::unpack(raw[u].y);
                     float4 t = make_float4(a.x, a.y, b2.x, b2.y);
                     if (RAW) {                                // log2(1 + 2^(-x log2 e)) = -log2 sigmoid(x)
@@ -419,7 +425,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_c
                         const F2 e01 = f2_add(one, f2_make(ex2(f2_lo(y01)), ex2(f2_hi(y01)))), e23 = f2_add(one, f2_make(ex2(f2_lo(y23)), ex2(f2_hi(y23))));
                         t.x = lg2(f2_lo(e01)); t.y = lg2(f2_hi(e01)); t.z = lg2(f2_lo(e23)); t.w = lg2(f2_hi(e23));
                     }
-                    const float cu = grp * 8 + ((half * 4 + u) ^ dmask) < n_valid ? coef : 0.f;   // padding rows: gate 0
+                    const float cu = grp * 8 + ((half * NTK + u) ^ dmask) < n_valid ? coef : 0.f;   // padding rows: gate 0
                     if (CLAMP) {
                         run.x += fmaxf(t.x * cu, clamp_lo); run.y += fmaxf(t.y * cu, clamp_lo);
                         run.z += fmaxf(t.z * cu, clamp_lo); run.w += fmaxf(t.w * cu, clamp_lo);
@@ -430,15 +436,21 @@ __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_c
                     }
                     gl[u] = run;
                 }
-                // the second half-warp continues the first half-warp's sum; it also knows the group's total
-                float4 first;
-                first.x = __shfl_sync(0xffffffffu, run.x, c4l); first.y = __shfl_sync(0xffffffffu, run.y, c4l);
-                first.z = __shfl_sync(0xffffffffu, run.z, c4l); first.w = __shfl_sync(0xffffffffu, run.w, c4l);
+                // a part continues the sums of the parts scanned before it; the last one also knows the group's total
+                float4 first = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int k = 0; k + 1 < NPART; ++k) {
+                    float4 t;
+                    t.x = __shfl_sync(0xffffffffu, run.x, lane_of(k)); t.y = __shfl_sync(0xffffffffu, run.y, lane_of(k));
+                    t.z = __shfl_sync(0xffffffffu, run.z, lane_of(k)); t.w = __shfl_sync(0xffffffffu, run.w, lane_of(k));
+                    if (k < half) { first.x += t.x; first.y += t.y; first.z += t.z; first.w += t.w; }
+                }
                 float* part = reinterpret_cast<float*>(smem + WO_PART) + (m & 1) * (W_PREP_WARPS * WDK);
                 if (half) {
-                    reinterpret_cast<float4*>(part)[grp * 16 + c4l] = make_float4(run.x + first.x, run.y + first.y, run.z + first.z, run.w + first.w);
+                    if (half == NPART - 1)
+                        reinterpret_cast<float4*>(part)[grp * 16 + c4l] = make_float4(run.x + first.x, run.y + first.y, run.z + first.z, run.w + first.w);
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) { gl[u].x += first.x; gl[u].y += first.y; gl[u].z += first.z; gl[u].w += first.w; }
+                    for (int u = 0; u < NTK; ++u) { gl[u].x += first.x; gl[u].y += first.y; gl[u].z += first.z; gl[u].w += first.w; }
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive_plain(bar(B_PART + (m & 1)));
@@ -515,12 +527,12 @@ __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_c
             // staging above ran while they arrived), so the wait below is a formality ----
             if (have) {
             // raw operand rows into registers
-            uint2 rk[4], rq[4];
-            uint32_t offs[4];
+            uint2 rk[NTK], rq[NTK];
+            uint32_t offs[NTK];
             const uint32_t pre_part = mbar_test_wait(bar(B_PART + (m & 1)), (m >> 1) & 1);
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const uint32_t r7 = (uint32_t)((half * 4 + u) ^ dmask);
+            for (int u = 0; u < NTK; ++u) {
+                const uint32_t r7 = (uint32_t)((half * NTK + u) ^ dmask);
                 offs[u] = (uint32_t)(grp * 8 + r7) * 128 + ((chunk ^ r7) << 4) + sw_in;
                 rk[u] = *reinterpret_cast<const uint2*>(stg + WS_K + offs[u]);
                 rq[u] = so ? make_uint2(0u, 0u) : *reinterpret_cast<const uint2*>(stg + WS_Q + offs[u]);
@@ -538,8 +550,8 @@ __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_c
                 // two-wide fp32 arithmetic (the workers are bound by instruction issue)
                 F2 s01 = f2_make(0.f, 0.f), s23 = s01, b01 = s01, b23 = s01;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int go = half * 8 + i;
+                for (int i = 0; i < W_PREP_WARPS / NPART; ++i) {
+                    const int go = half * (W_PREP_WARPS / NPART) + i;
                     const float4 t = part[(go ^ flip) * 16];
                     const F2 t01 = f2_make(t.x, t.y), t23 = f2_make(t.z, t.w);
                     s01 = f2_add(s01, t01); s23 = f2_add(s23, t23);
@@ -547,14 +559,20 @@ __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_c
                     const F2 kk = f2_make(k, k);
                     b01 = f2_fma(kk, t01, b01); b23 = f2_fma(kk, t23, b23);
                 }
-                const float4 sum = make_float4(f2_lo(s01), f2_hi(s01), f2_lo(s23), f2_hi(s23));
-                const float4 bef = make_float4(f2_lo(b01), f2_hi(b01), f2_lo(b23), f2_hi(b23));
+                float4 sum = make_float4(f2_lo(s01), f2_hi(s01), f2_lo(s23), f2_hi(s23));
+                float4 bef = make_float4(f2_lo(b01), f2_hi(b01), f2_lo(b23), f2_hi(b23));
+                auto add_from = [&](float4& v, int x) {
+                    v.x += __shfl_xor_sync(0xffffffffu, v.x, x); v.y += __shfl_xor_sync(0xffffffffu, v.y, x);
+                    v.z += __shfl_xor_sync(0xffffffffu, v.z, x); v.w += __shfl_xor_sync(0xffffffffu, v.w, x);
+                };
+                if (D32) { add_from(sum, 16); add_from(bef, 16); }        // quarters -> halves of the scan order
+                constexpr int X = D32 ? 8 : 16;
                 float4 osum, obef;
-                osum.x = __shfl_xor_sync(0xffffffffu, sum.x, 16); osum.y = __shfl_xor_sync(0xffffffffu, sum.y, 16);
-                osum.z = __shfl_xor_sync(0xffffffffu, sum.z, 16); osum.w = __shfl_xor_sync(0xffffffffu, sum.w, 16);
-                obef.x = __shfl_xor_sync(0xffffffffu, bef.x, 16); obef.y = __shfl_xor_sync(0xffffffffu, bef.y, 16);
-                obef.z = __shfl_xor_sync(0xffffffffu, bef.z, 16); obef.w = __shfl_xor_sync(0xffffffffu, bef.w, 16);
-                const float4 gref = half ? osum : sum;                    // the half-warp that read the first 8 groups has it
+                osum.x = __shfl_xor_sync(0xffffffffu, sum.x, X); osum.y = __shfl_xor_sync(0xffffffffu, sum.y, X);
+                osum.z = __shfl_xor_sync(0xffffffffu, sum.z, X); osum.w = __shfl_xor_sync(0xffffffffu, sum.w, X);
+                obef.x = __shfl_xor_sync(0xffffffffu, bef.x, X); obef.y = __shfl_xor_sync(0xffffffffu, bef.y, X);
+                obef.z = __shfl_xor_sync(0xffffffffu, bef.z, X); obef.w = __shfl_xor_sync(0xffffffffu, bef.w, X);
+                const float4 gref = half >= NPART / 2 ? osum : sum;       // the part that read the first 8 groups has it
                 off = make_float4(bef.x + obef.x - gref.x, bef.y + obef.y - gref.y, bef.z + obef.z - gref.z, bef.w + obef.w - gref.w);
                 if (grp == 0 && half == 0) {                              // [G_ref | G_last] of this iteration for the state warps
                     float4* ve = reinterpret_cast<float4*>(vec + (m & 3) * 128) + c4l;
@@ -566,12 +584,12 @@ __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_c
             // Log-gates are <= 0, so a lane's exponents are monotone along its 4 tokens: the largest magnitude is at one
             // of the two ends.  Beyond the range the factorisation covers, exponents are clamped and the call is flagged.
             float worst = fmaxf(fmaxf(fabsf(off.x + gl[0].x), fabsf(off.y + gl[0].y)), fmaxf(fabsf(off.z + gl[0].z), fabsf(off.w + gl[0].w)));
-            worst = fmaxf(worst, fmaxf(fmaxf(fabsf(off.x + gl[3].x), fabsf(off.y + gl[3].y)), fmaxf(fabsf(off.z + gl[3].z), fabsf(off.w + gl[3].w))));
+            worst = fmaxf(worst, fmaxf(fmaxf(fabsf(off.x + gl[NTK - 1].x), fabsf(off.y + gl[NTK - 1].y)), fmaxf(fabsf(off.z + gl[NTK - 1].z), fabsf(off.w + gl[NTK - 1].w))));
             const bool out_of_range = __any_sync(0xffffffffu, !(worst <= MAX_EXPONENT2));
             if (out_of_range) {                               // rare: clamp in place, flag the call
                 if (lane == 0 && p.status) atomicOr(p.status, 2);
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
+                for (int u = 0; u < NTK; ++u) {
                     gl[u].x = fminf(fmaxf(off.x + gl[u].x, -MAX_EXPONENT2), MAX_EXPONENT2) - off.x;
                     gl[u].y = fminf(fmaxf(off.y + gl[u].y, -MAX_EXPONENT2), MAX_EXPONENT2) - off.y;
                     gl[u].z = fminf(fmaxf(off.z + gl[u].z, -MAX_EXPONENT2), MAX_EXPONENT2) - off.z;
@@ -579,7 +597,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_c
                 }
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < NTK; ++u) {
                 const float ex = off.x + gl[u].x, ey = off.y + gl[u].y, ez = off.z + gl[u].z, ew = off.w + gl[u].w;
                 uint2 ko, qo;                                 // scale * out_scale is applied to the output instead
                 ko.x = ScalePair<T>::mul(rk[u].x, ex2(-ex), ex2(-ey)); ko.y = ScalePair<T>::mul(rk[u].y, ex2(-ez), ex2(-ew));
@@ -779,7 +797,7 @@ int launch_wave(const BiglaParams& p, const WaveMaps& maps, void* ws, cudaStream
     wp.mailbox = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(ws) + cb);
     cudaError_t e;
     if ((e = cudaMemsetAsync(ws, 0, cb, stream)) != cudaSuccess) return (int)e;
-    auto kern = bigla_wave_kernel<T, RAW, CLAMP, SO>;
+    auto kern = p.dk == 32 ? bigla_wave_kernel<T, RAW, CLAMP, SO, true> : bigla_wave_kernel<T, RAW, CLAMP, SO, false>;
     if ((e = ensure_smem_attr(reinterpret_cast<const void*>(kern), W_SMEM_BYTES)) != cudaSuccess) return (int)e;
     const int ndir = p.dir_mask == 3 ? 2 : 1;
     const long long items = (long long)BH * ndir * nseg;
@@ -793,8 +811,8 @@ int launch_wave(const BiglaParams& p, const WaveMaps& maps, void* ws, cudaStream
 bool bigla_wave_supported(const BiglaParams& p) {
     if (p.dtype != VIG_DTYPE_BF16 && p.dtype != VIG_DTYPE_F16) return false;
     // dk = 32 runs as dk = 64 with the upper 32 key channels zero: the q / k / gate boxes are declared 64 wide over tensors
-    // of 32 channels and the TMA unit fills the rest with zeros, which stay zero through the scaling; half of the MMA
-    // work on those operands is wasted, the DRAM traffic is that of dk = 32
+    // of 32 channels and the TMA unit fills the rest with zeros, which stay zero through the scaling; the worker
+    // warps and the MMAs that contract over the channels leave them out, the DRAM traffic is that of dk = 32
     if (p.dv != WDV || (p.dk != WDK && p.dk != 32) || p.B * p.H < 1 || p.L < 1) return false;
     if (p.o ? !p.q : !(p.final_f || p.final_b || p.logdecay_f || p.logdecay_b)) return false;   // an output, or a states-only call
     if (p.dir_mask < 1 || p.dir_mask > 3) return false;
