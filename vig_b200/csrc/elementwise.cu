@@ -223,29 +223,45 @@ __global__ void __launch_bounds__(EW_THREADS) add_rmsnorm_kernel(const T* __rest
     const int nv = N / V;
     const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    // wide rows: the warp's next row is in flight during this one's arithmetic (131072 x 768 with a residual 162 -> 142 us; at one
+    // vector a lane the extra registers cost more than it gives)
+    constexpr bool AHEAD = MAXV > 1;
+    Vec16<T> xn[MAXV], rn[MAXV];
+    auto fetch = [&](int64_t r) {
+#pragma unroll
+        for (int m = 0; m < MAXV; ++m) {
+            const int vi = lane + m * 32;
+            if (vi < nv) {
+                xn[m].load_nc(x + r * N + vi * V);
+                if (res) rn[m].load_nc(res + r * N + vi * V);
+            }
+        }
+    };
+    if (AHEAD && warp0 < rows) fetch(warp0);
     for (int64_t r = warp0; r < rows; r += nwarps) {
+        if (!AHEAD) fetch(r);
         float val[MAXV][V];
         float ss = 0.f;
 #pragma unroll
         for (int m = 0; m < MAXV; ++m) {
             const int vi = lane + m * 32;
             if (vi < nv) {
-                Vec16<T> xv; xv.load_nc(x + r * N + vi * V); xv.to_float(val[m]);
+                xn[m].to_float(val[m]);
                 if (res) {
-                    Vec16<T> rv; rv.load_nc(res + r * N + vi * V);
-                    float rf[V]; rv.to_float(rf);
+                    float rf[V]; rn[m].to_float(rf);
 #pragma unroll
                     for (int i = 0; i < V; ++i) val[m][i] += rf[i];
                     // the reference rounds the sum to the tensor dtype before the norm (rms_norm_ref: (x + residual).to(x.dtype))
                     Vec16<T> sv; sv.from_float(val[m]); sv.to_float(val[m]);
                     if (res_out) sv.store(res_out + r * N + vi * V);
                 } else if (res_out) {
-                    xv.store(res_out + r * N + vi * V);
+                    xn[m].store(res_out + r * N + vi * V);
                 }
 #pragma unroll
                 for (int i = 0; i < V; ++i) ss = fmaf(val[m][i], val[m][i], ss);
             }
         }
+        if (AHEAD && r + nwarps < rows) fetch(r + nwarps);
 #pragma unroll
         for (int m = 16; m >= 1; m >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
         const float rstd = rsqrtf(ss / (float)N + eps);
@@ -705,7 +721,7 @@ int add_rmsnorm_t(const void* x, const void* res, const void* w, void* y, void* 
     const int nv = N / V;
     const int grid = grid_for(rows * 32, EW_THREADS);
 #define VIG_RN(MV) add_rmsnorm_kernel<T, MV><<<grid, EW_THREADS, 0, s>>>((const T*)x, (const T*)res, (const T*)w, (T*)y, (T*)res_out, rows, N, eps)
-    if (nv <= 32) VIG_RN(1); else if (nv <= 64) VIG_RN(2); else if (nv <= 128) VIG_RN(4);
+    if (nv <= 32) VIG_RN(1); else if (nv <= 64) VIG_RN(2); else if (nv <= 96) VIG_RN(3); else if (nv <= 128) VIG_RN(4);
     else if (nv <= 256) VIG_RN(8); else if (nv <= 512 && V == 4) VIG_RN(16); else return VIG_ERR_SHAPE;
 #undef VIG_RN
     return (int)cudaGetLastError();
