@@ -1,5 +1,5 @@
 """The segment form of the forward (mma.sync; fp32, dv = 32, short and medium 16-bit sequences): segment edges, one-launch
-clusters of 1 to 8 segments and the three-launch form above, entering and final states, one direction, gates that leave the
+clusters of 1 to 16 segments and the three-launch form above, entering and final states, one direction, gates that leave the
 factorisation's range, and rows only the token-by-token form can read."""
 import pytest
 import torch
@@ -25,9 +25,9 @@ def test_forward_at_chunk_edges(dtype, dk, dv, L, strength):
 
 
 @pytest.mark.parametrize("dtype,dk,dv", [(torch.bfloat16, 64, 64), (torch.bfloat16, 32, 64), (torch.float16, 64, 64)])
-@pytest.mark.parametrize("B,L,strength", [(1, 64, 1.0), (1, 100, 1.0), (1, 513, 1.0), (40, 130, 1.0), (1, 1024, 1.0), (1, 1030, 1.0), (1, 300, 60.0)])
+@pytest.mark.parametrize("B,L,strength", [(1, 64, 1.0), (1, 100, 1.0), (1, 513, 1.0), (40, 130, 1.0), (1, 1024, 1.0), (1, 1030, 1.0), (2, 2048, 1.0), (1, 2049, 1.0), (1, 300, 60.0)])
 def test_forward_of_16_bit_heads(dtype, dk, dv, B, L, strength):
-    """64- and 128-token segments, 1 to 8 of them in a cluster, nine and more in three launches.  bf16 runs on bf16 operands (one
+    """64- and 128-token segments, 1 to 16 of them in a cluster, more in three launches.  bf16 runs on bf16 operands (one
     term): three roundings of 2^-9 per product on random signs, in the max norm."""
     import vig_b200
     from vig_b200 import _lib

@@ -9,7 +9,7 @@
 // Sf, Sb are the states entering the segment from its two sides.  A segment's own contribution, U = 2^(l-r) K^T V (l = total),
 // goes to the workspace; the segments of a sequence form one thread-block cluster, meet at its barrier after their products
 // (which need no state) and each sums the contributions that reach it: one launch, every input read once, for sequences of up
-// to 8 segments.  Longer ones run as states, scan over segments (bigla_simt_state_scan), outputs.
+// to 16 segments.  Longer ones run as states, scan over segments (bigla_simt_state_scan), outputs.
 //
 // Against the two-CTAs-per-SM tcgen05 form, which walks 128-token chunks one after the other in each direction with a tensor
 // memory round trip for the scores: P stays in registers, a segment's rows spread over all warps at once.  One segment takes
@@ -17,6 +17,7 @@
 // segments is that latency, one of many is bound by instruction issue at 16 warps an SM.
 // Operands are split into bf16 terms (mma_common.cuh): one term for bf16 with dv = 64 (as in the tcgen05 kernels), two for
 // fp16 and for dv = 32, three for fp32.  A segment whose |G - r| leaves the factorisation's range is evaluated token by token.
+#include <atomic>
 #include "mma_common.cuh"
 
 namespace vig {
@@ -521,13 +522,23 @@ int seg_launch_mode(const SegParams& s, cudaStream_t stream) {
     attr[0].val.clusterDim.x = s.nseg; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = MODE == SEG_ONE && s.nseg > 1 ? 1 : 0;
+    if (MODE == SEG_ONE && s.nseg > 8) {                 // more than the portable cluster size: allowed once per kernel and device
+        static std::atomic<uint64_t> allowed{0};
+        int dev = 0;
+        if ((e = cudaGetDevice(&dev)) != cudaSuccess) return (int)e;
+        const uint64_t bit = 1ull << (dev & 63);
+        if (!(allowed.load() & bit)) {
+            if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess) return (int)e;
+            allowed.fetch_or(bit);
+        }
+    }
     e = cudaLaunchKernelEx(&cfg, kern, s);
     return (int)(e != cudaSuccess ? e : cudaGetLastError());
 }
 
 template <int DK, int DV, typename T, int TOK>
 int seg_launch(SegParams& s, cudaStream_t stream) {
-    constexpr int CLUSTER = 8;                           // largest portable cluster
+    constexpr int CLUSTER = 16;                          // largest cluster of the architecture (1x3x2048 dk = 32: 12 us in one launch, 16 in three)
     BiglaParams& p = s.p;
     s.nseg = (p.L + TOK - 1) / TOK;
     s.seglen = ((p.L + s.nseg - 1) / s.nseg + 15) / 16 * 16;   // even segments: no nearly empty last one
