@@ -3,12 +3,14 @@
 //
 // The sliding-window kernel in elementwise.cu keeps only ~36 KB of loads in flight per SM (8-byte loads, nine per thread),
 // less than the ~44 KB the memory system needs to stream at full rate, and ran at a third of the copy bandwidth.  Here a
-// CTA per SM walks tiles of 2 image rows x WB columns x CC channels.  One TMA load brings the tile with its one-pixel
-// border -- 4 rows x (WB + 2) columns -- into a ring of two shared-memory stages (~100 KB each, so a whole tile is in
+// CTA per SM walks tiles of RP pairs of image rows x WB columns x CC channels.  One TMA load brings the tile with its one-pixel
+// border -- 2 RP + 2 rows x (WB + 2) columns -- into a ring of two shared-memory stages (up to ~100 KB each, so a whole tile is in
 // flight while the previous one is computed); coordinates outside the image are filled with zeros by the TMA unit, which
 // is exactly the conv's zero padding, so the kernel has no border cases.  A compute thread owns 4 channels and a run of
 // 8 columns: 36 taps live in registers as fp32, the 4-row window slides along the run and yields the outputs of both
-// image rows per step (4 shared-memory loads and 36 two-wide fp32 FMAs per 8 outputs).  Arithmetic (fp32, tap order, SiLU) is
+// image rows per step (4 shared-memory loads and 36 two-wide fp32 FMAs per 8 outputs).  Narrow images take several row pairs a
+// tile, so that no thread idles (128 x 14 x 14 x 384: 24 us with one pair, 15 with four).  Two channels and twice the threads
+// were slower on wide images (57 us against 50 at 64 x 64 x 64 x 192: twice the loads and stores).  Arithmetic (fp32, tap order, SiLU) is
 // that of the sliding-window kernel, so the two forms agree bit for bit.
 #include <type_traits>
 #include "tc_common.cuh"
@@ -21,7 +23,7 @@ using namespace tc;
 constexpr int DW_COMPUTE = 384;                // compute threads (12 warps)
 constexpr int DW_THREADS = DW_COMPUTE + 32;    // + the producer warp
 constexpr int DW_SEG = 8;                      // columns per thread
-constexpr int DW_ROWS = 2;                     // image rows per tile
+constexpr int DW_ROWS = 2;                     // image rows per thread
 constexpr int DW_STAGES = 2;
 
 // sigmoid of both lanes; 16-bit outputs take the one-MUFU form of sigmoid_t: 0.5 tanh(x / 2) + 0.5
@@ -38,7 +40,7 @@ struct DwParams {
     const void *wt, *bias;
     void* y;
     int B, h, w, C, act;
-    int CC, WB, groups, nseg;                  // channels and columns per tile; channel groups of 4 and column runs per tile
+    int CC, WB, groups, nseg, nrp;             // channels and columns per tile; channel groups of 4, column runs and row pairs per tile
     int ncb, nxb, nyb, ntiles;
     uint32_t stage_bytes, box_bytes;
     int32_t* status;
@@ -74,14 +76,14 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dwconv3x3_tma_kernel(const __gr
                 int b, yb, xb, cb;
                 decode(tile, b, yb, xb, cb);
                 mbar_expect_tx(bar_full + 8 * s, p.box_bytes);
-                // the tile with its border: columns x0-1 .. x0+WB, rows y0-1 .. y0+2; what lies outside the image reads as zero
-                tma_load_4d(sbase + s * p.stage_bytes, &map, cb * p.CC, xb * p.WB - 1, yb * DW_ROWS - 1, b, bar_full + 8 * s);
+                // the tile with its border: columns x0-1 .. x0+WB, rows y0-1 .. y0+2RP; what lies outside the image reads as zero
+                tma_load_4d(sbase + s * p.stage_bytes, &map, cb * p.CC, xb * p.WB - 1, yb * DW_ROWS * p.nrp - 1, b, bar_full + 8 * s);
             }
         }
     } else {
         // ---- compute warps ----
-        const int cg = tid % p.groups, seg = tid / p.groups;
-        const bool active = seg < p.nseg;
+        const int cg = tid % p.groups, run = tid / p.groups, seg = run % p.nseg, rp = run / p.nseg;
+        const bool active = rp < p.nrp;
         // Arithmetic runs on pairs of fp32 values held in 64-bit registers (fma / mul .f32x2: one instruction for two
         // channels, each lane an IEEE fma, so results equal the scalar form's): the kernel is bound by instruction issue.
         auto unpack4 = [](uint2 v, F2* f) {        // four packed 16-bit values -> two fp32 pairs
@@ -106,12 +108,12 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dwconv3x3_tma_kernel(const __gr
             }
             waiter.wait_lite(bar_full + 8 * s, (k / DW_STAGES) & 1);     // taken by the whole warp
             if (*abort_flag) break;
-            if (active) {
-                const int y0 = yb * DW_ROWS, x0 = xb * p.WB + seg * DW_SEG;
+            const int y0 = (yb * p.nrp + rp) * DW_ROWS, x0 = xb * p.WB + seg * DW_SEG;
+            if (active && y0 < p.h) {
                 // tile column of image column x is x - (xb * WB - 1); the window's left column of output x0 is tile column seg * SEG
                 uint32_t rowp[4];
 #pragma unroll
-                for (int r = 0; r < 4; ++r) rowp[r] = sbase + s * p.stage_bytes + (uint32_t)(seg * DW_SEG) * col_pitch + (uint32_t)cg * 8u + r * row_pitch;
+                for (int r = 0; r < 4; ++r) rowp[r] = sbase + s * p.stage_bytes + (uint32_t)(seg * DW_SEG) * col_pitch + (uint32_t)cg * 8u + (uint32_t)(DW_ROWS * rp + r) * row_pitch;
                 auto load_col = [&](F2 (*dst)[2]) {                        // the four rows of the next tile column
 #pragma unroll
                     for (int r = 0; r < 4; ++r) {
@@ -185,11 +187,18 @@ int dwconv_tma_try(const void* x, const void* wt, const void* bias, void* y, int
     if (nseg * DW_SEG > 248) nseg = 248 / DW_SEG;
     if (nseg < 1) return VIG_DWCONV_NOT_TAKEN;
     p.nseg = nseg; p.WB = nseg * DW_SEG; p.CC = CC;
-    p.box_bytes = 4u * (uint32_t)(p.WB + 2) * CC * 2u;
-    p.stage_bytes = (p.box_bytes + 1023u) & ~1023u;
-    const int smem = (int)(DW_STAGES * p.stage_bytes) + 16 * DW_STAGES + 16;
-    if (smem > 227 * 1024) return VIG_DWCONV_NOT_TAKEN;
-    p.ncb = C / CC; p.nxb = (w + p.WB - 1) / p.WB; p.nyb = (h + DW_ROWS - 1) / DW_ROWS;
+    // as many row pairs as there are threads for, evenly over the image's
+    const int pairs = (h + DW_ROWS - 1) / DW_ROWS;
+    int smem = 0;
+    for (p.nrp = DW_COMPUTE / (p.groups * nseg) < pairs ? DW_COMPUTE / (p.groups * nseg) : pairs;; --p.nrp) {
+        if (p.nrp < 1) return VIG_DWCONV_NOT_TAKEN;
+        p.nrp = (pairs + (pairs + p.nrp - 1) / p.nrp - 1) / ((pairs + p.nrp - 1) / p.nrp);
+        p.box_bytes = (uint32_t)(DW_ROWS * p.nrp + 2) * (uint32_t)(p.WB + 2) * CC * 2u;
+        p.stage_bytes = (p.box_bytes + 1023u) & ~1023u;
+        smem = (int)(DW_STAGES * p.stage_bytes) + 16 * DW_STAGES + 16;
+        if (smem <= 227 * 1024 && DW_ROWS * p.nrp + 2 <= 256) break;
+    }
+    p.ncb = C / CC; p.nxb = (w + p.WB - 1) / p.WB; p.nyb = (pairs + p.nrp - 1) / p.nrp;
     const int64_t ntiles = (int64_t)B * p.nyb * p.nxb * p.ncb;
     if (ntiles >= (1ll << 31)) return VIG_DWCONV_NOT_TAKEN;
     p.ntiles = (int)ntiles;
@@ -198,7 +207,7 @@ int dwconv_tma_try(const void* x, const void* wt, const void* bias, void* y, int
     key.base = x; key.rank = 4; key.dtype = dtype; key.swizzle = 0;
     key.dims[0] = (uint64_t)C; key.dims[1] = (uint64_t)w; key.dims[2] = (uint64_t)h; key.dims[3] = (uint64_t)B;
     key.strides[0] = (uint64_t)C * 2; key.strides[1] = (uint64_t)w * C * 2; key.strides[2] = (uint64_t)h * w * C * 2;
-    key.box[0] = (uint32_t)CC; key.box[1] = (uint32_t)(p.WB + 2); key.box[2] = 4; key.box[3] = 1;
+    key.box[0] = (uint32_t)CC; key.box[1] = (uint32_t)(p.WB + 2); key.box[2] = (uint32_t)(DW_ROWS * p.nrp + 2); key.box[3] = 1;
     CUtensorMap map;
     if (!tc::encode_cached(&map, key)) return VIG_DWCONV_NOT_TAKEN;
     int dev = 0, sms = 0;
