@@ -826,7 +826,7 @@ bool bigla_wave_supported(const BiglaParams& p) {
 
 // Measured on B200: with at least as many (sequence, direction) chains as SMs and two or more segments per sequence the
 // wavefront form beats the segment-parallel forms (0.46 against 0.58 ms at 64 x 3 sequences of 4096 tokens); with
-// fewer chains its CTAs idle, and a single segment has nothing to hand on.
+// fewer chains its CTAs idle.
 bool bigla_wave_preferred(const BiglaParams& p) {
     const int sms = wave_sm_count();
     const int ndir = p.dir_mask == 3 ? 2 : 1;
@@ -834,11 +834,15 @@ bool bigla_wave_preferred(const BiglaParams& p) {
     // work: 96 chains of 4096 tokens, dk = 64, 110 us against 142; 48 chains 107 against 79.  (dk = 32: 192 chains of 3136, 125
     // against 175.)
     const long long chains = (long long)p.B * p.H * ndir;
-    return sms > 0 && p.L > W_SEG_CHUNKS_MIN * CHUNK && chains * 16 >= sms * (p.dk == 64 ? 9ll : 13ll);
+    // One segment a sequence has nothing to hand on, but with many of them the roles of this form still overlap better: 768
+    // sequences of 196 tokens, dk = 64, 76 us against 84 (dk = 32: 76 against 68).
+    if (p.L <= W_SEG_CHUNKS_MIN * CHUNK) return sms > 0 && p.dk == 64 && chains >= 8ll * sms;
+    return sms > 0 && chains * 16 >= sms * (p.dk == 64 ? 9ll : 13ll);
 }
 
 // Counters (ticket, chain progress, chunk flags) followed by the state mailboxes.
 size_t bigla_wave_workspace(int B, int H, int L, int dk, int dv) {
+    if (L <= W_SEG_CHUNKS_MIN * CHUNK) return wave_counter_bytes(B, H, L);   // one step a chain: no mailbox
     (void)dk; (void)dv;                                     // the mailbox slots hold the kernel's 64 x 64 states whatever dk is
     return wave_counter_bytes(B, H, L) + (size_t)B * H * 2 * 2 * ((size_t)WDK * WDV + WDK) * sizeof(float);
 }
