@@ -31,11 +31,16 @@ template <int DK, int DV, typename T> struct SegTerms {
     static constexpr int RAW = Terms<T>::RAW, SC = (sizeof(T) == 2 && RAW == 1 && DV == 64) ? 1 : Terms<T>::SC;
 };
 
+// Warps that share 16 rows, each with its part of the value columns (the scores are formed by each of them): two for fp32, whose
+// three-term tiles leave room for one segment of at most 128 tokens an SM (2x3x196 64/64: 28.4 -> 20.0 us; 16x6x1000 64/64: 520 ->
+// 320).  16-bit inputs have two or three segments an SM and gain nothing from repeating the scores.
+template <typename T> struct SegWarps { static constexpr int CW = sizeof(T) == 4 ? 2 : 1; };
+
 template <int DK, int DV, typename T, int TOK> struct SegSmem {
     using TT = SegTerms<DK, DV, T>;
     static constexpr uint32_t QT = TT::SC * TOK * Pitch<DK>::B;        // one direction's Q or K terms
     static constexpr uint32_t V = 0, K = TT::RAW * TOK * Pitch<DV>::B, Q = K + 2 * QT, SUM = Q + 2 * QT,
-                              SCL = SUM + 2 * (TOK / 16) * DK * 4,      // per direction and warp: summed log-gates of the warp's rows
+                              SCL = SUM + 2 * (TOK / 16) * SegWarps<T>::CW * DK * 4,      // per direction and warp: summed log-gates of the warp's rows
                               BYTES = SCL + 4 * DK * 4;                 // [dir][0: 2^r, 1: 2^(l-r)]
     static_assert(TT::SC * DK * Pitch<DV>::B <= QT, "the entering states reuse the K tiles");
     static_assert(SUM >= TOK * DV * 4, "the exact form keeps its outputs in the tiles");
@@ -54,7 +59,7 @@ template <typename T, int SC> __device__ __forceinline__ void scaled(const Raw2<
 
 template <typename T, int COLS, int TERMS, int TOK> __device__ __forceinline__ void seg_load_v(uint8_t* dst, const T* src, int64_t stride_l, int n) {
     constexpr uint32_t P = Pitch<COLS>::B;
-    constexpr int NTH = 2 * TOK;
+    constexpr int NTH = 2 * TOK * SegWarps<T>::CW;
     if constexpr (TERMS == 1) {
         constexpr int VPR = COLS / 8;
 #pragma unroll
@@ -141,22 +146,22 @@ template <int DK, int DV, typename T, int MODE> __device__ __noinline__ void exa
 }
 
 template <int DK, int DV, typename T, int TOK> constexpr int seg_min_blocks() {
-    constexpr int fit = 225 * 1024 / (int)(SegSmem<DK, DV, T, TOK>::BYTES + 1024), regs = 512 / (2 * TOK);      // 128 registers a thread
+    constexpr int fit = 225 * 1024 / (int)(SegSmem<DK, DV, T, TOK>::BYTES + 1024), regs = 512 / (2 * TOK * SegWarps<T>::CW);      // 128 registers a thread
     return fit < 1 ? 1 : fit < regs ? fit : regs;
 }
 
 template <int DK, int DV, typename T, int TOK, int MODE>
-__global__ void __launch_bounds__(2 * TOK, seg_min_blocks<DK, DV, T, TOK>()) bigla_seg_kernel(const __grid_constant__ SegParams s) {
+__global__ void __launch_bounds__(2 * TOK * SegWarps<T>::CW, seg_min_blocks<DK, DV, T, TOK>()) bigla_seg_kernel(const __grid_constant__ SegParams s) {
     using SM = SegSmem<DK, DV, T, TOK>;
-    constexpr int RAW = SM::TT::RAW, SC = SM::TT::SC, NTH = 2 * TOK, W = NTH / 32;
-    constexpr int PAIRS = DK / 2, SUB = 32 / PAIRS, RPG = 16 / SUB, MT = DK / 16;   // a warp's gates: 16 rows, SUB groups of RPG
+    constexpr int RAW = SM::TT::RAW, SC = SM::TT::SC, CW = SegWarps<T>::CW, NTH = 2 * TOK * CW, W = NTH / 32, DC = DV / CW;   // DC: a warp's value columns
+    constexpr int PAIRS = DK / 2, SUB = 32 / PAIRS, RPG = 16 / CW / SUB, MT = DK / 16;   // a warp's gates: 16 / CW rows, SUB groups of RPG
     constexpr uint32_t PK = Pitch<DK>::B, PV = Pitch<DV>::B, TK = TOK * PK, TV = TOK * PV, TS = DK * PV;   // TK, TV, TS: from term to term
     const BiglaParams& p = s.p;
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t sb = tc::smem_u32(smem);
     float* gsum = reinterpret_cast<float*>(smem + SM::SUM);              // [dir][warp][DK]
     float* scl = reinterpret_cast<float*>(smem + SM::SCL);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, rb = w / CW, cb = w % CW;     // my block of 16 rows and part of the value columns in the products
     const int c = blockIdx.x, bh = blockIdx.y, b = bh / p.H, h = bh % p.H;
     const int64_t t0 = (int64_t)c * s.seglen;
     const int n = min(s.seglen, p.L - (int)t0), nb = (n + 15) / 16;
@@ -239,7 +244,7 @@ __global__ void __launch_bounds__(2 * TOK, seg_min_blocks<DK, DV, T, TOK>()) big
             }
         }
         __syncthreads();
-        const int wm = nb / 2;                                           // the reference lies between the rows of warps wm - 1 and wm
+        const int wm = nb / 2 * CW;                                           // the reference lies between the rows of warps wm - 1 and wm
         const float lim = range_limit<T>();
 #pragma unroll
         for (int dir = 0; dir < 2; ++dir) {
@@ -265,7 +270,7 @@ __global__ void __launch_bounds__(2 * TOK, seg_min_blocks<DK, DV, T, TOK>()) big
                 if (MODE != SEG_OUT && s.need_states && (dir ? bwd : fwd))
                     *reinterpret_cast<float2*>(p.ws_decay + (((size_t)bh * s.nseg + c) * 2 + dir) * DK + 2 * pr) = make_float2(f2_lo(run) * tc::LN2, f2_hi(run) * tc::LN2);
             }
-            if (!(dir ? bwd : fwd) || w >= nb) continue;
+            if (!(dir ? bwd : fwd) || rb >= nb) continue;
             uint8_t* kt = smem + SM::K + dir * SM::QT + r0 * PK + pr * 4;
             uint8_t* qt = smem + SM::Q + dir * SM::QT + r0 * PK + pr * 4;
             const F2 shift = MODE == SEG_STATES ? f2_fma(run, minus, off) : f2_fma(ref[dir], minus, off);    // G - (total or reference)
@@ -292,7 +297,7 @@ __global__ void __launch_bounds__(2 * TOK, seg_min_blocks<DK, DV, T, TOK>()) big
 #pragma unroll
         for (int dir = 0; dir < 2; ++dir) {
             if (gr == 0) *reinterpret_cast<float2*>(scl + dir * 2 * DK + DK + 2 * pr) = make_float2(1.f, 1.f);
-            if (w >= nb) continue;
+            if (rb >= nb) continue;
             const F2 rest = f2_fma(ref[dir], minus, tot[dir]);           // G holds G - ref
 #pragma unroll
             for (int r = 0; r < RPG; ++r) {
@@ -335,14 +340,14 @@ __global__ void __launch_bounds__(2 * TOK, seg_min_blocks<DK, DV, T, TOK>()) big
         if (MODE == SEG_STATES) return;
         if (s.nseg > 1) cluster_arrive();
     }
-    float o[DV / 8][4];
+    float o[DC / 8][4];
 #pragma unroll
-    for (int i = 0; i < DV / 8; ++i)
+    for (int i = 0; i < DC / 8; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) o[i][j] = 0.f;
-    const uint32_t aQ = sb + SM::Q + 16 * w * PK + frag_rows<PK>(lane);
-    if (want_out && !bad && w < nb) {                                    // ---- products inside the segment, my 16 rows
-        const uint32_t bK = sb + SM::K + frag_cols<PK>(lane), tV = sb + SM::V + frag_rows<PV>(lane);
+    const uint32_t aQ = sb + SM::Q + 16 * rb * PK + frag_rows<PK>(lane);
+    if (want_out && !bad && rb < nb) {                                    // ---- products inside the segment, my 16 rows
+        const uint32_t bK = sb + SM::K + frag_cols<PK>(lane), tV = sb + SM::V + cb * DC * 2 + frag_rows<PV>(lane);
         uint32_t ap[SC][4];
 #pragma unroll 1
         for (int dir = 0; dir < 2; ++dir) {                              // off-diagonal blocks: before mine with the forward tiles, after it with the backward ones
@@ -353,9 +358,9 @@ __global__ void __launch_bounds__(2 * TOK, seg_min_blocks<DK, DV, T, TOK>()) big
             for (int ks = 0; ks < DK / 16; ++ks)
 #pragma unroll
                 for (int t = 0; t < SC; ++t) ldsm4(q + t * TK + ks * 32, fq[ks][t]);
-            const int j1 = dir ? nb : w;
+            const int j1 = dir ? nb : rb;
 #pragma unroll 1
-            for (int jb = dir ? w + 1 : 0; jb < j1; jb += 2) {           // two blocks at a time: four independent chains of products
+            for (int jb = dir ? rb + 1 : 0; jb < j1; jb += 2) {           // two blocks at a time: four independent chains of products
                 const bool two = jb + 1 < j1;
                 float pb[4][4];
 #pragma unroll
@@ -374,10 +379,10 @@ __global__ void __launch_bounds__(2 * TOK, seg_min_blocks<DK, DV, T, TOK>()) big
                     }
                 }
                 mask_split<SC>(pb, false, lane, [](int, int) { return true; }, ap);
-                block_nn<DV, SC, RAW>(o, ap, tV + jb * 16 * PV, TV);
+                block_nn<DC, SC, RAW>(o, ap, tV + jb * 16 * PV, TV);
                 if (two) {
                     mask_split<SC>(pb + 2, false, lane, [](int, int) { return true; }, ap);
-                    block_nn<DV, SC, RAW>(o, ap, tV + (jb + 1) * 16 * PV, TV);
+                    block_nn<DC, SC, RAW>(o, ap, tV + (jb + 1) * 16 * PV, TV);
                 }
             }
         }
@@ -386,7 +391,7 @@ __global__ void __launch_bounds__(2 * TOK, seg_min_blocks<DK, DV, T, TOK>()) big
         for (int dir = 0; dir < 2; ++dir) {                              // the diagonal block: both directions' halves, a token sees itself in each
             if (!(dir ? bwd : fwd)) continue;
             float pb[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-            block_nt<DK, SC, SC>(pb, aQ + dir * SM::QT, TK, bK + dir * SM::QT + w * 16 * PK, TK);
+            block_nt<DK, SC, SC>(pb, aQ + dir * SM::QT, TK, bK + dir * SM::QT + rb * 16 * PK, TK);
             const int r = lane >> 2, q = 2 * (lane & 3);
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt)
@@ -397,7 +402,7 @@ __global__ void __launch_bounds__(2 * TOK, seg_min_blocks<DK, DV, T, TOK>()) big
                 }
         }
         mask_split<SC>(pd, false, lane, [](int, int) { return true; }, ap);
-        block_nn<DV, SC, RAW>(o, ap, tV + w * 16 * PV, TV);
+        block_nn<DC, SC, RAW>(o, ap, tV + rb * 16 * PV, TV);
     }
     const bool has_init = MODE == SEG_ONE && (p.init_f || p.init_b);
     if (MODE == SEG_ONE && s.nseg > 1) cluster_wait();                   // the other segments' contributions have landed
@@ -480,29 +485,29 @@ __global__ void __launch_bounds__(2 * TOK, seg_min_blocks<DK, DV, T, TOK>()) big
             }
         }
         __syncthreads();
-        if (w < nb) {
+        if (rb < nb) {
 #pragma unroll 1
             for (int dir = 0; dir < 2; ++dir) {
                 if (!(dir ? bwd : fwd)) continue;
-                const uint32_t tS = sb + SM::K + dir * SM::QT + frag_rows<PV>(lane);
+                const uint32_t tS = sb + SM::K + dir * SM::QT + cb * DC * 2 + frag_rows<PV>(lane);
 #pragma unroll
                 for (int ks = 0; ks < DK / 16; ++ks) {
                     uint32_t fa[SC][4];
 #pragma unroll
                     for (int t = 0; t < SC; ++t) ldsm4(aQ + dir * SM::QT + t * TK + ks * 32, fa[t]);
-                    block_nn<DV, SC, SC>(o, fa, tS + ks * 16 * PV, TS);
+                    block_nn<DC, SC, SC>(o, fa, tS + ks * 16 * PV, TS);
                 }
             }
         }
     }
-    if (w >= nb) return;
+    if (rb >= nb) return;
 #pragma unroll
     for (int hf = 0; hf < 2; ++hf) {
-        const int row = 16 * w + (lane >> 2) + 8 * hf;
+        const int row = 16 * rb + (lane >> 2) + 8 * hf;
         if (row >= n) continue;
-        T* out = reinterpret_cast<T*>(p.o) + b * p.so[0] + h * p.so[1] + (t0 + row) * p.so[2] + 2 * (lane & 3);
+        T* out = reinterpret_cast<T*>(p.o) + b * p.so[0] + h * p.so[1] + (t0 + row) * p.so[2] + cb * DC + 2 * (lane & 3);
 #pragma unroll
-        for (int i = 0; i < DV / 8; ++i) store2<T>(out + 8 * i, p.qscale * o[i][2 * hf], p.qscale * o[i][2 * hf + 1]);
+        for (int i = 0; i < DC / 8; ++i) store2<T>(out + 8 * i, p.qscale * o[i][2 * hf], p.qscale * o[i][2 * hf + 1]);
     }
 }
 
@@ -514,7 +519,7 @@ int seg_launch_mode(const SegParams& s, cudaStream_t stream) {
     if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(s.nseg, s.p.B * s.p.H);
-    cfg.blockDim = dim3(2 * TOK);
+    cfg.blockDim = dim3(2 * TOK * SegWarps<T>::CW);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
