@@ -47,6 +47,7 @@ __global__ void __launch_bounds__(NT) bwd_states_mma_kernel(const __grid_constan
         load_rows(x, (dir ? head_ptr<T>(p.gb, p.sgb, b, h, t0) : head_ptr<T>(p.gf, p.sgf, b, h, t0)) + 2 * pr, dir ? p.sgb[2] : p.sgf[2], r0, n);
     };
     const int first = one_dir ? blockIdx.z : p.dir_mask & 1 ? 0 : 1;
+    pdl_launch();
     load_gate(first);
     load_rows(k, head_ptr<T>(p.k, p.sk, b, h, t0) + 2 * pr, p.sk[2], r0, n);
     load_rows(q, head_ptr<T>(p.q, p.sq, b, h, t0) + 2 * pr, p.sq[2], r0, n);
@@ -95,6 +96,8 @@ __global__ void __launch_bounds__(NT) bwd_states_mma_kernel(const __grid_constan
 
 // ---- scan over chunks: local states -> entering states, in place.  S in scan order, Z against it. ---------------------
 __global__ void __launch_bounds__(256, 2) bwd_scan_kernel(const __grid_constant__ BwdParams p) {
+    pdl_launch();
+    pdl_wait();
     const int per = p.dk * p.dv / 4;
     const int64_t it = (int64_t)blockIdx.x * 256 + threadIdx.x;
     const int e = (int)(it % per);
@@ -155,6 +158,8 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 1 : 2) bwd_grads_mma_kern
     const uint32_t bV = sb + SM::V + frag_cols<PV>(lane), bO = sb + SM::O + frag_cols<PV>(lane), bQ = sb + SM::Q + frag_cols<PK>(lane);
     const uint32_t tK = sb + SM::K + frag_rows<PK>(lane), tQ = sb + SM::Q + frag_rows<PK>(lane), tO = sb + SM::O + frag_rows<PV>(lane);
     const bool have_states = p.nchunk > 1;
+    pdl_launch();
+    pdl_wait();
     if (have_states) {                                                   // both directions' states on their way to L2 while the tiles are made
         constexpr int LINES = DK * DV * 4 / 128;
         for (int i = threadIdx.x; i < 4 * LINES; i += NT) {
@@ -365,8 +370,7 @@ int launch_typed(const BwdParams& p, cudaStream_t stream) {
         if (int s = bigla_bwd_scan_launch(p, stream)) return s;
     }
     if ((e = tc::ensure_smem_attr(reinterpret_cast<const void*>(kC), (int)smC)) != cudaSuccess) return (int)e;
-    kC<<<dim3(p.nchunk, BH), NT, smC, stream>>>(p);
-    return (int)cudaGetLastError();
+    return (int)launch_overlapped(p.nchunk > 1, kC, dim3(p.nchunk, BH), dim3(NT), smC, stream, p);
 }
 
 template <typename T>
@@ -381,8 +385,7 @@ int launch_dims(const BwdParams& p, cudaStream_t stream) {
 
 int bigla_bwd_scan_launch(const BwdParams& p, cudaStream_t stream) {
     const int64_t threads = (int64_t)p.B * p.H * (p.dir_mask == 3 ? 2 : 1) * 2 * (p.dk * p.dv / 4);
-    bwd_scan_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, stream>>>(p);
-    return (int)cudaGetLastError();
+    return (int)launch_next(bwd_scan_kernel, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, stream, p);
 }
 
 // Rows are read as 16-byte vectors (16-bit v, d_out) or as pairs of values: base pointers on 16 bytes, strides that are

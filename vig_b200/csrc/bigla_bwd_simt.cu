@@ -128,6 +128,7 @@ __global__ void __launch_bounds__(NT) bwd_chunk_grads(BwdParams p, int flagged_o
     float* sv = sdk + CH * DK;
     float* sdo = sv + CH * DV;
     float* sdv = sdo + CH * DV;
+    pdl_wait();
     const bool have_states = !flagged_only || p.nchunk > 1;          // the tensor-core form leaves the states of a lone chunk unwritten (zero)
     const int items = p.nchunk * p.B * p.H;
     for (int item = blockIdx.x, look = 0; item < items; item += gridDim.x, ++look) {
@@ -284,8 +285,7 @@ int launch_typed(const BwdParams& p, int flagged_only, cudaStream_t stream) {
     const int items = p.nchunk * p.B * p.H;
     // flagged chunks are rare: a CTA per SM (the tiles fill its shared memory) walks the flags; as one CTA per chunk the
     // launch alone took 15 us for 3072 unflagged chunks
-    kC<<<flagged_only ? (items < 148 ? items : 148) : items, NT, smC, stream>>>(p, flagged_only);
-    return (int)cudaGetLastError();
+    return (int)launch_next(kC, dim3(flagged_only ? (items < 148 ? items : 148) : items), dim3(NT), smC, stream, p, flagged_only);
 }
 
 template <typename T>

@@ -32,7 +32,7 @@ template <int DK, int DV, typename T> struct SegTerms {
 };
 
 // Warps that share 16 rows, each with its part of the value columns (the scores are formed by each of them): two for fp32, whose
-// three-term tiles leave room for one segment of at most 128 tokens an SM (2x3x196 64/64: 28.4 -> 20.0 us; 16x6x1000 64/64: 520 ->
+// three-term tiles leave room for one or two 64-token segments an SM (2x3x196 64/64: 28.4 -> 20.0 us; 16x6x1000 64/64: 520 ->
 // 320).  16-bit inputs have two or three segments an SM and gain nothing from repeating the scores.
 template <typename T> struct SegWarps { static constexpr int CW = sizeof(T) == 4 ? 2 : 1; };
 
@@ -406,7 +406,10 @@ __global__ void __launch_bounds__(2 * TOK * SegWarps<T>::CW, seg_min_blocks<DK, 
     }
     const bool has_init = MODE == SEG_ONE && (p.init_f || p.init_b);
     if (MODE == SEG_ONE && s.nseg > 1) cluster_wait();                   // the other segments' contributions have landed
-    else __syncthreads();
+    else {
+        if (MODE == SEG_OUT) pdl_wait();                                 // all before this overlaps the scan over segments
+        __syncthreads();
+    }
     if (MODE == SEG_ONE && s.need_states) {
 #pragma unroll 1
         for (int dir = 0; dir < 2; ++dir) {                              // final states, summed log-gates: by the segment scanned last
@@ -522,6 +525,7 @@ int seg_launch_mode(const SegParams& s, cudaStream_t stream) {
     cfg.blockDim = dim3(2 * TOK * SegWarps<T>::CW);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
+    if (MODE == SEG_OUT) return (int)launch_next(kern, cfg.gridDim, cfg.blockDim, smem, stream, s);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = s.nseg; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;

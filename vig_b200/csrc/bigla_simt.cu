@@ -100,6 +100,8 @@ __global__ void __launch_bounds__(NT) bigla_simt_chunk_state(BiglaParams p) {
 
 // Phase B: one thread per four neighbouring state elements, sequential over chunks in scan order.
 __global__ void __launch_bounds__(NT, 2) bigla_simt_state_scan(BiglaParams p) {
+    pdl_launch();
+    pdl_wait();
     const int per = p.dk * p.dv / 4;
     const int64_t it = (int64_t)blockIdx.x * NT + threadIdx.x;
     const int e = (int)(it % per), dir = (int)(it / per % 2);
@@ -209,8 +211,7 @@ size_t bigla_simt_workspace(int B, int H, int L, int dk, int dv) {
 
 int bigla_scan_launch(const BiglaParams& p, cudaStream_t stream) {
     const int64_t threads = (int64_t)p.B * p.H * 2 * (p.dk * p.dv / 4);
-    bigla_simt_state_scan<<<(unsigned)((threads + NT - 1) / NT), NT, 0, stream>>>(p);
-    return (int)cudaGetLastError();
+    return (int)launch_next(bigla_simt_state_scan, dim3((unsigned)((threads + NT - 1) / NT)), dim3(NT), 0, stream, p);
 }
 
 int bigla_simt_launch(const BiglaParams& p_in, cudaStream_t stream) {

@@ -101,6 +101,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bigla_tc_kernel(const __grid_cons
         if (FUSED) *item_slot = (int)atomicAdd(p.ticket, 1u);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (MODE == 0) pdl_wait();                    // the scan over segments; before tensor memory is taken
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -109,6 +110,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) bigla_tc_kernel(const __grid_cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    if (STATES_ONLY) pdl_launch();
 
     // ---- thread roles ---------------------------------------------------------------------------
     // gate preparation: CPW lanes cover the channel pairs of one token row; a warp covers 32/CPW rows at once
@@ -696,7 +698,7 @@ int launch_tc(const BiglaParams& p_in, const TcMaps& maps, bool allow_fused, cud
     }
     if (p.o) {
         if ((e = ensure_smem_attr(reinterpret_cast<const void*>(kC), SMEM_BYTES)) != cudaSuccess) return (int)e;
-        kC<<<grid, NTHREADS, SMEM_BYTES, stream>>>(maps, p, use_ws);
+        return (int)launch_overlapped(use_ws, kC, grid, dim3(NTHREADS), SMEM_BYTES, stream, maps, p, use_ws);
     }
     return (int)cudaGetLastError();
 }

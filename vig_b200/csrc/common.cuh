@@ -120,16 +120,28 @@ __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.laun
 extern thread_local int chain_launches;
 
 template <typename... K, typename... A>
-inline cudaError_t launch_chained(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+inline cudaError_t launch_overlapped(bool overlap, void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = chain_launches ? 1 : 0;
+    cfg.numAttrs = overlap ? 1 : 0;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, K(args)...);
     return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+template <typename... K, typename... A>
+inline cudaError_t launch_chained(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+    return launch_overlapped(chain_launches != 0, kernel, grid, block, smem, stream, std::forward<A>(args)...);
+}
+
+// A later launch of one call, behind a first one in the ordinary way: the call's inputs were complete before that one began, so
+// they may be read before pdl_wait(), and only what the call itself wrote has to be waited for.
+template <typename... K, typename... A>
+inline cudaError_t launch_next(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+    return launch_overlapped(true, kernel, grid, block, smem, stream, std::forward<A>(args)...);
 }
 
 // Parameter block of the bi-GLA launchers (host fills it from the C ABI arguments).
