@@ -115,6 +115,13 @@ template <typename T> __device__ __forceinline__ float gelu_t(float x) {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// What an earlier kernel writes is not read through the non-coherent path by one that may have begun before that write.
+__device__ __forceinline__ uint2 ld_coherent(const void* p) {
+    uint2 v;
+    asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+
 // Whether this thread's launches may be chained: set around a model's forward, whose kernels read weights -- which none of them
 // writes -- before pdl_wait().
 extern thread_local int chain_launches;

@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(EW_THREADS, 2) dwconv3x3_rows_kernel(const T* 
     auto load_col = [&](int xx, uint2* raw) {                 // the three inputs of image column xx (zeros outside the image)
 #pragma unroll
         for (int ky = 0; ky < 3; ++ky)
-            raw[ky] = (rok[ky] && xx >= 0 && xx < w) ? __ldg(reinterpret_cast<const uint2*>(rowp[ky] + (size_t)xx * C)) : make_uint2(0u, 0u);
+            raw[ky] = (rok[ky] && xx >= 0 && xx < w) ? ld_coherent(rowp[ky] + (size_t)xx * C) : make_uint2(0u, 0u);
     };
     float win[3][3][4];                                       // [column slot][row][channel]; slot of image column xx is (xx - x0 + 1) % 3
     constexpr int PF = 3;                                     // columns in flight
