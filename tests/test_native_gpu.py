@@ -82,3 +82,20 @@ def test_small_forwards_are_replayed_and_stay_independent():
         assert all(torch.equal(o, ref[i % 3]) for i, o in enumerate(outs))
         m.head.bias.add_(1.0)
         assert torch.equal(m(xs[0]), m(xs[0])) and not torch.equal(m(xs[0]), ref[0])
+
+
+@pytest.mark.parametrize("kind", ["vig_s", "hier", "hier_mlp"])
+def test_replay_reads_the_images_of_its_call(kind):
+    """The kernel in front of the replayed part (8 x 8 cells with a border, the embedding's first convolution, the change to
+    channels-last) writes its input from the images at hand, whatever their strides: same kernels, same bits."""
+    m = _model(kind, torch.float16)
+    xs = [torch.randn(2, 3, 64, 96, device="cuda").half() for _ in range(2)]
+    xs.append(torch.randn(2, 3, 64, 192, device="cuda").half()[..., ::2])
+    with torch.no_grad():
+        from vig_b200 import native
+        ref = []
+        for x in xs:
+            native._plans.clear()
+            ref.append(m(x))
+        for _ in range(2):
+            assert all(torch.equal(m(x), r) for x, r in zip(xs, ref))

@@ -187,12 +187,15 @@ struct PlanBase {
                !(at::GradMode::is_enabled()) && !at::autocast::is_autocast_enabled(at::kCUDA) && status_known(device.index()) && watch.same();
     }
     Tensor finish(const Tensor& pooled) const { return at::linear(pooled, head_w, head_b.defined() ? OptT(head_b) : std::nullopt); }
-    // One forward.  ``work``: a measure of the activations (tokens x channels).  Small forwards are bound by their launches, on
-    // the host (5 - 10 us each through the GEMM library) and on the device (1.4 us between kernels): from the second call of a
-    // shape on a stream they are captured into a CUDA graph and replayed, with the images copied into the graph's input.  The
-    // graph and its memory (about 24 bytes per activation element, GRAPH_WORK elements in all per plan) belong to this plan, one
-    // per shape and stream, the least recently used given back first, and go with it.
-    static constexpr int64_t GRAPH_WORK = 8 << 20;
+    // One forward.  ``work``: a measure of the activations (tokens x channels).  Launched one by one, a forward of 50 to 150
+    // kernels spends 5 - 10 us a launch on the host (through the GEMM library), which small forwards wait for, and 1.4 us
+    // between kernels on the device, 7 % of one of three milliseconds (128 images of 224 x 224, width 384: 3465 -> 3220 us; 64
+    // through the hierarchical model 3380 -> 3100; 64 of 1024 x 1024, width 192: 11.6 -> 11.45 ms).  So from the second call of a
+    // shape on a stream it is captured into a CUDA graph and replayed.  The first kernel, which reads the images, stays outside
+    // and writes the graph's input, so that nothing is copied.  The graph and its memory (about 45 bytes per activation element,
+    // GRAPH_WORK elements in all per plan: 3 GB) belong to this plan, one per shape and stream, the least recently used given
+    // back first, and go with it.  Larger forwards gain little (8 of 2048 x 2048: 0.4 %) and would hold more.
+    static constexpr int64_t GRAPH_WORK = 64 << 20;
     struct Captured {
         int64_t B, H, W, work;
         cudaStream_t stream;
@@ -229,13 +232,12 @@ struct PlanBase {
         captured.emplace_back(x, work, st, ++clock);
         return captured.back();
     }
-    template <typename F> void capture(Captured& e, const Tensor& x, F body, const Ctx& c) {
+    template <typename F> void capture(Captured& e, const Tensor& x, F rest, const Ctx& c) {
         // one capture stream per device; a GEMM on it beforehand, so that the library's workspace for it is an ordinary allocation
         static std::unordered_map<int, at::cuda::CUDAStream>* streams = new std::unordered_map<int, at::cuda::CUDAStream>();
         auto it = streams->find(device.index());
         const bool fresh = it == streams->end();
         if (fresh) it = streams->emplace(device.index(), at::cuda::getStreamFromPool(false, device.index())).first;
-        e.in = at::empty(x.sizes(), x.options());
         c10::cuda::CUDAStreamGuard guard(it->second);
         if (fresh) {
             const Tensor a = at::zeros({16, 64}, x.options()), b = at::zeros({64}, x.options());
@@ -245,7 +247,7 @@ struct PlanBase {
         auto g = std::make_unique<at::cuda::CUDAGraph>();
         g->capture_begin({0, 0}, cudaStreamCaptureModeThreadLocal);
         try {
-            e.out = body(Ctx{it->second.stream(), c.status, c.code}, e.in);
+            e.out = rest(Ctx{it->second.stream(), c.status, c.code}, e.in);
         } catch (...) {
             e.failed = true;
         }
@@ -255,7 +257,8 @@ struct PlanBase {
         e.done = std::make_unique<at::cuda::CUDAEvent>();
     }
 
-    template <typename F> OptT run(const Tensor& x, int64_t work, F body) {
+    // ``first(c, images, y)``: the first kernel, into y (allocated if undefined); ``rest(c, y)``: everything behind it
+    template <typename F, typename R> OptT run(const Tensor& x, int64_t work, F first, R rest) {
         if (!takes(x)) return std::nullopt;
         c10::cuda::CUDAGuard guard(device);
         at::NoGradGuard ng;
@@ -270,15 +273,21 @@ struct PlanBase {
         Tensor y;
         if (!capturing && work <= GRAPH_WORK) {
             Captured& e = entry(x, st.stream(), work);
-            if (!e.graph && !e.failed && e.seen++ > 0) capture(e, x, body, c);
+            if (e.graph || (!e.failed && e.seen++ > 0)) {
+                first(c, x.contiguous(), e.in);
+                if (!e.graph) capture(e, x, rest, c);
+            }
             if (e.graph) {
-                e.in.copy_(x, true);
                 e.graph->replay();
                 y = e.out.clone();
                 e.done->record(st);
             }
         }
-        if (!y.defined()) y = body(c, x.contiguous());
+        if (!y.defined()) {
+            Tensor t;
+            first(c, x.contiguous(), t);
+            y = rest(c, t);
+        }
         peek.snapshot(device.index(), st.stream(), capturing);
         return y;
     }
@@ -309,21 +318,24 @@ struct VigPlan : PlanBase {
     OptT forward(const Tensor& x) {
         const int64_t H = x.dim() == 4 ? x.size(2) : 0, W = x.dim() == 4 ? x.size(3) : 0;
         if (H % 8 || W % 8 || H == 0) return std::nullopt;
-        return run(x, x.size(0) * ((H + 15) / 16) * ((W + 15) / 16) * C, [&](const Ctx& c, const Tensor& img) { return body(c, img); });
+        return run(x, x.size(0) * ((H + 15) / 16) * ((W + 15) / 16) * C, [&](const Ctx& c, const Tensor& img, Tensor& f) { first(c, img, f); },
+                   [&, B = x.size(0)](const Ctx& c, const Tensor& f) { return rest(c, f, B, H, W); });
     }
-    Tensor body(const Ctx& c, const Tensor& img) const {
-        const int64_t B = img.size(0), H = img.size(2), W = img.size(3);
+    bool folds(const Ctx& c, int64_t B, int64_t H, int64_t W) const { return w_gemm.defined() && api.vig_stem_conv_ln_supported(B, H / 8, W / 8, 192, C / 2, c.code); }
+    void first(const Ctx& c, const Tensor& img, Tensor& f) const {       // 8 x 8 pixel cells, with a border of cells for the 2 x 2 convolution
+        const int64_t B = img.size(0), H = img.size(2), W = img.size(3), edge = folds(c, B, H, W) ? 0 : 1;
+        if (!f.defined()) f = at::empty({B, H / 8 + edge, W / 8 + edge, 192}, img.options());
+        if (edge) ok(api.vig_stem_unfold_fwd(ptr(img), ptr(f), B, 3, H, W, 8, c.code, c.stream), "vig_stem_unfold_fwd");
+        else ok(api.vig_stem_fold_fwd(ptr(img), ptr(f), B, 3, H, W, c.code, c.stream), "vig_stem_fold_fwd");
+    }
+    Tensor rest(const Ctx& c, const Tensor& f, int64_t B, int64_t H, int64_t W) const {
         Tensor y;
-        if (w_gemm.defined() && api.vig_stem_conv_ln_supported(B, H / 8, W / 8, 192, C / 2, c.code)) {
-            Tensor f = at::empty({B, H / 8, W / 8, 192}, img.options());
-            ok(api.vig_stem_fold_fwd(ptr(img), ptr(f), B, 3, H, W, c.code, c.stream), "vig_stem_fold_fwd");
-            y = at::empty({B, H / 8, W / 8, C / 2}, img.options());
+        if (folds(c, B, H, W)) {
+            y = at::empty({B, H / 8, W / 8, C / 2}, f.options());
             ok(api.vig_stem_conv_ln_fwd(ptr(f), ptr(w_gemm), ptr(b1), ptr(ln1_w), ptr(ln1_b), ptr(y), B, H / 8, W / 8, 192, C / 2, (float)ln1_e, 1, c.code, c.status,
                                         c.stream), "vig_stem_conv_ln_fwd");
         } else {
-            Tensor u = at::empty({B, H / 8 + 1, W / 8 + 1, 192}, img.options());
-            ok(api.vig_stem_unfold_fwd(ptr(img), ptr(u), B, 3, H, W, 8, c.code, c.stream), "vig_stem_unfold_fwd");
-            y = layernorm(c, cells.forward(u, false), ln1_w, ln1_b, ln1_e, true, b1);
+            y = layernorm(c, cells.forward(f, false), ln1_w, ln1_b, ln1_e, true, b1);
         }
         y = conv2.forward(y, false);
         const int64_t h = y.size(1), w = y.size(2), L = h * w, rows = B * L;
@@ -331,9 +343,9 @@ struct VigPlan : PlanBase {
             pos = pos_fn(py::make_tuple(h, w)).cast<Tensor>().to(type).contiguous();
             pos_h = h; pos_w = w;
         }
-        Tensor tok = at::empty({B, L, C}, img.options());
+        Tensor tok = at::empty({B, L, C}, f.options());
         if (fused_norms) {
-            Tensor n = at::empty({B, L, C}, img.options());
+            Tensor n = at::empty({B, L, C}, f.options());
             ok(api.vig_layernorm_act_add_rmsnorm_fwd(ptr(y), ptr(conv2.b), ptr(ln2_w), ptr(ln2_b), ptr(pos), L, ptr(tok), ptr(blocks[0].n1), (float)blocks[0].e1,
                                                      ptr(n), rows, C, (float)ln2_e, 0, c.code, c.stream), "vig_layernorm_act_add_rmsnorm_fwd");
             for (size_t i = 0; i < blocks.size(); ++i) {
@@ -400,22 +412,25 @@ struct HierPlan : PlanBase {
     Norm last;
 
     OptT forward(const Tensor& x) {
-        return run(x, x.dim() == 4 ? x.size(0) * ((x.size(2) + 3) / 4) * ((x.size(3) + 3) / 4) * std::get<0>(embed.back()).w.size(0) : 0, [&](const Ctx& c, const Tensor& img) { return body(c, img); });
+        return run(x, x.dim() == 4 ? x.size(0) * ((x.size(2) + 3) / 4) * ((x.size(3) + 3) / 4) * std::get<0>(embed.back()).w.size(0) : 0, [&](const Ctx& c, const Tensor& img, Tensor& y) { first(c, img, y); },
+                   [&](const Ctx& c, const Tensor& y) { return rest(c, y); });
     }
-    Tensor body(const Ctx& c, const Tensor& img) const {
-        Tensor y;
-        size_t done = 0;
+    void first(const Ctx& c, const Tensor& img, Tensor& y) const {
+        const int64_t B = img.size(0), H = img.size(2), W = img.size(3);
         if (first_w.defined()) {                             // the first convolution with its norm and activation, from the image as it is
             const auto& [conv, has_norm, norm, act] = embed[0];
-            const int64_t B = img.size(0), H = img.size(2), W = img.size(3), O = first_w.size(0);
-            y = at::empty({B, (H + 1) / 2, (W + 1) / 2, O}, img.options());
+            const int64_t O = first_w.size(0);
+            if (!y.defined()) y = at::empty({B, (H + 1) / 2, (W + 1) / 2, O}, img.options());
             ok(api.vig_embed_conv_ln_fwd(ptr(img), ptr(first_w), ptr(conv.b), ptr(norm.w), ptr(norm.b), ptr(y), B, H, W, O, (float)norm.eps, act == 2, c.code, c.stream),
                "vig_embed_conv_ln_fwd");
-            done = 1;
-        } else {
-            y = img.permute({0, 2, 3, 1}).contiguous();
+        } else {                                             // channels-last
+            if (!y.defined()) y = at::empty({B, H, W, img.size(1)}, img.options());
+            y.copy_(img.permute({0, 2, 3, 1}));
         }
-        for (size_t i = done; i < embed.size(); ++i) {
+    }
+    Tensor rest(const Ctx& c, const Tensor& first_out) const {
+        Tensor y = first_out;
+        for (size_t i = first_w.defined() ? 1 : 0; i < embed.size(); ++i) {
             const auto& [conv, has_norm, norm, act] = embed[i];
             y = conv.forward(y, !has_norm);                      // the bias rides in the norm
             if (has_norm) y = add_layernorm(c, y, {}, norm, act, conv.b).first;
