@@ -84,18 +84,23 @@ def test_small_forwards_are_replayed_and_stay_independent():
         assert torch.equal(m(xs[0]), m(xs[0])) and not torch.equal(m(xs[0]), ref[0])
 
 
-@pytest.mark.parametrize("kind", ["vig_s", "hier", "hier_mlp"])
+@pytest.mark.parametrize("kind", ["vig_t", "vig_s", "hier", "hier_mlp"])
 def test_replay_reads_the_images_of_its_call(kind):
-    """The kernel in front of the replayed part (8 x 8 cells with a border, the embedding's first convolution, the change to
-    channels-last) writes its input from the images at hand, whatever their strides: same kernels, same bits."""
+    """The kernel in front of the replayed part (8 x 8 cells, with or without a border, the embedding's first convolution, the
+    change to channels-last) writes its input from the images at hand, whatever their strides: same kernels, same bits.  Forwards
+    of another size in between, and memory that they give back and others fill, change nothing."""
     m = _model(kind, torch.float16)
     xs = [torch.randn(2, 3, 64, 96, device="cuda").half() for _ in range(2)]
     xs.append(torch.randn(2, 3, 64, 192, device="cuda").half()[..., ::2])
+    other = torch.randn(1, 3, 96, 32, device="cuda").half()
     with torch.no_grad():
         from vig_b200 import native
         ref = []
         for x in xs:
             native._plans.clear()
             ref.append(m(x))
-        for _ in range(2):
+        for _ in range(3):
             assert all(torch.equal(m(x), r) for x, r in zip(xs, ref))
+            m(other)
+            filled = [torch.full((n,), float("nan"), device="cuda", dtype=torch.float16) for n in (1024, 4608, 9216, 18432, 73728) for _ in range(8)]
+            del filled

@@ -204,13 +204,13 @@ struct PlanBase {
         uint64_t used;
         std::unique_ptr<at::cuda::CUDAGraph> graph;
         std::unique_ptr<at::cuda::CUDAEvent> done;       // behind the last replay: the graph's memory is not given back before
-        Tensor in, out;
+        Tensor in, out, held;                            // held: what the graph reads and the plan may replace
         Captured(const Tensor& x, int64_t work, cudaStream_t st, uint64_t now)
             : B(x.size(0)), H(x.size(2)), W(x.size(3)), work(work), stream(st), seen(0), failed(false), used(now) {}
         Captured(Captured&&) = default;
         Captured& operator=(Captured&& o) { std::swap(B, o.B); std::swap(H, o.H); std::swap(W, o.W); std::swap(work, o.work); std::swap(stream, o.stream);
             std::swap(seen, o.seen); std::swap(failed, o.failed); std::swap(used, o.used); std::swap(graph, o.graph); std::swap(done, o.done);
-            std::swap(in, o.in); std::swap(out, o.out); return *this; }
+            std::swap(in, o.in); std::swap(out, o.out); std::swap(held, o.held); return *this; }
         ~Captured() {
             if (done) { try { done->synchronize(); } catch (...) {} }
         }
@@ -257,8 +257,9 @@ struct PlanBase {
         e.done = std::make_unique<at::cuda::CUDAEvent>();
     }
 
-    // ``first(c, images, y)``: the first kernel, into y (allocated if undefined); ``rest(c, y)``: everything behind it
-    template <typename F, typename R> OptT run(const Tensor& x, int64_t work, F first, R rest) {
+    // ``first(c, images, y)``: the first kernel, into y (allocated if undefined); ``rest(c, y)``: everything behind it; ``held()``:
+    // a tensor made for this shape before both, which the plan keeps for the last shape only
+    template <typename F, typename R, typename G> OptT run(const Tensor& x, int64_t work, F first, R rest, G held) {
         if (!takes(x)) return std::nullopt;
         c10::cuda::CUDAGuard guard(device);
         at::NoGradGuard ng;
@@ -268,6 +269,7 @@ struct PlanBase {
         const bool capturing = cap != cudaStreamCaptureStatusNone;
         StatusPeek& peek = StatusPeek::of(device.index());
         if (const int v = peek.poll(capturing)) { on_status(v); }
+        held();
         const Ctx c{st.stream(), status_ptr(device.index()), type == at::kBFloat16 ? VIG_DTYPE_BF16 : VIG_DTYPE_F16};
         const Chained chained;
         Tensor y;
@@ -275,7 +277,10 @@ struct PlanBase {
             Captured& e = entry(x, st.stream(), work);
             if (e.graph || (!e.failed && e.seen++ > 0)) {
                 first(c, x.contiguous(), e.in);
-                if (!e.graph) capture(e, x, rest, c);
+                if (!e.graph) {
+                    e.held = held();
+                    capture(e, x, rest, c);
+                }
             }
             if (e.graph) {
                 e.graph->replay();
@@ -319,7 +324,14 @@ struct VigPlan : PlanBase {
         const int64_t H = x.dim() == 4 ? x.size(2) : 0, W = x.dim() == 4 ? x.size(3) : 0;
         if (H % 8 || W % 8 || H == 0) return std::nullopt;
         return run(x, x.size(0) * ((H + 15) / 16) * ((W + 15) / 16) * C, [&](const Ctx& c, const Tensor& img, Tensor& f) { first(c, img, f); },
-                   [&, B = x.size(0)](const Ctx& c, const Tensor& f) { return rest(c, f, B, H, W); });
+                   [&, B = x.size(0)](const Ctx& c, const Tensor& f) { return rest(c, f, B, H, W); }, [&] { return position((H / 8 + 1) / 2, (W / 8 + 1) / 2); });
+    }
+    Tensor position(int64_t h, int64_t w) const {
+        if (!pos.defined() || pos_h != h || pos_w != w) {
+            pos = pos_fn(py::make_tuple(h, w)).cast<Tensor>().to(type).contiguous();
+            pos_h = h; pos_w = w;
+        }
+        return pos;
     }
     bool folds(const Ctx& c, int64_t B, int64_t H, int64_t W) const { return w_gemm.defined() && api.vig_stem_conv_ln_supported(B, H / 8, W / 8, 192, C / 2, c.code); }
     void first(const Ctx& c, const Tensor& img, Tensor& f) const {       // 8 x 8 pixel cells, with a border of cells for the 2 x 2 convolution
@@ -339,10 +351,7 @@ struct VigPlan : PlanBase {
         }
         y = conv2.forward(y, false);
         const int64_t h = y.size(1), w = y.size(2), L = h * w, rows = B * L;
-        if (!pos.defined() || pos_h != h || pos_w != w) {
-            pos = pos_fn(py::make_tuple(h, w)).cast<Tensor>().to(type).contiguous();
-            pos_h = h; pos_w = w;
-        }
+        const Tensor pos = position(h, w);
         Tensor tok = at::empty({B, L, C}, f.options());
         if (fused_norms) {
             Tensor n = at::empty({B, L, C}, f.options());
@@ -413,7 +422,7 @@ struct HierPlan : PlanBase {
 
     OptT forward(const Tensor& x) {
         return run(x, x.dim() == 4 ? x.size(0) * ((x.size(2) + 3) / 4) * ((x.size(3) + 3) / 4) * std::get<0>(embed.back()).w.size(0) : 0, [&](const Ctx& c, const Tensor& img, Tensor& y) { first(c, img, y); },
-                   [&](const Ctx& c, const Tensor& y) { return rest(c, y); });
+                   [&](const Ctx& c, const Tensor& y) { return rest(c, y); }, [] { return Tensor(); });
     }
     void first(const Ctx& c, const Tensor& img, Tensor& y) const {
         const int64_t B = img.size(0), H = img.size(2), W = img.size(3);
