@@ -1,0 +1,74 @@
+"""Gates at the far end of what a caller can pass, forward and backward, against the recurrences in fp64: raw 16-bit logits
+whose exponential overflows fp32."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+# relative 2-norm errors: results are rounded to the type once or twice on the way (2^-9, 2^-12)
+TOL = {torch.float32: 1e-5, torch.bfloat16: 1e-2, torch.float16: 2e-3}
+
+
+def _inputs(dtype, B, H, L, dk, dv, seed=0):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    rand = lambda d: torch.randn(B, H, L, d, generator=gen, device="cuda")  # noqa: E731
+    return [t.to(dtype) for t in (rand(dk), rand(dk), rand(dv))], [rand(dk), rand(dk)], rand(dv).to(dtype)
+
+
+def _scan64(q, k, v, g, c, reverse, d_out):
+    """One direction in fp64: (o, dq, dk, dv, d log-gate)."""
+    B, H, L, dk = k.shape
+    order = list(range(L - 1, -1, -1) if reverse else range(L))
+    S = torch.zeros(B, H, dk, v.shape[-1], dtype=torch.float64, device=k.device)
+    Z, a = torch.zeros_like(S), g.exp()
+    o, dq, dkk, dvv = torch.empty_like(v), torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+    for t in order:
+        S = S * a[:, :, t, :, None] + k[:, :, t, :, None] * v[:, :, t, None, :]
+        o[:, :, t] = c * (q[:, :, t, :, None] * S).sum(2)
+        dq[:, :, t] = c * (S * d_out[:, :, t, None, :]).sum(3)
+    for t in reversed(order):
+        D = c * q[:, :, t, :, None] * d_out[:, :, t, None, :] + Z
+        dkk[:, :, t], dvv[:, :, t] = (D * v[:, :, t, None, :]).sum(3), (D * k[:, :, t, :, None]).sum(2)
+        Z = D * a[:, :, t, :, None]
+    e = dq * q - dkk * k
+    return o, dq, dkk, dvv, e.cumsum(2) if reverse else e.flip(2).cumsum(2).flip(2)
+
+
+def _reference(q, k, v, xf, xb, d_out, out_scale, norm):
+    """Both directions: [o, dq, dk, dv, dx_fwd, dx_bwd]; x: raw logits (norm > 0) or log-gates."""
+    q, k, v, d_out = (t.double() for t in (q, k, v, d_out))
+    total, dxs = None, []
+    for reverse, x in ((False, xf.double()), (True, xb.double())):
+        g = torch.nn.functional.logsigmoid(x) / norm if norm else x
+        *parts, dg = _scan64(q, k, v, g, q.shape[-1] ** -0.5 * out_scale, reverse, d_out)
+        dxs.append(dg * torch.sigmoid(-x) / norm if norm else dg)
+        total = parts if total is None else [a + b for a, b in zip(total, parts)]
+    return total + dxs
+
+
+def _run(ins, d_out, **kw):
+    import vig_b200
+    leaves = [t.detach().requires_grad_(True) for t in ins]
+    o = vig_b200.bi_gla(*leaves, out_scale=0.5, **kw)
+    return [o.detach(), *torch.autograd.grad(o, leaves, d_out)]
+
+
+def _errors(got, ref):
+    return [float((a.double() - b).norm() / b.norm()) for a, b in zip(got, ref)]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("dk,dv", [(16, 32), (32, 32), (32, 64), (64, 64)])
+@pytest.mark.parametrize("L", [50, 196, 600, 3000])
+def test_raw_logits_whose_exponential_overflows(dtype, dk, dv, L):
+    """exp(100) and exp(1000) leave fp32, the gates logsigmoid(-100) / 16 and logsigmoid(-1000) / 16 do not; in the first, a
+    middle and the last segment of a sequence of one segment, a cluster of segments, and segments scanned by a launch of
+    their own."""
+    import vig_b200
+    (q, k, v), (xf, xb), d_out = _inputs(dtype, 1, 3, L, dk, dv, seed=L)
+    for i, at in enumerate((3, L // 2, L - 2)):
+        xf[0, 0, at, 1] = xb[0, 0, at, 2] = -100.0
+        xf[0, 1, at, i] = xb[0, 2, at, i] = -1000.0
+    xf, xb = xf.to(dtype), xb.to(dtype)
+    errs = _errors(_run((q, k, v, xf, xb), d_out, gate_logit_normalizer=16.0), _reference(q, k, v, xf, xb, d_out, 0.5, 16.0))
+    assert all(e < TOL[dtype] for e in errs), errs
+    vig_b200.check_status()

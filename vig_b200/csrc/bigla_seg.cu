@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(2 * TOK * SegWarps<T>::CW, seg_min_blocks<DK, 
                 for (int r = 0; r < RPG; ++r)
                     if (r0 + r >= n) { kr[r].zero(); qr[r].zero(); xr[0][r].open_gate(logits); xr[1][r].open_gate(logits); }
             }
-            const F2 zero = f2_make(0.f, 0.f), one = f2_make(1.f, 1.f);
+            const F2 zero = f2_make(0.f, 0.f);
             const F2 nlog2e = f2_make(-tc::LOG2E, -tc::LOG2E);
 #pragma unroll
             for (int dir = 0; dir < 2; ++dir) {
@@ -209,9 +209,7 @@ __global__ void __launch_bounds__(2 * TOK * SegWarps<T>::CW, seg_min_blocks<DK, 
 #pragma unroll
                     for (int rr = 0; rr < RPG; ++rr) {
                         const int r = dir ? RPG - 1 - rr : rr;
-                        const F2 y = f2_mul(xr[dir][r].f2(), nlog2e);
-                        const F2 z = f2_add(f2_make(tc::ex2(f2_lo(y)), tc::ex2(f2_hi(y))), one);
-                        run = f2_fma(f2_make(tc::lg2(f2_lo(z)), tc::lg2(f2_hi(z))), ninv, run);
+                        run = f2_fma(softplus2(f2_mul(xr[dir][r].f2(), nlog2e)), ninv, run);
                         G[dir][r] = run;
                     }
                 } else {

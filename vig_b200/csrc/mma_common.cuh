@@ -95,6 +95,13 @@ template <typename T> __device__ __forceinline__ float gate_log2(float x, float 
     return clamp_min == clamp_min ? fmaxf(g, clamp_min * tc::LOG2E) : g;
 }
 
+// log2(1 + 2^y) of a pair, the models' gate form.  The power overflows from y = 128 on; long before that the result is y itself.
+__device__ __forceinline__ F2 softplus2(F2 y) {
+    const float a = f2_lo(y), b = f2_hi(y);
+    const F2 z = f2_add(f2_make(tc::ex2(a), tc::ex2(b)), f2_make(1.f, 1.f));
+    return f2_make(a > 100.f ? a : tc::lg2(f2_lo(z)), b > 100.f ? b : tc::lg2(f2_hi(z)));
+}
+
 // derivative of the gate transform: d loss / d (gate input x) from d loss / d (log-gate)
 __device__ __forceinline__ float through_gate(float dg, float x, float gate_norm, float clamp_min) {
     if (clamp_min == clamp_min) {                                       // the gradient passes where the unclamped gate is at or above the bound
@@ -185,7 +192,7 @@ template <int DK, typename T> __device__ __forceinline__ void cum_gates(F2 (&G)[
 #pragma unroll
         for (int r = 0; r < CL::RPG; ++r) if (r0 + r >= n) x[r].open_gate(logits);
     }
-    const F2 zero = f2_make(0.f, 0.f), one = f2_make(1.f, 1.f), nlog2e = f2_make(-tc::LOG2E, -tc::LOG2E);
+    const F2 zero = f2_make(0.f, 0.f), nlog2e = f2_make(-tc::LOG2E, -tc::LOG2E);
     const float ni = logits ? -1.f / gate_norm : 0.f;
     const F2 ninv = f2_make(ni, ni);
     F2 run = zero;
@@ -194,8 +201,7 @@ template <int DK, typename T> __device__ __forceinline__ void cum_gates(F2 (&G)[
         const F2 v = x[r].f2();
         F2 g;
         if (sizeof(T) == 2 && logits && !clamp) {                        // the models' form: -log2(1 + 2^(-x log2 e)) / norm
-            const F2 y = f2_mul(v, nlog2e), z = f2_add(f2_make(tc::ex2(f2_lo(y)), tc::ex2(f2_hi(y))), one);
-            g = f2_mul(f2_make(tc::lg2(f2_lo(z)), tc::lg2(f2_hi(z))), ninv);
+            g = f2_mul(softplus2(f2_mul(v, nlog2e)), ninv);
         } else {
             g = r0 + r < n ? f2_make(gate_log2<T>(f2_lo(v), gate_norm, -ni, clamp_min), gate_log2<T>(f2_hi(v), gate_norm, -ni, clamp_min)) : zero;
         }
