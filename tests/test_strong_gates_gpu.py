@@ -1,5 +1,6 @@
 """Gates at the far end of what a caller can pass, forward and backward, against the recurrences in fp64: raw 16-bit logits
-whose exponential overflows fp32."""
+whose exponential overflows fp32, log-gates of -inf, of a type's lowest value, far outside the range that a segment's factored
+form covers, and growing ones."""
 import pytest
 import torch
 
@@ -72,3 +73,52 @@ def test_raw_logits_whose_exponential_overflows(dtype, dk, dv, L):
     errs = _errors(_run((q, k, v, xf, xb), d_out, gate_logit_normalizer=16.0), _reference(q, k, v, xf, xb, d_out, 0.5, 16.0))
     assert all(e < TOL[dtype] for e in errs), errs
     vig_b200.check_status()
+
+
+def _log_gates(kind, x):
+    """Log-gates that a segment's factored form cannot take, made from normal numbers x [B, H, L, dk]."""
+    g = torch.nn.functional.logsigmoid(x) / 16
+    L = g.shape[2]
+    if kind == "reset":                                                  # the state is dropped: exp(-inf) = 0
+        for i, at in enumerate((min(3, L - 1), L // 2, L - 1)):
+            g[0, i % g.shape[1], at, i::5] = -float("inf")
+    elif kind == "lowest":                                               # masks of the lowest finite value, two in a row
+        g[0, 0, L // 3:L // 3 + 2] = torch.finfo(torch.float16).min
+    elif kind == "strong":
+        g = g * 160
+    elif kind == "growing":
+        g[0, 0, :40, ::3] = 0.05                                         # 40 factors of the fast exponential, 2^-22 each: 1e-5
+    return g
+
+
+@pytest.mark.parametrize("kind", ["reset", "lowest", "strong", "growing"])
+@pytest.mark.parametrize("dtype,dk,dv", [(torch.float32, 16, 32), (torch.float32, 32, 32), (torch.float32, 32, 64), (torch.float32, 64, 64), (torch.bfloat16, 16, 32),
+                                         (torch.bfloat16, 64, 64), (torch.float16, 32, 32), (torch.float16, 32, 64)])
+@pytest.mark.parametrize("L", [5, 64, 150, 1000, 2500])
+def test_segments_outside_the_range(dtype, dk, dv, L, kind):
+    """Outputs in both directions and one, final and summed states, one launch (a lone segment, clusters) and three.  A segment
+    is evaluated as the recurrence, so fp32 results carry its roundings only."""
+    import vig_b200
+    (q, k, v), (xf, xb), _ = _inputs(dtype, 1, 3, L, dk, dv, seed=L + dk)
+    gf, gb = _log_gates(kind, xf).to(dtype), _log_gates(kind, xb).to(dtype)
+    q64, k64, v64 = q.double(), k.double(), v.double()
+    c = dk ** -0.5
+    of, S = _forward64(q64, k64, v64, gf.double(), c, False)
+    ob, _ = _forward64(q64, k64, v64, gb.double(), c, True)
+    o, ex = vig_b200.bi_gla(q, k, v, gf, gb, output_final_state=True, output_logdecay=True, impl=vig_b200._lib.IMPL_SEG)
+    one, state = vig_b200.fused_chunk_gla(q, k, v, gf, output_final_state=True) if dtype == torch.float32 or dv == 32 else (None, None)
+    pairs = [(o, of + ob), (ex["final_fwd"], S), (torch.exp(ex["logdecay_fwd"]), torch.exp(gf.double().sum(2)))]
+    if one is not None:
+        pairs += [(one, of), (state, S)]
+    for got, ref in pairs:
+        tol = TOL[dtype] if got.dtype == dtype or dtype == torch.bfloat16 and dv == 64 else 1e-4
+        assert float((got.double() - ref).norm()) <= tol * float(ref.norm()) + 1e-30, (kind, float((got.double() - ref).norm() / ref.norm()))
+
+
+def _forward64(q, k, v, g, c, reverse):
+    B, H, L, dk = k.shape
+    S, o, a = torch.zeros(B, H, dk, v.shape[-1], dtype=torch.float64, device=k.device), torch.empty_like(v), g.exp()
+    for t in range(L - 1, -1, -1) if reverse else range(L):
+        S = S * a[:, :, t, :, None] + k[:, :, t, :, None] * v[:, :, t, None, :]
+        o[:, :, t] = c * (q[:, :, t, :, None] * S).sum(2)
+    return o, S

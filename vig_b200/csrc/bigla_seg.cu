@@ -16,9 +16,10 @@
 // about 22 k cycles alone (loads and gates 6, tiles 3, contribution 4, products 3, states 3, read-out 2): a call of few
 // segments is that latency, one of many is bound by instruction issue at 16 warps an SM.
 // Operands are split into bf16 terms (mma_common.cuh): one term for bf16 with dv = 64 (as in the tcgen05 kernels), two for
-// fp16 and for dv = 32, three for fp32.  A segment whose |G - r| leaves the factorisation's range is evaluated token by token.
+// fp16 and for dv = 32, three for fp32.  A segment whose |G - r| leaves the factorisation's range, contribution included,
+// is evaluated token by token (bigla_exact.cuh).
 #include <atomic>
-#include "mma_common.cuh"
+#include "bigla_exact.cuh"
 
 namespace vig {
 namespace {
@@ -43,7 +44,6 @@ template <int DK, int DV, typename T, int TOK> struct SegSmem {
                               SCL = SUM + 2 * (TOK / 16) * SegWarps<T>::CW * DK * 4,      // per direction and warp: summed log-gates of the warp's rows
                               BYTES = SCL + 4 * DK * 4;                 // [dir][0: 2^r, 1: 2^(l-r)]
     static_assert(TT::SC * DK * Pitch<DV>::B <= QT, "the entering states reuse the K tiles");
-    static_assert(SUM >= TOK * DV * 4, "the exact form keeps its outputs in the tiles");
 };
 
 // x * e of a raw pair and a pair of fp32 factors, in SC bf16 terms (one term: factors rounded to bf16, packed multiply)
@@ -114,39 +114,143 @@ template <int DK, int DV, int MODE> __device__ __forceinline__ float4 entering(c
     return S;
 }
 
-// A segment token by token (any gates); so: [seglen][DV] floats of shared memory.  Thread j < DV owns value column j.
-template <int DK, int DV, typename T, int MODE> __device__ __noinline__ void exact_segment(const SegParams& s, float* so, int bh, int c, int n) {
+// A segment whose gates leave the factorisation's range, or are growing ones, token by token: what it contributes, and its
+// outputs.  Every thread works on it: at 96 sequences of 1000 tokens, fp32 64 / 64, all segments out of range, 14.6 ms with DV
+// threads to a segment, 0.83 with all (1.19 in the gate-independent form of bigla_simt.cu).  The segment's tiles give up their shared memory.
+template <int DK, int DV, typename T, int TOK> struct SegExact {
+    using SM = SegSmem<DK, DV, T, TOK>;
+    using L = rec::Lay<DK, DV, 2 * TOK * SegWarps<T>::CW>;
+    static constexpr uint32_t ROW = 3 * DK + DV;                         // floats staged for a token
+    static constexpr uint32_t bytes(int sub) { return (L::HALVES * sub * ROW + TOK * DV) * 4; }
+    static constexpr int SUB = bytes(32) <= SM::SUM ? 32 : bytes(16) <= SM::SUM ? 16 : 8;      // tokens staged at a time
+    static_assert(bytes(SUB) <= SM::SUM && SUB % rec::GROUP == 0, "the exact form works in the tiles");
+    // Tokens in an even number of blocks: with both directions under way at once, each block is visited by one, then, steps
+    // and barriers later, by the other.
+    static __device__ int blocks(int n) { return 2 * ((n + 2 * SUB - 1) / (2 * SUB)); }
+};
+
+template <int DK, int DV, typename T, int TOK> __device__ __noinline__ void exact_contribution(const SegParams& s, float* sm, int bh, int c, int n) {
+    using E = SegExact<DK, DV, T, TOK>;
+    using L = typename E::L;
     const BiglaParams& p = s.p;
-    const int b = bh / p.H, h = bh % p.H, j = threadIdx.x;
-    const int64_t t0 = (int64_t)c * s.seglen;
-    if (j >= DV) return;
-    for (int i = 0; i < n; ++i) so[i * DV + j] = 0.f;
-    for (int dir = 0; dir < 2; ++dir) {
-        if (!(p.dir_mask & (1 << dir))) continue;
-        float st[DK];
-        for (int d = 0; d < DK; ++d) {
-            const float4 x = entering<DK, DV, MODE>(s, bh, c, dir, (d * DV + j) / 4);
-            st[d] = (j & 3) == 0 ? x.x : (j & 3) == 1 ? x.y : (j & 3) == 2 ? x.z : x.w;
+    const int b = bh / p.H, h = bh % p.H, d0 = L::d0(), j0 = L::j0(), tid = threadIdx.x % L::HT;
+    const int blocks = E::blocks(n), size = (n + blocks - 1) / blocks;
+    float *sa = sm + L::half() * E::SUB * E::ROW, *sg = sa + E::SUB * DK, *sk = sg + E::SUB * DK, *sv = sk + E::SUB * DK;
+    for (int pass = 0; pass < 2 / L::HALVES; ++pass) {
+        const int dir = L::HALVES == 2 ? L::half() : pass;
+        const bool on = p.dir_mask & (1 << dir);
+        float S[L::JPT][L::DPT], sum = 0.f;
+#pragma unroll
+        for (int j = 0; j < L::JPT; ++j)
+#pragma unroll
+            for (int d = 0; d < L::DPT; ++d) S[j][d] = 0.f;
+        for (int bb = 0; bb < blocks; ++bb) {
+            const int at = (dir ? blocks - 1 - bb : bb) * size, m = on ? max(0, min(size, n - at)) : 0;
+            const int64_t t = (int64_t)c * s.seglen + at;
+            __syncthreads();
+            if (m > 0)
+                rec::stage<DK, DV, L::HT, T>(nullptr, sk, sv, sg, sa, nullptr, 0, 0.f, head_ptr<T>(p.k, p.sk, b, h, t), p.sk[2], 1.f, head_ptr<T>(p.v, p.sv, b, h, t), p.sv[2],
+                                             dir ? head_ptr<T>(p.gb, p.sgb, b, h, t) : head_ptr<T>(p.gf, p.sgf, b, h, t), dir ? p.sgb[2] : p.sgf[2], m, p.gate_norm, p.clamp_min, tid);
+            __syncthreads();
+            if (tid < DK) for (int i = 0; i < m; ++i) sum += sg[i * DK + tid];
+            rec::each(m, dir, [&](int i) { rec::update(S, sa + i * DK + d0, sk + i * DK + d0, sv + i * DV + j0); });
         }
-        for (int ii = 0; ii < n; ++ii) {
-            const int i = dir ? n - 1 - ii : ii;
-            const T* g = (dir ? head_ptr<T>(p.gb, p.sgb, b, h, t0 + i) : head_ptr<T>(p.gf, p.sgf, b, h, t0 + i));
-            const T *q = head_ptr<T>(p.q, p.sq, b, h, t0 + i), *k = head_ptr<T>(p.k, p.sk, b, h, t0 + i);
-            const float v = DType<T>::to_f(head_ptr<T>(p.v, p.sv, b, h, t0 + i)[j]);
-            float acc = 0.f;
-            for (int d = 0; d < DK; ++d) {
-                st[d] = fmaf(st[d], __expf(gate_transform(DType<T>::to_f(g[d]), p.gate_norm, p.clamp_min)), DType<T>::to_f(k[d]) * v);
-                acc = fmaf(p.qscale * DType<T>::to_f(q[d]), st[d], acc);
-            }
-            so[i * DV + j] += acc;
+        if (!on) continue;
+        const size_t slot = ((size_t)bh * s.nseg + c) * 2 + dir;
+#pragma unroll
+        for (int j = 0; j < L::JPT; ++j)
+#pragma unroll
+            for (int d = 0; d < L::DPT; ++d) p.ws_state[slot * DK * DV + (d0 + d) * DV + j0 + j] = S[j][d];
+        if (tid < DK) p.ws_decay[slot * DK + tid] = sum;
+    }
+}
+
+// N neighbouring values of a state, read as one vector
+template <int N> __device__ __forceinline__ void load_state_row(float (&x)[N], const float* p) {
+    if constexpr (N == 4) { const float4 v = __ldcg(reinterpret_cast<const float4*>(p)); x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w; }
+    else if constexpr (N == 2) { const float2 v = __ldcg(reinterpret_cast<const float2*>(p)); x[0] = v.x; x[1] = v.y; }
+    else x[0] = __ldcg(p);
+}
+
+// The state entering segment c, my channels and columns of it (as ``entering``, all of a contribution's values in flight together)
+template <int DK, int DV, int MODE, typename L> __device__ __forceinline__ void entering_rows(float (&S)[L::JPT][L::DPT], const SegParams& s, int bh, int c, int dir) {
+    const BiglaParams& p = s.p;
+    const int at = L::d0() * DV + L::j0(), m = MODE == SEG_OUT ? 0 : dir ? s.nseg - 1 - c : c;
+    const float* first = MODE == SEG_OUT ? p.ws_state + (((size_t)bh * s.nseg + c) * 2 + dir) * DK * DV : dir ? p.init_b : p.init_f;
+    if (MODE != SEG_OUT && first) first += (size_t)bh * DK * DV;
+    float u[L::DPT][L::JPT];
+#pragma unroll
+    for (int d = 0; d < L::DPT; ++d) {
+        if (first) load_state_row(u[d], first + at + d * DV);
+#pragma unroll
+        for (int j = 0; j < L::JPT; ++j) S[j][d] = first ? u[d][j] : 0.f;
+    }
+#pragma unroll 2
+    for (int g = 0; g < m; ++g) {
+        const size_t slot = ((size_t)bh * s.nseg + (dir ? s.nseg - 1 - g : g)) * 2 + dir;
+        float a[L::DPT];
+#pragma unroll
+        for (int d = 0; d < L::DPT; ++d) { load_state_row(u[d], p.ws_state + slot * DK * DV + at + d * DV); a[d] = __ldcg(p.ws_decay + slot * DK + L::d0() + d); }
+#pragma unroll
+        for (int d = 0; d < L::DPT; ++d) {
+            const float e = __expf(a[d]);
+#pragma unroll
+            for (int j = 0; j < L::JPT; ++j) S[j][d] = fmaf(S[j][d], e, u[d][j]);
         }
     }
-    for (int i = 0; i < n; ++i)
-        (reinterpret_cast<T*>(p.o) + b * p.so[0] + h * p.so[1] + (t0 + i) * p.so[2])[j] = DType<T>::from_f(so[i * DV + j]);
+}
+
+template <int DK, int DV, typename T, int TOK, int MODE> __device__ __noinline__ void exact_outputs(const SegParams& s, float* sm, int bh, int c, int n) {
+    using E = SegExact<DK, DV, T, TOK>;
+    using L = typename E::L;
+    constexpr int NTH = L::HT * L::HALVES, NV = rec::GROUP * L::JPT;
+    const BiglaParams& p = s.p;
+    const int b = bh / p.H, h = bh % p.H, d0 = L::d0(), j0 = L::j0(), tid = threadIdx.x % L::HT;
+    const int blocks = E::blocks(n), size = (n + blocks - 1) / blocks;
+    float *so = sm, *sa = so + TOK * DV + L::half() * E::SUB * E::ROW, *sq = sa + E::SUB * DK, *sk = sq + E::SUB * DK, *sv = sk + E::SUB * DK;
+    for (int pass = 0; pass < 2 / L::HALVES; ++pass) {
+        const int dir = L::HALVES == 2 ? L::half() : pass;
+        const bool on = p.dir_mask & (1 << dir), both = p.dir_mask == 3;
+        float S[L::JPT][L::DPT];
+        if (on) entering_rows<DK, DV, MODE, L>(S, s, bh, c, dir);
+        for (int bb = 0; bb < blocks; ++bb) {
+            const int at = (dir ? blocks - 1 - bb : bb) * size, m = on ? max(0, min(size, n - at)) : 0;
+            const int64_t t = (int64_t)c * s.seglen + at;
+            const bool add = both && (L::HALVES == 2 ? bb >= blocks / 2 : dir == 1);       // the block's second visit
+            __syncthreads();
+            if (m > 0)
+                rec::stage<DK, DV, L::HT, T>(sq, sk, sv, nullptr, sa, head_ptr<T>(p.q, p.sq, b, h, t), p.sq[2], p.qscale, head_ptr<T>(p.k, p.sk, b, h, t), p.sk[2], 1.f,
+                                             head_ptr<T>(p.v, p.sv, b, h, t), p.sv[2], dir ? head_ptr<T>(p.gb, p.sgb, b, h, t) : head_ptr<T>(p.gf, p.sgf, b, h, t), dir ? p.sgb[2] : p.sgf[2], m, p.gate_norm, p.clamp_min, tid);
+            __syncthreads();
+            const int np = rec::padded(m);
+#pragma unroll 1
+            for (int i0 = 0; i0 < np; i0 += rec::GROUP) {
+                float o[NV];
+#pragma unroll
+                for (int u = 0; u < rec::GROUP; ++u) {
+                    const int i = dir ? np - 1 - i0 - u : i0 + u;
+                    rec::update(S, sa + i * DK + d0, sk + i * DK + d0, sv + i * DV + j0);
+                    rec::read_out(o + u * L::JPT, S, sq + i * DK + d0);
+                }
+                const int first = rec::reduce_scatter<L::DG>(o);
+#pragma unroll
+                for (int e = 0; e < rec::Share<L::DG, NV>::V; ++e) {
+                    const int u = (first + e) / L::JPT, i = dir ? np - 1 - i0 - u : i0 + u;
+                    float* out = so + (at + i) * DV + j0 + (first + e) % L::JPT;
+                    if (first >= 0 && i < m) *out = add ? *out + o[e] : o[e];
+                }
+            }
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n * (DV / 2); i += NTH) {
+        const int r = i / (DV / 2), v = i % (DV / 2) * 2;
+        store2<T>(reinterpret_cast<T*>(p.o) + b * p.so[0] + h * p.so[1] + ((int64_t)c * s.seglen + r) * p.so[2] + v, so[r * DV + v], so[r * DV + v + 1]);
+    }
 }
 
 template <int DK, int DV, typename T, int TOK> constexpr int seg_min_blocks() {
-    constexpr int fit = 225 * 1024 / (int)(SegSmem<DK, DV, T, TOK>::BYTES + 1024), regs = 512 / (2 * TOK * SegWarps<T>::CW);      // 128 registers a thread
+    constexpr int fit = 225 * 1024 / (int)(SegSmem<DK, DV, T, TOK>::BYTES + 1024), regs = (DK == 16 ? 640 : 512) / (2 * TOK * SegWarps<T>::CW);   // 128 registers a thread, 96 at DK = 16
     return fit < 1 ? 1 : fit < regs ? fit : regs;
 }
 
@@ -169,9 +273,9 @@ __global__ void __launch_bounds__(2 * TOK * SegWarps<T>::CW, seg_min_blocks<DK, 
     pdl_launch();                                                        // a chained successor may fetch its weights meanwhile
     const bool want_out = MODE != SEG_STATES && p.o;
     const bool fwd = p.dir_mask & 1, bwd = p.dir_mask & 2;
-    F2 G[2][RPG], ref[2], tot[2];
+    F2 G[2][RPG], ref[2];
     Raw2<T> kr[RPG];
-    bool fine = true;
+    bool fine = true, bad;
     {   // ---- every input of the segment requested at once, gates cumulated, operand tiles written
         seg_load_v<T, DV, RAW, TOK>(smem + SM::V, head_ptr<T>(p.v, p.sv, b, h, t0), p.sv[2], n);
         const bool logits = p.gate_norm > 0.f, clamp = p.clamp_min == p.clamp_min;
@@ -244,6 +348,7 @@ __global__ void __launch_bounds__(2 * TOK * SegWarps<T>::CW, seg_min_blocks<DK, 
         __syncthreads();
         const int wm = nb / 2 * CW;                                           // the reference lies between the rows of warps wm - 1 and wm
         const float lim = range_limit<T>();
+        F2 shift[2];
 #pragma unroll
         for (int dir = 0; dir < 2; ++dir) {
             F2 run = f2_make(0.f, 0.f), before = run, lo = run, mine = run;
@@ -254,7 +359,6 @@ __global__ void __launch_bounds__(2 * TOK * SegWarps<T>::CW, seg_min_blocks<DK, 
                 if (o == wm) lo = run;
                 run = f2_add(run, x);
             }
-            tot[dir] = run;
             const F2 minus = f2_make(-1.f, -1.f);
             const F2 off = dir ? f2_fma(f2_add(before, mine), minus, run) : before;        // what the warps scanned earlier contribute
             ref[dir] = dir ? f2_fma(lo, minus, run) : lo;
@@ -268,14 +372,17 @@ __global__ void __launch_bounds__(2 * TOK * SegWarps<T>::CW, seg_min_blocks<DK, 
                 if (MODE != SEG_OUT && s.need_states && (dir ? bwd : fwd))
                     *reinterpret_cast<float2*>(p.ws_decay + (((size_t)bh * s.nseg + c) * 2 + dir) * DK + 2 * pr) = make_float2(f2_lo(run) * tc::LN2, f2_hi(run) * tc::LN2);
             }
-            if (!(dir ? bwd : fwd) || rb >= nb) continue;
+            shift[dir] = MODE == SEG_STATES ? f2_fma(run, minus, off) : f2_fma(ref[dir], minus, off);        // G - (total or reference)
+        }
+        bad = __syncthreads_or(!fine);
+#pragma unroll
+        for (int dir = 0; dir < 2; ++dir) {
+            if (bad || !(dir ? bwd : fwd) || rb >= nb) continue;
             uint8_t* kt = smem + SM::K + dir * SM::QT + r0 * PK + pr * 4;
             uint8_t* qt = smem + SM::Q + dir * SM::QT + r0 * PK + pr * 4;
-            const F2 shift = MODE == SEG_STATES ? f2_fma(run, minus, off) : f2_fma(ref[dir], minus, off);    // G - (total or reference)
 #pragma unroll
             for (int r = 0; r < RPG; ++r) {
-                const F2 x = f2_add(G[dir][r], shift);
-                if (MODE == SEG_ONE) G[dir][r] = x;
+                const F2 x = f2_add(G[dir][r], shift[dir]);
                 uint32_t t[SC];
                 if (MODE != SEG_STATES) {
                     scaled<T, SC>(qr[r], ex2_t<T>(f2_lo(x)), ex2_t<T>(f2_hi(x)), t);
@@ -289,26 +396,10 @@ __global__ void __launch_bounds__(2 * TOK * SegWarps<T>::CW, seg_min_blocks<DK, 
         }
     }
     if (RAW == 1) asm volatile("cp.async.wait_all;" ::: "memory");
-    const bool bad = __syncthreads_or(!fine && MODE != SEG_STATES);
-    if (bad && MODE == SEG_ONE && s.need_states) {                       // the contribution from tiles whose exponents are all <= 0
-        const F2 minus = f2_make(-1.f, -1.f);
-#pragma unroll
-        for (int dir = 0; dir < 2; ++dir) {
-            if (gr == 0) *reinterpret_cast<float2*>(scl + dir * 2 * DK + DK + 2 * pr) = make_float2(1.f, 1.f);
-            if (rb >= nb) continue;
-            const F2 rest = f2_fma(ref[dir], minus, tot[dir]);           // G holds G - ref
-#pragma unroll
-            for (int r = 0; r < RPG; ++r) {
-                const F2 x = f2_fma(G[dir][r], minus, rest);
-                uint32_t t[SC];
-                scaled<T, SC>(kr[r], ex2_t<T>(f2_lo(x)), ex2_t<T>(f2_hi(x)), t);
-#pragma unroll
-                for (int i = 0; i < SC; ++i) *reinterpret_cast<uint32_t*>(smem + SM::K + dir * SM::QT + i * TK + (r0 + r) * PK + pr * 4) = t[i];
-            }
-        }
-        __syncthreads();
-    }
-    if (MODE != SEG_OUT && s.need_states) {                              // ---- contributions: units of 16 key channels x NC value columns of one direction
+    __syncthreads();
+    if (MODE != SEG_OUT && s.need_states && bad) {
+        exact_contribution<DK, DV, T, TOK>(s, reinterpret_cast<float*>(smem), bh, c, n);
+    } else if (MODE != SEG_OUT && s.need_states) {                       // ---- contributions: units of 16 key channels x NC value columns of one direction
         constexpr int UNITS = 2 * MT, NSPLIT = W <= UNITS ? 1 : W / UNITS < DV / 8 ? W / UNITS : DV / 8, NC = DV / NSPLIT, NTL = NC / 8;
         for (int u = w; u < UNITS * NSPLIT; u += W) {
             const int dir = u / (MT * NSPLIT), mt = (u / NSPLIT) % MT, ns = u % NSPLIT;
@@ -335,9 +426,9 @@ __global__ void __launch_bounds__(2 * TOK * SegWarps<T>::CW, seg_min_blocks<DK, 
                 *reinterpret_cast<float2*>(out + 8 * DV + i * 8) = make_float2(acc[i][2] * s1, acc[i][3] * s1);
             }
         }
-        if (MODE == SEG_STATES) return;
-        if (s.nseg > 1) cluster_arrive();
     }
+    if (MODE == SEG_STATES) return;
+    if (MODE == SEG_ONE && s.nseg > 1) cluster_arrive();
     float o[DC / 8][4];
 #pragma unroll
     for (int i = 0; i < DC / 8; ++i)
@@ -434,7 +525,7 @@ __global__ void __launch_bounds__(2 * TOK * SegWarps<T>::CW, seg_min_blocks<DK, 
     }
     if (!want_out) return;
     if (bad) {
-        exact_segment<DK, DV, T, MODE>(s, reinterpret_cast<float*>(smem), bh, c, n);
+        exact_outputs<DK, DV, T, TOK, MODE>(s, reinterpret_cast<float*>(smem), bh, c, n);
         return;
     }
     if (MODE == SEG_OUT || s.nseg > 1 || has_init) {                     // ---- entering states, scaled, over the K tiles
