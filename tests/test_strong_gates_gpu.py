@@ -122,3 +122,18 @@ def _forward64(q, k, v, g, c, reverse):
         S = S * a[:, :, t, :, None] + k[:, :, t, :, None] * v[:, :, t, None, :]
         o[:, :, t] = c * (q[:, :, t, :, None] * S).sum(2)
     return o, S
+
+
+@pytest.mark.parametrize("kind", ["reset", "lowest", "strong", "growing"])
+@pytest.mark.parametrize("dtype,dk,dv", [(torch.float32, 16, 32), (torch.float32, 32, 64), (torch.float32, 64, 64), (torch.bfloat16, 32, 32), (torch.bfloat16, 64, 64),
+                                         (torch.float16, 16, 32), (torch.float16, 32, 64)])
+@pytest.mark.parametrize("L", [5, 64, 150, 1000])
+def test_gradients_of_chunks_outside_the_range(dtype, dk, dv, L, kind):
+    """One chunk and many: states of the chunk and its adjoint as recurrences, in both directions.  The gate gradients of decayed
+    states are small differences of large sums of fp32 products, hence their wider bound."""
+    (q, k, v), (xf, xb), d_out = _inputs(dtype, 1, 3, L, dk, dv, seed=L + dk)
+    gf, gb = _log_gates(kind, xf).to(dtype), _log_gates(kind, xb).to(dtype)
+    ref = _reference(q, k, v, gf, gb, d_out, 0.5, 0.0)
+    errs = _errors(_run((q, k, v, gf, gb), d_out), ref)
+    assert all(e < TOL[dtype] for e in errs[1:4]), errs
+    assert all(e < max(1e-4, TOL[dtype]) for e in errs[4:]), errs

@@ -13,7 +13,7 @@
 // chunks, chunk gradients.  A chunk whose |G - r| exceeds the range set below raises its flag and is left to the exact
 // token-by-token kernel, which runs afterwards and returns at once for every other chunk.
 #include "bigla_bwd.cuh"
-#include "mma_common.cuh"
+#include "bigla_exact.cuh"
 
 namespace vig {
 namespace {
@@ -27,8 +27,69 @@ template <int DK, int DV, typename T> struct StatesSmem {
                               Q = K + Terms<T>::SC * C * Pitch<DK>::B, SUM = Q + Terms<T>::SC * C * Pitch<DK>::B, BYTES = SUM + 2 * NT * 4;
 };
 
+// Whether a chunk's gates stay in the range of the factorised form, as far as my rows show it.  falling: no log-gate is above
+// zero, so that the ends bound what lies between.
+template <typename T, int RPG> __device__ __forceinline__ bool in_range(const F2 (&G)[RPG], F2 ref, F2 tot, bool falling) {
+    const float lim = range_limit<T>();
+    const F2 minus = f2_make(-1.f, -1.f), rest = f2_fma(ref, minus, tot);
+    bool fine = fabsf(f2_lo(ref)) <= lim && fabsf(f2_hi(ref)) <= lim && fabsf(f2_lo(rest)) <= lim && fabsf(f2_hi(rest)) <= lim;
+    if (!falling) {
+#pragma unroll
+        for (int r = 0; r < RPG; ++r) {
+            const F2 y = f2_fma(ref, minus, G[r]);
+            fine = fine && fabsf(f2_lo(y)) <= lim && fabsf(f2_hi(y)) <= lim;
+        }
+    }
+    return fine;
+}
+
+// States of a chunk outside that range, token by token: half of the threads run S, half its adjoint.  (As 2^(l-G) they are NaN
+// after a log-gate of -inf, and lose digits with large gates: the rounding of G grows with it.)  sm: the K and Q tiles.
+template <int DK, int DV, typename T> struct ExactStates {
+    using L = rec::Lay<DK, DV, NT>;
+    static constexpr int SUB = 16, ROW = 3 * DK + DV;                    // tokens staged at a time, floats of a token
+    static_assert(L::HALVES == 2 && 2 * SUB * ROW * 4 <= 2 * Terms<T>::SC * C * Pitch<DK>::B, "staged rows fit the scaled tiles");
+};
+template <int DK, int DV, typename T> __device__ __noinline__ void exact_states(const BwdParams& p, float* sm, int bh, int c, int dir, int n) {
+    using E = ExactStates<DK, DV, T>;
+    using L = typename E::L;
+    const int b = bh / p.H, h = bh % p.H, d0 = L::d0(), j0 = L::j0(), tid = threadIdx.x % L::HT, blocks = (n + E::SUB - 1) / E::SUB;
+    const bool adj = L::half() == 1, down = (dir != 0) != adj;           // the adjoint runs against the scan order
+    float *sa = sm + L::half() * E::SUB * E::ROW, *sg = sa + E::SUB * DK, *sk = sg + E::SUB * DK, *sv = sk + E::SUB * DK;
+    float S[L::JPT][L::DPT], sum = 0.f;
+#pragma unroll
+    for (int j = 0; j < L::JPT; ++j)
+#pragma unroll
+        for (int d = 0; d < L::DPT; ++d) S[j][d] = 0.f;
+    for (int bb = 0; bb < blocks; ++bb) {
+        const int at = (down ? blocks - 1 - bb : bb) * E::SUB, m = min(E::SUB, n - at);
+        const int64_t t = (int64_t)c * C + at;
+        __syncthreads();
+        rec::stage<DK, DV, L::HT, T>(nullptr, sk, sv, sg, sa, nullptr, 0, 0.f, adj ? head_ptr<T>(p.q, p.sq, b, h, t) : head_ptr<T>(p.k, p.sk, b, h, t), adj ? p.sq[2] : p.sk[2],
+                                     adj ? p.c : 1.f, adj ? head_ptr<T>(p.dout, p.sdo, b, h, t) : head_ptr<T>(p.v, p.sv, b, h, t), adj ? p.sdo[2] : p.sv[2],
+                                     dir ? head_ptr<T>(p.gb, p.sgb, b, h, t) : head_ptr<T>(p.gf, p.sgf, b, h, t), dir ? p.sgb[2] : p.sgf[2], m, p.gate_norm, p.clamp_min, tid);
+        __syncthreads();
+        if (tid < DK) for (int i = 0; i < m; ++i) sum += sg[i * DK + tid];
+        if (adj) rec::each(m, down, [&](int i) { rec::update_adjoint(S, sa + i * DK + d0, sk + i * DK + d0, sv + i * DV + j0); });
+        else rec::each(m, down, [&](int i) { rec::update(S, sa + i * DK + d0, sk + i * DK + d0, sv + i * DV + j0); });
+    }
+    const size_t slot = ((size_t)bh * p.nchunk + c) * 2 + dir;
+    float* out = (adj ? p.ws_Z : p.ws_S) + slot * DK * DV;
+#pragma unroll
+    for (int j = 0; j < L::JPT; ++j)
+#pragma unroll
+        for (int d = 0; d < L::DPT; ++d) out[(d0 + d) * DV + j0 + j] = S[j][d];
+    if (!adj && tid < DK) p.ws_decay[slot * DK + tid] = sum * tc::LOG2E;
+}
+
+// CTAs an SM as the registers of the factored form allow; the exact one, which nobody waits for, has to live with them
+template <int DK, int DV, typename T> constexpr int states_min_blocks() {
+    return DK * DV == 4096 ? (sizeof(T) == 4 ? 1 : 2) : DK * DV == 2048 ? (sizeof(T) == 4 ? 2 : 3) : DK * DV == 1024 ? (sizeof(T) == 4 ? 3 : 4)
+           : std::is_same<T, __nv_bfloat16>::value ? 5 : 4;
+}
+
 template <int DK, int DV, typename T>
-__global__ void __launch_bounds__(NT) bwd_states_mma_kernel(const __grid_constant__ BwdParams p) {
+__global__ void __launch_bounds__(NT, states_min_blocks<DK, DV, T>()) bwd_states_mma_kernel(const __grid_constant__ BwdParams p) {
     using CL = ColLay<DK>;
     using SM = StatesSmem<DK, DV, T>;
     constexpr int RAW = Terms<T>::RAW, SC = Terms<T>::SC;
@@ -55,6 +116,7 @@ __global__ void __launch_bounds__(NT) bwd_states_mma_kernel(const __grid_constan
     load_raw<T, DV, RAW>(smem + SM::O, head_ptr<T>(p.dout, p.sdo, b, h, t0), p.sdo[2], n);
     zero_rows(k, r0, n); zero_rows(q, r0, n);
     const int last = one_dir ? first : p.dir_mask & 2 ? 1 : 0;
+    int exact = 0;                                                       // directions left to the exact form, after the loop: nothing of it lives across the call
     for (int dir = first; dir <= last; ++dir) {
         const size_t slot = ((size_t)bh * p.nchunk + c) * 2 + dir;
         F2 G[CL::RPG], ref, tot;
@@ -76,7 +138,10 @@ __global__ void __launch_bounds__(NT) bwd_states_mma_kernel(const __grid_constan
             for (int i = 0; i < SC; ++i) *reinterpret_cast<uint32_t*>(smem + SM::Q + i * C * Pitch<DK>::B + (r0 + r) * Pitch<DK>::B + pr * 4) = t[i];
         }
         wait_raw();
-        __syncthreads();
+        if (__syncthreads_or(!in_range<T>(G, ref, tot, sizeof(T) == 2 && p.gate_norm > 0.f))) {
+            exact |= 1 << dir;
+            continue;
+        }
         const int which = warp >> 2, mt = (warp & 3) % MT, wn = (warp & 3) / MT;          // warps 0 - 3: S, 4 - 7: Z
         float acc[NTL][4];
 #pragma unroll
@@ -91,6 +156,11 @@ __global__ void __launch_bounds__(NT) bwd_states_mma_kernel(const __grid_constan
             *reinterpret_cast<float2*>(out + 8 * DV + i * 8) = make_float2(acc[i][2], acc[i][3]);
         }
         __syncthreads();
+    }
+    if (exact) {
+#pragma unroll 1
+        for (int dir = first; dir <= last; ++dir)
+            if (exact >> dir & 1) exact_states<DK, DV, T>(p, reinterpret_cast<float*>(smem + SM::K), bh, c, dir, n);
     }
 }
 

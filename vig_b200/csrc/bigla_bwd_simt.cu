@@ -14,6 +14,7 @@
 // chunks in each direction, then one CTA per chunk that replays both recurrences from its entering states.
 // Exact for any gates.  It is the whole backward where the tensor-core form (bigla_bwd_mma.cu) does not take the call, the
 // per-chunk fallback of that form, and it writes either e per direction or the finished gate gradients.
+#include <atomic>
 #include <cmath>
 #include "bigla_bwd.cuh"
 #include "mma_common.cuh"
@@ -283,9 +284,20 @@ int launch_typed(const BwdParams& p, int flagged_only, cudaStream_t stream) {
         if (int st = bigla_bwd_scan_launch(p, stream)) return st;
     }
     const int items = p.nchunk * p.B * p.H;
-    // flagged chunks are rare: a CTA per SM (the tiles fill its shared memory) walks the flags; as one CTA per chunk the
-    // launch alone took 15 us for 3072 unflagged chunks
-    return (int)launch_next(kC, dim3(flagged_only ? (items < 148 ? items : 148) : items), dim3(NT), smC, stream, p, flagged_only);
+    // flagged chunks are rare: as many CTAs as the GPU holds walk the flags (one an SM at 64 / 64, four at 16 / 32); as one
+    // CTA per chunk the launch alone took 15 us for 3072 unflagged chunks
+    int ctas = items;
+    if (flagged_only) {
+        static std::atomic<int> per_sm{0};                               // a property of the kernel, the same on every B200
+        int fit = per_sm.load(), dev = 0, sms = 0;
+        if (!fit) {
+            if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kC, NT, smC)) != cudaSuccess) return (int)e;
+            per_sm.store(fit = fit < 1 ? 1 : fit);
+        }
+        if ((e = cudaGetDevice(&dev)) != cudaSuccess || (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return (int)e;
+        ctas = items < fit * sms ? items : fit * sms;
+    }
+    return (int)launch_next(kC, dim3(ctas), dim3(NT), smC, stream, p, flagged_only);
 }
 
 template <typename T>
