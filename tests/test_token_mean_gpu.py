@@ -14,3 +14,16 @@ def test_token_mean(dtype, B, L, C):
     # fp32 sums in blocks of a few dozen, one rounding to the type
     tol = {torch.float32: 1e-6, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]
     assert float((got.double() - ref).abs().max()) <= tol * float(ref.abs().max())
+
+
+def test_many_small_images_at_once():
+    """Thousands of clusters at a time, of one CTA to eight: the first CTA of each runs before the others write its memory (a
+    cluster barrier on entry; a missing one would show as lost parts of the sums)."""
+    from vig_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    for B, L in ((4000, 129), (2000, 513), (900, 1025)):
+        x = torch.randn(B, L, 64, generator=gen, device="cuda").bfloat16()
+        ref = x.float().mean(dim=1)
+        for _ in range(3):
+            # one rounding of the mean (bf16: 8 significant bits, 2^-8 at most) and the order of fp32 sums; a lost part: L / S of L
+            assert float((ops.token_mean(x).float() - ref).abs().max()) <= 2 ** -8 * float(ref.abs().max()) + 1e-6

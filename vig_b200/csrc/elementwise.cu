@@ -571,6 +571,7 @@ __global__ void __launch_bounds__(EW_THREADS) token_mean_kernel(const T* __restr
     constexpr int V = DType<T>::VEC, LPT = MEAN_CH / V, ROWS = EW_THREADS / LPT;      // lanes per token, tokens at a time
     __shared__ float part[ROWS][MEAN_CH];
     __shared__ float sums[8][MEAN_CH];
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");          // I run; waited for before the first CTA's memory is written
     const int S = gridDim.x, rank = blockIdx.x, c0 = blockIdx.y * MEAN_CH + (threadIdx.x % LPT) * V, b = blockIdx.z;
     const int per = (L + S - 1) / S, l0 = rank * per, l1 = min(L, l0 + per);
     float acc[V];
@@ -590,6 +591,7 @@ __global__ void __launch_bounds__(EW_THREADS) token_mean_kernel(const T* __restr
 #pragma unroll
     for (int i = 0; i < V; ++i) part[threadIdx.x / LPT][(threadIdx.x % LPT) * V + i] = acc[i];
     __syncthreads();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (threadIdx.x < MEAN_CH) {
         float s = 0.f;
         for (int r = 0; r < ROWS; ++r) s += part[r][threadIdx.x];
