@@ -121,7 +121,8 @@ VIG_API int vig_bigla_fwd(const void* q, const void* k, const void* v, const voi
  * classification/models/vig.py:407-426 without the flipped copies.  fp32 arithmetic for every dtype.
  * q, k, g_*: [B,H,L,dk], v, d_out: [B,H,L,dv] with (b,h,l) element strides (NULL = contiguous); dq, dk, dv
  * (input dtype) and e_fwd, e_bwd (fp32) are contiguous [B,H,L,d].  dk in {16,32,64}, dv in {32,64,128}
- * (dk = 64 with dv = 128 included, dk = 16 only with dv = 32).
+ * (dk = 64 with dv = 128 included, dk = 16 only with dv = 32).  workspace: any 4-byte alignment; on 16 bytes the
+ * scan over chunks takes vector loads.
  */
 VIG_API size_t vig_bigla_bwd_workspace_bytes(int B, int H, int L, int dk, int dv);
 VIG_API int vig_bigla_bwd(const void* q, const void* k, const void* v, const void* g_fwd, const void* g_bwd, const void* d_out,

@@ -111,3 +111,25 @@ def test_clamped_gates_pass_gradient_like_torch_clamp_min():
     err = rel_err(dev[3].grad.float(), xr.grad)
     print(f"gate-logit gradient with clamp, bf16: {err:.2e}")
     assert err < 2e-2
+
+
+@pytest.mark.parametrize("dtype,dir_mask", [(torch.float32, 3), (torch.bfloat16, 2)])
+def test_the_e_form_takes_a_workspace_of_any_alignment(dtype, dir_mask):
+    """vig_bigla_bwd on a workspace 0, 4 and 8 bytes off a 16-byte boundary: the same bits."""
+    from vig_b200 import _lib
+    B, H, L, dk, dv = 1, 2, 200, 32, 64
+    ins = [t.to(dtype).cuda() for t in oracle.make_bigla_inputs(B, H, L, dk, dv, seed=5)]
+    d_out = torch.randn(B, H, L, dv, generator=torch.Generator().manual_seed(6)).to(dtype).cuda()
+    lib, nbytes = _lib.lib(), _lib.lib().vig_bigla_bwd_workspace_bytes(B, H, L, dk, dv)
+    ws, results = torch.empty(nbytes + 16, dtype=torch.uint8, device="cuda"), []
+    for offset in (0, 4, 8):
+        outs = [torch.empty(B, H, L, d, dtype=t, device="cuda") for d, t in ((dk, dtype), (dk, dtype), (dv, dtype), (dk, torch.float32), (dk, torch.float32))]
+        for o in outs:
+            o.zero_()
+        st = lib.vig_bigla_bwd(*map(_lib.ptr, ins), _lib.ptr(d_out), *map(_lib.ptr, outs), B, H, L, dk, dv, _lib.dtype_code(ins[0]), *[None] * 6, -1.0, 0.5, dir_mask,
+                               ws.data_ptr() + offset, nbytes, _lib.stream_ptr())
+        assert st == 0
+        results.append(outs)
+    assert all(torch.equal(a, b) for r in results[1:] for a, b in zip(r, results[0]))
+    assert lib.vig_bigla_bwd(*map(_lib.ptr, ins), _lib.ptr(d_out), *map(_lib.ptr, results[0]), B, H, L, dk, dv, _lib.dtype_code(ins[0]), *[None] * 6, -1.0, 0.5, dir_mask,
+                             ws.data_ptr() + 2, nbytes, _lib.stream_ptr()) == -4

@@ -183,6 +183,26 @@ __global__ void __launch_bounds__(256, 2) bwd_scan_kernel(const __grid_constant_
                 [&](int cc) { return ((size_t)bh * p.nchunk + (descending ? p.nchunk - 1 - cc : cc)) * 2 + dir; }, [](float g) { return exp2f(g); });
 }
 
+// the same on a workspace that is not aligned to 16 bytes (vig_bigla_bwd takes any): value by value
+__global__ void __launch_bounds__(256) bwd_scan_unaligned_kernel(const __grid_constant__ BwdParams p) {
+    pdl_launch();
+    pdl_wait();
+    const int per = p.dk * p.dv, ndir = p.dir_mask == 3 ? 2 : 1;
+    const int64_t it = (int64_t)blockIdx.x * 256 + threadIdx.x, r = it / per;
+    const int e = (int)(it % per), which = (int)(r & 1), dir = p.dir_mask == 3 ? (int)(r / 2 % 2) : p.dir_mask - 1;
+    const int64_t bh = r / 2 / ndir;
+    if (bh >= (int64_t)p.B * p.H) return;
+    const bool descending = (dir != 0) != (which != 0);
+    float S = 0.f;
+    for (int cc = 0; cc < p.nchunk; ++cc) {
+        const size_t slot = ((size_t)bh * p.nchunk + (descending ? p.nchunk - 1 - cc : cc)) * 2 + dir;
+        float* at = (which ? p.ws_Z : p.ws_S) + slot * per + e;
+        const float u = __ldcg(at);
+        __stcg(at, S);
+        S = fmaf(S, exp2f(__ldcg(p.ws_decay + slot * p.dk + e / p.dv)), u);
+    }
+}
+
 // ---- chunk gradients -----------------------------------------------------------------------------------------------
 template <int DK, int DV, typename T> struct GradSmem {
     static constexpr uint32_t EP = DK + 8, VP = DV + 8;                // row pitches of the fp32 tiles (floats)
@@ -454,6 +474,10 @@ int launch_dims(const BwdParams& p, cudaStream_t stream) {
 }  // namespace
 
 int bigla_bwd_scan_launch(const BwdParams& p, cudaStream_t stream) {
+    if (reinterpret_cast<uintptr_t>(p.ws_S) & 15) {
+        const int64_t threads = (int64_t)p.B * p.H * (p.dir_mask == 3 ? 2 : 1) * 2 * (p.dk * p.dv);
+        return (int)launch_next(bwd_scan_unaligned_kernel, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, stream, p);
+    }
     const int64_t threads = (int64_t)p.B * p.H * (p.dir_mask == 3 ? 2 : 1) * 2 * (p.dk * p.dv / 4);
     return (int)launch_next(bwd_scan_kernel, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, stream, p);
 }

@@ -379,6 +379,7 @@ extern "C" int vig_bigla_bwd(const void* q, const void* k, const void* v, const 
     if (s || B == 0 || L == 0) return s;
     if (((dir_mask & 1) && !e_fwd) || ((dir_mask & 2) && !e_bwd)) return VIG_ERR_NULL;
     if (!workspace || workspace_bytes < bwd_ws_bytes(B, H, L, dk, dv)) return VIG_ERR_WORKSPACE;
+    if (reinterpret_cast<uintptr_t>(workspace) & 3) return VIG_ERR_ALIGN;
     p.ef = e_fwd; p.eb = e_bwd;
     return bwd_simt(p, 0, (cudaStream_t)stream);
 }
