@@ -104,3 +104,28 @@ def test_replay_reads_the_images_of_its_call(kind):
             m(other)
             filled = [torch.full((n,), float("nan"), device="cuda", dtype=torch.float16) for n in (1024, 4608, 9216, 18432, 73728) for _ in range(8)]
             del filled
+
+
+def test_shapes_that_push_each_other_out_are_not_captured_for_ever():
+    """Two shapes that do not fit the graphs' budget together, in pairs: after a few exchanges both run without a capture, more
+    and more rarely interrupted by one; shapes seen once take no room; results stay what launches one by one give."""
+    from vig_b200 import native
+    m = _model("vig_t", torch.bfloat16)
+    small, big = [torch.randn(b, 3, 512, 1024, device="cuda").bfloat16() for b in (60, 120)]       # 23.6 M and 47.2 M of 64 M elements
+    once = [torch.randn(1, 3, 64, 64 + 16 * i, device="cuda").bfloat16() for i in range(12)]
+    held = []
+    with torch.no_grad():
+        m.replay_graphs = False
+        ref = {t: m(t) for t in (small, big)}
+        assert native._plans[m].graphs() == 0
+        m.replay_graphs = True
+        for _ in range(2):
+            assert torch.equal(m(small), ref[small])
+        for t in once:                                                   # seen once: the graph stays
+            m(t)
+        assert native._plans[m].graphs() == 1
+        for t in (big, big, small, small) * 8:
+            before = native._plans[m].captures()
+            assert torch.equal(m(t), ref[t])
+            held.append(native._plans[m].captures() - before)
+        assert sum(held[:16]) >= 1 and sum(held) <= 8, held

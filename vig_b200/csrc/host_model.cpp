@@ -8,6 +8,7 @@
 // modules themselves.  The check is some hundred pointer comparisons.
 #include "host.h"
 #include <cuda_runtime_api.h>
+#include <limits>
 #include <unordered_map>
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAEvent.h>
@@ -190,71 +191,93 @@ struct PlanBase {
     // One forward.  ``work``: a measure of the activations (tokens x channels).  Launched one by one, a forward of 50 to 150
     // kernels spends 5 - 10 us a launch on the host (through the GEMM library), which small forwards wait for, and 1.4 us
     // between kernels on the device, 7 % of one of three milliseconds (128 images of 224 x 224, width 384: 3465 -> 3220 us; 64
-    // through the hierarchical model 3380 -> 3100; 64 of 1024 x 1024, width 192: 11.6 -> 11.45 ms).  So from the second call of a
-    // shape on a stream it is captured into a CUDA graph and replayed.  The first kernel, which reads the images, stays outside
-    // and writes the graph's input, so that nothing is copied.  The graph and its memory (about 45 bytes per activation element,
-    // GRAPH_WORK elements in all per plan: 3 GB) belong to this plan, one per shape and stream, the least recently used given
-    // back first, and go with it.  Larger forwards gain little (8 of 2048 x 2048: 0.4 %) and would hold more.
+    // through the hierarchical model 3380 -> 3100; 64 of 1024 x 1024, width 192: 11.6 -> 11.45 ms).  So a shape that comes a
+    // second time on a stream is captured into a CUDA graph, behind that call's own launches and while they run (2 - 4 ms of
+    // host time), and replayed from the third call on.  The first kernel, which reads the images, stays outside and writes the
+    // graph's input, so that nothing is copied.  The graph and its memory (about 45 bytes per activation element, GRAPH_WORK
+    // elements in all per plan: 3 GB) belong to this plan, one per shape and stream, the least recently used given back first,
+    // and go with it.  Larger forwards gain little (8 of 2048 x 2048: 0.4 %) and would hold more.
     static constexpr int64_t GRAPH_WORK = 64 << 20;
-    struct Captured {
-        int64_t B, H, W, work;
+    static constexpr size_t GRAPHS = 8, SHAPES = 64;
+    struct Shape {
+        int64_t B, H, W;
         cudaStream_t stream;
-        int seen;
-        bool failed;
+        bool operator==(const Shape& o) const { return B == o.B && H == o.H && W == o.W && stream == o.stream; }
+    };
+    // Calls of a shape since its graph was last given back, and how many of them are worth a capture: twice as many every time,
+    // so that shapes which push each other out are not captured for ever.
+    struct Seen { Shape shape; int64_t calls, worth; uint64_t used; };
+    struct Captured {
+        Shape shape;
+        int64_t work;
         uint64_t used;
         std::unique_ptr<at::cuda::CUDAGraph> graph;
         std::unique_ptr<at::cuda::CUDAEvent> done;       // behind the last replay: the graph's memory is not given back before
         Tensor in, out, held;                            // held: what the graph reads and the plan may replace
-        Captured(const Tensor& x, int64_t work, cudaStream_t st, uint64_t now)
-            : B(x.size(0)), H(x.size(2)), W(x.size(3)), work(work), stream(st), seen(0), failed(false), used(now) {}
-        Captured(Captured&&) = default;
-        Captured& operator=(Captured&& o) { std::swap(B, o.B); std::swap(H, o.H); std::swap(W, o.W); std::swap(work, o.work); std::swap(stream, o.stream);
-            std::swap(seen, o.seen); std::swap(failed, o.failed); std::swap(used, o.used); std::swap(graph, o.graph); std::swap(done, o.done);
-            std::swap(in, o.in); std::swap(out, o.out); std::swap(held, o.held); return *this; }
         ~Captured() {
             if (done) { try { done->synchronize(); } catch (...) {} }
         }
     };
-    std::vector<Captured> captured;
+    bool graphs = true;
+    std::vector<Seen> seen;
+    std::vector<std::unique_ptr<Captured>> captured;
     uint64_t clock = 0;
+    int64_t captures = 0;
 
-    Captured& entry(const Tensor& x, cudaStream_t st, int64_t work) {
-        for (Captured& e : captured)
-            if (e.B == x.size(0) && e.H == x.size(2) && e.W == x.size(3) && e.stream == st) { e.used = ++clock; return e; }
-        int64_t held = work;
-        for (const Captured& e : captured) held += e.work;
-        while (!captured.empty() && (held > GRAPH_WORK || captured.size() >= 8)) {
-            size_t oldest = 0;
-            for (size_t i = 1; i < captured.size(); ++i) if (captured[i].used < captured[oldest].used) oldest = i;
-            held -= captured[oldest].work;
-            captured.erase(captured.begin() + oldest);
-        }
-        captured.emplace_back(x, work, st, ++clock);
-        return captured.back();
+    template <typename V> static size_t oldest(const V& v) {
+        auto used = [](const auto& e) { if constexpr (std::is_same_v<std::decay_t<decltype(e)>, Seen>) return e.used; else return e->used; };
+        size_t at = 0;
+        for (size_t i = 1; i < v.size(); ++i) if (used(v[i]) < used(v[at])) at = i;
+        return at;
     }
-    template <typename F> void capture(Captured& e, const Tensor& x, F rest, const Ctx& c) {
+    Captured* find(const Shape& s) {
+        for (auto& e : captured) if (e->shape == s) { e->used = ++clock; return e.get(); }
+        return nullptr;
+    }
+    Seen& record(const Shape& s) {
+        for (Seen& e : seen) if (e.shape == s) { e.used = ++clock; return e; }
+        if (seen.size() >= SHAPES) seen.erase(seen.begin() + oldest(seen));
+        seen.push_back({s, 0, 2, ++clock});
+        return seen.back();
+    }
+    void make_room(int64_t work) {
+        for (;;) {
+            int64_t held = work;
+            for (const auto& e : captured) held += e->work;
+            if (captured.empty() || (held <= GRAPH_WORK && captured.size() < GRAPHS)) return;
+            const size_t i = oldest(captured);
+            Seen& e = record(captured[i]->shape);
+            e.calls = 0;
+            e.worth *= 2;
+            captured.erase(captured.begin() + i);
+        }
+    }
+    // in: what the first kernel of this call wrote; the graph keeps it as its input
+    template <typename F> void capture(const Shape& s, int64_t work, const Tensor& in, Tensor held, F rest, const Ctx& c) {
         // one capture stream per device; a GEMM on it beforehand, so that the library's workspace for it is an ordinary allocation
         static std::unordered_map<int, at::cuda::CUDAStream>* streams = new std::unordered_map<int, at::cuda::CUDAStream>();
         auto it = streams->find(device.index());
         const bool fresh = it == streams->end();
         if (fresh) it = streams->emplace(device.index(), at::cuda::getStreamFromPool(false, device.index())).first;
+        make_room(work);
         c10::cuda::CUDAStreamGuard guard(it->second);
         if (fresh) {
-            const Tensor a = at::zeros({16, 64}, x.options()), b = at::zeros({64}, x.options());
-            at::linear(a, at::zeros({64, 64}, x.options()), b);
-            at::linear(a, at::zeros({64, 64}, x.options()));
+            const Tensor a = at::zeros({16, 64}, in.options()), b = at::zeros({64}, in.options());
+            at::linear(a, at::zeros({64, 64}, in.options()), b);
+            at::linear(a, at::zeros({64, 64}, in.options()));
         }
+        auto e = std::make_unique<Captured>();
+        e->shape = s; e->work = work; e->used = ++clock; e->in = in; e->held = std::move(held);
         auto g = std::make_unique<at::cuda::CUDAGraph>();
+        bool failed = false;
         g->capture_begin({0, 0}, cudaStreamCaptureModeThreadLocal);
-        try {
-            e.out = rest(Ctx{it->second.stream(), c.status, c.code}, e.in);
-        } catch (...) {
-            e.failed = true;
-        }
-        try { g->capture_end(); } catch (...) { e.failed = true; }
-        if (e.failed) { e.in = e.out = Tensor(); return; }
-        e.graph = std::move(g);
-        e.done = std::make_unique<at::cuda::CUDAEvent>();
+        try { e->out = rest(Ctx{it->second.stream(), c.status, c.code}, in); } catch (...) { failed = true; }
+        try { g->capture_end(); } catch (...) { failed = true; }
+        if (failed) { record(s).worth = std::numeric_limits<int64_t>::max() / 2; return; }
+        e->graph = std::move(g);
+        e->done = std::make_unique<at::cuda::CUDAEvent>();
+        captured.push_back(std::move(e));
+        ++captures;
     }
 
     // ``first(c, images, y)``: the first kernel, into y (allocated if undefined); ``rest(c, y)``: everything behind it; ``held()``:
@@ -269,29 +292,26 @@ struct PlanBase {
         const bool capturing = cap != cudaStreamCaptureStatusNone;
         StatusPeek& peek = StatusPeek::of(device.index());
         if (const int v = peek.poll(capturing)) { on_status(v); }
-        held();
+        const Tensor kept = held();
         const Ctx c{st.stream(), status_ptr(device.index()), type == at::kBFloat16 ? VIG_DTYPE_BF16 : VIG_DTYPE_F16};
         const Chained chained;
+        const bool replays = graphs && !capturing && work <= GRAPH_WORK;
+        const Shape shape{x.size(0), x.size(2), x.size(3), st.stream()};
+        Captured* e = replays ? find(shape) : nullptr;
         Tensor y;
-        if (!capturing && work <= GRAPH_WORK) {
-            Captured& e = entry(x, st.stream(), work);
-            if (e.graph || (!e.failed && e.seen++ > 0)) {
-                first(c, x.contiguous(), e.in);
-                if (!e.graph) {
-                    e.held = held();
-                    capture(e, x, rest, c);
-                }
-            }
-            if (e.graph) {
-                e.graph->replay();
-                y = e.out.clone();
-                e.done->record(st);
-            }
-        }
-        if (!y.defined()) {
+        if (e) {
+            first(c, x.contiguous(), e->in);
+            e->graph->replay();
+            y = e->out.clone();
+            e->done->record(st);
+        } else {
             Tensor t;
             first(c, x.contiguous(), t);
             y = rest(c, t);
+            if (replays) {
+                Seen& r = record(shape);
+                if (++r.calls >= r.worth) capture(shape, work, t, kept, rest, c);
+            }
         }
         peek.snapshot(device.index(), st.stream(), capturing);
         return y;
@@ -485,6 +505,7 @@ void base_of(PlanBase& p, const py::dict& d) {
     p.head_w = tensor_of(d, "head_w"); p.head_b = tensor_of(d, "head_b");
     p.type = p.head_w.scalar_type(); p.device = p.head_w.device();
     p.on_status = d["on_status"];
+    p.graphs = d["graphs"].cast<bool>();
 }
 
 VigPlan* make_vig(const py::dict& d) {
@@ -538,6 +559,8 @@ void bind_model(py::module_& m) {
         cls.def("watch_item", [](P& p, py::object d, py::object k, py::object v) { p.watch.item(d, k, v); })
             .def("watch_size", [](P& p, py::object d) { p.watch.size(d); })
             .def("watch_modules", [](P& p, const py::list& ms) { for (auto m : ms) p.watch.module(m); })
+            .def("graphs", [](const P& p) { return p.captured.size(); })
+            .def("captures", [](const P& p) { return p.captures; })
             .def("valid", [](const P& p) { return p.watch.same(); })
             .def("forward", &P::forward);
     };

@@ -109,6 +109,7 @@ class HierViG(nn.Module):
                  mlp_ratio=4.0, mlp_act_layer="gelu", gmlp=False, patch_norm=True, norm_layer="LN", downsample_version="v2",
                  patchembed_version="v1", rms_norm_eps=1e-6, **unused):
         super().__init__()
+        self.replay_graphs = True            # eval forwards of a repeated shape become a CUDA graph, up to 3 GB a model; False: never
         if rope_mode != "none":
             raise NotImplementedError("rotary variants are not part of the shipped configurations")
         if norm_layer.lower() not in ("ln", "ln2d"):

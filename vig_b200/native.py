@@ -66,7 +66,7 @@ def _vig(model):
     one_kernel = pe.fuse_conv1 and conv1.weight.shape[0] == 96
     ref = weakref.ref(model)
     return _lib.host().VigPlan(dict(
-        head_w=model.head.weight, head_b=model.head.bias, on_status=_status_seen(model.head.weight.device), blocks=blocks, fused_norms=fused,
+        head_w=model.head.weight, head_b=model.head.bias, on_status=_status_seen(model.head.weight.device), graphs=getattr(model, "replay_graphs", True), blocks=blocks, fused_norms=fused,
         w_gemm=pe._gemm_weight() if one_kernel else None, b1=conv1.bias, ln1=_norm(pe.proj[1]), ln2=_norm(pe.proj[4]),
         cells=_conv(conv1, weight=pe._block_weight(), stride=1, pad=0), conv2=_conv(pe.proj[3]), norm_w=model.norm.weight, norm_e=model.norm.eps,
         pos_fn=lambda hw: ref()._pos(hw)))
@@ -99,7 +99,7 @@ def _hier(model):
         has = not isinstance(down, nn.Identity)
         stages.append(dict(blocks=blocks, conv=_conv(down[1]) if has else None, norm=_norm(down[3]) if has else None))
     head = model.classifier.head
-    return _lib.host().HierPlan(dict(head_w=head.weight, head_b=head.bias, on_status=_status_seen(head.weight.device), embed=embed, stages=stages,
+    return _lib.host().HierPlan(dict(head_w=head.weight, head_b=head.bias, on_status=_status_seen(head.weight.device), graphs=getattr(model, "replay_graphs", True), embed=embed, stages=stages,
                                      first_w=c.weight.detach().contiguous() if own else None,
                                      last=_norm(model.classifier.norm)))
 

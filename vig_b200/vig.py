@@ -144,6 +144,7 @@ class ViG(nn.Module):
                  use_bias_in_dwconv=False, clamp_min=None, rms_norm_eps=1e-6, **unused):
         super().__init__()
         self.fuse_norm_epilogues = True
+        self.replay_graphs = True            # eval forwards of a repeated shape become a CUDA graph, up to 3 GB a model; False: never
         self.embed_dim, self.num_classes = embed_dim, num_classes
         self.config = SimpleNamespace(hidden_size=embed_dim, num_hidden_layers=depth, num_attention_heads=num_heads,
                                       expand_k=expand_k, expand_v=expand_v, rms_norm_eps=rms_norm_eps, use_out_act=use_out_act,
