@@ -129,3 +129,34 @@ def test_shapes_that_push_each_other_out_are_not_captured_for_ever():
             assert torch.equal(m(t), ref[t])
             held.append(native._plans[m].captures() - before)
         assert sum(held[:16]) >= 1 and sum(held) <= 8, held
+
+
+def test_graphs_own_the_scratch_their_gemms_write():
+    """Replays of two models on two streams at the same time, without waits between them, give what they give alone; and giving
+    back torch's GEMM workspaces takes nothing from a graph (tensors that then get that memory stay as they were)."""
+    from vig_b200 import native
+    models = [_model("vig_s", torch.bfloat16), _model("vig_s", torch.bfloat16)]
+    xs = [torch.randn(2, 3, 224, 224, device="cuda").bfloat16() for _ in models]
+    streams = [torch.cuda.Stream() for _ in models]
+    with torch.no_grad():
+        ref = [m(x) for m, x in zip(models, xs)]
+        torch.cuda.synchronize()
+        for m, x, s in zip(models, xs, streams):
+            with torch.cuda.stream(s):
+                for _ in range(3):
+                    m(x)
+            torch.cuda.synchronize()
+        assert all(native._plans[m].graphs() == 1 for m in models)
+        outs = []
+        for _ in range(50):
+            for m, x, s in zip(models, xs, streams):
+                with torch.cuda.stream(s):
+                    outs.append(m(x))
+        torch.cuda.synchronize()
+        assert all(torch.equal(o, ref[i % 2]) for i, o in enumerate(outs))
+        torch._C._cuda_clearCublasWorkspaces()
+        bystanders = [torch.full((1 << 20,), float(i), device="cuda") for i in range(64)]
+        with torch.cuda.stream(streams[0]):
+            again = models[0](xs[0])
+        torch.cuda.synchronize()
+        assert torch.equal(again, ref[0]) and all(bool((b == i).all()) for i, b in enumerate(bystanders))

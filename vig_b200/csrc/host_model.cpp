@@ -9,10 +9,12 @@
 #include "host.h"
 #include <cuda_runtime_api.h>
 #include <limits>
+#include <shared_mutex>
 #include <unordered_map>
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAEvent.h>
 #include <ATen/cuda/CUDAGraph.h>
+#include <c10/cuda/CUDAException.h>
 #include <ATen/ops/empty.h>
 
 namespace vig_host {
@@ -195,7 +197,7 @@ struct PlanBase {
     // second time on a stream is captured into a CUDA graph, behind that call's own launches and while they run (2 - 4 ms of
     // host time), and replayed from the third call on.  The first kernel, which reads the images, stays outside and writes the
     // graph's input, so that nothing is copied.  The graph and its memory (about 45 bytes per activation element, GRAPH_WORK
-    // elements in all per plan: 3 GB) belong to this plan, one per shape and stream, the least recently used given back first,
+    // elements in all per plan: 3 GB, and 32 MB of GEMM workspace) belong to this plan, one per shape and stream, the least recently used given back first,
     // and go with it.  Larger forwards gain little (8 of 2048 x 2048: 0.4 %) and would hold more.
     static constexpr int64_t GRAPH_WORK = 64 << 20;
     static constexpr size_t GRAPHS = 8, SHAPES = 64;
@@ -214,6 +216,7 @@ struct PlanBase {
         std::unique_ptr<at::cuda::CUDAGraph> graph;
         std::unique_ptr<at::cuda::CUDAEvent> done;       // behind the last replay: the graph's memory is not given back before
         Tensor in, out, held;                            // held: what the graph reads and the plan may replace
+        std::vector<c10::DataPtr> scratch;               // the GEMM library's workspaces that its kernels write
         ~Captured() {
             if (done) { try { done->synchronize(); } catch (...) {} }
         }
@@ -252,27 +255,45 @@ struct PlanBase {
             captured.erase(captured.begin() + i);
         }
     }
+    // A stream of its own to capture on: no one else's work is ever on it
+    at::cuda::CUDAStream capture_stream() const {
+        static std::unordered_map<int, cudaStream_t>* streams = new std::unordered_map<int, cudaStream_t>();
+        auto it = streams->find(device.index());
+        if (it == streams->end()) {
+            cudaStream_t st = nullptr;
+            C10_CUDA_CHECK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+            it = streams->emplace(device.index(), st).first;
+        }
+        return at::cuda::getStreamFromExternal(it->second, device.index());
+    }
+    // The GEMM library's workspaces for ``st``, out of torch's tables.  They are made on the first GEMM on a stream, so those of
+    // a capture come from the graph's own memory pool, and taken out here they are the graph's alone: graphs that run side by
+    // side on two streams share no scratch, and nobody else gives it back.
+    static void take_scratch(cudaStream_t st, std::vector<c10::DataPtr>& into) {
+        for (auto* table : {&at::cuda::cublas_handle_stream_to_workspace(), &at::cuda::cublaslt_handle_stream_to_workspace()}) {
+            std::unique_lock<std::shared_mutex> lock(table->mutex);
+            for (auto it = table->map.begin(); it != table->map.end();) {
+                if (std::get<1>(it->first) != static_cast<void*>(st)) { ++it; continue; }
+                into.push_back(std::move(it->second));
+                it = table->map.erase(it);
+            }
+        }
+    }
     // in: what the first kernel of this call wrote; the graph keeps it as its input
     template <typename F> void capture(const Shape& s, int64_t work, const Tensor& in, Tensor held, F rest, const Ctx& c) {
-        // one capture stream per device; a GEMM on it beforehand, so that the library's workspace for it is an ordinary allocation
-        static std::unordered_map<int, at::cuda::CUDAStream>* streams = new std::unordered_map<int, at::cuda::CUDAStream>();
-        auto it = streams->find(device.index());
-        const bool fresh = it == streams->end();
-        if (fresh) it = streams->emplace(device.index(), at::cuda::getStreamFromPool(false, device.index())).first;
         make_room(work);
-        c10::cuda::CUDAStreamGuard guard(it->second);
-        if (fresh) {
-            const Tensor a = at::zeros({16, 64}, in.options()), b = at::zeros({64}, in.options());
-            at::linear(a, at::zeros({64, 64}, in.options()), b);
-            at::linear(a, at::zeros({64, 64}, in.options()));
-        }
+        const at::cuda::CUDAStream on = capture_stream();
+        std::vector<c10::DataPtr> stale;
+        take_scratch(on.stream(), stale);                    // of a capture that failed half way
+        c10::cuda::CUDAStreamGuard guard(on);
         auto e = std::make_unique<Captured>();
         e->shape = s; e->work = work; e->used = ++clock; e->in = in; e->held = std::move(held);
         auto g = std::make_unique<at::cuda::CUDAGraph>();
         bool failed = false;
         g->capture_begin({0, 0}, cudaStreamCaptureModeThreadLocal);
-        try { e->out = rest(Ctx{it->second.stream(), c.status, c.code}, in); } catch (...) { failed = true; }
+        try { e->out = rest(Ctx{on.stream(), c.status, c.code}, in); } catch (...) { failed = true; }
         try { g->capture_end(); } catch (...) { failed = true; }
+        take_scratch(on.stream(), e->scratch);
         if (failed) { record(s).worth = std::numeric_limits<int64_t>::max() / 2; return; }
         e->graph = std::move(g);
         e->done = std::make_unique<at::cuda::CUDAEvent>();
