@@ -33,6 +33,7 @@ def test_native_forward_equals_the_modules(kind, size, dtype):
         assert run(m, x) is None
         ref = m(x)
         handle.remove()
+        assert run(m, x) is not None                                    # and no longer
     rel = float((got.float() - ref.float()).norm() / ref.float().norm())
     # hier: the branch's add is fused into the next norm; vig_t: the row-local half of a block is one kernel whose sums run in
     # another order, which flips roundings (2^-9) of stored activations
@@ -160,3 +161,23 @@ def test_graphs_own_the_scratch_their_gemms_write():
             again = models[0](xs[0])
         torch.cuda.synchronize()
         assert torch.equal(again, ref[0]) and all(bool((b == i).all()) for i, b in enumerate(bystanders))
+
+
+def test_a_refusal_lasts_as_long_as_its_reason():
+    """A call in training mode, a hook on a submodule, an overridden forward: the modules run while it lasts, the plan after it."""
+    from vig_b200 import native
+    x = torch.randn(1, 3, 64, 64, device="cuda").bfloat16()
+    with torch.no_grad():
+        m = _model("vig_t", torch.bfloat16).train()
+        assert native.vig_forward(m, x) is None and native.vig_forward(m, x) is None
+        m.eval()
+        ref = native.vig_forward(m, x)
+        assert ref is not None
+        handle = m.blocks[1].mlp.register_forward_pre_hook(lambda *a: None)
+        assert native.vig_forward(m, x) is None and native.vig_forward(m, x) is None
+        handle.remove()
+        assert torch.equal(native.vig_forward(m, x), ref)
+        m.blocks[0].forward = m.blocks[0].forward
+        assert native.vig_forward(m, x) is None and native.vig_forward(m, x) is None
+        del m.blocks[0].forward
+        assert torch.equal(native.vig_forward(m, x), ref)

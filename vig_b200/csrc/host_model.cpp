@@ -115,9 +115,9 @@ struct Watch {
     void item(py::object d, py::object k, py::object v) { items.push_back({d, k, v}); }
     void size(py::object d) { sizes.emplace_back(d, PyDict_Size(d.ptr())); }
     void missing(py::object d, py::object k) { absent.emplace_back(d, k); }
-    void param(const Tensor& t) { params.push_back({t, (int64_t)t._version(), t.data_ptr(), t.scalar_type()}); }
-    // a module's plain attributes, parameters, children, hooks and the absence of an overridden forward
-    void module(py::handle m) {
+    void param(const Tensor& t, bool values) { params.push_back({t, values ? (int64_t)t._version() : -1, values ? t.data_ptr() : nullptr, t.scalar_type()}); }
+    // a module's plain attributes, parameters (values: what is in them too), children, hooks and the forward it overrides or not
+    void module(py::handle m, bool values) {
         const py::dict d = m.attr("__dict__");
         const py::str fwd("forward");
         for (auto kv : d) {
@@ -130,18 +130,20 @@ struct Watch {
             const py::dict t = d[table];
             for (auto kv : t) {
                 item(t, py::reinterpret_borrow<py::object>(kv.first), py::reinterpret_borrow<py::object>(kv.second));
-                if (table[1] == 'p' && !kv.second.is_none()) param(kv.second.cast<Tensor>());
+                if (table[1] == 'p' && !kv.second.is_none()) param(kv.second.cast<Tensor>(), values);
             }
             size(t);
         }
         for (const char* h : {"_forward_hooks", "_forward_pre_hooks"}) size(d[h]);
-        missing(d, fwd);
+        if (PyObject* own = PyDict_GetItem(d.ptr(), fwd.ptr())) item(d, fwd, py::reinterpret_borrow<py::object>(own));
+        else missing(d, fwd);
     }
     bool same() const {
         for (const auto& i : items) if (PyDict_GetItem(i.dict.ptr(), i.key.ptr()) != i.value.ptr()) return false;
         for (const auto& s : sizes) if (PyDict_Size(s.first.ptr()) != s.second) return false;
         for (const auto& a : absent) if (PyDict_GetItem(a.first.ptr(), a.second.ptr())) return false;
-        for (const auto& p : params) if ((int64_t)p.t._version() != p.version || p.t.data_ptr() != p.data || p.t.scalar_type() != p.type) return false;
+        for (const auto& p : params)
+            if (p.t.scalar_type() != p.type || (p.version >= 0 && ((int64_t)p.t._version() != p.version || p.t.data_ptr() != p.data))) return false;
         return true;
     }
 };
@@ -579,12 +581,20 @@ void bind_model(py::module_& m) {
         using P = typename std::decay_t<decltype(cls)>::type;
         cls.def("watch_item", [](P& p, py::object d, py::object k, py::object v) { p.watch.item(d, k, v); })
             .def("watch_size", [](P& p, py::object d) { p.watch.size(d); })
-            .def("watch_modules", [](P& p, const py::list& ms) { for (auto m : ms) p.watch.module(m); })
+            .def("watch_modules", [](P& p, const py::list& ms) { for (auto m : ms) p.watch.module(m, true); })
             .def("graphs", [](const P& p) { return p.captured.size(); })
             .def("captures", [](const P& p) { return p.captures; })
             .def("valid", [](const P& p) { return p.watch.same(); })
             .def("forward", &P::forward);
     };
+    // what a model without a plan was refused for
+    py::class_<Watch>(m, "Refusal")
+        .def(py::init<>())
+        .def("watch_item", [](Watch& w, py::object d, py::object k, py::object v) { w.item(d, k, v); })
+        .def("watch_size", [](Watch& w, py::object d) { w.size(d); })
+        .def("watch_modules", [](Watch& w, const py::list& ms) { for (auto m : ms) w.module(m, false); })
+        .def("valid", &Watch::same)
+        .def("forward", [](const Watch&, py::object) { return py::none(); });
     py::class_<VigPlan> vig(m, "VigPlan");
     vig.def(py::init(&make_vig));
     watch(vig);

@@ -11,7 +11,7 @@ import torch.nn as nn
 
 from . import _lib, hier, modules, ops, vig
 
-_plans = weakref.WeakKeyDictionary()          # model -> plan, or False where the model has none
+_plans = weakref.WeakKeyDictionary()          # model -> plan, or refusal: why the model has none, for as long as that stands
 _OPS = {n: getattr(ops, n) for n in ("bi_gla", "dwconv3x3", "gate_inject", "add_rmsnorm", "layernorm_act", "add_layernorm", "linear_swiglu",
                                      "linear_add_rmsnorm", "linear_bias", "swiglu", "token_mean", "stem_fold", "stem_unfold", "stem_conv_ln")}
 _CLASSES = (vig.ViG, vig.V2PatchEmbed, vig.LayerNorm2d, modules.GLABlock, modules.GatedLinearAttention, modules.GLAMLP, modules.RMSNorm,
@@ -106,15 +106,14 @@ def _hier(model):
 
 def _build(model, make):
     mods = list(model.modules())
-    if model.training or any(type(m) not in _CLASSES or "forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks for m in mods):
-        return False
-    params = [p for m in mods for p in m._parameters.values() if p is not None]
-    if any(p.dtype != params[0].dtype or p.device != params[0].device for p in params):
-        return False
-    with torch.no_grad():
-        plan = make(model)
+    plan = None
+    if not (model.training or any(type(m) not in _CLASSES or "forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks for m in mods)):
+        params = [p for m in mods for p in m._parameters.values() if p is not None]
+        if all(p.dtype == params[0].dtype and p.device == params[0].device for p in params):
+            with torch.no_grad():
+                plan = make(model)
     if plan is None:
-        return False
+        plan = _lib.host().Refusal()
     _watch(plan, mods)
     return plan
 
@@ -123,19 +122,14 @@ def _forward(model, images, head, make):
     if torch.is_grad_enabled() or head.dtype not in (torch.bfloat16, torch.float16) or type(images) is not torch.Tensor or not images.is_cuda:
         return None
     plan = _plans.get(model)
-    if plan:
+    if plan is not None:
         y = plan.forward(images)
         if y is not None or plan.valid():
             return y
-    elif plan is False and model.__dict__.get("_plan_refused") is head.dtype:
-        return None
     if any(ops.__dict__[n] is not fn for n, fn in _OPS.items()) or head.device != images.device:
         return None
     ops.status_word(images.device)
     plan = _plans[model] = _build(model, make)
-    if not plan:
-        model._plan_refused = head.dtype              # not asked again for this precision: the modules run instead
-        return None
     return plan.forward(images)
 
 
