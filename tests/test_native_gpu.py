@@ -2,6 +2,7 @@
 staleness: changed parameters and attributes are seen, hooks and overridden forwards send the call to the modules."""
 import pytest
 import torch
+import torch.nn as nn
 
 pytestmark = pytest.mark.gpu
 
@@ -181,3 +182,25 @@ def test_a_refusal_lasts_as_long_as_its_reason():
         assert native.vig_forward(m, x) is None and native.vig_forward(m, x) is None
         del m.blocks[0].forward
         assert torch.equal(native.vig_forward(m, x), ref)
+
+
+def test_global_hooks_see_every_module():
+    """Hooks registered for all modules: before the first forward, between forwards, one in another's place."""
+    x = torch.randn(1, 3, 64, 64, device="cuda").bfloat16()
+    names = []
+    see = lambda mod, args, out=None: names.append(type(mod).__name__)  # noqa: E731
+    with torch.no_grad():
+        m = _model("vig_t", torch.bfloat16)
+        for register in (nn.modules.module.register_module_forward_hook, nn.modules.module.register_module_forward_pre_hook):
+            for warm in (False, True):
+                if warm:
+                    m(x), m(x), m(x)
+                for _ in range(2):
+                    handle = register(see)
+                    names.clear()
+                    m(x)
+                    handle.remove()
+                    assert names.count("GLABlock") == 2, names
+                names.clear()
+                m(x)
+                assert not names

@@ -14,6 +14,7 @@ from . import _lib, hier, modules, ops, vig
 _plans = weakref.WeakKeyDictionary()          # model -> plan, or refusal: why the model has none, for as long as that stands
 _OPS = {n: getattr(ops, n) for n in ("bi_gla", "dwconv3x3", "gate_inject", "add_rmsnorm", "layernorm_act", "add_layernorm", "linear_swiglu",
                                      "linear_add_rmsnorm", "linear_bias", "swiglu", "token_mean", "stem_fold", "stem_unfold", "stem_conv_ln")}
+_GLOBAL_HOOKS = ("_global_forward_hooks", "_global_forward_pre_hooks")
 _CLASSES = (vig.ViG, vig.V2PatchEmbed, vig.LayerNorm2d, modules.GLABlock, modules.GatedLinearAttention, modules.GLAMLP, modules.RMSNorm,
             hier.HierViG, hier.VSSBlock, hier.GLA2D, hier.Mlp, hier.gMlp, nn.Linear, nn.Conv2d, nn.LayerNorm, nn.SiLU, nn.GELU, nn.Identity,
             nn.Sequential, nn.ModuleList)
@@ -26,7 +27,7 @@ def _status_seen(device):
 def _watch(plan, mods):
     """Everything whose change makes the plan stale (the C++ side compares identities, versions and sizes)."""
     plan.watch_modules(mods)
-    for name in ("_global_forward_hooks", "_global_forward_pre_hooks"):
+    for name in _GLOBAL_HOOKS:
         plan.watch_size(getattr(nn.modules.module, name))
     for name, fn in _OPS.items():
         plan.watch_item(ops.__dict__, name, fn)
@@ -107,7 +108,7 @@ def _hier(model):
 def _build(model, make):
     mods = list(model.modules())
     plan = None
-    if not (model.training or any(type(m) not in _CLASSES or "forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks for m in mods)):
+    if not (model.training or any(getattr(nn.modules.module, name) for name in _GLOBAL_HOOKS) or any(type(m) not in _CLASSES or "forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks for m in mods)):
         params = [p for m in mods for p in m._parameters.values() if p is not None]
         if all(p.dtype == params[0].dtype and p.device == params[0].device for p in params):
             with torch.no_grad():
