@@ -204,3 +204,30 @@ def test_global_hooks_see_every_module():
                 names.clear()
                 m(x)
                 assert not names
+
+
+def test_parameters_of_other_strides_and_convolutions_of_other_kinds():
+    """Transposed and strided parameters, also where address, version and identity stay the same, and a convolution that pads
+    otherwise: the modules' results."""
+    from vig_b200 import native
+    x = torch.randn(1, 3, 64, 64, device="cuda").bfloat16()
+    with torch.no_grad():
+        m = _model("vig_t", torch.bfloat16)
+        ref = m(x)
+        w = m.blocks[0].attn.o_proj.weight
+        w.data = w.data.t().contiguous().t()                            # the same values, column by column
+        assert native.vig_forward(m, x) is None and float((m(x) - ref).norm() / ref.norm()) < 1e-2
+        w.data = w.data.contiguous()
+        assert native.vig_forward(m, x) is not None
+        before = w.data_ptr()
+        w.data = w.data.t()                                             # square: other values at the same address
+        assert w.data_ptr() == before
+        turned = m(x)
+        w.data = w.data.contiguous()
+        fresh = m(x)
+        assert float((turned - fresh).norm() / fresh.norm()) < 1e-2 < float((turned - ref).norm() / ref.norm())
+        h = _model("hier", torch.float16)
+        y = x.half()
+        assert native.hier_forward(h, y) is not None
+        h.layers[0].downsample[1].padding_mode = "circular"
+        assert native.hier_forward(h, y) is None

@@ -106,7 +106,7 @@ struct Attn {
 // ---- what a plan was built from --------------------------------------------------------------------------------------
 struct Watch {
     struct Item { py::object dict, key, value; };
-    struct Param { Tensor t; int64_t version; void* data; at::ScalarType type; };
+    struct Param { Tensor t; int64_t version; void* data; at::ScalarType type; std::vector<int64_t> sizes, strides; };
     std::vector<Item> items;
     std::vector<std::pair<py::object, Py_ssize_t>> sizes;
     std::vector<std::pair<py::object, py::object>> absent;
@@ -115,7 +115,7 @@ struct Watch {
     void item(py::object d, py::object k, py::object v) { items.push_back({d, k, v}); }
     void size(py::object d) { sizes.emplace_back(d, PyDict_Size(d.ptr())); }
     void missing(py::object d, py::object k) { absent.emplace_back(d, k); }
-    void param(const Tensor& t, bool values) { params.push_back({t, values ? (int64_t)t._version() : -1, values ? t.data_ptr() : nullptr, t.scalar_type()}); }
+    void param(const Tensor& t, bool values) { params.push_back({t, values ? (int64_t)t._version() : -1, values ? t.data_ptr() : nullptr, t.scalar_type(), t.sizes().vec(), t.strides().vec()}); }
     // a module's plain attributes, parameters (values: what is in them too), children, hooks and the forward it overrides or not
     void module(py::handle m, bool values) {
         const py::dict d = m.attr("__dict__");
@@ -143,7 +143,7 @@ struct Watch {
         for (const auto& s : sizes) if (PyDict_Size(s.first.ptr()) != s.second) return false;
         for (const auto& a : absent) if (PyDict_GetItem(a.first.ptr(), a.second.ptr())) return false;
         for (const auto& p : params)
-            if (p.t.scalar_type() != p.type || (p.version >= 0 && ((int64_t)p.t._version() != p.version || p.t.data_ptr() != p.data))) return false;
+            if (p.t.scalar_type() != p.type || p.t.sizes() != p.sizes || p.t.strides() != p.strides || (p.version >= 0 && ((int64_t)p.t._version() != p.version || p.t.data_ptr() != p.data))) return false;
         return true;
     }
 };

@@ -37,7 +37,13 @@ def _norm(m):
     return dict(w=m.weight, b=getattr(m, "bias", None), eps=m.eps)
 
 
+class _NoPlan(Exception):
+    """The model has something that only its modules can evaluate."""
+
+
 def _conv(m, weight=None, stride=None, pad=None):
+    if len(set(m.stride)) != 1 or isinstance(m.padding, str) or len(set(m.padding)) != 1 or m.dilation != (1, 1) or m.groups != 1 or m.padding_mode != "zeros":
+        raise _NoPlan
     w = (m.weight.detach() if weight is None else weight).contiguous(memory_format=torch.channels_last)
     return dict(w=w, b=m.bias, stride=m.stride[0] if stride is None else stride, pad=m.padding[0] if pad is None else pad)
 
@@ -110,9 +116,13 @@ def _build(model, make):
     plan = None
     if not (model.training or any(getattr(nn.modules.module, name) for name in _GLOBAL_HOOKS) or any(type(m) not in _CLASSES or "forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks for m in mods)):
         params = [p for m in mods for p in m._parameters.values() if p is not None]
-        if all(p.dtype == params[0].dtype and p.device == params[0].device for p in params):
-            with torch.no_grad():
-                plan = make(model)
+        # vectors and matrices go to kernels by address, filters to the library, which takes any strides
+        if all(p.dtype == params[0].dtype and p.device == params[0].device and (p.dim() == 4 or p.is_contiguous()) for p in params):
+            try:
+                with torch.no_grad():
+                    plan = make(model)
+            except _NoPlan:
+                pass
     if plan is None:
         plan = _lib.host().Refusal()
     _watch(plan, mods)
