@@ -231,3 +231,21 @@ def test_parameters_of_other_strides_and_convolutions_of_other_kinds():
         assert native.hier_forward(h, y) is not None
         h.layers[0].downsample[1].padding_mode = "circular"
         assert native.hier_forward(h, y) is None
+
+
+@pytest.mark.parametrize("kind", ["vig_t", "hier", "hier_mlp"])
+def test_weights_written_without_a_trace(kind):
+    """Writes through .data leave a parameter's version alone; what needs no derived form -- filters of the strided convolutions,
+    projections, norms -- is read where it lies, also by a replayed graph."""
+    m, fresh = _model(kind, torch.float16), _model(kind, torch.float16)
+    x = torch.randn(2, 3, 64, 96, device="cuda").half()
+    convs = [m.patch_embed.proj[3]] if kind == "vig_t" else [c for c in m.modules() if isinstance(c, nn.Conv2d) and c.groups == 1]
+    with torch.no_grad():
+        for _ in range(3):
+            m(x)
+        for part in (convs, [l for l in m.modules() if isinstance(l, nn.LayerNorm)]):
+            for c in part:
+                c.weight.data.mul_(1.25)
+        changed = m(x)
+        fresh.load_state_dict(m.state_dict())
+        assert torch.equal(changed, fresh(x))

@@ -171,7 +171,7 @@ struct StatusPeek {
 };
 
 struct Conv {
-    Tensor w, b;                                         // channels-last weight; bias may be undefined
+    Tensor w, b;                                         // bias may be undefined
     int64_t stride = 1, pad = 0;
     // NHWC in, NHWC out
     Tensor forward(const Tensor& x, bool with_bias) const {
@@ -460,7 +460,7 @@ struct HierStage {
 struct HierPlan : PlanBase {
     std::vector<std::tuple<Conv, bool, Norm, int>> embed;   // convolution, whether a LayerNorm follows, the norm, activation (0 / 2 = GELU)
     std::vector<HierStage> stages;
-    Tensor first_w;                                          // [O,3,3,3] contiguous where the embedding's first convolution has a kernel of its own
+    Tensor first_w;                                          // [O,3,3,3] where the embedding's first convolution has a kernel of its own
     Norm last;
 
     OptT forward(const Tensor& x) {
@@ -473,7 +473,8 @@ struct HierPlan : PlanBase {
             const auto& [conv, has_norm, norm, act] = embed[0];
             const int64_t O = first_w.size(0);
             if (!y.defined()) y = at::empty({B, (H + 1) / 2, (W + 1) / 2, O}, img.options());
-            ok(api.vig_embed_conv_ln_fwd(ptr(img), ptr(first_w), ptr(conv.b), ptr(norm.w), ptr(norm.b), ptr(y), B, H, W, O, (float)norm.eps, act == 2, c.code, c.stream),
+            const Tensor w = first_w.contiguous();
+            ok(api.vig_embed_conv_ln_fwd(ptr(img), ptr(w), ptr(conv.b), ptr(norm.w), ptr(norm.b), ptr(y), B, H, W, O, (float)norm.eps, act == 2, c.code, c.stream),
                "vig_embed_conv_ln_fwd");
         } else {                                             // channels-last
             if (!y.defined()) y = at::empty({B, H, W, img.size(1)}, img.options());

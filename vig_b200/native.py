@@ -44,8 +44,8 @@ class _NoPlan(Exception):
 def _conv(m, weight=None, stride=None, pad=None):
     if len(set(m.stride)) != 1 or isinstance(m.padding, str) or len(set(m.padding)) != 1 or m.dilation != (1, 1) or m.groups != 1 or m.padding_mode != "zeros":
         raise _NoPlan
-    w = (m.weight.detach() if weight is None else weight).contiguous(memory_format=torch.channels_last)
-    return dict(w=w, b=m.bias, stride=m.stride[0] if stride is None else stride, pad=m.padding[0] if pad is None else pad)
+    # the parameter itself: what is written to it without a trace (through .data, by a replayed graph) reaches the next call
+    return dict(w=m.weight if weight is None else weight, b=m.bias, stride=m.stride[0] if stride is None else stride, pad=m.padding[0] if pad is None else pad)
 
 
 def _attn(a):
@@ -107,7 +107,7 @@ def _hier(model):
         stages.append(dict(blocks=blocks, conv=_conv(down[1]) if has else None, norm=_norm(down[3]) if has else None))
     head = model.classifier.head
     return _lib.host().HierPlan(dict(head_w=head.weight, head_b=head.bias, on_status=_status_seen(head.weight.device), graphs=getattr(model, "replay_graphs", True), embed=embed, stages=stages,
-                                     first_w=c.weight.detach().contiguous() if own else None,
+                                     first_w=c.weight if own else None,
                                      last=_norm(model.classifier.norm)))
 
 
