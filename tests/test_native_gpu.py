@@ -200,7 +200,7 @@ def test_global_hooks_see_every_module():
                     names.clear()
                     m(x)
                     handle.remove()
-                    assert names.count("GLABlock") == 2, names
+                    assert names.count("GatedLinearAttention") == 2, names
                 names.clear()
                 m(x)
                 assert not names
