@@ -60,3 +60,19 @@ def test_unaligned_rows_take_the_exact_form():
     odd = torch.zeros(1, 2, 70, 33, device="cuda")
     odd[..., 1:] = ins[0].cuda()
     assert rel_err(vig_b200.bi_gla(odd[..., 1:], *[t.cuda() for t in ins[1:]]), oracle.naive_bi_gla(*ins)) < 2e-5
+
+
+def test_a_call_without_workspace_runs_where_one_segment_needs_none():
+    """vig_bigla_fwd leaves the form to the library: 16-bit sequences of up to 256 tokens with an output need no workspace."""
+    from vig_b200 import _lib
+    B, H, L, d = 1, 3, 196, 64
+    ins = [t.bfloat16() for t in oracle.make_bigla_inputs(B, H, L, d, d, seed=8)]
+    dev, o = [t.cuda() for t in ins], torch.empty(B, H, L, d, device="cuda", dtype=torch.bfloat16)
+    st = _lib.lib().vig_bigla_fwd(*map(_lib.ptr, dev), _lib.ptr(o), B, H, L, d, d, _lib.dtype_code(o), *[None] * 6, -1.0, 1.0, 0.0, float("nan"), *[None] * 6, 3, 0,
+                                  None, 0, None, _lib.stream_ptr())
+    assert st == 0
+    assert rel_err(o.float(), oracle.naive_bi_gla(*[t.float() for t in ins])) < 1.5e-2
+    f32 = [t.float().cuda() for t in ins]
+    st = _lib.lib().vig_bigla_fwd(*map(_lib.ptr, f32), _lib.ptr(o), B, H, L, d, d, 0, *[None] * 6, -1.0, 1.0, 0.0, float("nan"), *[None] * 6, 3, 0, None, 0, None,
+                                  _lib.stream_ptr())
+    assert st == -5                                                      # fp32 has no such form: refused before any launch

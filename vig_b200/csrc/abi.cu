@@ -117,11 +117,13 @@ int vig::bigla_fwd_internal(const void* q, const void* k, const void* v, const v
         if (workspace && (reinterpret_cast<uintptr_t>(workspace) & 255)) return VIG_ERR_ALIGN;
         return bigla_wave_launch(p, workspace, workspace_bytes, (cudaStream_t)stream);
     }
-    if (impl == VIG_IMPL_SEG || (impl == VIG_IMPL_AUTO && !no_single && bigla_seg_supported(p) && bigla_seg_preferred(p))) {
+    // A caller that leaves the choice to the library, with less workspace than this form needs, gets the tensor-core form that
+    // does with it (none for one segment of up to 256 tokens with an output), where there is one.
+    const bool ws_fits = workspace && workspace_bytes >= bigla_simt_workspace(B, H, L, dk, dv) && !(reinterpret_cast<uintptr_t>(workspace) & 15);
+    const bool seg_runs = !(need_states || L > 64) || ws_fits;
+    if (impl == VIG_IMPL_SEG || (impl == VIG_IMPL_AUTO && !no_single && bigla_seg_supported(p) && bigla_seg_preferred(p) && (seg_runs || !bigla_tc_supported(p)))) {
         if (!bigla_seg_supported(p)) return VIG_ERR_SHAPE;
-        const bool needs_ws = need_states || L > 64;
-        if (needs_ws && (!workspace || workspace_bytes < bigla_simt_workspace(B, H, L, dk, dv))) return VIG_ERR_WORKSPACE;
-        if (needs_ws && (reinterpret_cast<uintptr_t>(workspace) & 15)) return VIG_ERR_ALIGN;
+        if (!seg_runs) return workspace && workspace_bytes >= bigla_simt_workspace(B, H, L, dk, dv) ? VIG_ERR_ALIGN : VIG_ERR_WORKSPACE;
         p.ws_state = reinterpret_cast<float*>(workspace);
         return bigla_seg_launch(p, (cudaStream_t)stream);
     }
