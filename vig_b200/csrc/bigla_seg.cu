@@ -26,6 +26,7 @@ namespace {
 
 using namespace mm;
 
+constexpr int SEG_NO_CLUSTER = -1001;                    // the device cannot place a cluster of this size: three launches instead
 enum { SEG_ONE = 0, SEG_STATES = 1, SEG_OUT = 2 };       // one launch (cluster = sequence) / contributions only / outputs from entering states
 
 template <int DK, int DV, typename T> struct SegTerms {
@@ -620,15 +621,20 @@ int seg_launch_mode(const SegParams& s, cudaStream_t stream) {
     attr[0].val.clusterDim.x = s.nseg; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = MODE == SEG_ONE && s.nseg > 1 ? 1 : 0;
-    if (MODE == SEG_ONE && s.nseg > 8) {                 // more than the portable cluster size: allowed once per kernel and device
-        static std::atomic<uint64_t> allowed{0};
+    if (MODE == SEG_ONE && s.nseg > 8) {                 // more than the portable cluster size: the device is asked once whether it can place it
+        static std::atomic<uint32_t> answers[64];        // two bits a size: asked, yes
         int dev = 0;
         if ((e = cudaGetDevice(&dev)) != cudaSuccess) return (int)e;
-        const uint64_t bit = 1ull << (dev & 63);
-        if (!(allowed.load() & bit)) {
-            if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess) return (int)e;
-            allowed.fetch_or(bit);
+        const uint32_t asked = 1u << (2 * (s.nseg - 9)), yes = 2u << (2 * (s.nseg - 9));
+        uint32_t have = answers[dev & 63].load();
+        if (!(have & asked)) {
+            int n = 0;
+            if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) n = 0;
+            cudaGetLastError();                          // a refusal is an answer
+            have = asked | (n > 0 ? yes : 0u);
+            answers[dev & 63].fetch_or(have);
         }
+        if (!(have & yes)) return SEG_NO_CLUSTER;
     }
     e = cudaLaunchKernelEx(&cfg, kern, s);
     return (int)(e != cudaSuccess ? e : cudaGetLastError());
@@ -645,7 +651,10 @@ int seg_launch(SegParams& s, cudaStream_t stream) {
     s.need_states = s.nseg > 1 || finals;
     p.nchunk = s.nseg;
     p.ws_decay = p.ws_state ? p.ws_state + (size_t)p.B * p.H * s.nseg * 2 * DK * DV : nullptr;
-    if (s.nseg <= CLUSTER) return seg_launch_mode<DK, DV, T, TOK, SEG_ONE>(s, stream);
+    if (s.nseg <= CLUSTER) {
+        const int r = seg_launch_mode<DK, DV, T, TOK, SEG_ONE>(s, stream);
+        if (r != SEG_NO_CLUSTER) return r;
+    }
     if (int e = seg_launch_mode<DK, DV, T, TOK, SEG_STATES>(s, stream)) return e;
     if (int e = bigla_scan_launch(p, stream)) return e;
     return p.o ? seg_launch_mode<DK, DV, T, TOK, SEG_OUT>(s, stream) : 0;
