@@ -249,3 +249,36 @@ def test_weights_written_without_a_trace(kind):
         changed = m(x)
         fresh.load_state_dict(m.state_dict())
         assert torch.equal(changed, fresh(x))
+
+
+def test_an_error_is_reported_once():
+    """A bit in the device's error word, seen by a forward's copy of it: the next forward or ``check_status`` reports it, not both."""
+    import vig_b200
+    m = _model("vig_t", torch.bfloat16)
+    x = torch.randn(1, 3, 64, 64, device="cuda").bfloat16()
+    word = vig_b200.ops.status_word("cuda").tensor
+
+    def left_by_a_forward():
+        word.fill_(2)
+        m(x)
+        torch.cuda.synchronize()
+
+    with torch.no_grad():
+        m(x)
+        torch.cuda.synchronize()
+        m(x)
+        torch.cuda.synchronize()
+        vig_b200.check_status()
+        left_by_a_forward()
+        with pytest.raises(RuntimeError, match="status 2"):
+            vig_b200.check_status()
+        for _ in range(3):
+            m(x)
+            torch.cuda.synchronize()
+        left_by_a_forward()
+        with pytest.raises(RuntimeError, match="status 2"):
+            m(x)
+        vig_b200.check_status()
+        for _ in range(3):
+            m(x)
+            torch.cuda.synchronize()

@@ -152,11 +152,12 @@ struct Watch {
 struct StatusPeek {
     int32_t* host = nullptr;
     cudaEvent_t event = nullptr;
-    bool pending = false;
+    bool pending = false, drop = false;                  // drop: the value under way has been reported and cleared
     static StatusPeek& of(int device) { static StatusPeek s[64]; return s[device]; }
     int poll(bool capturing) {
         if (capturing || !pending || cudaEventQuery(event) != cudaSuccess) return 0;
         pending = false;
+        if (drop) { drop = false; return 0; }
         return *host;
     }
     void snapshot(int device, cudaStream_t st, bool capturing) {
@@ -578,6 +579,11 @@ HierPlan* make_hier(const py::dict& d) {
 }  // namespace
 
 void bind_model(py::module_& m) {
+    m.def("drop_status", [](int device) {                // the error word was read and cleared otherwise
+        if (device < 0 || device >= 64) return;
+        StatusPeek& peek = StatusPeek::of(device);
+        peek.drop = peek.pending;
+    });
     auto watch = [](auto& cls) {
         using P = typename std::decay_t<decltype(cls)>::type;
         cls.def("watch_item", [](P& p, py::object d, py::object k, py::object v) { p.watch.item(d, k, v); })

@@ -32,14 +32,20 @@ class StatusWord:
         self._host = torch.zeros(1, dtype=torch.int32).pin_memory()
         self._event = None
 
+    def _drop_copies(self):
+        """Copies of the word that are under way, here and in the C++ forwards, hold what is being reported now."""
+        self._event = None
+        _lib.host().drop_status(self.tensor.get_device())
+
     def _raise(self, value):
         self.tensor.zero_()
+        self._drop_copies()
         what = "; ".join(msg for bit, msg in self.BITS.items() if value & bit) or "unknown bits"
         raise RuntimeError(f"vig_b200 kernels reported status {value}: {what}")
 
     def check(self):
         """Blocking read; raises (and clears the word) when a kernel has reported an error."""
-        self._event = None
+        self._drop_copies()
         value = int(self.tensor.item())
         if value:
             self._raise(value)
