@@ -133,3 +133,13 @@ def test_the_e_form_takes_a_workspace_of_any_alignment(dtype, dir_mask):
     assert all(torch.equal(a, b) for r in results[1:] for a, b in zip(r, results[0]))
     assert lib.vig_bigla_bwd(*map(_lib.ptr, ins), _lib.ptr(d_out), *map(_lib.ptr, results[0]), B, H, L, dk, dv, _lib.dtype_code(ins[0]), *[None] * 6, -1.0, 0.5, dir_mask,
                              ws.data_ptr() + 2, nbytes, _lib.stream_ptr()) == -4
+
+
+def test_saved_tensors_that_come_back_in_another_layout():
+    import vig_b200
+    ins = [t.cuda().requires_grad_() for t in oracle.make_bigla_inputs(1, 2, 70, 32, 64, seed=9)]
+    d_out = torch.randn(1, 2, 70, 64, generator=torch.Generator().manual_seed(3)).cuda()
+    ref = torch.autograd.grad(vig_b200.bi_gla(*ins), ins, d_out)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t.transpose(2, 3).contiguous().transpose(2, 3)):
+        o = vig_b200.bi_gla(*ins)
+    assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(o, ins, d_out), ref))

@@ -77,12 +77,14 @@ struct BiGla : torch::autograd::Function<BiGla> {
     }
     static variable_list backward(AutogradContext* ctx, variable_list grad_out) {
         const auto saved = ctx->get_saved_variables();
-        const Tensor &q = saved[0], &k = saved[1], &v = saved[2], &gf = saved[3], &gb = saved[4];
+        // a saved-tensor hook may hand a tensor back in another layout
+        auto rows = [](const Tensor& t) { return t.defined() && t.stride(3) != 1 && t.size(3) != 1 ? t.contiguous() : t; };
+        const Tensor q = rows(saved[0]), k = rows(saved[1]), v = rows(saved[2]), gf = rows(saved[3]), gb = rows(saved[4]);
         Tensor d = grad_out[0];
         variable_list none(11);
         if (!d.defined()) return none;
         c10::cuda::CUDAGuard dev(k.device());
-        if (d.stride(3) != 1) d = d.contiguous();
+        d = rows(d);
         const int B = k.size(0), H = k.size(1), L = k.size(2), dk = k.size(3), dv = v.size(3), mask = (int)ctx->saved_data["mask"].toInt();
         const Tensor dq = at::empty({B, H, L, dk}, k.options()), dkk = at::empty({B, H, L, dk}, k.options()), dvv = at::empty({B, H, L, dv}, k.options());
         Tensor df, db;
