@@ -76,3 +76,15 @@ def test_a_call_without_workspace_runs_where_one_segment_needs_none():
     st = _lib.lib().vig_bigla_fwd(*map(_lib.ptr, f32), _lib.ptr(o), B, H, L, d, d, 0, *[None] * 6, -1.0, 1.0, 0.0, float("nan"), *[None] * 6, 3, 0, None, 0, None,
                                   _lib.stream_ptr())
     assert st == -5                                                      # fp32 has no such form: refused before any launch
+
+
+@pytest.mark.parametrize("dk,B,H,L", [(64, 1, 3, 196), (64, 4, 6, 450), (32, 4, 3, 1000)])
+def test_bf16_rounds_no_more_often_than_the_tcgen05_form(dk, B, H, L):
+    """Errors against fp64 of the two forms that share these calls: the same operands rounded once each, so the same error but
+    for the sums' order (10 % of it)."""
+    import vig_b200
+    from vig_b200 import _lib
+    ins = [t.bfloat16() for t in oracle.make_bigla_inputs(B, H, L, dk, 64, seed=12)]
+    ref = oracle.chunked_bi_gla_f64(*[t.double() for t in ins])
+    err = {impl: float((vig_b200.bi_gla(*[t.cuda() for t in ins], impl=impl).double().cpu() - ref).norm() / ref.norm()) for impl in (_lib.IMPL_SEG, _lib.IMPL_TC_SPLIT)}
+    assert err[_lib.IMPL_SEG] < 1.1 * err[_lib.IMPL_TC_SPLIT], err

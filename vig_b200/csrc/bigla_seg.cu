@@ -15,7 +15,7 @@
 // memory round trip for the scores: P stays in registers, a segment's rows spread over all warps at once.  One segment takes
 // about 22 k cycles alone (loads and gates 6, tiles 3, contribution 4, products 3, states 3, read-out 2): a call of few
 // segments is that latency, one of many is bound by instruction issue at 16 warps an SM.
-// Operands are split into bf16 terms (mma_common.cuh): one term for bf16 with dv = 64 (as in the tcgen05 kernels), two for
+// Operands are split into bf16 terms (mma_common.cuh): one term for bf16 with dv = 64 (as in the two-CTAs-per-SM tcgen05 form), two for
 // fp16 and for dv = 32, three for fp32.  A segment whose |G - r| leaves the factorisation's range, contribution included,
 // is evaluated token by token (bigla_exact.cuh).
 #include <atomic>
@@ -47,15 +47,10 @@ template <int DK, int DV, typename T, int TOK> struct SegSmem {
     static_assert(TT::SC * DK * Pitch<DV>::B <= QT, "the entering states reuse the K tiles");
 };
 
-// x * e of a raw pair and a pair of fp32 factors, in SC bf16 terms (one term: factors rounded to bf16, packed multiply)
+// x * e of a raw pair and a pair of fp32 factors, in SC bf16 terms: the product in fp32, then rounded
 template <typename T, int SC> __device__ __forceinline__ void scaled(const Raw2<T>& x, float ex, float ey, uint32_t* t) {
-    if constexpr (SC == 1) {
-        const __nv_bfloat162 e = __floats2bfloat162_rn(ex, ey), r = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&x.w), e);
-        t[0] = *reinterpret_cast<const uint32_t*>(&r);
-    } else {
-        const F2 v = f2_mul(x.f2(), f2_make(ex, ey));
-        split2<SC>(f2_lo(v), f2_hi(v), t);
-    }
+    const F2 v = f2_mul(x.f2(), f2_make(ex, ey));
+    split2<SC>(f2_lo(v), f2_hi(v), t);
 }
 
 template <typename T, int COLS, int TERMS, int TOK> __device__ __forceinline__ void seg_load_v(uint8_t* dst, const T* src, int64_t stride_l, int n) {
