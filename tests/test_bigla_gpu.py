@@ -352,3 +352,19 @@ def test_wavefront_form_raw_logits_clamp_and_range_flag():
     wild = [t.bfloat16() for t in _strong_gate_inputs(4.0, L=600)]
     o = vig_b200.bi_gla(*[t.cuda() for t in wild], impl=_lib.IMPL_TC_WAVE, status=status)
     assert int(status.item()) & 2 and torch.isfinite(o.float()).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,H,L,dk", [(200, 6, 196, 64), (16, 3, 1500, 64), (20, 3, 600, 32)])
+def test_calls_between_the_forms_keep_their_sums_in_fp32(dtype, B, H, L, dk):
+    """Sequences of one segment, and fewer chains than SMs: no less exact than the segment-parallel tcgen05 form, which adds both
+    directions before it rounds (5 % for the sums' order)."""
+    import vig_b200
+    from vig_b200 import _lib
+    gen = torch.Generator(device="cuda").manual_seed(L)
+    rand = lambda d: torch.randn(B, H, L, d, generator=gen, device="cuda")  # noqa: E731
+    q, k, v = rand(dk).to(dtype), rand(dk).to(dtype), rand(64).to(dtype)
+    gf, gb = [(torch.nn.functional.logsigmoid(rand(dk)) / 16).to(dtype) for _ in range(2)]
+    ref = oracle.chunked_bi_gla_f64(*[t[:2].double().cpu() for t in (q, k, v, gf, gb)])
+    err = {impl: float((vig_b200.bi_gla(q, k, v, gf, gb, impl=impl)[:2].double().cpu() - ref).norm() / ref.norm()) for impl in (_lib.IMPL_AUTO, _lib.IMPL_TC_SPLIT)}
+    assert err[_lib.IMPL_AUTO] < 1.05 * err[_lib.IMPL_TC_SPLIT], err

@@ -127,7 +127,7 @@ int vig::bigla_fwd_internal(const void* q, const void* k, const void* v, const v
         p.ws_state = reinterpret_cast<float*>(workspace);
         return bigla_seg_launch(p, (cudaStream_t)stream);
     }
-    if (impl == VIG_IMPL_AUTO && (!no_single || L <= 256) && bigla_wave_supported(p) && bigla_wave_preferred(p) && workspace &&
+    if (impl == VIG_IMPL_AUTO && !no_single && bigla_wave_supported(p) && bigla_wave_preferred(p) && workspace &&
         !(reinterpret_cast<uintptr_t>(workspace) & 255) && workspace_bytes >= bigla_wave_workspace(B, H, L, dk, dv))
         return bigla_wave_launch(p, workspace, workspace_bytes, (cudaStream_t)stream);
     bool use_tc = false;

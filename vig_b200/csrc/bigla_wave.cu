@@ -825,24 +825,18 @@ bool bigla_wave_supported(const BiglaParams& p) {
 }
 
 // Measured on B200: with at least as many (sequence, direction) chains as SMs and two or more segments per sequence the
-// wavefront form beats the segment-parallel forms (0.46 against 0.58 ms at 64 x 3 sequences of 4096 tokens); with
-// fewer chains its CTAs idle.
+// wavefront form beats the segment-parallel forms (0.46 against 0.58 ms at 64 x 3 sequences of 4096 tokens).  It would also do
+// so from 9/16 of a chain per SM on (96 chains of 4096 tokens, dk = 64, 110 us against 142) and for many sequences of a single
+// segment (768 of 196 tokens, 76 against 84), but its outputs are less exact -- the second direction is added to the stored
+// first one, both rounded to the type: 0.0043 against 0.0032 in bf16 -- so those calls stay where their sums are fp32.
 bool bigla_wave_preferred(const BiglaParams& p) {
     const int sms = wave_sm_count();
     const int ndir = p.dir_mask == 3 ? 2 : 1;
-    // Below one chain per SM this form still takes the time of one chain, the segment-parallel one time in proportion to the
-    // work: 96 chains of 4096 tokens, dk = 64, 110 us against 142; 48 chains 107 against 79.  (dk = 32: 192 chains of 3136, 125
-    // against 175.)
-    const long long chains = (long long)p.B * p.H * ndir;
-    // One segment a sequence has nothing to hand on, but with many of them the roles of this form still overlap better: 768
-    // sequences of 196 tokens, dk = 64, 76 us against 84 (dk = 32: 76 against 68).
-    if (p.L <= W_SEG_CHUNKS_MIN * CHUNK) return sms > 0 && p.dk == 64 && chains >= 8ll * sms;
-    return sms > 0 && chains * 16 >= sms * (p.dk == 64 ? 9ll : 13ll);
+    return sms > 0 && p.L > W_SEG_CHUNKS_MIN * CHUNK && (long long)p.B * p.H * ndir >= sms;
 }
 
 // Counters (ticket, chain progress, chunk flags) followed by the state mailboxes.
 size_t bigla_wave_workspace(int B, int H, int L, int dk, int dv) {
-    if (L <= W_SEG_CHUNKS_MIN * CHUNK) return wave_counter_bytes(B, H, L);   // one step a chain: no mailbox
     (void)dk; (void)dv;                                     // the mailbox slots hold the kernel's 64 x 64 states whatever dk is
     return wave_counter_bytes(B, H, L) + (size_t)B * H * 2 * 2 * ((size_t)WDK * WDV + WDK) * sizeof(float);
 }

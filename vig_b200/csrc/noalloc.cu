@@ -63,8 +63,7 @@ extern "C" int vig_bigla_fwd_noalloc(const void* q, const void* k, const void* v
     if (int st = scratch_for_current_device(&scratch)) return st;
     // The launcher sizes the scratch for the kernel family that will really run with these pointers and this shape
     // (nothing for a single 256-token segment on the tensor-core path) and refuses before any launch when the array
-    // is too small.  The single-launch form, and the wavefront form for more than one segment, need more scratch than the array
-    // holds: ruled out here.
+    // is too small.  The single-launch and wavefront forms need more scratch than the array holds: ruled out here.
     // Every workspace slot a call reads is written earlier in the same call, so nothing needs clearing
     // between calls; what the previous call left behind is simply overwritten.
     const int st = bigla_fwd_internal(q, k, v, g_fwd, g_bwd, o, B, H, L, dk, dv, dtype, strides_q, strides_k, strides_v, strides_gf,
