@@ -87,6 +87,27 @@ def test_fp32_is_as_exact_as_the_recurrence_in_fp32(dk, dv, L, norm):
     assert all(e < 2.8e-7 for e in errs[:4]) and all(e < 5e-7 for e in errs[4:]), errs
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("dk,dv,L", [(16, 32, 100), (64, 64, 300)])
+def test_fp32_gate_gradients_of_16_bit_inputs(dtype, dk, dv, L):
+    """``bi_gla_backward`` returns them in fp32 whatever the inputs' type, through the library call as through Python: sums of fp32
+    products (1e-6), the other gradients rounded once."""
+    import vig_b200
+    from vig_b200 import _lib
+    (q, k, v), (xf, xb), d_out = _inputs(dtype, 1, 3, L, dk, dv, seed=L + dk)
+    gf, gb = ((torch.nn.functional.logsigmoid(x) / 16).to(dtype) for x in (xf, xb))
+    ref = _reference(q, k, v, gf, gb, d_out, 0.5, 0.0)[1:]
+    got = vig_b200.bi_gla_backward(q, k, v, gf, gb, d_out, out_scale=0.5)
+    lib, outs = _lib.lib(), [torch.empty(*t.shape, dtype=torch.float32 if i > 2 else dtype, device="cuda") for i, t in enumerate(ref)]
+    ws = torch.empty(lib.vig_bigla_bwd_full_workspace_bytes(1, 3, L, dk, dv), dtype=torch.uint8, device="cuda")
+    assert lib.vig_bigla_bwd_full(*map(_lib.ptr, (q, k, v, gf, gb, d_out, *outs)), 1, 1, 3, L, dk, dv, _lib.dtype_code(q), *[None] * 6, -1.0, 0.5, 0.0, float("nan"), 3,
+                                  _lib.ptr(ws), ws.numel(), _lib.stream_ptr()) == 0
+    for grads in (got, outs):
+        errs = _errors(grads, ref)
+        assert [g.dtype for g in grads] == [dtype] * 3 + [torch.float32] * 2
+        assert all(e < 2e-6 for e in errs[3:]) and all(e < (2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12) for e in errs[:3]), errs
+
+
 def _log_gates(kind, x):
     """Log-gates that a segment's factored form cannot take, made from normal numbers x [B, H, L, dk]."""
     g = torch.nn.functional.logsigmoid(x) / 16

@@ -407,7 +407,9 @@ extern "C" int vig_bigla_bwd_full(const void* q, const void* k, const void* v, c
     if (reinterpret_cast<uintptr_t>(workspace) & 15) return VIG_ERR_ALIGN;
     p.dgf = dg_fwd; p.dgb = dg_bwd; p.dg_f32 = dg_fp32 != 0;
     p.gate_norm = gate_logit_normalizer; p.clamp_min = clamp_min;
-    if (!bigla_bwd_mma_supported(p)) return bwd_simt(p, 0, (cudaStream_t)stream);
+    // fp32 gate gradients of 16-bit inputs: token by token, whose sums are fp32 (1e-6 of them; the tensor-core form's operands
+    // carry 16 bits there, 1e-5)
+    if (!bigla_bwd_mma_supported(p) || (p.dg_f32 && dtype != VIG_DTYPE_F32)) return bwd_simt(p, 0, (cudaStream_t)stream);
     const int st = bigla_bwd_mma_launch(p, (cudaStream_t)stream);
     return st ? st : bwd_simt(p, 1, (cudaStream_t)stream);             // the chunks whose gates left the factorisation range
 }

@@ -206,6 +206,13 @@ def bi_gla(q, k, v, g_fwd, g_bwd, scale=-1, out_scale=1.0, *, out=None, gate_log
 
 def _backward(q, k, v, g_fwd, g_bwd, d_out, scale, out_scale, gate_norm, clamp_min, dir_mask, dg_fp32):
     """All gradients of ``bi_gla`` in one library call; gate gradients in fp32 or in the gates' dtype."""
+    if dg_fp32 and k.dtype in (torch.bfloat16, torch.float16):
+        # gate gradients finer than the inputs' type: everything in fp32 (the 16-bit kernels carry 16 bits of an operand, 1e-5 of
+        # the gate gradients; this is 3e-7), the other gradients rounded once
+        _check_scan_shapes(q, k, v, g_fwd, g_bwd, d_out)
+        wide = [None if t is None else t.float() for t in (q, k, v, g_fwd, g_bwd, d_out)]
+        dq, dk, dv, dg_f, dg_b = _backward(*wide, scale, out_scale, gate_norm, clamp_min, dir_mask, True)
+        return dq.to(k.dtype), dk.to(k.dtype), dv.to(k.dtype), dg_f, dg_b
     dev = _same_device(q, k, v, g_fwd, g_bwd, d_out)
     _check_scan_shapes(q, k, v, g_fwd, g_bwd, d_out)
     B, H, L, dk = k.shape
