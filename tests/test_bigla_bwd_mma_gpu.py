@@ -42,3 +42,23 @@ def test_unaligned_rows_take_the_exact_form():
     got = vig_b200.bi_gla_backward(odd[..., 1:], *[t.cuda() for t in (k, v, gf, gb, d_out)])
     errs = {n: rel_err(g.float(), r) for n, g, r in zip(NAMES, got, ref)}
     assert all(e < 2e-5 for e in errs.values()), errs
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("L,dk,dv,norm", [(63, 64, 64, 0.0), (64, 32, 64, 16.0), (65, 64, 64, 16.0), (128, 16, 32, 0.0), (193, 32, 32, 16.0), (200, 64, 64, 16.0)])
+def test_training_step_in_16_bits(dtype, L, dk, dv, norm):
+    """The 16-bit kernels, as training runs them: gate gradients in the gates' type, log-gates or raw logits without a clamp."""
+    import vig_b200
+    gen = torch.Generator().manual_seed(L)
+    q, k, v, xf, xb, d_out = [torch.randn(2, 2, L, d, generator=gen).to(dtype) for d in (dk, dk, dv, dk, dk, dv)]
+    if not norm:
+        xf, xb = ((torch.nn.functional.logsigmoid(x.float()) / 16).to(dtype) for x in (xf, xb))
+    leaves = [t.cuda().requires_grad_() for t in (q, k, v, xf, xb)]
+    o = vig_b200.bi_gla(*leaves, out_scale=0.5, gate_logit_normalizer=norm)
+    got = torch.autograd.grad(o, leaves, d_out.cuda())
+    gf, gb = (torch.nn.functional.logsigmoid(x.double()) / norm if norm else x.double() for x in (xf, xb))
+    _, ref = _reference_grads(q.float(), k.float(), v.float(), gf, gb, d_out.float(), 0.5, 3)
+    if norm:
+        ref = [*ref[:3], *(g * torch.sigmoid(-x.double()) / norm for g, x in zip(ref[3:], (xf, xb)))]
+    errs = {n: rel_err(g.float(), r) for n, g, r in zip(NAMES, got, ref)}
+    assert all(e < TOL[dtype] for e in errs.values()), errs
