@@ -170,3 +170,48 @@ def test_gradients_of_chunks_outside_the_range(dtype, dk, dv, L, kind):
     errs = _errors(_run((q, k, v, gf, gb), d_out), ref)
     assert all(e < TOL[dtype] for e in errs[1:4]), errs
     assert all(e < max(1e-4, TOL[dtype]) for e in errs[4:]), errs
+
+
+@pytest.mark.parametrize("dtype,dk,dv", [(torch.float32, 32, 64), (torch.float32, 64, 64), (torch.bfloat16, 32, 32), (torch.float16, 16, 32)])
+@pytest.mark.parametrize("L", [40, 150, 700])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_what_is_not_finite_stays_with_the_tokens_that_see_it(dtype, dk, dv, L, bad):
+    """Causal, one token's q, k or v: tokens before it, and value columns beside it, are those of the clean call."""
+    import vig_b200
+    (q, k, v), (x, _), d_out = _inputs(dtype, 1, 3, L, dk, dv, seed=L)
+    g = (torch.nn.functional.logsigmoid(x) / 16).to(dtype)
+    at = 2 * L // 3
+    clean, _ = vig_b200.fused_chunk_gla(q, k, v, g)
+    for which in range(3):
+        ins = [t.clone() for t in (q, k, v)]
+        ins[which][0, 1, at, 5] = bad
+        o, _ = vig_b200.fused_chunk_gla(*ins, g)
+        same = torch.ones_like(o, dtype=torch.bool)
+        same[0, 1, at:at + 1 if which == 0 else None] = False
+        if which == 2:
+            same[0, 1, at:] = torch.arange(dv, device="cuda") != 5
+        scale = float(clean.float().abs().max())
+        assert float((o.float() - clean.float())[same].abs().max()) <= TOL[dtype] * scale
+        assert not torch.isfinite(o[0, 1, at, 5] if which == 2 else o[0, 1, at]).all()
+
+
+@pytest.mark.parametrize("dtype,dk,dv", [(torch.float32, 32, 64), (torch.bfloat16, 64, 64), (torch.float16, 16, 32)])
+@pytest.mark.parametrize("L", [40, 150])
+def test_gradients_of_tokens_that_do_not_see_what_is_not_finite(dtype, dk, dv, L):
+    """Causal: d_out of one token is NaN.  The gradients of q before and after it, of k and v after it are those of the clean call."""
+    import vig_b200
+    (q, k, v), (x, _), d_out = _inputs(dtype, 1, 2, L, dk, dv, seed=L)
+    leaves = [t.requires_grad_(True) for t in (q, k, v, (torch.nn.functional.logsigmoid(x) / 16).to(dtype))]
+    at, spoilt = L // 2, d_out.clone()
+    spoilt[0, 1, at, 3] = float("nan")
+    o, _ = vig_b200.fused_chunk_gla(*leaves)
+    clean = torch.autograd.grad(o, leaves, d_out, retain_graph=True)
+    got = torch.autograd.grad(o, leaves, spoilt)
+    for i, (a, b) in enumerate(zip(got[:3], clean)):
+        same = torch.ones_like(a, dtype=torch.bool)
+        if i == 0:
+            same[0, 1, at] = False
+        else:
+            same[0, 1, :at + 1] = False
+        assert float((a.float() - b.float())[same].abs().max()) <= TOL[dtype] * float(b.float().abs().max()), i
+        assert torch.isnan(a[0, 1, at]).any()

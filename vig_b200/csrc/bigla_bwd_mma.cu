@@ -112,9 +112,14 @@ __global__ void __launch_bounds__(NT, states_min_blocks<DK, DV, T>()) bwd_states
     load_gate(first);
     load_rows(k, head_ptr<T>(p.k, p.sk, b, h, t0) + 2 * pr, p.sk[2], r0, n);
     load_rows(q, head_ptr<T>(p.q, p.sq, b, h, t0) + 2 * pr, p.sq[2], r0, n);
-    load_raw<T, DV, RAW>(smem + SM::V, head_ptr<T>(p.v, p.sv, b, h, t0), p.sv[2], n);
-    load_raw<T, DV, RAW>(smem + SM::O, head_ptr<T>(p.dout, p.sdo, b, h, t0), p.sdo[2], n);
+    float mark = 0.f;
+    load_raw<T, DV, RAW>(smem + SM::V, head_ptr<T>(p.v, p.sv, b, h, t0), p.sv[2], n, mark);
+    load_raw<T, DV, RAW>(smem + SM::O, head_ptr<T>(p.dout, p.sdo, b, h, t0), p.sdo[2], n, mark);
     zero_rows(k, r0, n); zero_rows(q, r0, n);
+    F2 seen = f2_make(0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < CL::RPG; ++r) { see(seen, k[r].f2()); see(seen, q[r].f2()); }
+    bool finite = clean(seen);
     const int last = one_dir ? first : p.dir_mask & 2 ? 1 : 0;
     int exact = 0;                                                       // directions left to the exact form, after the loop: nothing of it lives across the call
     for (int dir = first; dir <= last; ++dir) {
@@ -138,7 +143,8 @@ __global__ void __launch_bounds__(NT, states_min_blocks<DK, DV, T>()) bwd_states
             for (int i = 0; i < SC; ++i) *reinterpret_cast<uint32_t*>(smem + SM::Q + i * C * Pitch<DK>::B + (r0 + r) * Pitch<DK>::B + pr * 4) = t[i];
         }
         wait_raw();
-        if (__syncthreads_or(!in_range<T>(G, ref, tot, sizeof(T) == 2 && p.gate_norm > 0.f))) {
+        if (dir == first) finite = finite && raw_clean<T, DV, RAW>(smem + SM::V, mark) && raw_clean<T, DV, RAW>(smem + SM::O, mark);
+        if (__syncthreads_or(!finite || !in_range<T>(G, ref, tot, sizeof(T) == 2 && p.gate_norm > 0.f))) {
             exact |= 1 << dir;
             continue;
         }
@@ -241,8 +247,10 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 1 : 2) bwd_grads_mma_kern
     const T* qp = head_ptr<T>(p.q, p.sq, b, h, t0) + 2 * pr;
     const T* kp = head_ptr<T>(p.k, p.sk, b, h, t0) + 2 * pr;
     const F2 cc = f2_make(p.c, p.c), minus = f2_make(-1.f, -1.f);
-    load_raw<T, DV, RAW>(smem + SM::V, head_ptr<T>(p.v, p.sv, b, h, t0), p.sv[2], n);
-    load_raw<T, DV, RAW>(smem + SM::O, head_ptr<T>(p.dout, p.sdo, b, h, t0), p.sdo[2], n);
+    float mark = 0.f;
+    bool finite = true;
+    load_raw<T, DV, RAW>(smem + SM::V, head_ptr<T>(p.v, p.sv, b, h, t0), p.sv[2], n, mark);
+    load_raw<T, DV, RAW>(smem + SM::O, head_ptr<T>(p.dout, p.sdo, b, h, t0), p.sdo[2], n, mark);
     const uint32_t aV = sb + SM::V + 16 * w * PV + frag_rows<PV>(lane), aO = sb + SM::O + 16 * w * PV + frag_rows<PV>(lane);
     const uint32_t aK = sb + SM::K + 16 * w * PK + frag_rows<PK>(lane);
     const uint32_t bV = sb + SM::V + frag_cols<PV>(lane), bO = sb + SM::O + frag_cols<PV>(lane), bQ = sb + SM::Q + frag_cols<PK>(lane);
@@ -282,6 +290,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 1 : 2) bwd_grads_mma_kern
             F2 G[RPG], ref, tot;
             cum_gates<DK, T>(G, ref, tot, gsum, x, n, dir, p.gate_norm, p.clamp_min);
             zero_rows(q, r0, n); zero_rows(k, r0, n);
+            F2 seen = f2_make(0.f, 0.f);
             const float lim = range_limit<T>();
             const F2 rest = f2_fma(ref, minus, tot);
             bool fine = fabsf(f2_lo(ref)) <= lim && fabsf(f2_hi(ref)) <= lim && fabsf(f2_lo(rest)) <= lim && fabsf(f2_hi(rest)) <= lim;
@@ -295,6 +304,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 1 : 2) bwd_grads_mma_kern
                 fine = fine && fabsf(f2_lo(y)) <= lim && fabsf(f2_hi(y)) <= lim;
                 const F2 ex = f2_make(ex2_t<T>(f2_lo(y)), ex2_t<T>(f2_hi(y)));
                 X[r * NT + threadIdx.x] = ex;
+                see(seen, q[r].f2()); see(seen, k[r].f2());
                 uint32_t t[SC];
                 const F2 qs = f2_mul(f2_mul(q[r].f2(), cc), ex), ks = f2_mul(k[r].f2(), f2_make(ex2_t<T>(-f2_lo(y)), ex2_t<T>(-f2_hi(y))));
                 split2<SC>(f2_lo(qs), f2_hi(qs), t);
@@ -305,7 +315,8 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 1 : 2) bwd_grads_mma_kern
                 for (int i = 0; i < SC; ++i) *reinterpret_cast<uint32_t*>(smem + SM::K + i * TK + (r0 + r) * PK + pr * 4) = t[i];
             }
             wait_raw();
-            if (__syncthreads_or(!fine)) {                               // left to the exact kernel, outputs included
+            if (dir == 0 || !(p.dir_mask & 1)) finite = raw_clean<T, DV, RAW>(smem + SM::V, mark) && raw_clean<T, DV, RAW>(smem + SM::O, mark);
+            if (__syncthreads_or(!fine || !finite || !clean(seen))) {    // left to the exact kernel, outputs included
                 if (threadIdx.x == 0) p.flags[(size_t)bh * p.nchunk + c] = 1;
                 return;
             }

@@ -53,7 +53,7 @@ template <typename T, int SC> __device__ __forceinline__ void scaled(const Raw2<
     split2<SC>(f2_lo(v), f2_hi(v), t);
 }
 
-template <typename T, int COLS, int TERMS, int TOK> __device__ __forceinline__ void seg_load_v(uint8_t* dst, const T* src, int64_t stride_l, int n) {
+template <typename T, int COLS, int TERMS, int TOK> __device__ __forceinline__ void seg_load_v(uint8_t* dst, const T* src, int64_t stride_l, int n, float& mark) {
     constexpr uint32_t P = Pitch<COLS>::B;
     constexpr int NTH = 2 * TOK * SegWarps<T>::CW;
     if constexpr (TERMS == 1) {
@@ -73,12 +73,24 @@ template <typename T, int COLS, int TERMS, int TOK> __device__ __forceinline__ v
             const int i = i0 + threadIdx.x, r = i / PPR, v = i % PPR;
             float2 a = make_float2(0.f, 0.f), b = a;
             if (r < n) { a = load2<T>(src + r * stride_l + 4 * v); b = load2<T>(src + r * stride_l + 4 * v + 2); }
+            see(mark, a.x); see(mark, a.y); see(mark, b.x); see(mark, b.y);
             uint32_t ta[TERMS], tb[TERMS];
             split2<TERMS>(a.x, a.y, ta); split2<TERMS>(b.x, b.y, tb);
 #pragma unroll
             for (int t = 0; t < TERMS; ++t) *reinterpret_cast<uint2*>(dst + t * TOK * P + r * P + v * 8) = make_uint2(ta[t], tb[t]);
         }
     }
+}
+
+// whether the values this thread copied are finite (one-term tiles, after the copies have landed)
+template <int COLS, int TOK, int NTH> __device__ __forceinline__ bool seg_v_clean(const uint8_t* tile) {
+    uint32_t bad = 0;
+#pragma unroll
+    for (int i0 = 0; i0 < TOK * (COLS / 8); i0 += NTH) {
+        const int i = i0 + threadIdx.x;
+        bad |= bf16_unclean(*reinterpret_cast<const uint4*>(tile + i / (COLS / 8) * Pitch<COLS>::B + i % (COLS / 8) * 16));
+    }
+    return bad == 0;
 }
 
 struct SegParams {
@@ -273,7 +285,12 @@ __global__ void __launch_bounds__(2 * TOK * SegWarps<T>::CW, seg_min_blocks<DK, 
     Raw2<T> kr[RPG];
     bool fine = true, bad;
     {   // ---- every input of the segment requested at once, gates cumulated, operand tiles written
-        seg_load_v<T, DV, RAW, TOK>(smem + SM::V, head_ptr<T>(p.v, p.sv, b, h, t0), p.sv[2], n);
+        // fp32 calls and heads of dv = 32 keep infinities and NaN to the tokens that see them, as the recurrences do; the other
+        // 16-bit heads share a tcgen05 form in which they reach a chunk
+        constexpr bool CHECK = sizeof(T) == 4 || DV == 32;
+        float mark = 0.f;
+        F2 seen = f2_make(0.f, 0.f);
+        seg_load_v<T, DV, RAW, TOK>(smem + SM::V, head_ptr<T>(p.v, p.sv, b, h, t0), p.sv[2], n, mark);
         const bool logits = p.gate_norm > 0.f, clamp = p.clamp_min == p.clamp_min;
         Raw2<T> qr[RPG];
         {
@@ -297,6 +314,10 @@ __global__ void __launch_bounds__(2 * TOK * SegWarps<T>::CW, seg_min_blocks<DK, 
 #pragma unroll
                 for (int r = 0; r < RPG; ++r)
                     if (r0 + r >= n) { kr[r].zero(); qr[r].zero(); xr[0][r].open_gate(logits); xr[1][r].open_gate(logits); }
+            }
+            if (CHECK) {
+#pragma unroll
+                for (int r = 0; r < RPG; ++r) { see(seen, kr[r].f2()); see(seen, qr[r].f2()); }
             }
             const F2 zero = f2_make(0.f, 0.f);
             const F2 nlog2e = f2_make(-tc::LOG2E, -tc::LOG2E);
@@ -369,6 +390,10 @@ __global__ void __launch_bounds__(2 * TOK * SegWarps<T>::CW, seg_min_blocks<DK, 
                     *reinterpret_cast<float2*>(p.ws_decay + (((size_t)bh * s.nseg + c) * 2 + dir) * DK + 2 * pr) = make_float2(f2_lo(run) * tc::LN2, f2_hi(run) * tc::LN2);
             }
             shift[dir] = MODE == SEG_STATES ? f2_fma(run, minus, off) : f2_fma(ref[dir], minus, off);        // G - (total or reference)
+        }
+        if (CHECK) {
+            if (RAW == 1) asm volatile("cp.async.wait_all;" ::: "memory");
+            fine = fine && clean(seen) && (RAW == 1 ? seg_v_clean<DV, TOK, NTH>(smem + SM::V) : clean(mark));
         }
         bad = __syncthreads_or(!fine);
 #pragma unroll

@@ -42,6 +42,18 @@ __device__ __forceinline__ void mma16816(float* c, const uint32_t* a, const uint
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
+// Infinities and NaN among inputs.  In a masked product they would reach the tokens that the mask keeps from them (0 times inf),
+// and of an infinity's second term only NaN is left; the recurrences have neither.  ``mark`` becomes NaN once it has seen one;
+// packed bf16 pairs are asked by their exponent bits.
+__device__ __forceinline__ void see(float& mark, float x) { mark = fmaf(x, 0.f, mark); }
+__device__ __forceinline__ void see(F2& mark, F2 x) { mark = f2_fma(x, f2_make(0.f, 0.f), mark); }
+__device__ __forceinline__ bool clean(float mark) { return mark == 0.f; }
+__device__ __forceinline__ bool clean(F2 mark) { return f2_lo(mark) == 0.f && f2_hi(mark) == 0.f; }
+__device__ __forceinline__ uint32_t bf16_unclean(uint4 v) {
+    auto bits = [](uint32_t w) { return (w & 0x7F807F80u) + 0x00800080u; };
+    return (bits(v.x) | bits(v.y) | bits(v.z) | bits(v.w)) & 0x80008000u;
+}
+
 // Lane's address offset inside a tile for the four 8x8 matrices of an ldmatrix.x4 (PITCH in bytes):
 //   frag_rows: matrices (rows 0-7, cols 0-7), (rows 8-15, cols 0-7), (rows 0-7, cols 8-15), (rows 8-15, cols 8-15)
 //              A operand of a [m][k] tile; with .trans the B operand pair (n tiles 0, 1) of a [k][n] tile
@@ -134,7 +146,7 @@ template <typename T> __device__ __forceinline__ float ex2_t(float x) { return s
 
 // [C x COLS] rows of a strided tensor -> TERMS bf16 tiles (rows past n are zero); tile t at dst + t * C * pitch.  One term is
 // copied asynchronously: wait_raw() before the barrier that publishes the tiles.
-template <typename T, int COLS, int TERMS> __device__ __forceinline__ void load_raw(uint8_t* dst, const T* src, int64_t stride_l, int n) {
+template <typename T, int COLS, int TERMS> __device__ __forceinline__ void load_raw(uint8_t* dst, const T* src, int64_t stride_l, int n, float& mark) {
     constexpr uint32_t P = Pitch<COLS>::B;
     if constexpr (sizeof(T) == 2 && TERMS == 1) {
         constexpr int VPR = COLS / 8;                                  // 16-byte vectors per row
@@ -151,12 +163,26 @@ template <typename T, int COLS, int TERMS> __device__ __forceinline__ void load_
             const int i = i0 + threadIdx.x, r = i / PPR, v = i % PPR;
             float2 a = make_float2(0.f, 0.f), b = a;
             if (r < n) { a = load2<T>(src + r * stride_l + 4 * v); b = load2<T>(src + r * stride_l + 4 * v + 2); }
+            see(mark, a.x); see(mark, a.y); see(mark, b.x); see(mark, b.y);
             uint32_t ta[TERMS], tb[TERMS];
             split2<TERMS>(a.x, a.y, ta); split2<TERMS>(b.x, b.y, tb);
 #pragma unroll
             for (int t = 0; t < TERMS; ++t) *reinterpret_cast<uint2*>(dst + t * C * P + r * P + v * 8) = make_uint2(ta[t], tb[t]);
         }
     }
+}
+
+// whether the values this thread loaded are finite (after wait_raw(); one-term tiles are looked at where they lie)
+template <typename T, int COLS, int TERMS> __device__ __forceinline__ bool raw_clean(const uint8_t* tile, float mark) {
+    if constexpr (sizeof(T) == 2 && TERMS == 1) {
+        uint32_t bad = 0;
+#pragma unroll
+        for (int i0 = 0; i0 < C * (COLS / 8); i0 += NT) {
+            const int i = i0 + threadIdx.x;
+            bad |= bf16_unclean(*reinterpret_cast<const uint4*>(tile + i / (COLS / 8) * Pitch<COLS>::B + i % (COLS / 8) * 16));
+        }
+        return bad == 0;
+    } else return clean(mark);
 }
 
 // Thread layout of the per-channel passes over a chunk: thread = (pair of channels, group of RPG consecutive tokens).
