@@ -282,3 +282,24 @@ def test_an_error_is_reported_once():
         for _ in range(3):
             m(x)
             torch.cuda.synchronize()
+
+
+def test_a_plan_is_replaced_while_the_caller_captures():
+    """A change of the model inside the caller's own capture drops the plan and its graphs: the capture goes on."""
+    from vig_b200 import native
+    m = _model("vig_s", torch.bfloat16)
+    x = torch.randn(2, 3, 64, 64, device="cuda").bfloat16()
+    with torch.no_grad():
+        for _ in range(3):
+            m(x)
+        assert native._plans[m].graphs() == 1
+        ref = m(x)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            m.replay_graphs = False
+            y = m(x)
+        assert native._plans[m].graphs() == 0
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, ref)

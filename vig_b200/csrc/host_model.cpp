@@ -220,8 +220,14 @@ struct PlanBase {
         std::unique_ptr<at::cuda::CUDAEvent> done;       // behind the last replay: the graph's memory is not given back before
         Tensor in, out, held;                            // held: what the graph reads and the plan may replace
         std::vector<c10::DataPtr> scratch;               // the GEMM library's workspaces that its kernels write
+        // Also while the caller captures a graph of its own, where waiting for an event would spoil that capture but for the
+        // relaxed mode: the event was recorded outside it
         ~Captured() {
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            cudaThreadExchangeStreamCaptureMode(&mode);
             if (done) { try { done->synchronize(); } catch (...) {} }
+            graph.reset();
+            cudaThreadExchangeStreamCaptureMode(&mode);
         }
     };
     bool graphs = true;
