@@ -303,3 +303,24 @@ def test_a_plan_is_replaced_while_the_caller_captures():
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(y, ref)
+
+
+def test_dispatch_modes_see_the_forward():
+    """A mode that watches torch's operators (operation counters, loggers) sees a forward's GEMMs, also once it is replayed."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Count(TorchDispatchMode):
+        seen = 0
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.seen += "mm" in str(func)
+            return func(*args, **(kwargs or {}))
+
+    m = _model("vig_s", torch.bfloat16)
+    x = torch.randn(2, 3, 64, 64, device="cuda").bfloat16()
+    with torch.no_grad():
+        for _ in range(3):
+            ref = m(x)
+        with Count() as c:
+            y = m(x)
+        assert c.seen >= 4 and torch.equal(y, ref) and torch.equal(m(x), ref)

@@ -14,6 +14,7 @@
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAEvent.h>
 #include <ATen/cuda/CUDAGraph.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAException.h>
 #include <ATen/ops/empty.h>
 
@@ -190,7 +191,7 @@ struct PlanBase {
 
     bool takes(const Tensor& x) const {
         return x.is_cuda() && x.device() == device && x.scalar_type() == type && x.dim() == 4 && x.size(1) == 3 && x.numel() > 0 &&
-               !(at::GradMode::is_enabled()) && !at::autocast::is_autocast_enabled(at::kCUDA) && status_known(device.index()) && watch.same();
+               !(at::GradMode::is_enabled()) && !at::autocast::is_autocast_enabled(at::kCUDA) && !c10::impl::TorchDispatchModeTLS::any_modes_set() && status_known(device.index()) && watch.same();
     }
     Tensor finish(const Tensor& pooled) const { return at::linear(pooled, head_w, head_b.defined() ? OptT(head_b) : std::nullopt); }
     // One forward.  ``work``: a measure of the activations (tokens x channels).  Launched one by one, a forward of 50 to 150
