@@ -27,3 +27,9 @@ def test_many_small_images_at_once():
         for _ in range(3):
             # one rounding of the mean (bf16: 8 significant bits, 2^-8 at most) and the order of fp32 sums; a lost part: L / S of L
             assert float((ops.token_mean(x).float() - ref).abs().max()) <= 2 ** -8 * float(ref.abs().max()) + 1e-6
+
+
+def test_more_images_than_a_launch_takes():
+    from vig_b200 import ops
+    x = torch.randn(65535 * 2 + 3, 2, 32, generator=torch.Generator(device="cuda").manual_seed(4), device="cuda").half()
+    assert float((ops.token_mean(x).double() - x.double().mean(1)).abs().max()) <= 2.0 ** -11 * float(x.abs().max())

@@ -767,7 +767,7 @@ int add_layernorm_t(const void* x, const void* pb, const void* res, const void* 
 
 template <typename T>
 int token_mean_t(const void* x, void* y, int B, int L, int C, cudaStream_t s) {
-    if (C % DType<T>::VEC || B > 65535) return VIG_ERR_SHAPE;
+    if (C % DType<T>::VEC) return VIG_ERR_SHAPE;
     int S = (L + 127) / 128;                                 // 128 tokens and more a CTA
     S = S >= 8 ? 8 : S >= 4 ? 4 : S >= 2 ? 2 : 1;
     cudaLaunchConfig_t cfg{};
@@ -779,8 +779,12 @@ int token_mean_t(const void* x, void* y, int B, int L, int C, cudaStream_t s) {
     attr[0].val.clusterDim.x = S; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, token_mean_kernel<T>, (const T*)x, (T*)y, L, C);
-    return (int)(e != cudaSuccess ? e : cudaGetLastError());
+    for (int64_t b0 = 0; b0 < B; b0 += 65535) {              // images a launch: the grid's third dimension
+        cfg.gridDim.z = (unsigned)(B - b0 < 65535 ? B - b0 : 65535);
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, token_mean_kernel<T>, (const T*)x + b0 * L * C, (T*)y + b0 * C, L, C);
+        if (e != cudaSuccess) return (int)e;
+    }
+    return (int)cudaGetLastError();
 }
 
 template <typename T>
