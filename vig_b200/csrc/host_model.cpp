@@ -73,13 +73,18 @@ std::pair<Tensor, Tensor> linear_add_rmsnorm(const Ctx& c, const Tensor& x, cons
 
 // ---- the attention module ------------------------------------------------------------------------------------------
 struct Attn {
-    Tensor taps, conv_b, w_z, b_z, gn_w, ln_w, o_w;
+    // taps, w_z, b_z: derived weights, made by ``pack`` when the first forward gets here, so that the GPU works on the blocks
+    // before meanwhile (all of them ahead of the first launch: 64 images of 1024 x 1024 waited 1.5 of 14 ms)
+    mutable Tensor taps, w_z, b_z;
+    mutable py::object pack;
+    Tensor conv_b, gn_w, ln_w, o_w;
     int64_t H, dk, dv;
     bool act_conv, out_act;
     double eps, out_scale, norm, clamp;
 
     struct Scanned { Tensor o, xs, z; };                     // scan output [B,L,H,dv], conv output, stacked projection
     Scanned scan(const Ctx& c, const Tensor& x, int64_t h, int64_t w) const {
+        if (!w_z.defined()) std::tie(taps, w_z, b_z) = pack().cast<std::tuple<Tensor, Tensor, Tensor>>();
         const int64_t B = x.size(0), L = x.size(1), kd = H * dk, vd = H * dv;
         const Tensor xs = dwconv(c, x, taps, conv_b, h, w, act_conv);
         const Tensor z = at::linear(xs, w_z, b_z);
@@ -524,7 +529,7 @@ struct HierPlan : PlanBase {
 Tensor tensor_of(const py::dict& d, const char* key) { return d.contains(key) && !d[key].is_none() ? d[key].cast<Tensor>() : Tensor(); }
 Attn attn_of(const py::dict& d) {
     Attn a;
-    a.taps = tensor_of(d, "taps"); a.conv_b = tensor_of(d, "conv_b"); a.w_z = tensor_of(d, "w_z"); a.b_z = tensor_of(d, "b_z");
+    a.pack = d["pack"]; a.conv_b = tensor_of(d, "conv_b");
     a.gn_w = tensor_of(d, "gn_w"); a.ln_w = tensor_of(d, "ln_w"); a.o_w = tensor_of(d, "o_w");
     a.H = d["H"].cast<int64_t>(); a.dk = d["dk"].cast<int64_t>(); a.dv = d["dv"].cast<int64_t>();
     a.act_conv = d["act_conv"].cast<bool>(); a.out_act = d["out_act"].cast<bool>();

@@ -51,8 +51,7 @@ def _conv(m, weight=None, stride=None, pad=None):
 def _attn(a):
     if not a.fold_gate_bottleneck or a.own_in_proj_gemm or a.o_proj.bias is not None:
         return None
-    taps, w_z, b_z = a._pack(True)
-    return dict(taps=taps, conv_b=a.in_proj[0].bias, w_z=w_z, b_z=b_z, gn_w=a.g_norm.weight, ln_w=a.l_norm.weight, o_w=a.o_proj.weight,
+    return dict(pack=lambda: a._pack(True), conv_b=a.in_proj[0].bias, gn_w=a.g_norm.weight, ln_w=a.l_norm.weight, o_w=a.o_proj.weight,
                 H=a.num_heads, dk=a.head_qk_dim, dv=a.head_v_dim, act_conv=bool(a.use_act_in_conv), out_act=bool(a.use_out_act), eps=a.g_norm.eps,
                 out_scale=a.out_scale, norm=float(a.gate_logit_normalizer), clamp=math.nan if a.clamp_min is None else float(a.clamp_min))
 
