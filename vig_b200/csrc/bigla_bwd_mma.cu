@@ -466,7 +466,7 @@ int launch_typed(const BwdParams& p, cudaStream_t stream) {
     if (p.nchunk > 1) {                                                  // one chunk: both entering states are zero
         if ((e = tc::ensure_smem_attr(reinterpret_cast<const void*>(kA), (int)smA)) != cudaSuccess) return (int)e;
         // few chunks: one CTA per direction, so that more of the GPU works; many: one CTA reads v and d_out once for both
-        const int gz = p.dir_mask == 3 && (int64_t)p.nchunk * BH < 148 * 4 ? 2 : 1;
+        const int gz = p.dir_mask == 3 && (int64_t)p.nchunk * BH < device_sms() * 4 ? 2 : 1;
         kA<<<dim3(p.nchunk, BH, gz), NT, smA, stream>>>(p);
         if (int s = bigla_bwd_scan_launch(p, stream)) return s;
     }

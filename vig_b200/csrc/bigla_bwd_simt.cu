@@ -289,13 +289,12 @@ int launch_typed(const BwdParams& p, int flagged_only, cudaStream_t stream) {
     int ctas = items;
     if (flagged_only) {
         static std::atomic<int> per_sm{0};                               // a property of the kernel, the same on every B200
-        int fit = per_sm.load(), dev = 0, sms = 0;
+        int fit = per_sm.load();
         if (!fit) {
             if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kC, NT, smC)) != cudaSuccess) return (int)e;
             per_sm.store(fit = fit < 1 ? 1 : fit);
         }
-        if ((e = cudaGetDevice(&dev)) != cudaSuccess || (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return (int)e;
-        ctas = items < fit * sms ? items : fit * sms;
+        ctas = items < fit * device_sms() ? items : fit * device_sms();
     }
     return (int)launch_next(kC, dim3(ctas), dim3(NT), smC, stream, p, flagged_only);
 }

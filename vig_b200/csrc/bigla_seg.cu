@@ -730,7 +730,7 @@ int bigla_seg_launch(const BiglaParams& p, cudaStream_t stream) {
     s.p = p;
     // 64-token segments where more SMs can share the work of few sequences (1x3x196 dk = 64: 11 us against 13) and for dv = 32,
     // whose segments are too little work for eight warps (64x12x196 dk = 16: 47 us against 57); otherwise 128, half as many states
-    const int tok = p.dv == 32 || p.L <= 64 || (p.L <= 512 && (int64_t)p.B * p.H * ((p.L + 63) / 64) <= 148) ? 64 : 128;
+    const int tok = p.dv == 32 || p.L <= 64 || (p.L <= 512 && (int64_t)p.B * p.H * ((p.L + 63) / 64) <= device_sms()) ? 64 : 128;
     switch (p.dtype) {
         case VIG_DTYPE_F32: return seg_launch_dims<float>(s, 64, stream);
         case VIG_DTYPE_BF16: return seg_launch_dims<__nv_bfloat16>(s, tok, stream);

@@ -311,8 +311,8 @@ template <typename T, int RB, int WR> int bt_launch(const BtMaps& maps, const Bt
 
 template <typename T> int bt_dispatch(const BtMaps& maps, const BtParams& p, cudaStream_t st) {
     // the smallest row tile that is one wave of CTAs; beyond that the largest
-    if (p.M <= 148 * 16) return bt_launch<T, 1, 1>(maps, p, st);
-    if (p.M <= 148 * 32) return bt_launch<T, 2, 1>(maps, p, st);
+    if (p.M <= device_sms() * 16) return bt_launch<T, 1, 1>(maps, p, st);
+    if (p.M <= device_sms() * 32) return bt_launch<T, 2, 1>(maps, p, st);
     return bt_launch<T, 4, 2>(maps, p, st);
 }
 
@@ -329,7 +329,7 @@ extern "C" int vig_block_tail_supported(int64_t M, int H, int dv, int I, int dty
 
 // One wave of 64-token tiles; beyond it the tcgen05 kernels win (12544 tokens: 48 us here, 42 as four kernels; 8192: 26, 36).
 extern "C" int vig_block_tail_preferred(int64_t M, int H, int dv, int I, int dtype) {
-    return vig_block_tail_supported(M, H, dv, I, dtype) && M <= 148 * 64;
+    return vig_block_tail_supported(M, H, dv, I, dtype) && M <= (int64_t)device_sms() * 64;
 }
 
 extern "C" int vig_block_tail_fwd(const void* o, const void* local, const void* gate_logits, int64_t ld_gate, const void* w_gnorm, const void* w_lnorm,

@@ -4,6 +4,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <stdint.h>
+#include <atomic>
 #include "../../include/vig_b200.h"
 
 namespace vig {
@@ -95,6 +96,19 @@ __device__ __forceinline__ float4 scan_states(float4* ws, const float* decay, in
         run(c0 + PF, 1);
     }
     return S;
+}
+
+// SMs of the current device (1 where there is none to ask)
+inline int device_sms() {
+    static std::atomic<int> known[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
+    int n = known[dev].load(std::memory_order_relaxed);
+    if (!n) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) return 1;
+        known[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
 }
 
 // GELU in its erf form.  16-bit results: erf by Abramowitz & Stegun 7.1.26 (|error| <= 1.5e-7), one exponential and one

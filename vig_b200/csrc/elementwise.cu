@@ -669,7 +669,7 @@ __global__ void __launch_bounds__(EW_THREADS) stem_unfold_kernel(const T* __rest
 
 inline int grid_for(int64_t items, int per_block) {
     int64_t g = (items + per_block - 1) / per_block;
-    const int64_t cap = 148 * 16;       // 148 SMs x resident CTAs; the kernels are grid-stride
+    const int64_t cap = device_sms() * 16;   // SMs x resident CTAs; the kernels are grid-stride
     return (int)(g < 1 ? 1 : (g > cap ? cap : g));
 }
 
@@ -691,7 +691,7 @@ int dwconv_t(const void* x, const void* wt, const void* bias, void* y, int B, in
             return threads >= (1ll << 31) ? -1 : (int)launch_chained(kern, dim3((unsigned)((threads + EW_THREADS - 1) / EW_THREADS)), dim3(EW_THREADS), 0, s,
                 (const T*)x, (const T*)wt, (const T*)bias, (T*)y, B, h, w, C, act, (const T*)top, (const T*)bottom);
         };
-        const bool small = (int64_t)B * h * ((w + 15) / 16) * (C / 4) < 148 * 512;
+        const bool small = (int64_t)B * h * ((w + 15) / 16) * (C / 4) < device_sms() * 512;
         const int r = small ? launch(dwconv3x3_rows_kernel<T, 4>, 4) : launch(dwconv3x3_rows_kernel<T, 16>, 16);
         if (r >= 0) return r;
         if (top || bottom) return VIG_ERR_SHAPE;

@@ -125,7 +125,8 @@ template <typename T> int launch(const void* x, const void* w, const void* cb, c
                                  cudaStream_t s) {
     const int OH = (H + 1) / 2, OW = (W + 1) / 2;
     const int64_t pixels = (int64_t)B * OH * OW, blocks = (pixels + 127) / 128;
-    const int grid = (int)(blocks < 148 * 8 ? blocks : 148 * 8);
+    const int64_t most = device_sms() * 8;
+    const int grid = (int)(blocks < most ? blocks : most);
 #define VIG_EC(OO) case OO: embed_conv_kernel<T, OO><<<grid, 256, 0, s>>>((const T*)x, (const T*)w, (const T*)cb, (const T*)lw, (const T*)lb, (T*)y, pixels, H, W, OH, OW, eps, gelu); break;
     switch (O) { VIG_EC(32) VIG_EC(48) VIG_EC(64) default: return VIG_ERR_SHAPE; }
 #undef VIG_EC
