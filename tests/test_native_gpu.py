@@ -324,3 +324,36 @@ def test_dispatch_modes_see_the_forward():
         with Count() as c:
             y = m(x)
         assert c.seen >= 4 and torch.equal(y, ref) and torch.equal(m(x), ref)
+
+
+@pytest.mark.parametrize("kind", ["vig_t", "hier"])
+def test_changes_give_what_a_fresh_model_gives(kind):
+    """After each kind of change -- a weight in place, a replaced parameter, an attribute, another precision -- the plan's logits
+    are those of a model that was made with it."""
+    m = _model(kind, torch.bfloat16 if kind == "vig_t" else torch.float16)
+    x = torch.randn(2, 3, 64, 96, device="cuda").to(next(m.parameters()).dtype)
+    attn = (lambda n: n.blocks[0].attn) if kind == "vig_t" else (lambda n: n.layers[1].blocks[0].op)
+
+    def check():
+        fresh = _model(kind, next(m.parameters()).dtype)
+        fresh.load_state_dict(m.state_dict())
+        attn(fresh).out_scale = attn(m).out_scale
+        got = [m(x) for _ in range(3)]
+        want = fresh(x)
+        assert all(torch.equal(g, want) for g in got)
+        return want
+
+    with torch.no_grad():
+        outs = [check()]
+        attn(m).qkv_proj.weight.mul_(1.5)
+        outs.append(check())
+        attn(m).gk_proj[1].weight = nn.Parameter(attn(m).gk_proj[1].weight * -2, requires_grad=False)
+        outs.append(check())
+        attn(m).in_proj[0].weight.add_(0.1)
+        outs.append(check())
+        attn(m).out_scale = 0.25
+        outs.append(check())
+        m.half() if kind == "vig_t" else m.bfloat16()
+        x = x.to(next(m.parameters()).dtype)
+        outs.append(check())
+    assert all(not torch.equal(a.float(), b.float()) for a, b in zip(outs, outs[1:]))

@@ -34,7 +34,7 @@ template <int DK, int DV, typename T> struct SegTerms {
 };
 
 // Warps that share 16 rows, each with its part of the value columns (the scores are formed by each of them): two for fp32, whose
-// three-term tiles leave room for one or two 64-token segments an SM (2x3x196 64/64: 28.4 -> 20.0 us; 16x6x1000 64/64: 520 ->
+// three-term tiles leave room for one or two 64-token segments an SM (2x3x196 64/64: 28.4 -> 19.5 us; 16x6x1000 64/64: 520 ->
 // 320).  16-bit inputs have two or three segments an SM and gain nothing from repeating the scores.
 template <typename T> struct SegWarps { static constexpr int CW = sizeof(T) == 4 ? 2 : 1; };
 

@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_c
         // token 8*warp + (sp ^ dmask): the same code serves both directions.  Gate form (raw logits or log-gates) and the
         // lower clamp are template parameters: the token loops carry no branch, so their 16 elements overlap.
         // dk = 32: the rows are half as long, so a quarter-warp takes 2 consecutive scan positions and nobody works on the
-        // zero channels (96 sequences of 3136 tokens 124 -> 111 us); quarters lie so that the two of a half-warp read rows
+        // zero channels (96 sequences of 3136 tokens 124 -> 113 us); quarters lie so that the two of a half-warp read rows
         // whose swizzled chunks fall into different halves of the banks.
         constexpr int NTK = D32 ? 2 : 4, NPART = D32 ? 4 : 2;    // tokens of a lane; parts of a warp, in scan order
         const int grp = warp;

@@ -9,7 +9,7 @@
 // is exactly the conv's zero padding, so the kernel has no border cases.  A compute thread owns 4 channels and a run of
 // 8 columns: 36 taps live in registers as fp32, the 4-row window slides along the run and yields the outputs of both
 // image rows per step (4 shared-memory loads and 36 two-wide fp32 FMAs per 8 outputs).  Narrow images take several row pairs a
-// tile, so that no thread idles (128 x 14 x 14 x 384: 24 us with one pair, 15 with four).  Two channels and twice the threads
+// tile, so that no thread idles (128 x 14 x 14 x 384: 24 us with one pair, 14 with four).  Two channels and twice the threads
 // were slower on wide images (57 us against 50 at 64 x 64 x 64 x 192: twice the loads and stores).  Arithmetic (fp32, tap order, SiLU) is
 // that of the sliding-window kernel, so the two forms agree bit for bit.
 #include <type_traits>

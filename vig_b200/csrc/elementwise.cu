@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(EW_THREADS) add_rmsnorm_kernel(const T* __rest
     const int nv = N / V;
     const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    // wide rows: the warp's next row is in flight during this one's arithmetic (131072 x 768 with a residual 162 -> 142 us; at one
+    // wide rows: the warp's next row is in flight during this one's arithmetic (131072 x 768 with a residual 162 -> 143 us; at one
     // vector a lane the extra registers cost more than it gives)
     constexpr bool AHEAD = MAXV > 1;
     Vec16<T> xn[MAXV], rn[MAXV];
