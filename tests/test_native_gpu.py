@@ -344,6 +344,9 @@ def test_changes_give_what_a_fresh_model_gives(kind):
         return want
 
     with torch.no_grad():
+        for p in m.parameters():                                         # weights at which every one of these changes shows in 16 bits
+            if p.dim() > 1:
+                p.normal_(0, p[0].numel() ** -0.5)
         outs = [check()]
         attn(m).qkv_proj.weight.mul_(1.5)
         outs.append(check())
