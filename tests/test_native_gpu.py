@@ -337,7 +337,7 @@ def test_changes_give_what_a_fresh_model_gives(kind):
     def check():
         fresh = _model(kind, next(m.parameters()).dtype)
         fresh.load_state_dict(m.state_dict())
-        attn(fresh).out_scale = attn(m).out_scale
+        attn(fresh).use_out_act = attn(m).use_out_act
         got = [m(x) for _ in range(3)]
         want = fresh(x)
         assert all(torch.equal(g, want) for g in got)
@@ -354,7 +354,7 @@ def test_changes_give_what_a_fresh_model_gives(kind):
         outs.append(check())
         attn(m).in_proj[0].weight.add_(0.1)
         outs.append(check())
-        attn(m).out_scale = 0.25
+        attn(m).use_out_act = not attn(m).use_out_act
         outs.append(check())
         m.half() if kind == "vig_t" else m.bfloat16()
         x = x.to(next(m.parameters()).dtype)
