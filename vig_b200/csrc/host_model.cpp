@@ -3,7 +3,7 @@
 // kernels' time for one 224 x 224 image.
 //
 // A Plan is built by the Python layer (vig_b200/native.py) from a model's modules and stays valid while nothing it was built
-// from changes: it watches every parameter (identity, version, storage, type), every module's children, hooks, plain
+// from changes: it watches every parameter (identity, version, address, type, strides), every module's children, hooks, plain
 // attributes and overridden forwards, and answers None as soon as one differs, so that the caller rebuilds it or runs the
 // modules themselves.  The check is some hundred pointer comparisons.
 #include "host.h"
