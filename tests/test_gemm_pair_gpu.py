@@ -1,0 +1,40 @@
+"""Products on pairs of CTAs (tcgen05, cta_group::2) against fp64: rows around the 128 of a CTA and the 256 of a pair, features that do not
+fill the last tile of 128, one and many k boxes, W streamed (K = 448 and up, few row tiles) and kept for the launch, leading dimensions."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+# one rounding of the result (2^-9, 2^-12, uniform: over sqrt(3)) and, for SwiGLU, the sigmoid through tanh.approx (2^-11)
+TOL = {torch.bfloat16: 2.5e-3, torch.float16: 6e-4}
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,K,I", [(1, 64, 64), (127, 192, 512), (129, 384, 192), (255, 448, 128), (257, 768, 320), (1000, 1024, 2816), (9473, 384, 1024),
+                                   (19200, 320, 1024), (20001, 64, 128), (37500, 192, 320)])
+def test_swiglu(dtype, M, K, I):
+    import vig_b200
+    g = torch.Generator(device="cuda").manual_seed(M + K + I)
+    x = torch.randn(M, 2 * K, generator=g, device="cuda").to(dtype)[:, :K]          # rows of a wider matrix
+    w = (torch.randn(2 * I, K, generator=g, device="cuda") / K ** 0.5).to(dtype)
+    out = torch.full((M, I + 8), 7.0, device="cuda", dtype=dtype)
+    lib, ptr = vig_b200._lib.lib(), vig_b200._lib.ptr
+    assert lib.vig_linear_swiglu_supported(M, K, I, vig_b200._lib.dtype_code(x))
+    assert lib.vig_linear_swiglu_fwd(ptr(x), 2 * K, ptr(w), ptr(out), I + 8, M, K, I, vig_b200._lib.dtype_code(x), None, vig_b200._lib.stream_ptr()) == 0
+    rows = torch.cat([torch.arange(min(M, 3000)), torch.arange(max(0, M - 3000), M)]).cuda()
+    a, b = (x[rows].double() @ w.double().t()).chunk(2, -1)
+    ref = a * torch.sigmoid(a) * b
+    assert float((out[rows, :I].double() - ref).norm() / ref.norm()) < TOL[dtype]
+    assert torch.equal(out[:, I:], torch.full_like(out[:, I:], 7.0))                # nothing past the last feature
+
+
+def test_a_hooked_projection_runs_by_itself():
+    """A hook on the gate projection sees its output also where the fused kernel would take its place."""
+    import vig_b200
+    mlp = vig_b200.modules.GLAMLP(384).cuda().bfloat16()
+    x = torch.randn(1, 4096, 384, device="cuda", dtype=torch.bfloat16)
+    with torch.no_grad():
+        fused, seen = mlp(x), []
+        mlp.gate_proj.register_forward_hook(lambda m, i, o: seen.append(o))
+        hooked = mlp(x)
+    assert len(seen) == 1 and seen[0].shape[-1] == 2 * mlp.intermediate_size
+    assert float((fused.float() - hooked.float()).norm() / hooked.float().norm()) < 1e-2

@@ -126,6 +126,13 @@ class GatedLinearAttention(nn.Module):
         return self.o_proj(y)
 
 
+def plain_linear(m):
+    """Whether calling ``m`` is the product with its weight and nothing else, so that a fused kernel may take its place."""
+    g = nn.modules.module
+    return (type(m) is nn.Linear and m.bias is None and "forward" not in m.__dict__ and
+            not (m._forward_hooks or m._forward_pre_hooks or g._global_forward_hooks or g._global_forward_pre_hooks))
+
+
 class GLAMLP(nn.Module):
     def __init__(self, hidden_size, hidden_ratio: Optional[int] = None, intermediate_size: Optional[int] = None,
                  hidden_act="swish"):
@@ -140,7 +147,7 @@ class GLAMLP(nn.Module):
         self.down_proj = nn.Linear(intermediate_size, hidden_size, bias=False)
 
     def forward(self, x):
-        if ops.linear_swiglu_supported(x, self.gate_proj.weight, preferred=True):
+        if plain_linear(self.gate_proj) and ops.linear_swiglu_supported(x, self.gate_proj.weight, preferred=True):
             # gate projection and SwiGLU in one tensor-core kernel: the [.., 2I] intermediate never reaches HBM
             return F.linear(ops.linear_swiglu(x, self.gate_proj.weight), self.down_proj.weight, self.down_proj.bias)
         y = self.gate_proj(x)
@@ -184,7 +191,7 @@ class GLABlock(nn.Module):
         y = self.attn(h, skip_o_proj=True, **kwargs)
         h2, residual = ops.linear_add_rmsnorm(y, self.attn.o_proj.weight, residual, self.mlp_norm.weight, self.mlp_norm.eps)
         m = self.mlp
-        if ops.linear_swiglu_supported(h2, m.gate_proj.weight, preferred=True):
+        if plain_linear(m.gate_proj) and ops.linear_swiglu_supported(h2, m.gate_proj.weight, preferred=True):
             z = ops.linear_swiglu(h2, m.gate_proj.weight)
         else:
             gate, yy = m.gate_proj(h2).chunk(2, -1)

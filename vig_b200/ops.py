@@ -576,8 +576,8 @@ def block_tail(o, local, gate_logits, w_gnorm, w_lnorm, w_o, residual, norm_w, w
 
 
 def linear_swiglu_supported(x, weight, preferred=False):
-    """True when ``linear_swiglu`` has a fused kernel for this input (bf16 / fp16, K % 64 == 0, K <= 384, I % 64 == 0);
-    with ``preferred`` also that it beats the library GEMM followed by the SwiGLU kernel (K <= 192)."""
+    """True when ``linear_swiglu`` has a fused kernel for this input (bf16 / fp16, K % 64 == 0, I % 64 == 0); with
+    ``preferred`` also that it is taken instead of the library GEMM followed by the SwiGLU kernel (K <= 192, or rows enough)."""
     if not x.is_cuda or x.dtype not in (torch.bfloat16, torch.float16) or weight.dtype != x.dtype:
         return False
     K, I = x.shape[-1], weight.shape[0] // 2
