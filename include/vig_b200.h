@@ -329,9 +329,10 @@ VIG_API int vig_stem_conv_ln_fwd(const void* cells, const void* w2, const void* 
  * 497, 596-606; fla/modules/rmsnorm.py:491-512).  One tcgen05 GEMM kernel; the projection output is not written.
  * Same roundings as the unfused sequence (projection rounded to the tensor dtype, sum rounded to the tensor dtype).
  * x: [M, K] with row stride ldx; w: [N, K] contiguous; residual, out_r, out_h: [M, N] contiguous; K % 64 == 0,
- * N one of 64, 128, 192, 256, 384.  status_dev: optional int32 on the device, bit 0 = a bounded wait ran out.
+ * N one of 64, 128, 192, 256, 384, 768.  status_dev: optional int32 on the device, bit 0 = a bounded wait ran out.
  */
 VIG_API int vig_linear_add_rmsnorm_supported(int64_t M, int K, int N, int dtype);
+VIG_API int vig_linear_add_rmsnorm_preferred(int64_t M, int K, int N, int dtype);   /* supported AND to be taken instead of GEMM + norm */
 VIG_API int vig_linear_add_rmsnorm_fwd(const void* x, int64_t ldx, const void* w, const void* residual, const void* norm_weight,
                                        void* out_r, void* out_h, int64_t M, int K, int N, float eps, int dtype,
                                        int32_t* status_dev, void* stream);

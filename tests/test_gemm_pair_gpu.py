@@ -38,3 +38,41 @@ def test_a_hooked_projection_runs_by_itself():
         hooked = mlp(x)
     assert len(seen) == 1 and seen[0].shape[-1] == 2 * mlp.intermediate_size
     assert float((fused.float() - hooked.float()).norm() / hooked.float().norm()) < 1e-2
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,K,N,with_res", [(1, 64, 256, True), (129, 704, 256, False), (257, 384, 384, True), (19201, 128, 384, True), (300, 2048, 768, True),
+                                            (9473, 192, 768, True), (20000, 320, 768, False)])
+def test_projection_add_norm(dtype, M, K, N, with_res):
+    """Rows of 256, 384 and 768 (two pairs a row): the sum against fp64 with the projection rounded as the separate kernels round it, the
+    norm against fp64 of the sum that was returned; one and several tiles a cluster, ragged rows."""
+    import vig_b200
+    g = torch.Generator(device="cuda").manual_seed(M + K + N)
+    x = torch.randn(M, K, generator=g, device="cuda").to(dtype)
+    w = (torch.randn(N, K, generator=g, device="cuda") / K ** 0.5).to(dtype)
+    res = torch.randn(M, N, generator=g, device="cuda").to(dtype) if with_res else None
+    nw = (1 + 0.1 * torch.randn(N, generator=g, device="cuda")).to(dtype)
+    h, r = vig_b200.ops.linear_add_rmsnorm(x, w, res, nw, 1e-6)
+    vig_b200.check_status()
+    ref = x.double() @ w.double().t()
+    if with_res:
+        ref = ref + res.double()
+    rd = r.double()
+    norm = rd * torch.rsqrt((rd * rd).mean(-1, keepdim=True) + 1e-6) * nw.double()
+    # the sum: two roundings, of values of up to its own size; the norm: one
+    assert float((rd - ref).norm() / ref.norm()) < 2 * TOL[dtype]
+    assert float((h.double() - norm).norm() / norm.norm()) < TOL[dtype]
+
+
+def test_a_hooked_norm_runs_by_itself():
+    """Hooks on a wide block's projections and norms see their calls also where one kernel would take their place."""
+    import vig_b200
+    model = vig_b200.build_vig("vig_s", num_classes=10).cuda().bfloat16().eval()
+    x = torch.randn(2, 3, 64, 64, device="cuda").bfloat16()
+    with torch.no_grad():
+        ref, seen = model(x), []
+        model.blocks[0].mlp_norm.register_forward_hook(lambda m, i, o: seen.append("norm"))
+        model.blocks[1].attn.o_proj.register_forward_hook(lambda m, i, o: seen.append("proj"))
+        got = model(x)
+    assert seen == ["norm", "proj"]
+    assert float((ref.float() - got.float()).norm() / ref.float().norm()) < 2e-2

@@ -40,6 +40,7 @@ _SIGNATURES = {
     "vig_linear_swiglu_preferred": (c_int, [c_int64, c_int, c_int, c_int]),
     "vig_linear_swiglu_fwd": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_int64, c_int, c_int, c_int, c_void_p, c_void_p]),
     "vig_linear_add_rmsnorm_supported": (c_int, [c_int64, c_int, c_int, c_int]),
+    "vig_linear_add_rmsnorm_preferred": (c_int, [c_int64, c_int, c_int, c_int]),
     "vig_linear_add_rmsnorm_fwd": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_float, c_int, c_void_p, c_void_p]),
     "vig_layernorm_act_add_fwd": (c_int, [c_void_p] * 5 + [c_int64, c_void_p, c_int64, c_int, c_float, c_int, c_int, c_void_p]),
     "vig_layernorm_act_add_rmsnorm_fwd": (c_int, [c_void_p] * 5 + [c_int64, c_void_p, c_void_p, c_float, c_void_p, c_int64, c_int, c_float, c_int, c_int, c_void_p]),

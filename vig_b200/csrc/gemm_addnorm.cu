@@ -4,18 +4,20 @@
 // prenorm).  The projection output never goes to HBM: instead of (GEMM: write y) + (norm: read y, read residual,
 // write r, write h) the kernel reads the residual and writes r and h.
 //
+// Here: rows of up to 192 values, on single CTAs; longer ones in gemm_pair_norm.cu.
+//
 // tcgen05 GEMM with full output rows per tile.  A persistent CTA owns tiles of 128 rows; x and W stream through a ring
 // of stages [128 x 64 of x | N x 64 of W] (TMA, 128-byte swizzle); the accumulator [128 x N] fp32 lives in tensor
-// memory (N <= 384 columns; two buffers when 2N <= 512, so the epilogue of a tile overlaps the MMAs of the next).
+// memory (two buffers: the epilogue of a tile overlaps the MMAs of the next).
 // Roles: warp 0 TMA producer, warp 1 MMA issuer, warps 2..9 epilogue.  Every wait is bounded.
-// Epilogue for rows of up to 192 values: the tile's residual rows arrive by TMA in 128-byte-swizzled boxes (two tile
+// Epilogue: the tile's residual rows arrive by TMA in 128-byte-swizzled boxes (two tile
 // buffers); a thread owns half a row (its TMEM lane, two warps per lane quadrant): pass 1 adds the residual with the
 // roundings of the unfused path (projection rounded to T, sum rounded to T), writes r in place and keeps it in
 // registers, the halves' sums of squares meet in shared memory; a TMA store sends r out; pass 2 writes h over the same
 // boxes once that store has read them and a second TMA store sends h out.  (Per-thread row stores, the first version,
-// cost 32 sectors per request and made the kernel slower than the pair it replaces.)  Wider rows still use per-thread
-// loads and stores.
+// cost 32 sectors per request and made the kernel slower than the two it replaces.)
 #include "tc_common.cuh"
+#include "gemm_pair.h"
 
 namespace vig {
 namespace {
@@ -41,12 +43,9 @@ __global__ void __launch_bounds__(AN_THREADS, 1) linear_add_rmsnorm_kernel(const
     constexpr int N = NT;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t stage_bytes = AN_A_BYTES + (uint32_t)N * AN_BK * 2;
-    // rows of up to 192 values leave through shared memory and TMA stores (coalesced by the hardware); wider rows use
-    // per-thread row stores
-    constexpr bool TMA_EPI = NT <= 192;
     constexpr uint32_t E_BYTES = (uint32_t)(NT / 64) * 128 * 128;      // one [128 x N] tile as N/64 swizzled boxes
     const uint32_t off_e = (uint32_t)nstage * stage_bytes;
-    const uint32_t off_bar = off_e + (TMA_EPI ? 2 * E_BYTES : 0);
+    const uint32_t off_bar = off_e + 2 * E_BYTES;
     const uint32_t bar_full = sbase + off_bar, bar_empty = bar_full + 8 * 8;          // up to 8 stages
     const uint32_t bar_acc_full = bar_empty + 8 * 8, bar_acc_empty = bar_acc_full + 16;
     const uint32_t bar_res_full = bar_acc_empty + 16, bar_e_free = bar_res_full + 16;
@@ -60,7 +59,7 @@ __global__ void __launch_bounds__(AN_THREADS, 1) linear_add_rmsnorm_kernel(const
     if (tid == 0) {
         for (int s = 0; s < nstage; ++s) { mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, 1); }
         for (int b = 0; b < 2; ++b) {
-            mbar_init(bar_acc_full + 8 * b, 1); mbar_init(bar_acc_empty + 8 * b, TMA_EPI ? 256 : 128);
+            mbar_init(bar_acc_full + 8 * b, 1); mbar_init(bar_acc_empty + 8 * b, 256);
             mbar_init(bar_res_full + 8 * b, 1); mbar_init(bar_e_free + 8 * b, 1);
         }
         *abort_flag = 0;
@@ -80,7 +79,7 @@ __global__ void __launch_bounds__(AN_THREADS, 1) linear_add_rmsnorm_kernel(const
         if (lane == 0) {                          // ---- TMA producer -------------------------------------------
             uint32_t st = 0, phase = 0, t_it = 0;
             for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++t_it) {
-                if (TMA_EPI) {                        // the tile's residual rows, into the epilogue buffer of this tile
+                {                                     // the tile's residual rows, into the epilogue buffer of this tile
                     const uint32_t eb = t_it & 1u;
                     waiter.wait(bar_e_free + 8 * eb, ((t_it >> 1) & 1u) ^ 1u);
                     if (*abort_flag) break;
@@ -139,7 +138,7 @@ __global__ void __launch_bounds__(AN_THREADS, 1) linear_add_rmsnorm_kernel(const
                 __syncwarp();
             }
         }
-    } else if (TMA_EPI) {                         // ---- epilogue through shared memory and TMA stores ----------------
+    } else {                                      // ---- epilogue through shared memory and TMA stores ----------------
         // One thread per row (its TMEM lane).  The residual tile arrives by TMA in 128-byte-swizzled boxes; pass 1 turns
         // it into r in place (and keeps r in registers), a TMA store sends it out; pass 2 writes h over the same boxes
         // once that store has read them, and a second TMA store sends h out.
@@ -224,68 +223,6 @@ __global__ void __launch_bounds__(AN_THREADS, 1) linear_add_rmsnorm_kernel(const
             }
         }
         if (leader) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // all stores have landed before the CTA exits
-    } else if (warp < 6) {                        // ---- epilogue for wide rows: one thread per row, per-thread stores ----
-        // The thread's residual row is requested before the tile's accumulator is waited for (its latency hides behind
-        // the MMAs), the sums r replace it in the same registers, and pass 2 works from registers: no dependent global
-        // round trips inside the loops.  (192 threads per CTA: registers are plentiful.)
-        constexpr int NV = NT / 8;                // 16-byte vectors per row
-        const uint32_t lane_base = (uint32_t)(32 * (warp & 3)) << 16;
-        const int r_in_tile = 32 * (warp & 3) + lane;
-        uint32_t acc_it = 0;
-        for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++acc_it) {
-            const uint32_t buf = nbuf == 2 ? (acc_it & 1u) : 0u;
-            const uint32_t use = nbuf == 2 ? (acc_it >> 1) : acc_it;
-            const int64_t row = (int64_t)tile * 128 + r_in_tile;
-            const bool live = row < M;
-            uint4 rr[NV];
-#pragma unroll
-            for (int v = 0; v < NV; ++v) rr[v] = (live && residual) ? __ldg(reinterpret_cast<const uint4*>(residual + row * NT) + v) : make_uint4(0u, 0u, 0u, 0u);
-            waiter.wait(bar_acc_full + 8 * buf, use & 1u);     // by the whole warp: a wait by one lane with the others parked at a warp barrier resumes microseconds late
-            __syncwarp();
-            if (*abort_flag) break;
-            tc_fence_after();
-            const uint32_t acc = tmem + lane_base + buf * (uint32_t)NT;
-            float ss = 0.f;
-#pragma unroll
-            for (int c = 0; c < NT; c += 32) {    // pass 1: r = T(T(acc) + residual), sum of squares
-                float a[32];
-                tc_ld32(acc + c, a);
-                tc_wait_ld();
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    uint4& rv = rr[c / 8 + j];
-                    uint32_t* rw = reinterpret_cast<uint32_t*>(&rv);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        // the unfused path rounds the projection to T before the add, and the sum to T before the norm
-                        const float2 y = Pack2<T>::unpack(Pack2<T>::pack(a[8 * j + 2 * e], a[8 * j + 2 * e + 1]));
-                        const float2 rf = Pack2<T>::unpack(rw[e]);
-                        rw[e] = Pack2<T>::pack(y.x + rf.x, y.y + rf.y);       // residual words are zero when there is none
-                        const float2 s2 = Pack2<T>::unpack(rw[e]);
-                        ss = fmaf(s2.x, s2.x, ss); ss = fmaf(s2.y, s2.y, ss);
-                    }
-                    if (live) reinterpret_cast<uint4*>(out_r + row * NT + c)[j] = rv;
-                }
-            }
-            tc_fence_before();
-            mbar_arrive_plain(bar_acc_empty + 8 * buf);       // the accumulator is read: pass 2 works from registers
-            if (live) {
-                const float rstd = rsqrtf(ss / (float)NT + eps);
-#pragma unroll
-                for (int v = 0; v < NV; ++v) {    // pass 2: h = r * rstd * norm_weight
-                    const uint4 wv = __ldg(reinterpret_cast<const uint4*>(norm_w) + v);
-                    const uint32_t* rw = reinterpret_cast<const uint32_t*>(&rr[v]);
-                    const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w};
-                    uint32_t o[4];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const float2 rf = Pack2<T>::unpack(rw[e]), wf = Pack2<T>::unpack(ww[e]);
-                        o[e] = Pack2<T>::pack(rf.x * rstd * wf.x, rf.y * rstd * wf.y);
-                    }
-                    reinterpret_cast<uint4*>(out_h + row * NT)[v] = make_uint4(o[0], o[1], o[2], o[3]);
-                }
-            }
-        }
     }
     tc_fence_before();
     __syncthreads();
@@ -295,7 +232,7 @@ __global__ void __launch_bounds__(AN_THREADS, 1) linear_add_rmsnorm_kernel(const
     }
 }
 
-int an_chunk(int N) { return N % 192 == 0 ? 192 : (N % 128 == 0 ? 128 : 64); }
+int an_chunk(int N) { return N == 192 ? 192 : (N == 128 ? 128 : 64); }
 
 }  // namespace
 }  // namespace vig
@@ -304,8 +241,18 @@ using namespace vig;
 
 extern "C" int vig_linear_add_rmsnorm_supported(int64_t M, int K, int N, int dtype) {
     if (dtype != VIG_DTYPE_BF16 && dtype != VIG_DTYPE_F16) return 0;
-    if (M <= 0 || K <= 0 || K % AN_BK || !(N == 64 || N == 128 || N == 192 || N == 256 || N == 384)) return 0;
+    if (M <= 0 || K <= 0 || K % AN_BK || !(N == 64 || N == 128 || N == 192 || N == 256 || N == 384 || N == 768)) return 0;
     return tc::encode_fn() != nullptr;
+}
+
+// Whether the one kernel is to be taken instead of the library's GEMM and the norm kernel.  Rows of up to 192 values always (17-22 % faster from
+// 50000 rows on).  Longer rows are 256-row tiles of CTA pairs, whose epilogue shows behind a last or only tile; measured (us, one kernel / two):
+// N = 384, K = 384: 12544 rows 13.9 / 13.5, 25088 21 / 26, 131072 92 / 111; K = 1024: 25088 36 / 33, 50176 57 / 60, 131072 130 / 146;
+// N = 768, K = 768: 12544 26 / 26, 25088 46 / 51, 131072 192 / 255; K = 2048: 25088 79 / 79, 50176 150 / 156, 131072 395 / 415;
+// N = 256, K = 256: 25088 16 / 14, 50176 25 / 27, 131072 54 / 65.
+extern "C" int vig_linear_add_rmsnorm_preferred(int64_t M, int K, int N, int dtype) {
+    if (!vig_linear_add_rmsnorm_supported(M, K, N, dtype)) return 0;
+    return N <= 192 || M >= 40000 || (N >= 384 && K <= N && M >= 20000);
 }
 
 extern "C" int vig_linear_add_rmsnorm_fwd(const void* x, int64_t ldx, const void* w, const void* residual, const void* norm_weight,
@@ -318,23 +265,17 @@ extern "C" int vig_linear_add_rmsnorm_fwd(const void* x, int64_t ldx, const void
          reinterpret_cast<uintptr_t>(norm_weight) | reinterpret_cast<uintptr_t>(out_r) | reinterpret_cast<uintptr_t>(out_h)) & 15)
         return VIG_ERR_ALIGN;
     if (ldx < K || (ldx * 2) % 16 || M >= (1ll << 31) - 128) return VIG_ERR_ARG;
+    if (N > 192) return pair_norm_launch(x, ldx, w, residual, norm_weight, out_r, out_h, M, K, N, eps, dtype, status_dev, (cudaStream_t)stream);
     const int CH = an_chunk(N);
     AnMaps maps;
     if (!tc::make_map_2d(&maps.x, x, M, K, ldx, 128, dtype) || !tc::make_map_2d(&maps.w, w, N, K, K, CH, dtype)) return VIG_ERR_DEVICE;
     const int stage_bytes = AN_A_BYTES + N * AN_BK * 2;
-    int nstage = (200 * 1024) / stage_bytes;
+    const size_t e_bytes = 2 * (size_t)(N / 64) * 16384;
+    int nstage = (int)((227 * 1024 - 4096 - e_bytes) / stage_bytes);     // the ring gets what the two epilogue tiles leave of the 227 KB
     if (nstage > 6) nstage = 6;
-    if (nstage < 2) return VIG_ERR_SHAPE;
-    const bool tma_epi = N <= 192;
-    const size_t e_bytes = tma_epi ? 2 * (size_t)(N / 64) * 16384 : 0;
-    if (tma_epi) {                                  // the ring gets what the two epilogue tiles leave of the 227 KB
-        nstage = (int)((227 * 1024 - 4096 - e_bytes) / stage_bytes);
-        if (nstage > 6) nstage = 6;
-        if (nstage < 2) return VIG_ERR_SHAPE;
-    }
     const size_t smem = (size_t)nstage * stage_bytes + e_bytes + 8 * 24 + 16 + 2 * 128 * 4 + 1024;
-    if (tma_epi && ((residual && !tc::make_map_2d(&maps.res, residual, M, N, N, 128, dtype)) || !tc::make_map_2d(&maps.r, out_r, M, N, N, 128, dtype) ||
-                    !tc::make_map_2d(&maps.h, out_h, M, N, N, 128, dtype)))
+    if ((residual && !tc::make_map_2d(&maps.res, residual, M, N, N, 128, dtype)) || !tc::make_map_2d(&maps.r, out_r, M, N, N, 128, dtype) ||
+                    !tc::make_map_2d(&maps.h, out_h, M, N, N, 128, dtype))
         return VIG_ERR_DEVICE;
     static int sm_count[64] = {};
     int dev = 0;
@@ -359,9 +300,7 @@ extern "C" int vig_linear_add_rmsnorm_fwd(const void* x, int64_t ldx, const void
     switch (N) {                                                                                                               \
         case 64: VIG_AN_LAUNCH(TT, 64) break;                                                                                  \
         case 128: VIG_AN_LAUNCH(TT, 128) break;                                                                                \
-        case 192: VIG_AN_LAUNCH(TT, 192) break;                                                                                \
-        case 256: VIG_AN_LAUNCH(TT, 256) break;                                                                                \
-        default: VIG_AN_LAUNCH(TT, 384) break;                                                                                 \
+        default: VIG_AN_LAUNCH(TT, 192) break;                                                                                 \
     }
     if (dtype == VIG_DTYPE_BF16) VIG_AN_WIDTHS(__nv_bfloat16) else VIG_AN_WIDTHS(__half)
 #undef VIG_AN_WIDTHS

@@ -15,7 +15,7 @@ namespace py = pybind11;
 #define VIG_HOST_API(X)                                                                                                     \
     X(vig_strerror) X(vig_bigla_fwd) X(vig_bigla_workspace_bytes) X(vig_bigla_bwd_full) X(vig_bigla_bwd_full_workspace_bytes) \
     X(vig_dwconv3x3_fwd) X(vig_gate_inject_fwd) X(vig_add_rmsnorm_fwd) X(vig_layernorm_act_fwd) X(vig_layernorm_act_add_fwd)  \
-    X(vig_layernorm_act_add_rmsnorm_fwd) X(vig_linear_swiglu_fwd) X(vig_linear_swiglu_preferred) X(vig_linear_add_rmsnorm_fwd) \
+    X(vig_layernorm_act_add_rmsnorm_fwd) X(vig_linear_swiglu_fwd) X(vig_linear_swiglu_preferred) X(vig_linear_add_rmsnorm_fwd) X(vig_linear_add_rmsnorm_preferred) \
     X(vig_stem_fold_fwd) X(vig_stem_unfold_fwd) X(vig_stem_conv_ln_fwd)                   \
     X(vig_stem_conv_ln_supported) X(vig_swiglu_fwd) X(vig_add_layernorm_fwd) X(vig_chain_launches) X(vig_token_mean_fwd) X(vig_embed_conv_ln_fwd) X(vig_block_tail_preferred) X(vig_block_tail_fwd)
 struct Api {

@@ -64,8 +64,10 @@ Tensor mlp_in(const Ctx& c, const Tensor& x, const Tensor& w) {
     ok(api.vig_swiglu_fwd(ptr(z), (uint8_t*)ptr(z) + I * z.element_size(), ptr(out), M, I, 2 * I, I, c.code, c.stream), "vig_swiglu_fwd");
     return out;
 }
+// r = x W^T + residual, h = RMSNorm(r): one kernel where it is the faster one
 std::pair<Tensor, Tensor> linear_add_rmsnorm(const Ctx& c, const Tensor& x, const Tensor& w, const Tensor& res, const Tensor& nw, double eps) {
     const int64_t K = x.size(-1), N = w.size(0), M = x.numel() / K;
+    if (!api.vig_linear_add_rmsnorm_preferred(M, K, N, c.code)) return add_rmsnorm(c, at::linear(x, w), nw, res, eps, true);
     Tensor h = at::empty({x.size(0), x.size(1), N}, x.options()), r = at::empty({x.size(0), x.size(1), N}, x.options());
     ok(api.vig_linear_add_rmsnorm_fwd(ptr(x), K, ptr(w), ptr(res), ptr(nw), ptr(r), ptr(h), M, K, N, (float)eps, c.code, c.status, c.stream), "vig_linear_add_rmsnorm_fwd");
     return {h, r};

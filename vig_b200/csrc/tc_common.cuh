@@ -130,10 +130,14 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4}], [%2];"
                  ::"r"(dst), "l"(map), "r"(cluster_bar), "r"(c0), "r"(c1) : "memory");
 }
-// arrives at the barrier of this offset in both CTAs when the MMAs issued so far are done
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
-    asm volatile("{\n\t.reg .b16 m;\n\tmov.b16 m, 3;\n\t"
-                 "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m;\n\t}" ::"r"(bar) : "memory");
+// arrives at the barrier of this offset in both CTAs of the pair (ranks ``even`` and ``even`` + 1 of the cluster) when the MMAs issued so far are done
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar, uint32_t even = 0) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(bar), "h"((uint16_t)(3u << even)) : "memory");
+}
+// a value into another CTA's shared memory; that CTA's barrier counts its four bytes
+__device__ __forceinline__ void st_async_f32(uint32_t cluster_addr, float v, uint32_t cluster_bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(cluster_addr), "r"(__float_as_uint(v)), "r"(cluster_bar) : "memory");
 }
 __device__ __forceinline__ void tc_mma_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
     asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -186,11 +190,13 @@ template <> struct Pack2<__nv_bfloat16> {
     static constexpr uint32_t FMT = 1;
     __device__ static uint32_t pack(float a, float b) { __nv_bfloat162 t = __floats2bfloat162_rn(a, b); return *reinterpret_cast<uint32_t*>(&t); }
     __device__ static float2 unpack(uint32_t u) { return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&u)); }
+    __device__ static uint32_t add(uint32_t a, uint32_t b) { __nv_bfloat162 t = __hadd2(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<__nv_bfloat162*>(&b)); return *reinterpret_cast<uint32_t*>(&t); }
 };
 template <> struct Pack2<__half> {
     static constexpr uint32_t FMT = 0;
     __device__ static uint32_t pack(float a, float b) { __half2 t = __floats2half2_rn(a, b); return *reinterpret_cast<uint32_t*>(&t); }
     __device__ static float2 unpack(uint32_t u) { return __half22float2(*reinterpret_cast<__half2*>(&u)); }
+    __device__ static uint32_t add(uint32_t a, uint32_t b) { __half2 t = __hadd2(*reinterpret_cast<__half2*>(&a), *reinterpret_cast<__half2*>(&b)); return *reinterpret_cast<uint32_t*>(&t); }
 };
 
 struct Waiter {

@@ -133,6 +133,12 @@ def plain_linear(m):
             not (m._forward_hooks or m._forward_pre_hooks or g._global_forward_hooks or g._global_forward_pre_hooks))
 
 
+def plain_norm(m):
+    g = nn.modules.module
+    return (type(m) is RMSNorm and "forward" not in m.__dict__ and
+            not (m._forward_hooks or m._forward_pre_hooks or g._global_forward_hooks or g._global_forward_pre_hooks))
+
+
 class GLAMLP(nn.Module):
     def __init__(self, hidden_size, hidden_ratio: Optional[int] = None, intermediate_size: Optional[int] = None,
                  hidden_act="swish"):
@@ -179,24 +185,32 @@ class GLABlock(nn.Module):
 
     def fused_epilogues_supported(self, x):
         """True when both projections of the block can run with the residual add and the following RMSNorm as their
-        epilogue (``ops.linear_add_rmsnorm``: 16-bit CUDA tensors, hidden size <= 384, no projection bias)."""
-        return (self.attn.o_proj.bias is None and self.mlp.down_proj.bias is None and x.shape[-1] <= 192 and
-                ops.linear_add_rmsnorm_supported(x, self.attn.o_proj.weight) and
-                x.shape[-1] == self.mlp.down_proj.weight.shape[0] and self.mlp.down_proj.weight.shape[1] % 64 == 0)
+        epilogue (``ops.linear_add_rmsnorm``: 16-bit CUDA tensors, plain projections)."""
+        o, down = self.attn.o_proj, self.mlp.down_proj
+        wide = x.shape[-1] > 192                              # rows of up to 192 values look at the biases only
+        return (o.bias is None and down.bias is None and not (wide and not (plain_linear(o) and plain_linear(down) and plain_norm(self.attn_norm) and plain_norm(self.mlp_norm))) and
+                ops.linear_add_rmsnorm_supported(x, o.weight) and x.shape[-1] == down.weight.shape[0] and down.weight.shape[1] % 64 == 0)
+
+    @staticmethod
+    def _project(y, linear, residual, norm):
+        """``(norm(r), r)`` with ``r = linear(y) + residual``: one kernel where it is the faster one, the same roundings in two."""
+        if ops.linear_add_rmsnorm_supported(y, linear.weight, preferred=True):
+            return ops.linear_add_rmsnorm(y, linear.weight, residual, norm.weight, norm.eps)
+        return ops.add_rmsnorm(F.linear(y, linear.weight), norm.weight, residual, norm.eps, True)
 
     def forward_prenormed(self, h, residual, next_norm, **kwargs):
         """The block with its norms moved into the projections' epilogues: takes ``h = attn_norm(residual stream)`` and
         the residual stream, returns ``(next_norm(new residual stream), new residual stream)`` -- ``next_norm`` is the
         next block's ``attn_norm`` or the model's final norm.  Same arithmetic as ``forward_deferred`` chained."""
         y = self.attn(h, skip_o_proj=True, **kwargs)
-        h2, residual = ops.linear_add_rmsnorm(y, self.attn.o_proj.weight, residual, self.mlp_norm.weight, self.mlp_norm.eps)
+        h2, residual = self._project(y, self.attn.o_proj, residual, self.mlp_norm)
         m = self.mlp
         if plain_linear(m.gate_proj) and ops.linear_swiglu_supported(h2, m.gate_proj.weight, preferred=True):
             z = ops.linear_swiglu(h2, m.gate_proj.weight)
         else:
             gate, yy = m.gate_proj(h2).chunk(2, -1)
             z = ops.swiglu(gate, yy)
-        return ops.linear_add_rmsnorm(z, m.down_proj.weight, residual, next_norm.weight, next_norm.eps)
+        return self._project(z, m.down_proj, residual, next_norm)
 
     def forward_deferred(self, hidden_states, residual, **kwargs):
         """Same block, but the trailing residual add is left to the caller's next norm: takes the pair

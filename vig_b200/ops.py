@@ -451,13 +451,15 @@ def embed_conv_ln(x, weight, conv_bias, ln_weight, ln_bias, eps=1e-5, act_gelu=T
     return y
 
 
-def linear_add_rmsnorm_supported(x, w):
-    """True when ``linear_add_rmsnorm`` can run on these operands (16-bit CUDA tensors, K % 64 == 0, N in {64, 128, 192, 256, 384})."""
+def linear_add_rmsnorm_supported(x, w, preferred=False):
+    """True when ``linear_add_rmsnorm`` can run on these operands (16-bit CUDA tensors, K % 64 == 0, N in {64, 128, 192, 256, 384, 768});
+    with ``preferred`` also that it is to be taken instead of the library's GEMM and the norm kernel."""
     if not (x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and w.dtype == x.dtype and x.stride(-1) == 1):
         return False
     N, K = w.shape
     M = x.numel() // K
-    return bool(_lib.lib().vig_linear_add_rmsnorm_supported(M, K, N, _lib.dtype_code(x)))
+    fn = _lib.lib().vig_linear_add_rmsnorm_preferred if preferred else _lib.lib().vig_linear_add_rmsnorm_supported
+    return bool(fn(M, K, N, _lib.dtype_code(x)))
 
 
 def linear_add_rmsnorm(x, w, residual, norm_weight, eps=1e-6):
