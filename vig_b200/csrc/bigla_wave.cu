@@ -383,7 +383,8 @@ __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_c
             const uint32_t s = m % 3;
             bool have = false;
             const int dir_mask_it = dir_prev;                 // direction of iteration m - 1 (the one whose scores are masked in this trip)
-            float4 gl[NTK];                                   // cumulative log2-gates of my tokens, from the group's first token
+            F2 gl01[NTK], gl23[NTK];                          // cumulative log2-gates of my tokens, from the part's first token
+            F2 first01 = f2_make(0.f, 0.f), first23 = first01;   // what the group's parts before mine add to them
             uint8_t* stg = smem + s * W_STAGE_B;
             int dmask = 0;
             // A test of an mbarrier costs a few hundred cycles even when its phase completed long ago (it queues behind the
@@ -414,43 +415,39 @@ __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_c
 #pragma unroll
                 for (int u = 0; u < NTK; ++u)
                     raw[u] = *reinterpret_cast<const uint2*>(stg + WS_G + (grp * 8 + ((half * NTK + u) ^ dmask)) * 128 + c4l * 8);
-                float4 run = make_float4(0.f, 0.f, 0.f, 0.f);
+                F2 run01 = f2_make(0.f, 0.f), run23 = run01;
 #pragma unroll
                 for (int u = 0; u < NTK; ++u) {
                     const float2 a = Pack2<T>::unpack(raw[u].x), b2 = Pack2<T>::unpack(raw[u].y);
-                    float4 t = make_float4(a.x, a.y, b2.x, b2.y);
+                    F2 t01 = f2_make(a.x, a.y), t23 = f2_make(b2.x, b2.y);
                     if (RAW) {                                // log2(1 + 2^(-x log2 e)) = -log2 sigmoid(x)
                         const F2 nl = f2_make(-LOG2E, -LOG2E), one = f2_make(1.f, 1.f);
-                        const F2 y01 = f2_mul(f2_make(t.x, t.y), nl), y23 = f2_mul(f2_make(t.z, t.w), nl);
+                        const F2 y01 = f2_mul(t01, nl), y23 = f2_mul(t23, nl);
                         const F2 e01 = f2_add(one, f2_make(ex2(f2_lo(y01)), ex2(f2_hi(y01)))), e23 = f2_add(one, f2_make(ex2(f2_lo(y23)), ex2(f2_hi(y23))));
-                        t.x = lg2(f2_lo(e01)); t.y = lg2(f2_hi(e01)); t.z = lg2(f2_lo(e23)); t.w = lg2(f2_hi(e23));
+                        t01 = f2_make(lg2(f2_lo(e01)), lg2(f2_hi(e01))); t23 = f2_make(lg2(f2_lo(e23)), lg2(f2_hi(e23)));
                     }
                     const float cu = grp * 8 + ((half * NTK + u) ^ dmask) < n_valid ? coef : 0.f;   // padding rows: gate 0
+                    const F2 c2 = f2_make(cu, cu);
                     if (CLAMP) {
-                        run.x += fmaxf(t.x * cu, clamp_lo); run.y += fmaxf(t.y * cu, clamp_lo);
-                        run.z += fmaxf(t.z * cu, clamp_lo); run.w += fmaxf(t.w * cu, clamp_lo);
+                        const F2 g01 = f2_mul(t01, c2), g23 = f2_mul(t23, c2);
+                        run01 = f2_add(run01, f2_make(fmaxf(f2_lo(g01), clamp_lo), fmaxf(f2_hi(g01), clamp_lo)));
+                        run23 = f2_add(run23, f2_make(fmaxf(f2_lo(g23), clamp_lo), fmaxf(f2_hi(g23), clamp_lo)));
                     } else {
-                        const F2 c2 = f2_make(cu, cu);
-                        const F2 r01 = f2_fma(f2_make(t.x, t.y), c2, f2_make(run.x, run.y)), r23 = f2_fma(f2_make(t.z, t.w), c2, f2_make(run.z, run.w));
-                        run = make_float4(f2_lo(r01), f2_hi(r01), f2_lo(r23), f2_hi(r23));
+                        run01 = f2_fma(t01, c2, run01); run23 = f2_fma(t23, c2, run23);
                     }
-                    gl[u] = run;
+                    gl01[u] = run01; gl23[u] = run23;
                 }
                 // a part continues the sums of the parts scanned before it; the last one also knows the group's total
-                float4 first = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (int k = 0; k + 1 < NPART; ++k) {
-                    float4 t;
-                    t.x = __shfl_sync(0xffffffffu, run.x, lane_of(k)); t.y = __shfl_sync(0xffffffffu, run.y, lane_of(k));
-                    t.z = __shfl_sync(0xffffffffu, run.z, lane_of(k)); t.w = __shfl_sync(0xffffffffu, run.w, lane_of(k));
-                    if (k < half) { first.x += t.x; first.y += t.y; first.z += t.z; first.w += t.w; }
+                    const F2 t01 = f2_make(__shfl_sync(0xffffffffu, f2_lo(run01), lane_of(k)), __shfl_sync(0xffffffffu, f2_hi(run01), lane_of(k)));
+                    const F2 t23 = f2_make(__shfl_sync(0xffffffffu, f2_lo(run23), lane_of(k)), __shfl_sync(0xffffffffu, f2_hi(run23), lane_of(k)));
+                    if (k < half) { first01 = f2_add(first01, t01); first23 = f2_add(first23, t23); }
                 }
                 float* part = reinterpret_cast<float*>(smem + WO_PART) + (m & 1) * (W_PREP_WARPS * WDK);
-                if (half) {
-                    if (half == NPART - 1)
-                        reinterpret_cast<float4*>(part)[grp * 16 + c4l] = make_float4(run.x + first.x, run.y + first.y, run.z + first.z, run.w + first.w);
-#pragma unroll
-                    for (int u = 0; u < NTK; ++u) { gl[u].x += first.x; gl[u].y += first.y; gl[u].z += first.z; gl[u].w += first.w; }
+                if (half == NPART - 1) {
+                    const F2 s01 = f2_add(run01, first01), s23 = f2_add(run23, first23);
+                    reinterpret_cast<float4*>(part)[grp * 16 + c4l] = make_float4(f2_lo(s01), f2_hi(s01), f2_lo(s23), f2_hi(s23));
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive_plain(bar(B_PART + (m & 1)));
@@ -541,8 +538,10 @@ __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_c
             __syncwarp();
             if (*abort_flag) break;
             // ---- my group's offset: (sum of the groups scanned before mine) - G_ref, G_ref = sum of the first 8 groups in
-            // scan order.  Half-warp gq reads groups 8 gq .. 8 gq + 7 (scan order) for its 4 channels; one exchange. ----
-            float4 off;
+            // scan order.  Half-warp gq reads groups 8 gq .. 8 gq + 7 (scan order) for its 4 channels and takes its share of the
+            // difference; one exchange adds the shares (exchanging both sums took eight shuffles for every warp instead of four: 64 x 3 sequences
+            // of 4096 283 -> 280 us, with the cumulative gates kept as pairs). ----
+            F2 off01, off23;
             {
                 const float4* part = reinterpret_cast<const float4*>(smem + WO_PART) + (m & 1) * (W_PREP_WARPS * 16) + c4l;
                 const int flip = cur.dir ? W_PREP_WARPS - 1 : 0;          // scan position go <-> group go ^ flip
@@ -559,46 +558,42 @@ __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_c
                     const F2 kk = f2_make(k, k);
                     b01 = f2_fma(kk, t01, b01); b23 = f2_fma(kk, t23, b23);
                 }
-                float4 sum = make_float4(f2_lo(s01), f2_hi(s01), f2_lo(s23), f2_hi(s23));
-                float4 bef = make_float4(f2_lo(b01), f2_hi(b01), f2_lo(b23), f2_hi(b23));
-                auto add_from = [&](float4& v, int x) {
-                    v.x += __shfl_xor_sync(0xffffffffu, v.x, x); v.y += __shfl_xor_sync(0xffffffffu, v.y, x);
-                    v.z += __shfl_xor_sync(0xffffffffu, v.z, x); v.w += __shfl_xor_sync(0xffffffffu, v.w, x);
-                };
-                if (D32) { add_from(sum, 16); add_from(bef, 16); }        // quarters -> halves of the scan order
+                auto from = [&](F2 v, int x) { return f2_make(__shfl_xor_sync(0xffffffffu, f2_lo(v), x), __shfl_xor_sync(0xffffffffu, f2_hi(v), x)); };
+                const float r = half < NPART / 2 ? -1.f : 0.f;            // the parts that read the first 8 groups hold G_ref
+                const F2 rr = f2_make(r, r);
+                b01 = f2_fma(rr, s01, b01); b23 = f2_fma(rr, s23, b23);
                 constexpr int X = D32 ? 8 : 16;
-                float4 osum, obef;
-                osum.x = __shfl_xor_sync(0xffffffffu, sum.x, X); osum.y = __shfl_xor_sync(0xffffffffu, sum.y, X);
-                osum.z = __shfl_xor_sync(0xffffffffu, sum.z, X); osum.w = __shfl_xor_sync(0xffffffffu, sum.w, X);
-                obef.x = __shfl_xor_sync(0xffffffffu, bef.x, X); obef.y = __shfl_xor_sync(0xffffffffu, bef.y, X);
-                obef.z = __shfl_xor_sync(0xffffffffu, bef.z, X); obef.w = __shfl_xor_sync(0xffffffffu, bef.w, X);
-                const float4 gref = half >= NPART / 2 ? osum : sum;       // the part that read the first 8 groups has it
-                off = make_float4(bef.x + obef.x - gref.x, bef.y + obef.y - gref.y, bef.z + obef.z - gref.z, bef.w + obef.w - gref.w);
-                if (grp == 0 && half == 0) {                              // [G_ref | G_last] of this iteration for the state warps
-                    float4* ve = reinterpret_cast<float4*>(vec + (m & 3) * 128) + c4l;
-                    ve[0] = gref;
-                    ve[16] = make_float4(sum.x + osum.x, sum.y + osum.y, sum.z + osum.z, sum.w + osum.w);
+                if (D32) { b01 = f2_add(b01, from(b01, 16)); b23 = f2_add(b23, from(b23, 16)); }     // quarters -> halves of the scan order
+                off01 = f2_add(f2_add(b01, from(b01, X)), first01); off23 = f2_add(f2_add(b23, from(b23, X)), first23);
+                if (grp == 0) {                                           // [G_ref | G_last] of this iteration for the state warps
+                    if (D32) { s01 = f2_add(s01, from(s01, 16)); s23 = f2_add(s23, from(s23, 16)); }
+                    const F2 l01 = f2_add(s01, from(s01, X)), l23 = f2_add(s23, from(s23, X));
+                    if (half == 0) {
+                        float4* ve = reinterpret_cast<float4*>(vec + (m & 3) * 128) + c4l;
+                        ve[0] = make_float4(f2_lo(s01), f2_hi(s01), f2_lo(s23), f2_hi(s23));
+                        ve[16] = make_float4(f2_lo(l01), f2_hi(l01), f2_lo(l23), f2_hi(l23));
+                    }
                 }
             }
             // ---- scale phase ----
             // Log-gates are <= 0, so a lane's exponents are monotone along its 4 tokens: the largest magnitude is at one
             // of the two ends.  Beyond the range the factorisation covers, exponents are clamped and the call is flagged.
-            float worst = fmaxf(fmaxf(fabsf(off.x + gl[0].x), fabsf(off.y + gl[0].y)), fmaxf(fabsf(off.z + gl[0].z), fabsf(off.w + gl[0].w)));
-            worst = fmaxf(worst, fmaxf(fmaxf(fabsf(off.x + gl[NTK - 1].x), fabsf(off.y + gl[NTK - 1].y)), fmaxf(fabsf(off.z + gl[NTK - 1].z), fabsf(off.w + gl[NTK - 1].w))));
+#pragma unroll
+            for (int u = 0; u < NTK; ++u) { gl01[u] = f2_add(off01, gl01[u]); gl23[u] = f2_add(off23, gl23[u]); }
+            auto largest = [](F2 a, F2 b) { return fmaxf(fmaxf(fabsf(f2_lo(a)), fabsf(f2_hi(a))), fmaxf(fabsf(f2_lo(b)), fabsf(f2_hi(b)))); };
+            const float worst = fmaxf(largest(gl01[0], gl23[0]), largest(gl01[NTK - 1], gl23[NTK - 1]));
             const bool out_of_range = __any_sync(0xffffffffu, !(worst <= MAX_EXPONENT2));
             if (out_of_range) {                               // rare: clamp in place, flag the call
                 if (lane == 0 && p.status) atomicOr(p.status, 2);
+                auto clamp = [](F2 v) {
+                    return f2_make(fminf(fmaxf(f2_lo(v), -MAX_EXPONENT2), MAX_EXPONENT2), fminf(fmaxf(f2_hi(v), -MAX_EXPONENT2), MAX_EXPONENT2));
+                };
 #pragma unroll
-                for (int u = 0; u < NTK; ++u) {
-                    gl[u].x = fminf(fmaxf(off.x + gl[u].x, -MAX_EXPONENT2), MAX_EXPONENT2) - off.x;
-                    gl[u].y = fminf(fmaxf(off.y + gl[u].y, -MAX_EXPONENT2), MAX_EXPONENT2) - off.y;
-                    gl[u].z = fminf(fmaxf(off.z + gl[u].z, -MAX_EXPONENT2), MAX_EXPONENT2) - off.z;
-                    gl[u].w = fminf(fmaxf(off.w + gl[u].w, -MAX_EXPONENT2), MAX_EXPONENT2) - off.w;
-                }
+                for (int u = 0; u < NTK; ++u) { gl01[u] = clamp(gl01[u]); gl23[u] = clamp(gl23[u]); }
             }
 #pragma unroll
             for (int u = 0; u < NTK; ++u) {
-                const float ex = off.x + gl[u].x, ey = off.y + gl[u].y, ez = off.z + gl[u].z, ew = off.w + gl[u].w;
+                const float ex = f2_lo(gl01[u]), ey = f2_hi(gl01[u]), ez = f2_lo(gl23[u]), ew = f2_hi(gl23[u]);
                 uint2 ko, qo;                                 // scale * out_scale is applied to the output instead
                 ko.x = ScalePair<T>::mul(rk[u].x, ex2(-ex), ex2(-ey)); ko.y = ScalePair<T>::mul(rk[u].y, ex2(-ez), ex2(-ew));
                 if (!so) { qo.x = ScalePair<T>::mul(rq[u].x, ex2(ex), ex2(ey)); qo.y = ScalePair<T>::mul(rq[u].y, ex2(ez), ex2(ew)); }
