@@ -1,5 +1,5 @@
 """The row-local half of a block as one kernel (vig_block_tail_fwd) against the separate kernels it stands for, at the edges of
-its 16-, 32- and 64-token tiles and of the rule that picks them."""
+its 16-, 32- and 64-token tiles, of the clusters of 8, 4 and 2 that share one, and of the rule that picks them."""
 import pytest
 import torch
 
@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("M,I,out_act", [(1, 512, True), (16, 64, False), (17, 512, True), (196, 512, True), (2368, 512, False), (2369, 512, True),
-                                         (2401, 128, True), (4736, 512, True), (4737, 512, True), (9999, 512, False)])
+                                         (256, 512, False), (257, 512, True), (512, 448, True), (513, 512, False), (1024, 128, True), (1025, 512, True), (100, 256, True), (2401, 128, True), (4736, 512, True), (4737, 512, True), (9999, 512, False)])
 def test_block_tail_equals_the_separate_kernels(dtype, M, I, out_act):
     import vig_b200
     from vig_b200 import ops

@@ -8,7 +8,9 @@
 // intermediates in shared memory; the three weight matrices (664 KB) stream from L2 through a ring of 24 KB stages in the
 // order they are used, and do not wait for the preceding kernel.  Bound: the stream for R = 16 (one CTA draws about 120 B/ns
 // from L2: 5.5 us), the mma.sync rate for R = 64 (21 M multiply-adds per CTA at 1024 a cycle: 11 us); R is the smallest that
-// keeps the call in one wave of CTAs.  Large calls run the tcgen05 kernels, whose MMAs are three times faster per SM.
+// keeps the call in one wave of CTAs.  Where 16-token tiles leave most SMs idle, a cluster of 2, 4 or 8 CTAs shares a tile: each does
+// the injection and the output projection for itself (72 KB) and its part of the MLP's features, and the first one adds up the
+// others' down projections, which they write into its shared memory in fp32.  Large calls run the tcgen05 kernels, whose MMAs are three times faster per SM.
 //
 // Roundings are those of the separate kernels: injection, projections, sums, norms and activation are each rounded to the type.
 #include "mma_common.cuh"
@@ -42,10 +44,13 @@ template <> __device__ __forceinline__ void mma_t<__half>(float* c, const uint32
 }
 __device__ __forceinline__ void bt_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
-template <int RB> struct BtSmem {
-    static constexpr int NST = RB == 1 ? 7 : RB == 2 ? 6 : 4;             // what the token tiles leave of the 227 KB
+constexpr int BT_CLUSTER = 8;                             // largest cluster of a tile
+
+template <int RB, bool CL> struct BtSmem {
+    static constexpr int NST = CL ? 4 : RB == 1 ? 7 : RB == 2 ? 6 : 4;    // what the token tiles (and partial sums) leave of the 227 KB
     static constexpr uint32_t R = 16 * RB, RING = 0, A = RING + NST * BT_STAGE, RES = A + R * BT_PA, Z = RES + R * BT_PA, PART = Z + R * BT_PZ,
-                              BAR = PART + R * 8 * 4, BYTES = BAR + 2 * NST * 8 + 16 + 1024;
+                              SUMS = PART + R * 8 * 4,
+                              BAR = SUMS + (CL ? (BT_CLUSTER - 1) * R * BT_C * 4 : 0), BYTES = BAR + 2 * NST * 8 + 16 + 1024;
     static_assert(BYTES <= 227 * 1024, "shared memory");
 };
 
@@ -64,10 +69,10 @@ template <int NT> __device__ __forceinline__ void bt_load_b(uint32_t (*b)[2], ui
     }
 }
 
-// RB: blocks of 16 tokens; WR: warp rows (the other 8 / WR warps share the columns)
-template <typename T, int RB, int WR>
+// RB: blocks of 16 tokens; WR: warp rows (the other 8 / WR warps share the columns); CL: a cluster's CTAs share a tile
+template <typename T, int RB, int WR, bool CL>
 __global__ void __launch_bounds__(BT_THREADS, 1) block_tail_kernel(const __grid_constant__ BtMaps maps, const __grid_constant__ BtParams p) {
-    using SM = BtSmem<RB>;
+    using SM = BtSmem<RB, CL>;
     constexpr int NST = SM::NST, R = 16 * RB, WC = 8 / WR, MB = RB / WR, NT = BT_C / WC / 8, FT = 64 / WC / 8;   // row blocks, projection n tiles, feature tiles of a warp
     extern __shared__ uint8_t bt_raw[];
     uint8_t* smem = bt_raw + ((1024u - (smem_u32(bt_raw) & 1023u)) & 1023u);
@@ -77,7 +82,9 @@ __global__ void __launch_bounds__(BT_THREADS, 1) block_tail_kernel(const __grid_
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + SM::BAR + 16 * NST);
     const Waiter waiter{abort_flag, p.status};
     const int IB = p.I / 64;                                 // 64-feature chunks of the MLP
-    const int64_t row0 = (int64_t)blockIdx.x * R;
+    const int share = CL ? (int)cluster_size() : 1, rank = CL ? (int)cluster_rank() : 0;
+    const int c0 = rank * IB / share, c1 = (rank + 1) * IB / share;       // mine
+    const int64_t row0 = (int64_t)(blockIdx.x / share) * R;
     const int n = (int)min((int64_t)R, p.M - row0);
     if (tid == 0) {
         for (int s = 0; s < NST; ++s) { mbar_init(full + 8 * s, 1); mbar_init(empty + 8 * s, 8); }
@@ -85,24 +92,30 @@ __global__ void __launch_bounds__(BT_THREADS, 1) block_tail_kernel(const __grid_
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    if (CL) asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");     // every CTA of the cluster runs before its shared memory is written
     if (warp == 8) {                                         // ---- weights, in the order of use: output projection, 64-feature chunks of the gate projection, down projection
         if (lane == 0) {
-            const int T1 = BT_C / 64, T2 = T1 + IB * (BT_C / 64), T3 = T2 + IB;
+            const int T1 = BT_C / 64, T2 = T1 + (c1 - c0) * (BT_C / 64), T3 = T2 + c1 - c0;
             for (int t = 0; t < T3; ++t) {
                 const int s = t % NST;
                 waiter.wait(empty + 8 * s, ((t / NST) & 1) ^ 1);
                 if (*abort_flag) break;
                 const uint32_t dst = sb + SM::RING + s * BT_STAGE, bar = full + 8 * s;
                 if (t >= T1 && t < T2) {
-                    const int c = (t - T1) / (BT_C / 64), kb = (t - T1) % (BT_C / 64);
+                    const int c = c0 + (t - T1) / (BT_C / 64), kb = (t - T1) % (BT_C / 64);
                     mbar_expect_tx(bar, 2 * 64 * 128);
                     tma_load_2d(dst, &maps.wg, kb * 64, c * 64, bar);                    // gate rows
                     tma_load_2d(dst + 64 * 128, &maps.wg, kb * 64, p.I + c * 64, bar);   // the matching y rows
                 } else {
                     mbar_expect_tx(bar, BT_STAGE);
-                    tma_load_2d(dst, t < T1 ? &maps.wo : &maps.wd, (t < T1 ? t : t - T2) * 64, 0, bar);
+                    tma_load_2d(dst, t < T1 ? &maps.wo : &maps.wd, (t < T1 ? t : c0 + t - T2) * 64, 0, bar);
                 }
             }
+        }
+        if (CL) {                                            // both cluster barriers are for all threads
+            asm volatile("barrier.cluster.wait;" ::: "memory");
+            asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+            asm volatile("barrier.cluster.wait;" ::: "memory");
         }
         return;
     }
@@ -244,7 +257,7 @@ __global__ void __launch_bounds__(BT_THREADS, 1) block_tail_kernel(const __grid_
 #pragma unroll
             for (int m = 0; m < MB; ++m) mm::ldsm4(aA + m * 16 * BT_PA + ks * 32, fa[ks][m]);
 #pragma unroll 1
-        for (int c = 0; c < IB; ++c) {
+        for (int c = c0; c < c1; ++c) {
             float g[MB][FT][4], y[MB][FT][4];
 #pragma unroll
             for (int m = 0; m < MB; ++m)
@@ -292,7 +305,30 @@ __global__ void __launch_bounds__(BT_THREADS, 1) block_tail_kernel(const __grid_
     }
     bt_sync();
     zero();
-    project(acc, aZ, BT_PZ, IB);
+    project(acc, aZ + c0 * 128, BT_PZ, c1 - c0);
+    if constexpr (CL) {                                      // the others' sums over their features go to the first CTA
+        const uint32_t mine = sb + SM::SUMS + (uint32_t)tid * (MB * NT * 16);
+        constexpr uint32_t PER = 256 * MB * NT * 16;         // bytes of a CTA's sums
+        asm volatile("barrier.cluster.wait;" ::: "memory");
+        if (rank) {
+#pragma unroll
+            for (int m = 0; m < MB; ++m)
+#pragma unroll
+                for (int j = 0; j < NT; ++j)
+                    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(map_rank(mine + (rank - 1) * PER, 0) + (m * NT + j) * 16),
+                                 "f"(acc[m][j][0]), "f"(acc[m][j][1]), "f"(acc[m][j][2]), "f"(acc[m][j][3]) : "memory");
+        }
+        cluster_sync();
+        if (rank) return;
+        for (int o = 0; o < share - 1; ++o)
+#pragma unroll
+            for (int m = 0; m < MB; ++m)
+#pragma unroll
+                for (int j = 0; j < NT; ++j) {
+                    const float4 v = *reinterpret_cast<const float4*>(smem + SM::SUMS + o * PER + tid * (MB * NT * 16) + (m * NT + j) * 16);
+                    acc[m][j][0] += v.x; acc[m][j][1] += v.y; acc[m][j][2] += v.z; acc[m][j][3] += v.w;
+                }
+    }
     add_norm(acc, p.n2_w, p.n2_eps);
     for (int i = tid; i < n * (BT_C / 8); i += 256) {
         const int r = i / (BT_C / 8), v = i % (BT_C / 8);
@@ -303,13 +339,36 @@ __global__ void __launch_bounds__(BT_THREADS, 1) block_tail_kernel(const __grid_
 }
 
 template <typename T, int RB, int WR> int bt_launch(const BtMaps& maps, const BtParams& p, cudaStream_t st) {
-    auto k = block_tail_kernel<T, RB, WR>;
-    const cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(k), (int)BtSmem<RB>::BYTES);
+    auto k = block_tail_kernel<T, RB, WR, false>;
+    const cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(k), (int)BtSmem<RB, false>::BYTES);
     if (e != cudaSuccess) return (int)e;
-    return (int)launch_chained(k, dim3((unsigned)((p.M + 16 * RB - 1) / (16 * RB))), dim3(BT_THREADS), BtSmem<RB>::BYTES, st, maps, p);
+    return (int)launch_chained(k, dim3((unsigned)((p.M + 16 * RB - 1) / (16 * RB))), dim3(BT_THREADS), BtSmem<RB, false>::BYTES, st, maps, p);
+}
+
+// a cluster of ``share`` CTAs a tile of 16 tokens
+template <typename T> int bt_launch_shared(const BtMaps& maps, const BtParams& p, int share, cudaStream_t st) {
+    auto k = block_tail_kernel<T, 1, 1, true>;
+    const cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(k), (int)BtSmem<1, true>::BYTES);
+    if (e != cudaSuccess) return (int)e;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)((p.M + 15) / 16 * share)); cfg.blockDim = dim3(BT_THREADS); cfg.dynamicSmemBytes = BtSmem<1, true>::BYTES; cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = share; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = chain_launches ? 2 : 1;
+    const cudaError_t r = cudaLaunchKernelEx(&cfg, k, maps, p);
+    return (int)(r != cudaSuccess ? r : cudaGetLastError());
 }
 
 template <typename T> int bt_dispatch(const BtMaps& maps, const BtParams& p, cudaStream_t st) {
+    // A tile's CTAs: as many as leave the call in one wave (clusters do not fill every group of SMs, hence seven eighths of the GPU) and have a
+    // chunk of features each.
+    const int tiles = (p.M + 15) / 16;
+    for (int share = BT_CLUSTER; share >= 2; share /= 2)
+        if (tiles * share * 8 <= device_sms() * 7 && p.I / 64 >= share) return bt_launch_shared<T>(maps, p, share, st);
     // the smallest row tile that is one wave of CTAs; beyond that the largest
     if (p.M <= device_sms() * 16) return bt_launch<T, 1, 1>(maps, p, st);
     if (p.M <= device_sms() * 32) return bt_launch<T, 2, 1>(maps, p, st);

@@ -112,6 +112,7 @@ __device__ __forceinline__ void tc_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint
 // ---- CTA pairs (cta_group::2): the two CTAs of a cluster work on one tile.  Each loads its half of the rows of A and of B into its own
 // shared memory at the same offsets, the even CTA issues the MMAs, each CTA's tensor memory holds its 128 rows of the result.
 __device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ uint32_t cluster_size() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(r)); return r; }
 // the same shared-memory offset in CTA ``rank`` of the cluster
 __device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
     uint32_t r;
