@@ -1,5 +1,5 @@
 """The row-local half of a block as one kernel (vig_block_tail_fwd) against the separate kernels it stands for, at the edges of
-its 16-, 32- and 64-token tiles, of the clusters of 8, 4 and 2 that share one, and of the rule that picks them."""
+its 16-, 32- and 64-token tiles, of the clusters of 4 and 2 that share one, and of the rule that picks them."""
 import pytest
 import torch
 

@@ -8,7 +8,7 @@
 // intermediates in shared memory; the three weight matrices (664 KB) stream from L2 through a ring of 24 KB stages in the
 // order they are used, and do not wait for the preceding kernel.  Bound: the stream for R = 16 (one CTA draws about 120 B/ns
 // from L2: 5.5 us), the mma.sync rate for R = 64 (21 M multiply-adds per CTA at 1024 a cycle: 11 us); R is the smallest that
-// keeps the call in one wave of CTAs.  Where 16-token tiles leave most SMs idle, a cluster of 2, 4 or 8 CTAs shares a tile: each does
+// keeps the call in one wave of CTAs.  Where 16-token tiles leave most SMs idle, a cluster of 2 or 4 CTAs shares a tile: each does
 // the injection and the output projection for itself (72 KB) and its part of the MLP's features, and the first one adds up the
 // others' down projections, which they write into its shared memory in fp32.  Large calls run the tcgen05 kernels, whose MMAs are three times faster per SM.
 //
@@ -44,10 +44,10 @@ template <> __device__ __forceinline__ void mma_t<__half>(float* c, const uint32
 }
 __device__ __forceinline__ void bt_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
-constexpr int BT_CLUSTER = 8;                             // largest cluster of a tile
+constexpr int BT_CLUSTER = 4;                             // largest cluster of a tile
 
 template <int RB, bool CL> struct BtSmem {
-    static constexpr int NST = CL ? 4 : RB == 1 ? 7 : RB == 2 ? 6 : 4;    // what the token tiles (and partial sums) leave of the 227 KB
+    static constexpr int NST = CL ? 6 : RB == 1 ? 7 : RB == 2 ? 6 : 4;    // what the token tiles (and partial sums) leave of the 227 KB
     static constexpr uint32_t R = 16 * RB, RING = 0, A = RING + NST * BT_STAGE, RES = A + R * BT_PA, Z = RES + R * BT_PA, PART = Z + R * BT_PZ,
                               SUMS = PART + R * 8 * 4,
                               BAR = SUMS + (CL ? (BT_CLUSTER - 1) * R * BT_C * 4 : 0), BYTES = BAR + 2 * NST * 8 + 16 + 1024;
@@ -365,7 +365,9 @@ template <typename T> int bt_launch_shared(const BtMaps& maps, const BtParams& p
 
 template <typename T> int bt_dispatch(const BtMaps& maps, const BtParams& p, cudaStream_t st) {
     // A tile's CTAs: as many as leave the call in one wave (clusters do not fill every group of SMs, hence seven eighths of the GPU) and have a
-    // chunk of features each.
+    // chunk of features each.  Whole forwards of ViG-T in us with 1 / 2 / 4 / 8 of them: 64 tokens 284 / 266 / 256 / 266, 196 tokens 331 / 313 / 297 / 312 (eight
+    // start and meet later), 392 tokens 334 / 317 / 302, 588 tokens 339 / 321 / 386 (148 CTAs in fours are two waves), 980 tokens 345 / 336; with six ring
+    // stages instead of four, which clusters of four leave room for, 249, 290, 300, 314 and 330.
     const int tiles = (p.M + 15) / 16;
     for (int share = BT_CLUSTER; share >= 2; share /= 2)
         if (tiles * share * 8 <= device_sms() * 7 && p.I / 64 >= share) return bt_launch_shared<T>(maps, p, share, st);
