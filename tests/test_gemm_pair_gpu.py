@@ -64,15 +64,25 @@ def test_projection_add_norm(dtype, M, K, N, with_res):
     assert float((h.double() - norm).norm() / norm.norm()) < TOL[dtype]
 
 
-def test_a_hooked_norm_runs_by_itself():
-    """Hooks on a wide block's projections and norms see their calls also where one kernel would take their place."""
+@pytest.mark.parametrize("name", ["vig_t", "vig_s"])
+@pytest.mark.parametrize("pick", [lambda m: m.blocks[0].mlp_norm, lambda m: m.blocks[1].attn.o_proj, lambda m: m.blocks[1].mlp, lambda m: m.blocks[0].attn,
+                                  lambda m: m.norm, lambda m: m.patch_embed], ids=["mlp_norm", "o_proj", "mlp", "attn", "norm", "patch_embed"])
+def test_a_hooked_module_runs_by_itself(name, pick):
+    """A hook on a module that one kernel would stand for sees what the module gives, and what it returns instead is taken."""
     import vig_b200
-    model = vig_b200.build_vig("vig_s", num_classes=10).cuda().bfloat16().eval()
+    model = vig_b200.ViG(depth=3, **vig_b200.vig._PRESETS[name], num_classes=10).cuda().bfloat16().eval()
     x = torch.randn(2, 3, 64, 64, device="cuda").bfloat16()
+    seen = []
+
+    def half(m, i, o):
+        seen.append((o[0] if isinstance(o, tuple) else o).float())
+        return (o[0] * 0.5, *o[1:]) if isinstance(o, tuple) else o * 0.5
+
     with torch.no_grad():
-        ref, seen = model(x), []
-        model.blocks[0].mlp_norm.register_forward_hook(lambda m, i, o: seen.append("norm"))
-        model.blocks[1].attn.o_proj.register_forward_hook(lambda m, i, o: seen.append("proj"))
+        plain = model(x)
+        pick(model).register_forward_hook(half)
         got = model(x)
-    assert seen == ["norm", "proj"]
-    assert float((ref.float() - got.float()).norm() / ref.float().norm()) < 2e-2
+        model.fuse_norm_epilogues = False
+        want = model(x)
+    assert len(seen) == 2 and float((seen[0] - seen[1]).norm() / seen[1].norm()) < 2e-2
+    assert float((got.float() - want.float()).norm() / want.float().norm()) < 2e-2 and not torch.equal(got, plain)

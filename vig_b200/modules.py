@@ -126,17 +126,17 @@ class GatedLinearAttention(nn.Module):
         return self.o_proj(y)
 
 
+def as_built(m, cls):
+    """Whether calling ``m`` runs ``cls.forward`` and nothing else, so that its work may be done without the call: no subclass, no
+    ``forward`` of its own, no hooks."""
+    g = nn.modules.module
+    return (type(m) is cls and "forward" not in m.__dict__ and
+            not (m._forward_hooks or m._forward_pre_hooks or g._global_forward_hooks or g._global_forward_pre_hooks))
+
+
 def plain_linear(m):
     """Whether calling ``m`` is the product with its weight and nothing else, so that a fused kernel may take its place."""
-    g = nn.modules.module
-    return (type(m) is nn.Linear and m.bias is None and "forward" not in m.__dict__ and
-            not (m._forward_hooks or m._forward_pre_hooks or g._global_forward_hooks or g._global_forward_pre_hooks))
-
-
-def plain_norm(m):
-    g = nn.modules.module
-    return (type(m) is RMSNorm and "forward" not in m.__dict__ and
-            not (m._forward_hooks or m._forward_pre_hooks or g._global_forward_hooks or g._global_forward_pre_hooks))
+    return as_built(m, nn.Linear) and m.bias is None
 
 
 class GLAMLP(nn.Module):
@@ -183,13 +183,20 @@ class GLABlock(nn.Module):
         h, residual = self.forward_deferred(hidden_states, None, **kwargs)
         return (residual + h,)
 
+    def unchanged(self):
+        """Whether ``forward_prenormed`` may stand for ``forward_deferred``: what that one calls, or reads the weights of, is what
+        the constructor put there, without hooks."""
+        return (type(self).forward_deferred is GLABlock.forward_deferred and "forward_deferred" not in self.__dict__ and
+                as_built(self.attn_norm, RMSNorm) and as_built(self.attn, GatedLinearAttention) and plain_linear(self.attn.o_proj) and
+                as_built(self.mlp_norm, RMSNorm) and as_built(self.mlp, GLAMLP) and plain_linear(self.mlp.down_proj))
+
     def fused_epilogues_supported(self, x):
         """True when both projections of the block can run with the residual add and the following RMSNorm as their
-        epilogue (``ops.linear_add_rmsnorm``: 16-bit CUDA tensors, plain projections)."""
+        epilogue (``ops.linear_add_rmsnorm``: 16-bit CUDA tensors, the block's own modules)."""
+        if not self.unchanged():
+            return False
         o, down = self.attn.o_proj, self.mlp.down_proj
-        wide = x.shape[-1] > 192                              # rows of up to 192 values look at the biases only
-        return (o.bias is None and down.bias is None and not (wide and not (plain_linear(o) and plain_linear(down) and plain_norm(self.attn_norm) and plain_norm(self.mlp_norm))) and
-                ops.linear_add_rmsnorm_supported(x, o.weight) and x.shape[-1] == down.weight.shape[0] and down.weight.shape[1] % 64 == 0)
+        return ops.linear_add_rmsnorm_supported(x, o.weight) and x.shape[-1] == down.weight.shape[0] and down.weight.shape[1] % 64 == 0
 
     @staticmethod
     def _project(y, linear, residual, norm):

@@ -57,18 +57,21 @@ def _attn(a):
 
 
 def _vig(model):
+    # every module is of a known class, but one may be in the place of another
+    if not (type(model.patch_embed) is vig.V2PatchEmbed and modules.as_built(model.norm, modules.RMSNorm) and
+            all(type(b) is modules.GLABlock and b.unchanged() for b in model.blocks)):
+        return None
     pe, conv1 = model.patch_embed, model.patch_embed.proj[0]
     if pe.stride != 8 or conv1.weight.shape[1] != 3 or not isinstance(model.head, nn.Linear) or not len(model.blocks):
         return None
     blocks = []
     for b in model.blocks:
         attn = _attn(b.attn)
-        if attn is None or b.mlp.down_proj.bias is not None or b.mlp.gate_proj.bias is not None:
+        if attn is None or b.mlp.gate_proj.bias is not None:
             return None
         blocks.append(dict(n1=b.attn_norm.weight, e1=b.attn_norm.eps, n2=b.mlp_norm.weight, e2=b.mlp_norm.eps, gate_w=b.mlp.gate_proj.weight,
                            down_w=b.mlp.down_proj.weight, attn=attn))
-    probe = model.head.weight.new_empty(1, 1, model.embed_dim)
-    fused = model.fuse_norm_epilogues and all(b.fused_epilogues_supported(probe) for b in model.blocks)
+    fused = model.fused_norms(model.head.weight)
     one_kernel = pe.fuse_conv1 and conv1.weight.shape[0] == 96
     ref = weakref.ref(model)
     return _lib.host().VigPlan(dict(

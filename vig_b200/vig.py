@@ -12,7 +12,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from .modules import GLABlock, RMSNorm
+from .modules import GLABlock, RMSNorm, as_built
 
 
 class LayerNorm2d(nn.LayerNorm):
@@ -179,13 +179,19 @@ class ViG(nn.Module):
             self._pos_cache = {key: resize_pos_embed(self.pos_embed.detach(), self.patch_resolution, hw)}
         return self._pos_cache[key]
 
-    def forward_features(self, x):
-        # ``fuse_norm_epilogues``: every residual add + RMSNorm runs as the epilogue of the projection in front of it
-        # (hidden size <= 192, 16-bit tensors; measured 74 + 104 us against 112 + 141 us for cuBLAS + the norm kernel),
-        # and the first block's norm comes out of the stem's last kernel.
-        from . import ops
+    def fused_norms(self, x):
+        """Whether the forward takes the fused path: every residual add + RMSNorm of ``forward_features`` is handed to the step in front
+        of it, so none of the modules concerned is called as it stands."""
         probe = x.new_empty(1, 1, self.embed_dim)
-        if self.fuse_norm_epilogues and len(self.blocks) and all(blk.fused_epilogues_supported(probe) for blk in self.blocks):
+        return bool(self.fuse_norm_epilogues and len(self.blocks) and as_built(self.patch_embed, V2PatchEmbed) and as_built(self.norm, RMSNorm) and
+                    all(blk.fused_epilogues_supported(probe) for blk in self.blocks))
+
+    def forward_features(self, x):
+        # Fused: the first block's norm comes out of the stem's last kernel, every other one with its residual add out of the projection in
+        # front of it -- one kernel or GEMM + norm, chosen by width and rows (``vig_linear_add_rmsnorm_preferred``; rows of up to 192 values
+        # always one: 74 + 104 us against 112 + 141 us for 262144 of 192).
+        from . import ops
+        if self.fused_norms(x):
             x, hw, h = self.patch_embed(x, pos_fn=self._pos, next_norm=self.blocks[0].attn_norm)
             residual = x
             for i, blk in enumerate(self.blocks):
