@@ -319,7 +319,10 @@ __global__ void __launch_bounds__(BT_THREADS, 1) block_tail_kernel(const __grid_
                                  "f"(acc[m][j][0]), "f"(acc[m][j][1]), "f"(acc[m][j][2]), "f"(acc[m][j][3]) : "memory");
         }
         cluster_sync();
-        if (rank) return;
+        if (rank) {                                          // a wait of this CTA that ran out made its sums wrong
+            if (tid == 0 && *abort_flag && p.status) atomicOr(p.status, 1);
+            return;
+        }
         for (int o = 0; o < share - 1; ++o)
 #pragma unroll
             for (int m = 0; m < MB; ++m)
