@@ -86,3 +86,45 @@ def test_a_hooked_module_runs_by_itself(name, pick):
         want = model(x)
     assert len(seen) == 2 and float((seen[0] - seen[1]).norm() / seen[1].norm()) < 2e-2
     assert float((got.float() - want.float()).norm() / want.float().norm()) < 2e-2 and not torch.equal(got, plain)
+
+
+def _off16(t):
+    """The same values two bytes off a 16-byte boundary, as a view into a flat buffer has them."""
+    flat = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+    return flat[1:].view(t.shape).copy_(t)
+
+
+@pytest.mark.parametrize("name,size,batch", [("vig_t", 64, 2), ("vig_t", 224, 52), ("vig_s", 224, 106), ("vig_b", 64, 2)])
+def test_matrices_off_16_bytes(name, size, batch):
+    """Matrices that TMA cannot read go to the library's GEMM, from the modules and from the C++ forward, one at a time."""
+    import vig_b200
+    from vig_b200 import native
+    model = vig_b200.ViG(depth=1, **vig_b200.vig._PRESETS[name], num_classes=10).cuda().bfloat16().eval().requires_grad_(False)
+    x = torch.randn(batch, 3, size, size, device="cuda").bfloat16()
+    blk = model.blocks[0]
+    with torch.no_grad():
+        ref = model(x).float()
+        for linear in (blk.attn.o_proj, blk.mlp.gate_proj, blk.mlp.down_proj):
+            keep = linear.weight.data
+            linear.weight.data = _off16(keep)
+            assert linear.weight.data_ptr() % 16
+            got = native.vig_forward(model, x)
+            assert got is not None
+            for y in (got, model.head(model.forward_features(x))):
+                assert float((y.float() - ref).norm() / ref.norm()) < 1e-2
+            linear.weight.data = keep
+
+
+def test_rows_off_16_bytes():
+    """Inputs of an MLP by itself that TMA cannot read: off 16 bytes, an odd row stride, one row for all."""
+    import vig_b200
+    mlp = vig_b200.modules.GLAMLP(384).cuda().bfloat16().requires_grad_(False)
+    x = torch.randn(2, 2048, 384, device="cuda").bfloat16()
+    wide = torch.empty(2, 2048, 387, device="cuda", dtype=torch.bfloat16)
+    wide[..., :384] = x
+    with torch.no_grad():
+        ref = mlp(x).float()
+        for y in (_off16(x), wide[..., :384]):
+            assert float((mlp(y).float() - ref).norm() / ref.norm()) < 1e-2
+        one = mlp(x[:1, :1].expand(1, 4096, 384)).float()
+        assert float((one - ref[:1, :1]).norm() / one.norm()) < 1e-2

@@ -52,11 +52,13 @@ Tensor token_mean(const Ctx& c, const Tensor& x) {
     ok(api.vig_token_mean_fwd(ptr(x), ptr(y), x.size(0), x.size(1), x.size(2), c.code, c.stream), "vig_token_mean_fwd");
     return y;
 }
+// a matrix that TMA can read; the GEMM library takes others too
+bool on16(const Tensor& w) { return (reinterpret_cast<uintptr_t>(ptr(w)) & 15) == 0; }
 // swiglu(x W^T): one kernel where it is the faster one, GEMM + activation kernel otherwise
 Tensor mlp_in(const Ctx& c, const Tensor& x, const Tensor& w) {
     const int64_t K = x.size(-1), I = w.size(0) / 2, M = x.numel() / K;
     Tensor out = at::empty({x.size(0), x.size(1), I}, x.options());
-    if (api.vig_linear_swiglu_preferred(M, K, I, c.code)) {
+    if (on16(w) && api.vig_linear_swiglu_preferred(M, K, I, c.code)) {
         ok(api.vig_linear_swiglu_fwd(ptr(x), K, ptr(w), ptr(out), I, M, K, I, c.code, c.status, c.stream), "vig_linear_swiglu_fwd");
         return out;
     }
@@ -67,7 +69,7 @@ Tensor mlp_in(const Ctx& c, const Tensor& x, const Tensor& w) {
 // r = x W^T + residual, h = RMSNorm(r): one kernel where it is the faster one
 std::pair<Tensor, Tensor> linear_add_rmsnorm(const Ctx& c, const Tensor& x, const Tensor& w, const Tensor& res, const Tensor& nw, double eps) {
     const int64_t K = x.size(-1), N = w.size(0), M = x.numel() / K;
-    if (!api.vig_linear_add_rmsnorm_preferred(M, K, N, c.code)) return add_rmsnorm(c, at::linear(x, w), nw, res, eps, true);
+    if (!on16(w) || !api.vig_linear_add_rmsnorm_preferred(M, K, N, c.code)) return add_rmsnorm(c, at::linear(x, w), nw, res, eps, true);
     Tensor h = at::empty({x.size(0), x.size(1), N}, x.options()), r = at::empty({x.size(0), x.size(1), N}, x.options());
     ok(api.vig_linear_add_rmsnorm_fwd(ptr(x), K, ptr(w), ptr(res), ptr(nw), ptr(r), ptr(h), M, K, N, (float)eps, c.code, c.status, c.stream), "vig_linear_add_rmsnorm_fwd");
     return {h, r};
@@ -421,7 +423,7 @@ struct VigPlan : PlanBase {
                 const int64_t I = b.down_w.size(1);
                 const Tensor& next_w = last ? norm_w : blocks[i + 1].n1;
                 const double next_e = last ? norm_e : blocks[i + 1].e1;
-                if (api.vig_block_tail_preferred(rows, b.attn.H, b.attn.dv, I, c.code)) {
+                if (on16(b.attn.o_w) && on16(b.gate_w) && on16(b.down_w) && api.vig_block_tail_preferred(rows, b.attn.H, b.attn.dv, I, c.code)) {
                     const auto [o, xs, z] = b.attn.scan(c, n, h, w);
                     Tensor r = at::empty_like(tok), hn = at::empty_like(tok);
                     ok(api.vig_block_tail_fwd(ptr(o), ptr(xs), b.attn.gate_logits(z), z.size(2), ptr(b.attn.gn_w), ptr(b.attn.ln_w), (float)b.attn.eps, b.attn.out_act,

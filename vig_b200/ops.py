@@ -451,10 +451,22 @@ def embed_conv_ln(x, weight, conv_bias, ln_weight, ln_bias, eps=1e-5, act_gelu=T
     return y
 
 
+def _rows_on_16(x, K):
+    """Whether the ``[M, K]`` rows of a 16-bit ``x`` begin on 16 bytes, as the copies to shared memory want them; rows that have to be
+    gathered into a copy do."""
+    try:
+        rows = x.view(-1, K)
+    except RuntimeError:
+        return True
+    return rows.stride(1) != 1 or (x.data_ptr() % 16 == 0 and rows.stride(0) >= K and rows.stride(0) % 8 == 0)
+
+
 def linear_add_rmsnorm_supported(x, w, preferred=False):
-    """True when ``linear_add_rmsnorm`` can run on these operands (16-bit CUDA tensors, K % 64 == 0, N in {64, 128, 192, 256, 384, 768});
+    """True when ``linear_add_rmsnorm`` can run on these operands (16-bit CUDA tensors on 16 bytes, K % 64 == 0, N in {64, 128, 192, 256, 384, 768});
     with ``preferred`` also that it is to be taken instead of the library's GEMM and the norm kernel."""
     if not (x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and w.dtype == x.dtype and x.stride(-1) == 1):
+        return False
+    if not _rows_on_16(x, w.shape[1]) or (w.is_contiguous() and w.data_ptr() % 16):
         return False
     N, K = w.shape
     M = x.numel() // K
@@ -578,14 +590,14 @@ def block_tail(o, local, gate_logits, w_gnorm, w_lnorm, w_o, residual, norm_w, w
 
 
 def linear_swiglu_supported(x, weight, preferred=False):
-    """True when ``linear_swiglu`` has a fused kernel for this input (bf16 / fp16, K % 64 == 0, I % 64 == 0); with
+    """True when ``linear_swiglu`` has a fused kernel for this input (bf16 / fp16 on 16 bytes, K % 64 == 0, I % 64 == 0); with
     ``preferred`` also that it is taken instead of the library GEMM followed by the SwiGLU kernel (K <= 192, or rows enough)."""
     if not x.is_cuda or x.dtype not in (torch.bfloat16, torch.float16) or weight.dtype != x.dtype:
         return False
     K, I = x.shape[-1], weight.shape[0] // 2
     L_ = _lib.lib()
     fn = L_.vig_linear_swiglu_preferred if preferred else L_.vig_linear_swiglu_supported
-    return weight.is_contiguous() and bool(fn(x.numel() // K, K, I, _lib.dtype_code(x)))
+    return weight.is_contiguous() and weight.data_ptr() % 16 == 0 and _rows_on_16(x, K) and bool(fn(x.numel() // K, K, I, _lib.dtype_code(x)))
 
 
 def linear_swiglu(x, weight):
