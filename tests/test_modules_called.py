@@ -6,8 +6,16 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 import vig_b200
+from torch.utils._python_dispatch import _disable_current_modes
+
 from vig_b200 import modules, ops
 from vig_b200.vig import V2PatchEmbed
+
+
+def _kernel_product(x, w):
+    """What a fused kernel makes of the bytes it is given; neither a tensor's own operators nor a mode sees it."""
+    with _disable_current_modes(), torch._C.DisableTorchFunctionSubclass():
+        return x @ w.as_subclass(torch.Tensor).t()
 
 
 def _rms(x, w, eps):
@@ -29,7 +37,11 @@ def plain_ops(monkeypatch):
         return (_rms(r, weight, eps), r) if prenorm else _rms(r, weight, eps)
 
     def linear_add_rmsnorm(x, w, residual, norm_weight, eps=1e-6):
-        return add_rmsnorm(F.linear(x, w), norm_weight, residual, eps, True)
+        return add_rmsnorm(_kernel_product(x, w), norm_weight, residual, eps, True)
+
+    def linear_swiglu(x, w):
+        gate, y = _kernel_product(x, w).chunk(2, -1)
+        return F.silu(gate) * y
 
     def layernorm_act(x, weight, bias, eps=1e-5, act_swish=False, pre_bias=None, post_add=None, rms_weight=None, rms_eps=1e-6):
         y = F.layer_norm(x if pre_bias is None else x + pre_bias, x.shape[-1:], weight, bias, eps)
@@ -46,13 +58,12 @@ def plain_ops(monkeypatch):
     monkeypatch.setattr(ops, "status_word", lambda device: _Status())
     monkeypatch.setattr(ops, "linear_add_rmsnorm_supported", lambda x, w, preferred=False: True)
     monkeypatch.setattr(ops, "linear_swiglu_supported", lambda x, w, preferred=False: True)
-    monkeypatch.setattr(ops, "linear_swiglu", lambda x, w: F.silu(F.linear(x, w).chunk(2, -1)[0]) * F.linear(x, w).chunk(2, -1)[1])
     monkeypatch.setattr(ops, "swiglu", lambda g, y: F.silu(g) * y)
     monkeypatch.setattr(ops, "dwconv3x3", lambda x, taps, bias, hw, act: F.silu(x * taps[4]))
     monkeypatch.setattr(ops, "token_mean", lambda x: x.mean(1))
     monkeypatch.setattr(ops, "stem_unfold", lambda x, s: F.pad(x.permute(0, 2, 3, 1), (0, 0, 1, s - 1, 1, s - 1)).unflatten(1, (-1, s)).unflatten(3, (-1, s))
                         .permute(0, 1, 3, 2, 4, 5).flatten(3))
-    for f in (add_rmsnorm, linear_add_rmsnorm, layernorm_act, bi_gla, gate_inject):
+    for f in (add_rmsnorm, linear_add_rmsnorm, linear_swiglu, layernorm_act, bi_gla, gate_inject):
         monkeypatch.setattr(ops, f.__name__, f)
 
 
@@ -111,6 +122,22 @@ def _replace(owner, name, make):
     return put
 
 
+class Doubled(torch.Tensor):
+    """A weight with a product of its own."""
+
+    @classmethod
+    def __torch_function__(cls, func, types, args=(), kwargs=None):
+        out = super().__torch_function__(func, types, args, kwargs or {})
+        return (out * 2).as_subclass(torch.Tensor) if func is F.linear else out
+
+
+def _own_product(pick):
+    def put(model):
+        linear = pick(model)
+        linear.weight = nn.Parameter(linear.weight.detach().as_subclass(Doubled), requires_grad=False)
+    return put
+
+
 def _own_forward(model):
     mlp = model.blocks[0].mlp
     mlp.forward = lambda x: x * 0.25
@@ -126,6 +153,9 @@ REPLACED = {
     "final norm": _replace(lambda m: m, "norm", lambda m: Sign(m.embed_dim)),
     "attention norm": _replace(lambda m: m.blocks[1], "attn_norm", lambda m: Sign(m.embed_dim)),
     "MLP norm": _replace(lambda m: m.blocks[1], "mlp_norm", lambda m: Sign(m.embed_dim)),
+    "output weight": _own_product(lambda m: m.blocks[0].attn.o_proj),
+    "gate weight": _own_product(lambda m: m.blocks[1].mlp.gate_proj),
+    "down weight": _own_product(lambda m: m.blocks[1].mlp.down_proj),
 }
 HOOKED = {
     "attention": lambda m: m.blocks[0].attn, "output projection": lambda m: m.blocks[1].attn.o_proj, "mlp": lambda m: m.blocks[1].mlp,

@@ -135,8 +135,9 @@ def as_built(m, cls):
 
 
 def plain_linear(m):
-    """Whether calling ``m`` is the product with its weight and nothing else, so that a fused kernel may take its place."""
-    return as_built(m, nn.Linear) and m.bias is None
+    """Whether calling ``m`` is the product with its weight and nothing else, so that a fused kernel may take its place.  A tensor of
+    another kind (quantised, wrapped) brings a product of its own."""
+    return as_built(m, nn.Linear) and m.bias is None and type(m.weight) in (nn.Parameter, torch.Tensor)
 
 
 class GLAMLP(nn.Module):

@@ -119,7 +119,7 @@ def _build(model, make):
     if not (model.training or any(getattr(nn.modules.module, name) for name in _GLOBAL_HOOKS) or any(type(m) not in _CLASSES or "forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks for m in mods)):
         params = [p for m in mods for p in m._parameters.values() if p is not None]
         # vectors and matrices go to kernels by address, filters to the library, which takes any strides
-        if all(p.dtype == params[0].dtype and p.device == params[0].device and (p.dim() == 4 or p.is_contiguous()) for p in params):
+        if all(type(p) in (nn.Parameter, torch.Tensor) and p.dtype == params[0].dtype and p.device == params[0].device and (p.dim() == 4 or p.is_contiguous()) for p in params):
             try:
                 with torch.no_grad():
                     plan = make(model)
