@@ -6,7 +6,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 import vig_b200
-from torch.utils._python_dispatch import _disable_current_modes
+from torch.utils._python_dispatch import TorchDispatchMode, _disable_current_modes
 
 from vig_b200 import modules, ops
 from vig_b200.vig import V2PatchEmbed
@@ -202,3 +202,28 @@ def test_hooks_see_and_replace_the_outputs(plain_ops, width):
             assert len(seen) == 2, name
             torch.testing.assert_close(seen[0], seen[1], rtol=1e-4, atol=1e-5, msg=name)
             torch.testing.assert_close(got, want, rtol=1e-4, atol=1e-5, msg=name)
+
+
+class Products(TorchDispatchMode):
+    seen = 0
+
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        self.seen += "mm" in str(func)
+        return func(*args, **(kwargs or {}))
+
+
+@pytest.mark.parametrize("width", [256, 384, 768])
+def test_modes_see_the_products(plain_ops, width):
+    """A mode that counts operators sees the four products of each block and the classifier's."""
+    model = _model(width)
+    x = torch.randn(2, 3, 32, 48)
+    with torch.no_grad():
+        ref = model(x)
+        with Products() as p:
+            y = model(x)
+        assert p.seen >= 4 * 2 + 1
+        torch.testing.assert_close(y, ref, rtol=1e-4, atol=1e-5)
+        mlp = vig_b200.hier.gMlp(width)
+        with Products() as p:
+            mlp(torch.randn(2, 6, width))
+        assert p.seen == 2

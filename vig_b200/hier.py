@@ -15,7 +15,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import ops
-from .modules import GatedLinearAttention, plain_linear
+from .modules import GatedLinearAttention, plain_linear, products_watched
 
 
 class GLA2D(GatedLinearAttention):
@@ -66,7 +66,7 @@ class gMlp(nn.Module):
         self.fc2 = nn.Linear(self.intermediate_size, in_features, bias=False)
 
     def forward(self, x):
-        if plain_linear(self.fc1) and ops.linear_swiglu_supported(x, self.fc1.weight, preferred=True):
+        if plain_linear(self.fc1) and not products_watched(x.shape[-1]) and ops.linear_swiglu_supported(x, self.fc1.weight, preferred=True):
             return self.fc2(ops.linear_swiglu(x, self.fc1.weight))
         gate, y = self.fc1(x).chunk(2, -1)
         return self.fc2(ops.swiglu(gate, y))

@@ -12,7 +12,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from .modules import GLABlock, RMSNorm, as_built
+from .modules import GLABlock, RMSNorm, as_built, products_watched
 
 
 class LayerNorm2d(nn.LayerNorm):
@@ -191,7 +191,7 @@ class ViG(nn.Module):
         # front of it -- one kernel or GEMM + norm, chosen by width and rows (``vig_linear_add_rmsnorm_preferred``; rows of up to 192 values
         # always one: 74 + 104 us against 112 + 141 us for 262144 of 192).
         from . import ops
-        if self.fused_norms(x):
+        if self.fused_norms(x) and not products_watched(self.embed_dim):
             x, hw, h = self.patch_embed(x, pos_fn=self._pos, next_norm=self.blocks[0].attn_norm)
             residual = x
             for i, blk in enumerate(self.blocks):
