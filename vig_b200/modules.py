@@ -193,17 +193,20 @@ class GLABlock(nn.Module):
     def unchanged(self):
         """Whether ``forward_prenormed`` may stand for ``forward_deferred``: what that one calls, or reads the weights of, is what
         the constructor put there, without hooks."""
+        attn, mlp = self.attn, self.mlp
         return (type(self).forward_deferred is GLABlock.forward_deferred and "forward_deferred" not in self.__dict__ and
-                as_built(self.attn_norm, RMSNorm) and as_built(self.attn, GatedLinearAttention) and plain_linear(self.attn.o_proj) and
-                as_built(self.mlp_norm, RMSNorm) and as_built(self.mlp, GLAMLP) and plain_linear(self.mlp.down_proj))
+                as_built(self.attn_norm, RMSNorm) and as_built(attn, GatedLinearAttention) and plain_linear(attn.o_proj) and
+                as_built(self.mlp_norm, RMSNorm) and as_built(mlp, GLAMLP) and plain_linear(mlp.down_proj))
+
+    def epilogues_fit(self, x):
+        """Whether the widths and types of both projections are those of ``ops.linear_add_rmsnorm`` (16-bit CUDA tensors)."""
+        down = self.mlp.down_proj.weight
+        return ops.linear_add_rmsnorm_supported(x, self.attn.o_proj.weight) and x.shape[-1] == down.shape[0] and down.shape[1] % 64 == 0
 
     def fused_epilogues_supported(self, x):
         """True when both projections of the block can run with the residual add and the following RMSNorm as their
-        epilogue (``ops.linear_add_rmsnorm``: 16-bit CUDA tensors, the block's own modules)."""
-        if not self.unchanged():
-            return False
-        o, down = self.attn.o_proj, self.mlp.down_proj
-        return ops.linear_add_rmsnorm_supported(x, o.weight) and x.shape[-1] == down.weight.shape[0] and down.weight.shape[1] % 64 == 0
+        epilogue: the block's own modules, of widths and types that fit."""
+        return self.unchanged() and self.epilogues_fit(x)
 
     @staticmethod
     def _project(y, linear, residual, norm):

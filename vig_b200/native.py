@@ -57,21 +57,28 @@ def _attn(a):
 
 
 def _vig(model):
-    # every module is of a known class, but one may be in the place of another
-    if not (type(model.patch_embed) is vig.V2PatchEmbed and modules.as_built(model.norm, modules.RMSNorm) and
-            all(type(b) is modules.GLABlock and b.unchanged() for b in model.blocks)):
+    # every module is of a known class, without hooks or a forward of its own, but one may be in the place of another
+    if not (type(model.patch_embed) is vig.V2PatchEmbed and type(model.norm) is modules.RMSNorm):
         return None
     pe, conv1 = model.patch_embed, model.patch_embed.proj[0]
     if pe.stride != 8 or conv1.weight.shape[1] != 3 or not isinstance(model.head, nn.Linear) or not len(model.blocks):
         return None
     blocks = []
     for b in model.blocks:
-        attn = _attn(b.attn)
-        if attn is None or b.mlp.gate_proj.bias is not None:
+        if type(b) is not modules.GLABlock or "forward_deferred" in b.__dict__:
             return None
-        blocks.append(dict(n1=b.attn_norm.weight, e1=b.attn_norm.eps, n2=b.mlp_norm.weight, e2=b.mlp_norm.eps, gate_w=b.mlp.gate_proj.weight,
-                           down_w=b.mlp.down_proj.weight, attn=attn))
-    fused = model.fused_norms(model.head.weight)
+        a, mlp, n1, n2 = b.attn, b.mlp, b.attn_norm, b.mlp_norm
+        if type(a) is not modules.GatedLinearAttention or type(mlp) is not modules.GLAMLP or type(n1) is not modules.RMSNorm or type(n2) is not modules.RMSNorm:
+            return None
+        o, gate, down = a.o_proj, mlp.gate_proj, mlp.down_proj
+        if any(type(m) is not nn.Linear or m.bias is not None for m in (o, gate, down)):
+            return None
+        attn = _attn(a)
+        if attn is None:
+            return None
+        blocks.append(dict(n1=n1.weight, e1=n1.eps, n2=n2.weight, e2=n2.eps, gate_w=gate.weight, down_w=down.weight, attn=attn))
+    probe = model.head.weight.new_empty(1, 1, model.embed_dim)
+    fused = bool(model.fuse_norm_epilogues and all(b.epilogues_fit(probe) for b in model.blocks))
     one_kernel = pe.fuse_conv1 and conv1.weight.shape[0] == 96
     ref = weakref.ref(model)
     return _lib.host().VigPlan(dict(
