@@ -129,3 +129,20 @@ def test_rows_off_16_bytes():
             assert float((mlp(y).float() - ref).norm() / ref.norm()) < 1e-2
         one = mlp(x[:1, :1].expand(1, 4096, 384)).float()
         assert float((one - ref[:1, :1]).norm() / one.norm()) < 1e-2
+
+
+@pytest.mark.parametrize("N,K", [(256, 256), (256, 704), (384, 384), (384, 1024), (768, 768), (768, 2048)])
+def test_long_rows_are_counted_in_rounds(N, K):
+    """The one kernel works on as many tiles of 256 rows at a time as there are pairs of SMs (clusters of four for rows of 768): while rounds
+    are few it is taken for full ones and not for a single tile more; many rounds always are."""
+    import math
+
+    import vig_b200
+    lib = vig_b200._lib.lib()
+    bf16 = vig_b200._lib.dtype_code(torch.empty(0, dtype=torch.bfloat16))
+    takes = lambda tiles: bool(lib.vig_linear_add_rmsnorm_preferred(tiles * 256, K, N, bf16))  # noqa: E731
+    most = torch.cuda.get_device_properties(0).multi_processor_count // (4 if N == 768 else 2)
+    given_up = [t for t in range(1, 4 * most + 1) if takes(t) and not takes(t + 1)]
+    full = math.gcd(*given_up)
+    assert given_up and 0.75 * most <= full <= most
+    assert not takes(1) and all(takes(t) for t in range(40 * most, 44 * most))

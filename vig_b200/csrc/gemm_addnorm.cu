@@ -246,13 +246,20 @@ extern "C" int vig_linear_add_rmsnorm_supported(int64_t M, int K, int N, int dty
 }
 
 // Whether the one kernel is to be taken instead of the library's GEMM and the norm kernel.  Rows of up to 192 values always (17-22 % faster from
-// 50000 rows on).  Longer rows are 256-row tiles of CTA pairs, whose epilogue shows behind a last or only tile; measured (us, one kernel / two):
-// N = 384, K = 384: 12544 rows 13.9 / 13.5, 25088 21 / 26, 131072 92 / 111; K = 1024: 25088 36 / 33, 50176 57 / 60, 131072 130 / 146;
-// N = 768, K = 768: 12544 26 / 26, 25088 46 / 51, 131072 192 / 255; K = 2048: 25088 79 / 79, 50176 150 / 156, 131072 395 / 415;
-// N = 256, K = 256: 25088 16 / 14, 50176 25 / 27, 131072 54 / 65.
+// 50000 rows on).  Longer rows go in rounds of 256-row tiles, 74 pairs or 33 clusters of four at a time; a round costs about the same however
+// full it is, while the two kernels' time grows with the rows, so the line is how much of its rounds a call fills (tenths).  Measured (us, one kernel / two; f rounds filled):
+//   N = 384, K = 384:  f 0.65 13.6 / 13.6, 0.74 13.7 / 14.0, 1.05 20.4 / 19.7, 1.16 20.5 / 21.3, 1.32 21.0 / 25.6, 2.0 32.6 / 37.3  (rows in DRAM bound it: a round that follows is cheap)
+//   N = 384, K = 1024: f 0.85 19.5 / 21.5, 1.57 38.4 / 37.4, 1.69 39.3 / 40.3, 2.2 51.8 / 50.2, 2.4 52.5 / 55.4, 3.0 65.9 / 69.7
+//   N = 256, K = 256:  f 0.74 10.5 / 9.7, 0.95 10.7 / 11.1, 1.51 15.4 / 15.2, 1.69 15.6 / 17.0, 2.1 20.7 / 20.1, 2.4 21.6 / 23.1
+//   N = 256, K = 704:  f 0.95 13.2 / 13.7, 1.51 19.8 / 21.2, 2.1 30.6 / 28.0, 2.4 31.6 / 30.7, 2.5 32.6 / 33.9
+//   N = 768, K = 768:  f 0.76 16.3 / 14.6, 1.3 25.5 / 23.2, 1.67 26.8 / 29.1, 2.4 42.9 / 41.9, 2.6 43.8 / 45.9, 3.2 54.4 / 53.2, 3.4 55.0 / 59.4, 4.03 65.7 / 69.7
+//   N = 768, K = 2048: f 1.9 54.3 / 52.7, 2.6 75.5 / 73.2, 3.0 78.4 / 80.4, 3.4 97.0 / 97.3, 3.8 100 / 105, 9.1 267 / 252, 15.5 395 / 415
 extern "C" int vig_linear_add_rmsnorm_preferred(int64_t M, int K, int N, int dtype) {
     if (!vig_linear_add_rmsnorm_supported(M, K, N, dtype)) return 0;
-    return N <= 192 || M >= 40000 || (N >= 384 && K <= N && M >= 20000);
+    if (N <= 192) return 1;
+    const int64_t all = pair_norm_clusters(N, dtype), tiles = (M + 255) / 256, rounds = (tiles + all - 1) / all;
+    const int64_t tenths = N == 384 && K <= N ? 5 * rounds + 2 : K > (N == 768 ? 768 : 1024) ? 9 * rounds + 2 : N == 768 ? 8 * rounds + (rounds == 1) : 7 * rounds + 2;
+    return 10 * tiles >= all * tenths;
 }
 
 extern "C" int vig_linear_add_rmsnorm_fwd(const void* x, int64_t ldx, const void* w, const void* residual, const void* norm_weight,

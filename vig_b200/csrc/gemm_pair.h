@@ -9,5 +9,7 @@ int pair_swiglu_launch(const void* x, int64_t ldx, const void* w, void* out, int
 // rows of 256, 384 or 768 values
 int pair_norm_launch(const void* x, int64_t ldx, const void* w, const void* residual, const void* norm_w, void* out_r, void* out_h, int64_t M, int K, int N, float eps,
                      int dtype, int32_t* status, cudaStream_t stream);
+// tiles of 256 rows that the GPU works on at a time
+int pair_norm_clusters(int N, int dtype);
 
 }  // namespace vig

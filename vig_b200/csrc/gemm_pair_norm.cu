@@ -251,6 +251,29 @@ gemm_pair_norm_kernel(const __grid_constant__ NormMaps maps, bool has_res, const
     }
 }
 
+// Clusters at a time: pairs fill the GPU, clusters of four do not have to (33 of them on 148 SMs).
+template <typename T, int BN, int NP> int norm_clusters() {
+    using Cfg = NormCfg<BN, NP>;
+    if (NP == 1) return device_sms() / 2;
+    static std::atomic<int> known[64];
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return device_sms() / 4;
+    if ((n = known[dev & 63].load())) return n;
+    auto kfn = gemm_pair_norm_kernel<T, BN, NP>;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[1];
+    cfg.gridDim = dim3(2 * NP); cfg.blockDim = dim3(Cfg::THREADS); cfg.dynamicSmemBytes = Cfg::SMEM;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2 * NP; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    if (ensure_smem_attr(reinterpret_cast<const void*>(kfn), Cfg::SMEM) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, kfn, &cfg) != cudaSuccess || n < 1) {
+        cudaGetLastError();
+        n = device_sms() / 4;
+    }
+    known[dev & 63].store(n);
+    return n;
+}
+
 template <typename T, int BN, int NP>
 int norm_launch(const void* x, int64_t ldx, const void* w, const void* residual, const void* norm_w, void* out_r, void* out_h, int64_t M, int K, float eps,
                 int dtype, int32_t* status, cudaStream_t stream) {
@@ -261,28 +284,9 @@ int norm_launch(const void* x, int64_t ldx, const void* w, const void* residual,
         !make_map_2d(&maps.res, residual ? residual : out_r, M, N, N, 128, dtype) || !make_map_2d(&maps.r, out_r, M, N, N, 32, dtype) || !make_map_2d(&maps.h, out_h, M, N, N, 32, dtype))
         return VIG_ERR_DEVICE;
     auto kfn = gemm_pair_norm_kernel<T, BN, NP>;
-    cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(kfn), Cfg::SMEM);
+    const cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(kfn), Cfg::SMEM);
     if (e != cudaSuccess) return (int)e;
-    // clusters at a time: pairs fill the GPU, clusters of four do not have to
-    int64_t clusters = device_sms() / 2;
-    if (NP == 2) {
-        static std::atomic<int> known[64];
-        int dev = 0, n = 0;
-        if ((e = cudaGetDevice(&dev)) != cudaSuccess) return (int)e;
-        if (!(n = known[dev & 63].load())) {
-            cudaLaunchConfig_t cfg{};
-            cudaLaunchAttribute attr[1];
-            cfg.gridDim = dim3(2 * NP); cfg.blockDim = dim3(Cfg::THREADS); cfg.dynamicSmemBytes = Cfg::SMEM;
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = 2 * NP; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-            cfg.attrs = attr; cfg.numAttrs = 1;
-            if ((e = cudaOccupancyMaxActiveClusters(&n, kfn, &cfg)) != cudaSuccess || n < 1) { cudaGetLastError(); n = device_sms() / 4; }
-            known[dev & 63].store(n);
-        }
-        clusters = n;
-    }
-    const int64_t ntiles = (M + 255) / 256;
-    if (clusters > ntiles) clusters = ntiles;
+    const int64_t ntiles = (M + 255) / 256, all = norm_clusters<T, BN, NP>(), clusters = all < ntiles ? all : ntiles;
     return (int)launch_chained(kfn, dim3((unsigned)(2 * NP * clusters)), dim3(Cfg::THREADS), Cfg::SMEM, stream, maps, residual != nullptr, (const T*)norm_w, (int)M, K / PN_BK,
                                (int)ntiles, eps, status);
 }
@@ -299,6 +303,11 @@ int pair_norm_launch(const void* x, int64_t ldx, const void* w, const void* resi
     if (dtype == VIG_DTYPE_BF16) { VIG_PN(__nv_bfloat16) }
     VIG_PN(__half)
 #undef VIG_PN
+}
+
+int pair_norm_clusters(int N, int dtype) {
+    if (N != 768) return device_sms() / 2;
+    return dtype == VIG_DTYPE_BF16 ? norm_clusters<__nv_bfloat16, 384, 2>() : norm_clusters<__half, 384, 2>();
 }
 
 }  // namespace vig
