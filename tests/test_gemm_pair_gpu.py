@@ -129,6 +129,9 @@ def test_rows_off_16_bytes():
             assert float((mlp(y).float() - ref).norm() / ref.norm()) < 1e-2
         one = mlp(x[:1, :1].expand(1, 4096, 384)).float()
         assert float((one - ref[:1, :1]).norm() / one.norm()) < 1e-2
+        row = torch.randn(192, 1, device="cuda").bfloat16().t()                     # one row, "contiguous" with a row stride of 1
+        narrow = vig_b200.modules.GLAMLP(192).cuda().bfloat16().requires_grad_(False)
+        assert row.stride(0) == 1 and float((narrow(row) - narrow(row.clone(memory_format=torch.contiguous_format))).norm()) < 1e-2 * float(narrow(row).norm())
 
 
 @pytest.mark.parametrize("N,K", [(256, 256), (256, 704), (384, 384), (384, 1024), (768, 768), (768, 2048)])

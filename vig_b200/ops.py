@@ -454,6 +454,8 @@ def embed_conv_ln(x, weight, conv_bias, ln_weight, ln_bias, eps=1e-5, act_gelu=T
 def _rows_on_16(x, K):
     """Whether the ``[M, K]`` rows of a 16-bit ``x`` begin on 16 bytes, as the copies to shared memory want them; rows that have to be
     gathered into a copy do."""
+    if x.is_contiguous() and x.numel() > K and x.shape[-1] == K:              # (a single row may have any stride)
+        return x.data_ptr() % 16 == 0
     try:
         rows = x.view(-1, K)
     except RuntimeError:
