@@ -33,10 +33,8 @@ struct AnMaps { CUtensorMap x, w, res, r, h; };
 __device__ __forceinline__ void epi_bar_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
 template <typename T, int NT>            // NT = N, the row width, a compile-time constant so that a row lives in registers
-__global__ void __launch_bounds__(AN_THREADS, 1) linear_add_rmsnorm_kernel(const __grid_constant__ AnMaps maps, const T* __restrict__ residual,
-                                                                           const T* __restrict__ norm_w, T* __restrict__ out_r,
-                                                                           T* __restrict__ out_h, int M, int KB, int CH, int nstage,
-                                                                           float eps, int32_t* status) {
+__global__ void __launch_bounds__(AN_THREADS, 1) linear_add_rmsnorm_kernel(const __grid_constant__ AnMaps maps, bool has_res, const T* __restrict__ norm_w, int M, int KB,
+                                                                           int nstage, float eps, int32_t* status) {
     extern __shared__ uint8_t an_smem_raw[];
     uint8_t* smem = an_smem_raw + ((1024u - (smem_u32(an_smem_raw) & 1023u)) & 1023u);
     const uint32_t sbase = smem_u32(smem);
@@ -53,8 +51,6 @@ __global__ void __launch_bounds__(AN_THREADS, 1) linear_add_rmsnorm_kernel(const
     float* ss_part = reinterpret_cast<float*>(smem + off_bar + 8 * 24 + 16);       // [2 column halves][128 rows]
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const Waiter waiter{abort_flag, status};
-    const int nbuf = 2 * N <= 512 ? 2 : 1;
-    const int nch = N / CH;                                   // MMAs of N = CH columns per k step
 
     if (tid == 0) {
         for (int s = 0; s < nstage; ++s) { mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, 1); }
@@ -79,17 +75,15 @@ __global__ void __launch_bounds__(AN_THREADS, 1) linear_add_rmsnorm_kernel(const
         if (lane == 0) {                          // ---- TMA producer -------------------------------------------
             uint32_t st = 0, phase = 0, t_it = 0;
             for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++t_it) {
-                {                                     // the tile's residual rows, into the epilogue buffer of this tile
-                    const uint32_t eb = t_it & 1u;
-                    waiter.wait(bar_e_free + 8 * eb, ((t_it >> 1) & 1u) ^ 1u);
-                    if (*abort_flag) break;
-                    if (residual) {
-                        mbar_expect_tx(bar_res_full + 8 * eb, E_BYTES);
-                        for (int bx = 0; bx < NT / 64; ++bx)
-                            tma_load_2d(sbase + off_e + eb * E_BYTES + bx * 16384, &maps.res, bx * 64, tile * 128, bar_res_full + 8 * eb);
-                    } else {
-                        mbar_arrive_plain(bar_res_full + 8 * eb);
-                    }
+                const uint32_t eb = t_it & 1u;        // the tile's residual rows, into the epilogue buffer of this tile
+                waiter.wait(bar_e_free + 8 * eb, ((t_it >> 1) & 1u) ^ 1u);
+                if (*abort_flag) break;
+                if (has_res) {
+                    mbar_expect_tx(bar_res_full + 8 * eb, E_BYTES);
+                    for (int bx = 0; bx < NT / 64; ++bx)
+                        tma_load_2d(sbase + off_e + eb * E_BYTES + bx * 16384, &maps.res, bx * 64, tile * 128, bar_res_full + 8 * eb);
+                } else {
+                    mbar_arrive_plain(bar_res_full + 8 * eb);
                 }
                 for (int kb = 0; kb < KB; ++kb) {
                     waiter.wait(bar_empty + 8 * st, phase ^ 1u);
@@ -97,49 +91,41 @@ __global__ void __launch_bounds__(AN_THREADS, 1) linear_add_rmsnorm_kernel(const
                     mbar_expect_tx(bar_full + 8 * st, stage_bytes);
                     const uint32_t dst = sbase + st * stage_bytes;
                     tma_load_2d(dst, &maps.x, kb * AN_BK, tile * 128, bar_full + 8 * st);
-                    for (int c = 0; c < nch; ++c)
-                        tma_load_2d(dst + AN_A_BYTES + (uint32_t)c * CH * AN_BK * 2, &maps.w, kb * AN_BK, c * CH, bar_full + 8 * st);
+                    tma_load_2d(dst + AN_A_BYTES, &maps.w, kb * AN_BK, 0, bar_full + 8 * st);
                     if (++st == (uint32_t)nstage) { st = 0; phase ^= 1u; }
                 }
             }
         }
-    } else if (warp == 1) {
-        {                                         // ---- MMA issuer ---------------------------------------------
-            // The whole warp walks the loop (uniform control flow keeps the descriptor arithmetic cheap), lane 0 issues;
-            // a descriptor's low word advances by adding to its address field (16-byte units).
-            const uint32_t idesc = (1u << 4) | (Pack2<T>::FMT << 7) | (Pack2<T>::FMT << 10) | (((uint32_t)CH >> 3) << 17) | ((128u >> 4) << 24);
-            const uint32_t ch_lo = ((uint32_t)CH * AN_BK * 2) >> 4;
-            uint32_t st = 0, phase = 0, acc_it = 0;
-            for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++acc_it) {
-                const uint32_t buf = nbuf == 2 ? (acc_it & 1u) : 0u;
-                const uint32_t use = nbuf == 2 ? (acc_it >> 1) : acc_it;       // how often this buffer has been used before
-                waiter.wait(bar_acc_empty + 8 * buf, (use & 1u) ^ 1u);         // the epilogue has drained this buffer
-                if (*abort_flag) break;
+    } else if (warp == 1) {                       // ---- MMA issuer ---------------------------------------------
+        // The whole warp walks the loop (uniform control flow keeps the descriptor arithmetic cheap), lane 0 issues;
+        // a descriptor's low word advances by adding to its address field (16-byte units).
+        constexpr uint32_t IDESC = make_idesc(Pack2<T>::FMT, 0, 0, 128, N);
+        uint32_t st = 0, phase = 0, acc_it = 0;
+        for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++acc_it) {
+            const uint32_t buf = acc_it & 1u;
+            waiter.wait(bar_acc_empty + 8 * buf, ((acc_it >> 1) & 1u) ^ 1u);   // the epilogue has drained this buffer
+            if (*abort_flag) break;
+            tc_fence_after();
+            const uint32_t d = tmem + buf * (uint32_t)N;
+            for (int kb = 0; kb < KB; ++kb) {
+                waiter.wait(bar_full + 8 * st, phase);
                 tc_fence_after();
-                const uint32_t d0 = tmem + buf * (uint32_t)N;
-                for (int kb = 0; kb < KB; ++kb) {
-                    waiter.wait(bar_full + 8 * st, phase);
-                    tc_fence_after();
-                    const uint32_t a_lo = make_desc(sbase + st * stage_bytes), b_lo = make_desc(sbase + st * stage_bytes + AN_A_BYTES);
-                    if (lane == 0) {
-                        for (int c = 0; c < nch; ++c) {
-                            const uint32_t d = d0 + (uint32_t)c * CH, b_c = b_lo + (uint32_t)c * ch_lo;
-                            tc_mma(d, a_lo, b_c, idesc, kb > 0 ? 1u : 0u);
-                            tc_mma(d, a_lo + 2, b_c + 2, idesc, 1u);
-                            tc_mma(d, a_lo + 4, b_c + 4, idesc, 1u);
-                            tc_mma(d, a_lo + 6, b_c + 6, idesc, 1u);
-                        }
-                        tc_commit(bar_empty + 8 * st);                          // the stage is free when these MMAs are done
-                    }
-                    __syncwarp();
-                    if (++st == (uint32_t)nstage) { st = 0; phase ^= 1u; }
+                const uint32_t a_lo = make_desc(sbase + st * stage_bytes), b_lo = make_desc(sbase + st * stage_bytes + AN_A_BYTES);
+                if (lane == 0) {
+                    tc_mma(d, a_lo, b_lo, IDESC, kb > 0 ? 1u : 0u);
+                    tc_mma(d, a_lo + 2, b_lo + 2, IDESC, 1u);
+                    tc_mma(d, a_lo + 4, b_lo + 4, IDESC, 1u);
+                    tc_mma(d, a_lo + 6, b_lo + 6, IDESC, 1u);
+                    tc_commit(bar_empty + 8 * st);                          // the stage is free when these MMAs are done
                 }
-                if (lane == 0) tc_commit(bar_acc_full + 8 * buf);
                 __syncwarp();
+                if (++st == (uint32_t)nstage) { st = 0; phase ^= 1u; }
             }
+            if (lane == 0) tc_commit(bar_acc_full + 8 * buf);
+            __syncwarp();
         }
     } else {                                      // ---- epilogue through shared memory and TMA stores ----------------
-        // One thread per row (its TMEM lane).  The residual tile arrives by TMA in 128-byte-swizzled boxes; pass 1 turns
+        // Two threads a row (its TMEM lane).  The residual tile arrives by TMA in 128-byte-swizzled boxes; pass 1 turns
         // it into r in place (and keeps r in registers), a TMA store sends it out; pass 2 writes h over the same boxes
         // once that store has read them, and a second TMA store sends h out.
         constexpr int NH = NT / 2, NV = NH / 8;   // my half of the row: NH columns = NV 16-byte vectors
@@ -149,16 +135,14 @@ __global__ void __launch_bounds__(AN_THREADS, 1) linear_add_rmsnorm_kernel(const
         const bool leader = warp == 2 && lane == 0;
         uint32_t acc_it = 0;
         for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++acc_it) {
-            const uint32_t buf = nbuf == 2 ? (acc_it & 1u) : 0u;
-            const uint32_t use = nbuf == 2 ? (acc_it >> 1) : acc_it;
-            const uint32_t eb = acc_it & 1u;
+            const uint32_t eb = acc_it & 1u, par = (acc_it >> 1) & 1u;         // buffers of this tile, uses of them before
             uint8_t* ebuf = smem + off_e + eb * E_BYTES;
             // both waits by the whole warp: a wait by one lane with the others parked at a warp barrier resumes microseconds late
-            waiter.wait(bar_res_full + 8 * eb, (acc_it >> 1) & 1u);
-            waiter.wait(bar_acc_full + 8 * buf, use & 1u);
+            waiter.wait(bar_res_full + 8 * eb, par);
+            waiter.wait(bar_acc_full + 8 * eb, par);
             __syncwarp();                         // (no early exit on an abort: the four warps meet at named barriers below,
             tc_fence_after();                     //  and after an abort every wait returns at once)
-            const uint32_t acc = tmem + lane_base + buf * (uint32_t)NT;
+            const uint32_t acc = tmem + lane_base + eb * (uint32_t)NT;
             uint4 rr[NV];
             float ss = 0.f;
 #pragma unroll
@@ -171,7 +155,7 @@ __global__ void __launch_bounds__(AN_THREADS, 1) linear_add_rmsnorm_kernel(const
                 for (int j = 0; j < 4; ++j) {
                     const int v = c / 8 + j;      // 16-byte vector of the row: box v / 8, chunk v % 8
                     uint4* cell = reinterpret_cast<uint4*>(ebuf + (v / 8) * 16384 + rr_ * 128 + (((v % 8) ^ (rr_ & 7)) << 4));
-                    uint4 rv = residual ? *cell : make_uint4(0u, 0u, 0u, 0u);
+                    uint4 rv = has_res ? *cell : make_uint4(0u, 0u, 0u, 0u);
                     uint32_t* rw = reinterpret_cast<uint32_t*>(&rv);
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
@@ -187,7 +171,7 @@ __global__ void __launch_bounds__(AN_THREADS, 1) linear_add_rmsnorm_kernel(const
                 }
             }
             tc_fence_before();
-            mbar_arrive_plain(bar_acc_empty + 8 * buf);       // the accumulator is read
+            mbar_arrive_plain(bar_acc_empty + 8 * eb);        // the accumulator is read
             ss_part[chalf * 128 + rr_] = ss;                  // the other half of my row belongs to another warp
             fence_proxy_async();
             epi_bar_sync();
@@ -232,8 +216,6 @@ __global__ void __launch_bounds__(AN_THREADS, 1) linear_add_rmsnorm_kernel(const
     }
 }
 
-int an_chunk(int N) { return N == 192 ? 192 : (N == 128 ? 128 : 64); }
-
 }  // namespace
 }  // namespace vig
 
@@ -273,9 +255,8 @@ extern "C" int vig_linear_add_rmsnorm_fwd(const void* x, int64_t ldx, const void
         return VIG_ERR_ALIGN;
     if (ldx < K || (ldx * 2) % 16 || M >= (1ll << 31) - 128) return VIG_ERR_ARG;
     if (N > 192) return pair_norm_launch(x, ldx, w, residual, norm_weight, out_r, out_h, M, K, N, eps, dtype, status_dev, (cudaStream_t)stream);
-    const int CH = an_chunk(N);
     AnMaps maps;
-    if (!tc::make_map_2d(&maps.x, x, M, K, ldx, 128, dtype) || !tc::make_map_2d(&maps.w, w, N, K, K, CH, dtype)) return VIG_ERR_DEVICE;
+    if (!tc::make_map_2d(&maps.x, x, M, K, ldx, 128, dtype) || !tc::make_map_2d(&maps.w, w, N, K, K, N, dtype)) return VIG_ERR_DEVICE;
     const int stage_bytes = AN_A_BYTES + N * AN_BK * 2;
     const size_t e_bytes = 2 * (size_t)(N / 64) * 16384;
     int nstage = (int)((227 * 1024 - 4096 - e_bytes) / stage_bytes);     // the ring gets what the two epilogue tiles leave of the 227 KB
@@ -284,24 +265,14 @@ extern "C" int vig_linear_add_rmsnorm_fwd(const void* x, int64_t ldx, const void
     if ((residual && !tc::make_map_2d(&maps.res, residual, M, N, N, 128, dtype)) || !tc::make_map_2d(&maps.r, out_r, M, N, N, 128, dtype) ||
                     !tc::make_map_2d(&maps.h, out_h, M, N, N, 128, dtype))
         return VIG_ERR_DEVICE;
-    static int sm_count[64] = {};
-    int dev = 0;
     cudaError_t e;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return (int)e;
-    if (dev < 0 || dev >= 64) return VIG_ERR_DEVICE;
-    if (!sm_count[dev]) {
-        int sms = 0;
-        if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return (int)e;
-        sm_count[dev] = sms;
-    }
     const int64_t ntiles = (M + 127) / 128;
-    const int grid = (int)(ntiles < sm_count[dev] ? ntiles : sm_count[dev]);
+    const int sms = device_sms(), grid = (int)(ntiles < sms ? ntiles : sms);
 #define VIG_AN_LAUNCH(TT, NN)                                                                                                  \
     {                                                                                                                          \
         auto kfn = linear_add_rmsnorm_kernel<TT, NN>;                                                                          \
         if ((e = tc::ensure_smem_attr(reinterpret_cast<const void*>(kfn), (int)smem)) != cudaSuccess) return (int)e; \
-        kfn<<<grid, AN_THREADS, smem, (cudaStream_t)stream>>>(maps, (const TT*)residual, (const TT*)norm_weight, (TT*)out_r,   \
-                                                               (TT*)out_h, (int)M, K / AN_BK, CH, nstage, eps, status_dev);   \
+        kfn<<<grid, AN_THREADS, smem, (cudaStream_t)stream>>>(maps, residual != nullptr, (const TT*)norm_weight, (int)M, K / AN_BK, nstage, eps, status_dev); \
     }
 #define VIG_AN_WIDTHS(TT)                                                                                                      \
     switch (N) {                                                                                                               \

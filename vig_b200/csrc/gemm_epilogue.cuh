@@ -35,9 +35,8 @@ __device__ __forceinline__ void swiglu_pack(const float* g, const float* y, uint
 // A warp's [32 rows x 32 columns] piece goes out through its 2 KB box of shared memory as one TMA store.  A row is 64 bytes, its
 // 16-byte pieces swizzled (64-byte swizzle) so that eight lanes write all banks; unswizzled they met on a quarter of them, and the
 // operands of the MMAs come out of the same shared memory.
-template <int BOXES = 1>
 __device__ __forceinline__ void send_box(uint8_t* box, const uint32_t* pk, const CUtensorMap* map, int col, int row, bool in_range, int lane) {
-    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(BOXES - 1) : "memory");   // an earlier store has read the box
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the warp's earlier store has read the box
     __syncwarp();
 #pragma unroll
     for (int j = 0; j < 4; ++j)

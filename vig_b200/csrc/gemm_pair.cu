@@ -20,7 +20,8 @@ using namespace tc;
 constexpr int PR_BK = 64;                                // k elements of a box (128-byte rows)
 constexpr int PR_A = 128 * PR_BK * 2;                    // one CTA's [128 rows x 64 k] box of x
 
-template <int BN> struct PairCfg {
+struct PairCfg {
+    static constexpr int BN = 256;                       // columns of the product in a tile
     static constexpr int B = BN / 2 * PR_BK * 2;         // one CTA's half of a k box of W
     static constexpr int OCOLS = BN / 2, COLS = 32;      // output columns of a tile, of an epilogue warp
     static constexpr int EPI_WARPS = 4 * OCOLS / COLS, THREADS = 64 + 32 * EPI_WARPS;
@@ -33,10 +34,11 @@ template <int BN> struct PairCfg {
 struct PairMaps { CUtensorMap x, w, o; };
 
 // stat: stationary form, ``nst`` boxes of x in the ring; otherwise ``nst`` boxes of x and W
-template <typename T, int BN, bool STAT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<BN>::THREADS, 1)
+template <typename T, bool STAT>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg::THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ PairMaps maps, int M, int N, int KB, int ntn, int ntm, int nst, int32_t* status) {
-    using Cfg = PairCfg<BN>;
+    using Cfg = PairCfg;
+    constexpr int BN = Cfg::BN;
     constexpr int STAGE = PR_A + (STAT ? 0 : Cfg::B);
     extern __shared__ uint8_t pr_smem_raw[];
     uint8_t* smem = pr_smem_raw + ((1024u - (smem_u32(pr_smem_raw) & 1023u)) & 1023u);
@@ -175,9 +177,10 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, int M, int N, int KB, in
     }
 }
 
-template <typename T, int BN>
+template <typename T>
 int pair_launch(const void* x, int64_t ldx, const void* w, void* out, int64_t ldo, int64_t M, int K, int N, int dtype, int32_t* status, cudaStream_t stream) {
-    using Cfg = PairCfg<BN>;
+    using Cfg = PairCfg;
+    constexpr int BN = Cfg::BN;
     PairMaps maps;
     if (!make_map_2d(&maps.x, x, M, K, ldx, 128, dtype) || !make_map_2d(&maps.w, w, 2 * (int64_t)N, K, K, BN / 2, dtype) ||
         !make_out_map(&maps.o, out, M, N, ldo, dtype)) return VIG_ERR_DEVICE;
@@ -191,7 +194,7 @@ int pair_launch(const void* x, int64_t ldx, const void* w, void* out, int64_t ld
     const int nst = stat ? (xst < Cfg::MAX_ST ? xst : Cfg::MAX_ST) : Cfg::RING / (PR_A + Cfg::B);
     const int smem = (stat ? KB * Cfg::B + nst * PR_A : nst * (PR_A + Cfg::B)) + Cfg::OUT + Cfg::BARS + 16 + 1024;
     const int64_t pairs = stat ? all / ntn * ntn : ntm * ntn < all ? ntm * ntn : all;
-    auto kfn = stat ? gemm_pair_kernel<T, BN, true> : gemm_pair_kernel<T, BN, false>;
+    auto kfn = stat ? gemm_pair_kernel<T, true> : gemm_pair_kernel<T, false>;
     const cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(kfn), 227 * 1024);
     if (e != cudaSuccess) return (int)e;
     return (int)launch_chained(kfn, dim3(2 * (unsigned)pairs), dim3(Cfg::THREADS), smem, stream, maps, (int)M, N, KB, ntn, (int)ntm, nst, status);
@@ -200,8 +203,8 @@ int pair_launch(const void* x, int64_t ldx, const void* w, void* out, int64_t ld
 }  // namespace
 
 int pair_swiglu_launch(const void* x, int64_t ldx, const void* w, void* out, int64_t ldo, int64_t M, int K, int I, int dtype, int32_t* status, cudaStream_t stream) {
-    if (dtype == VIG_DTYPE_BF16) return pair_launch<__nv_bfloat16, 256>(x, ldx, w, out, ldo, M, K, I, dtype, status, stream);
-    return pair_launch<__half, 256>(x, ldx, w, out, ldo, M, K, I, dtype, status, stream);
+    if (dtype == VIG_DTYPE_BF16) return pair_launch<__nv_bfloat16>(x, ldx, w, out, ldo, M, K, I, dtype, status, stream);
+    return pair_launch<__half>(x, ldx, w, out, ldo, M, K, I, dtype, status, stream);
 }
 
 }  // namespace vig
