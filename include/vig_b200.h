@@ -328,7 +328,7 @@ VIG_API int vig_stem_conv_ln_fwd(const void* cells, const void* w2, const void* 
  * and `down_proj` followed by the next block's `attn_norm` / the model's final norm (classification/models/vig.py:463,
  * 497, 596-606; fla/modules/rmsnorm.py:491-512).  One tcgen05 GEMM kernel; the projection output is not written.
  * Same roundings as the unfused sequence (projection rounded to the tensor dtype, sum rounded to the tensor dtype).
- * x: [M, K] with row stride ldx; w: [N, K] contiguous; residual, out_r, out_h: [M, N] contiguous; K % 64 == 0,
+ * x: [M, K] with row stride ldx; w: [N, K] contiguous; residual, out_r, out_h: [M, N] contiguous (out_r may be the residual); K % 64 == 0,
  * N one of 64, 128, 192, 256, 384, 768.  status_dev: optional int32 on the device, bit 0 = a bounded wait ran out.
  */
 VIG_API int vig_linear_add_rmsnorm_supported(int64_t M, int K, int N, int dtype);

@@ -149,3 +149,58 @@ def test_long_rows_are_counted_in_rounds(N, K):
     full = math.gcd(*given_up)
     assert given_up and 0.75 * most <= full <= most
     assert not takes(1) and all(takes(t) for t in range(40 * most, 44 * most))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,K,I", [(300, 384, 192), (38000, 192, 128), (19200, 384, 1024), (700, 768, 320)])
+def test_swiglu_infinities_stay_in_their_rows(dtype, M, K, I):
+    """Infinities and NaN in a few rows of x, the last one among them: the other rows keep their bits."""
+    import vig_b200
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randn(M, K, generator=g, device="cuda").to(dtype)
+    w = (torch.randn(2 * I, K, generator=g, device="cuda") / K ** 0.5).to(dtype)
+    clean = vig_b200.ops.linear_swiglu(x, w)
+    bad = torch.tensor([0, 127, 130, M // 2, M - 1], device="cuda")
+    x[bad, torch.tensor([0, K - 1, 5, 63, 64 % K], device="cuda")] = torch.tensor([float("inf"), float("nan"), -float("inf"), float("nan"), float("inf")], device="cuda").to(dtype)
+    out = vig_b200.ops.linear_swiglu(x, w)
+    vig_b200.check_status()
+    rest = torch.ones(M, dtype=torch.bool, device="cuda")
+    rest[bad] = False
+    assert torch.equal(out[rest], clean[rest]) and not bool(out[bad].isfinite().all(-1).any())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,K,N", [(300, 512, 192), (300, 256, 256), (19201, 384, 384), (600, 2048, 768), (9473, 768, 768)])
+def test_projection_add_norm_infinities_stay_in_their_rows(dtype, M, K, N):
+    """Infinities and NaN in rows of x and of the residual, in either half of a row that two pairs share: the other rows keep their bits."""
+    import vig_b200
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randn(M, K, generator=g, device="cuda").to(dtype)
+    w = (torch.randn(N, K, generator=g, device="cuda") / K ** 0.5).to(dtype)
+    res = torch.randn(M, N, generator=g, device="cuda").to(dtype)
+    nw = (1 + 0.1 * torch.randn(N, generator=g, device="cuda")).to(dtype)
+    clean = vig_b200.ops.linear_add_rmsnorm(x, w, res, nw)
+    x[0, 3], x[130, K - 1] = float("nan"), float("inf")
+    res[127, 0], res[M // 2, N - 1], res[M - 1, N // 2] = float("inf"), float("nan"), -float("inf")
+    got = vig_b200.ops.linear_add_rmsnorm(x, w, res, nw)
+    vig_b200.check_status()
+    bad = torch.tensor([0, 127, 130, M // 2, M - 1], device="cuda")
+    rest = torch.ones(M, dtype=torch.bool, device="cuda")
+    rest[bad] = False
+    for a, b in zip(got, clean):
+        assert torch.equal(a[rest], b[rest]) and not bool(a[bad].isfinite().all(-1).any())
+
+
+@pytest.mark.parametrize("M,K,N", [(20000, 512, 192), (300, 256, 256), (19201, 384, 384), (9473, 768, 768)])
+def test_projection_add_norm_in_place(M, K, N):
+    """The sum may be written over the residual."""
+    import vig_b200
+    from vig_b200 import _lib
+    x = torch.randn(M, K, device="cuda").bfloat16()
+    w = (torch.randn(N, K, device="cuda") / K ** 0.5).bfloat16()
+    res, nw = torch.randn(M, N, device="cuda").bfloat16(), torch.randn(N, device="cuda").bfloat16()
+    want_h, want_r = vig_b200.ops.linear_add_rmsnorm(x, w, res, nw, 1e-6)
+    h = torch.empty_like(res)
+    assert _lib.lib().vig_linear_add_rmsnorm_fwd(_lib.ptr(x), K, _lib.ptr(w), _lib.ptr(res), _lib.ptr(nw), _lib.ptr(res), _lib.ptr(h), M, K, N, 1e-6, _lib.dtype_code(x),
+                                                 None, _lib.stream_ptr()) == 0
+    assert torch.equal(h, want_h) and torch.equal(res, want_r)
