@@ -70,8 +70,8 @@ def _vig(model):
         a, mlp, n1, n2 = b.attn, b.mlp, b.attn_norm, b.mlp_norm
         if type(a) is not modules.GatedLinearAttention or type(mlp) is not modules.GLAMLP or type(n1) is not modules.RMSNorm or type(n2) is not modules.RMSNorm:
             return None
-        o, gate, down = a.o_proj, mlp.gate_proj, mlp.down_proj
-        if any(type(m) is not nn.Linear or m.bias is not None for m in (o, gate, down)):
+        gate, down = mlp.gate_proj, mlp.down_proj
+        if not (type(a.o_proj) is type(gate) is type(down) is nn.Linear and gate.bias is None and down.bias is None):
             return None
         attn = _attn(a)
         if attn is None:

@@ -454,13 +454,18 @@ def embed_conv_ln(x, weight, conv_bias, ln_weight, ln_bias, eps=1e-5, act_gelu=T
 def _rows_on_16(x, K):
     """Whether the ``[M, K]`` rows of a 16-bit ``x`` begin on 16 bytes, as the copies to shared memory want them; rows that have to be
     gathered into a copy do."""
-    if x.is_contiguous() and x.numel() > K and x.shape[-1] == K:              # (a single row may have any stride)
+    if x.is_contiguous() and x.shape[-1] == K:
         return x.data_ptr() % 16 == 0
     try:
         rows = x.view(-1, K)
     except RuntimeError:
         return True
-    return rows.stride(1) != 1 or (x.data_ptr() % 16 == 0 and rows.stride(0) >= K and rows.stride(0) % 8 == 0)
+    return rows.stride(1) != 1 or (x.data_ptr() % 16 == 0 and _row_stride(rows) >= K and _row_stride(rows) % 8 == 0)
+
+
+def _row_stride(rows):
+    """Elements between two rows; a single row may have any stride."""
+    return rows.stride(0) if rows.shape[0] > 1 else rows.shape[1]
 
 
 def linear_add_rmsnorm_supported(x, w, preferred=False):
@@ -489,7 +494,7 @@ def linear_add_rmsnorm(x, w, residual, norm_weight, eps=1e-6):
     res = residual.reshape(M, N).contiguous() if residual is not None else None
     out_r = torch.empty(M, N, dtype=x.dtype, device=x.device)
     out_h = torch.empty(M, N, dtype=x.dtype, device=x.device)
-    st = _lib.lib().vig_linear_add_rmsnorm_fwd(_lib.ptr(x2), x2.stride(0), _lib.ptr(w.contiguous()), _lib.ptr(res), _lib.ptr(norm_weight),
+    st = _lib.lib().vig_linear_add_rmsnorm_fwd(_lib.ptr(x2), _row_stride(x2), _lib.ptr(w.contiguous()), _lib.ptr(res), _lib.ptr(norm_weight),
                                                _lib.ptr(out_r), _lib.ptr(out_h), M, K, N, float(eps), _lib.dtype_code(x),
                                                _status_ptr(None, x.device), _lib.stream_ptr())
     _lib.check(st, "vig_linear_add_rmsnorm_fwd")
@@ -611,7 +616,7 @@ def linear_swiglu(x, weight):
     if x2.stride(1) != 1:
         x2 = x2.contiguous()
     out = torch.empty(*x.shape[:-1], I, dtype=x.dtype, device=x.device)
-    st = _lib.lib().vig_linear_swiglu_fwd(_lib.ptr(x2), x2.stride(0), _lib.ptr(weight), _lib.ptr(out), I, x2.shape[0], K, I,
+    st = _lib.lib().vig_linear_swiglu_fwd(_lib.ptr(x2), _row_stride(x2), _lib.ptr(weight), _lib.ptr(out), I, x2.shape[0], K, I,
                                           _lib.dtype_code(x), _status_ptr(None, x.device), _lib.stream_ptr())
     _lib.check(st, "vig_linear_swiglu_fwd")
     return out
