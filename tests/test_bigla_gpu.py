@@ -355,6 +355,35 @@ def test_wavefront_form_raw_logits_clamp_and_range_flag():
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("dk", [64, 32])
+@pytest.mark.parametrize("normalizer", [0.0, 16.0])
+def test_wavefront_form_flags_infinite_gates(dtype, dk, normalizer):
+    """A log-gate of -inf, and a raw logit whose exponential overflows, in every group of tokens of a chunk, in either direction: the call is
+    flagged and the other sequences keep their bits.  A NaN is no gate out of range: its sequence is NaN, the call not flagged."""
+    import vig_b200
+    from vig_b200 import _lib
+    B, H, L = 2, 2, 300
+    gen = torch.Generator(device="cuda").manual_seed(dk)
+    rand = lambda d: torch.randn(B, H, L, d, generator=gen, device="cuda")  # noqa: E731
+    q, k, v = rand(dk).to(dtype), rand(dk).to(dtype), rand(64).to(dtype)
+    gates = [(x if normalizer else torch.nn.functional.logsigmoid(x) / 16).to(dtype) for x in (rand(dk), rand(dk))]
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    run = lambda g: vig_b200.bi_gla(q, k, v, *g, gate_logit_normalizer=normalizer, impl=_lib.IMPL_TC_WAVE, status=status)  # noqa: E731
+    clean = run(gates)
+    assert int(status.item()) == 0
+    for bad in (-float("inf"), *([-600.0] if normalizer else []), float("nan")):
+        for which in (0, 1):
+            for at in (*range(128, 256, 8), 0, 63, 64, 127, 129, 255, 256, 299):
+                g = [t.clone() for t in gates]
+                g[which][1, 1, at, dk - 3] = bad
+                status.zero_()
+                o = run(g)
+                assert int(status.item()) == (0 if bad != bad else 2), (bad, which, at, int(status.item()))
+                assert torch.equal(o[0], clean[0]) and torch.equal(o[1, 0], clean[1, 0])
+                assert bad == bad or bool(o[1, 1].isnan().any())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("B,H,L,dk", [(200, 6, 196, 64), (16, 3, 1500, 64), (20, 3, 600, 32)])
 def test_calls_between_the_forms_keep_their_sums_in_fp32(dtype, B, H, L, dk):
     """Sequences of one segment, and fewer chains than SMs: no less exact than the segment-parallel tcgen05 form, which adds both

@@ -620,6 +620,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_c
         constexpr int NE = WDK * WDV, SLOT = NE + WDK;
         float S[32];
         float gacc = 0.f;                                     // summed log2-gates of my channel along the chain so far
+        bool infinite = false;                                // a chunk of this segment had a total that is
         Item cur; cur.nch = 0; cur.bh = cur.c0 = cur.dir = cur.w = 0;
         int items = 0, ci = 0;
         bool s_zero = true;
@@ -696,6 +697,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_c
                     }
                 }
                 gacc += g_last;
+                infinite |= fabsf(g_last) == INFINITY;
             }
             tc_fence_before();
             s_zero = false;
@@ -712,6 +714,10 @@ __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_c
                     float* box = wp.mailbox + (((size_t)cur.bh * 2 + cur.dir) * 2 + (cur.w & 1)) * SLOT;
                     dst = box; gdst = box + NE;
                 }
+                // An infinite gate makes the workers' differences of sums NaN, which their range test does not see; the chunk's total is
+                // infinite.  (A NaN among the gates makes it NaN: that sequence's outputs say so.)
+                if (infinite && st_row < p.dk && p.status) atomicOr(p.status, 2);
+                infinite = false;
                 const bool row_out = !last || st_row < p.dk;        // the caller's tensors end at dk rows
                 if (dst && row_out) {
 #pragma unroll
