@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) bigla_wave_kernel(const __grid_c
             // ---- my group's offset: (sum of the groups scanned before mine) - G_ref, G_ref = sum of the first 8 groups in
             // scan order.  Half-warp gq reads groups 8 gq .. 8 gq + 7 (scan order) for its 4 channels and takes its share of the
             // difference; one exchange adds the shares (exchanging both sums took eight shuffles for every warp instead of four: 64 x 3 sequences
-            // of 4096 283 -> 280 us, with the cumulative gates kept as pairs). ----
+            // of 4096 277.8 -> 276.8 us, with the cumulative gates kept as pairs). ----
             F2 off01, off23;
             {
                 const float4* part = reinterpret_cast<const float4*>(smem + WO_PART) + (m & 1) * (W_PREP_WARPS * 16) + c4l;

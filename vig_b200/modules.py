@@ -2,8 +2,9 @@
 arguments as ``classification/models/vig.py`` (``GatedLinearAttention`` :241-464, ``GLAMLP`` :469-497,
 ``GLABlock`` :530-618) and ``fla/modules/rmsnorm.py:491-512`` (``RMSNorm``), so a reference state dict
 loads unchanged.  Inference only: the forward is the reference's ``eval()`` branch, with the scan, the
-depthwise conv, the gating injection, the norms and SwiGLU running as the library's CUDA kernels and the
-dense projections as cuBLAS GEMMs (``F.linear``).
+depthwise conv, the gating injection, the norms and SwiGLU running as the library's CUDA kernels.  The stacked
+input projection is the GEMM library's; the gate projection with its SwiGLU, and the output and down projections
+with the residual add and norm behind them, are kernels of this library where these are the faster ones (16-bit).
 """
 from typing import Optional
 

@@ -2,8 +2,8 @@
 the configuration every shipped YAML uses (v2 patch embed, absolute pos-embed, no cls token, average-pool
 head, RMSNorm + SwiGLU blocks).  Parameter names match the reference so its checkpoints load.
 The stem's first stage (convolution + LayerNorm2d + swish) is one kernel of this library for ViG-T in 16 bits; its
-second convolution, wider first stages, the bicubic pos-embed resize, pooling and the classifier run as PyTorch
-library calls; everything inside the blocks except the stacked input projection is this library's kernels.
+second convolution, wider first stages, the bicubic pos-embed resize and the classifier run as PyTorch library
+calls; inside the blocks the stacked input projection does, and products that the GEMM library does faster.
 """
 import math
 from types import SimpleNamespace
