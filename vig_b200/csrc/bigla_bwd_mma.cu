@@ -323,9 +323,20 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 1 : 2) bwd_grads_mma_kern
         }
         if (have_states) {
             const int next = dir ? c - 1 : c + 1;                       // the chunk scanned after this one
-            load_state<DK, DV, SC>(smem + SM::S, p.ws_S + slot * DK * DV, scl, nullptr, nullptr);
-            load_state<DK, DV, SC>(smem + SM::Z, p.ws_Z + slot * DK * DV, scl + DK,
-                                   next < 0 || next >= p.nchunk ? nullptr : p.ws_S + (((size_t)bh * p.nchunk + next) * 2 + dir) * DK * DV, carry);
+            if (StateLay<DK, DV>::mine()) {
+                float4 a[StateLay<DK, DV>::KN], z[StateLay<DK, DV>::KN];
+                fetch_state<DK, DV>(a, p.ws_S + slot * DK * DV);
+                fetch_state<DK, DV>(z, p.ws_Z + slot * DK * DV);
+                put_state<DK, DV, SC>(smem + SM::S, a, scl);
+                if (next < 0 || next >= p.nchunk) {
+#pragma unroll
+                    for (float4& x : a) x = make_float4(0.f, 0.f, 0.f, 0.f);
+                } else {
+                    fetch_state<DK, DV>(a, p.ws_S + (((size_t)bh * p.nchunk + next) * 2 + dir) * DK * DV);
+                }
+                put_state<DK, DV, SC>(smem + SM::Z, z, scl + DK);
+                state_dots<DK, DV>(carry, z, a);
+            }
             __syncthreads();
         }
         float acc[DK / 8][4];
@@ -393,7 +404,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 1 : 2) bwd_grads_mma_kern
             for (int r = 0; r < RPG; ++r) {
                 const F2 ex = X[r * NT + threadIdx.x];
                 const F2 dq = f2_mul(f2_mul(*reinterpret_cast<const F2*>(EQ + (r0 + r) * SM::EP + 2 * pr), ex), cc);
-                const F2 dk = f2_mul(*reinterpret_cast<const F2*>(EK + (r0 + r) * SM::EP + 2 * pr), f2_make(__fdividef(1.f, f2_lo(ex)), __fdividef(1.f, f2_hi(ex))));
+                const F2 dk = f2_mul(*reinterpret_cast<const F2*>(EK + (r0 + r) * SM::EP + 2 * pr), f2_make(tc::rcp(f2_lo(ex)), tc::rcp(f2_hi(ex))));
                 dqt[r] = f2_add(dqt[r], dq); dkt[r] = f2_add(dkt[r], dk);
                 e[r] = f2_fma(f2_mul(dk, minus), k[r].f2(), f2_mul(dq, q[r].f2()));
                 sum = f2_add(sum, e[r]);
@@ -404,24 +415,19 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 1 : 2) bwd_grads_mma_kern
 #pragma unroll
             for (int o = 0; o < CL::GROUPS; ++o)
                 if (dir ? o < gr : o > gr) run = f2_add(run, *reinterpret_cast<const F2*>(gsum + o * DK + 2 * pr));
-            const int64_t base = ((int64_t)bh * p.L + t0) * DK + 2 * pr;
+            // static register indices for both orders: the backward direction sums upwards, the forward one downwards
+            if (dir) {
 #pragma unroll
-            for (int rr = 0; rr < RPG; ++rr) {
-                // static register indices for both orders: the backward direction sums upwards, the forward one downwards
-                const F2 ev = dir ? e[rr] : e[RPG - 1 - rr];
-                const int row = r0 + (dir ? rr : RPG - 1 - rr);
-                run = f2_add(run, ev);
-                if (row < n) {
-                    float2 dg = make_float2(f2_lo(run), f2_hi(run));
-                    if (p.gate_norm > 0.f || p.clamp_min == p.clamp_min) {
-                        const F2 gx = dir ? x[rr].f2() : x[RPG - 1 - rr].f2();
-                        dg.x = through_gate(dg.x, f2_lo(gx), p.gate_norm, p.clamp_min); dg.y = through_gate(dg.y, f2_hi(gx), p.gate_norm, p.clamp_min);
-                    }
-                    void* out = dir ? p.dgb : p.dgf;
-                    if (p.dg_f32) store2<float>(reinterpret_cast<float*>(out) + base + (int64_t)row * DK, dg.x, dg.y);
-                    else store2<T>(reinterpret_cast<T*>(out) + base + (int64_t)row * DK, dg.x, dg.y);
-                }
+                for (int r = 0; r < RPG; ++r) e[r] = run = f2_add(run, e[r]);
+            } else {
+#pragma unroll
+                for (int r = RPG - 1; r >= 0; --r) e[r] = run = f2_add(run, e[r]);
             }
+            rows_through_gate(e, x, p.gate_norm, p.clamp_min);
+            T* out = reinterpret_cast<T*>(dir ? p.dgb : p.dgf) + ((int64_t)bh * p.L + t0 + r0) * DK + 2 * pr;
+#pragma unroll
+            for (int r = 0; r < RPG; ++r)
+                if (r0 + r < n) store2<T>(out + r * DK, f2_lo(e[r]), f2_hi(e[r]));
         }
         __syncthreads();                                                // the tiles, gsum and carry may be rewritten
     }

@@ -238,9 +238,10 @@ __device__ __forceinline__ F2 f2_add(F2 a, F2 b) { F2 d; asm("add.rn.f32x2 %0, %
 
 constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
 
-// single-instruction exp2 / log2 (flush-to-zero forms: no denormal fix-up code around the MUFU)
+// single-instruction exp2 / log2 / reciprocal (flush-to-zero forms: no denormal fix-up code around the MUFU)
 __device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 __device__ __forceinline__ float lg2(float x) { float y; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ float rcp(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 constexpr float MAX_EXPONENT2 = MAX_EXPONENT * LOG2E;   // the exponent bound in log2 units
 
 // Log-gate in LOG2 units.  From a raw logit: logsigmoid(x) = min(x,0) - log(1 + exp(-|x|)), here with y = x log2(e):
