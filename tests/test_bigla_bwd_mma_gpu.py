@@ -62,3 +62,18 @@ def test_training_step_in_16_bits(dtype, L, dk, dv, norm):
         ref = [*ref[:3], *(g * torch.sigmoid(-x.double()) / norm for g, x in zip(ref[3:], (xf, xb)))]
     errs = {n: rel_err(g.float(), r) for n, g, r in zip(NAMES, got, ref)}
     assert all(e < TOL[dtype] for e in errs.values()), errs
+
+
+@pytest.mark.parametrize("dk,dv", [(16, 32), (32, 64), (64, 64)])
+@pytest.mark.parametrize("which", ["fwd", "bwd"])
+def test_a_chunk_that_one_direction_leaves(dk, dv, which):
+    """The two directions of a chunk are two CTAs that add up their results: where one of them leaves the range, the exact form replaces what
+    the other has written, and the chunks beside it are as they were."""
+    import vig_b200
+    q, k, v, gf, gb = oracle.make_bigla_inputs(2, 2, 200, dk, dv, seed=dk)
+    (gf if which == "fwd" else gb)[0, 1, 64:128] *= 200
+    d_out = torch.randn(2, 2, 200, dv, generator=torch.Generator().manual_seed(3))
+    _, ref = _reference_grads(q, k, v, gf, gb, d_out, 0.5, 3)
+    got = vig_b200.bi_gla_backward(*[t.cuda() for t in (q, k, v, gf, gb, d_out)], out_scale=0.5)
+    errs = {n: rel_err(g, r) for n, g, r in zip(NAMES, got, ref)}
+    assert all(e < TOL[torch.float32] for e in errs.values()), errs

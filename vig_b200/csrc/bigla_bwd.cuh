@@ -16,7 +16,7 @@ struct BwdParams {
     float gate_norm, clamp_min;      // as in the forward: > 0 = raw logits; NaN = no clamp
     int dir_mask;
     float *ws_S, *ws_Z, *ws_decay;   // [BH][nchunk][2][dk*dv] x2, [BH][nchunk][2][dk] (summed log-gates, log2 units)
-    int32_t* flags;                  // [BH][nchunk]: 1 = the chunk's gates left the factorisation range, take the exact form
+    int32_t* flags;                  // [BH][nchunk]: not 0 = the chunk's gates left the factorisation range, take the exact form
     int nchunk;
 };
 

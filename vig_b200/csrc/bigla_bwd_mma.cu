@@ -212,149 +212,183 @@ __global__ void __launch_bounds__(256) bwd_scan_unaligned_kernel(const __grid_co
 // ---- chunk gradients -----------------------------------------------------------------------------------------------
 template <int DK, int DV, typename T> struct GradSmem {
     static constexpr uint32_t EP = DK + 8, VP = DV + 8;                // row pitches of the fp32 tiles (floats)
-    static constexpr uint32_t TQ = Terms<T>::SC * C * Pitch<DK>::B, TS = Terms<T>::SC * DK * Pitch<DV>::B;
+    static constexpr uint32_t TQ = Terms<T>::SC * C * Pitch<DK>::B, TS = Terms<T>::SC * DK * Pitch<DV>::B, TD = C * VP * 4;
     static constexpr uint32_t V = 0, O = V + Terms<T>::RAW * C * Pitch<DV>::B, K = O + Terms<T>::RAW * C * Pitch<DV>::B,
-                              Q = K + TQ, S = Q + TQ, Z = S + TS, X = Z + TS, SUM = X + C * DK * 4, CARRY = SUM + 2 * NT * 4,
-                              SCL = CARRY + DK * 4, BYTES = SCL + 2 * DK * 4;
-    static_assert(C * EP * 4 <= TQ && C * VP * 4 <= 2 * TQ, "the fp32 tiles reuse the operand tiles");
+                              Q = K + TQ, S = Q + TQ, Z = S + TS, X = S + (2 * TS > TD ? 2 * TS : TD), SUM = X + C * DK * 4, CARRY = SUM + NT * 8,
+                              SCL = CARRY + DK * 4, BAR = SCL + 2 * DK * 4, BYTES = BAR + 16,
+                              SENT = C * DK * 4 + C / 2 * DV * 4;       // what arrives from the other direction: dq or dk, half of dv's rows
+    static_assert(C * EP * 4 <= TQ && TD <= K - V && C / 2 * DV * 4 <= TQ, "the fp32 tiles reuse the operand tiles");
 };
 
-// Eight warps on a chunk: warps 0 - 3 form dQ and the state term of dV, warps 4 - 7 dK and the term of dV inside the chunk, 16
-// rows each.  (Four warps with all of it in 255 registers: two CTAs, eight warps an SM, 12 % of the tensor rate.)  What follows
-// the products -- the factors 2^(G-r), e and its sums, both directions' totals -- is done by channel pairs, in which q, k and
-// the gates are read coalesced.
+// The barrier orders no data here (what it protects has been read before; what is sent carries its own count): an arrival
+// that releases waits for every access of the warp, 2500 cycles each time.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// 16 bytes into the other CTA's shared memory; its barrier counts them
+__device__ __forceinline__ void send(uint32_t at, float a, float b, float c, float d, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
+                 ::"r"(at), "f"(a), "f"(b), "f"(c), "f"(d), "r"(bar) : "memory");
+}
+
+// CTAs an SM as shared memory has room for, where that leaves the registers that the products need (bf16 at 32 / 64: three are
+// 2 % faster than two, at 80 registers instead of 128)
+template <int DK, int DV, typename T> constexpr int grads_min_blocks() {
+    return sizeof(T) == 4 ? 1 : DK == 64 ? 2 : DK * DV == 2048 ? (std::is_same<T, __half>::value ? 2 : 3) : DK == 32 ? 3 : 4;
+}
+
+// A CTA forms one chunk's gradients of one direction; with both, the two CTAs of a cluster add them up through each other's
+// shared memory, one finishing dq, the other dk, each half of the rows of dv.  Both directions in turn in one CTA keep dq, dk
+// and dv of the first, 64 of 128 registers at 64 / 64, alive through the products of the second: the spills were as long as the
+// second reading of v and dO is now, and left no registers to ask for the states ahead of a barrier or to keep q, k and the gates
+// (backward of 8 x 6 x 4096, bf16: 513 -> 488 us; 128 x 6 x 196: 531 -> 499; 128 x 3 x 196, 32 / 64, where nothing spilled, 148 -> 150).
+// Bound: latency at 16 warps an SM and shared memory's rate (59 % of it; ldmatrix two thirds of that); the tensor pipe is 27 % busy.
+// Eight warps: warps 0 - 3 form dQ and dV inside the chunk, warps 4 - 7 dK and the state's part of dV, 16 rows each: 160 - 288
+// products a warp and direction; dV on the other side makes it 136 - 352.  What follows the products -- the factors 2^(G-r), e
+// and its sums -- is done by channel pairs, in which q, k and the gates are read coalesced.
 template <int DK, int DV, typename T>
-__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 1 : 2) bwd_grads_mma_kernel(const __grid_constant__ BwdParams p) {
+__global__ void __launch_bounds__(NT, grads_min_blocks<DK, DV, T>()) bwd_grads_mma_kernel(const __grid_constant__ BwdParams p) {
     using CL = ColLay<DK>;
     using SM = GradSmem<DK, DV, T>;
+    using ST = StateLay<DK, DV>;
     constexpr int RAW = Terms<T>::RAW, SC = Terms<T>::SC, RPG = CL::RPG;
     constexpr uint32_t PK = Pitch<DK>::B, PV = Pitch<DV>::B;
     constexpr uint32_t TK = C * PK, TV = C * PV, TS = DK * PV;          // bytes from one term's tile to the next
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t sb = tc::smem_u32(smem);
-    F2* X = reinterpret_cast<F2*>(smem + SM::X);                        // [RPG][NT]: 2^(G-r) of each thread's rows, private
+    F2* X = reinterpret_cast<F2*>(smem + SM::X);                        // [RPG][NT]: 2^(G-r) of each thread's rows, private; then what the other direction sends
     float* gsum = reinterpret_cast<float*>(smem + SM::SUM);
     float* carry = reinterpret_cast<float*>(smem + SM::CARRY);
     float* scl = reinterpret_cast<float*>(smem + SM::SCL);              // [0]: 2^r, [1]: 2^(l-r)
-    float* EQ = reinterpret_cast<float*>(smem + SM::Q);                 // dQ, dK of a direction once the products are done
+    float* EQ = reinterpret_cast<float*>(smem + SM::Q);                 // dQ, dK once the products are done
     float* EK = reinterpret_cast<float*>(smem + SM::K);
     const int lane = threadIdx.x & 31, role = threadIdx.x >> 7, w = (threadIdx.x >> 5) & 3;
-    const int c = blockIdx.x, bh = blockIdx.y, b = bh / p.H, h = bh % p.H;
+    const bool both = p.dir_mask == 3;
+    const int dir = both ? blockIdx.x & 1 : p.dir_mask - 1;
+    const int c = both ? blockIdx.x >> 1 : blockIdx.x, bh = blockIdx.y, b = bh / p.H, h = bh % p.H;
     const int64_t t0 = (int64_t)c * C;
     const int n = min(C, p.L - (int)t0);
     const int pr = threadIdx.x % CL::PAIRS, gr = threadIdx.x / CL::PAIRS, r0 = gr * RPG;
     const int fr = 16 * w + (lane >> 2), fc = 2 * (lane & 3);           // my fragment rows fr, fr + 8; columns 8 nt + fc, + 1
     const T* qp = head_ptr<T>(p.q, p.sq, b, h, t0) + 2 * pr;
     const T* kp = head_ptr<T>(p.k, p.sk, b, h, t0) + 2 * pr;
-    const F2 cc = f2_make(p.c, p.c), minus = f2_make(-1.f, -1.f);
-    float mark = 0.f;
-    bool finite = true;
-    load_raw<T, DV, RAW>(smem + SM::V, head_ptr<T>(p.v, p.sv, b, h, t0), p.sv[2], n, mark);
-    load_raw<T, DV, RAW>(smem + SM::O, head_ptr<T>(p.dout, p.sdo, b, h, t0), p.sdo[2], n, mark);
-    const uint32_t aV = sb + SM::V + 16 * w * PV + frag_rows<PV>(lane), aO = sb + SM::O + 16 * w * PV + frag_rows<PV>(lane);
-    const uint32_t aK = sb + SM::K + 16 * w * PK + frag_rows<PK>(lane);
-    const uint32_t bV = sb + SM::V + frag_cols<PV>(lane), bO = sb + SM::O + frag_cols<PV>(lane), bQ = sb + SM::Q + frag_cols<PK>(lane);
-    const uint32_t tK = sb + SM::K + frag_rows<PK>(lane), tQ = sb + SM::Q + frag_rows<PK>(lane), tO = sb + SM::O + frag_rows<PV>(lane);
+    const T* gp = (dir ? head_ptr<T>(p.gb, p.sgb, b, h, t0) : head_ptr<T>(p.gf, p.sgf, b, h, t0)) + 2 * pr;
+    const int64_t sgl = dir ? p.sgb[2] : p.sgf[2];
+    const size_t slot = ((size_t)bh * p.nchunk + c) * 2 + dir;
+    const F2 cc = f2_make(p.c, p.c), minus = f2_make(-1.f, -1.f), zero = f2_make(0.f, 0.f);
     const bool have_states = p.nchunk > 1;
+    bool bad;
     pdl_launch();
-    pdl_wait();
-    if (have_states) {                                                   // both directions' states on their way to L2 while the tiles are made
-        constexpr int LINES = DK * DV * 4 / 128;
-        for (int i = threadIdx.x; i < 4 * LINES; i += NT) {
-            const int dir = i / (2 * LINES), which = i / LINES % 2;
-            if (p.dir_mask & (1 << dir)) {
-                const float* at = (which ? p.ws_Z : p.ws_S) + (((size_t)bh * p.nchunk + c) * 2 + dir) * DK * DV + i % LINES * 32;
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(at));
-            }
-        }
+    if (both && threadIdx.x == 0) {
+        tc::mbar_init(sb + SM::BAR, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        tc::mbar_expect_tx(sb + SM::BAR, SM::SENT);
     }
-    float dv[DV / 8][4];
+    Raw2<T> x[RPG], q[RPG], k[RPG];
+    {   // ---- gates, scaled operand tiles
+        load_rows(x, gp, sgl, r0, n);
+        load_rows(q, qp, p.sq[2], r0, n);
+        load_rows(k, kp, p.sk[2], r0, n);
+        float mark = 0.f;
+        load_raw<T, DV, RAW>(smem + SM::V, head_ptr<T>(p.v, p.sv, b, h, t0), p.sv[2], n, mark);
+        load_raw<T, DV, RAW>(smem + SM::O, head_ptr<T>(p.dout, p.sdo, b, h, t0), p.sdo[2], n, mark);
+        F2 G[RPG], ref, tot;
+        cum_gates<DK, T>(G, ref, tot, gsum, x, n, dir, p.gate_norm, p.clamp_min);
+        zero_rows(q, r0, n); zero_rows(k, r0, n);
+        F2 seen = zero;
+        const float lim = range_limit<T>();
+        const F2 rest = f2_fma(ref, minus, tot);
+        bool fine = fabsf(f2_lo(ref)) <= lim && fabsf(f2_hi(ref)) <= lim && fabsf(f2_lo(rest)) <= lim && fabsf(f2_hi(rest)) <= lim;
+        if (gr == 0) {
+            *reinterpret_cast<float2*>(scl + 2 * pr) = make_float2(ex2_t<T>(f2_lo(ref)), ex2_t<T>(f2_hi(ref)));
+            *reinterpret_cast<float2*>(scl + DK + 2 * pr) = make_float2(ex2_t<T>(f2_lo(rest)), ex2_t<T>(f2_hi(rest)));
+        }
 #pragma unroll
-    for (int i = 0; i < DV / 8; ++i)
+        for (int r = 0; r < RPG; ++r) {
+            const F2 y = f2_fma(ref, minus, G[r]);
+            fine = fine && fabsf(f2_lo(y)) <= lim && fabsf(f2_hi(y)) <= lim;
+            const F2 ex = f2_make(ex2_t<T>(f2_lo(y)), ex2_t<T>(f2_hi(y)));
+            X[r * NT + threadIdx.x] = ex;
+            see(seen, q[r].f2()); see(seen, k[r].f2());
+            uint32_t t[SC];
+            const F2 qs = f2_mul(f2_mul(q[r].f2(), cc), ex), ks = f2_mul(k[r].f2(), f2_make(ex2_t<T>(-f2_lo(y)), ex2_t<T>(-f2_hi(y))));
+            split2<SC>(f2_lo(qs), f2_hi(qs), t);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) dv[i][j] = 0.f;
-    F2 dqt[RPG], dkt[RPG];
+            for (int i = 0; i < SC; ++i) *reinterpret_cast<uint32_t*>(smem + SM::Q + i * TK + (r0 + r) * PK + pr * 4) = t[i];
+            split2<SC>(f2_lo(ks), f2_hi(ks), t);
 #pragma unroll
-    for (int r = 0; r < RPG; ++r) dqt[r] = dkt[r] = f2_make(0.f, 0.f);
-#pragma unroll 1
-    for (int dir = 0; dir < 2; ++dir) {
-        if (!(p.dir_mask & (1 << dir))) continue;
-        const T* gp = (dir ? head_ptr<T>(p.gb, p.sgb, b, h, t0) : head_ptr<T>(p.gf, p.sgf, b, h, t0)) + 2 * pr;
-        const int64_t sgl = dir ? p.sgb[2] : p.sgf[2];
-        const size_t slot = ((size_t)bh * p.nchunk + c) * 2 + dir;
-        {   // ---- gates, scaled operand tiles
-            Raw2<T> x[RPG], q[RPG], k[RPG];
-            load_rows(x, gp, sgl, r0, n);
-            load_rows(q, qp, p.sq[2], r0, n);
-            load_rows(k, kp, p.sk[2], r0, n);
-            F2 G[RPG], ref, tot;
-            cum_gates<DK, T>(G, ref, tot, gsum, x, n, dir, p.gate_norm, p.clamp_min);
-            zero_rows(q, r0, n); zero_rows(k, r0, n);
-            F2 seen = f2_make(0.f, 0.f);
-            const float lim = range_limit<T>();
-            const F2 rest = f2_fma(ref, minus, tot);
-            bool fine = fabsf(f2_lo(ref)) <= lim && fabsf(f2_hi(ref)) <= lim && fabsf(f2_lo(rest)) <= lim && fabsf(f2_hi(rest)) <= lim;
-            if (gr == 0) {
-                *reinterpret_cast<float2*>(scl + 2 * pr) = make_float2(ex2_t<T>(f2_lo(ref)), ex2_t<T>(f2_hi(ref)));
-                *reinterpret_cast<float2*>(scl + DK + 2 * pr) = make_float2(ex2_t<T>(f2_lo(rest)), ex2_t<T>(f2_hi(rest)));
-            }
+            for (int i = 0; i < SC; ++i) *reinterpret_cast<uint32_t*>(smem + SM::K + i * TK + (r0 + r) * PK + pr * 4) = t[i];
+        }
+        pdl_wait();                                                      // all of the above read the call's inputs only
+        const int next = dir ? c - 1 : c + 1;                           // the chunk scanned after this one
+        float4 st[ST::KN], adj[ST::KN], ahead[ST::KN];
+        if (have_states && ST::mine()) {                                 // asked for ahead of the barrier that the tiles need
+            fetch_state<DK, DV>(st, p.ws_S + slot * DK * DV);
+            fetch_state<DK, DV>(adj, p.ws_Z + slot * DK * DV);
+            if (next >= 0 && next < p.nchunk) {
+                fetch_state<DK, DV>(ahead, p.ws_S + (((size_t)bh * p.nchunk + next) * 2 + dir) * DK * DV);
+            } else {
 #pragma unroll
-            for (int r = 0; r < RPG; ++r) {
-                const F2 y = f2_fma(ref, minus, G[r]);
-                fine = fine && fabsf(f2_lo(y)) <= lim && fabsf(f2_hi(y)) <= lim;
-                const F2 ex = f2_make(ex2_t<T>(f2_lo(y)), ex2_t<T>(f2_hi(y)));
-                X[r * NT + threadIdx.x] = ex;
-                see(seen, q[r].f2()); see(seen, k[r].f2());
-                uint32_t t[SC];
-                const F2 qs = f2_mul(f2_mul(q[r].f2(), cc), ex), ks = f2_mul(k[r].f2(), f2_make(ex2_t<T>(-f2_lo(y)), ex2_t<T>(-f2_hi(y))));
-                split2<SC>(f2_lo(qs), f2_hi(qs), t);
-#pragma unroll
-                for (int i = 0; i < SC; ++i) *reinterpret_cast<uint32_t*>(smem + SM::Q + i * TK + (r0 + r) * PK + pr * 4) = t[i];
-                split2<SC>(f2_lo(ks), f2_hi(ks), t);
-#pragma unroll
-                for (int i = 0; i < SC; ++i) *reinterpret_cast<uint32_t*>(smem + SM::K + i * TK + (r0 + r) * PK + pr * 4) = t[i];
-            }
-            wait_raw();
-            if (dir == 0 || !(p.dir_mask & 1)) finite = raw_clean<T, DV, RAW>(smem + SM::V, mark) && raw_clean<T, DV, RAW>(smem + SM::O, mark);
-            if (__syncthreads_or(!fine || !finite || !clean(seen))) {    // left to the exact kernel, outputs included
-                if (threadIdx.x == 0) p.flags[(size_t)bh * p.nchunk + c] = 1;
-                return;
+                for (float4& v : ahead) v = make_float4(0.f, 0.f, 0.f, 0.f);
             }
         }
-        if (have_states) {
-            const int next = dir ? c - 1 : c + 1;                       // the chunk scanned after this one
-            if (StateLay<DK, DV>::mine()) {
-                float4 a[StateLay<DK, DV>::KN], z[StateLay<DK, DV>::KN];
-                fetch_state<DK, DV>(a, p.ws_S + slot * DK * DV);
-                fetch_state<DK, DV>(z, p.ws_Z + slot * DK * DV);
-                put_state<DK, DV, SC>(smem + SM::S, a, scl);
-                if (next < 0 || next >= p.nchunk) {
-#pragma unroll
-                    for (float4& x : a) x = make_float4(0.f, 0.f, 0.f, 0.f);
-                } else {
-                    fetch_state<DK, DV>(a, p.ws_S + (((size_t)bh * p.nchunk + next) * 2 + dir) * DK * DV);
-                }
-                put_state<DK, DV, SC>(smem + SM::Z, z, scl + DK);
-                state_dots<DK, DV>(carry, z, a);
+        wait_raw();
+        const bool finite = raw_clean<T, DV, RAW>(smem + SM::V, mark) && raw_clean<T, DV, RAW>(smem + SM::O, mark) && clean(seen);
+        bad = __syncthreads_or(!fine || !finite);
+        if (!bad && have_states) {
+            if (ST::mine()) {
+                put_state<DK, DV, SC>(smem + SM::S, st, scl);
+                put_state<DK, DV, SC>(smem + SM::Z, adj, scl + DK);
+                state_dots<DK, DV>(carry, adj, ahead);
             }
             __syncthreads();
         }
-        float acc[DK / 8][4];
+    }
+    F2 dq[RPG], dk[RPG], e[RPG];
+    if (!bad) {
+        float acc[DK / 8][4], dv[DV / 8][4];
 #pragma unroll
         for (int i = 0; i < DK / 8; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-        if (role == 0) {                                                 // ---- dQ of my rows: 16-token blocks scanned at or before mine
+#pragma unroll
+        for (int i = 0; i < DV / 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) dv[i][j] = 0.f;
+        const uint32_t aV = sb + SM::V + 16 * w * PV + frag_rows<PV>(lane), aO = sb + SM::O + 16 * w * PV + frag_rows<PV>(lane);
+        const uint32_t aK = sb + SM::K + 16 * w * PK + frag_rows<PK>(lane);
+        const uint32_t bV = sb + SM::V + frag_cols<PV>(lane), bO = sb + SM::O + frag_cols<PV>(lane), bQ = sb + SM::Q + frag_cols<PK>(lane);
+        const uint32_t tK = sb + SM::K + frag_rows<PK>(lane), tQ = sb + SM::Q + frag_rows<PK>(lane), tO = sb + SM::O + frag_rows<PV>(lane);
+        uint32_t mine[DV / 16][RAW][4];                                  // my rows of dO (of V): operand of every block and of the state's product
+        load_a<DV, RAW>(mine, role ? aV : aO, TV);
+        if (role == 0) {                                                 // ---- dQ and dV inside the chunk
 #pragma unroll 1
-            for (int jb = dir ? w : 0; jb < (dir ? C / 16 : w + 1); ++jb) {
+            for (int jb = dir ? w : 0; jb < (dir ? C / 16 : w + 1); ++jb) {   // 16-token blocks scanned at or before my rows
                 float pb[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
                 uint32_t ap[SC][4];
-                block_nt<DV, RAW, RAW>(pb, aO, TV, bV + jb * 16 * PV, TV);
+                block_nt<DV, RAW, RAW>(pb, mine, bV + jb * 16 * PV, TV);
                 mask_split<SC>(pb, jb == w, lane, [&](int r, int j) { return dir ? j >= r : j <= r; }, ap);
                 block_nn<DK, SC, SC>(acc, ap, tK + jb * 16 * PK, TK);
             }
+            if (have_states) rows_nt<DK, DV, PV, RAW, SC>(acc, mine, sb + SM::S + frag_cols<PV>(lane), TS);
+#pragma unroll 1
+            for (int ib = dir ? 0 : w; ib < (dir ? w + 1 : C / 16); ++ib) {   // blocks scanned at or after them
+                float pb[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+                uint32_t ap[SC][4];
+                block_nt<DK, SC, SC>(pb, aK, TK, bQ + ib * 16 * PK, TK);
+                mask_split<SC>(pb, ib == w, lane, [&](int j, int i) { return dir ? i <= j : i >= j; }, ap);
+                block_nn<DV, SC, RAW>(dv, ap, tO + ib * 16 * PV, TV);
+            }
+        } else {                                                         // ---- dK, and the state's part of dV
+#pragma unroll 1
+            for (int ib = dir ? 0 : w; ib < (dir ? w + 1 : C / 16); ++ib) {
+                float pb[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+                uint32_t ap[SC][4];
+                block_nt<DV, RAW, RAW>(pb, mine, bO + ib * 16 * PV, TV);
+                mask_split<SC>(pb, ib == w, lane, [&](int j, int i) { return dir ? i <= j : i >= j; }, ap);
+                block_nn<DK, SC, SC>(acc, ap, tQ + ib * 16 * PK, TK);
+            }
             if (have_states) {
-                rows_nt<DK, DV, PV, RAW, SC>(acc, aO, TV, sb + SM::S + frag_cols<PV>(lane), TS);
+                rows_nt<DK, DV, PV, RAW, SC>(acc, mine, sb + SM::Z + frag_cols<PV>(lane), TS);
                 const uint32_t tZ = sb + SM::Z + frag_rows<PV>(lane);
 #pragma unroll
                 for (int ks = 0; ks < DK / 16; ++ks) {
@@ -364,100 +398,116 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 1 : 2) bwd_grads_mma_kern
                     block_nn<DV, SC, SC>(dv, fa, tZ + ks * 16 * PV, TS);
                 }
             }
-        } else {                                                         // ---- dK and dV of my rows: blocks scanned at or after mine
-            auto keep = [&](int j, int i) { return dir ? i <= j : i >= j; };
-#pragma unroll 1
-            for (int ib = dir ? 0 : w; ib < (dir ? w + 1 : C / 16); ++ib) {
-                float pb[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-                uint32_t ap[SC][4];
-                block_nt<DV, RAW, RAW>(pb, aV, TV, bO + ib * 16 * PV, TV);
-                mask_split<SC>(pb, ib == w, lane, keep, ap);
-                block_nn<DK, SC, SC>(acc, ap, tQ + ib * 16 * PK, TK);
-#pragma unroll
-                for (int i = 0; i < 2; ++i)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) pb[i][j] = 0.f;
-                block_nt<DK, SC, SC>(pb, aK, TK, bQ + ib * 16 * PK, TK);
-                mask_split<SC>(pb, ib == w, lane, keep, ap);
-                block_nn<DV, SC, RAW>(dv, ap, tO + ib * 16 * PV, TV);
-            }
-            if (have_states) rows_nt<DK, DV, PV, RAW, SC>(acc, aV, TV, sb + SM::Z + frag_cols<PV>(lane), TS);
         }
         __syncthreads();                                                 // the operand tiles are read
         {
             float* E = (role ? EK : EQ) + fr * SM::EP + fc;
+            float* D = reinterpret_cast<float*>(smem + (role ? SM::S : SM::V)) + fr * SM::VP + fc;
 #pragma unroll
             for (int i = 0; i < DK / 8; ++i) {
                 *reinterpret_cast<float2*>(E + 8 * i) = make_float2(acc[i][0], acc[i][1]);
                 *reinterpret_cast<float2*>(E + 8 * SM::EP + 8 * i) = make_float2(acc[i][2], acc[i][3]);
             }
+#pragma unroll
+            for (int i = 0; i < DV / 8; ++i) {
+                *reinterpret_cast<float2*>(D + 8 * i) = make_float2(dv[i][0], dv[i][1]);
+                *reinterpret_cast<float2*>(D + 8 * SM::VP + 8 * i) = make_float2(dv[i][2], dv[i][3]);
+            }
         }
-        Raw2<T> x[RPG], q[RPG], k[RPG];
-        load_rows(q, qp, p.sq[2], r0, n);
-        load_rows(k, kp, p.sk[2], r0, n);
-        if (p.gate_norm > 0.f || p.clamp_min == p.clamp_min) load_rows(x, gp, sgl, r0, n);
         __syncthreads();
-        {   // ---- by channel pairs: totals, e, and the gate gradient = sum of e over the tokens scanned at or after t plus the value just past the chunk
-            F2 e[RPG], sum = f2_make(0.f, 0.f);
-            zero_rows(q, r0, n); zero_rows(k, r0, n);
+        // ---- by channel pairs: dq, dk, e, and the gate gradient = sum of e over the tokens scanned at or after t plus the value just past the chunk
+        F2 sum = zero;
 #pragma unroll
-            for (int r = 0; r < RPG; ++r) {
-                const F2 ex = X[r * NT + threadIdx.x];
-                const F2 dq = f2_mul(f2_mul(*reinterpret_cast<const F2*>(EQ + (r0 + r) * SM::EP + 2 * pr), ex), cc);
-                const F2 dk = f2_mul(*reinterpret_cast<const F2*>(EK + (r0 + r) * SM::EP + 2 * pr), f2_make(tc::rcp(f2_lo(ex)), tc::rcp(f2_hi(ex))));
-                dqt[r] = f2_add(dqt[r], dq); dkt[r] = f2_add(dkt[r], dk);
-                e[r] = f2_fma(f2_mul(dk, minus), k[r].f2(), f2_mul(dq, q[r].f2()));
-                sum = f2_add(sum, e[r]);
-            }
-            *reinterpret_cast<F2*>(gsum + gr * DK + 2 * pr) = sum;
-            __syncthreads();
-            F2 run = have_states ? *reinterpret_cast<const F2*>(carry + 2 * pr) : f2_make(0.f, 0.f);
-#pragma unroll
-            for (int o = 0; o < CL::GROUPS; ++o)
-                if (dir ? o < gr : o > gr) run = f2_add(run, *reinterpret_cast<const F2*>(gsum + o * DK + 2 * pr));
-            // static register indices for both orders: the backward direction sums upwards, the forward one downwards
-            if (dir) {
-#pragma unroll
-                for (int r = 0; r < RPG; ++r) e[r] = run = f2_add(run, e[r]);
-            } else {
-#pragma unroll
-                for (int r = RPG - 1; r >= 0; --r) e[r] = run = f2_add(run, e[r]);
-            }
-            rows_through_gate(e, x, p.gate_norm, p.clamp_min);
-            T* out = reinterpret_cast<T*>(dir ? p.dgb : p.dgf) + ((int64_t)bh * p.L + t0 + r0) * DK + 2 * pr;
-#pragma unroll
-            for (int r = 0; r < RPG; ++r)
-                if (r0 + r < n) store2<T>(out + r * DK, f2_lo(e[r]), f2_hi(e[r]));
+        for (int r = 0; r < RPG; ++r) {
+            const F2 ex = X[r * NT + threadIdx.x];
+            dq[r] = f2_mul(f2_mul(*reinterpret_cast<const F2*>(EQ + (r0 + r) * SM::EP + 2 * pr), ex), cc);
+            dk[r] = f2_mul(*reinterpret_cast<const F2*>(EK + (r0 + r) * SM::EP + 2 * pr), f2_make(tc::rcp(f2_lo(ex)), tc::rcp(f2_hi(ex))));
+            e[r] = f2_fma(f2_mul(dk[r], minus), k[r].f2(), f2_mul(dq[r], q[r].f2()));
+            sum = f2_add(sum, e[r]);
         }
-        __syncthreads();                                                // the tiles, gsum and carry may be rewritten
+        *reinterpret_cast<F2*>(gsum + gr * DK + 2 * pr) = sum;
+        __syncthreads();
+        if (both) cluster_arrive();                                      // my X and K tiles may be written by the other direction
+        F2 run = have_states ? *reinterpret_cast<const F2*>(carry + 2 * pr) : zero;
+#pragma unroll
+        for (int o = 0; o < CL::GROUPS; ++o)
+            if (dir ? o < gr : o > gr) run = f2_add(run, *reinterpret_cast<const F2*>(gsum + o * DK + 2 * pr));
+        // static register indices for both orders: the backward direction sums upwards, the forward one downwards
+        if (dir) {
+#pragma unroll
+            for (int r = 0; r < RPG; ++r) e[r] = run = f2_add(run, e[r]);
+        } else {
+#pragma unroll
+            for (int r = RPG - 1; r >= 0; --r) e[r] = run = f2_add(run, e[r]);
+        }
+        rows_through_gate(e, x, p.gate_norm, p.clamp_min);
+    } else {                                                             // the other direction waits for its share all the same
+#pragma unroll
+        for (int r = 0; r < RPG; ++r) dq[r] = dk[r] = zero;
+        if (both) cluster_arrive();
     }
-    if (threadIdx.x == 0) p.flags[(size_t)bh * p.nchunk + c] = 0;
+    // ---- the other direction's share: rank 0 (forward) finishes dq and rows 0 - 31 of dv, rank 1 dk and rows 32 - 63
+    constexpr int VPT = C / 2 * DV / NT, VTR = DV / VPT;                 // columns of dv a thread sends or finishes, threads of a row
+    const int vr = threadIdx.x / VTR, vc = threadIdx.x % VTR * VPT;
+    const float* D0 = reinterpret_cast<const float*>(smem + SM::V);
+    const float* D1 = reinterpret_cast<const float*>(smem + SM::S);
+    if (both) {
+        cluster_wait();
+        const uint32_t peer = tc::map_rank(sb, dir ^ 1), bar = peer + SM::BAR;
+#pragma unroll
+        for (int r = 0; r < RPG; r += 2) {
+            const F2 u = dir ? dq[r] : dk[r], v = dir ? dq[r + 1] : dk[r + 1];
+            send(peer + SM::X + (r / 2 * NT + threadIdx.x) * 16, f2_lo(u), f2_hi(u), f2_lo(v), f2_hi(v), bar);
+        }
+        const int row = vr + (dir ? 0 : C / 2);
+#pragma unroll
+        for (int i = 0; i < VPT; i += 4) {
+            const float4 a = *reinterpret_cast<const float4*>(D0 + row * SM::VP + vc + i), z = *reinterpret_cast<const float4*>(D1 + row * SM::VP + vc + i);
+            send(peer + SM::K + (vr * DV + vc + i) * 4, a.x + z.x, a.y + z.y, a.z + z.z, a.w + z.w, bar);
+        }
+    }
+    if (!bad) {
+        T* out = reinterpret_cast<T*>(dir ? p.dgb : p.dgf) + ((int64_t)bh * p.L + t0 + r0) * DK + 2 * pr;
+#pragma unroll
+        for (int r = 0; r < RPG; ++r)
+            if (r0 + r < n) store2<T>(out + r * DK, f2_lo(e[r]), f2_hi(e[r]));
+    }
+    if (both) {                                                          // bounded: about a second, then the chunk is left to the exact form like one out of range
+        int tries = 0;
+        while (!tc::mbar_try_wait_parked(sb + SM::BAR, 0, 2000u) && tries < 1 << 19) ++tries;
+        bad = __syncthreads_or(bad || tries >= 1 << 19);
+    }
+    // a half of the flag for each direction: a chunk that either leaves is left whole, outputs included
+    if (threadIdx.x == 0) {
+        int32_t* flag = p.flags + (size_t)bh * p.nchunk + c;
+        if (both) reinterpret_cast<int16_t*>(flag)[dir] = bad;
+        else *flag = bad;
+    }
+    if (bad) return;
+    const int64_t base = ((int64_t)bh * p.L + t0 + r0) * DK + 2 * pr;
 #pragma unroll
     for (int r = 0; r < RPG; ++r) {
-        if (r0 + r >= n) break;
-        const int64_t at = ((int64_t)bh * p.L + t0 + r0 + r) * DK + 2 * pr;
-        store2<T>(reinterpret_cast<T*>(p.out_dq) + at, f2_lo(dqt[r]), f2_hi(dqt[r]));
-        store2<T>(reinterpret_cast<T*>(p.out_dk) + at, f2_lo(dkt[r]), f2_hi(dkt[r]));
-    }
-    float* D = reinterpret_cast<float*>(smem + SM::K) + fr * SM::VP + fc;    // the two parts of dV meet in shared memory
-    if (role == 0) {
-#pragma unroll
-        for (int i = 0; i < DV / 8; ++i) {
-            *reinterpret_cast<float2*>(D + 8 * i) = make_float2(dv[i][0], dv[i][1]);
-            *reinterpret_cast<float2*>(D + 8 * SM::VP + 8 * i) = make_float2(dv[i][2], dv[i][3]);
+        if (r0 + r < n) {
+            if (both) {
+                const F2 v = f2_add(dir ? dk[r] : dq[r], X[(r / 2 * NT + threadIdx.x) * 2 + (r & 1)]);
+                store2<T>(reinterpret_cast<T*>(dir ? p.out_dk : p.out_dq) + base + r * DK, f2_lo(v), f2_hi(v));
+            } else {
+                store2<T>(reinterpret_cast<T*>(p.out_dq) + base + r * DK, f2_lo(dq[r]), f2_hi(dq[r]));
+                store2<T>(reinterpret_cast<T*>(p.out_dk) + base + r * DK, f2_lo(dk[r]), f2_hi(dk[r]));
+            }
         }
     }
-    __syncthreads();
-    if (role == 0) return;
+    const float* sent = reinterpret_cast<const float*>(smem + SM::K) + vr * DV + vc;
+    for (int row = vr + (both && dir ? C / 2 : 0); row < (both && !dir ? C / 2 : C); row += C / 2) {
+        if (row >= n) break;
+        T* out = reinterpret_cast<T*>(p.out_dv) + ((int64_t)bh * p.L + t0 + row) * DV + vc;
 #pragma unroll
-    for (int hf = 0; hf < 2; ++hf) {
-        const int row = fr + 8 * hf;
-        if (row >= n) continue;
-        T* out = reinterpret_cast<T*>(p.out_dv) + ((int64_t)bh * p.L + t0 + row) * DV + fc;
-#pragma unroll
-        for (int i = 0; i < DV / 8; ++i) {
-            const float2 o = *reinterpret_cast<const float2*>(D + 8 * hf * SM::VP + 8 * i);
-            store2<T>(out + 8 * i, dv[i][2 * hf] + o.x, dv[i][2 * hf + 1] + o.y);
+        for (int i = 0; i < VPT; i += 4) {
+            float4 a = *reinterpret_cast<const float4*>(D0 + row * SM::VP + vc + i);
+            const float4 z = *reinterpret_cast<const float4*>(D1 + row * SM::VP + vc + i);
+            a.x += z.x; a.y += z.y; a.z += z.z; a.w += z.w;
+            if (both) { const float4 s = *reinterpret_cast<const float4*>(sent + i); a.x += s.x; a.y += s.y; a.z += s.z; a.w += s.w; }
+            store2<T>(out + i, a.x, a.y); store2<T>(out + i + 2, a.z, a.w);
         }
     }
 }
@@ -477,7 +527,15 @@ int launch_typed(const BwdParams& p, cudaStream_t stream) {
         if (int s = bigla_bwd_scan_launch(p, stream)) return s;
     }
     if ((e = tc::ensure_smem_attr(reinterpret_cast<const void*>(kC), (int)smC)) != cudaSuccess) return (int)e;
-    return (int)launch_overlapped(p.nchunk > 1, kC, dim3(p.nchunk, BH), dim3(NT), smC, stream, p);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((p.dir_mask == 3 ? 2 : 1) * p.nchunk, BH); cfg.blockDim = dim3(NT); cfg.dynamicSmemBytes = smC; cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    int na = 0;
+    if (p.nchunk > 1) { attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[na++].val.programmaticStreamSerializationAllowed = 1; }
+    if (p.dir_mask == 3) { attr[na].id = cudaLaunchAttributeClusterDimension; attr[na].val.clusterDim.x = 2; attr[na].val.clusterDim.y = attr[na].val.clusterDim.z = 1; ++na; }
+    cfg.attrs = attr; cfg.numAttrs = na;
+    e = cudaLaunchKernelEx(&cfg, kC, p);
+    return (int)(e != cudaSuccess ? e : cudaGetLastError());
 }
 
 template <typename T>

@@ -280,7 +280,7 @@ template <int RPG, typename T> __device__ __forceinline__ void rows_through_gate
 }
 
 // Inclusive cumulative log-gates of the chunk in scan order (log2 units): G[r] of my rows; also the sum at the chunk's
-// middle (reference of the factorisation) and the total.  gsum: GROUPS x DK floats of shared memory; contains two barriers.
+// middle (reference of the factorisation) and the total.  gsum: GROUPS x DK floats of shared memory, written again only behind the caller's next barrier; contains one.
 template <int DK, typename T> __device__ __forceinline__ void cum_gates(F2 (&G)[ColLay<DK>::RPG], F2& ref, F2& tot, float* gsum, const Raw2<T> (&x)[ColLay<DK>::RPG],
                                                                         int n, int dir, float gate_norm, float clamp_min) {
     using CL = ColLay<DK>;
@@ -302,7 +302,6 @@ template <int DK, typename T> __device__ __forceinline__ void cum_gates(F2 (&G)[
         if (o == CL::GROUPS / 2) lo = sum;
         sum = f2_add(sum, *reinterpret_cast<const F2*>(gsum + o * DK + 2 * pr));
     }
-    __syncthreads();
     tot = sum;
     if (dir) {                                                           // total minus everything before the row
         ref = f2_fma(lo, minus, sum);
@@ -423,6 +422,23 @@ template <int KD, int NA, int NB> __device__ __forceinline__ void block_nt(float
     }
 }
 
+// A operand of my 16 rows, all k steps
+template <int KD, int NA> __device__ __forceinline__ void load_a(uint32_t (*fa)[NA][4], uint32_t a, uint32_t a_term) {
+#pragma unroll
+    for (int ks = 0; ks < KD / 16; ++ks)
+#pragma unroll
+        for (int t = 0; t < NA; ++t) ldsm4(a + t * a_term + ks * 32, fa[ks][t]);
+}
+// as block_nt with the A operand at hand
+template <int KD, int NA, int NB> __device__ __forceinline__ void block_nt(float (*acc)[4], const uint32_t (*fa)[NA][4], uint32_t b, uint32_t b_term) {
+#pragma unroll
+    for (int ks = 0; ks < KD / 16; ++ks) {
+        uint32_t fb[2][NB][2];
+        load_b_nt<NB, 2, 0>(fb, b + ks * 32, b_term);
+        mma_group<NA, NB, 2>(acc, fa[ks], fb);
+    }
+}
+
 // zero the entries of a diagonal 16 x 16 block that ``keep(row, col)`` rejects, then split it into an A operand
 template <int SC, typename F> __device__ __forceinline__ void mask_split(float (*p)[4], bool diag, int lane, F keep, uint32_t (*out)[4]) {
     if (diag) {
@@ -458,21 +474,17 @@ template <int ND, int NA, int NB> __device__ __forceinline__ void block_nn(float
     }
 }
 
-// acc[ND/8][4] += A B^T over KD: A = my 16 rows of an [m][k] tile, B an [n][k] tile of ND rows with pitch PB
-template <int ND, int KD, uint32_t PB, int NA, int NB> __device__ __forceinline__ void rows_nt(float (*acc)[4], uint32_t a, uint32_t a_term, uint32_t b, uint32_t b_term) {
+// acc[ND/8][4] += A B^T over KD: A = my 16 rows, all k steps, B an [n][k] tile of ND rows with pitch PB
+template <int ND, int KD, uint32_t PB, int NA, int NB> __device__ __forceinline__ void rows_nt(float (*acc)[4], const uint32_t (*fa)[NA][4], uint32_t b, uint32_t b_term) {
     constexpr int G = Group<ND / 8>::G;
 #pragma unroll
-    for (int ks = 0; ks < KD / 16; ++ks) {
-        uint32_t fa[NA][4];
-#pragma unroll
-        for (int t = 0; t < NA; ++t) ldsm4(a + t * a_term + ks * 32, fa[t]);
+    for (int ks = 0; ks < KD / 16; ++ks)
 #pragma unroll
         for (int n = 0; n < ND / 8; n += G) {
             uint32_t fb[G][NB][2];
             load_b_nt<NB, G, PB>(fb, b + n * 8 * PB + ks * 32, b_term);
-            mma_group<NA, NB, G>(acc + n, fa, fb);
+            mma_group<NA, NB, G>(acc + n, fa[ks], fb);
         }
-    }
 }
 
 }  // namespace mm
