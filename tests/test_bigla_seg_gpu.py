@@ -88,3 +88,25 @@ def test_bf16_rounds_no_more_often_than_the_tcgen05_form(dk, B, H, L):
     ref = oracle.chunked_bi_gla_f64(*[t.double() for t in ins])
     err = {impl: float((vig_b200.bi_gla(*[t.cuda() for t in ins], impl=impl).double().cpu() - ref).norm() / ref.norm()) for impl in (_lib.IMPL_SEG, _lib.IMPL_TC_SPLIT)}
     assert err[_lib.IMPL_SEG] < 1.1 * err[_lib.IMPL_TC_SPLIT], err
+
+
+@pytest.mark.parametrize("dtype,dk,dv", [(torch.float32, 64, 64), (torch.float32, 32, 64), (torch.float16, 64, 64), (torch.bfloat16, 16, 32)])
+@pytest.mark.parametrize("L", [65, 96, 97, 480, 512])
+def test_small_calls_in_segments_of_32(dtype, dk, dv, L):
+    """Up to 16 segments of 32 tokens a cluster, states at both ends, a direction out of the factorised range in the middle; a workspace for
+    64-token segments, which earlier callers hold, gives the same."""
+    import vig_b200
+    from vig_b200 import _lib
+    q, k, v, gf, gb = oracle.make_bigla_inputs(1, 2, L, dk, dv, seed=L)
+    gb[:, 1, 32:64] *= 200
+    ins = [t.to(dtype) for t in (q, k, v, gf, gb)]
+    ref = oracle.naive_bi_gla(*[t.float() for t in ins])
+    dev = [t.cuda() for t in ins]
+    tol = 2e-3 if dtype == torch.float16 else TOL[dtype]
+    assert rel_err(vig_b200.bi_gla(*dev, impl=_lib.IMPL_SEG).float(), ref) < tol
+    need = [_lib.lib().vig_bigla_workspace_bytes(1, 2, L, dk, dv, _lib.dtype_code(dev[0]), i) for i in (_lib.IMPL_SEG, _lib.IMPL_SIMT)]
+    assert need[0] > need[1] or L % 64 == 0
+    ws, o = torch.empty(need[1], dtype=torch.uint8, device="cuda"), torch.empty(1, 2, L, dv, device="cuda", dtype=dtype)
+    st = _lib.lib().vig_bigla_fwd(*map(_lib.ptr, dev), _lib.ptr(o), 1, 2, L, dk, dv, _lib.dtype_code(o), *[None] * 6, -1.0, 1.0, 0.0, float("nan"), *[None] * 6, 3,
+                                  _lib.IMPL_SEG, _lib.ptr(ws), need[1], None, _lib.stream_ptr())
+    assert st == 0 and rel_err(o.float(), ref) < tol

@@ -52,7 +52,9 @@ size_t vig::bigla_workspace_internal(int B, int H, int L, int dk, int dv, int dt
     size_t wave = (dtype != VIG_DTYPE_F32 && (impl == VIG_IMPL_TC_WAVE || impl == VIG_IMPL_AUTO) && (dk == 64 || dk == 32) && dv == 64) ? bigla_wave_workspace(B, H, L, dk, dv) : 0;
     if (impl == VIG_IMPL_TC_WAVE) return wave;
     if (no_single) wave = 0;
+    const size_t seg = !no_single && (impl == VIG_IMPL_AUTO || impl == VIG_IMPL_SEG) ? bigla_seg_workspace(B, H, L, dk, dv, dtype) : 0;
     size_t m = simt > tc ? simt : tc;
+    if (seg > m) m = seg;
     return m > wave ? m : wave;
 }
 
@@ -125,7 +127,7 @@ int vig::bigla_fwd_internal(const void* q, const void* k, const void* v, const v
         if (!bigla_seg_supported(p)) return VIG_ERR_SHAPE;
         if (!seg_runs) return workspace && workspace_bytes >= bigla_simt_workspace(B, H, L, dk, dv) ? VIG_ERR_ALIGN : VIG_ERR_WORKSPACE;
         p.ws_state = reinterpret_cast<float*>(workspace);
-        return bigla_seg_launch(p, (cudaStream_t)stream);
+        return bigla_seg_launch(p, ws_fits ? workspace_bytes : 0, (cudaStream_t)stream);
     }
     if (impl == VIG_IMPL_AUTO && !no_single && bigla_wave_supported(p) && bigla_wave_preferred(p) && workspace &&
         !(reinterpret_cast<uintptr_t>(workspace) & 255) && workspace_bytes >= bigla_wave_workspace(B, H, L, dk, dv))

@@ -13,7 +13,7 @@
 //
 // Against the two-CTAs-per-SM tcgen05 form, which walks 128-token chunks one after the other in each direction with a tensor
 // memory round trip for the scores: P stays in registers, a segment's rows spread over all warps at once.  One segment takes
-// about 22 k cycles alone (loads and gates 6, tiles 3, contribution 4, products 3, states 3, read-out 2): a call of few
+// about 22 k cycles alone in fp32 (loads and gates 5, tiles 3, contribution 5, products 5, states 4; 10 k in bf16): a call of few
 // segments is that latency, one of many is bound by instruction issue at 16 warps an SM.
 // Operands are split into bf16 terms (mma_common.cuh): one term for bf16 with dv = 64 (as in the two-CTAs-per-SM tcgen05 form), two for
 // fp16 and for dv = 32, three for fp32.  A segment whose |G - r| leaves the factorisation's range, contribution included,
@@ -35,16 +35,19 @@ template <int DK, int DV, typename T> struct SegTerms {
 
 // Warps that share 16 rows, each with its part of the value columns (the scores are formed by each of them): two for fp32, whose
 // three-term tiles leave room for one or two 64-token segments an SM (2x3x196 64/64: 28.4 -> 19.5 us; 16x6x1000 64/64: 520 ->
-// 320).  16-bit inputs have two or three segments an SM and gain nothing from repeating the scores.
-template <typename T> struct SegWarps { static constexpr int CW = sizeof(T) == 4 ? 2 : 1; };
+// 320), and for 16-bit segments of 64 tokens, which are for calls that leave SMs idle (1x3x196 32/64, bf16: 10.3 -> 8.8 us one call behind
+// another); twice as many for segments of 32 tokens.  Other 16-bit calls have two or three segments an SM and gain nothing from repeating
+// the scores.
+template <int DV, typename T, int TOK> struct SegWarps {
+    static constexpr int CW = (sizeof(T) == 4 ? 2 : TOK == 32 || (TOK == 64 && DV == 64) ? 2 : 1) * (sizeof(T) == 4 && TOK == 32 ? 2 : 1);
+};
 
 template <int DK, int DV, typename T, int TOK> struct SegSmem {
     using TT = SegTerms<DK, DV, T>;
-    static constexpr uint32_t QT = TT::SC * TOK * Pitch<DK>::B;        // one direction's Q or K terms
+    static constexpr uint32_t QT = TT::SC * (TOK * Pitch<DK>::B > DK * Pitch<DV>::B ? TOK * Pitch<DK>::B : DK * Pitch<DV>::B);   // one direction's Q or K terms, or its entering state
     static constexpr uint32_t V = 0, K = TT::RAW * TOK * Pitch<DV>::B, Q = K + 2 * QT, SUM = Q + 2 * QT,
-                              SCL = SUM + 2 * (TOK / 16) * SegWarps<T>::CW * DK * 4,      // per direction and warp: summed log-gates of the warp's rows
+                              SCL = SUM + 2 * (TOK / 16) * SegWarps<DV, T, TOK>::CW * DK * 4,      // per direction and warp: summed log-gates of the warp's rows
                               BYTES = SCL + 4 * DK * 4;                 // [dir][0: 2^r, 1: 2^(l-r)]
-    static_assert(TT::SC * DK * Pitch<DV>::B <= QT, "the entering states reuse the K tiles");
 };
 
 // x * e of a raw pair and a pair of fp32 factors, in SC bf16 terms: the product in fp32, then rounded
@@ -53,9 +56,8 @@ template <typename T, int SC> __device__ __forceinline__ void scaled(const Raw2<
     split2<SC>(f2_lo(v), f2_hi(v), t);
 }
 
-template <typename T, int COLS, int TERMS, int TOK> __device__ __forceinline__ void seg_load_v(uint8_t* dst, const T* src, int64_t stride_l, int n, float& mark) {
+template <typename T, int COLS, int TERMS, int TOK, int NTH> __device__ __forceinline__ void seg_load_v(uint8_t* dst, const T* src, int64_t stride_l, int n, float& mark) {
     constexpr uint32_t P = Pitch<COLS>::B;
-    constexpr int NTH = 2 * TOK * SegWarps<T>::CW;
     if constexpr (TERMS == 1) {
         constexpr int VPR = COLS / 8;
 #pragma unroll
@@ -97,6 +99,7 @@ struct SegParams {
     BiglaParams p;
     int nseg, seglen;            // segments per sequence, tokens per segment (a multiple of 16; the last one may be shorter)
     int need_states;             // contributions are wanted (more than one segment, or final states)
+    int finals;                  // final states or summed log-gates are wanted
 };
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
@@ -127,7 +130,7 @@ template <int DK, int DV, int MODE> __device__ __forceinline__ float4 entering(c
 // threads to a segment, 0.83 with all (1.19 in the gate-independent form of bigla_simt.cu).  The segment's tiles give up their shared memory.
 template <int DK, int DV, typename T, int TOK> struct SegExact {
     using SM = SegSmem<DK, DV, T, TOK>;
-    using L = rec::Lay<DK, DV, 2 * TOK * SegWarps<T>::CW>;
+    using L = rec::Lay<DK, DV, 2 * TOK * SegWarps<DV, T, TOK>::CW>;
     static constexpr uint32_t ROW = 3 * DK + DV;                         // floats staged for a token
     static constexpr uint32_t bytes(int sub) { return (L::HALVES * sub * ROW + TOK * DV) * 4; }
     static constexpr int SUB = bytes(32) <= SM::SUM ? 32 : bytes(16) <= SM::SUM ? 16 : 8;      // tokens staged at a time
@@ -258,14 +261,14 @@ template <int DK, int DV, typename T, int TOK, int MODE> __device__ __noinline__
 }
 
 template <int DK, int DV, typename T, int TOK> constexpr int seg_min_blocks() {
-    constexpr int fit = 225 * 1024 / (int)(SegSmem<DK, DV, T, TOK>::BYTES + 1024), regs = (DK == 16 ? 640 : 512) / (2 * TOK * SegWarps<T>::CW);   // 128 registers a thread, 96 at DK = 16
+    constexpr int fit = 225 * 1024 / (int)(SegSmem<DK, DV, T, TOK>::BYTES + 1024), regs = (DK == 16 ? 640 : 512) / (2 * TOK * SegWarps<DV, T, TOK>::CW);   // 128 registers a thread, 96 at DK = 16
     return fit < 1 ? 1 : fit < regs ? fit : regs;
 }
 
 template <int DK, int DV, typename T, int TOK, int MODE>
-__global__ void __launch_bounds__(2 * TOK * SegWarps<T>::CW, seg_min_blocks<DK, DV, T, TOK>()) bigla_seg_kernel(const __grid_constant__ SegParams s) {
+__global__ void __launch_bounds__(2 * TOK * SegWarps<DV, T, TOK>::CW, seg_min_blocks<DK, DV, T, TOK>()) bigla_seg_kernel(const __grid_constant__ SegParams s) {
     using SM = SegSmem<DK, DV, T, TOK>;
-    constexpr int RAW = SM::TT::RAW, SC = SM::TT::SC, CW = SegWarps<T>::CW, NTH = 2 * TOK * CW, W = NTH / 32, DC = DV / CW;   // DC: a warp's value columns
+    constexpr int RAW = SM::TT::RAW, SC = SM::TT::SC, CW = SegWarps<DV, T, TOK>::CW, NTH = 2 * TOK * CW, W = NTH / 32, DC = DV / CW;   // DC: a warp's value columns
     constexpr int PAIRS = DK / 2, SUB = 32 / PAIRS, RPG = 16 / CW / SUB, MT = DK / 16;   // a warp's gates: 16 / CW rows, SUB groups of RPG
     constexpr uint32_t PK = Pitch<DK>::B, PV = Pitch<DV>::B, TK = TOK * PK, TV = TOK * PV, TS = DK * PV;   // TK, TV, TS: from term to term
     const BiglaParams& p = s.p;
@@ -290,7 +293,7 @@ __global__ void __launch_bounds__(2 * TOK * SegWarps<T>::CW, seg_min_blocks<DK, 
         constexpr bool CHECK = sizeof(T) == 4 || DV == 32;
         float mark = 0.f;
         F2 seen = f2_make(0.f, 0.f);
-        seg_load_v<T, DV, RAW, TOK>(smem + SM::V, head_ptr<T>(p.v, p.sv, b, h, t0), p.sv[2], n, mark);
+        seg_load_v<T, DV, RAW, TOK, NTH>(smem + SM::V, head_ptr<T>(p.v, p.sv, b, h, t0), p.sv[2], n, mark);
         const bool logits = p.gate_norm > 0.f, clamp = p.clamp_min == p.clamp_min;
         Raw2<T> qr[RPG];
         {
@@ -334,14 +337,12 @@ __global__ void __launch_bounds__(2 * TOK * SegWarps<T>::CW, seg_min_blocks<DK, 
                         G[dir][r] = run;
                     }
                 } else {
-                    const float inv = logits ? 1.f / p.gate_norm : 0.f;
+                    row_gates(G[dir], xr[dir], p.gate_norm, p.clamp_min);
                     float top = 0.f;
 #pragma unroll
                     for (int rr = 0; rr < RPG; ++rr) {
                         const int r = dir ? RPG - 1 - rr : rr;
-                        const F2 x = xr[dir][r].f2();
-                        const float gx = gate_log2<T>(f2_lo(x), p.gate_norm, inv, p.clamp_min), gy = gate_log2<T>(f2_hi(x), p.gate_norm, inv, p.clamp_min);
-                        if (r0 + r < n && (dir ? bwd : fwd)) { top = fmaxf(top, fmaxf(gx, gy)); run = f2_add(run, f2_make(gx, gy)); }
+                        if (r0 + r < n && (dir ? bwd : fwd)) { top = fmaxf(top, fmaxf(f2_lo(G[dir][r]), f2_hi(G[dir][r]))); run = f2_add(run, G[dir][r]); }
                         G[dir][r] = run;
                     }
                     fine = fine && top <= 0.f;                            // growing gates: G is not monotone, its ends do not bound it
@@ -520,7 +521,7 @@ __global__ void __launch_bounds__(2 * TOK * SegWarps<T>::CW, seg_min_blocks<DK, 
         if (MODE == SEG_OUT) pdl_wait();                                 // all before this overlaps the scan over segments
         __syncthreads();
     }
-    if (MODE == SEG_ONE && s.need_states) {
+    if (MODE == SEG_ONE && s.finals) {
 #pragma unroll 1
         for (int dir = 0; dir < 2; ++dir) {                              // final states, summed log-gates: by the segment scanned last
             float* fin = dir ? p.final_b : p.final_f;
@@ -632,7 +633,7 @@ int seg_launch_mode(const SegParams& s, cudaStream_t stream) {
     if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(s.nseg, s.p.B * s.p.H);
-    cfg.blockDim = dim3(2 * TOK * SegWarps<T>::CW);
+    cfg.blockDim = dim3(2 * TOK * SegWarps<DV, T, TOK>::CW);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     if (MODE == SEG_OUT) return (int)launch_next(kern, cfg.gridDim, cfg.blockDim, smem, stream, s);
@@ -667,8 +668,8 @@ int seg_launch(SegParams& s, cudaStream_t stream) {
     s.nseg = (p.L + TOK - 1) / TOK;
     s.seglen = ((p.L + s.nseg - 1) / s.nseg + 15) / 16 * 16;   // even segments: no nearly empty last one
     s.nseg = (p.L + s.seglen - 1) / s.seglen;
-    const bool finals = p.final_f || p.final_b || p.logdecay_f || p.logdecay_b;
-    s.need_states = s.nseg > 1 || finals;
+    s.finals = p.final_f || p.final_b || p.logdecay_f || p.logdecay_b;
+    s.need_states = s.nseg > 1 || s.finals;
     p.nchunk = s.nseg;
     p.ws_decay = p.ws_state ? p.ws_state + (size_t)p.B * p.H * s.nseg * 2 * DK * DV : nullptr;
     if (s.nseg <= CLUSTER) {
@@ -682,8 +683,8 @@ int seg_launch(SegParams& s, cudaStream_t stream) {
 
 template <int DK, int DV, typename T>
 int seg_launch_tok(SegParams& s, int tok, cudaStream_t stream) {
-    if constexpr (sizeof(T) == 4) return seg_launch<DK, DV, T, 64>(s, stream);
-    else if constexpr (DV == 32) return seg_launch<DK, DV, T, 64>(s, stream);
+    if constexpr (SegTerms<DK, DV, T>::SC > 1) if (tok == 32) return seg_launch<DK, DV, T, 32>(s, stream);
+    if constexpr (sizeof(T) == 4 || DV == 32) return seg_launch<DK, DV, T, 64>(s, stream);
     else return tok == 64 ? seg_launch<DK, DV, T, 64>(s, stream) : seg_launch<DK, DV, T, 128>(s, stream);
 }
 
@@ -725,14 +726,29 @@ bool bigla_seg_preferred(const BiglaParams& p) {
     return segs <= (p.dk == 32 ? (p.L <= 256 ? 1600 : p.L <= 1024 ? 600 : 400) : p.L <= 1024 ? 400 : 200);
 }
 
-int bigla_seg_launch(const BiglaParams& p, cudaStream_t stream) {
+// Segments of 32 tokens: calls of few segments, whose operands have two or three terms (bigla_seg_launch says why).
+static bool seg_fine(int dtype, int dv, int L) { return !(dtype == VIG_DTYPE_BF16 && dv == 64) && L > 64 && L <= 512; }
+static size_t seg_fine_bytes(int64_t BH, int L, int dk, int dv) { return (size_t)BH * ((L + 31) / 32) * 2 * ((size_t)dk * dv + dk) * sizeof(float); }
+
+size_t bigla_seg_workspace(int B, int H, int L, int dk, int dv, int dtype) {
+    const int64_t BH = (int64_t)B * H;
+    return seg_fine(dtype, dv, L) && BH * ((L + 31) / 32) <= 256 ? seg_fine_bytes(BH, L, dk, dv) : 0;   // asked without a device: a bound for all
+}
+
+int bigla_seg_launch(const BiglaParams& p, size_t ws_bytes, cudaStream_t stream) {
     SegParams s{};
     s.p = p;
     // 64-token segments where more SMs can share the work of few sequences (1x3x196 dk = 64: 11 us against 13) and for dv = 32,
-    // whose segments are too little work for eight warps (64x12x196 dk = 16: 47 us against 57); otherwise 128, half as many states
-    const int tok = p.dv == 32 || p.L <= 64 || (p.L <= 512 && (int64_t)p.B * p.H * ((p.L + 63) / 64) <= device_sms()) ? 64 : 128;
+    // whose segments are too little work for eight warps (64x12x196 dk = 16: 47 us against 57); otherwise 128, half as many states.
+    // 32 tokens where operands have two or three terms and all segments find an SM of their own, clusters placed whole (us of a launch at 32 / 64
+    // tokens): fp32 2x3x196 64/64 14.4 / 19.9, 4x3x256 32/64 11.9 / 13.2, 2x3x512 16/32 9.3 / 10.2; fp16 1x3x196 32/64 9.0 / 10.4, but 3x3x480 (135
+    // segments) 12.4 / 11.5; bf16 32/32 2x12x128 7.8 / 9.0; fp16 16/32 1x24x49 6.5 / 5.9.  One-term operands gain nothing: bf16 1x3x196 32/64 8.4 / 8.5,
+    // 1x12x196 64/64 11.9 / 11.1.
+    const int64_t BH = (int64_t)p.B * p.H;
+    const int tok = seg_fine(p.dtype, p.dv, p.L) && 3 * BH * ((p.L + 31) / 32) <= 2 * device_sms() && ws_bytes >= seg_fine_bytes(BH, p.L, p.dk, p.dv) ? 32
+                    : p.dtype == VIG_DTYPE_F32 || p.dv == 32 || p.L <= 64 || (p.L <= 512 && BH * ((p.L + 63) / 64) <= device_sms()) ? 64 : 128;
     switch (p.dtype) {
-        case VIG_DTYPE_F32: return seg_launch_dims<float>(s, 64, stream);
+        case VIG_DTYPE_F32: return seg_launch_dims<float>(s, tok, stream);
         case VIG_DTYPE_BF16: return seg_launch_dims<__nv_bfloat16>(s, tok, stream);
         case VIG_DTYPE_F16: return seg_launch_dims<__half>(s, tok, stream);
     }

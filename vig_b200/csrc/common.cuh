@@ -199,7 +199,8 @@ size_t bigla_simt_workspace(int B, int H, int L, int dk, int dv);
 // mma.sync form, both directions of a segment in one sweep (short and medium sequences, dv = 32, fp32)
 bool bigla_seg_supported(const BiglaParams& p);
 bool bigla_seg_preferred(const BiglaParams& p);
-int bigla_seg_launch(const BiglaParams& p, cudaStream_t stream);
+int bigla_seg_launch(const BiglaParams& p, size_t ws_bytes, cudaStream_t stream);
+size_t bigla_seg_workspace(int B, int H, int L, int dk, int dv, int dtype);   // with which small calls run in their finest segments; bigla_simt_workspace is enough
 // scan over p.nchunk per-chunk (or per-segment) local states in the workspace, in place (phase B)
 int bigla_scan_launch(const BiglaParams& p, cudaStream_t stream);
 int bigla_tc_launch(const BiglaParams& p, void* ws, size_t ws_bytes, bool allow_fused, cudaStream_t stream);
