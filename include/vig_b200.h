@@ -150,6 +150,17 @@ VIG_API int vig_bigla_bwd_full(const void* q, const void* k, const void* v, cons
                   void* workspace, size_t workspace_bytes, void* stream);
 
 /*
+ * Depthwise 3x3 convolution and the stacked input projection of a block in one launch, bf16 / fp16, C = 96 or 192, N a multiple of C:
+ * xs = vig_dwconv3x3_fwd(x, taps, conv_bias), z = xs W^T + bias (classification/models/vig.py:427-433), with the roundings of the separate calls.
+ * x, xs: [B, h, wd, C]; taps [9, C]; w [N, C]; z [B, h*wd, N]; conv_bias [C] and bias [N] may be NULL; all on 16 bytes.
+ * ``preferred``: whether it beats the separate calls at M = B*h*wd tokens.
+ */
+VIG_API int vig_conv_proj_supported(int64_t M, int C, int N, int dtype);
+VIG_API int vig_conv_proj_preferred(int64_t M, int C, int N, int dtype);
+VIG_API int vig_conv_proj_fwd(const void* x, const void* taps, const void* conv_bias, const void* w, const void* bias, void* xs, void* z, int B, int h, int wd, int C, int N,
+                              int act_silu, int dtype, void* stream);
+
+/*
  * The row-local half of a block of width 192 (3 heads of 64) in one kernel, bf16 / fp16, any M: y = gating injection of
  * (o, local, gate_logits) as vig_gate_inject_fwd, r = y W_o^T + residual, h = RMSNorm(r) * norm_w,
  * z = swiglu(h W_gate^T) as vig_linear_swiglu_fwd, out_r = z W_down^T + r, out_h = RMSNorm(out_r) * next_w

@@ -47,6 +47,9 @@ _SIGNATURES = {
     "vig_embed_conv_ln_fwd": (c_int, [c_void_p] * 6 + [c_int] * 4 + [c_float, c_int, c_int, c_void_p]),
     "vig_token_mean_fwd": (c_int, [c_void_p] * 2 + [c_int] * 4 + [c_void_p]),
     "vig_chain_launches": (c_int, [c_int]),
+    "vig_conv_proj_supported": (c_int, [c_int64] + [c_int] * 3),
+    "vig_conv_proj_preferred": (c_int, [c_int64] + [c_int] * 3),
+    "vig_conv_proj_fwd": (c_int, [c_void_p] * 7 + [c_int] * 7 + [c_void_p]),
     "vig_block_tail_supported": (c_int, [c_int64] + [c_int] * 4),
     "vig_block_tail_preferred": (c_int, [c_int64] + [c_int] * 4),
     "vig_block_tail_fwd": (c_int, [c_void_p] * 3 + [c_int64] + [c_void_p] * 2 + [c_float, c_int] + [c_void_p] * 3 + [c_float] + [c_void_p] * 3 +

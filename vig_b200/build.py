@@ -10,7 +10,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libvig_b200.so")
 HOST = os.path.join(HERE, "_host.so")
 HOST_SOURCES = ["host_ops.cpp", "host_model.cpp"]
-SOURCES = ["abi.cu", "bigla_simt.cu", "bigla_tc.cu", "bigla_wave.cu", "elementwise.cu", "noalloc.cu", "bigla_bwd_simt.cu", "bigla_bwd_mma.cu", "bigla_seg.cu", "block_tail.cu", "embed_conv.cu", "gemm_swiglu.cu", "gemm_pair.cu", "gemm_pair_norm.cu", "gemm_addnorm.cu", "dwconv_tma.cu", "gemm_bias.cu", "gemm_stem.cu"]
+SOURCES = ["abi.cu", "bigla_simt.cu", "bigla_tc.cu", "bigla_wave.cu", "elementwise.cu", "noalloc.cu", "bigla_bwd_simt.cu", "bigla_bwd_mma.cu", "bigla_seg.cu", "block_tail.cu", "conv_proj.cu", "embed_conv.cu", "gemm_swiglu.cu", "gemm_pair.cu", "gemm_pair_norm.cu", "gemm_addnorm.cu", "dwconv_tma.cu", "gemm_bias.cu", "gemm_stem.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]
 

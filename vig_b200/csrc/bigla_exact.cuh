@@ -47,11 +47,11 @@ __device__ __forceinline__ void stage(float* sq, float* sk, float* sv, float* lg
 #pragma unroll
         for (int e = 0; e < VP; ++e) xv[e] = xq;
         if (r < n) {
-            xk = mm::load2<T>(k + r * lk + c);
-            if (q) xq = mm::load2<T>(q + r * lq + c);
-            xg = mm::load2<T>(g + r * lgs + c);
+            xk = mm::load2_coherent<T>(k + r * lk + c);
+            if (q) xq = mm::load2_coherent<T>(q + r * lq + c);
+            xg = mm::load2_coherent<T>(g + r * lgs + c);
 #pragma unroll
-            for (int e = 0; e < VP; ++e) xv[e] = mm::load2<T>(v + r * lv + c * VP + 2 * e);
+            for (int e = 0; e < VP; ++e) xv[e] = mm::load2_coherent<T>(v + r * lv + c * VP + 2 * e);
             xg = make_float2(gate_transform(xg.x, gate_norm, clamp_min), gate_transform(xg.y, gate_norm, clamp_min));
         }
         *reinterpret_cast<float2*>(sk + r * DK + c) = make_float2(xk.x * kmul, xk.y * kmul);

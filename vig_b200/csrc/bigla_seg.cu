@@ -74,7 +74,7 @@ template <typename T, int COLS, int TERMS, int TOK, int NTH> __device__ __forcei
         for (int i0 = 0; i0 < TOK * PPR; i0 += NTH) {
             const int i = i0 + threadIdx.x, r = i / PPR, v = i % PPR;
             float2 a = make_float2(0.f, 0.f), b = a;
-            if (r < n) { a = load2<T>(src + r * stride_l + 4 * v); b = load2<T>(src + r * stride_l + 4 * v + 2); }
+            if (r < n) { a = load2_coherent<T>(src + r * stride_l + 4 * v); b = load2_coherent<T>(src + r * stride_l + 4 * v + 2); }
             see(mark, a.x); see(mark, a.y); see(mark, b.x); see(mark, b.y);
             uint32_t ta[TERMS], tb[TERMS];
             split2<TERMS>(a.x, a.y, ta); split2<TERMS>(b.x, b.y, tb);
@@ -282,6 +282,7 @@ __global__ void __launch_bounds__(2 * TOK * SegWarps<DV, T, TOK>::CW, seg_min_bl
     const int n = min(s.seglen, p.L - (int)t0), nb = (n + 15) / 16;
     const int pr = threadIdx.x % PAIRS, gr = threadIdx.x / PAIRS, r0 = gr * RPG;   // my channel pair, my rows
     pdl_launch();                                                        // a chained successor may fetch its weights meanwhile
+    if (MODE == SEG_ONE) pdl_wait();                                     // chained itself: the launch before it may have written the inputs
     const bool want_out = MODE != SEG_STATES && p.o;
     const bool fwd = p.dir_mask & 1, bwd = p.dir_mask & 2;
     F2 G[2][RPG], ref[2];
@@ -308,10 +309,10 @@ __global__ void __launch_bounds__(2 * TOK * SegWarps<DV, T, TOK>::CW, seg_min_bl
 #pragma unroll
             for (int r = 0; r < RPG; ++r) {
                 const int64_t row = min(r0 + r, n - 1);
-                xr[0][r].load(fp + row * lf);
-                xr[1][r].load(bp + row * lb);
-                kr[r].load(kp + row * lk);
-                if (MODE != SEG_STATES) qr[r].load(qp + row * lq); else qr[r].zero();
+                xr[0][r].load_coherent(fp + row * lf);
+                xr[1][r].load_coherent(bp + row * lb);
+                kr[r].load_coherent(kp + row * lk);
+                if (MODE != SEG_STATES) qr[r].load_coherent(qp + row * lq); else qr[r].zero();
             }
             if (r0 + RPG > n) {
 #pragma unroll
@@ -637,11 +638,13 @@ int seg_launch_mode(const SegParams& s, cudaStream_t stream) {
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     if (MODE == SEG_OUT) return (int)launch_next(kern, cfg.gridDim, cfg.blockDim, smem, stream, s);
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = s.nseg; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2];
     cfg.attrs = attr;
-    cfg.numAttrs = MODE == SEG_ONE && s.nseg > 1 ? 1 : 0;
+    if (MODE == SEG_ONE && s.nseg > 1) {
+        cudaLaunchAttribute& c = attr[cfg.numAttrs++];
+        c.id = cudaLaunchAttributeClusterDimension;
+        c.val.clusterDim.x = s.nseg; c.val.clusterDim.y = 1; c.val.clusterDim.z = 1;
+    }
     if (MODE == SEG_ONE && s.nseg > 8) {                 // more than the portable cluster size: the device is asked once whether it can place it
         static std::atomic<uint32_t> answers[64];        // two bits a size: asked, yes
         int dev = 0;
@@ -657,6 +660,9 @@ int seg_launch_mode(const SegParams& s, cudaStream_t stream) {
         }
         if (!(have & yes)) return SEG_NO_CLUSTER;
     }
+    // Begins before the launch ahead of it ends, and reads its inputs coherently for that reason (ViG-T of one 224 x 224 image 253 -> 248 us a forward).  Not
+    // the first of three launches: the later ones read the inputs before they wait, for launches of this call only.
+    if (MODE == SEG_ONE && chain_launches) { attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1; }
     e = cudaLaunchKernelEx(&cfg, kern, s);
     return (int)(e != cudaSuccess ? e : cudaGetLastError());
 }

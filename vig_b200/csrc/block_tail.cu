@@ -36,12 +36,6 @@ struct BtParams {
     int32_t* status;
 };
 
-template <typename T> __device__ __forceinline__ void mma_t(float* c, const uint32_t* a, const uint32_t* b);
-template <> __device__ __forceinline__ void mma_t<__nv_bfloat16>(float* c, const uint32_t* a, const uint32_t* b) { mm::mma16816(c, a, b); }
-template <> __device__ __forceinline__ void mma_t<__half>(float* c, const uint32_t* a, const uint32_t* b) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
 __device__ __forceinline__ void bt_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
 constexpr int BT_CLUSTER = 4;                             // largest cluster of a tile
@@ -191,7 +185,7 @@ __global__ void __launch_bounds__(BT_THREADS, 1) block_tail_kernel(const __grid_
 #pragma unroll
                 for (int m = 0; m < MB; ++m)
 #pragma unroll
-                    for (int j = 0; j < NT; ++j) mma_t<T>(acc[m][j], fa[ks & 1][m], fb[ks & 1][j]);
+                    for (int j = 0; j < NT; ++j) mm::mma_t<T>(acc[m][j], fa[ks & 1][m], fb[ks & 1][j]);
             }
             __syncwarp();
             if (lane == 0) mbar_arrive_plain(empty + 8 * s);
@@ -283,8 +277,8 @@ __global__ void __launch_bounds__(BT_THREADS, 1) block_tail_kernel(const __grid_
                     for (int m = 0; m < MB; ++m)
 #pragma unroll
                         for (int j = 0; j < FT; ++j) {
-                            mma_t<T>(g[m][j], fa[kb * 4 + ks][m], bg[ks & 1][j]);
-                            mma_t<T>(y[m][j], fa[kb * 4 + ks][m], by[ks & 1][j]);
+                            mm::mma_t<T>(g[m][j], fa[kb * 4 + ks][m], bg[ks & 1][j]);
+                            mm::mma_t<T>(y[m][j], fa[kb * 4 + ks][m], by[ks & 1][j]);
                         }
                 }
                 __syncwarp();

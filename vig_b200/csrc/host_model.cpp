@@ -90,8 +90,15 @@ struct Attn {
     Scanned scan(const Ctx& c, const Tensor& x, int64_t h, int64_t w) const {
         if (!w_z.defined()) std::tie(taps, w_z, b_z) = pack().cast<std::tuple<Tensor, Tensor, Tensor>>();
         const int64_t B = x.size(0), L = x.size(1), kd = H * dk, vd = H * dv;
-        const Tensor xs = dwconv(c, x, taps, conv_b, h, w, act_conv);
-        const Tensor z = at::linear(xs, w_z, b_z);
+        Tensor xs, z;
+        if (api.vig_conv_proj_preferred(B * L, (int)x.size(2), (int)w_z.size(0), c.code) && on16(x) && on16(taps) && on16(w_z) && on16(b_z) && (!conv_b.defined() || on16(conv_b))) {
+            xs = at::empty_like(x);
+            z = at::empty({B, L, w_z.size(0)}, x.options());
+            ok(api.vig_conv_proj_fwd(ptr(x), ptr(taps), ptr(conv_b), ptr(w_z), ptr(b_z), ptr(xs), ptr(z), B, h, w, x.size(2), w_z.size(0), act_conv, c.code, c.stream), "vig_conv_proj_fwd");
+        } else {
+            xs = dwconv(c, x, taps, conv_b, h, w, act_conv);
+            z = at::linear(xs, w_z, b_z);
+        }
         const int64_t W = z.size(2);
         auto view = [&](int64_t col, int64_t d) { return z.as_strided({B, H, L, d}, {L * W, d, W, 1}, z.storage_offset() + col); };
         Tensor o = at::empty({B, L, H, dv}, x.options());

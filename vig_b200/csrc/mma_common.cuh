@@ -42,6 +42,14 @@ __device__ __forceinline__ void mma16816(float* c, const uint32_t* a, const uint
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
+// the same on operands of the type itself
+template <typename T> __device__ __forceinline__ void mma_t(float* c, const uint32_t* a, const uint32_t* b);
+template <> __device__ __forceinline__ void mma_t<__nv_bfloat16>(float* c, const uint32_t* a, const uint32_t* b) { mma16816(c, a, b); }
+template <> __device__ __forceinline__ void mma_t<__half>(float* c, const uint32_t* a, const uint32_t* b) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
 // Infinities and NaN among inputs.  In a masked product they would reach the tokens that the mask keeps from them (0 times inf),
 // and of an infinity's second term only NaN is left; the recurrences have neither.  ``mark`` becomes NaN once it has seen one;
 // packed bf16 pairs are asked by their exponent bits.
@@ -112,6 +120,10 @@ template <typename T> __device__ __forceinline__ float2 load2(const T* p);
 template <> __device__ __forceinline__ float2 load2<float>(const float* p) { return __ldg(reinterpret_cast<const float2*>(p)); }
 template <> __device__ __forceinline__ float2 load2<__nv_bfloat16>(const __nv_bfloat16* p) { return tc::Pack2<__nv_bfloat16>::unpack(__ldg(reinterpret_cast<const uint32_t*>(p))); }
 template <> __device__ __forceinline__ float2 load2<__half>(const __half* p) { return tc::Pack2<__half>::unpack(__ldg(reinterpret_cast<const uint32_t*>(p))); }
+// the same for kernels that may have begun before the launch that writes what they read
+__device__ __forceinline__ uint32_t ld_coherent32(const void* p) { uint32_t v; asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p)); return v; }
+template <typename T> __device__ __forceinline__ float2 load2_coherent(const T* p) { return tc::Pack2<T>::unpack(ld_coherent32(p)); }
+template <> __device__ __forceinline__ float2 load2_coherent<float>(const float* p) { const uint2 v = ld_coherent(p); return make_float2(__uint_as_float(v.x), __uint_as_float(v.y)); }
 template <typename T> __device__ __forceinline__ void store2(T* p, float a, float b);
 template <> __device__ __forceinline__ void store2<float>(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
 template <> __device__ __forceinline__ void store2<__nv_bfloat16>(__nv_bfloat16* p, float a, float b) { *reinterpret_cast<uint32_t*>(p) = tc::Pack2<__nv_bfloat16>::pack(a, b); }
@@ -198,6 +210,7 @@ __device__ __forceinline__ void wait_raw() { asm volatile("cp.async.wait_all;" :
 template <typename T> struct Raw2 {
     uint32_t w;
     __device__ __forceinline__ void load(const T* p) { w = __ldg(reinterpret_cast<const uint32_t*>(p)); }
+    __device__ __forceinline__ void load_coherent(const T* p) { w = ld_coherent32(p); }
     __device__ __forceinline__ void zero() { w = 0u; }
     __device__ __forceinline__ void open_gate(bool logits) { w = logits ? (std::is_same<T, __half>::value ? 0x7C007C00u : 0x7F807F80u) : 0u; }
     __device__ __forceinline__ F2 f2() const {
@@ -208,6 +221,7 @@ template <typename T> struct Raw2 {
 template <> struct Raw2<float> {
     float2 w;
     __device__ __forceinline__ void load(const float* p) { w = __ldg(reinterpret_cast<const float2*>(p)); }
+    __device__ __forceinline__ void load_coherent(const float* p) { w = load2_coherent<float>(p); }
     __device__ __forceinline__ void zero() { w = make_float2(0.f, 0.f); }
     __device__ __forceinline__ void open_gate(bool logits) { w.x = w.y = logits ? INFINITY : 0.f; }
     __device__ __forceinline__ F2 f2() const { return f2_make(w.x, w.y); }
