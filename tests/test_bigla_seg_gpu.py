@@ -105,7 +105,7 @@ def test_small_calls_in_segments_of_32(dtype, dk, dv, L):
     tol = 2e-3 if dtype == torch.float16 else TOL[dtype]
     assert rel_err(vig_b200.bi_gla(*dev, impl=_lib.IMPL_SEG).float(), ref) < tol
     need = [_lib.lib().vig_bigla_workspace_bytes(1, 2, L, dk, dv, _lib.dtype_code(dev[0]), i) for i in (_lib.IMPL_SEG, _lib.IMPL_SIMT)]
-    assert need[0] > need[1] or L % 64 == 0
+    assert need[0] > need[1] or (dtype == torch.float16 and L > 256)
     ws, o = torch.empty(need[1], dtype=torch.uint8, device="cuda"), torch.empty(1, 2, L, dv, device="cuda", dtype=dtype)
     st = _lib.lib().vig_bigla_fwd(*map(_lib.ptr, dev), _lib.ptr(o), 1, 2, L, dk, dv, _lib.dtype_code(o), *[None] * 6, -1.0, 1.0, 0.0, float("nan"), *[None] * 6, 3,
                                   _lib.IMPL_SEG, _lib.ptr(ws), need[1], None, _lib.stream_ptr())

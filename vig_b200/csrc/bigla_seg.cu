@@ -733,7 +733,7 @@ bool bigla_seg_preferred(const BiglaParams& p) {
 }
 
 // Segments of 32 tokens: calls of few segments, whose operands have two or three terms (bigla_seg_launch says why).
-static bool seg_fine(int dtype, int dv, int L) { return !(dtype == VIG_DTYPE_BF16 && dv == 64) && L > 64 && L <= 512; }
+static bool seg_fine(int dtype, int dv, int L) { return !(dtype == VIG_DTYPE_BF16 && dv == 64) && L > 64 && L <= (dtype == VIG_DTYPE_F16 && dv == 64 ? 256 : 512); }
 static size_t seg_fine_bytes(int64_t BH, int L, int dk, int dv) { return (size_t)BH * ((L + 31) / 32) * 2 * ((size_t)dk * dv + dk) * sizeof(float); }
 
 size_t bigla_seg_workspace(int B, int H, int L, int dk, int dv, int dtype) {
@@ -745,14 +745,17 @@ int bigla_seg_launch(const BiglaParams& p, size_t ws_bytes, cudaStream_t stream)
     SegParams s{};
     s.p = p;
     // 64-token segments where more SMs can share the work of few sequences (1x3x196 dk = 64: 11 us against 13) and for dv = 32,
-    // whose segments are too little work for eight warps (64x12x196 dk = 16: 47 us against 57); otherwise 128, half as many states.
+    // whose segments are too little work for eight warps (64x12x196 dk = 16: 46 us against 56; 64x6x784 91 / 114, 64x3x3136 154 / 215; dk = 32 161 / 155);
+    // otherwise 128, half as many states.  Clusters of more than eight want room around them: fp16 32/64 1x3x836 12.6 / 16.7, bf16 1x3x1024
+    // 10.6 / 12.5, 64/64 1x6x784 14.5 / 16.5, but 1x12x784 (156 segments) 18.7 / 16.6 and 3x3x836 (126) no difference.
     // 32 tokens where operands have two or three terms and all segments find an SM of their own, clusters placed whole (us of a launch at 32 / 64
     // tokens): fp32 2x3x196 64/64 14.4 / 19.9, 4x3x256 32/64 11.9 / 13.2, 2x3x512 16/32 9.3 / 10.2; fp16 1x3x196 32/64 9.0 / 10.4, but 3x3x480 (135
-    // segments) 12.4 / 11.5; bf16 32/32 2x12x128 7.8 / 9.0; fp16 16/32 1x24x49 6.5 / 5.9.  One-term operands gain nothing: bf16 1x3x196 32/64 8.4 / 8.5,
+    // segments) 12.4 / 11.5, 1x3x512 11.3 / 11.3, 64/64 1x6x196 13.1 / 13.7, 1x3x400 15.9 / 14.2; bf16 32/32 2x12x128 7.8 / 9.0; fp16 16/32 1x24x49 6.5 / 5.9, 1x24x98 6.8 / 7.4.
+    // One-term operands gain nothing: bf16 1x3x196 32/64 8.4 / 8.5,
     // 1x12x196 64/64 11.9 / 11.1.
     const int64_t BH = (int64_t)p.B * p.H;
     const int tok = seg_fine(p.dtype, p.dv, p.L) && 3 * BH * ((p.L + 31) / 32) <= 2 * device_sms() && ws_bytes >= seg_fine_bytes(BH, p.L, p.dk, p.dv) ? 32
-                    : p.dtype == VIG_DTYPE_F32 || p.dv == 32 || p.L <= 64 || (p.L <= 512 && BH * ((p.L + 63) / 64) <= device_sms()) ? 64 : 128;
+                    : p.dtype == VIG_DTYPE_F32 || p.dv == 32 || p.L <= 64 || (p.L <= 1024 && 3 * BH * ((p.L + 63) / 64) <= (p.L <= 512 ? 3 : 2) * device_sms()) ? 64 : 128;
     switch (p.dtype) {
         case VIG_DTYPE_F32: return seg_launch_dims<float>(s, tok, stream);
         case VIG_DTYPE_BF16: return seg_launch_dims<__nv_bfloat16>(s, tok, stream);
