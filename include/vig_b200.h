@@ -236,7 +236,11 @@ VIG_API int vig_dwconv3x3_halo_fwd(const void* x, const void* top, const void* b
  * x: [M, K] rows ldx elements apart, w: [N, K] contiguous, bias: [N] or NULL, out: [M, N] rows ldo apart; bf16 / fp16.
  * vig_linear_bias_supported: K % 64 == 0, K <= 192, N % 8 == 0 and at least 256 rows per SM of the current device
  * (smaller problems are left to a library GEMM).  status_dev: optional int32 on the device, bit 0 = a bounded wait ran out.
+ * vig_linear_pair_fwd: the same for any K that is a multiple of 64 and any M; ``preferred``: whether it beats a library GEMM.
  */
+VIG_API int vig_linear_pair_preferred(int64_t M, int K, int N, int dtype);
+VIG_API int vig_linear_pair_fwd(const void* x, int64_t ldx, const void* w, const void* bias, void* out, int64_t ldo,
+                        int64_t M, int K, int N, int dtype, int32_t* status_dev, void* stream);
 VIG_API int vig_linear_bias_supported(int64_t M, int K, int N, int dtype);
 VIG_API int vig_linear_bias_fwd(const void* x, int64_t ldx, const void* w, const void* bias, void* out, int64_t ldo,
                         int64_t M, int K, int N, int dtype, int32_t* status_dev, void* stream);

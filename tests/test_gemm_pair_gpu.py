@@ -3,6 +3,8 @@ fill the last tile of 128, one and many k boxes, W streamed (K = 448 and up, few
 import pytest
 import torch
 
+from conftest import rel_err
+
 pytestmark = pytest.mark.gpu
 # one rounding of the result (2^-9, 2^-12, uniform: over sqrt(3)) and, for SwiGLU, the sigmoid through tanh.approx (2^-11)
 TOL = {torch.bfloat16: 2.5e-3, torch.float16: 6e-4}
@@ -204,3 +206,19 @@ def test_projection_add_norm_in_place(M, K, N):
     assert _lib.lib().vig_linear_add_rmsnorm_fwd(_lib.ptr(x), K, _lib.ptr(w), _lib.ptr(res), _lib.ptr(nw), _lib.ptr(res), _lib.ptr(h), M, K, N, 1e-6, _lib.dtype_code(x),
                                                  None, _lib.stream_ptr()) == 0
     assert torch.equal(h, want_h) and torch.equal(res, want_r)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,K,N,biased", [(1, 64, 8, True), (255, 192, 264, True), (257, 384, 256, False), (19000, 192, 768, True), (19001, 384, 520, True), (2500, 768, 1544, True), (20000, 320, 2304, False)])
+def test_pair_linear(dtype, M, K, N, biased):
+    """x W^T + bias on CTA pairs: W streamed and kept, partial tiles on every side, strided rows.  One rounding of fp32 sums: 2^-9, 2^-12 of the largest."""
+    from vig_b200 import _lib
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    rand = lambda *s: torch.randn(*s, generator=gen, device="cuda").to(dtype)  # noqa: E731
+    x, w, b = rand(M, K + 8)[:, :K], rand(N, K) / K ** 0.5, rand(N) if biased else None
+    out = torch.full((M, N + 8), 7.0, device="cuda", dtype=dtype)
+    st = _lib.lib().vig_linear_pair_fwd(_lib.ptr(x), K + 8, _lib.ptr(w), _lib.ptr(b), _lib.ptr(out), N + 8, M, K, N, _lib.dtype_code(x), None, _lib.stream_ptr())
+    assert st == 0 and bool((out[:, N:] == 7).all())
+    ref = torch.nn.functional.linear(x.float(), w.float(), None if b is None else b.float())
+    assert rel_err(out[:, :N].float(), ref) < (4e-3 if dtype == torch.bfloat16 else 5e-4)
+    assert _lib.lib().vig_linear_pair_fwd(_lib.ptr(x), K + 8, _lib.ptr(w), _lib.ptr(b), _lib.ptr(out), N + 8, M, K - 8, N, _lib.dtype_code(x), None, _lib.stream_ptr()) == -2

@@ -1,5 +1,7 @@
 // y = x W^T on pairs of CTAs (tcgen05, cta_group::2), with the work that follows the product as its epilogue (bf16 / fp16):
 //   SwiGLU:  out[M, I] = silu(x Wg^T) * (x Wy^T), W = [Wg ; Wy] of shape [2I, K]   (classification/models/vig.py:494-497)
+//   linear:  out[M, N] = x W^T + bias; an epilogue warp sends its two pieces one behind the other through one box (with a box for each the ring is a
+//            stage shorter and W of K = 384 does not fit beside it: 25088 x 384 x 2304 45.6 us against 43.5)
 //
 // A tile is 256 rows x BN columns of the product and belongs to the two SMs of a cluster: each loads its 128 rows of x and
 // its half of the tile's rows of W (TMA, 128-byte swizzle), and its tensor memory holds its 128 rows of the result, two buffers of up to
@@ -20,11 +22,12 @@ using namespace tc;
 constexpr int PR_BK = 64;                                // k elements of a box (128-byte rows)
 constexpr int PR_A = 128 * PR_BK * 2;                    // one CTA's [128 rows x 64 k] box of x
 
-struct PairCfg {
+// GATED: SwiGLU of gate and y columns, half as many output columns; otherwise the columns with a bias
+template <bool GATED> struct PairCfg {
     static constexpr int BN = 256;                       // columns of the product in a tile
     static constexpr int B = BN / 2 * PR_BK * 2;         // one CTA's half of a k box of W
-    static constexpr int OCOLS = BN / 2, COLS = 32;      // output columns of a tile, of an epilogue warp
-    static constexpr int EPI_WARPS = 4 * OCOLS / COLS, THREADS = 64 + 32 * EPI_WARPS;
+    static constexpr int OCOLS = GATED ? BN / 2 : BN, COLS = 32;         // output columns of a tile, of a box
+    static constexpr int EPI_WARPS = 16, THREADS = 64 + 32 * EPI_WARPS;
     static constexpr int OUT = EPI_WARPS * OUT_BOX_BYTES;
     static constexpr int MAX_ST = 8;
     static constexpr int BARS = 8 * (2 * MAX_ST + 5);
@@ -34,10 +37,10 @@ struct PairCfg {
 struct PairMaps { CUtensorMap x, w, o; };
 
 // stat: stationary form, ``nst`` boxes of x in the ring; otherwise ``nst`` boxes of x and W
-template <typename T, bool STAT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg::THREADS, 1)
-gemm_pair_kernel(const __grid_constant__ PairMaps maps, int M, int N, int KB, int ntn, int ntm, int nst, int32_t* status) {
-    using Cfg = PairCfg;
+template <typename T, bool STAT, bool GATED>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<GATED>::THREADS, 1)
+gemm_pair_kernel(const __grid_constant__ PairMaps maps, const T* bias, int M, int N, int KB, int ntn, int ntm, int nst, int32_t* status) {
+    using Cfg = PairCfg<GATED>;
     constexpr int BN = Cfg::BN;
     constexpr int STAGE = PR_A + (STAT ? 0 : Cfg::B);
     extern __shared__ uint8_t pr_smem_raw[];
@@ -81,14 +84,14 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, int M, int N, int KB, in
         // (a lane that waits while the others are parked at a warp barrier resumes microseconds late).
         uint32_t st = 0, phase = 0;
         if (STAT && lane == 0) {
-            const int wrow = pair % ntn * (BN / 2) + (rank ? N : 0);      // the even CTA has the gate rows, the odd one their y rows
+            const int wrow = pair % ntn * Cfg::OCOLS + (rank ? GATED ? N : BN / 2 : 0);   // the even CTA has the gate rows, the odd one their y rows
             if (rank == 0) mbar_expect_tx(bar_w, 2u * KB * Cfg::B);
             for (int kb = 0; kb < KB; ++kb) tma_load_2d_pair(sbase + kb * Cfg::B, &maps.w, kb * PR_BK, wrow, map_rank(bar_w, 0));
         }
         __syncwarp();
         for (int tile = first; tile < ntiles; tile += step) {
             const int row = (tile / ntn) * 256 + 128 * (int)rank, nb = tile % ntn;
-            const int wrow = nb * (BN / 2) + (rank ? N : 0);
+            const int wrow = nb * Cfg::OCOLS + (rank ? GATED ? N : BN / 2 : 0);
             for (int kb = 0; kb < KB; ++kb) {
                 waiter.wait_lite(bar_empty + 8 * st, phase ^ 1u);            // the MMAs of a ring ago have read the stage, in both CTAs
                 if (*abort_flag) break;
@@ -161,8 +164,26 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, int M, int N, int KB, in
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(drained + 8 * buf);
             uint32_t pk[16];
-            swiglu_pack<T>(g, g + 32, pk);
-            send_box(box, pk, &maps.o, col, row, row < M && col < N, lane);
+            if constexpr (GATED) {
+                swiglu_pack<T>(g, g + 32, pk);
+                send_box(box, pk, &maps.o, col, row, row < M && col < N, lane);
+            } else {
+#pragma unroll
+                for (int hf = 0; hf < 2; ++hf) {
+                    const int c = col + hf * (BN / 2);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {        // the same addresses for all lanes; N is a multiple of 8
+                        const uint4 b = bias && c + 8 * j < N ? __ldg(reinterpret_cast<const uint4*>(bias + c + 8 * j)) : make_uint4(0u, 0u, 0u, 0u);
+                        const uint32_t b4[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float2 bv = Pack2<T>::unpack(b4[i]);
+                            pk[4 * j + i] = Pack2<T>::pack(g[32 * hf + 8 * j + 2 * i] + bv.x, g[32 * hf + 8 * j + 2 * i + 1] + bv.y);
+                        }
+                    }
+                    send_box(box, pk, &maps.o, c, row, row < M && c < N, lane);
+                }
+            }
         }
         if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the stores have read their boxes
     }
@@ -177,12 +198,12 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, int M, int N, int KB, in
     }
 }
 
-template <typename T>
-int pair_launch(const void* x, int64_t ldx, const void* w, void* out, int64_t ldo, int64_t M, int K, int N, int dtype, int32_t* status, cudaStream_t stream) {
-    using Cfg = PairCfg;
+template <typename T, bool GATED>
+int pair_launch(const void* x, int64_t ldx, const void* w, const void* bias, void* out, int64_t ldo, int64_t M, int K, int N, int dtype, int32_t* status, cudaStream_t stream) {
+    using Cfg = PairCfg<GATED>;
     constexpr int BN = Cfg::BN;
     PairMaps maps;
-    if (!make_map_2d(&maps.x, x, M, K, ldx, 128, dtype) || !make_map_2d(&maps.w, w, 2 * (int64_t)N, K, K, BN / 2, dtype) ||
+    if (!make_map_2d(&maps.x, x, M, K, ldx, 128, dtype) || !make_map_2d(&maps.w, w, (GATED ? 2 : 1) * (int64_t)N, K, K, BN / 2, dtype) ||
         !make_out_map(&maps.o, out, M, N, ldo, dtype)) return VIG_ERR_DEVICE;
     const int ntn = (N + Cfg::OCOLS - 1) / Cfg::OCOLS, KB = K / PR_BK, all = device_sms() / 2;
     const int64_t ntm = (M + 255) / 256;
@@ -194,17 +215,22 @@ int pair_launch(const void* x, int64_t ldx, const void* w, void* out, int64_t ld
     const int nst = stat ? (xst < Cfg::MAX_ST ? xst : Cfg::MAX_ST) : Cfg::RING / (PR_A + Cfg::B);
     const int smem = (stat ? KB * Cfg::B + nst * PR_A : nst * (PR_A + Cfg::B)) + Cfg::OUT + Cfg::BARS + 16 + 1024;
     const int64_t pairs = stat ? all / ntn * ntn : ntm * ntn < all ? ntm * ntn : all;
-    auto kfn = stat ? gemm_pair_kernel<T, true> : gemm_pair_kernel<T, false>;
+    auto kfn = stat ? gemm_pair_kernel<T, true, GATED> : gemm_pair_kernel<T, false, GATED>;
     const cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(kfn), 227 * 1024);
     if (e != cudaSuccess) return (int)e;
-    return (int)launch_chained(kfn, dim3(2 * (unsigned)pairs), dim3(Cfg::THREADS), smem, stream, maps, (int)M, N, KB, ntn, (int)ntm, nst, status);
+    return (int)launch_chained(kfn, dim3(2 * (unsigned)pairs), dim3(Cfg::THREADS), smem, stream, maps, (const T*)bias, (int)M, N, KB, ntn, (int)ntm, nst, status);
 }
 
 }  // namespace
 
 int pair_swiglu_launch(const void* x, int64_t ldx, const void* w, void* out, int64_t ldo, int64_t M, int K, int I, int dtype, int32_t* status, cudaStream_t stream) {
-    if (dtype == VIG_DTYPE_BF16) return pair_launch<__nv_bfloat16>(x, ldx, w, out, ldo, M, K, I, dtype, status, stream);
-    return pair_launch<__half>(x, ldx, w, out, ldo, M, K, I, dtype, status, stream);
+    if (dtype == VIG_DTYPE_BF16) return pair_launch<__nv_bfloat16, true>(x, ldx, w, nullptr, out, ldo, M, K, I, dtype, status, stream);
+    return pair_launch<__half, true>(x, ldx, w, nullptr, out, ldo, M, K, I, dtype, status, stream);
+}
+
+int pair_linear_launch(const void* x, int64_t ldx, const void* w, const void* bias, void* out, int64_t ldo, int64_t M, int K, int N, int dtype, int32_t* status, cudaStream_t stream) {
+    if (dtype == VIG_DTYPE_BF16) return pair_launch<__nv_bfloat16, false>(x, ldx, w, bias, out, ldo, M, K, N, dtype, status, stream);
+    return pair_launch<__half, false>(x, ldx, w, bias, out, ldo, M, K, N, dtype, status, stream);
 }
 
 }  // namespace vig

@@ -17,7 +17,7 @@ namespace py = pybind11;
     X(vig_dwconv3x3_fwd) X(vig_gate_inject_fwd) X(vig_add_rmsnorm_fwd) X(vig_layernorm_act_fwd) X(vig_layernorm_act_add_fwd)  \
     X(vig_layernorm_act_add_rmsnorm_fwd) X(vig_linear_swiglu_fwd) X(vig_linear_swiglu_preferred) X(vig_linear_add_rmsnorm_fwd) X(vig_linear_add_rmsnorm_preferred) \
     X(vig_stem_fold_fwd) X(vig_stem_unfold_fwd) X(vig_stem_conv_ln_fwd)                   \
-    X(vig_stem_conv_ln_supported) X(vig_swiglu_fwd) X(vig_add_layernorm_fwd) X(vig_chain_launches) X(vig_token_mean_fwd) X(vig_embed_conv_ln_fwd) X(vig_conv_proj_preferred) X(vig_conv_proj_fwd) X(vig_block_tail_preferred) X(vig_block_tail_fwd)
+    X(vig_stem_conv_ln_supported) X(vig_swiglu_fwd) X(vig_add_layernorm_fwd) X(vig_chain_launches) X(vig_token_mean_fwd) X(vig_embed_conv_ln_fwd) X(vig_linear_pair_preferred) X(vig_linear_pair_fwd) X(vig_conv_proj_preferred) X(vig_conv_proj_fwd) X(vig_block_tail_preferred) X(vig_block_tail_fwd)
 struct Api {
 #define X(name) decltype(&::name) name = nullptr;
     VIG_HOST_API(X)

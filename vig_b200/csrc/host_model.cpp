@@ -97,7 +97,13 @@ struct Attn {
             ok(api.vig_conv_proj_fwd(ptr(x), ptr(taps), ptr(conv_b), ptr(w_z), ptr(b_z), ptr(xs), ptr(z), B, h, w, x.size(2), w_z.size(0), act_conv, c.code, c.stream), "vig_conv_proj_fwd");
         } else {
             xs = dwconv(c, x, taps, conv_b, h, w, act_conv);
-            z = at::linear(xs, w_z, b_z);
+            const int64_t M = B * L, K = x.size(2), N = w_z.size(0);
+            if (on16(w_z) && on16(b_z) && api.vig_linear_pair_preferred(M, K, N, c.code)) {
+                z = at::empty({B, L, N}, x.options());
+                ok(api.vig_linear_pair_fwd(ptr(xs), K, ptr(w_z), ptr(b_z), ptr(z), N, M, K, N, c.code, c.status, c.stream), "vig_linear_pair_fwd");
+            } else {
+                z = at::linear(xs, w_z, b_z);
+            }
         }
         const int64_t W = z.size(2);
         auto view = [&](int64_t col, int64_t d) { return z.as_strided({B, H, L, d}, {L * W, d, W, 1}, z.storage_offset() + col); };

@@ -3,7 +3,7 @@ arguments as ``classification/models/vig.py`` (``GatedLinearAttention`` :241-464
 ``GLABlock`` :530-618) and ``fla/modules/rmsnorm.py:491-512`` (``RMSNorm``), so a reference state dict
 loads unchanged.  Inference only: the forward is the reference's ``eval()`` branch, with the scan, the
 depthwise conv, the gating injection, the norms and SwiGLU running as the library's CUDA kernels.  The stacked
-input projection is the GEMM library's; the gate projection with its SwiGLU, and the output and down projections
+input projection is the GEMM library's in these modules; the gate projection with its SwiGLU, and the output and down projections
 with the residual add and norm behind them, are kernels of this library where these are the faster ones (16-bit).
 """
 from typing import Optional
@@ -101,8 +101,8 @@ class GatedLinearAttention(nn.Module):
         else:
             xs = local_fn(x, taps, self.in_proj[0].bias, hw, self.use_act_in_conv)
         n_main = 2 * kd + 2 * vd
-        # the vendor GEMM by default: the library's own kernel for this product (``ops.linear_bias``) measures 171 us against
-        # 160-165 us at the benchmark's shape; ``own_in_proj_gemm`` switches it in where it is supported
+        # the vendor GEMM here; the C++ forward takes the library's own kernel where it is the faster one, ``own_in_proj_gemm`` switches it in
+        # here where ``ops.linear_bias`` supports it
         use_own = self.own_in_proj_gemm and ops.linear_bias_supported(xs, w_z)
         z = ops.linear_bias(xs, w_z, b_z) if use_own else F.linear(xs, w_z, b_z)
         heads = lambda t, d: t.unflatten(-1, (H, d)).permute(0, 2, 1, 3)           # [B,H,L,d] views, no copy
