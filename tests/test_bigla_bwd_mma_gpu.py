@@ -77,3 +77,21 @@ def test_a_chunk_that_one_direction_leaves(dk, dv, which):
     got = vig_b200.bi_gla_backward(*[t.cuda() for t in (q, k, v, gf, gb, d_out)], out_scale=0.5)
     errs = {n: rel_err(g, r) for n, g, r in zip(NAMES, got, ref)}
     assert all(e < TOL[torch.float32] for e in errs.values()), errs
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("L", [128, 256, 257, 384, 385])
+@pytest.mark.parametrize("strong", [False, True])
+def test_few_chunks_sum_their_states_themselves(dtype, L, strong):
+    """Both sides of the lines behind which a launch forms the entering states (4 and 6 chunks), with a chunk for the exact form, which needs them too."""
+    import vig_b200
+    q, k, v, gf, gb = oracle.make_bigla_inputs(1, 2, L, 32, 64, seed=L)
+    if strong:
+        gf[0, 0, 64:128] *= 200
+    q, k, v, gf, gb = (t.to(dtype) for t in (q, k, v, gf, gb))
+    d_out = torch.randn(1, 2, L, 64, generator=torch.Generator().manual_seed(5)).to(dtype)
+    _, ref = _reference_grads(q.float(), k.float(), v.float(), gf.float(), gb.float(), d_out.float(), 0.5, 3)
+    leaves = [t.cuda().requires_grad_() for t in (q, k, v, gf, gb)]
+    got = torch.autograd.grad(vig_b200.bi_gla(*leaves, out_scale=0.5), leaves, d_out.cuda())
+    errs = {n: rel_err(g.float(), r) for n, g, r in zip(NAMES, got, ref)}
+    assert all(e < TOL[dtype] for e in errs.values()), errs

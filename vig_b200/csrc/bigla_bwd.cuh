@@ -18,9 +18,15 @@ struct BwdParams {
     float *ws_S, *ws_Z, *ws_decay;   // [BH][nchunk][2][dk*dv] x2, [BH][nchunk][2][dk] (summed log-gates, log2 units)
     int32_t* flags;                  // [BH][nchunk]: not 0 = the chunk's gates left the factorisation range, take the exact form
     int nchunk;
+    int scanned;                     // 1: ws_S, ws_Z hold the states entering each chunk; 0: what each chunk contributes, summed by who needs them
 };
 
 constexpr int BWD_CHUNK = 64;
+// Chunks of a sequence up to which the contributions are summed where they are used instead of by a launch over chunks.  With n chunks that reads
+// n - 1 states more a chunk and direction; the launch reads and writes two each.  Forward + backward in us, summed / launched: 2 chunks 128x3x128 32/64
+// bf16 92 / 105; 4 chunks 128x3x196 32/64 179 / 189, 128x6x196 64/64 529 / 590, fp32 128x3x196 243 / 243, 2x3x196 84 / 88; 6 chunks 64x3x384 64/64 227 / 236; 8 chunks
+// 64x3x512 64/64 304 / 308, 64x6x512 32/64 371 / 374; fp32 64x3x320 (5) 323 / 322, 64x3x512 449 / 444.
+inline int bwd_fold(int dtype) { return dtype == VIG_DTYPE_F32 ? 4 : 6; }
 
 inline size_t bwd_state_floats(int B, int H, int nchunk, int dk, int dv) { return (size_t)B * H * nchunk * 2 * dk * dv; }
 

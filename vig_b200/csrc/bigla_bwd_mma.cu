@@ -10,7 +10,7 @@
 //   dg_t = <S_next, Z> over value columns + sum of e over the chunk's tokens scanned at or after t
 // The first term of dg is the gate gradient just past the chunk: d loss / d g_T = <a_T S_{T-1}, D_T> = <S_{T-1}, Z_T>, so no
 // sum ever runs over the whole sequence.  Three launches: chunk states (U = (k 2^(l-G))^T V and its adjoint), a scan over
-// chunks, chunk gradients.  A chunk whose |G - r| exceeds the range set below raises its flag and is left to the exact
+// chunks (a few chunks: none, the gradients sum what they need), chunk gradients.  A chunk whose |G - r| exceeds the range set below raises its flag and is left to the exact
 // token-by-token kernel, which runs afterwards and returns at once for every other chunk.
 #include "bigla_bwd.cuh"
 #include "bigla_exact.cuh"
@@ -230,6 +230,28 @@ __device__ __forceinline__ void send(uint32_t at, float a, float b, float c, flo
                  ::"r"(at), "f"(a), "f"(b), "f"(c), "f"(d), "r"(bar) : "memory");
 }
 
+// The contributions of the first m chunks, from the sequence's start or (down) from its end, into the state behind them: what bwd_scan_kernel
+// leaves in the chunk that follows, the same operations in the same order.
+template <int DK, int DV> __device__ __forceinline__ void sum_states(float4 (&S)[StateLay<DK, DV>::KN], const BwdParams& p, const float* U, int bh, int dir, int down, int m) {
+    using ST = StateLay<DK, DV>;
+#pragma unroll
+    for (float4& s : S) s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+    for (int g = 0; g < m; ++g) {
+        const size_t slot = ((size_t)bh * p.nchunk + (down ? p.nchunk - 1 - g : g)) * 2 + dir;
+        float4 u[ST::KN];
+        float a[ST::KN];
+        fetch_state<DK, DV>(u, U + slot * DK * DV);
+#pragma unroll
+        for (int k = 0; k < ST::KN; ++k) a[k] = __ldcg(p.ws_decay + slot * DK + (threadIdx.x + k * NT) / ST::TPR);
+#pragma unroll
+        for (int k = 0; k < ST::KN; ++k) {
+            const float e = exp2f(a[k]);
+            S[k].x = fmaf(S[k].x, e, u[k].x); S[k].y = fmaf(S[k].y, e, u[k].y); S[k].z = fmaf(S[k].z, e, u[k].z); S[k].w = fmaf(S[k].w, e, u[k].w);
+        }
+    }
+}
+
 // CTAs an SM as shared memory has room for, where that leaves the registers that the products need (bf16 at 32 / 64: three are
 // 2 % faster than two, at 80 registers instead of 128)
 template <int DK, int DV, typename T> constexpr int grads_min_blocks() {
@@ -245,7 +267,8 @@ template <int DK, int DV, typename T> constexpr int grads_min_blocks() {
 // Eight warps: warps 0 - 3 form dQ and dV inside the chunk, warps 4 - 7 dK and the state's part of dV, 16 rows each: 160 - 288
 // products a warp and direction; dV on the other side makes it 136 - 352.  What follows the products -- the factors 2^(G-r), e
 // and its sums -- is done by channel pairs, in which q, k and the gates are read coalesced.
-template <int DK, int DV, typename T>
+// SUM: the contributions are summed here (a form of its own: the other one is 1.5 % slower with this code among its instructions)
+template <int DK, int DV, typename T, bool SUM>
 __global__ void __launch_bounds__(NT, grads_min_blocks<DK, DV, T>()) bwd_grads_mma_kernel(const __grid_constant__ BwdParams p) {
     using CL = ColLay<DK>;
     using SM = GradSmem<DK, DV, T>;
@@ -321,7 +344,21 @@ __global__ void __launch_bounds__(NT, grads_min_blocks<DK, DV, T>()) bwd_grads_m
         pdl_wait();                                                      // all of the above read the call's inputs only
         const int next = dir ? c - 1 : c + 1;                           // the chunk scanned after this one
         float4 st[ST::KN], adj[ST::KN], ahead[ST::KN];
-        if (have_states && ST::mine()) {                                 // asked for ahead of the barrier that the tiles need
+        if (SUM && ST::mine()) {
+            sum_states<DK, DV>(st, p, p.ws_S, bh, dir, dir, dir ? p.nchunk - 1 - c : c);
+            sum_states<DK, DV>(adj, p, p.ws_Z, bh, dir, dir ^ 1, dir ? c : p.nchunk - 1 - c);
+            fetch_state<DK, DV>(ahead, p.ws_S + slot * DK * DV);
+#pragma unroll
+            for (int k = 0; k < ST::KN; ++k) {
+                const float a = exp2f(__ldcg(p.ws_decay + slot * DK + (threadIdx.x + k * NT) / ST::TPR));
+                ahead[k].x = fmaf(st[k].x, a, ahead[k].x); ahead[k].y = fmaf(st[k].y, a, ahead[k].y);
+                ahead[k].z = fmaf(st[k].z, a, ahead[k].z); ahead[k].w = fmaf(st[k].w, a, ahead[k].w);
+            }
+            if (next < 0 || next >= p.nchunk) {
+#pragma unroll
+                for (float4& v : ahead) v = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        } else if (!SUM && have_states && ST::mine()) {                  // asked for ahead of the barrier that the tiles need
             fetch_state<DK, DV>(st, p.ws_S + slot * DK * DV);
             fetch_state<DK, DV>(adj, p.ws_Z + slot * DK * DV);
             if (next >= 0 && next < p.nchunk) {
@@ -517,14 +554,14 @@ int launch_typed(const BwdParams& p, cudaStream_t stream) {
     const int BH = p.B * p.H;
     constexpr uint32_t smA = StatesSmem<DK, DV, T>::BYTES, smC = GradSmem<DK, DV, T>::BYTES;
     auto kA = bwd_states_mma_kernel<DK, DV, T>;
-    auto kC = bwd_grads_mma_kernel<DK, DV, T>;
+    auto kC = p.nchunk > 1 && !p.scanned ? bwd_grads_mma_kernel<DK, DV, T, true> : bwd_grads_mma_kernel<DK, DV, T, false>;
     cudaError_t e;
     if (p.nchunk > 1) {                                                  // one chunk: both entering states are zero
         if ((e = tc::ensure_smem_attr(reinterpret_cast<const void*>(kA), (int)smA)) != cudaSuccess) return (int)e;
         // few chunks: one CTA per direction, so that more of the GPU works; many: one CTA reads v and d_out once for both
         const int gz = p.dir_mask == 3 && (int64_t)p.nchunk * BH < device_sms() * 4 ? 2 : 1;
         kA<<<dim3(p.nchunk, BH, gz), NT, smA, stream>>>(p);
-        if (int s = bigla_bwd_scan_launch(p, stream)) return s;
+        if (p.scanned) if (int s = bigla_bwd_scan_launch(p, stream)) return s;
     }
     if ((e = tc::ensure_smem_attr(reinterpret_cast<const void*>(kC), (int)smC)) != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg{};

@@ -114,6 +114,20 @@ __global__ void __launch_bounds__(NT) bwd_chunk_states(BwdParams p) {
     }
 }
 
+// Value e of key channel d of the state (adj: of the adjoint state) entering chunk c
+__device__ __forceinline__ float entering(const BwdParams& p, bool adj, int bh, int c, int dir, int per, int d, int e) {
+    const float* U = adj ? p.ws_Z : p.ws_S;
+    if (p.scanned) return U[(((size_t)bh * p.nchunk + c) * 2 + dir) * per + e];
+    const bool down = (dir != 0) != adj;
+    float S = 0.f;
+#pragma unroll 1
+    for (int g = 0; g < (down ? p.nchunk - 1 - c : c); ++g) {
+        const size_t slot = ((size_t)bh * p.nchunk + (down ? p.nchunk - 1 - g : g)) * 2 + dir;
+        S = fmaf(S, exp2f(p.ws_decay[slot * p.dk + d]), U[slot * per + e]);
+    }
+    return S;
+}
+
 // ---- phase C: gradients of one chunk -----------------------------------------------------------------------------
 template <int DK, int DV, typename T>
 __global__ void __launch_bounds__(NT) bwd_chunk_grads(BwdParams p, int flagged_only) {
@@ -162,9 +176,8 @@ __global__ void __launch_bounds__(NT) bwd_chunk_grads(BwdParams p, int flagged_o
         {   // layout B: dq from the rebuilt state (scan order), then dk from Z (reverse scan order)
             const int d = threadIdx.x / Bl::TPB, s = threadIdx.x % Bl::TPB;
             float st[Bl::JPT];
-            const float* Sin = p.ws_S + slot * DK * DV + d * DV + s * Bl::JPT;
 #pragma unroll
-            for (int jj = 0; jj < Bl::JPT; ++jj) st[jj] = have_states ? Sin[jj] : 0.f;
+            for (int jj = 0; jj < Bl::JPT; ++jj) st[jj] = have_states ? entering(p, false, bh, c, dir, DK * DV, d, d * DV + s * Bl::JPT + jj) : 0.f;
             for (int ii = 0; ii < n; ++ii) {
                 const int i = dir ? n - 1 - ii : ii;
                 const float a = sg[i * DK + d], kd = sk[i * DK + d];
@@ -183,9 +196,8 @@ __global__ void __launch_bounds__(NT) bwd_chunk_grads(BwdParams p, int flagged_o
                     se[i * DK + d] = dqd * sq[i * DK + d];
                 }
             }
-            const float* Zin = p.ws_Z + slot * DK * DV + d * DV + s * Bl::JPT;
 #pragma unroll
-            for (int jj = 0; jj < Bl::JPT; ++jj) st[jj] = have_states ? Zin[jj] : 0.f;
+            for (int jj = 0; jj < Bl::JPT; ++jj) st[jj] = have_states ? entering(p, true, bh, c, dir, DK * DV, d, d * DV + s * Bl::JPT + jj) : 0.f;
             for (int ii = n - 1; ii >= 0; --ii) {
                 const int i = dir ? n - 1 - ii : ii;
                 const float a = sg[i * DK + d], cq = p.c * sq[i * DK + d];
@@ -208,9 +220,8 @@ __global__ void __launch_bounds__(NT) bwd_chunk_grads(BwdParams p, int flagged_o
         {   // layout A: dv from Z (reverse scan order)
             const int j = threadIdx.x / A::TPC, s = threadIdx.x % A::TPC;
             float st[A::DPT];
-            const float* Zin = p.ws_Z + slot * DK * DV;
 #pragma unroll
-            for (int dd = 0; dd < A::DPT; ++dd) st[dd] = have_states ? Zin[(s * A::DPT + dd) * DV + j] : 0.f;
+            for (int dd = 0; dd < A::DPT; ++dd) st[dd] = have_states ? entering(p, true, bh, c, dir, DK * DV, s * A::DPT + dd, (s * A::DPT + dd) * DV + j) : 0.f;
             for (int ii = n - 1; ii >= 0; --ii) {
                 const int i = dir ? n - 1 - ii : ii;
                 const float dj = p.c * sdo[i * DV + j];
@@ -240,9 +251,8 @@ __global__ void __launch_bounds__(NT) bwd_chunk_grads(BwdParams p, int flagged_o
                 const int d = threadIdx.x;
                 float run = 0.f;
                 if (have_states && next >= 0 && next < p.nchunk) {
-                    const float* Zin = p.ws_Z + slot * DK * DV + d * DV;
-                    const float* Sn = p.ws_S + (((size_t)bh * p.nchunk + next) * 2 + dir) * DK * DV + d * DV;
-                    for (int j = 0; j < DV; ++j) run = fmaf(Sn[j], Zin[j], run);
+                    for (int j = 0; j < DV; ++j)
+                        run = fmaf(entering(p, false, bh, next, dir, DK * DV, d, d * DV + j), entering(p, true, bh, c, dir, DK * DV, d, d * DV + j), run);
                 }
                 for (int ii = n - 1; ii >= 0; --ii) {
                     const int i = dir ? n - 1 - ii : ii;
@@ -343,6 +353,7 @@ static int bwd_fill(BwdParams& p, const void* q, const void* k, const void* v, c
     p.gate_norm = 0.f; p.clamp_min = nanf("");
     p.dir_mask = dir_mask;
     p.nchunk = (L + BWD_CHUNK - 1) / BWD_CHUNK;
+    p.scanned = 1;
     const size_t states = bwd_state_floats(B, H, p.nchunk, dk, dv);
     p.ws_S = reinterpret_cast<float*>(workspace);
     p.ws_Z = p.ws_S + states;
@@ -409,6 +420,7 @@ extern "C" int vig_bigla_bwd_full(const void* q, const void* k, const void* v, c
     // fp32 gate gradients of 16-bit inputs: token by token, whose sums are fp32 (1e-6 of them; the tensor-core form's operands
     // carry 16 bits there, 1e-5)
     if (!bigla_bwd_mma_supported(p) || (p.dg_f32 && dtype != VIG_DTYPE_F32)) return bwd_simt(p, 0, (cudaStream_t)stream);
+    p.scanned = p.nchunk > bwd_fold(dtype);
     const int st = bigla_bwd_mma_launch(p, (cudaStream_t)stream);
     return st ? st : bwd_simt(p, 1, (cudaStream_t)stream);             // the chunks whose gates left the factorisation range
 }
