@@ -134,7 +134,7 @@ template <typename T, int C> int cp_launch(const CpParams& p, cudaStream_t st) {
 using namespace vig;
 
 extern "C" int vig_conv_proj_supported(int64_t M, int C, int N, int dtype) {
-    return (dtype == VIG_DTYPE_BF16 || dtype == VIG_DTYPE_F16) && M > 0 && M < (1 << 24) && (C == 96 || C == 192) && N > 0 && N % C == 0 && N / C < 65536;
+    return (dtype == VIG_DTYPE_BF16 || dtype == VIG_DTYPE_F16) && M > 0 && M < (1 << 22) && (C == 96 || C == 192) && N > 0 && N % C == 0 && N / C < 65536;
 }
 
 // As long as every CTA has an SM of its own.  Whole forwards in us, one launch / two: ViG-T (768 columns) 64 tokens 215 / 237, 196 tokens 249 / 277, 392
