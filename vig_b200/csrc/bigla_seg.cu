@@ -1,4 +1,4 @@
-// Bi-directional gated linear attention, segments of up to 64 or 128 tokens on mma.sync tensor cores, both directions of a
+// Bi-directional gated linear attention, segments of up to 32, 64 or 128 tokens on mma.sync tensor cores, both directions of a
 // segment in one sweep: the forward of short and medium sequences, of head sizes the tcgen05 kernels do not take (dv = 32),
 // and of fp32 calls.
 //
