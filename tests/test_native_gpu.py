@@ -360,3 +360,27 @@ def test_changes_give_what_a_fresh_model_gives(kind):
         x = x.to(next(m.parameters()).dtype)
         outs.append(check())
     assert all(not torch.equal(a.float(), b.float()) for a, b in zip(outs, outs[1:]))
+
+
+@pytest.mark.parametrize("kind,size", [("vig_t", 64), ("vig_t", 512), ("hier", 64)])
+def test_weights_made_on_the_way_are_complete_before_they_are_read(kind, size):
+    """A plan's first forward makes the stacked weights between its launches: neither the launch behind them nor the last of the launches that make them
+    overlaps, and the result is that of the second forward, also in memory that held something else."""
+    from vig_b200 import _lib
+    m, seen = _model(kind, torch.bfloat16), []
+    attns = [a for a in m.modules() if hasattr(a, "_pack")]
+    for a in attns:
+        def pack(fold, own=a._pack):
+            seen.append(_lib.lib().vig_chain_launches(0))
+            _lib.lib().vig_chain_launches(seen[-1])
+            return own(fold)
+        a._pack = pack
+    x = torch.randn(1, 3, size, size, device="cuda").bfloat16()
+    with torch.no_grad():
+        before = [torch.full((1 << n,), float("nan"), device="cuda", dtype=torch.bfloat16) for n in range(8, 20) for _ in range(8)]
+        del before
+        first = m(x)
+        assert len(seen) == len(attns) and not any(seen)
+        for _ in range(3):
+            assert torch.equal(m(x), first)
+    assert len(seen) == len(attns)

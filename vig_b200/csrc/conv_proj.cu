@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(2 * C) conv_proj_kernel(const __grid_constant_
 #pragma unroll
     for (int j = 0; j < NS; ++j) {
         const int col = n0 + (warp * NS + j) * 8 + 2 * (lane & 3);
-        const float2 bv = p.bias ? Pack2<T>::unpack(__ldg(reinterpret_cast<const uint32_t*>(reinterpret_cast<const T*>(p.bias) + col))) : make_float2(0.f, 0.f);
+        const float2 bv = p.bias ? mm::load2_coherent(reinterpret_cast<const T*>(p.bias) + col) : make_float2(0.f, 0.f);
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
             const int row = row0 + (lane >> 2) + 8 * hf;

@@ -25,8 +25,9 @@ using OptT = std::optional<Tensor>;
 
 // ---- library calls on tensors --------------------------------------------------------------------------------------
 struct Ctx { void* stream; int32_t* status; int code; };
-struct Chained {                                             // launches of this scope may overlap the end of the kernel before them
-    const int was = api.vig_chain_launches(1);
+struct Chained {                                             // launches of this scope may overlap the end of the kernel before them, or may not
+    const int was;
+    explicit Chained(bool on) : was(api.vig_chain_launches(on)) {}
     ~Chained() { api.vig_chain_launches(was); }
 };
 
@@ -88,15 +89,19 @@ struct Attn {
 
     struct Scanned { Tensor o, xs, z; };                     // scan output [B,L,H,dv], conv output, stacked projection
     Scanned scan(const Ctx& c, const Tensor& x, int64_t h, int64_t w) const {
-        if (!w_z.defined()) std::tie(taps, w_z, b_z) = pack().cast<std::tuple<Tensor, Tensor, Tensor>>();
+        // the first launch behind the kernels that make the weights reads them, and waits for their end like any other
+        std::optional<Chained> apart;
+        if (!w_z.defined()) { apart.emplace(false); std::tie(taps, w_z, b_z) = pack().cast<std::tuple<Tensor, Tensor, Tensor>>(); }
         const int64_t B = x.size(0), L = x.size(1), kd = H * dk, vd = H * dv;
         Tensor xs, z;
         if (api.vig_conv_proj_preferred(B * L, (int)x.size(2), (int)w_z.size(0), c.code) && on16(x) && on16(taps) && on16(w_z) && on16(b_z) && (!conv_b.defined() || on16(conv_b))) {
             xs = at::empty_like(x);
             z = at::empty({B, L, w_z.size(0)}, x.options());
             ok(api.vig_conv_proj_fwd(ptr(x), ptr(taps), ptr(conv_b), ptr(w_z), ptr(b_z), ptr(xs), ptr(z), B, h, w, x.size(2), w_z.size(0), act_conv, c.code, c.stream), "vig_conv_proj_fwd");
+            apart.reset();
         } else {
             xs = dwconv(c, x, taps, conv_b, h, w, act_conv);
+            apart.reset();
             const int64_t M = B * L, K = x.size(2), N = w_z.size(0);
             if (on16(w_z) && on16(b_z) && api.vig_linear_pair_preferred(M, K, N, c.code)) {
                 z = at::empty({B, L, N}, x.options());
@@ -347,7 +352,7 @@ struct PlanBase {
         if (const int v = peek.poll(capturing)) { on_status(v); }
         const Tensor kept = held();
         const Ctx c{st.stream(), status_ptr(device.index()), type == at::kBFloat16 ? VIG_DTYPE_BF16 : VIG_DTYPE_F16};
-        const Chained chained;
+        const Chained chained(true);
         const bool replays = graphs && !capturing && work <= GRAPH_WORK;
         const Shape shape{x.size(0), x.size(2), x.size(3), st.stream()};
         Captured* e = replays ? find(shape) : nullptr;
