@@ -28,3 +28,40 @@ def test_one_launch_equals_convolution_and_projection(dtype, C, N, B, h, w, act,
     assert torch.equal(xs, ref)
     assert rel_err(z.float(), torch.nn.functional.linear(ref.float(), W.float(), None if b is None else b.float())) < TOL[dtype]
     assert _lib.lib().vig_conv_proj_supported(B * h * w, 384, N, _lib.dtype_code(x)) == 0 and _lib.lib().vig_conv_proj_preferred(1 << 20, C, N, _lib.dtype_code(x)) == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("side", [4, 8, 14])
+def test_overlapping_launches_give_the_same_bits(dtype, side):
+    """Convolution + projection, scan and block tail over and over through the same buffers, each launch let in before the one ahead has ended, and one
+    by one: whatever is read too early holds the values of a layer before.  16 and 64 tokens in one segment, 196 in segments of 64 (bf16) or 32 (fp16)."""
+    from vig_b200 import _lib, ops
+    lib, P, C, H, dk, dv, I, L = _lib.lib(), _lib.ptr, 192, 3, 32, 64, 512, side * side
+    kd, vd = H * dk, H * dv
+    N = 4 * kd + 2 * vd
+    assert lib.vig_conv_proj_preferred(L, C, N, _lib.dtype_code(torch.empty(0, dtype=dtype)))
+    gen = torch.Generator(device="cuda").manual_seed(side)
+    rand = lambda *s: torch.randn(*s, generator=gen, device="cuda").to(dtype)  # noqa: E731
+    layers = [dict(taps=rand(9, C) / 3, cb=rand(C) * 0.1, w=rand(N, C) / C ** 0.5, b=rand(N) * 0.1, wo=rand(C, C) / C ** 0.5, wg=rand(2 * I, C) / C ** 0.5, wd=rand(C, I) / I ** 0.5)
+              for _ in range(4)]
+    one, head = torch.ones(C, device="cuda", dtype=dtype), torch.ones(dv, device="cuda", dtype=dtype)
+    x, xs, z, o = rand(1, L, C), torch.empty(1, L, C, device="cuda", dtype=dtype), torch.empty(1, L, N, device="cuda", dtype=dtype), torch.empty(1, L, H, dv, device="cuda", dtype=dtype)
+    part = lambda col, d: z.as_strided((1, H, L, d), (L * N, d, N, 1), col)  # noqa: E731
+
+    def forward(on):
+        h, r, outs = x[0], x[0], []
+        was = lib.vig_chain_launches(on)
+        for i in range(24):
+            p = layers[i % 4]
+            assert lib.vig_conv_proj_fwd(*map(P, (h, p["taps"], p["cb"], p["w"], p["b"], xs, z)), 1, side, side, C, N, 1, _lib.dtype_code(x), _lib.stream_ptr()) == 0
+            ops.bi_gla(part(0, dk), part(kd, dk), part(2 * kd, dv), part(2 * kd + 2 * vd, dk), part(3 * kd + 2 * vd, dk), gate_logit_normalizer=16.0, out_scale=0.5,
+                       out=o.permute(0, 2, 1, 3))
+            h, r = ops.block_tail(o.view(L, C), xs[0], z[0, :, 2 * kd + vd:2 * kd + 2 * vd], head, head, p["wo"], r, one, p["wg"], p["wd"], one)
+            outs.append(h)
+        lib.vig_chain_launches(was)
+        torch.cuda.synchronize()
+        return outs
+    apart = forward(0)
+    assert bool(apart[-1].isfinite().all())
+    for _ in range(20):
+        assert all(torch.equal(a, b) for a, b in zip(forward(1), apart))
