@@ -502,6 +502,7 @@ __global__ void __launch_bounds__(NT, grads_min_blocks<DK, DV, T>()) bwd_grads_m
             const float4 a = *reinterpret_cast<const float4*>(D0 + row * SM::VP + vc + i), z = *reinterpret_cast<const float4*>(D1 + row * SM::VP + vc + i);
             send(peer + SM::K + (vr * DV + vc + i) * 4, a.x + z.x, a.y + z.y, a.z + z.z, a.w + z.w, bar);
         }
+        cluster_arrive();                                                // my share is on its way
     }
     if (!bad) {
         T* out = reinterpret_cast<T*>(dir ? p.dgb : p.dgf) + ((int64_t)bh * p.L + t0 + r0) * DK + 2 * pr;
@@ -509,7 +510,10 @@ __global__ void __launch_bounds__(NT, grads_min_blocks<DK, DV, T>()) bwd_grads_m
         for (int r = 0; r < RPG; ++r)
             if (r0 + r < n) store2<T>(out + r * DK, f2_lo(e[r]), f2_hi(e[r]));
     }
-    if (both) {                                                          // bounded: about a second, then the chunk is left to the exact form like one out of range
+    if (both) {
+        // No way out ahead of the other direction's sends, which write into this CTA's shared memory.  What is left to wait for are stores under way:
+        // should they take a second, the chunk is left to the exact form like one out of range.
+        cluster_wait();
         int tries = 0;
         while (!tc::mbar_try_wait_parked(sb + SM::BAR, 0, 2000u) && tries < 1 << 19) ++tries;
         bad = __syncthreads_or(bad || tries >= 1 << 19);
