@@ -110,3 +110,35 @@ def test_small_calls_in_segments_of_32(dtype, dk, dv, L):
     st = _lib.lib().vig_bigla_fwd(*map(_lib.ptr, dev), _lib.ptr(o), 1, 2, L, dk, dv, _lib.dtype_code(o), *[None] * 6, -1.0, 1.0, 0.0, float("nan"), *[None] * 6, 3,
                                   _lib.IMPL_SEG, _lib.ptr(ws), need[1], None, _lib.stream_ptr())
     assert st == 0 and rel_err(o.float(), ref) < tol
+
+
+def _threads(f, tmp_path):
+    """Threads a CTA of the segment kernels that ``f`` launches"""
+    import json
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        f()
+        torch.cuda.synchronize()
+    prof.export_chrome_trace(str(tmp_path / "trace.json"))
+    events = json.load(open(tmp_path / "trace.json"))["traceEvents"]
+    return [e["args"]["block"][0] for e in events if e.get("cat") == "kernel" and "bigla_seg_kernel" in e["name"]]
+
+
+@pytest.mark.parametrize("dtype,dk", [(torch.bfloat16, 32), (torch.bfloat16, 64), (torch.float16, 32)])
+@pytest.mark.parametrize("L", [1, 17, 49, 64])
+@pytest.mark.parametrize("more", [0, 1])
+def test_sequences_of_one_segment_around_one_an_sm(dtype, dk, L, more, tmp_path):
+    """Up to one sequence an SM two warps share 16 rows; beyond that the scores are not formed twice.  Both with a sequence whose gates leave the
+    factorisation's range, and with final states."""
+    import vig_b200
+    B, H = torch.cuda.get_device_properties(0).multi_processor_count + more, 1
+    q, k, v, gf, gb = oracle.make_bigla_inputs(B, H, L, dk, 64, seed=L)
+    gb[B // 2] *= 200
+    ins = [t.to(dtype) for t in (q, k, v, gf, gb)]
+    ref = oracle.naive_bi_gla(*[t.float() for t in ins])
+    dev = [t.cuda() for t in ins]
+    tol = 1.5e-2 if dtype == torch.bfloat16 else 2e-3
+    assert rel_err(vig_b200.bi_gla(*dev).float(), ref) < tol
+    assert _threads(lambda: vig_b200.bi_gla(*dev), tmp_path) == [128 if more else 256]
+    o, h = vig_b200.fused_chunk_gla(*dev[:3], dev[4], output_final_state=True)
+    want, state = oracle.naive_gla(*[t.float() for t in (*ins[:3], ins[4])])
+    assert rel_err(o.float(), want) < tol and rel_err(h, state) < (1e-2 if dtype == torch.bfloat16 else 1e-4)

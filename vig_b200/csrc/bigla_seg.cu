@@ -33,20 +33,20 @@ template <int DK, int DV, typename T> struct SegTerms {
     static constexpr int RAW = Terms<T>::RAW, SC = (sizeof(T) == 2 && RAW == 1 && DV == 64) ? 1 : Terms<T>::SC;
 };
 
-// Warps that share 16 rows, each with its part of the value columns (the scores are formed by each of them): two for fp32, whose
+// Warps that share 16 rows (CW below), each with its part of the value columns (the scores are formed by each of them): two for fp32, whose
 // three-term tiles leave room for one or two 64-token segments an SM (2x3x196 64/64: 28.4 -> 19.5 us; 16x6x1000 64/64: 520 ->
-// 320), and for 16-bit segments of 64 tokens, which are for calls that leave SMs idle (1x3x196 32/64, bf16: 10.3 -> 8.8 us one call behind
-// another); twice as many for segments of 32 tokens.  Other 16-bit calls have two or three segments an SM and gain nothing from repeating
-// the scores.
-template <int DV, typename T, int TOK> struct SegWarps {
-    static constexpr int CW = (sizeof(T) == 4 ? 2 : TOK == 32 || (TOK == 64 && DV == 64) ? 2 : 1) * (sizeof(T) == 4 && TOK == 32 ? 2 : 1);
-};
+// 320), and for 16-bit segments of 64 tokens and dv = 64 while each has an SM of its own (1x3x196 32/64, bf16: 10.3 -> 8.8 us one call behind
+// another); twice as many for segments of 32 tokens.  Where two or more 16-bit segments share an SM, its issue slots go to the scores formed twice: one
+// warp (seg_launch_tok has the figures).
+template <int DV, typename T, int TOK> constexpr int seg_warps() {
+    return (sizeof(T) == 4 ? 2 : TOK == 32 || (TOK == 64 && DV == 64) ? 2 : 1) * (sizeof(T) == 4 && TOK == 32 ? 2 : 1);
+}
 
-template <int DK, int DV, typename T, int TOK> struct SegSmem {
+template <int DK, int DV, typename T, int TOK, int CW> struct SegSmem {
     using TT = SegTerms<DK, DV, T>;
     static constexpr uint32_t QT = TT::SC * (TOK * Pitch<DK>::B > DK * Pitch<DV>::B ? TOK * Pitch<DK>::B : DK * Pitch<DV>::B);   // one direction's Q or K terms, or its entering state
     static constexpr uint32_t V = 0, K = TT::RAW * TOK * Pitch<DV>::B, Q = K + 2 * QT, SUM = Q + 2 * QT,
-                              SCL = SUM + 2 * (TOK / 16) * SegWarps<DV, T, TOK>::CW * DK * 4,      // per direction and warp: summed log-gates of the warp's rows
+                              SCL = SUM + 2 * (TOK / 16) * CW * DK * 4,      // per direction and warp: summed log-gates of the warp's rows
                               BYTES = SCL + 4 * DK * 4;                 // [dir][0: 2^r, 1: 2^(l-r)]
 };
 
@@ -128,9 +128,9 @@ template <int DK, int DV, int MODE> __device__ __forceinline__ float4 entering(c
 // A segment whose gates leave the factorisation's range, or are growing ones, token by token: what it contributes, and its
 // outputs.  Every thread works on it: at 96 sequences of 1000 tokens, fp32 64 / 64, all segments out of range, 14.6 ms with DV
 // threads to a segment, 0.83 with all (1.19 in the gate-independent form of bigla_simt.cu).  The segment's tiles give up their shared memory.
-template <int DK, int DV, typename T, int TOK> struct SegExact {
-    using SM = SegSmem<DK, DV, T, TOK>;
-    using L = rec::Lay<DK, DV, 2 * TOK * SegWarps<DV, T, TOK>::CW>;
+template <int DK, int DV, typename T, int TOK, int CW> struct SegExact {
+    using SM = SegSmem<DK, DV, T, TOK, CW>;
+    using L = rec::Lay<DK, DV, 2 * TOK * CW>;
     static constexpr uint32_t ROW = 3 * DK + DV;                         // floats staged for a token
     static constexpr uint32_t bytes(int sub) { return (L::HALVES * sub * ROW + TOK * DV) * 4; }
     static constexpr int SUB = bytes(32) <= SM::SUM ? 32 : bytes(16) <= SM::SUM ? 16 : 8;      // tokens staged at a time
@@ -140,8 +140,8 @@ template <int DK, int DV, typename T, int TOK> struct SegExact {
     static __device__ int blocks(int n) { return 2 * ((n + 2 * SUB - 1) / (2 * SUB)); }
 };
 
-template <int DK, int DV, typename T, int TOK> __device__ __noinline__ void exact_contribution(const SegParams& s, float* sm, int bh, int c, int n) {
-    using E = SegExact<DK, DV, T, TOK>;
+template <int DK, int DV, typename T, int TOK, int CW> __device__ __noinline__ void exact_contribution(const SegParams& s, float* sm, int bh, int c, int n) {
+    using E = SegExact<DK, DV, T, TOK, CW>;
     using L = typename E::L;
     const BiglaParams& p = s.p;
     const int b = bh / p.H, h = bh % p.H, d0 = L::d0(), j0 = L::j0(), tid = threadIdx.x % L::HT;
@@ -211,8 +211,8 @@ template <int DK, int DV, int MODE, typename L> __device__ __forceinline__ void 
     }
 }
 
-template <int DK, int DV, typename T, int TOK, int MODE> __device__ __noinline__ void exact_outputs(const SegParams& s, float* sm, int bh, int c, int n) {
-    using E = SegExact<DK, DV, T, TOK>;
+template <int DK, int DV, typename T, int TOK, int CW, int MODE> __device__ __noinline__ void exact_outputs(const SegParams& s, float* sm, int bh, int c, int n) {
+    using E = SegExact<DK, DV, T, TOK, CW>;
     using L = typename E::L;
     constexpr int NTH = L::HT * L::HALVES, NV = rec::GROUP * L::JPT;
     const BiglaParams& p = s.p;
@@ -260,15 +260,15 @@ template <int DK, int DV, typename T, int TOK, int MODE> __device__ __noinline__
     }
 }
 
-template <int DK, int DV, typename T, int TOK> constexpr int seg_min_blocks() {
-    constexpr int fit = 225 * 1024 / (int)(SegSmem<DK, DV, T, TOK>::BYTES + 1024), regs = (DK == 16 ? 640 : 512) / (2 * TOK * SegWarps<DV, T, TOK>::CW);   // 128 registers a thread, 96 at DK = 16
+template <int DK, int DV, typename T, int TOK, int CW> constexpr int seg_min_blocks() {
+    constexpr int fit = 225 * 1024 / (int)(SegSmem<DK, DV, T, TOK, CW>::BYTES + 1024), regs = (DK == 16 ? 640 : 512) / (2 * TOK * CW);   // 128 registers a thread, 96 at DK = 16
     return fit < 1 ? 1 : fit < regs ? fit : regs;
 }
 
-template <int DK, int DV, typename T, int TOK, int MODE>
-__global__ void __launch_bounds__(2 * TOK * SegWarps<DV, T, TOK>::CW, seg_min_blocks<DK, DV, T, TOK>()) bigla_seg_kernel(const __grid_constant__ SegParams s) {
-    using SM = SegSmem<DK, DV, T, TOK>;
-    constexpr int RAW = SM::TT::RAW, SC = SM::TT::SC, CW = SegWarps<DV, T, TOK>::CW, NTH = 2 * TOK * CW, W = NTH / 32, DC = DV / CW;   // DC: a warp's value columns
+template <int DK, int DV, typename T, int TOK, int CW, int MODE>
+__global__ void __launch_bounds__(2 * TOK * CW, seg_min_blocks<DK, DV, T, TOK, CW>()) bigla_seg_kernel(const __grid_constant__ SegParams s) {
+    using SM = SegSmem<DK, DV, T, TOK, CW>;
+    constexpr int RAW = SM::TT::RAW, SC = SM::TT::SC, NTH = 2 * TOK * CW, W = NTH / 32, DC = DV / CW;   // DC: a warp's value columns
     constexpr int PAIRS = DK / 2, SUB = 32 / PAIRS, RPG = 16 / CW / SUB, MT = DK / 16;   // a warp's gates: 16 / CW rows, SUB groups of RPG
     constexpr uint32_t PK = Pitch<DK>::B, PV = Pitch<DV>::B, TK = TOK * PK, TV = TOK * PV, TS = DK * PV;   // TK, TV, TS: from term to term
     const BiglaParams& p = s.p;
@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(2 * TOK * SegWarps<DV, T, TOK>::CW, seg_min_bl
     if (RAW == 1) asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     if (MODE != SEG_OUT && s.need_states && bad) {
-        exact_contribution<DK, DV, T, TOK>(s, reinterpret_cast<float*>(smem), bh, c, n);
+        exact_contribution<DK, DV, T, TOK, CW>(s, reinterpret_cast<float*>(smem), bh, c, n);
     } else if (MODE != SEG_OUT && s.need_states) {                       // ---- contributions: units of 16 key channels x NC value columns of one direction
         constexpr int UNITS = 2 * MT, NSPLIT = W <= UNITS ? 1 : W / UNITS < DV / 8 ? W / UNITS : DV / 8, NC = DV / NSPLIT, NTL = NC / 8;
         for (int u = w; u < UNITS * NSPLIT; u += W) {
@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(2 * TOK * SegWarps<DV, T, TOK>::CW, seg_min_bl
     }
     if (!want_out) return;
     if (bad) {
-        exact_outputs<DK, DV, T, TOK, MODE>(s, reinterpret_cast<float*>(smem), bh, c, n);
+        exact_outputs<DK, DV, T, TOK, CW, MODE>(s, reinterpret_cast<float*>(smem), bh, c, n);
         return;
     }
     if (MODE == SEG_OUT || s.nseg > 1 || has_init) {                     // ---- entering states, scaled, over the K tiles
@@ -626,15 +626,15 @@ __global__ void __launch_bounds__(2 * TOK * SegWarps<DV, T, TOK>::CW, seg_min_bl
     }
 }
 
-template <int DK, int DV, typename T, int TOK, int MODE>
+template <int DK, int DV, typename T, int TOK, int CW, int MODE>
 int seg_launch_mode(const SegParams& s, cudaStream_t stream) {
-    auto kern = bigla_seg_kernel<DK, DV, T, TOK, MODE>;
-    constexpr uint32_t smem = SegSmem<DK, DV, T, TOK>::BYTES;
+    auto kern = bigla_seg_kernel<DK, DV, T, TOK, CW, MODE>;
+    constexpr uint32_t smem = SegSmem<DK, DV, T, TOK, CW>::BYTES;
     cudaError_t e = tc::ensure_smem_attr(reinterpret_cast<const void*>(kern), (int)smem);
     if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(s.nseg, s.p.B * s.p.H);
-    cfg.blockDim = dim3(2 * TOK * SegWarps<DV, T, TOK>::CW);
+    cfg.blockDim = dim3(2 * TOK * CW);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     if (MODE == SEG_OUT) return (int)launch_next(kern, cfg.gridDim, cfg.blockDim, smem, stream, s);
@@ -667,7 +667,7 @@ int seg_launch_mode(const SegParams& s, cudaStream_t stream) {
     return (int)(e != cudaSuccess ? e : cudaGetLastError());
 }
 
-template <int DK, int DV, typename T, int TOK>
+template <int DK, int DV, typename T, int TOK, int CW = seg_warps<DV, T, TOK>()>
 int seg_launch(SegParams& s, cudaStream_t stream) {
     constexpr int CLUSTER = 16;                          // largest cluster of the architecture (1x3x2048 dk = 32: 12 us in one launch, 16 in three)
     BiglaParams& p = s.p;
@@ -678,20 +678,31 @@ int seg_launch(SegParams& s, cudaStream_t stream) {
     s.need_states = s.nseg > 1 || s.finals;
     p.nchunk = s.nseg;
     p.ws_decay = p.ws_state ? p.ws_state + (size_t)p.B * p.H * s.nseg * 2 * DK * DV : nullptr;
-    if (s.nseg <= CLUSTER) {
-        const int r = seg_launch_mode<DK, DV, T, TOK, SEG_ONE>(s, stream);
-        if (r != SEG_NO_CLUSTER) return r;
+    if constexpr (CW < seg_warps<DV, T, TOK>()) {        // sequences of one segment
+        return seg_launch_mode<DK, DV, T, TOK, CW, SEG_ONE>(s, stream);
+    } else {
+        if (s.nseg <= CLUSTER) {
+            const int r = seg_launch_mode<DK, DV, T, TOK, CW, SEG_ONE>(s, stream);
+            if (r != SEG_NO_CLUSTER) return r;
+        }
+        if (int e = seg_launch_mode<DK, DV, T, TOK, CW, SEG_STATES>(s, stream)) return e;
+        if (int e = bigla_scan_launch(p, stream)) return e;
+        return p.o ? seg_launch_mode<DK, DV, T, TOK, CW, SEG_OUT>(s, stream) : 0;
     }
-    if (int e = seg_launch_mode<DK, DV, T, TOK, SEG_STATES>(s, stream)) return e;
-    if (int e = bigla_scan_launch(p, stream)) return e;
-    return p.o ? seg_launch_mode<DK, DV, T, TOK, SEG_OUT>(s, stream) : 0;
 }
 
+// 16-bit calls of dv = 64 have 64-token segments on a shared SM only where a sequence is one of them (bigla_seg_launch).  us with one warp / two to 16
+// rows at sequences x tokens: bf16 32/64 147 x 64 5.1 / 5.1, 198 x 64 5.9 / 6.4, 768 x 49 12.0 / 15.7, 1596 x 64 20.0 / 28.9; 64/64 147 x 64 6.8 / 6.6, 198 x 64 8.4 / 8.8, 399 x 64
+// 10.5 / 12.9; fp16 32/64 147 x 64 6.7 / 6.3, 198 x 49 7.7 / 8.3.
 template <int DK, int DV, typename T>
 int seg_launch_tok(SegParams& s, int tok, cudaStream_t stream) {
     if constexpr (SegTerms<DK, DV, T>::SC > 1) if (tok == 32) return seg_launch<DK, DV, T, 32>(s, stream);
-    if constexpr (sizeof(T) == 4 || DV == 32) return seg_launch<DK, DV, T, 64>(s, stream);
-    else return tok == 64 ? seg_launch<DK, DV, T, 64>(s, stream) : seg_launch<DK, DV, T, 128>(s, stream);
+    if constexpr (sizeof(T) == 4 || DV == 32) {
+        return seg_launch<DK, DV, T, 64>(s, stream);
+    } else {
+        if (s.p.L <= 64 && (int64_t)s.p.B * s.p.H > device_sms()) return seg_launch<DK, DV, T, 64, 1>(s, stream);
+        return tok == 64 ? seg_launch<DK, DV, T, 64>(s, stream) : seg_launch<DK, DV, T, 128>(s, stream);
+    }
 }
 
 template <typename T>
