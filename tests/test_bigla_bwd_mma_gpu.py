@@ -95,3 +95,43 @@ def test_few_chunks_sum_their_states_themselves(dtype, L, strong):
     got = torch.autograd.grad(vig_b200.bi_gla(*leaves, out_scale=0.5), leaves, d_out.cuda())
     errs = {n: rel_err(g.float(), r) for n, g, r in zip(NAMES, got, ref)}
     assert all(e < TOL[dtype] for e in errs.values()), errs
+
+
+@pytest.mark.parametrize("dtype,dk,dv", [(torch.float32, 64, 64), (torch.bfloat16, 64, 64), (torch.float16, 32, 64), (torch.bfloat16, 32, 32), (torch.bfloat16, 16, 32)])
+@pytest.mark.parametrize("L", [130, 250, 384, 448])
+@pytest.mark.parametrize("dirs", [3, 1, 2])
+def test_every_chunk_left_to_the_exact_form(dtype, dk, dv, L, dirs):
+    """The exact form's own sums of the states that other chunks contribute, with 3 to 6 chunks, and the launched ones with 7 (fp32: from 5)."""
+    import vig_b200
+    q, k, v, gf, gb = oracle.make_bigla_inputs(1, 2, L, dk, dv, seed=L + dk)
+    ins = [t.to(dtype) for t in (q, k, v, gf * 25, gb * 25)]
+    d_out = torch.randn(1, 2, L, dv, generator=torch.Generator().manual_seed(6)).to(dtype)
+    _, ref = _reference_grads(*[t.float() for t in ins], d_out.float(), 0.5, dirs)
+    if dirs == 3:
+        leaves = [t.cuda().requires_grad_() for t in ins]
+        got = torch.autograd.grad(vig_b200.bi_gla(*leaves, out_scale=0.5), leaves, d_out.cuda())
+    else:
+        got = vig_b200.bi_gla_backward(*[t.cuda() for t in (*ins, d_out)], out_scale=0.5, dir_mask=dirs)
+    errs = {n: rel_err(g.float(), r) for n, g, r in zip(NAMES, got, ref) if r is not None and g is not None}
+    assert all(e < TOL[dtype] for e in errs.values()), errs
+
+
+def test_exact_chunks_cost_the_same_with_and_without_a_launch_over_chunks():
+    """Backward per chunk, gates of all chunks out of range: 4 chunks sum the contributions in the exact form itself, 5 have a launch for it.  1.06 of it, 1.33
+    when each value was summed by itself."""
+    import vig_b200
+
+    def per_chunk(chunks):
+        q, k, v, d_out = (torch.randn(64, 3, 64 * chunks, 64, device="cuda") for _ in range(4))
+        g = torch.full_like(q, -4.0)
+        times = []
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            vig_b200.bi_gla_backward(q, k, v, g, g, d_out)
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times) / chunks
+    folded, launched = per_chunk(4), per_chunk(5)
+    assert folded < 1.2 * launched, (folded, launched)

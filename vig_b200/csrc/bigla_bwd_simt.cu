@@ -114,18 +114,59 @@ __global__ void __launch_bounds__(NT) bwd_chunk_states(BwdParams p) {
     }
 }
 
-// Value e of key channel d of the state (adj: of the adjoint state) entering chunk c
-__device__ __forceinline__ float entering(const BwdParams& p, bool adj, int bh, int c, int dir, int per, int d, int e) {
-    const float* U = adj ? p.ws_Z : p.ws_S;
-    if (p.scanned) return U[(((size_t)bh * p.nchunk + c) * 2 + dir) * per + e];
-    const bool down = (dir != 0) != adj;
-    float S = 0.f;
-#pragma unroll 1
-    for (int g = 0; g < (down ? p.nchunk - 1 - c : c); ++g) {
-        const size_t slot = ((size_t)bh * p.nchunk + (down ? p.nchunk - 1 - g : g)) * 2 + dir;
-        S = fmaf(S, exp2f(p.ws_decay[slot * p.dk + d]), U[slot * per + e]);
+// N values of a row from x; vec: on 16 bytes, as folded contributions are (vig_bigla_bwd_full)
+template <int N> __device__ __forceinline__ void load_row(float (&y)[N], const float* x, bool vec) {
+    if (N % 4 == 0 && vec) {
+#pragma unroll
+        for (int i = 0; i < N; i += 4) { const float4 t = *reinterpret_cast<const float4*>(x + i); y[i] = t.x; y[i + 1] = t.y; y[i + 2] = t.z; y[i + 3] = t.w; }
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; ++i) y[i] = x[i];
     }
-    return S;
+}
+
+// Values d * dv + e0 .. e0 + N - 1 of the state and of the adjoint state entering chunk c, and <state leaving the chunk, adjoint state entering from there>
+// over these.  Where no launch has summed the contributions (p.scanned = 0) they are summed here, a thread's values of both states at a time: one by one
+// each waited for the one before.  Training steps of bf16 64x3x384, 64/64, with the forward gates of every chunk out of range: 2180 us (one by one
+// 3980, a launch that sums them 2184), of one chunk 461 (725, 531).
+template <int N> __device__ __forceinline__ float entering(float (&S)[N], float (&Z)[N], const BwdParams& p, int bh, int c, int dir, int d, int e0) {
+    const int per = p.dk * p.dv, at = d * p.dv + e0, next = dir ? c - 1 : c + 1;
+    const size_t row = (size_t)bh * p.nchunk;
+    const bool goes_on = next >= 0 && next < p.nchunk;
+    float leaving[N], past = 0.f;
+    if (p.scanned) {
+        load_row(S, p.ws_S + ((row + c) * 2 + dir) * per + at, false);
+        load_row(Z, p.ws_Z + ((row + c) * 2 + dir) * per + at, false);
+        if (goes_on) load_row(leaving, p.ws_S + ((row + next) * 2 + dir) * per + at, false);
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; ++i) S[i] = Z[i] = 0.f;
+        const int before = dir ? p.nchunk - 1 - c : c, behind = p.nchunk - 1 - before;   // chunks scanned ahead of this one, and after it
+#pragma unroll 1
+        for (int g = 0; g < max(before, behind); ++g) {
+            const size_t sa = (row + (dir ? p.nchunk - 1 - g : g)) * 2 + dir, sz = (row + (dir ? g : p.nchunk - 1 - g)) * 2 + dir;
+            float x[N], y[N], a = 0.f, z = 0.f;
+            if (g < before) { load_row(x, p.ws_S + sa * per + at, true); a = p.ws_decay[sa * p.dk + d]; }
+            if (g < behind) { load_row(y, p.ws_Z + sz * per + at, true); z = p.ws_decay[sz * p.dk + d]; }
+            a = exp2f(a); z = exp2f(z);
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                if (g < before) S[i] = fmaf(S[i], a, x[i]);
+                if (g < behind) Z[i] = fmaf(Z[i], z, y[i]);
+            }
+        }
+        if (goes_on) {
+            load_row(leaving, p.ws_S + ((row + c) * 2 + dir) * per + at, true);
+            const float a = exp2f(p.ws_decay[((row + c) * 2 + dir) * p.dk + d]);
+#pragma unroll
+            for (int i = 0; i < N; ++i) leaving[i] = fmaf(S[i], a, leaving[i]);
+        }
+    }
+    if (goes_on) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) past = fmaf(leaving[i], Z[i], past);
+    }
+    return past;
 }
 
 // ---- phase C: gradients of one chunk -----------------------------------------------------------------------------
@@ -143,6 +184,7 @@ __global__ void __launch_bounds__(NT) bwd_chunk_grads(BwdParams p, int flagged_o
     float* sv = sdk + CH * DK;
     float* sdo = sv + CH * DV;
     float* sdv = sdo + CH * DV;
+    __shared__ float carry[DK];            // gradient of the log-gates just past the chunk
     pdl_wait();
     const bool have_states = !flagged_only || p.nchunk > 1;          // the tensor-core form leaves the states of a lone chunk unwritten (zero)
     const int items = p.nchunk * p.B * p.H;
@@ -173,11 +215,46 @@ __global__ void __launch_bounds__(NT) bwd_chunk_grads(BwdParams p, int flagged_o
         const size_t slot = ((size_t)bh * p.nchunk + c) * 2 + dir;
         __syncthreads();
         load_gates_exp<DK, T>(sg, p, dir, b, h, t0, n, nullptr);
-        {   // layout B: dq from the rebuilt state (scan order), then dk from Z (reverse scan order)
-            const int d = threadIdx.x / Bl::TPB, s = threadIdx.x % Bl::TPB;
-            float st[Bl::JPT];
+        const int d = threadIdx.x / Bl::TPB, s = threadIdx.x % Bl::TPB;
+        float st[Bl::JPT], adj[Bl::JPT], past = 0.f;
 #pragma unroll
-            for (int jj = 0; jj < Bl::JPT; ++jj) st[jj] = have_states ? entering(p, false, bh, c, dir, DK * DV, d, d * DV + s * Bl::JPT + jj) : 0.f;
+        for (int jj = 0; jj < Bl::JPT; ++jj) st[jj] = adj[jj] = 0.f;
+        if (have_states) past = entering(st, adj, p, bh, c, dir, d, s * Bl::JPT);
+#pragma unroll
+        for (int m = 1; m < Bl::TPB; m <<= 1) past += __shfl_xor_sync(0xffffffffu, past, m);
+        if (s == 0) carry[d] = past;
+        {   // layout A: dv from Z (reverse scan order)
+            const int j = threadIdx.x / A::TPC, s = threadIdx.x % A::TPC;
+            float st[A::DPT];
+#pragma unroll
+            for (int dd = 0; dd < A::DPT; ++dd) st[dd] = have_states && p.scanned ? p.ws_Z[slot * DK * DV + (s * A::DPT + dd) * DV + j] : 0.f;
+            if constexpr (DK * DV <= CH * DK) {
+                if (have_states && !p.scanned) {                         // summed by the threads of layout B; se is not in use yet
+#pragma unroll
+                    for (int jj = 0; jj < Bl::JPT; ++jj) se[threadIdx.x * Bl::JPT + jj] = adj[jj];
+                    __syncthreads();
+#pragma unroll
+                    for (int dd = 0; dd < A::DPT; ++dd) st[dd] = se[(s * A::DPT + dd) * DV + j];
+                    __syncthreads();
+                }
+            }
+            for (int ii = n - 1; ii >= 0; --ii) {
+                const int i = dir ? n - 1 - ii : ii;
+                const float dj = p.c * sdo[i * DV + j];
+                float acc = 0.f;
+#pragma unroll
+                for (int dd = 0; dd < A::DPT; ++dd) {
+                    const int d = s * A::DPT + dd;
+                    const float ds = fmaf(sq[i * DK + d], dj, st[dd]);
+                    acc = fmaf(sk[i * DK + d], ds, acc);
+                    st[dd] = ds * sg[i * DK + d];
+                }
+#pragma unroll
+                for (int m = 1; m < A::TPC; m <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
+                if (s == 0) sdv[i * DV + j] += acc;
+            }
+        }
+        {   // layout B: dq from the rebuilt state (scan order), then dk from Z (reverse scan order)
             for (int ii = 0; ii < n; ++ii) {
                 const int i = dir ? n - 1 - ii : ii;
                 const float a = sg[i * DK + d], kd = sk[i * DK + d];
@@ -196,8 +273,6 @@ __global__ void __launch_bounds__(NT) bwd_chunk_grads(BwdParams p, int flagged_o
                     se[i * DK + d] = dqd * sq[i * DK + d];
                 }
             }
-#pragma unroll
-            for (int jj = 0; jj < Bl::JPT; ++jj) st[jj] = have_states ? entering(p, true, bh, c, dir, DK * DV, d, d * DV + s * Bl::JPT + jj) : 0.f;
             for (int ii = n - 1; ii >= 0; --ii) {
                 const int i = dir ? n - 1 - ii : ii;
                 const float a = sg[i * DK + d], cq = p.c * sq[i * DK + d];
@@ -205,9 +280,9 @@ __global__ void __launch_bounds__(NT) bwd_chunk_grads(BwdParams p, int flagged_o
 #pragma unroll
                 for (int jj = 0; jj < Bl::JPT; ++jj) {
                     const int j = s * Bl::JPT + jj;
-                    const float ds = fmaf(cq, sdo[i * DV + j], st[jj]);
+                    const float ds = fmaf(cq, sdo[i * DV + j], adj[jj]);
                     acc = fmaf(ds, sv[i * DV + j], acc);
-                    st[jj] = ds * a;
+                    adj[jj] = ds * a;
                 }
 #pragma unroll
                 for (int m = 1; m < Bl::TPB; m <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
@@ -217,43 +292,17 @@ __global__ void __launch_bounds__(NT) bwd_chunk_grads(BwdParams p, int flagged_o
                 }
             }
         }
-        {   // layout A: dv from Z (reverse scan order)
-            const int j = threadIdx.x / A::TPC, s = threadIdx.x % A::TPC;
-            float st[A::DPT];
-#pragma unroll
-            for (int dd = 0; dd < A::DPT; ++dd) st[dd] = have_states ? entering(p, true, bh, c, dir, DK * DV, s * A::DPT + dd, (s * A::DPT + dd) * DV + j) : 0.f;
-            for (int ii = n - 1; ii >= 0; --ii) {
-                const int i = dir ? n - 1 - ii : ii;
-                const float dj = p.c * sdo[i * DV + j];
-                float acc = 0.f;
-#pragma unroll
-                for (int dd = 0; dd < A::DPT; ++dd) {
-                    const int d = s * A::DPT + dd;
-                    const float ds = fmaf(sq[i * DK + d], dj, st[dd]);
-                    acc = fmaf(sk[i * DK + d], ds, acc);
-                    st[dd] = ds * sg[i * DK + d];
-                }
-#pragma unroll
-                for (int m = 1; m < A::TPC; m <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
-                if (s == 0) sdv[i * DV + j] += acc;
-            }
-        }
         __syncthreads();
         if (float* e_dir = dir ? p.eb : p.ef) {
             float* e_out = e_dir + ((size_t)bh * p.L + t0) * DK;
             for (int idx = threadIdx.x; idx < n * DK; idx += NT) e_out[idx] = se[idx];
         }
         if (void* dg = dir ? p.dgb : p.dgf) {
-            // finished gate gradient: the value just past the chunk, <state leaving the chunk, adjoint state entering from
-            // there>, plus the sum of e over the tokens scanned at or after t; then the derivative of the gate transform
-            const int next = dir ? c - 1 : c + 1;
+            // finished gate gradient: the value just past the chunk plus the sum of e over the tokens scanned at or after t;
+            // then the derivative of the gate transform
             if (threadIdx.x < DK) {
                 const int d = threadIdx.x;
-                float run = 0.f;
-                if (have_states && next >= 0 && next < p.nchunk) {
-                    for (int j = 0; j < DV; ++j)
-                        run = fmaf(entering(p, false, bh, next, dir, DK * DV, d, d * DV + j), entering(p, true, bh, c, dir, DK * DV, d, d * DV + j), run);
-                }
+                float run = carry[d];
                 for (int ii = n - 1; ii >= 0; --ii) {
                     const int i = dir ? n - 1 - ii : ii;
                     run += se[i * DK + d];
