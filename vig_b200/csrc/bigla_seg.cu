@@ -674,7 +674,6 @@ int seg_launch(SegParams& s, cudaStream_t stream) {
     s.nseg = (p.L + TOK - 1) / TOK;
     s.seglen = ((p.L + s.nseg - 1) / s.nseg + 15) / 16 * 16;   // even segments: no nearly empty last one
     s.nseg = (p.L + s.seglen - 1) / s.seglen;
-    s.finals = p.final_f || p.final_b || p.logdecay_f || p.logdecay_b;
     s.need_states = s.nseg > 1 || s.finals;
     p.nchunk = s.nseg;
     p.ws_decay = p.ws_state ? p.ws_state + (size_t)p.B * p.H * s.nseg * 2 * DK * DV : nullptr;
@@ -755,6 +754,7 @@ size_t bigla_seg_workspace(int B, int H, int L, int dk, int dv, int dtype) {
 int bigla_seg_launch(const BiglaParams& p, size_t ws_bytes, cudaStream_t stream) {
     SegParams s{};
     s.p = p;
+    s.finals = p.final_f || p.final_b || p.logdecay_f || p.logdecay_b;
     // 64-token segments where more SMs can share the work of few sequences (1x3x196 dk = 64: 11 us against 13) and for dv = 32,
     // whose segments are too little work for eight warps (64x12x196 dk = 16: 46 us against 56; 64x6x784 91 / 114, 64x3x3136 154 / 215; dk = 32 161 / 155);
     // otherwise 128, half as many states.  Clusters of more than eight want room around them: fp16 32/64 1x3x836 12.6 / 16.7, bf16 1x3x1024
@@ -764,9 +764,13 @@ int bigla_seg_launch(const BiglaParams& p, size_t ws_bytes, cudaStream_t stream)
     // segments) 12.4 / 11.5, 1x3x512 11.3 / 11.3, 64/64 1x6x196 13.1 / 13.7, 1x3x400 15.9 / 14.2; bf16 32/32 2x12x128 7.8 / 9.0; fp16 16/32 1x24x49 6.5 / 5.9, 1x24x98 6.8 / 7.4.
     // One-term operands gain nothing: bf16 1x3x196 32/64 8.4 / 8.5,
     // 1x12x196 64/64 11.9 / 11.1.
+    // Final states are summed over all segments by the one scanned last, so there calls take fewer.  One direction with states at both ends, 32 / 64 tokens: fp16 64/64
+    // 3x100 15.8 / 11.1, 3x196 18.4 / 12.6, 32/64 3x196 11.0 / 8.4; fp32 64/64 3x100 11.4 / 12.1, 6x300 13.7 / 13.3, 6x512 18.9 / 18.3, 16/32 6x512 8.8 / 8.1; 64 / 128
+    // tokens: bf16 64/64 3x700 15.5 / 13.8, 6x1000 18.4 / 16.9, 32/64 6x700 10.5 / 9.3; fp16 64/64 6x700 17.1 / 15.8, 32/64 6x850 11.7 / 12.3.
     const int64_t BH = (int64_t)p.B * p.H;
-    const int tok = seg_fine(p.dtype, p.dv, p.L) && 3 * BH * ((p.L + 31) / 32) <= 2 * device_sms() && ws_bytes >= seg_fine_bytes(BH, p.L, p.dk, p.dv) ? 32
-                    : p.dtype == VIG_DTYPE_F32 || p.dv == 32 || p.L <= 64 || (p.L <= 1024 && 3 * BH * ((p.L + 63) / 64) <= (p.L <= 512 ? 3 : 2) * device_sms()) ? 64 : 128;
+    const bool fine = seg_fine(p.dtype, p.dv, p.L) && !(s.finals && (p.L > 256 || (p.dtype == VIG_DTYPE_F16 && p.dv == 64)));
+    const int tok = fine && 3 * BH * ((p.L + 31) / 32) <= 2 * device_sms() && ws_bytes >= seg_fine_bytes(BH, p.L, p.dk, p.dv) ? 32
+                    : p.dtype == VIG_DTYPE_F32 || p.dv == 32 || p.L <= 64 || (p.L <= (s.finals ? 512 : 1024) && 3 * BH * ((p.L + 63) / 64) <= (p.L <= 512 ? 3 : 2) * device_sms()) ? 64 : 128;
     switch (p.dtype) {
         case VIG_DTYPE_F32: return seg_launch_dims<float>(s, tok, stream);
         case VIG_DTYPE_BF16: return seg_launch_dims<__nv_bfloat16>(s, tok, stream);
