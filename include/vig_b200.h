@@ -59,7 +59,7 @@ extern "C" {
                               CTA per SM, states handed from segment to segment; built for batches with at least as
                               many (sequence, direction) chains as the GPU has SMs */
 
-#define VIG_IMPL_SEG 6       /* mma.sync form, both directions of a 64- or 128-token segment in one sweep ((dk, dv) of (16,32), (32,32),
+#define VIG_IMPL_SEG 6       /* mma.sync form, both directions of a 32-, 64- or 128-token segment in one sweep ((dk, dv) of (16,32), (32,32),
                               (32,64), (64,64), every type) */
 
 VIG_API int vig_version(void);
@@ -235,7 +235,8 @@ VIG_API int vig_dwconv3x3_halo_fwd(const void* x, const void* top, const void* b
  * (classification/models/vig.py:283-290, 431-439), so their weights are stacked into one [N, K] matrix.
  * x: [M, K] rows ldx elements apart, w: [N, K] contiguous, bias: [N] or NULL, out: [M, N] rows ldo apart; bf16 / fp16.
  * vig_linear_bias_supported: K % 64 == 0, K <= 192, N % 8 == 0 and at least 256 rows per SM of the current device
- * (smaller problems are left to a library GEMM).  status_dev: optional int32 on the device, bit 0 = a bounded wait ran out.
+ * (smaller problems are left to a library GEMM).  The call refuses more than 192 columns per SM (VIG_ERR_SHAPE).  status_dev: optional int32 on the
+ * device, bit 0 = a bounded wait ran out.
  * vig_linear_pair_fwd: the same for any K that is a multiple of 64 and any M; ``preferred``: whether it beats a library GEMM.
  */
 VIG_API int vig_linear_pair_preferred(int64_t M, int K, int N, int dtype);

@@ -222,3 +222,13 @@ def test_pair_linear(dtype, M, K, N, biased):
     ref = torch.nn.functional.linear(x.float(), w.float(), None if b is None else b.float())
     assert rel_err(out[:, :N].float(), ref) < (4e-3 if dtype == torch.bfloat16 else 5e-4)
     assert _lib.lib().vig_linear_pair_fwd(_lib.ptr(x), K + 8, _lib.ptr(w), _lib.ptr(b), _lib.ptr(out), N + 8, M, K - 8, N, _lib.dtype_code(x), None, _lib.stream_ptr()) == -2
+
+
+def test_linear_bias_refuses_what_it_refused():
+    """``vig_linear_bias_fwd`` takes up to 192 columns for each SM; ``vig_linear_pair_fwd`` any number."""
+    from vig_b200 import _lib
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    M, K, N = 256 * sms, 64, 192 * sms + 8
+    x, w, out = (torch.empty(*s, device="cuda", dtype=torch.bfloat16) for s in ((M, K), (N, K), (M, N)))
+    call = lambda n: _lib.lib().vig_linear_bias_fwd(_lib.ptr(x), K, _lib.ptr(w), None, _lib.ptr(out), N, M, K, n, _lib.dtype_code(x), None, _lib.stream_ptr())  # noqa: E731
+    assert call(N) == -2 and call(N - 8) == 0

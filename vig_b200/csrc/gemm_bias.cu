@@ -25,7 +25,7 @@ extern "C" int vig_linear_bias_fwd(const void* x, int64_t ldx, const void* w, co
                                    int64_t M, int K, int N, int dtype, int32_t* status_dev, void* stream) {
     if (!x || !w || !out) return VIG_ERR_NULL;
     if (M == 0) return VIG_OK;
-    if (!vig_linear_bias_supported(M, K, N, dtype)) return VIG_ERR_SHAPE;
+    if (!vig_linear_bias_supported(M, K, N, dtype) || (N + 191) / 192 > device_sms()) return VIG_ERR_SHAPE;
     return lb_launch(x, ldx, w, bias, out, ldo, M, K, N, dtype, status_dev, stream);
 }
 
