@@ -65,3 +65,34 @@ def test_overlapping_launches_give_the_same_bits(dtype, side):
     assert bool(apart[-1].isfinite().all())
     for _ in range(20):
         assert all(torch.equal(a, b) for a, b in zip(forward(1), apart))
+
+
+@pytest.mark.parametrize("more", [0, 1])
+def test_scans_of_more_segments_than_sms_wait_for_the_launch_ahead(more, tmp_path):
+    """A chained scan begins under the end of the launch ahead of it only while each segment has an SM of its own."""
+    import json
+    from vig_b200 import _lib, ops
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    x, taps = torch.randn(128, 64, 192, device="cuda").bfloat16(), torch.randn(9, 192, device="cuda").bfloat16()
+    q, k, gf, gb = (torch.randn(sms + more, 1, 64, 32, device="cuda").bfloat16() for _ in range(4))
+    v = torch.randn(sms + more, 1, 64, 64, device="cuda").bfloat16()
+    o, graph = torch.empty_like(v), torch.cuda.CUDAGraph()
+
+    def both():
+        y = ops.dwconv3x3(x, taps, None, (8, 8), True)
+        was = _lib.lib().vig_chain_launches(1)
+        ops.bi_gla(q, k, v, gf, gb, gate_logit_normalizer=16.0, out=o)
+        _lib.lib().vig_chain_launches(was)
+        return y
+    both()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        both()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        for _ in range(5):
+            graph.replay()
+            torch.cuda.synchronize()
+    prof.export_chrome_trace(str(tmp_path / "trace.json"))
+    events = sorted((e for e in json.load(open(tmp_path / "trace.json"))["traceEvents"] if e.get("cat") == "kernel"), key=lambda e: e["ts"])
+    ahead = [b["ts"] < a["ts"] + a["dur"] - 0.05 for a, b in zip(events, events[1:]) if "dwconv" in a["name"] and "bigla_seg" in b["name"]]
+    assert len(ahead) == 5 and any(ahead) == (not more), ahead

@@ -661,8 +661,13 @@ int seg_launch_mode(const SegParams& s, cudaStream_t stream) {
         if (!(have & yes)) return SEG_NO_CLUSTER;
     }
     // Begins before the launch ahead of it ends, and reads its inputs coherently for that reason (ViG-T of one 224 x 224 image 253 -> 248 us a forward).  Not
-    // the first of three launches: the later ones read the inputs before they wait, for launches of this call only.
-    if (MODE == SEG_ONE && chain_launches) { attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1; }
+    // the first of three launches: the later ones read the inputs before they wait, for launches of this call only.  Nor with more segments than SMs: they
+    // crowd on the SMs that the projection ahead leaves idle, and the block tail behind finds its SMs late (ViG-T bf16, 128 x 128 x 128: 626 - 637 us
+    // chained, in 9 of 9 processes; 598 - 603 in 11 of 17 otherwise, 619 - 634 in the others; 32 of 224 x 224: 651 - 660 in 4 of 4, 635 - 638 in 8 of 12).
+    if (MODE == SEG_ONE && chain_launches && (int64_t)s.nseg * s.p.B * s.p.H <= device_sms()) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
     e = cudaLaunchKernelEx(&cfg, kern, s);
     return (int)(e != cudaSuccess ? e : cudaGetLastError());
 }
