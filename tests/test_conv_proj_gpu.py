@@ -96,3 +96,29 @@ def test_scans_of_more_segments_than_sms_wait_for_the_launch_ahead(more, tmp_pat
     events = sorted((e for e in json.load(open(tmp_path / "trace.json"))["traceEvents"] if e.get("cat") == "kernel"), key=lambda e: e["ts"])
     ahead = [b["ts"] < a["ts"] + a["dur"] - 0.05 for a, b in zip(events, events[1:]) if "dwconv" in a["name"] and "bigla_seg" in b["name"]]
     assert ahead and any(ahead) == (not more), ahead          # the profiler may lose a replay
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("L", [40, 100])
+def test_overlapping_scans_continue_from_each_others_states(dtype, L):
+    """Each call begins under the end of the one that writes the state it starts from, in one of two buffers in turn."""
+    import vig_b200
+    from vig_b200 import _lib
+    gen = torch.Generator(device="cuda").manual_seed(L)
+    rand = lambda *s: torch.randn(*s, generator=gen, device="cuda")  # noqa: E731
+    q, k, v = (rand(2, 3, L, 64).to(dtype) for _ in range(3))
+    g = (torch.nn.functional.logsigmoid(rand(2, 3, L, 64)) / 16).to(dtype)
+    start = rand(2, 3, 64, 64)
+
+    def stream(on):
+        h, outs = start, []
+        was = _lib.lib().vig_chain_launches(on)
+        with torch.no_grad():
+            for _ in range(30):
+                o, h = vig_b200.fused_chunk_gla(q, k, v, g, initial_state=h, output_final_state=True)   # h: a buffer that the call before last has read
+                outs.append(o)
+        _lib.lib().vig_chain_launches(was)
+        torch.cuda.synchronize()
+        return outs
+    apart = stream(0)
+    assert all(all(torch.equal(a, b) for a, b in zip(stream(1), apart)) for _ in range(10))

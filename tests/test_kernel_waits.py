@@ -52,3 +52,9 @@ def test_no_cta_leaves_before_its_peer_has_written_to_it(body):
             opener -= 1
             depth += {"}": 1, "{": -1}.get(body[opener], 0)
         assert re.search(r"if \(both\) $", body[:opener]), body[max(0, opener - 60):opener]
+
+
+def test_scans_read_what_may_still_be_written_coherently():
+    """The one-launch scan may begin before the launch that writes what it reads, states included: no load of it goes through the non-coherent path."""
+    text = open(os.path.join(CSRC, "bigla_seg.cu")).read()
+    assert not re.findall(r"__ldg\(|ld\.global\.nc", re.sub(r"//[^\n]*", "", text))

@@ -113,7 +113,7 @@ template <int DK, int DV, int MODE> __device__ __forceinline__ float4 entering(c
     constexpr int per = DK * DV / 4;
     if (MODE == SEG_OUT) return __ldcg(U + (((size_t)bh * s.nseg + c) * 2 + dir) * per + e4);
     const float* init = dir ? p.init_b : p.init_f;
-    float4 S = init ? __ldg(reinterpret_cast<const float4*>(init) + (size_t)bh * per + e4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 S = init ? __ldcg(reinterpret_cast<const float4*>(init) + (size_t)bh * per + e4) : make_float4(0.f, 0.f, 0.f, 0.f);
     const int d = e4 * 4 / DV, m = dir ? s.nseg - 1 - c : c;
 #pragma unroll 4
     for (int i = 0; i < m; ++i) {
@@ -570,7 +570,7 @@ __global__ void __launch_bounds__(2 * TOK * CW, seg_min_blocks<DK, DV, T, TOK, C
                 for (int k = 0; k < KB; ++k) {
                     const int i = i0 + k * NTH;
                     S[k] = MODE == SEG_OUT ? __ldcg(reinterpret_cast<const float4*>(p.ws_state) + (((size_t)bh * s.nseg + c) * 2 + dir) * (DK * DV / 4) + i)
-                           : init ? __ldg(reinterpret_cast<const float4*>(init) + (size_t)bh * (DK * DV / 4) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                           : init ? __ldcg(reinterpret_cast<const float4*>(init) + (size_t)bh * (DK * DV / 4) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
 #pragma unroll 2
                 for (int g = 0; g < m; ++g) {
