@@ -9,9 +9,9 @@
 //   dV = A^T dO + Kt (2^(l-r) Z)                   e  = dQ q - dK k
 //   dg_t = <S_next, Z> over value columns + sum of e over the chunk's tokens scanned at or after t
 // The first term of dg is the gate gradient just past the chunk: d loss / d g_T = <a_T S_{T-1}, D_T> = <S_{T-1}, Z_T>, so no
-// sum ever runs over the whole sequence.  Three launches: chunk states (U = (k 2^(l-G))^T V and its adjoint), a scan over
-// chunks (a few chunks: none, the gradients sum what they need), chunk gradients.  A chunk whose |G - r| exceeds the range set below raises its flag and is left to the exact
-// token-by-token kernel, which runs afterwards and returns at once for every other chunk.
+// sum ever runs over the whole sequence.  Launches: chunk states (U = (k 2^(l-G))^T V and its adjoint; not for a lone chunk); a scan over
+// chunks, where there are more than a few (bwd_fold: fewer are summed by the gradients themselves); chunk gradients; and the exact token-by-token
+// kernel, to which a chunk is left whose |G - r| exceeds the range set below (it raises its flag), and which returns at once for every other chunk.
 #include "bigla_bwd.cuh"
 #include "bigla_exact.cuh"
 
@@ -263,7 +263,8 @@ template <int DK, int DV, typename T> constexpr int grads_min_blocks() {
 // and dv of the first, 64 of 128 registers at 64 / 64, alive through the products of the second: the spills were as long as the
 // second reading of v and dO is now, and left no registers to ask for the states ahead of a barrier or to keep q, k and the gates
 // (backward of 8 x 6 x 4096, bf16: 513 -> 488 us; 128 x 6 x 196: 531 -> 499; 128 x 3 x 196, 32 / 64, where nothing spilled, 148 -> 150).
-// Bound: latency at 16 warps an SM and shared memory's rate (59 % of it; ldmatrix two thirds of that); the tensor pipe is 27 % busy.
+// Bound, 64 / 64 in 16 bits: latency at 16 warps an SM and shared memory's rate (59 % of it; ldmatrix two thirds of that); the tensor pipe is 27 % busy.
+// Smaller heads have 24 or 32 warps an SM (grads_min_blocks), fp32 has 8.
 // Eight warps: warps 0 - 3 form dQ and dV inside the chunk, warps 4 - 7 dK and the state's part of dV, 16 rows each: 160 - 288
 // products a warp and direction; dV on the other side makes it 136 - 352.  What follows the products -- the factors 2^(G-r), e
 // and its sums -- is done by channel pairs, in which q, k and the gates are read coalesced.

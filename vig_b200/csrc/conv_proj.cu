@@ -138,7 +138,10 @@ extern "C" int vig_conv_proj_supported(int64_t M, int C, int N, int dtype) {
 }
 
 // As long as every CTA has an SM of its own.  Whole forwards in us, one launch / two: ViG-T (768 columns) 64 tokens 215 / 237, 196 tokens 249 / 277, 392
-// tokens (100 CTAs) 273 / 279, 784 tokens (1152 columns, 294 CTAs) 340 / 337, 2508 tokens 549 / 478; widths of 384 (196 tokens) 404 / 392.
+// tokens (100 CTAs) 273 / 279, 784 tokens (1152 columns, 294 CTAs) 340 / 337, 2508 tokens 549 / 478.  Width 96 (the hierarchical model's first stage, images
+// of up to about 96 x 96; 384 columns): the two blocks of the stage 61.7 / 65.9 at 576 tokens (144 CTAs), 54.9 / 60.2 at 512.  By themselves, one behind the
+// other: width 96 256 tokens 3.2 / 5.6, 576 3.4 / 5.9; width 192, 768 columns, 576 5.0 / 5.9, 1024 (256 CTAs) 6.9 / 6.2.  Width 384 was slower (196 tokens, a
+// forward 404 / 392) and is not built.
 extern "C" int vig_conv_proj_preferred(int64_t M, int C, int N, int dtype) {
     return vig_conv_proj_supported(M, C, N, dtype) && (M + CP_TOKENS - 1) / CP_TOKENS * (N / C) <= device_sms();
 }
